@@ -130,6 +130,32 @@ def lib() -> ctypes.CDLL:
     return _LIB
 
 
+BINDING_PATH = os.path.join(_HERE, "lib", "b200lora_binding.so")
+_NATIVE = None
+
+
+def native():
+    """The compiled host path of the operators (``csrc/binding.cpp``), bound to the loaded C-ABI library. Its functions
+    return None for argument combinations they leave to the Python form of the same call."""
+    global _NATIVE
+    if _NATIVE is None:
+        if not os.path.exists(BINDING_PATH):
+            raise NativeLibraryError(f"{BINDING_PATH} is missing: build it with `python -m nanovllm_voxcpm_b200.build`")
+        import importlib.machinery
+        import importlib.util
+
+        from .lora import SGMV_MIN_TOKENS, scratch_for
+
+        loader = importlib.machinery.ExtensionFileLoader("b200lora_binding", BINDING_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200lora_binding", loader))
+        loader.exec_module(module)
+        handle = lib()
+        addresses = {name: ctypes.cast(getattr(handle, name), c_void_p).value for name in _SIGNATURES}
+        module.bind(addresses, scratch_for, SGMV_MIN_TOKENS)
+        _NATIVE = module
+    return _NATIVE
+
+
 def exported_symbols() -> list[str]:
     return list(_SIGNATURES)
 

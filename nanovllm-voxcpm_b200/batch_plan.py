@@ -13,6 +13,7 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
+from . import _native as N
 from .context import LoRAContext
 
 
@@ -31,6 +32,9 @@ def bucket_arrays(token_to_slot) -> tuple[list[int], list[int], list[int], list[
 
     Stable counting sort: ascending slot id, original order inside a slot, rows with
     slot < 0 left out (``engine/lora_manager.py:77-91``)."""
+    got = N.native().bucket_lists(token_to_slot)
+    if got is not None:
+        return got
     tts = np.asarray(token_to_slot, dtype=np.int64).reshape(-1)
     rows = np.nonzero(tts >= 0)[0]
     if rows.size == 0:
@@ -57,13 +61,17 @@ def expand_token_counts(slots_per_seq: list[int], token_counts: list[int]) -> li
 def _to_device_packed(lists: list[list[int]], device) -> list[torch.Tensor]:
     """All int lists in ONE pinned buffer and one H2D copy; views are returned
     (``engine/lora_manager.py:118-146``)."""
+    dev = torch.device(device)
+    index = -1 if dev.type != "cuda" else dev.index if dev.index is not None else torch.cuda.current_device()
+    views = N.native().pack_lists(lists, index)
+    if views is not None:
+        return views
     sizes = [len(x) for x in lists]
     total = sum(sizes)
     if total == 0:
         return [torch.empty(0, dtype=torch.int32, device=device) for _ in lists]
     flat = np.concatenate([np.asarray(x, dtype=np.int32) for x in lists if len(x)])
     host = torch.from_numpy(flat)
-    dev = torch.device(device)
     if dev.type == "cuda":
         host = host.pin_memory()
     packed = host.to(dev, non_blocking=True)
@@ -151,8 +159,6 @@ class GraphLoRABuffers:
         """Same buffers as :meth:`load_plan`, built on the GPU from a device-resident slot map in two
         launches (a copy and ``lora_b200_build_metadata``): no Python loop over the rows, no staging
         copy, nothing to synchronise. Slot ids outside the graph slots count as "no adapter"."""
-        from . import _native as N
-
         n = token_to_slot.numel()
         rows = self.token_to_slot.numel()
         if n > rows:

@@ -27,6 +27,11 @@ def add_rms_norm(x: torch.Tensor, residual: torch.Tensor | None, weight: torch.T
     Returns ``(normed, hidden)``; ``hidden`` is ``None`` without a residual. ``hidden_out`` may be ``residual``
     itself (in place). ``norm_of_rounded_sum=False`` gives ``RMSNorm.add_rms_forward``'s rounding.
     """
+    if out is None and hidden_out is None:
+        got = N.native().add_rms_norm(x, residual, weight, eps, norm_of_rounded_sum)
+        if got is not None:
+            N.check(got[0])
+            return got[1], got[2]
     N.require_cuda(x, residual, weight, out, hidden_out)
     shape = x.shape
     x2 = _rows(x.reshape(-1, shape[-1]), "x")
@@ -70,6 +75,11 @@ class RMSNorm(nn.Module):
 
 
 def silu_and_mul(x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    if out is None:
+        got = N.native().silu_mul(x)
+        if got is not None:
+            N.check(got[0])
+            return got[1]
     N.require_cuda(x, out)
     shape = x.shape
     if shape[-1] % 2:
@@ -102,6 +112,10 @@ def rope_kv_store(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, head_dim
     head_dim / 2]``; ``positions`` int64. Without them nothing is rotated. ``slot_mapping`` int32, -1 = skip;
     the caches are ``[..., kv_heads, head_dim]`` contiguous.
     """
+    got = N.native().rope_kv_store(qkv, num_heads, num_kv_heads, head_dim, positions, cos, sin, k_cache, v_cache, slot_mapping)
+    if got is not None:
+        N.check(got[0])
+        return got[1], got[2], got[3]
     N.require_cuda(qkv, positions, cos, sin, k_cache, v_cache, slot_mapping)
     qkv2 = _rows(qkv, "qkv")
     T = qkv2.size(0)

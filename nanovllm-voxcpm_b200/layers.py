@@ -29,6 +29,7 @@ import torch.nn.functional as F
 
 from .context import LM_LORA_DOMAIN, get_lora_context, set_lora_context
 from .distributed import get_tp_rank, get_tp_world_size
+from . import lora as _lora
 from .lora import B200LoRABackend, LoRAMetadata, get_backend
 
 
@@ -86,6 +87,23 @@ class _LoRALayerBase(nn.Module):
         """(width, first output column) of every LoRA slice inside the layer output."""
         raise NotImplementedError
 
+    def _active_slices(self) -> tuple[list, list, list[int], list[int]]:
+        """(lora_A, lora_B, widths, columns) of the slices that have rows, as a launch takes them. The views are made once
+        (indexing a stacked ``lora_A`` costs microseconds per slice) and again whenever a slab parameter was replaced
+        or its storage moved."""
+        params = self._parameters
+        plan = self.__dict__.get("_slices_plan")
+        if plan is not None and all(params.get(name) is p and p.data_ptr() == ptr for name, p, ptr in plan[0]):
+            return plan[1]
+        widths, cols = self._slice_layout()
+        active = [i for i, w in enumerate(widths) if w > 0]
+        a, b = self._a_slices(), self._b_slices()
+        slices = ([a[i].detach() for i in active], [b[i].detach() for i in active], [widths[i] for i in active],
+                  [cols[i] for i in active])
+        key = [(name, p, p.data_ptr()) for name, p in params.items() if name.startswith("lora_")]
+        self.__dict__["_slices_plan"] = (key, slices)
+        return slices
+
     @property
     def lora_enabled(self) -> bool:
         return self.supports_lora
@@ -109,7 +127,7 @@ class _LoRALayerBase(nn.Module):
             )
         # Host-only shortcut: nothing resident in this module. Never taken during graph
         # capture, where the captured launch must stay valid for later slot loads.
-        if not _is_cuda_graph_capture() and not any(self._effective_lora_rank_values):
+        if not any(self._effective_lora_rank_values) and not _is_cuda_graph_capture():
             return None
         return tts
 
@@ -146,32 +164,22 @@ class _LoRALayerBase(nn.Module):
             if x_flat.size(0) >= SGMV_MIN_TOKENS and fused_linear_supported(x_flat, weight, self.max_lora_rank):
                 token_to_slot = self._resolve_token_slots(x_flat)
                 if token_to_slot is not None:
-                    widths, cols = self._slice_layout()
-                    active = [i for i, w in enumerate(widths) if w > 0]
-                    a, b = self._a_slices(), self._b_slices()
-                    y = linear_lora(
-                        x_flat, weight, bias, [a[i] for i in active], [b[i] for i in active],
-                        [widths[i] for i in active], [cols[i] for i in active], token_to_slot, 1.0,
-                    )
+                    a, b, widths, cols = self._active_slices()
+                    y = linear_lora(x_flat, weight, bias, a, b, widths, cols, token_to_slot, 1.0)
                     return y if x.dim() == 2 else y.view(*x.shape[:-1], y.size(-1))
         if LORA_FIRST and not mixed and bias is None and x.is_cuda and isinstance(get_backend(), B200LoRABackend):
-            from .lora import launch_add
-
             x_flat = x if x.dim() == 2 else x.reshape(-1, x.size(-1))
             if x_flat.dtype == torch.bfloat16:
                 token_to_slot = self._resolve_token_slots(x_flat)
                 metadata = self._runtime_metadata()
-                widths, cols = self._slice_layout()
-                active = [i for i, w in enumerate(widths) if w > 0]
-                covered = sorted((cols[i], cols[i] + widths[i]) for i in active)
+                a, b, widths, cols = self._active_slices()
+                covered = sorted((c, c + w) for w, c in zip(widths, cols))
                 whole = bool(covered) and covered[0][0] == 0 and covered[-1][1] == weight.size(0) and all(
                     covered[i][1] == covered[i + 1][0] for i in range(len(covered) - 1))
                 if token_to_slot is not None and metadata is not None and whole:
                     # the delta first (its launch does not wait for the GEMM), then the GEMM accumulates into it
-                    a, b = self._a_slices(), self._b_slices()
                     y = torch.empty(x_flat.size(0), weight.size(0), dtype=x.dtype, device=x.device)
-                    launch_add(y, x_flat, [a[i] for i in active], [b[i] for i in active], [widths[i] for i in active],
-                               [cols[i] for i in active], metadata, 1.0, rank_per_slot=self.effective_lora_rank,
+                    _lora.launch_add(y, x_flat, a, b, widths, cols, metadata, 1.0, rank_per_slot=self.effective_lora_rank,
                                impl=get_backend().impl, overwrite=True)
                     y.addmm_(x_flat, weight.t())
                     return y if x.dim() == 2 else y.view(*x.shape[:-1], y.size(-1))
@@ -206,27 +214,21 @@ class _LoRALayerBase(nn.Module):
         if token_to_slot is None:
             return y
         y_flat = y if y.dim() == 2 else y.view(-1, y.size(-1))
-        widths, cols = self._slice_layout()
-        views = [y_flat[:, c : c + w] for w, c in zip(widths, cols)]
         backend = get_backend()
         metadata = self._runtime_metadata()
         if isinstance(backend, B200LoRABackend):
             # In-place at explicit column offsets; also covers partial target sets.
-            from .lora import launch_add
-
             if metadata is None:
                 raise RuntimeError("LoRA metadata must be prepared by the model runner before backend execution")
-            active = [i for i, w in enumerate(widths) if w > 0]
-            if active:
-                a, b = self._a_slices(), self._b_slices()
-                launch_add(
-                    y_flat, x_flat, [a[i] for i in active], [b[i] for i in active], [widths[i] for i in active],
-                    [cols[i] for i in active], metadata, 1.0, rank_per_slot=self.effective_lora_rank,
-                    impl=backend.impl,
-                )
+            a, b, widths, cols = self._active_slices()
+            if a:
+                _lora.launch_add(y_flat, x_flat, a, b, widths, cols, metadata, 1.0,
+                           rank_per_slot=self._buffers["effective_lora_rank"], impl=backend.impl)
             return y
         # Foreign backend (e.g. a test double): protocol call, then copy back if it
         # returned fresh tensors (legacy contract of lora.py:283-286).
+        widths, cols = self._slice_layout()
+        views = [y_flat[:, c : c + w] for w, c in zip(widths, cols)]
         contiguous_cover = cols == [sum(widths[:i]) for i in range(len(widths))] and sum(widths) == y_flat.size(1)
         out = backend.add_lora(
             views, x_flat, self._a_slices(), self._b_slices(), indices=token_to_slot, metadata=metadata, scaling=1.0,

@@ -149,6 +149,10 @@ def launch_add(
 ) -> None:
     """One ``lora_b200_add`` call: all slices share (slots, rank, in). ``overwrite=True`` is ``lora_b200_delta``:
     ``y_packed`` receives the delta (and -0.0 in rows without one) instead of being added to."""
+    rc = N.native().add(y_packed, x, a_slabs, b_slabs, out_sizes, col_offsets, metadata, scaling, rank_per_slot,
+                        scale_per_slot, impl, workspace, overwrite)
+    if rc is not None:
+        return N.check(rc)
     T = x.size(0)
     N.require_cuda(y_packed, x, *a_slabs, *b_slabs, metadata.token_to_slot)
     if y_packed.dim() != 2 or x.dim() != 2:
@@ -222,6 +226,12 @@ def linear_lora(
     """``x @ weight.T (+ bias)`` plus the multi-LoRA delta in one pass over the output
     (``lora_b200_linear_lora``): what the reference computes as ``F.linear`` followed by
     ``add_lora`` (``layers/lora.py:341-366``). ``token_to_slot=None`` gives the plain linear."""
+    if token_to_slot is not None:
+        got = N.native().linear(x, weight, bias, a_slabs, b_slabs, out_sizes, col_offsets, token_to_slot, scaling,
+                                scale_per_slot, out)
+        if got is not None:
+            N.check(got[0])
+            return got[1]
     N.require_cuda(x, weight, bias, token_to_slot, *a_slabs, *b_slabs)
     T, in_dim = x.shape
     out_total = weight.size(0)
@@ -306,6 +316,12 @@ class B200LoRABackend:
         the reference (``lora.py:291``).  ``rank_per_slot`` / ``scale_per_slot`` are
         optional extensions (device int32 / float32 ``[slots]``).
         """
+        if y_packed is not None and metadata is not None and not metadata.no_lora_flag and y_slices:
+            rc = N.native().add(y_packed, x, lora_a_slices, lora_b_slices, y_slices, None, metadata, scaling, rank_per_slot,
+                                scale_per_slot, self.impl, None, False)
+            if rc is not None:
+                N.check(rc)
+                return list(y_slices)
         if not y_slices:
             return []
         if len(y_slices) != len(lora_a_slices) or len(y_slices) != len(lora_b_slices):
