@@ -329,6 +329,8 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
   bp.S = S; bp.r_max = r_max; bp.rank_per_slot = rank_per_slot; bp.scale_per_slot = scale_per_slot;
   bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets;
   bp.n_buckets = n_buckets; bp.scaling = scaling;
+  const bool is16 = dtype == B200_LORA_BF16 || dtype == B200_LORA_F16;
+  bp.kind = dtype == B200_LORA_F16 ? 2 : (r_max % 32 != 0 ? 1 : 0);
 
   SgmvProblem sp;
   sp.y = y; sp.y_ld = y_ld; sp.x = x; sp.x_ld = x_ld; sp.T = T; sp.in_dim = in_dim; sp.S = S; sp.r_max = r_max;
@@ -337,6 +339,8 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
   if (overwrite) {
     // decode batches: the row-split kernel writes the delta (and the -0.0 rows) itself; everything else
     // fills y with -0.0 first and then adds as usual (-0.0 + d == d)
+    const int kind = bp.kind;
+    bp.kind = 0;
     bp.mode = 3;
     bp.token_to_slot = token_to_slot;
     const bool decode_like = T < kSgmvAutoMinTokens || T < 32 * n_buckets;
@@ -344,6 +348,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
         (impl == B200_LORA_IMPL_BGMV || (impl == B200_LORA_IMPL_AUTO && decode_like)) && bgmv_supported(bp, nullptr))
       return bgmv_launch(bp, st_);
     bp.mode = 0;
+    bp.kind = kind;
     bp.token_to_slot = nullptr;
     // prefill batches: the tile kernel stores the delta tiles instead of reduce-adding them
     {
@@ -363,7 +368,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     // batches to the fused kernel, everything else (other dtypes, odd shapes) to the generic one.
     int n_act = 0;
     for (int s = 0; s < st.n; ++s) n_act += st.out[s] > 0;
-    const bool bgmv_ok = dtype == B200_LORA_BF16 && have_buckets && bgmv_supported(bp, nullptr);
+    const bool bgmv_ok = is16 && have_buckets && bgmv_supported(bp, nullptr);
     // The prefill kernels tile rows in token order and pay one stage per run of equal slot, so they
     // want request-contiguous rows: with bucket arrays at hand, fewer than 32 rows per bucket on
     // average means a decode-like batch (slots scattered over the rows) and goes to the bucket kernel.
@@ -388,7 +393,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
       return launch_generic_add<float>(y, y_ld, x, x_ld, T, in_dim, st, S, r_max, rank_per_slot,
                                        scale_per_slot, token_to_slot, scaling, st_);
     case B200_LORA_IMPL_BGMV: {
-      if (dtype != B200_LORA_BF16) return fail(B200_LORA_EUNSUPPORTED, "fused decode kernel is bf16 only");
+      if (!is16) return fail(B200_LORA_EUNSUPPORTED, "fused decode kernel is bf16 / fp16 only");
       if (!have_buckets) return fail(B200_LORA_EINVAL, "fused decode kernel needs the bucket arrays");
       const char* why = nullptr;
       if (bgmv_supported(bp, &why)) return bgmv_launch(bp, st_);

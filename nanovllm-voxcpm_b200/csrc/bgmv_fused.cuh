@@ -76,6 +76,11 @@ struct BgmvProblem {
   // read); a base GEMM that then accumulates into y (beta = 1) gives base + delta, and x + (-0.0) == x
   // keeps rows without adapter bit-identical to the base result.
   int mode = 0;
+  // Precision of the rank-r intermediate and of the update. 0 (bf16, r_max % 32 == 0): tmp rounded to bf16, the delta
+  // rounded to bf16 and added at the L2. 1 (bf16) / 2 (fp16): tmp kept as the sum of two 16-bit numbers, y read, added to
+  // in fp32 and rounded once; mode 0 only, r_max % 16 == 0. What the per-token kernel computes, which these sizes and
+  // types used to take (a 37-row batch of rank-16 adapters: 45 us per projection there, 3 us here).
+  int kind = 0;
   float* tmp_io = nullptr;  // [n_slices, T, r_max] fp32
   const int32_t* token_to_slot = nullptr;  // mode 3: which rows have no adapter
 };
@@ -95,6 +100,8 @@ struct BgmvParams {
   int stage_bytes, NS;
   int red_pitch;    // floats per token row of the cross-warp reduction buffer
   int pitchT;       // bytes per token row of tmp
+  int lo_off;       // kinds 1, 2: bytes from a token's high halves to its low halves
+  int kind;
   int tmp_bytes;    // bytes of one tmp buffer
   int off_red, off_tmp, off_tab, off_bar;
   int full_k;       // every K part has all 1024 columns
@@ -136,7 +143,8 @@ __device__ __forceinline__ void bgmv_fill_rows_without_delta(const BgmvParams& p
 #endif
 // kMode = BgmvParams::mode, compiled separately so that no path carries the branches of another;
 // kFullK = every K part has all 1024 columns (in_dim a multiple of 1024): no column checks in the shrink
-template <int kMode, bool kFullK>
+// kKind = BgmvProblem::kind
+template <int kMode, bool kFullK, int kKind>
 __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kernel(const __grid_constant__ BgmvParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -145,6 +153,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   const int c = (int)cluster_ctarank();
   const int NS = p.NS;
   constexpr bool kOverwrite = kMode == 3;
+  constexpr bool kPrecise = kKind != 0, kF16 = kKind == 2;
   constexpr int mode = kMode;
 
   B200_TRACE_POINT(0)
@@ -180,7 +189,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
 
   int rank = p.r_max;
   if (p.rank_per_slot != nullptr && slot >= 0 && slot < p.S) rank = min(max(p.rank_per_slot[slot], 0), p.r_max);
-  const int r_eff = min(p.r_max, (rank + 31) & ~31);
+  const int r_eff = min(p.r_max, kPrecise ? (rank + 15) & ~15 : (rank + 31) & ~31);
   // (a bucket whose row range leaves the batch is ignored; the bounds-checked build reports it)
   if (cnt > 0 && slot >= 0) (void)B200_IN_BOUNDS(slot < p.S && start >= 0 && start <= p.T - cnt);
   if (slot < 0 || slot >= p.S || cnt <= 0 || start < 0 || start > p.T - cnt || r_eff == 0) {
@@ -227,7 +236,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   const int total = (shrink_tiles + tiles_exp) * npass;
   // bytes a pass delivers into this CTA: 16 token rows of all Q stacked rank rows, as bf16 once
   // (all-gather) or as fp32 from every CTA of the cluster (K split)
-  const uint32_t gather_bytes = ksplit ? (uint32_t)(C * kBgmvTok * Q * 4) : (uint32_t)(kBgmvTok * Q * 2);
+  const uint32_t gather_bytes = ksplit ? (uint32_t)(C * kBgmvTok * Q * 4) : (uint32_t)(kBgmvTok * Q * (kPrecise ? 4 : 2));
   if (tid == 0 && (mode == 0 || mode == 3)) {
     mbar_arrive_expect_tx(tmp_ready_bars, gather_bytes);                      // pass 0
     if (npass > 1) mbar_arrive_expect_tx(tmp_ready_bars + 8u, gather_bytes);  // pass 1
@@ -428,7 +437,9 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   // then owns 8 consecutive output columns 8t..8t+7 of the block.
   const uint32_t t_off = (uint32_t)(g * p.pitchT + t * 16);                             // tmp: token row g
   float* const red_wr = red + ((size_t)warp * kBgmvTok + g) * p.red_pitch + 2 * t;      // + 8 * pitch: token g + 8
-  const int kblocks = r_eff >> 5;
+  // expand: 32-column blocks of the intermediate; kinds 1 and 2 run through [high halves | low halves], 2 r_eff columns,
+  // against the same weights twice
+  const int kblocks = kPrecise ? r_eff >> 4 : r_eff >> 5;
   // all-gather item of this thread: one token row x four consecutive rank rows of this CTA
   const int groups = rows_c >> 2;
   const bool has_item = tid < kBgmvTok * groups;
@@ -502,8 +513,8 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
           }
 #pragma unroll
           for (int u = 0; u < kTiles; ++u) {
-            mma_bf16_16816(acc[u][0], xlo[i].x, xhi[i].x, xlo[i].y, xhi[i].y, w[u].x, w[u].y);
-            mma_bf16_16816(acc[u][1], xlo[i].z, xhi[i].z, xlo[i].w, xhi[i].w, w[u].z, w[u].w);
+            mma_16816<kF16>(acc[u][0], xlo[i].x, xhi[i].x, xlo[i].y, xhi[i].y, w[u].x, w[u].y);
+            mma_16816<kF16>(acc[u][1], xlo[i].z, xhi[i].z, xlo[i].w, xhi[i].w, w[u].z, w[u].w);
           }
         }
 #pragma unroll
@@ -604,10 +615,14 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
         } else {
           // to every CTA of the cluster (this one included): 8 bytes of tmp + their count on the
           // receiver's barrier in one operation
-          const uint32_t v0 = pack_bf16x2(a.x * sc, a.y * sc), v1 = pack_bf16x2(a.z * sc, a.w * sc);
+          const uint32_t v0 = pack_16x2<kF16>(a.x * sc, a.y * sc), v1 = pack_16x2<kF16>(a.z * sc, a.w * sc);
+          const uint32_t l0 = kPrecise ? pack_rest<kF16>(a.x * sc, a.y * sc, v0) : 0u, l1 = kPrecise ? pack_rest<kF16>(a.z * sc, a.w * sc, v1) : 0u;
 #pragma unroll 1
-          for (int rc = 0; rc < C; ++rc)
+          for (int rc = 0; rc < C; ++rc) {
             st_async_b32x2(mapa_shared(tmp_cur + it_off, (uint32_t)rc), v0, v1, mapa_shared(tmp_ready_bar, (uint32_t)rc));
+            if (kPrecise)
+              st_async_b32x2(mapa_shared(tmp_cur + it_off + (uint32_t)p.lo_off, (uint32_t)rc), l0, l1, mapa_shared(tmp_ready_bar, (uint32_t)rc));
+          }
         }
       }
       if (mode == 1) {
@@ -629,8 +644,12 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
             const float4 v = *reinterpret_cast<const float4*>(src + (size_t)rc * kBgmvTok * p.pitchR);
             a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
           }
-          *reinterpret_cast<uint2*>(tmp_base + (size_t)(pass & 1) * p.tmp_bytes + it_off) =
-              make_uint2(pack_bf16x2(a.x * sc, a.y * sc), pack_bf16x2(a.z * sc, a.w * sc));
+          const uint32_t v0 = pack_16x2<kF16>(a.x * sc, a.y * sc), v1 = pack_16x2<kF16>(a.z * sc, a.w * sc);
+          uint8_t* dst = tmp_base + (size_t)(pass & 1) * p.tmp_bytes + it_off;
+          *reinterpret_cast<uint2*>(dst) = make_uint2(v0, v1);
+          if (kPrecise)
+            *reinterpret_cast<uint2*>(dst + p.lo_off) =
+                make_uint2(pack_rest<kF16>(a.x * sc, a.y * sc, v0), pack_rest<kF16>(a.z * sc, a.w * sc, v1));
         }
         named_bar_sync(1, kBgmvConsumers);
       }
@@ -640,8 +659,20 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
     // ===== expand: y[tok, cols] += tmp[16 tok, r] . B_rows^T ======================
     // one tile of the ring per step: one 32-row block per warp (ER <= 256). Rows of a stage beyond the
     // tile's rows hold stale bytes; their products land in columns that are not written.
+    // kinds 1 and 2: y of the next tile is requested while this one is multiplied (the first one here, behind the wait)
+    uint4 y_next[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+    auto load_y = [&](int e) {
+      if (e >= tiles_exp) return;
+      const int2 te = etab[e];
+      if (y_col >= (te.y & 0xffff) || !B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) return;
+      if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + te.x);
+      if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + te.x);
+    };
+    if (kPrecise) load_y(0);
     auto expand_fn = [&](int e, uint32_t tile_addr) {
       const int2 te = etab[e];
+      const uint4 y_lo = y_next[0], y_hi = y_next[1];
+      if (kPrecise) load_y(e + 1);
       float d[4][4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.f;
@@ -649,17 +680,33 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
       const uint32_t w_addr = tile_addr + w_off;
 #pragma unroll 1
       for (int kb = 0; kb < kblocks; ++kb) {
-        const uint4 alo = lds128(a_addr + 64u * kb);
-        const uint4 ahi = lds128(a_addr + 64u * kb + 8u * (uint32_t)p.pitchT);
+        uint32_t a_kb = a_addr + 64u * kb, w_kb = w_addr + 64u * kb;
+        if (kPrecise) {
+          // this thread's eight columns start at 32 kb + 8 t of [high | low]; a_addr and w_addr already hold 16 t bytes
+          const int at = 32 * kb + 8 * t, low = at >= r_eff;
+          a_kb = a_addr + (uint32_t)(64 * kb + (low ? p.lo_off - 2 * r_eff : 0));
+          w_kb = w_addr + (uint32_t)(64 * kb - (low ? 2 * r_eff : 0));
+        }
+        const uint4 alo = lds128(a_kb);
+        const uint4 ahi = lds128(a_kb + 8u * (uint32_t)p.pitchT);
         uint4 w[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) w[j] = lds128(w_addr + 64u * kb + 2u * j * pitchB);
+        for (int j = 0; j < 4; ++j) w[j] = lds128(w_kb + 2u * j * pitchB);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) mma_bf16_16816(d[j], alo.x, ahi.x, alo.y, ahi.y, w[j].x, w[j].y);
+        for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.x, ahi.x, alo.y, ahi.y, w[j].x, w[j].y);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) mma_bf16_16816(d[j], alo.z, ahi.z, alo.w, ahi.w, w[j].z, w[j].w);
+        for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.z, ahi.z, alo.w, ahi.w, w[j].z, w[j].w);
       }
       if (y_col < (te.y & 0xffff) && B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) {
+        if (kPrecise) {
+          if (tok_lo >= 0)
+            stg128(ylo_p + te.x, make_uint4(add_16x2<kF16>(y_lo.x, d[0][0], d[0][1]), add_16x2<kF16>(y_lo.y, d[1][0], d[1][1]),
+                                            add_16x2<kF16>(y_lo.z, d[2][0], d[2][1]), add_16x2<kF16>(y_lo.w, d[3][0], d[3][1])));
+          if (tok_hi >= 0)
+            stg128(yhi_p + te.x, make_uint4(add_16x2<kF16>(y_hi.x, d[0][2], d[0][3]), add_16x2<kF16>(y_hi.y, d[1][2], d[1][3]),
+                                            add_16x2<kF16>(y_hi.z, d[2][2], d[2][3]), add_16x2<kF16>(y_hi.w, d[3][2], d[3][3])));
+          return;
+        }
         const uint4 lo4 = make_uint4(pack_bf16x2(d[0][0], d[0][1]), pack_bf16x2(d[1][0], d[1][1]),
                                      pack_bf16x2(d[2][0], d[2][1]), pack_bf16x2(d[3][0], d[3][1]));
         const uint4 hi4 = make_uint4(pack_bf16x2(d[0][2], d[0][3]), pack_bf16x2(d[1][2], d[1][3]),
@@ -726,7 +773,11 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
     ++st.n;
   }
   if (st.n == 0) { *why = "no active slice"; return false; }
-  if (b.r_max % 32 != 0 || b.r_max > 256) { *why = "r_max must be a multiple of 32, <= 256"; return false; }
+  if (b.r_max % (b.kind != 0 ? 16 : 32) != 0 || b.r_max > 256) {
+    *why = b.kind != 0 ? "r_max must be a multiple of 16, <= 256" : "r_max must be a multiple of 32, <= 256";
+    return false;
+  }
+  if (b.kind != 0 && b.mode != 0) { *why = "the other modes are for bf16 with r_max a multiple of 32"; return false; }
   if (b.in_dim % 32 != 0) { *why = "in_dim must be a multiple of 32"; return false; }
   if (b.x_ld % 8 != 0 || b.y_ld % 8 != 0) { *why = "row strides must be multiples of 8 elements"; return false; }
   if (!aligned16(b.x) || !aligned16(b.y)) { *why = "x / y must be 16-byte aligned"; return false; }
@@ -791,7 +842,9 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   // rows of a half warp start in different banks
   p.red_pitch = (Rc % 16 == 8) ? Rc : Rc + 8;
   const int red_bytes = round_up_i(kBgmvWarps * kBgmvTok * p.red_pitch * 4, 128);
-  p.pitchT = round_up_i(Q * 2, 128) + 64;
+  p.kind = b.kind;
+  p.lo_off = Q * 2;
+  p.pitchT = round_up_i(Q * (b.kind != 0 ? 4 : 2), 128) + 64;
   p.tmp_bytes = round_up_i(kBgmvTok * p.pitchT, 128);
   const int bar_bytes = 256;
   int exp_tiles = 0;
@@ -839,10 +892,12 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_device != dev) {
-    const void* kernels[8] = {(const void*)bgmv_fused_kernel<0, false>, (const void*)bgmv_fused_kernel<0, true>,
-                              (const void*)bgmv_fused_kernel<1, false>, (const void*)bgmv_fused_kernel<1, true>,
-                              (const void*)bgmv_fused_kernel<2, false>, (const void*)bgmv_fused_kernel<2, true>,
-                              (const void*)bgmv_fused_kernel<3, false>, (const void*)bgmv_fused_kernel<3, true>};
+    const void* kernels[12] = {(const void*)bgmv_fused_kernel<0, false, 0>, (const void*)bgmv_fused_kernel<0, true, 0>,
+                               (const void*)bgmv_fused_kernel<1, false, 0>, (const void*)bgmv_fused_kernel<1, true, 0>,
+                               (const void*)bgmv_fused_kernel<2, false, 0>, (const void*)bgmv_fused_kernel<2, true, 0>,
+                               (const void*)bgmv_fused_kernel<3, false, 0>, (const void*)bgmv_fused_kernel<3, true, 0>,
+                               (const void*)bgmv_fused_kernel<0, false, 1>, (const void*)bgmv_fused_kernel<0, true, 1>,
+                               (const void*)bgmv_fused_kernel<0, false, 2>, (const void*)bgmv_fused_kernel<0, true, 2>};
     for (const void* k : kernels) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kBgmvSmemMax);
       if (e != cudaSuccess) return fail(B200_LORA_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -869,13 +924,15 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
   cfg.attrs = attrs;
   cfg.numAttrs = (unsigned)na;
   cudaError_t e;
-#define B200_BGMV_LAUNCH(M) \
-  (p.full_k ? cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, true>, p) : cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, false>, p))
-  switch (p.mode) {
-    case 1: e = B200_BGMV_LAUNCH(1); break;
-    case 2: e = B200_BGMV_LAUNCH(2); break;
-    case 3: e = B200_BGMV_LAUNCH(3); break;
-    default: e = B200_BGMV_LAUNCH(0); break;
+#define B200_BGMV_LAUNCH(M, K) \
+  (p.full_k ? cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, true, K>, p) : cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, false, K>, p))
+  switch (p.kind != 0 ? 3 + p.kind : p.mode) {
+    case 1: e = B200_BGMV_LAUNCH(1, 0); break;
+    case 2: e = B200_BGMV_LAUNCH(2, 0); break;
+    case 3: e = B200_BGMV_LAUNCH(3, 0); break;
+    case 4: e = B200_BGMV_LAUNCH(0, 1); break;
+    case 5: e = B200_BGMV_LAUNCH(0, 2); break;
+    default: e = B200_BGMV_LAUNCH(0, 0); break;
   }
 #undef B200_BGMV_LAUNCH
   if (e != cudaSuccess) {

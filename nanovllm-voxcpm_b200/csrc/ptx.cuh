@@ -3,6 +3,7 @@
 // launch, warp-level bf16 MMA. Every blocking wait here is bounded.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -223,9 +224,47 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+// the same with fp16 operands
+__device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                              uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+template <bool kF16>
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  if (kF16) mma_f16_16816(d, a0, a1, a2, a3, b0, b1);
+  else mma_bf16_16816(d, a0, a1, a2, a3, b0, b1);
+}
+__device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_f16x2(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2*>(&v)); }
+template <bool kF16>
+__device__ __forceinline__ uint32_t pack_16x2(float lo, float hi) { return kF16 ? pack_f16x2(lo, hi) : pack_bf16x2(lo, hi); }
+// what the two numbers of `packed` = pack_16x2(lo, hi) left over, rounded to the same type
+template <bool kF16>
+__device__ __forceinline__ uint32_t pack_rest(float lo, float hi, uint32_t packed) {
+  if (kF16) {
+    const float2 h = unpack_f16x2(packed);
+    return pack_f16x2(lo - h.x, hi - h.y);
+  }
+  return pack_bf16x2(lo - bf16_lo(packed), hi - bf16_hi(packed));
+}
 // two packed bf16 + two fp32 deltas, rounded once
 __device__ __forceinline__ uint32_t add_bf16x2(uint32_t y, float d0, float d1) {
   return pack_bf16x2(bf16_lo(y) + d0, bf16_hi(y) + d1);
+}
+template <bool kF16>
+__device__ __forceinline__ uint32_t add_16x2(uint32_t y, float d0, float d1) {
+  if (kF16) {
+    const float2 h = unpack_f16x2(y);
+    return pack_f16x2(h.x + d0, h.y + d1);
+  }
+  return add_bf16x2(y, d0, d1);
 }
 
 }  // namespace b200lora
