@@ -1,9 +1,11 @@
 // Fused decode multi-LoRA kernel (bf16): shrink + expand in ONE launch.
 //
 // Work decomposition
-//   grid = (C, n_buckets), thread-block cluster = (C, 1, 1): one cluster per slot
+//   grid = (C, n_buckets + extra), thread-block cluster = (C, 1, 1): one cluster per slot
 //   bucket of the batch (bucket g = tokens sorted_idx[offsets[g] .. +counts[g]) that
 //   all use adapter slot slot_ids[g]); buckets with id -1 or no tokens exit at once.
+//   A cluster takes at most `window` tokens (16, one pass, unless the GPU is full); the
+//   rest of a popular bucket goes to the extra clusters, window by window.
 //   Inside a cluster the adapter's weights are split so that every byte of
 //   lora_A[slot] and lora_B[slot] is pulled from HBM by exactly one CTA:
 //     shrink : the n*r stacked rank rows are split across the C CTAs (full K each)
@@ -78,10 +80,13 @@ struct BgmvProblem {
   int mode = 0;
   // Precision of the rank-r intermediate and of the update. 0 (bf16, r_max % 32 == 0): tmp rounded to bf16, the delta
   // rounded to bf16 and added at the L2. 1 (bf16) / 2 (fp16): tmp kept as the sum of two 16-bit numbers, y read, added to
-  // in fp32 and rounded once; mode 0 only, r_max % 16 == 0. What the per-token kernel computes, which these sizes and
+  // in fp32 and rounded once; modes 0, 1 and 2, r_max % 16 == 0. What the per-token kernel computes, which these sizes and
   // types used to take (a 37-row batch of rank-16 adapters: 45 us per projection there, 3 us here).
   int kind = 0;
-  float* tmp_io = nullptr;  // [n_slices, T, r_max] fp32
+  void* tmp_io = nullptr;  // [n_slices, T, r_max], fp32 or (io16) values of the activations' type
+  int io16 = 0;
+  int zero_rows = 0;       // mode 1: rows without adapter are written as zeros (token_to_slot tells which)
+  int no_add = 0;          // mode 2, kinds 1 and 2: y = delta in rows with an adapter instead of y += delta
   const int32_t* token_to_slot = nullptr;  // mode 3: which rows have no adapter
 };
 
@@ -92,6 +97,7 @@ struct BgmvParams {
   const int32_t* rank_per_slot; const float* scale_per_slot;
   const int32_t *sorted_idx, *slot_ids, *counts, *offsets;
   int n_buckets; float scaling;
+  int window;       // tokens per cluster (multiple of 16)
   int c_shift;      // cluster size C = 1 << c_shift
   int KP, nkp;      // columns per shrink tile (min(in, 1024)) and number of K parts
   int pitchA;       // bytes between rows of a shrink tile (KP*2, +64 when rows are copied one by one)
@@ -110,7 +116,8 @@ struct BgmvParams {
   int pitchR, recv_bytes, off_recv;  // K split: floats per token row / bytes of one buffer of received partial sums
   int use_pdl;
   int mode;         // 0 fused, 1 shrink only (tmp_io written), 2 expand only (tmp_io read), 3 overwrite y
-  float* tmp_io;
+  void* tmp_io;
+  int io16, zero_rows, no_add;
   const int32_t* token_to_slot;
 };
 
@@ -136,6 +143,19 @@ __device__ __forceinline__ void bgmv_fill_rows_without_delta(const BgmvParams& p
   }
 }
 
+// mode 1 with zero_rows: rows without adapter of the intermediate [n, T, r_max], dealt as above
+__device__ __forceinline__ void bgmv_zero_rows_without_adapter(const BgmvParams& p, int cta, int n_ctas, int thread, int nthreads) {
+  const int vecs = (p.r_max * (p.io16 ? 2 : 4)) >> 4;  // 16-byte pieces of a row
+  for (int row = cta; row < p.T; row += n_ctas) {
+    const int sl = p.token_to_slot[row];
+    if (sl >= 0 && sl < p.S) continue;
+    for (int i = thread; i < p.st.n * vecs; i += nthreads) {
+      const int s = i / vecs;
+      stg128(static_cast<uint8_t*>(p.tmp_io) + (((int64_t)s * p.T + row) * vecs + (i - s * vecs)) * 16, make_uint4(0, 0, 0, 0));
+    }
+  }
+}
+
 // Two CTAs per SM: the CTAs of the next launch of the stream become resident while this launch still
 // runs, so their weight copies and L2 prefetches overlap this launch's dependent chain.
 #ifndef BGMV_MINBLOCKS
@@ -143,12 +163,13 @@ __device__ __forceinline__ void bgmv_fill_rows_without_delta(const BgmvParams& p
 #endif
 // kMode = BgmvParams::mode, compiled separately so that no path carries the branches of another;
 // kFullK = every K part has all 1024 columns (in_dim a multiple of 1024): no column checks in the shrink
-// kKind = BgmvProblem::kind
-template <int kMode, bool kFullK, int kKind>
+// kKind = BgmvProblem::kind; kWide = r_max > 32: output tiles are less than 256 rows high and a step of the expand takes
+// several (the general step costs 12 % where a tile is a step)
+template <int kMode, bool kFullK, int kKind, bool kWide>
 __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kernel(const __grid_constant__ BgmvParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int bucket = blockIdx.y;
+  int bucket = blockIdx.y;
   const int C = 1 << p.c_shift;
   const int c = (int)cluster_ctarank();
   const int NS = p.NS;
@@ -162,9 +183,27 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   // traffic overlaps this kernel's compute and keeps HBM busy across launch boundaries.
   if (p.use_pdl) griddep_launch_dependents();
   // ---- bucket metadata (uniform across the cluster); barrier set-up overlaps the loads
-  const int slot = p.slot_ids[bucket];
-  const int cnt = p.counts[bucket];
-  const int start = p.offsets[bucket];
+  // Extra cluster e looks after multiple m = (e + 1) * window of the window inside the sorted rows: if m lies behind the
+  // first row of a bucket [start, start + cnt), it is the i-th such multiple there, and the cluster takes the bucket's i-th
+  // window. (A bucket of cnt rows has ceil(cnt / window) - 1 windows beyond its first and at least that many multiples.)
+  int window_no = 0;
+  if (bucket >= p.n_buckets) {
+    volatile int* owner = reinterpret_cast<volatile int*>(smem + p.off_bar + 8 * (2 * kBgmvMaxStages + 2)) + 1;  // behind the abort flag
+    const int m = (bucket - p.n_buckets + 1) * p.window;
+    if (tid == 0) *owner = -1;
+    __syncthreads();
+    for (int b = tid; b < p.n_buckets; b += kBgmvThreads) {
+      const int lo = p.offsets[b];
+      if (lo < m && m - lo < p.counts[b]) *owner = b;
+    }
+    __syncthreads();
+    bucket = *owner;
+    if (bucket >= 0) window_no = m / p.window - p.offsets[bucket] / p.window;
+  }
+  const int slot = bucket >= 0 ? p.slot_ids[bucket] : -1;
+  const int rows_all = bucket >= 0 ? p.counts[bucket] : 0, start_all = bucket >= 0 ? p.offsets[bucket] : 0;
+  const int cnt = min(p.window, rows_all - window_no * p.window);
+  const int start = start_all + window_no * p.window;
 
   float* red = reinterpret_cast<float*>(smem + p.off_red);
   uint8_t* tmp_base = smem + p.off_tmp;
@@ -176,6 +215,22 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   const uint32_t tmp_ready_bars = bar_base + 8u * (uint32_t)(2 * kBgmvMaxStages);
   auto full_bar = [&](int s) { return bar_base + 8u * (uint32_t)s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (uint32_t)(kBgmvMaxStages + s); };
+
+  int rank = p.r_max;
+  if (p.rank_per_slot != nullptr && slot >= 0 && slot < p.S) rank = min(max(p.rank_per_slot[slot], 0), p.r_max);
+  const int r_eff = min(p.r_max, kPrecise ? (rank + 15) & ~15 : (rank + 31) & ~31);
+  // (a bucket whose row range leaves the batch is ignored; the bounds-checked build reports it)
+  if (cnt > 0 && slot >= 0) (void)B200_IN_BOUNDS(slot < p.S && start_all >= 0 && start_all <= p.T - rows_all);
+  if (slot < 0 || slot >= p.S || cnt <= 0 || start_all < 0 || start_all > p.T - rows_all || r_eff == 0) {
+    // An idle cluster holds nothing, but one CTA of every launch must outlive the previous launch
+    // of the stream: a launch that ended before its predecessor would let the launch behind it
+    // pass its own wait too early.
+    if (p.use_pdl && (kOverwrite || (kMode == 1 && p.zero_rows) || (blockIdx.y == 0 && c == 0))) griddep_wait();
+    if (kMode == 1 && p.zero_rows) bgmv_zero_rows_without_adapter(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvThreads);
+    if (kOverwrite)  // an idle cluster still does its share of the -0.0 rows
+      bgmv_fill_rows_without_delta(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvThreads);
+    return;
+  }
   if (tid < NS) {
     mbar_init(full_bar(tid), 1);
     mbar_init(empty_bar(tid), kBgmvWarps);
@@ -185,21 +240,6 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
       *abort_flag = 0;
     }
     mbar_fence_init();
-  }
-
-  int rank = p.r_max;
-  if (p.rank_per_slot != nullptr && slot >= 0 && slot < p.S) rank = min(max(p.rank_per_slot[slot], 0), p.r_max);
-  const int r_eff = min(p.r_max, kPrecise ? (rank + 15) & ~15 : (rank + 31) & ~31);
-  // (a bucket whose row range leaves the batch is ignored; the bounds-checked build reports it)
-  if (cnt > 0 && slot >= 0) (void)B200_IN_BOUNDS(slot < p.S && start >= 0 && start <= p.T - cnt);
-  if (slot < 0 || slot >= p.S || cnt <= 0 || start < 0 || start > p.T - cnt || r_eff == 0) {
-    // An idle cluster holds nothing, but one CTA of every launch must outlive the previous launch
-    // of the stream: a launch that ended before its predecessor would let the launch behind it
-    // pass its own wait too early.
-    if (p.use_pdl && (kOverwrite || (bucket == 0 && c == 0))) griddep_wait();
-    if (kOverwrite)  // an idle cluster still does its share of the -0.0 rows
-      bgmv_fill_rows_without_delta(p, bucket * C + c, (int)gridDim.y * C, tid, kBgmvThreads);
-    return;
   }
   const float sc = p.scaling * (p.scale_per_slot != nullptr ? p.scale_per_slot[slot] : 1.0f);
   B200_TRACE_POINT(1)
@@ -404,7 +444,10 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   }
   named_bar_sync(1, kBgmvConsumers);  // table complete
 
-  const int rb = warp * 32;             // expand: out rows of this warp inside a tile
+  // expand: a step takes U tiles of ER rows, 256 rows in all, one 32-row block per warp: this warp's tile of the step and
+  // its rows inside that tile. (With one tile per step half of the warps had no rows at rank 64, and read past the stage.)
+  const int U = kWide ? (kBgmvWarps * 32) >> p.er_shift : 1, sub = kWide ? (warp * 32) >> p.er_shift : 0;
+  const int rb = kWide ? (warp * 32) & (ER - 1) : warp * 32;
   const int x_col = warp * 32 + t * 8;  // shrink: first column of the thread inside a K part (block i adds 256)
   const int y_col = rb + 8 * t;         // expand: first of the thread's 8 output columns inside a tile
   if (p.use_pdl) {
@@ -419,7 +462,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
     }
     if (!kOverwrite) {  // the lines of y that this thread's reductions will land in
 #pragma unroll 1
-      for (int e = 0; e < tiles_exp; ++e) {
+      for (int e = sub; e < tiles_exp; e += U) {
         const int2 te = etab[e];
         if (y_col < (te.y & 0xffff)) {
           if (tok0_lo >= 0) prefetch_l2(p.y + (int64_t)tok0_lo * p.y_ld + te.x + y_col);
@@ -452,7 +495,8 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   const uint32_t it_roff = (uint32_t)(it_tok * p.pitchR + it_q) * 4u;  // K split: the item inside one sender's block
 
   if (p.use_pdl) griddep_wait();  // x and y of this launch are final from here on
-  if (kOverwrite) bgmv_fill_rows_without_delta(p, bucket * C + c, (int)gridDim.y * C, tid, kBgmvConsumers);
+  if (kOverwrite) bgmv_fill_rows_without_delta(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvConsumers);
+  if (kMode == 1 && p.zero_rows) bgmv_zero_rows_without_adapter(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvConsumers);
   B200_TRACE_POINT(4)
 
   int c_stage = 0;
@@ -582,9 +626,18 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
 #pragma unroll 1
       for (int pr = tid & 15; pr < (Q >> 1); pr += 16) {
         const int q = 2 * pr, s = q / r_eff, rr = q - s * r_eff;
-        float2 v = make_float2(0.f, 0.f);
-        if (trow >= 0) v = *reinterpret_cast<const float2*>(p.tmp_io + ((int64_t)s * p.T + trow) * p.r_max + rr);
-        *reinterpret_cast<uint32_t*>(tmp_full + (size_t)tok * p.pitchT + (size_t)q * 2) = pack_bf16x2(v.x, v.y);
+        const int64_t at = ((int64_t)s * p.T + trow) * p.r_max + rr;
+        uint32_t* const dst = reinterpret_cast<uint32_t*>(tmp_full + (size_t)tok * p.pitchT + (size_t)q * 2);
+        if (p.io16) {
+          *dst = trow >= 0 ? *reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(p.tmp_io) + at) : 0u;
+          if (kPrecise) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(dst) + p.lo_off) = 0u;
+        } else {
+          float2 v = make_float2(0.f, 0.f);
+          if (trow >= 0) v = *reinterpret_cast<const float2*>(static_cast<const float*>(p.tmp_io) + at);
+          const uint32_t h = pack_16x2<kF16>(v.x, v.y);
+          *dst = h;
+          if (kPrecise) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(dst) + p.lo_off) = pack_rest<kF16>(v.x, v.y, h);
+        }
       }
       named_bar_sync(1, kBgmvConsumers);
     } else {
@@ -601,9 +654,15 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
           if (pass * kBgmvTok + it_tok < cnt) trow = p.sorted_idx[start + pass * kBgmvTok + it_tok];
           if (trow >= 0 && trow < p.T) {
             const int s = it_q / r_eff, rr = it_q - s * r_eff;
-            float2* dst = reinterpret_cast<float2*>(p.tmp_io + ((int64_t)s * p.T + trow) * p.r_max + rr);
-            dst[0] = make_float2(a.x * sc, a.y * sc);
-            dst[1] = make_float2(a.z * sc, a.w * sc);
+            const int64_t at = ((int64_t)s * p.T + trow) * p.r_max + rr;
+            if (p.io16) {
+              *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.tmp_io) + at) =
+                  make_uint2(pack_16x2<kF16>(a.x * sc, a.y * sc), pack_16x2<kF16>(a.z * sc, a.w * sc));
+            } else {
+              float2* dst = reinterpret_cast<float2*>(static_cast<float*>(p.tmp_io) + at);
+              dst[0] = make_float2(a.x * sc, a.y * sc);
+              dst[1] = make_float2(a.z * sc, a.w * sc);
+            }
           }
         } else if (ksplit) {
           // to every CTA of the cluster (this one included): this CTA's fp32 partial sums over its K parts,
@@ -657,22 +716,21 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
     }
 
     // ===== expand: y[tok, cols] += tmp[16 tok, r] . B_rows^T ======================
-    // one tile of the ring per step: one 32-row block per warp (ER <= 256). Rows of a stage beyond the
-    // tile's rows hold stale bytes; their products land in columns that are not written.
+    // Rows of a stage beyond the tile's rows hold stale bytes; their products land in columns that are not written.
     // kinds 1 and 2: y of the next tile is requested while this one is multiplied (the first one here, behind the wait)
     uint4 y_next[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
     auto load_y = [&](int e) {
-      if (e >= tiles_exp) return;
+      if (e >= tiles_exp || (kMode == 2 && p.no_add)) return;
       const int2 te = etab[e];
       if (y_col >= (te.y & 0xffff) || !B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) return;
       if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + te.x);
       if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + te.x);
     };
-    if (kPrecise) load_y(0);
+    if (kPrecise) load_y(sub);
     auto expand_fn = [&](int e, uint32_t tile_addr) {
       const int2 te = etab[e];
       const uint4 y_lo = y_next[0], y_hi = y_next[1];
-      if (kPrecise) load_y(e + 1);
+      if (kPrecise) load_y(e + U);
       float d[4][4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.f;
@@ -723,16 +781,36 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
         }
       }
     };
-    int e = 0;
+    if (!kWide) {
 #pragma unroll 1
-    for (; e < tiles_exp; ++e) {
-      mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
-      if (pass == 0 && e < 10) { B200_TRACE_POINT(12 + 2 * e) }
-      expand_fn(e, stage_addr);
-      if (pass == 0 && e < 10) { B200_TRACE_POINT(13 + 2 * e) }
+      for (int e = 0; e < tiles_exp; ++e) {
+        mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
+        if (pass == 0 && e < 10) { B200_TRACE_POINT(12 + 2 * e) }
+        expand_fn(e, stage_addr);
+        if (pass == 0 && e < 10) { B200_TRACE_POINT(13 + 2 * e) }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_relaxed(empty_bar(c_stage));
+        advance();
+      }
+    } else {
+#pragma unroll 1
+    for (int e = 0; e < tiles_exp; e += U) {
+      // (every warp waits for every tile of the step: a wait that skipped phases of a stage could no longer tell them apart)
+      const int n_here = min(U, tiles_exp - e), stage0 = c_stage;
+      uint32_t mine = 0;
+#pragma unroll 1
+      for (int u = 0; u < n_here; ++u) {
+        mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
+        if (u == sub) mine = stage_addr;
+        advance();
+      }
+      if (sub < n_here) expand_fn(e + sub, mine);
       __syncwarp();
-      if (lane == 0) mbar_arrive_relaxed(empty_bar(c_stage));
-      advance();
+      if (lane < n_here) {
+        const int st = stage0 + lane;
+        mbar_arrive_relaxed(empty_bar(st >= NS ? st - NS : st));
+      }
+    }
     }
     if (pass == 0) { B200_TRACE_POINT(10) }
   }
@@ -777,7 +855,7 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
     *why = b.kind != 0 ? "r_max must be a multiple of 16, <= 256" : "r_max must be a multiple of 32, <= 256";
     return false;
   }
-  if (b.kind != 0 && b.mode != 0) { *why = "the other modes are for bf16 with r_max a multiple of 32"; return false; }
+  if (b.kind != 0 && b.mode == 3) { *why = "overwrite mode is for bf16 with r_max a multiple of 32"; return false; }
   if (b.in_dim % 32 != 0) { *why = "in_dim must be a multiple of 32"; return false; }
   if (b.x_ld % 8 != 0 || b.y_ld % 8 != 0) { *why = "row strides must be multiples of 8 elements"; return false; }
   if (!aligned16(b.x) || !aligned16(b.y)) { *why = "x / y must be 16-byte aligned"; return false; }
@@ -785,7 +863,7 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
     if (st.out[s] % 8 != 0 || st.col[s] % 8 != 0) { *why = "slice widths / offsets must be multiples of 8"; return false; }
     if (!aligned16(st.a[s]) || !aligned16(st.b[s])) { *why = "slabs must be 16-byte aligned"; return false; }
   }
-  if (b.n_buckets < 1 || b.n_buckets > 65535) { *why = "n_buckets outside [1, 65535]"; return false; }
+  if (b.n_buckets < 1 || b.n_buckets + b.T / kBgmvTok > 65535) { *why = "n_buckets outside [1, 65535]"; return false; }
 
   const int Q = st.n * b.r_max;
   int C = bgmv_options().cluster;
@@ -799,24 +877,32 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
     const double nb = (double)b.n_buckets;
     const double in_use = nb * (1.0 - std::exp(-(double)std::max(b.T, 1) / nb));
     C = in_use <= 56.0 ? 4 : (in_use <= 112.0 ? 2 : 1);
-    // Large adapters (rank 64 on 4096-wide layers: 1 - 5 MB per bucket) keep an SM busy for tens of microseconds;
-    // then the balance over the SMs matters more than room for the next launch: at most 512 KB of slab per CTA.
-    // Measured on a 4-layer slice of a 32-head decoder, 512 rows over 175 adapters: 20.8 ms per step with one CTA
-    // per bucket, 19.7 with 2, 19.0 with 4.
+    // A CTA streams its share of the slabs at 25 - 30 GB/s (loads, multiplication and exchange take turns): large adapters
+    // want more CTAs, as far as those are resident together or their streams are long. Measured, us per projection with
+    // clusters of 4 / 8: one row of 4096-wide layers, rank 64: 23.1 / 9.8; 64 rows over 32 adapters of 2048-wide layers, rank
+    // 64: 15.3 / 9.3; gate_up of 200 rows over 20 adapters, 2048-wide, rank 32 (262 KB a CTA at 4): 11.0 / 8.0, its o (66 KB):
+    // 4.0 / 4.5; gate_up of 384 rows over 64 adapters, 1024-wide, rank 32, with 2 / 4: 15.2 / 12.3; above about 300 CTAs
+    // only streams of more than 512 KB gain: 32-head decoder, 512 rows over 175 adapters, 4 layers: 20.8 ms a step with one
+    // CTA per bucket, 19.7 with 2, 19.0 with 4.
     int64_t bucket_bytes = 0;
     for (int s = 0; s < st.n; ++s) bucket_bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + st.out[s]);
-    while (C < 4 && bucket_bytes / C > 512 * 1024) C *= 2;
+    const double resident = 2.0 * 148;
+    while (C < 4 && (bucket_bytes / C > 512 * 1024 || (bucket_bytes / C > 256 * 1024 && in_use * C * 2 <= resident))) C *= 2;
+    const double clusters = in_use + (b.T - 1) / kBgmvTok;
+    if (C == 4 && ((bucket_bytes / 4 > 128 * 1024 && clusters * 8 <= resident) || (bucket_bytes / 4 >= 256 * 1024 && in_use * 8 <= resident))) C = 8;
   }
   // K split: at least one K part (1024 columns) per CTA of the cluster and all rank rows in one CTA;
   // the shrink-only / expand-only pair of the tensor-parallel exchange keeps the row split
   const int nkp_all = ceil_div_i(b.in_dim, kBgmvKP);
-  const bool ksplit = bgmv_options().ksplit && C > 1 && (b.mode == 0 || b.mode == 3) && nkp_all >= C && Q <= kBgmvMaxRc;
+  const bool ksplit = bgmv_options().ksplit && C > 1 && (b.mode == 0 || b.mode == 3) && nkp_all >= C && Q <= kBgmvMaxRc &&
+                      2 * C * kBgmvTok * (Q + 4) * 4 <= 40 * 1024;  // (received partial sums: more would cost the second CTA per SM)
   if (!ksplit)
     while (C < 8 && round_up_i(ceil_div_i(Q, C), 8) > kBgmvMaxRc) C *= 2;
   const int Rc = ksplit ? Q : round_up_i(ceil_div_i(Q, C), 8);
   if (Rc > kBgmvMaxRc) { *why = "n_slices * r_max too large for one cluster"; return false; }
 
   BgmvParams p;
+  p.window = kBgmvTok;
   p.y = static_cast<__nv_bfloat16*>(b.y); p.y_ld = b.y_ld;
   p.x = static_cast<const __nv_bfloat16*>(b.x); p.x_ld = b.x_ld;
   p.T = b.T; p.in_dim = b.in_dim; p.S = b.S; p.r_max = b.r_max; p.st = st;
@@ -857,11 +943,11 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   const int fixed = red_bytes + 2 * p.tmp_bytes + 2 * p.recv_bytes + tab_bytes + bar_bytes;
   // ring: what fits beside a second CTA on the SM, unless the caller set a size (up to the whole SM)
   const int ring_bytes = bgmv_options().ring_kb > 0 ? bgmv_options().ring_kb * 1024
-                                                    : std::max(kBgmvSmemCoResident - fixed - 256, 2 * p.stage_bytes);
-  int NS = std::min(std::max(tiles, 2), (kBgmvSmemMax - fixed - 256) / p.stage_bytes);
+                                                    : std::max(kBgmvSmemCoResident - fixed - 256, std::max(2, 256 / p.ER) * p.stage_bytes);
+  int NS = std::min(std::max(tiles, std::max(2, 256 / p.ER)), (kBgmvSmemMax - fixed - 256) / p.stage_bytes);
   NS = std::min(NS, kBgmvMaxStages);
-  NS = std::min(NS, std::max(2, ring_bytes / p.stage_bytes));
-  if (NS < 2) { *why = "shared memory too small for two stages"; return false; }
+  NS = std::min(NS, std::max(std::max(2, 256 / p.ER), ring_bytes / p.stage_bytes));
+  if (NS < std::max(2, 256 / p.ER)) { *why = "shared memory too small for the stages of a step"; return false; }
   p.NS = NS;
   p.off_red = NS * p.stage_bytes;
   p.off_tmp = p.off_red + red_bytes;
@@ -873,7 +959,7 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   for (int s = 0; s < st.n; ++s) p.y_cols = std::max(p.y_cols, st.col[s] + st.out[s]);
   p.use_pdl = bgmv_options().pdl ? 1 : 0;
   p.mode = b.mode;
-  p.tmp_io = b.tmp_io;
+  p.tmp_io = b.tmp_io; p.io16 = b.io16; p.zero_rows = b.zero_rows; p.no_add = b.no_add;
   p.token_to_slot = b.token_to_slot;
   if ((b.mode == 1 || b.mode == 2) && b.tmp_io == nullptr) { *why = "shrink-only / expand-only need the tmp array"; return false; }
   if (b.mode == 3 && b.token_to_slot == nullptr) { *why = "overwrite mode needs token_to_slot"; return false; }
@@ -892,12 +978,12 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_device != dev) {
-    const void* kernels[12] = {(const void*)bgmv_fused_kernel<0, false, 0>, (const void*)bgmv_fused_kernel<0, true, 0>,
-                               (const void*)bgmv_fused_kernel<1, false, 0>, (const void*)bgmv_fused_kernel<1, true, 0>,
-                               (const void*)bgmv_fused_kernel<2, false, 0>, (const void*)bgmv_fused_kernel<2, true, 0>,
-                               (const void*)bgmv_fused_kernel<3, false, 0>, (const void*)bgmv_fused_kernel<3, true, 0>,
-                               (const void*)bgmv_fused_kernel<0, false, 1>, (const void*)bgmv_fused_kernel<0, true, 1>,
-                               (const void*)bgmv_fused_kernel<0, false, 2>, (const void*)bgmv_fused_kernel<0, true, 2>};
+#define B200_BGMV_ALL(M, K)                                                                                                  \
+  (const void*)bgmv_fused_kernel<M, false, K, false>, (const void*)bgmv_fused_kernel<M, true, K, false>,                     \
+      (const void*)bgmv_fused_kernel<M, false, K, true>, (const void*)bgmv_fused_kernel<M, true, K, true>
+    const void* kernels[] = {B200_BGMV_ALL(0, 0), B200_BGMV_ALL(1, 0), B200_BGMV_ALL(2, 0), B200_BGMV_ALL(3, 0), B200_BGMV_ALL(0, 1), B200_BGMV_ALL(0, 2), B200_BGMV_ALL(1, 1),
+                             B200_BGMV_ALL(1, 2), B200_BGMV_ALL(2, 1), B200_BGMV_ALL(2, 2)};
+#undef B200_BGMV_ALL
     for (const void* k : kernels) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kBgmvSmemMax);
       if (e != cudaSuccess) return fail(B200_LORA_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -905,7 +991,7 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
     configured_device = dev;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(1u << p.c_shift, (unsigned)p.n_buckets, 1);
+  cfg.gridDim = dim3(1u << p.c_shift, (unsigned)(p.n_buckets + (p.T - 1) / p.window), 1);
   cfg.blockDim = dim3(kBgmvThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -924,14 +1010,21 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
   cfg.attrs = attrs;
   cfg.numAttrs = (unsigned)na;
   cudaError_t e;
-#define B200_BGMV_LAUNCH(M, K) \
-  (p.full_k ? cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, true, K>, p) : cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, false, K>, p))
-  switch (p.kind != 0 ? 3 + p.kind : p.mode) {
+#define B200_BGMV_LAUNCH(M, K)                                                               \
+  (p.ER == 256 ? (p.full_k ? cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, true, K, false>, p)   \
+                           : cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, false, K, false>, p)) \
+               : (p.full_k ? cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, true, K, true>, p)    \
+                           : cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, false, K, true>, p)))
+  switch (4 * p.kind + p.mode) {
     case 1: e = B200_BGMV_LAUNCH(1, 0); break;
     case 2: e = B200_BGMV_LAUNCH(2, 0); break;
     case 3: e = B200_BGMV_LAUNCH(3, 0); break;
     case 4: e = B200_BGMV_LAUNCH(0, 1); break;
-    case 5: e = B200_BGMV_LAUNCH(0, 2); break;
+    case 5: e = B200_BGMV_LAUNCH(1, 1); break;
+    case 6: e = B200_BGMV_LAUNCH(2, 1); break;
+    case 8: e = B200_BGMV_LAUNCH(0, 2); break;
+    case 9: e = B200_BGMV_LAUNCH(1, 2); break;
+    case 10: e = B200_BGMV_LAUNCH(2, 2); break;
     default: e = B200_BGMV_LAUNCH(0, 0); break;
   }
 #undef B200_BGMV_LAUNCH
