@@ -42,6 +42,7 @@ extern "C" {
 #define B200_LORA_IMPL_GENERIC 1 /* one CTA per token, any dtype / shape / stride */
 #define B200_LORA_IMPL_BGMV 2    /* fused decode kernel: cluster per slot bucket, bulk-copy ring + mma */
 #define B200_LORA_IMPL_SGMV 3    /* prefill kernels: tcgen05 shrink + tcgen05 expand, scratch from `workspace` */
+#define B200_LORA_IMPL_GROUPED 4 /* bucketed tcgen05 shrink + expand (bf16 / fp16), scratch from `workspace` */
 
 /* error codes */
 #define B200_LORA_OK 0

@@ -22,7 +22,7 @@ LIB_PATH = os.environ.get("B200_LORA_LIB") or os.path.join(_HERE, "lib", "libb20
 ABI_VERSION = 1
 
 DT_BF16, DT_F16, DT_F32 = 0, 1, 2
-IMPL_AUTO, IMPL_GENERIC, IMPL_BGMV, IMPL_SGMV = 0, 1, 2, 3
+IMPL_AUTO, IMPL_GENERIC, IMPL_BGMV, IMPL_SGMV, IMPL_GROUPED = 0, 1, 2, 3, 4
 MAX_SLICES = 4
 
 E_INVAL, E_UNSUPPORTED, E_CUDA, E_WORKSPACE = -1, -2, -3, -4
@@ -144,14 +144,14 @@ def native():
         import importlib.machinery
         import importlib.util
 
-        from .lora import SGMV_MIN_TOKENS, scratch_for
+        from .lora import scratch_for
 
         loader = importlib.machinery.ExtensionFileLoader("b200lora_binding", BINDING_PATH)
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200lora_binding", loader))
         loader.exec_module(module)
         handle = lib()
         addresses = {name: ctypes.cast(getattr(handle, name), c_void_p).value for name in _SIGNATURES}
-        module.bind(addresses, scratch_for, SGMV_MIN_TOKENS)
+        module.bind(addresses, scratch_for)
         _NATIVE = module
     return _NATIVE
 

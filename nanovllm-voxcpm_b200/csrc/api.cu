@@ -9,6 +9,7 @@
 #include "glue.cuh"
 #include "sgmv_tc.cuh"
 #include "gemm_tc.cuh"
+#include "grouped_tc.cuh"
 
 using namespace b200lora;
 
@@ -221,7 +222,7 @@ int lora_b200_linear_lora(void* y, int64_t y_ld, const void* x, int64_t x_ld, in
 
 size_t lora_b200_workspace_bytes(int32_t T, int32_t n_slices, int32_t r_max) {
   if (T < 0 || n_slices < 1 || r_max < 1) return 0;
-  return sgmv_workspace_bytes(T, n_slices, r_max);
+  return std::max(sgmv_workspace_bytes(T, n_slices, r_max), grouped_workspace_bytes(T, n_slices, r_max));
 }
 
 int lora_b200_shrink_allreduce_expand(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,
@@ -336,6 +337,11 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
   sp.y = y; sp.y_ld = y_ld; sp.x = x; sp.x_ld = x_ld; sp.T = T; sp.in_dim = in_dim; sp.S = S; sp.r_max = r_max;
   sp.st = st; sp.scale_per_slot = scale_per_slot; sp.token_to_slot = token_to_slot; sp.scaling = scaling;
 
+  GroupedProblem gp;
+  gp.y = y; gp.y_ld = y_ld; gp.x = x; gp.x_ld = x_ld; gp.T = T; gp.in_dim = in_dim; gp.S = S; gp.r_max = r_max; gp.st = st;
+  gp.rank_per_slot = rank_per_slot; gp.scale_per_slot = scale_per_slot; gp.sorted_idx = sorted_idx; gp.slot_ids = slot_ids;
+  gp.counts = counts; gp.offsets = offsets; gp.n_buckets = n_buckets; gp.scaling = scaling; gp.dtype = dtype;
+
   if (overwrite) {
     // decode batches: the row-split kernel writes the delta (and the -0.0 rows) itself; everything else
     // fills y with -0.0 first and then adds as usual (-0.0 + d == d)
@@ -376,8 +382,11 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     if (dtype == B200_LORA_BF16 && T >= kSgmvAutoMinTokens && !scattered && sgmv_supported(sp, nullptr) &&
         workspace != nullptr && workspace_bytes >= sgmv_workspace_bytes(T, n_act, r_max))
       impl = B200_LORA_IMPL_SGMV;
-    else if (bgmv_ok)
+    else if (bgmv_ok && !(grouped_preferred(gp) && workspace != nullptr && workspace_bytes >= grouped_workspace_bytes(T, n_act, r_max) &&
+                          grouped_supported(gp, nullptr)))
       impl = B200_LORA_IMPL_BGMV;
+    else if (bgmv_ok)
+      impl = B200_LORA_IMPL_GROUPED;
     else
       impl = B200_LORA_IMPL_GENERIC;
   }
@@ -402,6 +411,9 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     case B200_LORA_IMPL_SGMV:
       if (dtype != B200_LORA_BF16) return fail(B200_LORA_EUNSUPPORTED, "prefill kernels are bf16 only");
       return prefill_add_launch(sp, workspace, workspace_bytes, st_);
+    case B200_LORA_IMPL_GROUPED:
+      // (where the fused decode kernel takes the batch too, the delta is rounded to bf16 and added at the L2 as there)
+      return grouped_add_launch(gp, workspace, workspace_bytes, dtype == B200_LORA_BF16 && r_max % 32 == 0, st_);
     default:
       return fail(B200_LORA_EUNSUPPORTED, "impl %d is not available", impl);
   }

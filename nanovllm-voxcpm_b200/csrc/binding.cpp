@@ -34,7 +34,6 @@ decltype(&lora_b200_glue_add_rmsnorm) p_rmsnorm = nullptr;
 decltype(&lora_b200_glue_silu_mul) p_silu = nullptr;
 decltype(&lora_b200_glue_rope_kv_store) p_rope = nullptr;
 PyObject* scratch_for = nullptr;  // lora.scratch_for(device, bytes)
-long sgmv_min_tokens = 512;       // lora.SGMV_MIN_TOKENS
 PyObject *s_tts, *s_sorted, *s_ids, *s_counts, *s_offsets, *s_num_active;
 
 inline const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
@@ -209,11 +208,13 @@ PyObject* add(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const void *rank, *scale;
   if (!optional_vector(args[8], at::kInt, sl.S, dev, &rank) || !optional_vector(args[9], at::kFloat, sl.S, dev, &scale))
     return not_handled();
-  const bool tiled = code == B200_LORA_BF16 && (impl == B200_LORA_IMPL_SGMV || (impl == B200_LORA_IMPL_AUTO && T >= sgmv_min_tokens));
+  // (the tensor-core kernels keep the rank-r intermediate in scratch)
+  const bool scratch = code != B200_LORA_F32 &&
+                       (impl == B200_LORA_IMPL_AUTO || impl == B200_LORA_IMPL_SGMV || impl == B200_LORA_IMPL_GROUPED);
   PyObject* keep;
   void* ws;
   size_t ws_bytes;
-  if (!workspace(args[11], *x, tiled ? p_workspace_bytes((int)T, sl.n, (int)sl.r) : 0, &keep, &ws, &ws_bytes)) return nullptr;
+  if (!workspace(args[11], *x, scratch ? p_workspace_bytes((int)T, sl.n, (int)sl.r) : 0, &keep, &ws, &ws_bytes)) return nullptr;
   void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   const auto fn = args[12] == Py_True ? p_delta : p_add;
   int rc;
@@ -470,9 +471,9 @@ PyObject* pack_lists(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(addresses: dict name -> int, scratch_for, sgmv_min_tokens)
+// bind(addresses: dict name -> int, scratch_for)
 PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-  if (nargs != 3 || !PyDict_Check(args[0])) { PyErr_SetString(PyExc_TypeError, "bind(dict, callable, int)"); return nullptr; }
+  if (nargs != 2 || !PyDict_Check(args[0])) { PyErr_SetString(PyExc_TypeError, "bind(dict, callable)"); return nullptr; }
   auto address = [&](const char* name) -> void* {
     PyObject* v = PyDict_GetItemString(args[0], name);
     return v == nullptr ? nullptr : PyLong_AsVoidPtr(v);
@@ -490,8 +491,6 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Py_INCREF(args[1]);
   Py_XDECREF(scratch_for);
   scratch_for = args[1];
-  sgmv_min_tokens = PyLong_AsLong(args[2]);
-  if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
 }
 

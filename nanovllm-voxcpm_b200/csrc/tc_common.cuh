@@ -138,6 +138,14 @@ inline std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash>& tmap_cache() {
 }
 
 inline int make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
+                        uint32_t box_rows, uint32_t box_cols);
+
+// Map for gathered rows (tile::gather4): boxes of one row and 64 columns.
+inline int make_tmap_rows(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld) {
+  return make_tmap_2d(out, base, rows, cols, ld, 1, 64);
+}
+
+inline int make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                         uint32_t box_rows, uint32_t box_cols) {
   const TmapKey key = {base, rows, cols, ld, box_rows, box_cols};
   auto& cache = tmap_cache();
@@ -161,6 +169,31 @@ inline int make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint6
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(B200_LORA_ECUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  if (cache.size() >= kTmapCacheEntries) cache.clear();
+  cache.emplace(key, *out);
+  return B200_LORA_OK;
+}
+
+// 3-D view of a dense row-major [rows, cols] matrix as 64-column panels: coordinates (column in panel, row, panel), boxes of
+// 64 columns x box_rows x box_panels that arrive panel by panel. cols must be a multiple of 64.
+inline int make_tmap_panels(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_panels) {
+  const TmapKey key = {base, rows, cols, cols, box_rows, 64u | box_panels << 16};
+  auto& cache = tmap_cache();
+  auto hit = cache.find(key);
+  if (hit != cache.end()) {
+    *out = hit->second;
+    return B200_LORA_OK;
+  }
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (fn == nullptr) return fail(B200_LORA_ECUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[3] = {64, rows, cols / 64};
+  cuuint64_t strides[2] = {cols * 2, 128};
+  cuuint32_t box[3] = {64, box_rows, box_panels};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(B200_LORA_ECUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
   if (cache.size() >= kTmapCacheEntries) cache.clear();
   cache.emplace(key, *out);

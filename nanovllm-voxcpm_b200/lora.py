@@ -184,9 +184,7 @@ def launch_add(
     if n_buckets <= 0:
         srt = ids = cnt = off = None
         n_buckets = 0
-    if workspace is None and x.dtype == torch.bfloat16 and (
-        impl == N.IMPL_SGMV or (impl == N.IMPL_AUTO and T >= SGMV_MIN_TOKENS)
-    ):
+    if workspace is None and x.dtype != torch.float32 and impl in (N.IMPL_AUTO, N.IMPL_SGMV, N.IMPL_GROUPED):
         workspace = scratch_for(x.device, N.workspace_bytes(T, len(a_slabs), r_max))
     with N.on_device(x.device):
         rc = (N.lib().lora_b200_delta if overwrite else N.lib().lora_b200_add)(
