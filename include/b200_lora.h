@@ -165,6 +165,17 @@ int lora_b200_shrink(void* out, int32_t out_dtype, const void* x, int64_t x_ld, 
                      void* stream);
 
 /*
+ * lora_b200_shrink with the bucket arrays of lora_b200_add: batches of scattered rows run on the shrink half of the fused
+ * decode kernel (bf16 / fp16, r_max a multiple of 16), which fetches an adapter once per bucket instead of once per row.
+ * The arrays and token_to_slot must describe one routing.
+ */
+int lora_b200_shrink_buckets(void* out, int32_t out_dtype, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,
+                             int32_t n_slices, const void* const* a_slabs, int32_t S, int32_t r_max,
+                             const int32_t* token_to_slot, const int32_t* sorted_idx, const int32_t* slot_ids,
+                             const int32_t* counts, const int32_t* offsets, int32_t n_buckets, float scaling,
+                             int32_t dtype, void* stream);
+
+/*
  * y[t, offset_start + sum(out_sizes[:s]) + c] (+)= tmp[s, t, :] . B_s[slot_t][c, :]
  * for slot_t >= 0; `add_inputs` = 0 overwrites instead of accumulating.
  *
@@ -176,6 +187,13 @@ int lora_b200_expand(void* y, int64_t y_ld, const void* tmp, int32_t tmp_dtype, 
                      const int32_t* col_offsets, int32_t S, int32_t r_max,
                      const int32_t* token_to_slot, int32_t add_inputs, int32_t dtype,
                      void* stream);
+
+/* lora_b200_expand with the bucket arrays (see lora_b200_shrink_buckets). */
+int lora_b200_expand_buckets(void* y, int64_t y_ld, const void* tmp, int32_t tmp_dtype, int32_t T, int32_t n_slices,
+                             const void* const* b_slabs, const int32_t* out_sizes, const int32_t* col_offsets, int32_t S,
+                             int32_t r_max, const int32_t* token_to_slot, const int32_t* sorted_idx,
+                             const int32_t* slot_ids, const int32_t* counts, const int32_t* offsets,
+                             int32_t n_buckets, int32_t add_inputs, int32_t dtype, void* stream);
 
 /*
  * Prefill multi-LoRA add for callers that cannot allocate device memory (code running

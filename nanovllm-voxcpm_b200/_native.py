@@ -55,6 +55,16 @@ _SIGNATURES = {
         [c_void_p, c_int64, c_void_p, c_int32, c_int32, c_int32, POINTER(c_void_p), POINTER(c_int32),
          POINTER(c_int32), c_int32, c_int32, c_void_p, c_int32, c_int32, c_void_p],
     ),
+    "lora_b200_shrink_buckets": (
+        c_int32,
+        [c_void_p, c_int32, c_void_p, c_int64, c_int32, c_int32, c_int32, POINTER(c_void_p), c_int32, c_int32,
+         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_float, c_int32, c_void_p],
+    ),
+    "lora_b200_expand_buckets": (
+        c_int32,
+        [c_void_p, c_int64, c_void_p, c_int32, c_int32, c_int32, POINTER(c_void_p), POINTER(c_int32),
+         POINTER(c_int32), c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p],
+    ),
     "lora_b200_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
     "lora_b200_linear_lora": (
         c_int32,

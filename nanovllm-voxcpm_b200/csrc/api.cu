@@ -445,10 +445,11 @@ int lora_b200_delta(void* delta, int64_t delta_ld, const void* x, int64_t x_ld, 
                       scaling, dtype, impl, workspace, workspace_bytes, stream, 1);
 }
 
-int lora_b200_shrink(void* out, int32_t out_dtype, const void* x, int64_t x_ld, int32_t T,
-                     int32_t in_dim, int32_t n_slices, const void* const* a_slabs, int32_t S,
-                     int32_t r_max, const int32_t* token_to_slot, float scaling, int32_t dtype,
-                     void* stream) {
+int lora_b200_shrink_buckets(void* out, int32_t out_dtype, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,
+                             int32_t n_slices, const void* const* a_slabs, int32_t S, int32_t r_max,
+                             const int32_t* token_to_slot, const int32_t* sorted_idx, const int32_t* slot_ids,
+                             const int32_t* counts, const int32_t* offsets, int32_t n_buckets, float scaling, int32_t dtype,
+                             void* stream) {
   if (!valid_dtype(dtype) || !valid_dtype(out_dtype)) return fail(B200_LORA_EINVAL, "unknown dtype");
   if (out_dtype != dtype && out_dtype != B200_LORA_F32)
     return fail(B200_LORA_EUNSUPPORTED, "shrink output must have the input dtype or be f32");
@@ -459,7 +460,21 @@ int lora_b200_shrink(void* out, int32_t out_dtype, const void* x, int64_t x_ld, 
   SliceTable st;
   if (int rc = fill_slices(st, n_slices, a_slabs, nullptr, nullptr, nullptr, true, false)) return rc;
   cudaStream_t st_ = static_cast<cudaStream_t>(stream);
-  if (dtype == B200_LORA_BF16 && out_dtype == B200_LORA_BF16 && T >= kSgmvAutoMinTokens) {
+  // With bucket arrays: the shrink half of the fused decode kernel (same sums as the per-token kernel, which reads an
+  // adapter again for every row), except for long batches of contiguous rows, which the tensor-core shrink takes.
+  const bool buckets = sorted_idx && slot_ids && counts && offsets && n_buckets > 0;
+  const bool contiguous = T >= kSgmvAutoMinTokens && !(buckets && T < 32 * n_buckets);
+  if (buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && !(dtype == B200_LORA_BF16 && out_dtype == B200_LORA_BF16 && contiguous)) {
+    BgmvProblem bp = {};
+    bp.y = nullptr; bp.y_ld = 8; bp.x = x; bp.x_ld = x_ld; bp.T = T; bp.in_dim = in_dim; bp.st = st; bp.S = S; bp.r_max = r_max;
+    for (int s = 0; s < st.n; ++s) bp.st.out[s] = 8;  // (no output columns here)
+    bp.rank_per_slot = nullptr; bp.scale_per_slot = nullptr;
+    bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets;
+    bp.n_buckets = n_buckets; bp.scaling = scaling; bp.mode = 1; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
+    bp.tmp_io = out; bp.io16 = out_dtype != B200_LORA_F32; bp.zero_rows = 1; bp.token_to_slot = token_to_slot;
+    if (aligned16(out) && bgmv_supported(bp, nullptr)) return bgmv_launch(bp, st_);
+  }
+  if (dtype == B200_LORA_BF16 && out_dtype == B200_LORA_BF16 && contiguous) {
     // prefill-sized bf16 batches: the tensor-core shrink (rows without adapter are written as zeros, as the
     // per-token kernel does); anything it does not take falls through to the per-token kernel
     SgmvProblem sp;
@@ -483,11 +498,11 @@ int lora_b200_shrink(void* out, int32_t out_dtype, const void* x, int64_t x_ld, 
 #undef B200_SHRINK
 }
 
-int lora_b200_expand(void* y, int64_t y_ld, const void* tmp, int32_t tmp_dtype, int32_t T,
-                     int32_t n_slices, const void* const* b_slabs, const int32_t* out_sizes,
-                     const int32_t* col_offsets, int32_t S, int32_t r_max,
-                     const int32_t* token_to_slot, int32_t add_inputs, int32_t dtype,
-                     void* stream) {
+int lora_b200_expand_buckets(void* y, int64_t y_ld, const void* tmp, int32_t tmp_dtype, int32_t T, int32_t n_slices,
+                             const void* const* b_slabs, const int32_t* out_sizes, const int32_t* col_offsets, int32_t S,
+                             int32_t r_max, const int32_t* token_to_slot, const int32_t* sorted_idx, const int32_t* slot_ids,
+                             const int32_t* counts, const int32_t* offsets, int32_t n_buckets, int32_t add_inputs, int32_t dtype,
+                             void* stream) {
   if (!valid_dtype(dtype) || !valid_dtype(tmp_dtype)) return fail(B200_LORA_EINVAL, "unknown dtype");
   if (tmp_dtype != dtype && tmp_dtype != B200_LORA_F32)
     return fail(B200_LORA_EUNSUPPORTED, "expand input must have the weight dtype or be f32");
@@ -501,7 +516,21 @@ int lora_b200_expand(void* y, int64_t y_ld, const void* tmp, int32_t tmp_dtype, 
   for (int s = 0; s < st.n; ++s)
     if (y_ld < (int64_t)st.col[s] + st.out[s]) return fail(B200_LORA_EINVAL, "y_ld smaller than slice end");
   cudaStream_t st_ = static_cast<cudaStream_t>(stream);
-  if (dtype == B200_LORA_BF16 && tmp_dtype == B200_LORA_BF16 && add_inputs && T >= kSgmvAutoMinTokens) {
+  const bool buckets = sorted_idx && slot_ids && counts && offsets && n_buckets > 0;
+  const bool contiguous = T >= kSgmvAutoMinTokens && !(buckets && T < 32 * n_buckets);
+  if (buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) &&
+      !(dtype == B200_LORA_BF16 && tmp_dtype == B200_LORA_BF16 && add_inputs && contiguous)) {
+    bool dense = true;  // tmp is indexed by slice position
+    for (int s = 0; s < st.n; ++s) dense = dense && st.out[s] > 0;
+    BgmvProblem bp = {};
+    bp.y = y; bp.y_ld = y_ld; bp.x = nullptr; bp.x_ld = 32; bp.T = T; bp.in_dim = 32; bp.st = st; bp.S = S; bp.r_max = r_max;
+    bp.rank_per_slot = nullptr; bp.scale_per_slot = nullptr;
+    bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets;
+    bp.n_buckets = n_buckets; bp.scaling = 1.0f; bp.mode = 2; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
+    bp.tmp_io = const_cast<void*>(tmp); bp.io16 = tmp_dtype != B200_LORA_F32; bp.no_add = add_inputs ? 0 : 1;
+    if (dense && aligned16(tmp) && bgmv_supported(bp, nullptr)) return bgmv_launch(bp, st_);
+  }
+  if (dtype == B200_LORA_BF16 && tmp_dtype == B200_LORA_BF16 && add_inputs && contiguous) {
     // prefill-sized bf16 batches: the tensor-core expand (reduce-add tile kernel when the slices tile the
     // columns they cover in 64-column units, run-based kernel otherwise)
     int first = -1;
@@ -538,6 +567,20 @@ int lora_b200_expand(void* y, int64_t y_ld, const void* tmp, int32_t tmp_dtype, 
   if (dtype == B200_LORA_F16) return B200_EXPAND(__half);
   return launch_generic_expand<float, float>(y, y_ld, tmp, T, st, S, r_max, token_to_slot, add_inputs, st_);
 #undef B200_EXPAND
+}
+
+int lora_b200_shrink(void* out, int32_t out_dtype, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, int32_t n_slices,
+                     const void* const* a_slabs, int32_t S, int32_t r_max, const int32_t* token_to_slot, float scaling,
+                     int32_t dtype, void* stream) {
+  return lora_b200_shrink_buckets(out, out_dtype, x, x_ld, T, in_dim, n_slices, a_slabs, S, r_max, token_to_slot, nullptr, nullptr,
+                                  nullptr, nullptr, 0, scaling, dtype, stream);
+}
+
+int lora_b200_expand(void* y, int64_t y_ld, const void* tmp, int32_t tmp_dtype, int32_t T, int32_t n_slices,
+                     const void* const* b_slabs, const int32_t* out_sizes, const int32_t* col_offsets, int32_t S, int32_t r_max,
+                     const int32_t* token_to_slot, int32_t add_inputs, int32_t dtype, void* stream) {
+  return lora_b200_expand_buckets(y, y_ld, tmp, tmp_dtype, T, n_slices, b_slabs, out_sizes, col_offsets, S, r_max, token_to_slot,
+                                  nullptr, nullptr, nullptr, nullptr, 0, add_inputs, dtype, stream);
 }
 
 }  // extern "C"

@@ -33,6 +33,8 @@ decltype(&lora_b200_linear_lora) p_linear = nullptr;
 decltype(&lora_b200_glue_add_rmsnorm) p_rmsnorm = nullptr;
 decltype(&lora_b200_glue_silu_mul) p_silu = nullptr;
 decltype(&lora_b200_glue_rope_kv_store) p_rope = nullptr;
+decltype(&lora_b200_shrink_buckets) p_shrink = nullptr;
+decltype(&lora_b200_expand_buckets) p_expand = nullptr;
 PyObject* scratch_for = nullptr;  // lora.scratch_for(device, bytes)
 PyObject *s_tts, *s_sorted, *s_ids, *s_counts, *s_offsets, *s_num_active;
 
@@ -224,6 +226,120 @@ PyObject* add(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
           k.counts, k.offsets, k.n, (float)scaling, code, (int)impl, ws, ws_bytes, stream);
   Py_END_ALLOW_THREADS
   Py_XDECREF(keep);
+  return PyLong_FromLong(rc);
+  END_HANDLE_TH_ERRORS
+}
+
+// Bucket arrays given one by one (mapping, sorted, counts, offsets, ids: five tensors, n_active as an int)
+bool read_arrays(PyObject* const* args, int64_t T, int dev, Buckets* k) {
+  const at::Tensor* t[5];
+  for (int i = 0; i < 5; ++i) {
+    t[i] = tensor_of(args[i]);
+    if (t[i] == nullptr) {
+      if (i == 0 || args[i] != Py_None) return false;
+      continue;
+    }
+    if (t[i]->scalar_type() != at::kInt || t[i]->dim() != 1 || !t[i]->is_contiguous() || !on(*t[i], dev)) return false;
+  }
+  if (t[0]->numel() < T) return false;
+  const long active = PyLong_AsLong(args[5]);
+  if (active == -1 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+  k->tts = static_cast<const int32_t*>(t[0]->data_ptr());
+  k->n = 0;
+  k->sorted = k->ids = k->counts = k->offsets = nullptr;
+  if (t[1] && t[2] && t[3] && t[4]) {
+    int64_t nb = std::min(t[4]->numel(), std::min(t[2]->numel(), t[3]->numel() - 1));
+    if (active > 0) nb = std::min<int64_t>(nb, active);
+    if (nb > 0) {
+      k->n = (int)nb;
+      k->sorted = static_cast<const int32_t*>(t[1]->data_ptr()); k->counts = static_cast<const int32_t*>(t[2]->data_ptr());
+      k->offsets = static_cast<const int32_t*>(t[3]->data_ptr()); k->ids = static_cast<const int32_t*>(t[4]->data_ptr());
+    }
+  }
+  return true;
+}
+
+// Slabs [S, a, b] of one list (lora_A: one shape; lora_B: widths may differ); false = not handled
+bool read_slabs(PyObject* list, bool lora_a, at::ScalarType dt, int dev, const void** ptr, int32_t* widths, int* n, int64_t (&shape)[3]) {
+  PyObject** it;
+  const Py_ssize_t m = items(list, &it);
+  if (m < 1 || m > B200_LORA_MAX_SLICES) return false;
+  for (Py_ssize_t i = 0; i < m; ++i) {
+    const at::Tensor* t = tensor_of(it[i]);
+    if (t == nullptr || t->dim() != 3 || !t->is_contiguous() || t->scalar_type() != dt || !on(*t, dev)) return false;
+    const auto z = t->sizes();
+    if (i == 0) { shape[0] = z[0]; shape[1] = z[1]; shape[2] = z[2]; }
+    if (z[0] != shape[0] || z[2] != shape[2] || (lora_a && z[1] != shape[1]) || z[1] > INT32_MAX) return false;
+    ptr[i] = t->data_ptr();
+    widths[i] = (int32_t)z[1];
+  }
+  *n = (int)m;
+  return shape[0] <= INT32_MAX && shape[2] <= INT32_MAX;
+}
+
+// shrink(x, a_slabs, out, mapping, sorted, counts, offsets, ids, n_active, scaling) -> status, or None
+PyObject* shrink(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 10) { PyErr_SetString(PyExc_TypeError, "shrink takes 10 arguments"); return nullptr; }
+  const at::Tensor *x = tensor_of(args[0]), *out = tensor_of(args[2]);
+  if (x == nullptr || out == nullptr || !x->is_cuda() || x->dim() != 2 || x->stride(1) != 1 || out->dim() != 3) return not_handled();
+  const int dev = x->get_device();
+  const int code = dtype_code(x->scalar_type()), out_code = dtype_code(out->scalar_type());
+  const int64_t T = x->size(0);
+  if (code < 0 || out_code < 0 || dev != c10::cuda::current_device() || !on(*out, dev) || !out->is_contiguous() || T > INT32_MAX) return not_handled();
+  const void* a[B200_LORA_MAX_SLICES];
+  int32_t widths[B200_LORA_MAX_SLICES];
+  int n;
+  int64_t shape[3];
+  Buckets k;
+  if (!read_slabs(args[1], true, x->scalar_type(), dev, a, widths, &n, shape) || shape[2] != x->size(1) || out->size(0) != n ||
+      out->size(1) != T || out->size(2) != shape[1] || !read_arrays(args + 3, T, dev, &k))
+    return not_handled();
+  const double scaling = PyFloat_AsDouble(args[9]);
+  if (PyErr_Occurred()) { PyErr_Clear(); return not_handled(); }
+  void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = p_shrink(out->data_ptr(), out_code, x->data_ptr(), x->stride(0), (int)T, (int)shape[2], n, a, (int)shape[0], (int)shape[1], k.tts,
+                k.sorted, k.ids, k.counts, k.offsets, k.n, (float)scaling, code, stream);
+  Py_END_ALLOW_THREADS
+  return PyLong_FromLong(rc);
+  END_HANDLE_TH_ERRORS
+}
+
+// expand(tmp, b_slabs, y, mapping, sorted, counts, offsets, ids, n_active, offset_start, add_inputs) -> status, or None
+PyObject* expand(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 11) { PyErr_SetString(PyExc_TypeError, "expand takes 11 arguments"); return nullptr; }
+  const at::Tensor *tmp = tensor_of(args[0]), *y = tensor_of(args[2]);
+  if (tmp == nullptr || y == nullptr || !y->is_cuda() || y->dim() != 2 || y->stride(1) != 1 || tmp->dim() != 3 || !tmp->is_contiguous())
+    return not_handled();
+  const int dev = y->get_device();
+  const int code = dtype_code(y->scalar_type()), tmp_code = dtype_code(tmp->scalar_type());
+  const int64_t T = y->size(0);
+  if (code < 0 || tmp_code < 0 || dev != c10::cuda::current_device() || !on(*tmp, dev) || T > INT32_MAX) return not_handled();
+  const void* b[B200_LORA_MAX_SLICES];
+  int32_t widths[B200_LORA_MAX_SLICES], cols[B200_LORA_MAX_SLICES];
+  int n;
+  int64_t shape[3];
+  Buckets k;
+  if (!read_slabs(args[1], false, y->scalar_type(), dev, b, widths, &n, shape) || tmp->size(0) != n || tmp->size(1) != T ||
+      tmp->size(2) != shape[2] || !read_arrays(args + 3, T, dev, &k))
+    return not_handled();
+  int64_t col = PyLong_AsLongLong(args[9]);
+  if (PyErr_Occurred()) { PyErr_Clear(); return not_handled(); }
+  for (int i = 0; i < n; ++i) {
+    if (col < 0 || col + widths[i] > y->size(1)) return not_handled();
+    cols[i] = (int32_t)col;
+    col += widths[i];
+  }
+  void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const int add_inputs = args[10] == Py_True;
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = p_expand(y->data_ptr(), y->stride(0), tmp->data_ptr(), tmp_code, (int)T, n, b, widths, cols, (int)shape[0], (int)shape[2], k.tts,
+                k.sorted, k.ids, k.counts, k.offsets, k.n, add_inputs, code, stream);
+  Py_END_ALLOW_THREADS
   return PyLong_FromLong(rc);
   END_HANDLE_TH_ERRORS
 }
@@ -486,6 +602,8 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   B200_BIND(p_linear, lora_b200_linear_lora)
   B200_BIND(p_rmsnorm, lora_b200_glue_add_rmsnorm)
   B200_BIND(p_silu, lora_b200_glue_silu_mul)
+  B200_BIND(p_shrink, lora_b200_shrink_buckets)
+  B200_BIND(p_expand, lora_b200_expand_buckets)
   B200_BIND(p_rope, lora_b200_glue_rope_kv_store)
 #undef B200_BIND
   Py_INCREF(args[1]);
@@ -495,7 +613,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 }
 
 #define B200_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {B200_METHOD(add), B200_METHOD(linear), B200_METHOD(add_rms_norm), B200_METHOD(silu_mul),
+PyMethodDef methods[] = {B200_METHOD(add), B200_METHOD(shrink), B200_METHOD(expand), B200_METHOD(linear), B200_METHOD(add_rms_norm), B200_METHOD(silu_mul),
                          B200_METHOD(rope_kv_store), B200_METHOD(bucket_lists), B200_METHOD(pack_lists), B200_METHOD(bind), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "b200lora_binding", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -89,7 +89,6 @@ def expand_into(
     N.check(rc)
 
 
-@torch.inference_mode()
 def lora_shrink(
     inputs: torch.Tensor,
     lora_a_weights: list[torch.Tensor],
@@ -105,14 +104,18 @@ def lora_shrink(
 ) -> None:
     """``output[s, t] = scaling * inputs[t] @ A_s[slot_t].T``; rows without an adapter are zero.
 
-    The kernel routes by ``token_lora_mapping``; the bucket tensors are accepted for
-    signature compatibility (a per-token shrink needs nothing else)."""
+    Batches of scattered rows are grouped by the bucket tensors; without them (``None``) every row is routed by
+    ``token_lora_mapping``."""
     if no_lora_flag:
         return
-    shrink_into(output_tensor, inputs, lora_a_weights, token_lora_mapping, scaling)
+    rc = N.native().shrink(inputs, lora_a_weights, output_tensor, token_lora_mapping, token_indices_sorted_by_lora_ids,
+                           num_tokens_per_lora, lora_token_start_loc, lora_ids, num_active_loras, scaling)
+    if rc is not None:
+        return N.check(rc)
+    with torch.inference_mode():
+        shrink_into(output_tensor, inputs, lora_a_weights, token_lora_mapping, scaling)
 
 
-@torch.inference_mode()
 def lora_expand(
     inputs: torch.Tensor,
     lora_b_weights: list[torch.Tensor],
@@ -130,9 +133,12 @@ def lora_expand(
     """``output[t, offset_start + ...] (+)= inputs[s, t] @ B_s[slot_t].T`` for rows with an adapter."""
     if no_lora_flag:
         return
-    expand_into(
-        output_tensor, inputs, lora_b_weights, token_lora_mapping, offset_start=offset_start, add_inputs=add_inputs
-    )
+    rc = N.native().expand(inputs, lora_b_weights, output_tensor, token_lora_mapping, token_indices_sorted_by_lora_ids,
+                           num_tokens_per_lora, lora_token_start_loc, lora_ids, num_active_loras, offset_start, add_inputs)
+    if rc is not None:
+        return N.check(rc)
+    with torch.inference_mode():
+        expand_into(output_tensor, inputs, lora_b_weights, token_lora_mapping, offset_start=offset_start, add_inputs=add_inputs)
 
 
 @dataclass

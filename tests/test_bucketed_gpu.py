@@ -1,4 +1,4 @@
-"""The kernel for bucketed batches of both 16-bit types (``csrc/bgmv_fused.cuh``): parity with the
+"""The kernels for bucketed batches of both 16-bit types (``csrc/grouped_tc.cuh``, ``csrc/bgmv_fused.cuh``): parity with the
 CPU oracle at the edges of their tiles - one token, 16- and 32-token chunks and their remainders, partial 128-row output
 tiles, K tails and K parts, every rank, popular buckets, mixed ranks, slots of rank 0 - through ``lora_b200_add`` with the
 kernel asked for by name."""
@@ -10,6 +10,7 @@ from helpers import assert_lora_close
 from nanovllm_voxcpm_b200 import _native as N
 from nanovllm_voxcpm_b200 import lora as LORA
 from nanovllm_voxcpm_b200 import workloads as W
+from nanovllm_voxcpm_b200.lora_ops import LoRAKernelMeta, lora_expand, lora_shrink
 from oracle import lora_oracle as O
 from test_parity_gpu import metadata_for
 
@@ -31,8 +32,26 @@ CASES = [
 ]
 
 
+@pytest.mark.parametrize("cluster", [1, 4, 8])
+@pytest.mark.parametrize("r", [64, 128, 256])
+def test_fused_decode_kernel_wide_ranks(r, cluster):
+    """Ranks whose output tiles are 128, 64 and 32 rows high (several tiles per step), clusters with few rank rows each."""
+    p = W.make_projection(70 + r, 21, 2048, [1184, 96], 3, r)
+    d = p.to_device(DEV)
+    y = d.y.clone()
+    N.set_option(N.OPT_CLUSTER, cluster)
+    try:
+        LORA.launch_add(y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata_for(p.token_to_slot, "graph", 3), 1.0,
+                        impl=N.IMPL_BGMV)
+        torch.cuda.synchronize()
+    finally:
+        N.set_option(N.OPT_CLUSTER, 0)
+    assert N.device_status(reset=True) == 0
+    assert_lora_close(y, O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets), max_abs=6e-2, what=f"r{r}")
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
-@pytest.mark.parametrize("impl", [N.IMPL_BGMV], ids=["bgmv"])
+@pytest.mark.parametrize("impl", [N.IMPL_GROUPED, N.IMPL_BGMV], ids=["grouped", "bgmv"])
 @pytest.mark.parametrize("case", range(len(CASES)))
 def test_bucketed_kernels_match_oracle(case, impl, dtype):
     T, in_dim, outs, S, r, kw = CASES[case]
@@ -52,3 +71,34 @@ def test_bucketed_kernels_match_oracle(case, impl, dtype):
     assert_lora_close(y, ref, what=f"{CASES[case]} {dtype}")
     none = p.token_to_slot < 0
     assert torch.equal(y.cpu()[none].view(torch.int16), p.y[none].view(torch.int16)), "rows without adapter changed"
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("case", [0, 2, 5, 7, 8, 9])
+def test_operators_with_bucket_arrays_match_oracle(case, dtype):
+    """``lora_shrink`` and ``lora_expand`` with the vLLM-style arrays: intermediate in the activations' type and in fp32, rows
+    without adapter zero, expand adding and overwriting."""
+    T, in_dim, outs, S, r, kw = CASES[case]
+    p = W.make_projection(300 + case, T, in_dim, outs, S, r, dtype=dtype, **kw)
+    d = p.to_device(DEV)
+    km = LoRAKernelMeta.make(S, T, DEV)
+    km.prepare_tensors(d.token_to_slot)
+    args = km.meta_args(T, specialize_active_lora=True)
+    none = p.token_to_slot < 0
+    for out_dtype in (dtype, torch.float32):
+        tmp = torch.full((len(outs), T, r), 3.0, device=DEV, dtype=out_dtype)
+        lora_shrink(d.x, d.a_slabs, tmp, *args, 0.5)
+        ref_tmp = O.shrink(p.x, p.a_slabs, p.token_to_slot, 0.5)
+        assert_lora_close(tmp, ref_tmp, what=f"shrink {out_dtype}")
+        assert not tmp.cpu()[:, none].any()
+        y = d.y.clone()
+        lora_expand(tmp, d.b_slabs, y, *args, offset_start=0, add_inputs=True)
+        assert_lora_close(y, O.expand(p.y, tmp.float().cpu(), p.b_slabs, p.token_to_slot), what="expand")
+        assert torch.equal(y.cpu()[none].view(torch.int16), p.y[none].view(torch.int16))
+        k = len(outs) - 1
+        y2 = torch.zeros_like(d.y)
+        lora_expand(tmp[k:].contiguous(), d.b_slabs[k:], y2, *args, offset_start=p.col_offsets[k], add_inputs=False)
+        want = O.expand(torch.zeros_like(p.y), tmp[k:].float().cpu(), p.b_slabs[k:], p.token_to_slot, p.col_offsets[k], False)
+        assert_lora_close(y2, want, what="expand, overwriting")
+        assert not y2.cpu()[:, : p.col_offsets[k]].any()
+    assert N.device_status(reset=True) == 0
