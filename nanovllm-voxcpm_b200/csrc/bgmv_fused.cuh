@@ -370,46 +370,10 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
       }
       __syncwarp();
       if (++p_stage == NS) { p_stage = 0; ++p_round; }
-      if (it + 1 == npro) {
-        B200_TRACE_PRODUCER(3)
-        // The ring is full and the previous launch of the stream may still be running: ask the L2 for
-        // the rest of this CTA's weights now, so that the refills that follow the wait find them there.
-        if (shrink_tiles + tiles_exp > npro && ksplit) {
-          // one row piece per lane: rank row q of this CTA's K part ikp
-#pragma unroll 1
-          for (int idx = lane; idx < rows_c * nkp_c; idx += 32) {
-            const int ikp = idx / max(rows_c, 1), q = idx - ikp * rows_c;
-            const int s = q / r_eff, r0 = q - s * r_eff, k0 = (kp0 + ikp * kstep) * KP;
-            const void* aptr = nullptr;
-#pragma unroll
-            for (int ss = 0; ss < B200_LORA_MAX_SLICES; ++ss)
-              if (ss == s) aptr = p.st.a[ss];
-            bulk_prefetch_l2(static_cast<const __nv_bfloat16*>(aptr) + ((int64_t)slot * p.r_max + r0) * in_dim + k0,
-                             (uint32_t)min(KP, in_dim - k0) * 2u);
-          }
-        }
-        if (shrink_tiles + tiles_exp > npro && lane == 0) {
-          int q = q_lo;
-          const int q_hi = ksplit ? q_lo : q_lo + rows_c;
-#pragma unroll 1
-          while (q < q_hi) {
-            const int s = q / r_eff, r0 = q - s * r_eff;
-            const int nr = min(r_eff - r0, q_hi - q);
-            const void* aptr = nullptr;
-#pragma unroll
-            for (int ss = 0; ss < B200_LORA_MAX_SLICES; ++ss)
-              if (ss == s) aptr = p.st.a[ss];
-            bulk_prefetch_l2(static_cast<const __nv_bfloat16*>(aptr) + ((int64_t)slot * p.r_max + r0) * in_dim,
-                             (uint32_t)nr * (uint32_t)in_dim * 2u);
-            q += nr;
-          }
-#pragma unroll
-          for (int s = 0; s < B200_LORA_MAX_SLICES; ++s)
-            if (s < n && e_n[s] > 0)
-              bulk_prefetch_l2(static_cast<const __nv_bfloat16*>(p.st.b[s]) + ((int64_t)slot * p.st.out[s] + e_lo[s]) * p.r_max,
-                               (uint32_t)e_n[s] * (uint32_t)p.r_max * 2u);
-        }
-      }
+      if (it + 1 == npro) { B200_TRACE_PRODUCER(3) }
+      // (What the ring cannot hold is not prefetched to the L2 either: on top of a full ring on every SM it only queued in
+      // front of the copies that are waited for. Without it 200 rows over 128 adapters, 2048-wide: 17.1 -> 14.2 us, 256 rows
+      // over 32: 4.91 -> 4.79.)
     }
     cluster_wait();
     return;
@@ -417,7 +381,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
 
   // ============================= consumer warps =============================
   // Everything that does not depend on the previous launch of the stream is done before the wait:
-  // token rows, the table of this CTA's expand tiles, thread-constant address pieces and L2 prefetches
+  // token rows, the table of this CTA's expand tiles, thread-constant address pieces and L2 prefetches of x
   // (a prefetch never creates stale data: L2 is the point of coherence). What runs after the wait is
   // the dependent chain activations -> shrink -> all-gather -> expand, kept as short as possible.
   int tok0_lo = -1, tok0_hi = -1;
@@ -458,16 +422,6 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
       for (int kc = k0 + x_col; kc < min(k0 + KP, in_dim); kc += kBgmvWarps * 32) {
         if (tok0_lo >= 0) prefetch_l2(p.x + (int64_t)tok0_lo * p.x_ld + kc);
         if (tok0_hi >= 0) prefetch_l2(p.x + (int64_t)tok0_hi * p.x_ld + kc);
-      }
-    }
-    if (!kOverwrite) {  // the lines of y that this thread's reductions will land in
-#pragma unroll 1
-      for (int e = sub; e < tiles_exp; e += U) {
-        const int2 te = etab[e];
-        if (y_col < (te.y & 0xffff)) {
-          if (tok0_lo >= 0) prefetch_l2(p.y + (int64_t)tok0_lo * p.y_ld + te.x + y_col);
-          if (tok0_hi >= 0) prefetch_l2(p.y + (int64_t)tok0_hi * p.y_ld + te.x + y_col);
-        }
       }
     }
   }
