@@ -145,18 +145,32 @@ inline bool optional_vector(PyObject* o, at::ScalarType dt, int64_t S, int dev, 
   return true;
 }
 
-// Scratch of the prefill kernels: the caller's tensor, or the package's per-device buffer.
+// Scratch of the tensor-core kernels: the caller's tensor, or the package's per-device buffer. That buffer only grows and an
+// outgrown one stays allocated, so the last one seen per device is asked again only when it is too small (asking costs 1 us).
 // Returns a new reference in *keep (may be null); false with a Python error set.
+constexpr int kMaxDevices = 64;
+PyObject* scratch_seen[kMaxDevices] = {};
 bool workspace(PyObject* given, const at::Tensor& x, size_t need, PyObject** keep, void** ptr, size_t* bytes) {
   *keep = nullptr; *ptr = nullptr; *bytes = 0;
   PyObject* o = given;
   if (o == Py_None) {
     if (need == 0) return true;
-    PyObject* device = THPDevice_New(x.device());
-    if (device == nullptr) return false;
-    *keep = PyObject_CallFunction(scratch_for, "On", device, (Py_ssize_t)need);
-    Py_DECREF(device);
-    if (*keep == nullptr) return false;
+    const int dev = x.get_device();
+    PyObject* seen = dev < kMaxDevices ? scratch_seen[dev] : nullptr;
+    if (seen != nullptr && (size_t)THPVariable_Unpack(seen).nbytes() >= need) {
+      Py_INCREF(seen);
+      *keep = seen;
+    } else {
+      PyObject* device = THPDevice_New(x.device());
+      if (device == nullptr) return false;
+      *keep = PyObject_CallFunction(scratch_for, "On", device, (Py_ssize_t)need);
+      Py_DECREF(device);
+      if (*keep == nullptr) return false;
+      if (dev < kMaxDevices && THPVariable_Check(*keep)) {
+        Py_INCREF(*keep);
+        Py_XSETREF(scratch_seen[dev], *keep);
+      }
+    }
     o = *keep;
   }
   const at::Tensor* t = tensor_of(o);
