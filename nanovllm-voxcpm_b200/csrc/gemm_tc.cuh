@@ -205,40 +205,46 @@ tc_tile_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a) {
   // The four roles walk the same stage sequence:
   //   for tile j: [nk base stages], then for run u, for slice s intersecting the tile: one LoRA stage
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&maps.x); tma_prefetch_desc(&maps.w); tma_prefetch_desc(&maps.t); tma_prefetch_desc(&maps.y);
-      const uint64_t w_policy = l2_policy_evict_last();
-      int st = 0, round = 0;
-      bool waited = false;
-      if (!a.after_shrink) { griddep_wait(); waited = true; }
-      for (int sg = 0; sg < nseg; ++sg) {
+    const uint32_t leader = elect_one();
+    if (leader) { tma_prefetch_desc(&maps.x); tma_prefetch_desc(&maps.w); tma_prefetch_desc(&maps.t); tma_prefetch_desc(&maps.y); }
+    const uint64_t w_policy = l2_policy_evict_last();
+    int st = 0, round = 0;
+    bool waited = false;
+    if (!a.after_shrink) { griddep_wait(); waited = true; }
+    for (int sg = 0; sg < nseg; ++sg) {
       int blk, ja, jb, nruns;
       seg_range(sg, blk, ja, jb, nruns);
+      ja = uniform(ja); jb = uniform(jb); nruns = uniform(nruns);
       for (int j = ja; j < jb; ++j) {
         for (int kc = 0; kc < nk; ++kc) {
           if (round > 0) mbar_wait_bounded(empty_bar(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
-          const uint32_t base = smem_base + (uint32_t)st * kGemmStageBytes;
-          mbar_arrive_expect_tx(full_bar(st), kGemmStageBytes);
-          tma_load_2d(base, &maps.x, kc * kSgmvBK, blk * kSgmvBM, full_bar(st));
-          tma_load_2d_hint(base + kSgmvBM * kSgmvBK * 2, &maps.w, kc * kSgmvBK, j * kSgmvBN, full_bar(st), w_policy);
+          if (leader) {
+            const uint32_t base = smem_base + (uint32_t)st * kGemmStageBytes, bar = full_bar(st);
+            mbar_arrive_expect_tx(bar, kGemmStageBytes);
+            tma_load_2d(base, &maps.x, kc * kSgmvBK, blk * kSgmvBM, bar);
+            tma_load_2d_hint(base + kSgmvBM * kSgmvBK * 2, &maps.w, kc * kSgmvBK, j * kSgmvBN, bar, w_policy);
+          }
+          __syncwarp();
           if (++st == kGemmStages) { st = 0; ++round; }
         }
         for (int u = 0; u < nruns; ++u) {
-          const int slot = run_slot[sg][u];
+          const int slot = uniform(run_slot[sg][u]);
           for (int s = 0; s < n; ++s) {
             const int lo = max(a.col[s], j * kSgmvBN), hi = min(a.col[s] + a.out[s], (j + 1) * kSgmvBN);
             if (lo >= hi) continue;
             if (round > 0) mbar_wait_bounded(empty_bar(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
             if (!waited) { griddep_wait(); waited = true; }  // tmp is final from here on
-            const uint32_t base = smem_base + (uint32_t)st * kGemmStageBytes;
-            mbar_arrive_expect_tx(full_bar(st), t_tile_bytes + b_tile_bytes);
-            tma_load_2d(base, &maps.t, 0, s * a.T + blk * kSgmvBM, full_bar(st));
-            tma_load_2d(base + t_tile_bytes, &maps.b[s], 0, slot * a.out[s] + (lo - a.col[s]), full_bar(st));
-            B200_TILE_TRACE(768 + min(j - ja, 63) + 64 * sg)
+            if (leader) {
+              const uint32_t base = smem_base + (uint32_t)st * kGemmStageBytes, bar = full_bar(st);
+              mbar_arrive_expect_tx(bar, t_tile_bytes + b_tile_bytes);
+              tma_load_2d(base, &maps.t, 0, s * a.T + blk * kSgmvBM, bar);
+              tma_load_2d(base + t_tile_bytes, &maps.b[s], 0, slot * a.out[s] + (lo - a.col[s]), bar);
+              B200_TILE_TRACE(768 + min(j - ja, 63) + 64 * sg)
+            }
+            __syncwarp();
             if (++st == kGemmStages) { st = 0; ++round; }
           }
         }
-      }
       }
     }
   } else if (warp == 6) {
@@ -284,13 +290,16 @@ tc_tile_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a) {
     }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_base = umma_idesc_bf16(kSgmvBM, kSgmvBN);
-      int st = 0, round = 0, job = 0;
-      uint32_t mphase = 0;  // bit st: parity of the next phase of masked_bar(st)
-      for (int sg = 0; sg < nseg; ++sg) {
+    const uint32_t leader = elect_one();
+    const uint64_t desc_x = umma_smem_desc(smem_base, 128), desc_t = umma_smem_desc(smem_base, row_bytes);
+    const uint32_t hi_x = (uint32_t)(desc_x >> 32), hi_t = (uint32_t)(desc_t >> 32), lo0 = (uint32_t)desc_x;
+    const uint32_t idesc_base = umma_idesc_bf16(kSgmvBM, kSgmvBN);
+    int st = 0, round = 0, job = 0;
+    uint32_t mphase = 0;  // bit st: parity of the next phase of masked_bar(st)
+    for (int sg = 0; sg < nseg; ++sg) {
       int blk, ja, jb, nruns;
       seg_range(sg, blk, ja, jb, nruns);
+      ja = uniform(ja); jb = uniform(jb); nruns = uniform(nruns);
       for (int j = ja; j < jb; ++j, ++job) {
         const int buf = job & 1;
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kSgmvBN);
@@ -300,13 +309,11 @@ tc_tile_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a) {
         for (int kc = 0; kc < nk; ++kc) {
           mbar_wait_bounded(full_bar(st), (uint32_t)(round & 1), &abort_flag);
           tc_fence_after_sync();
-          const uint32_t base = smem_base + (uint32_t)st * kGemmStageBytes;
-          const uint64_t xdesc = umma_smem_desc(base, 128);
-          const uint64_t wdesc = umma_smem_desc(base + kSgmvBM * kSgmvBK * 2, 128);
+          const uint32_t xl = lo0 + ((uint32_t)st * kGemmStageBytes >> 4), wl = xl + (kSgmvBM * kSgmvBK * 2 >> 4);
 #pragma unroll
           for (int k4 = 0; k4 < kSgmvBK / 16; ++k4)
-            umma_bf16(d_tmem, xdesc + 2u * k4, wdesc + 2u * k4, idesc_base, (kc > 0 || k4 > 0) ? 1u : 0u);
-          umma_commit(empty_bar(st));
+            umma_elected(d_tmem, xl + 2u * k4, wl + 2u * k4, hi_x, idesc_base, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
+          umma_commit_elected(empty_bar(st), leader);
           if (++st == kGemmStages) { st = 0; ++round; }
         }
         uint32_t started = 0;  // bit s: the D columns of slice s already hold a partial sum
@@ -318,22 +325,20 @@ tc_tile_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a) {
             B200_TILE_TRACE(512 + 4 * min(job, 31) + 1)
             mphase ^= 1u << st;
             tc_fence_after_sync();
-            const uint32_t base = smem_base + (uint32_t)st * kGemmStageBytes;
-            const uint64_t tdesc = umma_smem_desc(base, row_bytes);
-            const uint64_t bdesc = umma_smem_desc(base + t_tile_bytes, row_bytes);
+            const uint32_t tl = lo0 + ((uint32_t)st * kGemmStageBytes >> 4), bl = tl + (t_tile_bytes >> 4);
             const uint32_t idesc = umma_idesc_bf16(kSgmvBM, (hi - lo + 15) & ~15);
             const bool fresh = nk == 0 && ((started >> s) & 1u) == 0;
-            for (int k4 = 0; k4 < r / 16; ++k4)
-              umma_bf16(d_tmem + (uint32_t)(lo - j * kSgmvBN), tdesc + 2u * k4, bdesc + 2u * k4, idesc,
-                        (fresh && k4 == 0) ? 0u : 1u);
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4)
+              if (16 * k4 < r)
+                umma_elected(d_tmem + (uint32_t)(lo - j * kSgmvBN), tl + 2u * k4, bl + 2u * k4, hi_t, idesc, (fresh && k4 == 0) ? 0u : 1u, leader);
             started |= 1u << s;
-            umma_commit(empty_bar(st));
+            umma_commit_elected(empty_bar(st), leader);
             if (++st == kGemmStages) { st = 0; ++round; }
           }
         }
-        umma_commit(acc_full(buf));
+        umma_commit_elected(acc_full(buf), leader);
         B200_TILE_TRACE(512 + 4 * min(job, 31) + 2)
-      }
       }
     }
   } else if (warp >= 2 && warp <= 5) {

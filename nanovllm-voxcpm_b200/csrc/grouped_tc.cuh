@@ -73,33 +73,6 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&v)[16])
       : "r"(taddr));
 }
 
-// The MMA warps below run converged: every lane walks the loop and computes the (warp-uniform) descriptors, one lane
-// issues. With the loop inside `if (lane == 0)` the descriptors went through vector registers and an issue cost 110 cycles.
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t leader;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
-  return leader;
-}
-// D (+)= A . B^T where `leader`; descriptors as low words plus the shared high word
-__device__ __forceinline__ void umma_elected(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate,
-                                             uint32_t leader) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
-      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(leader)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit_elected(uint32_t bar, uint32_t leader) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(bar), "r"(leader)
-      : "memory");
-}
-__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
-
 // kind::f16 instruction descriptor for bf16 or fp16 operands (both of one type)
 __device__ __forceinline__ uint32_t umma_idesc_16bit(int M, int N, int f16) {
   const uint32_t t = f16 ? 0u : 1u;

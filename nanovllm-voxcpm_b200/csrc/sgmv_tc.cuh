@@ -170,52 +170,57 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
   const int npass = (nruns + G - 1) / G;
 
   if (warp == 0) {
-    if (lane == 0) {
+    const uint32_t leader = elect_one();
+    if (leader) {
       tma_prefetch_desc(&maps.xs);
       for (int s = 0; s < n; ++s) tma_prefetch_desc(&maps.a[s]);
-      int st = 0, round = 0;
-      for (int pi = 0; pi < npass; ++pi) {
-        const int u0 = pi * G, g = min(G, nruns - u0);
-        for (int kc = 0; kc < nk; ++kc) {
-          if (round > 0) mbar_wait_bounded(empty_bar(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
-          const uint32_t base = smem_base + (uint32_t)st * stage_bytes;
-          mbar_arrive_expect_tx(full_bar(st), x_load_bytes + (uint32_t)(g * n) * a_tile_bytes);
-          tma_load_2d(base, &maps.xs, kc * kSgmvBK, blk * kShrinkRows, full_bar(st));
-          for (int ui = 0; ui < g; ++ui) {
-            const int slot = run_slot[u0 + ui];
-            for (int s = 0; s < n; ++s)
-              tma_load_2d(base + x_tile_bytes + (uint32_t)(ui * n + s) * a_tile_bytes, &maps.a[s], kc * kSgmvBK, slot * r,
-                          full_bar(st));
-          }
-          if (++st == NS) { st = 0; ++round; }
+    }
+    int st = 0, round = 0;
+    for (int pi = 0; pi < npass; ++pi) {
+      const int u0 = pi * G, g = min(G, nruns - u0);
+      int row[4];  // first lora_A row of each run of the pass (G <= 4)
+#pragma unroll
+      for (int ui = 0; ui < 4; ++ui) row[ui] = uniform(ui < g ? run_slot[u0 + ui] * r : 0);
+      for (int kc = 0; kc < nk; ++kc) {
+        if (round > 0) mbar_wait_bounded(empty_bar(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
+        if (leader) {
+          const uint32_t base = smem_base + (uint32_t)st * stage_bytes, bar = full_bar(st);
+          mbar_arrive_expect_tx(bar, x_load_bytes + (uint32_t)(g * n) * a_tile_bytes);
+          tma_load_2d(base, &maps.xs, kc * kSgmvBK, blk * kShrinkRows, bar);
+          uint32_t dst = base + x_tile_bytes;
+#pragma unroll
+          for (int ui = 0; ui < 4; ++ui)
+            if (ui < g)
+              for (int s = 0; s < n; ++s, dst += a_tile_bytes) tma_load_2d(dst, &maps.a[s], kc * kSgmvBK, row[ui], bar);
         }
+        __syncwarp();
+        if (++st == NS) { st = 0; ++round; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16(kSgmvBM, r);
-      int st = 0, round = 0;
-      for (int pi = 0; pi < npass; ++pi) {
-        const int g = min(G, nruns - pi * G);
-        if (pi > 0) mbar_wait_bounded(acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
+    const uint32_t leader = elect_one();
+    const uint64_t desc0 = umma_smem_desc(smem_base, 128);
+    const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
+    const uint32_t idesc = umma_idesc_bf16(kSgmvBM, r);
+    int st = 0, round = 0;
+    for (int pi = 0; pi < npass; ++pi) {
+      const int jobs = uniform(min(G, nruns - pi * G)) * n;
+      if (pi > 0) mbar_wait_bounded(acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
+      tc_fence_after_sync();
+      for (int kc = 0; kc < nk; ++kc) {
+        mbar_wait_bounded(full_bar(st), (uint32_t)(round & 1), &abort_flag);
+        B200_SHRINK_TRACE_K(kc)
         tc_fence_after_sync();
-        for (int kc = 0; kc < nk; ++kc) {
-          mbar_wait_bounded(full_bar(st), (uint32_t)(round & 1), &abort_flag);
-          B200_SHRINK_TRACE_K(kc)
-          tc_fence_after_sync();
-          const uint32_t base = smem_base + (uint32_t)st * stage_bytes;
-          const uint64_t xdesc = umma_smem_desc(base, 128);
-          for (int q = 0; q < g * n; ++q) {  // q = run in pass * n + slice
-            const uint64_t adesc = umma_smem_desc(base + x_tile_bytes + (uint32_t)q * a_tile_bytes, 128);
+        const uint32_t xl = lo0 + ((uint32_t)st * stage_bytes >> 4);
+        uint32_t al = xl + (x_tile_bytes >> 4), d = tmem_base;
+        for (int q = 0; q < jobs; ++q, al += a_tile_bytes >> 4, d += (uint32_t)r) {  // q = run in pass * n + slice
 #pragma unroll
-            for (int k4 = 0; k4 < kSgmvBK / 16; ++k4)
-              umma_bf16(tmem_base + (uint32_t)(q * r), xdesc + 2u * k4, adesc + 2u * k4, idesc, (kc > 0 || k4 > 0) ? 1u : 0u);
-          }
-          umma_commit(empty_bar(st));  // stage reusable once these MMAs have read it
-          if (++st == NS) { st = 0; ++round; }
+          for (int k4 = 0; k4 < kSgmvBK / 16; ++k4) umma_elected(d, xl + 2u * k4, al + 2u * k4, hi, idesc, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
         }
-        umma_commit(acc_full);
+        umma_commit_elected(empty_bar(st), leader);  // stage reusable once these MMAs have read it
+        if (++st == NS) { st = 0; ++round; }
       }
+      umma_commit_elected(acc_full, leader);
     }
   } else if ((warp & 3) < kShrinkRows / 32) {
     // epilogue: thread <-> row; a warp may only touch its own quarter of the 128 TMEM lanes (the warps of the
