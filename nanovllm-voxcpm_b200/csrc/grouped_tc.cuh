@@ -64,15 +64,6 @@ struct GroupedMaps {
   CUtensorMap w[B200_LORA_MAX_SLICES]; // shrink: lora_A [S*r, in], box r x 64; expand: lora_B [S*out, r], box 128 x r
 };
 
-// 32 lanes x 16 consecutive fp32 columns
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
-}
-
 // kind::f16 instruction descriptor for bf16 or fp16 operands (both of one type)
 __device__ __forceinline__ uint32_t umma_idesc_16bit(int M, int N, int f16) {
   const uint32_t t = f16 ? 0u : 1u;

@@ -145,6 +145,11 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t local_addr, uint32_t ct
 __device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+  return v;
+}
 // 8-byte store into the shared memory of a CTA of the cluster that also counts its bytes on
 // an mbarrier of that CTA (both addresses from mapa_shared): data and signal in one operation.
 __device__ __forceinline__ void st_async_b32x2(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t cluster_bar) {

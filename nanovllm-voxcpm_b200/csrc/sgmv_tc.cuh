@@ -20,7 +20,6 @@ namespace b200lora {
 
 constexpr int kSgmvThreads = 192;   // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-5: epilogue
 constexpr int kSgmvBM = 128;        // rows per block / MMA M
-constexpr int kShrinkRows = 64;     // rows of x one shrink CTA owns (the upper half of its M = 128 tiles is idle)
 constexpr int kSgmvBK = 64;         // K columns per shrink stage (one 128-byte swizzle row)
 constexpr int kSgmvBN = 256;        // output columns per expand tile
 constexpr int kSgmvShrinkMaxStages = 12; // the launch picks as many 64-column stages as fit into shared memory
@@ -38,24 +37,24 @@ struct SgmvArgs {
   int skip_clean;                           // expand: leave blocks in which every row has an adapter to tc_tile_kernel
   int shrink_gmax;                          // shrink: runs of a block whose K loops share one pass over x (set by the launch)
   int shrink_ring_bytes;                    // shrink: bytes of the TMA ring (set by the launch)
+  int shrink_ck;                            // shrink: CTAs of a cluster = parts of K (set by the launch)
 };
 
 struct SgmvMaps {
   CUtensorMap x;                            // [T, in]            box 128 x 64
-  CUtensorMap xs;                           // [T, in]            box  64 x 64 (shrink)
   CUtensorMap a[B200_LORA_MAX_SLICES];      // [S*r_max, in]      box r_max x 64
   CUtensorMap t;                            // [n*T, r_max]       box 128 x r_max
   CUtensorMap b[B200_LORA_MAX_SLICES];      // [S*out_s, r_max]   box 256 x r_max
 };
 
-// Runs of equal slot inside block `blk`, written to shared memory by thread 0.
-// (table element types are the caller's: slot ids fit int16 for S <= 32767, row bounds 0..128 fit uint8)
-template <typename TS, typename TR, int ROWS = kSgmvBM>
+// Runs of equal slot inside the 128-row block `blk`, found by the CTA's first four warps (a scan of the block by one thread
+// took 2 us per block). (table element types are the caller's: slot ids fit int16 for S <= 32767, row bounds 0..128 fit uint8)
+template <typename TS, typename TR>
 __device__ __forceinline__ void sgmv_find_runs(const int32_t* tts, int T, int S, int blk, TS* s_slot, TS* run_slot,
                                                TR* run_lo, TR* run_hi, int* nruns) {
-  const int row0 = blk * ROWS;
-  for (int i = threadIdx.x; i < ROWS; i += blockDim.x) {
-    const int row = row0 + i;
+  __shared__ int warp_starts[4];
+  const int i = threadIdx.x, row = blk * kSgmvBM + i;
+  if (i < kSgmvBM) {
     int sl = -1;
     if (row < T) sl = tts[row];
     (void)B200_IN_BOUNDS(sl >= -1 && sl < S);  // ids outside [-1, S) are treated as "no adapter"; the checked build reports them
@@ -63,18 +62,23 @@ __device__ __forceinline__ void sgmv_find_runs(const int32_t* tts, int T, int S,
     s_slot[i] = (TS)sl;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int n = 0, i = 0;
-    while (i < ROWS) {
-      const int sl = s_slot[i];
-      if (sl < 0) { ++i; continue; }
-      int j = i + 1;
-      while (j < ROWS && s_slot[j] == sl) ++j;
-      run_slot[n] = (TS)sl; run_lo[n] = (TR)i; run_hi[n] = (TR)j; ++n;
-      i = j;
-    }
-    *nruns = n;
+  bool starts = false, ends = false;
+  unsigned before = 0;
+  if (i < kSgmvBM) {
+    const int sl = s_slot[i];
+    starts = sl >= 0 && (i == 0 || s_slot[i - 1] != sl);
+    ends = sl >= 0 && (i == kSgmvBM - 1 || s_slot[i + 1] != sl);
+    const unsigned mask = __ballot_sync(0xffffffffu, starts);
+    before = __popc(mask & ((2u << (i & 31)) - 1u));  // runs of this warp that start at or before this row
+    if ((i & 31) == 0) warp_starts[i >> 5] = __popc(mask);
   }
+  __syncthreads();
+  if (i < kSgmvBM) {
+    for (int w = 0; w < i >> 5; ++w) before += (unsigned)warp_starts[w];
+    if (starts) { run_slot[before - 1] = s_slot[i]; run_lo[before - 1] = (TR)i; }
+    if (ends) run_hi[before - 1] = (TR)(i + 1);
+  }
+  if (i == 0) *nruns = warp_starts[0] + warp_starts[1] + warp_starts[2] + warp_starts[3];
   __syncthreads();
 }
 
@@ -110,39 +114,40 @@ __device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const uint32_t
 #endif
 
 // ============================================================================ shrink
+// One cluster per 128-row block. Its CTAs split K: a CTA's K loop is a chain of latencies (0.5 us per 64 columns, 31 us for
+// 1000 rows of 2048-wide layers on 16 CTAs), so the loop is made short and the GPU filled; the partial sums meet in
+// distributed shared memory. The lora_A tiles of a run's slices lie side by side and are one MMA operand of n * r columns.
 __global__ void __launch_bounds__(kSgmvThreads, 1)
 sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ int s_slot[kSgmvBM], run_slot[kSgmvBM], run_lo[kSgmvBM], run_hi[kSgmvBM];
   __shared__ int nruns_s;
-  __shared__ __align__(8) uint64_t bars[2 * kSgmvShrinkMaxStages + 2];
+  __shared__ __align__(8) uint64_t bars[2 * kSgmvShrinkMaxStages + 4];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int blk = blockIdx.x;
-  const int r = a.r_max, n = a.n;
+  const int CK = a.shrink_ck, ck = CK > 1 ? (int)cluster_ctarank() : 0;
+  const int blk = (int)blockIdx.x / CK;
+  const int r = a.r_max, n = a.n, width = n * r;
   B200_SHRINK_TRACE_CTA(0)
-  // A CTA owns kShrinkRows = 64 rows of x: twice as many CTAs as 128-row blocks, so that most SMs of the GPU
-  // stream x (a CTA's rate is bound by the bytes its ring keeps in flight). The MMAs stay M = 128: the x slot of a
-  // stage has room for 128 rows, TMA fills the lower 64, the upper 64 hold stale bytes whose accumulator rows
-  // (TMEM lanes 64..127) are never read.
   const uint32_t a_tile_bytes = (uint32_t)r * kSgmvBK * 2;
   const uint32_t x_tile_bytes = kSgmvBM * kSgmvBK * 2;
-  const uint32_t x_load_bytes = kShrinkRows * kSgmvBK * 2;
   const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;  // swizzled tiles need 1024-byte alignment
   const uint32_t bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * (uint32_t)s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (uint32_t)(kSgmvShrinkMaxStages + s); };
   const uint32_t acc_full = bar0 + 8u * (2 * kSgmvShrinkMaxStages);
-  const uint32_t acc_empty = acc_full + 8u;
+  const uint32_t acc_empty = acc_full + 8u, part_ready = acc_full + 16u, part_done = acc_full + 24u;
   int tmem_cols = 32;  // the last slice is read in 32-column chunks
   while (tmem_cols < (a.shrink_gmax * n - 1) * r + ((r + 31) & ~31)) tmem_cols *= 2;
 
   if (tid == 0) {
     for (int s = 0; s < kSgmvShrinkMaxStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     mbar_init(acc_full, 1);
-    mbar_init(acc_empty, kShrinkRows);
+    mbar_init(acc_empty, kSgmvBM);
+    mbar_init(part_ready, (uint32_t)CK);  // every CTA of the cluster has written / read the partial sums of an exchange
+    mbar_init(part_done, (uint32_t)CK);
     abort_flag = 0;
     mbar_fence_init();
   }
@@ -150,7 +155,8 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
     tmem_alloc(smem_u32(&tmem_base_s), (uint32_t)tmem_cols);
     tc_fence_before_sync();
   }
-  sgmv_find_runs<int, int, kShrinkRows>(a.token_to_slot, a.T, a.S, blk, s_slot, run_slot, run_lo, run_hi, &nruns_s);  // has __syncthreads
+  sgmv_find_runs(a.token_to_slot, a.T, a.S, blk, s_slot, run_slot, run_lo, run_hi, &nruns_s);  // has __syncthreads
+  if (CK > 1) { cluster_arrive(); cluster_wait(); }  // the barriers of every CTA of the cluster are initialised
   // Launched under programmatic dependent launch: everything above (barriers, TMEM, the run table from the index
   // metadata) may overlap the previous kernel of the stream; x is read and tmp written only from here on.
   griddep_wait();
@@ -160,10 +166,11 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
   const int nruns = nruns_s;
-  const int nk = a.in_dim / kSgmvBK;
+  const int nk_all = a.in_dim / kSgmvBK, nk_per = (nk_all + CK - 1) / CK;
+  const int kc0 = min(ck * nk_per, nk_all), nk = min(nk_per, nk_all - kc0);  // this CTA's K steps (at least one: see the launch)
   // The runs of a block (two at a request boundary) share ONE pass over x: every K step loads the x tile once
   // and one lora_A tile per run and slice, and the MMAs of run i accumulate into their own TMEM columns
-  // [(i * n + s) * r, +r). Up to G runs per pass; the ring depth follows from the stage size of this block.
+  // [i * n * r, +n * r). Up to G runs per pass; the ring depth follows from the stage size of this block.
   const int G = min(a.shrink_gmax, max(nruns, 1));
   const uint32_t stage_bytes = x_tile_bytes + (uint32_t)(G * n) * a_tile_bytes;
   const int NS = min(kSgmvShrinkMaxStages, (int)((uint32_t)a.shrink_ring_bytes / stage_bytes));
@@ -172,11 +179,13 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
   if (warp == 0) {
     const uint32_t leader = elect_one();
     if (leader) {
-      tma_prefetch_desc(&maps.xs);
+      tma_prefetch_desc(&maps.x);
       for (int s = 0; s < n; ++s) tma_prefetch_desc(&maps.a[s]);
     }
     int st = 0, round = 0;
     for (int pi = 0; pi < npass; ++pi) {
+      // the partial sums of a pass lie where the ring is
+      if (CK > 1 && pi > 0) mbar_wait_bounded(acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
       const int u0 = pi * G, g = min(G, nruns - u0);
       int row[4];  // first lora_A row of each run of the pass (G <= 4)
 #pragma unroll
@@ -185,13 +194,13 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
         if (round > 0) mbar_wait_bounded(empty_bar(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
         if (leader) {
           const uint32_t base = smem_base + (uint32_t)st * stage_bytes, bar = full_bar(st);
-          mbar_arrive_expect_tx(bar, x_load_bytes + (uint32_t)(g * n) * a_tile_bytes);
-          tma_load_2d(base, &maps.xs, kc * kSgmvBK, blk * kShrinkRows, bar);
+          mbar_arrive_expect_tx(bar, x_tile_bytes + (uint32_t)(g * n) * a_tile_bytes);
+          tma_load_2d(base, &maps.x, (kc0 + kc) * kSgmvBK, blk * kSgmvBM, bar);
           uint32_t dst = base + x_tile_bytes;
 #pragma unroll
           for (int ui = 0; ui < 4; ++ui)
             if (ui < g)
-              for (int s = 0; s < n; ++s, dst += a_tile_bytes) tma_load_2d(dst, &maps.a[s], kc * kSgmvBK, row[ui], bar);
+              for (int s = 0; s < n; ++s, dst += a_tile_bytes) tma_load_2d(dst, &maps.a[s], (kc0 + kc) * kSgmvBK, row[ui], bar);
         }
         __syncwarp();
         if (++st == NS) { st = 0; ++round; }
@@ -201,10 +210,10 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
     const uint32_t leader = elect_one();
     const uint64_t desc0 = umma_smem_desc(smem_base, 128);
     const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
-    const uint32_t idesc = umma_idesc_bf16(kSgmvBM, r);
+    const uint32_t idesc = umma_idesc_bf16(kSgmvBM, width);
     int st = 0, round = 0;
     for (int pi = 0; pi < npass; ++pi) {
-      const int jobs = uniform(min(G, nruns - pi * G)) * n;
+      const int jobs = uniform(min(G, nruns - pi * G));
       if (pi > 0) mbar_wait_bounded(acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
       tc_fence_after_sync();
       for (int kc = 0; kc < nk; ++kc) {
@@ -213,7 +222,7 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
         tc_fence_after_sync();
         const uint32_t xl = lo0 + ((uint32_t)st * stage_bytes >> 4);
         uint32_t al = xl + (x_tile_bytes >> 4), d = tmem_base;
-        for (int q = 0; q < jobs; ++q, al += a_tile_bytes >> 4, d += (uint32_t)r) {  // q = run in pass * n + slice
+        for (int q = 0; q < jobs; ++q, al += (uint32_t)n * a_tile_bytes >> 4, d += (uint32_t)width) {  // runs of the pass
 #pragma unroll
           for (int k4 = 0; k4 < kSgmvBK / 16; ++k4) umma_elected(d, xl + 2u * k4, al + 2u * k4, hi, idesc, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
         }
@@ -222,18 +231,17 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
       }
       umma_commit_elected(acc_full, leader);
     }
-  } else if ((warp & 3) < kShrinkRows / 32) {
-    // epilogue: thread <-> row; a warp may only touch its own quarter of the 128 TMEM lanes (the warps of the
-    // idle upper half have nothing to do)
-    const int quarter = warp & 3;
-    const int row_in_blk = quarter * 32 + lane;
-    const int row = blk * kShrinkRows + row_in_blk;
-    if (a.zero_fill && row < a.T && s_slot[row_in_blk] < 0) {
+  } else {
+    // epilogue: thread <-> row; a warp may only touch its own quarter of the 128 TMEM lanes
+    const int quarter = warp & 3, row_in_blk = quarter * 32 + lane, etid = tid - 64;
+    const int row = blk * kSgmvBM + row_in_blk;
+    if (a.zero_fill && ck == 0 && row < a.T && s_slot[row_in_blk] < 0) {
       for (int s = 0; s < n; ++s) {
         __nv_bfloat16* dst = a.tmp + ((int64_t)s * a.T + row) * r;
         for (int c = 0; c < r; c += 8) stg128(dst + c, make_uint4(0, 0, 0, 0));
       }
     }
+    int exchange = 0;
     for (int pi = 0; pi < npass; ++pi) {
       const int u0 = pi * G, g = min(G, nruns - u0);
       mbar_wait_bounded(acc_full, (uint32_t)(pi & 1), &abort_flag);
@@ -243,19 +251,85 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
         // (a TMEM load is a warp-wide operation on one column range: a warp whose 32 rows straddle two runs
         //  reads both runs' columns and every lane keeps the ones of its own run)
         const int lo_row = run_lo[u], hi_row = run_hi[u];
-        if (hi_row <= quarter * 32 || lo_row >= quarter * 32 + 32) continue;  // warp-uniform: no row of this warp
-        const bool mine = row_in_blk >= lo_row && row_in_blk < hi_row && row < a.T;
+        const bool touched = hi_row > quarter * 32 && lo_row < quarter * 32 + 32;  // warp-uniform
         const int slot = run_slot[u];
         const float sc = a.scaling * (a.scale_per_slot != nullptr ? a.scale_per_slot[slot] : 1.0f);
-        for (int s = 0; s < n; ++s) {
-          for (int c = 0; c < r; c += 32) {
-            uint32_t v[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((ui * n + s) * r + c), v);
+        if (CK == 1) {
+          if (!touched) continue;
+          const bool mine = row_in_blk >= lo_row && row_in_blk < hi_row && row < a.T;
+          for (int s = 0; s < n; ++s) {
+            for (int c = 0; c < r; c += 32) {
+              uint32_t v[32];
+              tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((ui * n + s) * r + c), v);
+              tmem_ld_wait();
+              if (mine) store_bf16x32(a.tmp + ((int64_t)s * a.T + row) * r + c, v, sc, min(32, r - c));
+            }
+          }
+          continue;
+        }
+        // this CTA's partial sums into its own shared memory, as [4 columns][row] pieces of 16 bytes: the lanes of a remote read
+        // then cover consecutive bytes (row-major sums, 16 bytes a lane at a pitch, came at 8 bytes per clock) ...
+        if (exchange > 0) mbar_wait_bounded_acquire_cluster(part_done, (uint32_t)((exchange - 1) & 1), &abort_flag);
+        if (touched) {
+          for (int c = 0; c < width; c += 16) {
+            uint32_t v[16];
+            tmem_ld_32x16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ui * width + c), v);
             tmem_ld_wait();
-            if (mine) store_bf16x32(a.tmp + ((int64_t)s * a.T + row) * r + c, v, sc, min(32, r - c));
+            const uint32_t dst = smem_base + (uint32_t)((c >> 2) * kSgmvBM + row_in_blk) * 16u;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sts128(dst + 16u * kSgmvBM * q, make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
           }
         }
+        named_bar_sync(2, kSgmvBM);
+        if (etid < CK) mbar_arrive_remote_release(mapa_shared(part_ready, (uint32_t)etid));
+        mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)(exchange & 1), &abort_flag);
+        // ... then every CTA adds its share of (8 columns x row) pieces over the cluster
+        const int pieces = (width >> 3) * kSgmvBM, per = (pieces + CK - 1) / CK;
+        const int first = ck * per + etid, last = min((ck + 1) * per, pieces);
+        auto add_pieces = [&](auto parts) {
+          // eight remote reads of 32 bytes in flight per thread: one at a time each costs a round trip of 500 cycles
+          constexpr int kParts = decltype(parts)::value, kBatch = 8 / kParts;
+          for (int e0 = first; e0 < last; e0 += kBatch * kSgmvBM) {
+            float4 v[8][2];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const int e = e0 + (q / kParts) * kSgmvBM, er = e & (kSgmvBM - 1);
+              v[q][0] = v[q][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (e < last && er >= lo_row && er < hi_row) {
+                const uint32_t src = mapa_shared(smem_base + (uint32_t)(2 * (e >> 7) * kSgmvBM + er) * 16u, (uint32_t)(q % kParts));
+                v[q][0] = ld_cluster_f32x4(src);
+                v[q][1] = ld_cluster_f32x4(src + 16u * kSgmvBM);
+              }
+            }
+#pragma unroll
+            for (int h = 0; h < kBatch; ++h) {
+              const int e = e0 + h * kSgmvBM, er = e & (kSgmvBM - 1), grow = blk * kSgmvBM + er;
+              if (e >= last || er < lo_row || er >= hi_row || grow >= a.T) continue;
+              float4 s0 = v[h * kParts][0], s1 = v[h * kParts][1];
+#pragma unroll
+              for (int q = 1; q < kParts; ++q) {
+                const float4 w0 = v[h * kParts + q][0], w1 = v[h * kParts + q][1];
+                s0.x += w0.x; s0.y += w0.y; s0.z += w0.z; s0.w += w0.w;
+                s1.x += w1.x; s1.y += w1.y; s1.z += w1.z; s1.w += w1.w;
+              }
+              const int col = 8 * (e >> 7), s = col / r, c = col - s * r;
+              stg128(a.tmp + ((int64_t)s * a.T + grow) * r + c,
+                     make_uint4(pack_bf16x2(s0.x * sc, s0.y * sc), pack_bf16x2(s0.z * sc, s0.w * sc), pack_bf16x2(s1.x * sc, s1.y * sc),
+                                pack_bf16x2(s1.z * sc, s1.w * sc)));
+            }
+          }
+        };
+        if (CK == 8) add_pieces(std::integral_constant<int, 8>{});
+        else if (CK == 4) add_pieces(std::integral_constant<int, 4>{});
+        else add_pieces(std::integral_constant<int, 2>{});
+        if (++exchange < nruns) {  // (after the last one the cluster barrier at the end keeps the sums in place)
+          named_bar_sync(2, kSgmvBM);
+          if (etid < CK) mbar_arrive_remote_release(mapa_shared(part_done, (uint32_t)etid));
+        }
       }
+      // (the partial sums lie where the ring is: no refill before every CTA has read them)
+      if (CK > 1 && pi + 1 < npass) mbar_wait_bounded_acquire_cluster(part_done, (uint32_t)((exchange - 1) & 1), &abort_flag);
+      if (CK > 1) fence_proxy_async_smem();
       tc_fence_before_sync();
       mbar_arrive(acc_empty);
     }
@@ -264,6 +338,7 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
   B200_SHRINK_TRACE_CTA(1)
   if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)tmem_cols);
   if (tid == 0 && abort_flag != 0) atomicOr(&g_b200_status, kStatusWaitGaveUp);
+  if (CK > 1) { cluster_arrive(); cluster_wait(); }  // the peers have read this CTA's partial sums
 }
 
 // ============================================================================ expand
@@ -466,9 +541,8 @@ inline int sgmv_prepare_tmp(const SgmvProblem& b, void* tmp, uint64_t tmp_rows, 
   if (int rc = make_tmap_2d(&maps->t, a.tmp, tmp_rows, (uint64_t)b.r_max, (uint64_t)b.r_max, kSgmvBM, (uint32_t)b.r_max)) return rc;
   if (with_x) {
     if (int rc = make_tmap_2d(&maps->x, b.x, (uint64_t)b.T, (uint64_t)b.in_dim, (uint64_t)b.x_ld, kSgmvBM, kSgmvBK)) return rc;
-    if (int rc = make_tmap_2d(&maps->xs, b.x, (uint64_t)b.T, (uint64_t)b.in_dim, (uint64_t)b.x_ld, kShrinkRows, kSgmvBK)) return rc;
   } else {
-    maps->x = maps->xs = maps->t;  // never dereferenced by the expand half
+    maps->x = maps->t;  // never dereferenced by the expand half
   }
   for (int s = 0; s < a.n; ++s) {
     if (with_x) {
@@ -506,9 +580,9 @@ inline int sgmv_set_smem(const void* kernel, size_t bytes) {
 
 inline int sgmv_launch_shrink(const SgmvMaps& maps, const SgmvArgs& a_in, cudaStream_t stream) {
   SgmvArgs a = a_in;
-  // One CTA per SM streams its 128 rows of x through a ring that fills the shared memory of the SM: the more
-  // bytes in flight, the better. Up to 4 runs of a block share a pass, as long as their accumulators fit into
-  // the 512 TMEM columns and three stages of that size fit into the ring.
+  // A CTA streams its 128 rows of x through a ring that fills the shared memory of the SM: the more bytes in flight, the
+  // better. Up to 4 runs of a block share a pass, as long as their accumulators fit into the 512 TMEM columns and three
+  // stages of that size fit into the ring.
   const size_t ring = 216 * 1024;
   const size_t x_tile = kSgmvBM * kSgmvBK * 2, a_tiles = (size_t)a.n * a.r_max * kSgmvBK * 2;
   int gmax = 1;
@@ -520,17 +594,23 @@ inline int sgmv_launch_shrink(const SgmvMaps& maps, const SgmvArgs& a_in, cudaSt
   a.shrink_ring_bytes = (int)ring;
   const size_t smem = ring + 1024;
   if (int rc = sgmv_set_smem(reinterpret_cast<const void*>(sgmv_shrink_kernel), smem)) return rc;
-  const int nblk = (a.T + kShrinkRows - 1) / kShrinkRows;
+  const int nblk = (a.T + kSgmvBM - 1) / kSgmvBM, nk = a.in_dim / kSgmvBK;
+  // K parts: as many as fill the SMs once, every part at least one K step
+  a.shrink_ck = 1;
+  while (a.shrink_ck < 8 && nblk * a.shrink_ck * 2 <= 148 && ((nk + 2 * a.shrink_ck - 1) / (2 * a.shrink_ck)) * (2 * a.shrink_ck - 1) < nk) a.shrink_ck *= 2;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)nblk, 1, 1);
+  cfg.gridDim = dim3((unsigned)(nblk * a.shrink_ck), 1, 1);
   cfg.blockDim = dim3(kSgmvThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)a.shrink_ck;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = bgmv_options().pdl ? 1 : 0;  // B200_LORA_OPT_PDL = 0: strict stream order (the waits in the kernel are then no-ops)
+  cfg.numAttrs = bgmv_options().pdl ? 2 : 1;  // B200_LORA_OPT_PDL = 0: strict stream order (the waits in the kernel are then no-ops)
   cudaError_t e = cudaLaunchKernelEx(&cfg, sgmv_shrink_kernel, maps, a);
   if (e != cudaSuccess) {
     cudaGetLastError();
