@@ -369,6 +369,41 @@ int lora_b200_device_status(int32_t* status, int32_t reset);
 int lora_b200_debug_trace(long long* out, int32_t n_values);
 #endif
 
+/*
+ * A decode step's layer chain for small batches (bf16, T <= 128): the result of a projection is left as fp32 planes
+ * [n, T, out] that its consumer adds up - the K parts of the base product and, last, the LoRA delta - so that base product
+ * and delta run side by side and no pass reads or rounds the sum in between. Counterpart in the reference: F.linear + add_lora
+ * of the layer forwards followed by layernorm / rotary embedding + attention / activation
+ * (nanovllm_voxcpm/layers/lora.py:341-366, models/voxcpm2/model.py:81-94,291-297, layers/attention.py:10-79).
+ *
+ * lora_b200_decode_planes: planes of an [in -> out] projection with adapters (one less without).
+ * lora_b200_decode_linear: fills them (n_slices = 0: base product only). The slices must cover the output.
+ * lora_b200_decode_add_rmsnorm: hidden_out = residual + sum, normed = rms_norm(hidden_out) * weight; hidden_out may be residual.
+ * lora_b200_decode_silu_mul: out = silu(gate) * up of planes [n, T, 2 * intermediate].
+ * lora_b200_decode_attention: q, k, v = sum of planes [n, T, (heads + 2 kv_heads) * head_dim]; rotates q and k, stores k and v at
+ *   slot_mapping (int64, < 0 = nowhere) and attends over the context_lens[t] first tokens of the request's block table, the
+ *   new one being the last of them. head_dim 64 or 128, at most 16 q heads per kv head. after_delta: the planes come from a
+ *   lora_b200_decode_linear with adapters directly before this call.
+ */
+int lora_b200_decode_planes(int32_t in_dim, int32_t out);
+int lora_b200_decode_linear(float* planes, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight,
+                            int64_t w_ld, int32_t out_total, int32_t n_slices, const void* const* a_slabs,
+                            const void* const* b_slabs, const int32_t* out_sizes, const int32_t* col_offsets, int32_t S,
+                            int32_t r_max, const int32_t* rank_per_slot, const int32_t* token_to_slot,
+                            const int32_t* sorted_idx, const int32_t* slot_ids, const int32_t* counts,
+                            const int32_t* offsets, int32_t n_buckets, void* stream);
+int lora_b200_decode_add_rmsnorm(void* normed, void* hidden_out, const float* planes, int32_t n_planes,
+                                 const void* residual, const void* weight, int32_t T, int32_t hidden, float eps,
+                                 void* stream);
+int lora_b200_decode_silu_mul(void* out, const float* planes, int32_t n_planes, int32_t T, int32_t intermediate,
+                              void* stream);
+int lora_b200_decode_attention(void* out, const float* planes, int32_t n_planes, int32_t T, int32_t num_heads,
+                               int32_t num_kv_heads, int32_t head_dim, const int64_t* positions, const void* cos_table,
+                               const void* sin_table, int32_t table_dim, int32_t table_dtype, int32_t max_position,
+                               void* k_cache, void* v_cache, const int32_t* block_tables, int32_t max_blocks,
+                               int32_t block_size, const int32_t* context_lens, const int64_t* slot_mapping, float scale,
+                               int32_t after_delta, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

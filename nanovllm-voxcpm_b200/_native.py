@@ -91,6 +91,22 @@ _SIGNATURES = {
                   c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_void_p],
     ),
     "lora_b200_glue_silu_mul": (c_int32, [c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32, c_int32, c_void_p]),
+    "lora_b200_decode_planes": (c_int32, [c_int32, c_int32]),
+    "lora_b200_decode_linear": (
+        c_int32,
+        [c_void_p, c_void_p, c_int64, c_int32, c_int32, c_void_p, c_int64, c_int32, c_int32, POINTER(c_void_p), POINTER(c_void_p),
+         POINTER(c_int32), POINTER(c_int32), c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32,
+         c_void_p],
+    ),
+    "lora_b200_decode_add_rmsnorm": (
+        c_int32, [c_void_p, c_void_p, c_void_p, c_int32, c_void_p, c_void_p, c_int32, c_int32, c_float, c_void_p],
+    ),
+    "lora_b200_decode_silu_mul": (c_int32, [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p]),
+    "lora_b200_decode_attention": (
+        c_int32,
+        [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
+         c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_float, c_int32, c_void_p],
+    ),
     "lora_b200_tp_allreduce": (
         c_int32, [c_void_p, c_void_p, c_int32, POINTER(c_void_p), c_int32, c_int32, c_int32, c_void_p],
     ),

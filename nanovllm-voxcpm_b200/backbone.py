@@ -23,11 +23,12 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import _native as N
 from . import glue as G
 from . import layers as L
 from . import lora as LORA
 from .batch_plan import GraphLoRABuffers, build_lora_batch_plan_from_token_to_slot, build_lora_context_from_batch_plan
-from .context import LoRAContext, build_mixed_lora_context, reset_lora_context, set_lora_context
+from .context import LM_LORA_DOMAIN, LoRAContext, build_mixed_lora_context, get_lora_context, reset_lora_context, set_lora_context
 
 
 @dataclass
@@ -184,8 +185,105 @@ class Decoder(nn.Module):
             normed, hidden = G.add_rms_norm(down, hidden, following, eps)
         return normed
 
+    def _decode_chain_ok(self, embeds, positions, step: AttentionStep) -> bool:
+        """Whether this step can run as the short decode chain (``csrc/decode_step.cuh``): a bf16 decode batch of at most 128
+        rows on one GPU, adapters (if any) on every output of every projection, and contexts short enough that one CTA
+        per request and kv head is the faster attention."""
+        cfg, T = self.cfg, embeds.size(0)
+        if step.is_prefill or not 1 <= T <= 128 or not embeds.is_cuda or embeds.dtype != torch.bfloat16 or not embeds.is_contiguous():
+            return False
+        if cfg.head_dim not in (64, 128) or cfg.num_heads % cfg.num_kv_heads or cfg.num_heads // cfg.num_kv_heads > 16:
+            return False
+        if cfg.hidden_size % 64 or cfg.hidden_size > 4096 or cfg.intermediate_size % 64 or (cfg.num_heads * cfg.head_dim) % 64:
+            return False
+        if step.block_tables.size(1) * cfg.kv_block_size > 4096 or not step.block_tables.is_contiguous():
+            return False
+        if step.context_lens.dtype != torch.int32 or step.block_tables.dtype != torch.int32 or step.slot_mapping.dtype != torch.int64 \
+                or positions.dtype != torch.int64:
+            return False
+        backend = LORA.get_backend()
+        if not isinstance(backend, LORA.B200LoRABackend) or backend.impl != N.IMPL_AUTO:
+            return False
+        ctx = get_lora_context()
+        with_lora = ctx.token_to_slot is not None and not ctx.no_lora_flag
+        if ctx.parts or (with_lora and (ctx.token_to_slot.numel() != T or ctx.token_indices_sorted_by_slot is None
+                                        or ctx.active_slot_ids is None or ctx.num_tokens_per_slot is None or ctx.slot_start_offsets is None)):
+            return False
+        for layer in self.layers:
+            for mod in (layer.self_attn.qkv_proj, layer.self_attn.o_proj, layer.mlp.gate_up_proj, layer.mlp.down_proj):
+                if mod.bias is not None or mod.tp_size != 1 or mod.weight.dtype != torch.bfloat16 or mod.lora_domain != LM_LORA_DOMAIN:
+                    return False
+                if with_lora and (not mod.supports_lora or mod.max_lora_rank % 16 or mod.max_lora_rank > 256
+                                  or sum(mod._active_slices()[2]) != mod.weight.size(0)):
+                    return False
+            if layer.self_attn.k_cache is None or layer.self_attn.k_cache.dtype != torch.bfloat16:
+                return False
+        return True
+
+    def _decode_chain(self, embeds, positions, step: AttentionStep):
+        """One decode step as nine dependent launches per layer whose projections leave their parts to the consumer."""
+        cfg, T, dev = self.cfg, embeds.size(0), embeds.device
+        heads, kv_heads, dim, inter, eps = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.intermediate_size, cfg.rms_norm_eps
+        lib, stream = N.lib(), N.current_stream(dev)
+        ctx = get_lora_context()
+        with_lora = ctx.token_to_slot is not None and not ctx.no_lora_flag
+        meta = self.layers[0].self_attn.qkv_proj._runtime_metadata() if with_lora else None
+        n_buckets = 0
+        if with_lora:
+            n_buckets = min(meta.active_slot_ids.numel(), meta.num_tokens_per_slot.numel(), meta.slot_start_offsets.numel() - 1)
+            if meta.num_active_loras > 0:
+                n_buckets = min(n_buckets, meta.num_active_loras)
+        shapes = [(m.weight.size(1), m.weight.size(0)) for m in (
+            self.layers[0].self_attn.qkv_proj, self.layers[0].self_attn.o_proj, self.layers[0].mlp.gate_up_proj, self.layers[0].mlp.down_proj)]
+        planes_of = {s: lib.lora_b200_decode_planes(*s) - (0 if with_lora else 1) for s in shapes}
+        planes = torch.empty(max(n * T * s[1] for s, n in planes_of.items()), dtype=torch.float32, device=dev)
+        attn = torch.empty(T, heads * dim, dtype=embeds.dtype, device=dev)
+        act = torch.empty(T, inter, dtype=embeds.dtype, device=dev)
+        hidden = torch.empty_like(embeds)
+        normed, _ = G.add_rms_norm(embeds, None, self.layers[0].input_layernorm, eps)
+        residual = embeds
+
+        def linear(mod, x) -> int:
+            w = mod.weight
+            if with_lora:
+                a, b, widths, cols = mod._active_slices()
+                S, r, _ = a[0].shape
+                lora = (len(a), N.ptr_array(a), N.ptr_array(b), N.int_array(widths), N.int_array(cols), S, r,
+                        mod._buffers["effective_lora_rank"].data_ptr(), meta.token_to_slot.data_ptr(),
+                        meta.token_indices_sorted_by_slot.data_ptr(), meta.active_slot_ids.data_ptr(),
+                        meta.num_tokens_per_slot.data_ptr(), meta.slot_start_offsets.data_ptr(), n_buckets)
+            else:
+                lora = (0, None, None, None, None, 0, 0, None, None, None, None, None, None, 0)
+            N.check(lib.lora_b200_decode_linear(planes.data_ptr(), x.data_ptr(), x.stride(0), T, w.size(1), w.data_ptr(), w.stride(0),
+                                                w.size(0), *lora, stream))
+            return planes_of[(w.size(1), w.size(0))]
+
+        def add_norm(n, weight):
+            nonlocal residual
+            N.check(lib.lora_b200_decode_add_rmsnorm(normed.data_ptr(), hidden.data_ptr(), planes.data_ptr(), n, residual.data_ptr(),
+                                                     weight.data_ptr(), T, cfg.hidden_size, eps, stream))
+            residual = hidden
+
+        with N.on_device(dev):
+            for i, layer in enumerate(self.layers):
+                sa = layer.self_attn
+                n = linear(sa.qkv_proj, normed)
+                N.check(lib.lora_b200_decode_attention(
+                    attn.data_ptr(), planes.data_ptr(), n, T, heads, kv_heads, dim, positions.data_ptr(), self.cos.data_ptr(),
+                    self.sin.data_ptr(), self.cos.size(1), N.dtype_code(self.cos.dtype), self.cos.size(0), sa.k_cache.data_ptr(),
+                    sa.v_cache.data_ptr(), step.block_tables.data_ptr(), step.block_tables.size(1), cfg.kv_block_size,
+                    step.context_lens.data_ptr(), step.slot_mapping.data_ptr(), dim ** -0.5, 1 if with_lora else 0, stream))
+                add_norm(linear(sa.o_proj, attn), layer.post_attention_layernorm)
+                n = linear(layer.mlp.gate_up_proj, normed)
+                N.check(lib.lora_b200_decode_silu_mul(act.data_ptr(), planes.data_ptr(), n, T, inter, stream))
+                following = self.layers[i + 1].input_layernorm if i + 1 < len(self.layers) else self.norm
+                add_norm(linear(layer.mlp.down_proj, act), following)
+        return normed
+
     def forward(self, embeds, positions, step: AttentionStep):
         if self.fused_glue:
+            if self._decode_chain_ok(embeds, positions, step):
+                return self._decode_chain(embeds, positions, step)
             return self._forward_fused(embeds, positions, step)
         cos_sin = (self.cos[positions].unsqueeze(1), self.sin[positions].unsqueeze(1))
         hidden = embeds

@@ -10,6 +10,7 @@
 #include "sgmv_tc.cuh"
 #include "gemm_tc.cuh"
 #include "grouped_tc.cuh"
+#include "decode_step.cuh"
 
 using namespace b200lora;
 
@@ -161,6 +162,93 @@ int lora_b200_glue_rope_kv_store(void* qkv, int64_t qkv_ld, int32_t T, int32_t n
 int lora_b200_glue_silu_mul(void* out, int64_t out_ld, const void* gate_up, int64_t gate_up_ld, int32_t T,
                             int32_t intermediate, int32_t dtype, void* stream) {
   return silu_mul_launch(out, out_ld, gate_up, gate_up_ld, T, intermediate, dtype, static_cast<cudaStream_t>(stream));
+}
+
+int lora_b200_decode_planes(int32_t in_dim, int32_t out) {
+  if (in_dim < 1 || out < 1) return 0;
+  return decode_gemm_parts(in_dim, out) + 1;
+}
+
+int lora_b200_decode_linear(float* planes, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight, int64_t w_ld,
+                            int32_t out_total, int32_t n_slices, const void* const* a_slabs, const void* const* b_slabs,
+                            const int32_t* out_sizes, const int32_t* col_offsets, int32_t S, int32_t r_max,
+                            const int32_t* rank_per_slot, const int32_t* token_to_slot, const int32_t* sorted_idx,
+                            const int32_t* slot_ids, const int32_t* counts, const int32_t* offsets, int32_t n_buckets,
+                            void* stream) {
+  if (T < 1 || T > kDecMaxRows || in_dim < 1 || out_total < 1) return fail(B200_LORA_EINVAL, "decode_linear: bad sizes T=%d in=%d out=%d", T, in_dim, out_total);
+  if (planes == nullptr || x == nullptr || weight == nullptr) return fail(B200_LORA_EINVAL, "decode_linear: null pointer");
+  if (in_dim % 64 != 0 || x_ld % 8 != 0 || w_ld % 8 != 0 || x_ld < in_dim || w_ld < in_dim || out_total % 8 != 0 || !aligned16(planes) || !aligned16(x) ||
+      !aligned16(weight))
+    return fail(B200_LORA_EUNSUPPORTED, "decode_linear: in_dim must be a multiple of 64, out of 8, rows 16-byte aligned");
+  cudaStream_t st_ = static_cast<cudaStream_t>(stream);
+  if (n_slices > 0) {
+    if (out_sizes == nullptr || col_offsets == nullptr || token_to_slot == nullptr) return fail(B200_LORA_EINVAL, "decode_linear: null slice or slot array");
+    BgmvProblem bp = {};
+    if (int rc = fill_slices(bp.st, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, true, true)) return rc;
+    int covered = 0;
+    for (int s = 0; s < bp.st.n; ++s) {
+      if (bp.st.col[s] + bp.st.out[s] > out_total) return fail(B200_LORA_EINVAL, "slice %d exceeds the output width", s);
+      covered += bp.st.out[s];
+    }
+    if (covered != out_total) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: the slices must cover the output");
+    bp.y = planes + (size_t)decode_gemm_parts(in_dim, out_total) * T * out_total; bp.y_ld = out_total;
+    bp.x = x; bp.x_ld = x_ld; bp.T = T; bp.in_dim = in_dim; bp.S = S; bp.r_max = r_max;
+    bp.rank_per_slot = rank_per_slot; bp.scale_per_slot = nullptr;
+    bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets; bp.n_buckets = n_buckets;
+    bp.scaling = 1.0f; bp.mode = 4; bp.kind = r_max % 32 != 0 ? 1 : 0; bp.token_to_slot = token_to_slot;
+    const char* why = nullptr;
+    if (sorted_idx == nullptr || slot_ids == nullptr || counts == nullptr || offsets == nullptr)
+      return fail(B200_LORA_EINVAL, "decode_linear: needs the bucket arrays");
+    if (!bgmv_supported(bp, &why)) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: %s", why);
+    if (int rc = bgmv_launch(bp, st_)) return rc;
+  }
+  float* delta = n_slices > 0 ? planes + (size_t)decode_gemm_parts(in_dim, out_total) * T * out_total : nullptr;
+  return decode_gemm_launch(planes, x, x_ld, T, in_dim, weight, w_ld, out_total, delta, token_to_slot, rank_per_slot, S, st_);
+}
+
+int lora_b200_decode_add_rmsnorm(void* normed, void* hidden_out, const float* planes, int32_t n_planes, const void* residual,
+                                 const void* weight, int32_t T, int32_t hidden, float eps, void* stream) {
+  if (T < 1 || hidden < 8 || hidden % 8 != 0 || hidden > 4096) return fail(B200_LORA_EUNSUPPORTED, "decode_add_rmsnorm: bad shape T=%d H=%d", T, hidden);
+  if (n_planes < 1 || n_planes > kDecMaxPlanes) return fail(B200_LORA_EINVAL, "decode_add_rmsnorm: %d planes", n_planes);
+  if (!normed || !hidden_out || !planes || !residual || !weight) return fail(B200_LORA_EINVAL, "decode_add_rmsnorm: null pointer");
+  if (!aligned16(normed) || !aligned16(hidden_out) || !aligned16(planes) || !aligned16(residual) || !aligned16(weight))
+    return fail(B200_LORA_EUNSUPPORTED, "decode_add_rmsnorm: rows must be 16-byte aligned");
+  using B = __nv_bfloat16;
+  return launch_dependent(decode_add_rmsnorm_kernel, "decode_add_rmsnorm_kernel", dim3((unsigned)T), round_up_i(hidden / 8, 32), 0,
+                          static_cast<cudaStream_t>(stream), static_cast<B*>(normed), static_cast<B*>(hidden_out), planes, n_planes,
+                          static_cast<const B*>(residual), static_cast<const B*>(weight), T, hidden, eps);
+}
+
+int lora_b200_decode_silu_mul(void* out, const float* planes, int32_t n_planes, int32_t T, int32_t intermediate, void* stream) {
+  if (T < 1 || intermediate < 8 || intermediate % 8 != 0) return fail(B200_LORA_EUNSUPPORTED, "decode_silu_mul: bad shape T=%d I=%d", T, intermediate);
+  if (n_planes < 1 || n_planes > kDecMaxPlanes) return fail(B200_LORA_EINVAL, "decode_silu_mul: %d planes", n_planes);
+  if (!out || !planes || !aligned16(out) || !aligned16(planes)) return fail(B200_LORA_EINVAL, "decode_silu_mul: null or misaligned pointer");
+  const int ctas = std::min(2 * 148, ceil_div_i(T * (intermediate / 8), 256));
+  return launch_dependent(decode_silu_mul_kernel, "decode_silu_mul_kernel", dim3((unsigned)ctas), 256, 0, static_cast<cudaStream_t>(stream),
+                          static_cast<__nv_bfloat16*>(out), planes, n_planes, T, intermediate);
+}
+
+int lora_b200_decode_attention(void* out, const float* planes, int32_t n_planes, int32_t T, int32_t num_heads, int32_t num_kv_heads,
+                               int32_t head_dim, const int64_t* positions, const void* cos_table, const void* sin_table,
+                               int32_t table_dim, int32_t table_dtype, int32_t max_position, void* k_cache, void* v_cache,
+                               const int32_t* block_tables, int32_t max_blocks, int32_t block_size, const int32_t* context_lens,
+                               const int64_t* slot_mapping, float scale, int32_t after_delta, void* stream) {
+  if (T < 1 || T > 65535 || num_kv_heads < 1 || num_heads % num_kv_heads != 0 || num_heads / num_kv_heads > 16 || (head_dim != 64 && head_dim != 128))
+    return fail(B200_LORA_EUNSUPPORTED, "decode_attention: T=%d heads=%d / %d of %d", T, num_heads, num_kv_heads, head_dim);
+  if (n_planes < 1 || n_planes > kDecMaxPlanes || max_blocks < 1 || block_size < 1 || max_position < 1)
+    return fail(B200_LORA_EINVAL, "decode_attention: bad sizes");
+  if ((table_dim != head_dim && table_dim != head_dim / 2) || !valid_dtype(table_dtype)) return fail(B200_LORA_EINVAL, "decode_attention: bad rotation table");
+  if (!out || !planes || !positions || !cos_table || !sin_table || !k_cache || !v_cache || !block_tables || !context_lens || !slot_mapping)
+    return fail(B200_LORA_EINVAL, "decode_attention: null pointer");
+  if (!aligned16(k_cache) || !aligned16(v_cache) || !aligned16(planes) || (reinterpret_cast<uintptr_t>(out) & 3u))
+    return fail(B200_LORA_EUNSUPPORTED, "decode_attention: caches must be 16-byte aligned");
+  DecAttnArgs a;
+  a.part = planes; a.planes = n_planes; a.ld = (num_heads + 2 * num_kv_heads) * head_dim; a.T = T; a.Hq = num_heads; a.Hk = num_kv_heads;
+  a.positions = positions; a.cos = cos_table; a.sin = sin_table; a.table_dim = table_dim; a.table_dtype = table_dtype; a.max_pos = max_position;
+  a.k_cache = static_cast<__nv_bfloat16*>(k_cache); a.v_cache = static_cast<__nv_bfloat16*>(v_cache);
+  a.block_tables = block_tables; a.max_blocks = max_blocks; a.block_size = block_size; a.context_lens = context_lens; a.slot_mapping = slot_mapping;
+  a.out = static_cast<__nv_bfloat16*>(out); a.scale = scale; a.early = after_delta;
+  return decode_attention_launch(a, head_dim, static_cast<cudaStream_t>(stream));
 }
 
 size_t lora_b200_tp_exchange_bytes(int32_t tp, int32_t capacity) { return tp_exchange_bytes(tp, capacity); }

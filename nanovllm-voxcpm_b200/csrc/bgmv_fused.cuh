@@ -77,6 +77,8 @@ struct BgmvProblem {
   // 3 = overwrite: y[t, cols] = delta for rows with an adapter and -0.0 for every other row (y is not
   // read); a base GEMM that then accumulates into y (beta = 1) gives base + delta, and x + (-0.0) == x
   // keeps rows without adapter bit-identical to the base result.
+  // 4 = y = delta in fp32 [T, y_ld], rows with an adapter only: one of the planes that decode_step.cuh adds up. Its
+  // successor in the stream may start when this launch has passed its own wait, and need not wait for what came before.
   int mode = 0;
   // Precision of the rank-r intermediate and of the update. 0 (bf16, r_max % 32 == 0): tmp rounded to bf16, the delta
   // rounded to bf16 and added at the L2. 1 (bf16) / 2 (fp16): tmp kept as the sum of two 16-bit numbers, y read, added to
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   const int C = 1 << p.c_shift;
   const int c = (int)cluster_ctarank();
   const int NS = p.NS;
-  constexpr bool kOverwrite = kMode == 3;
+  constexpr bool kF32Out = kMode == 4, kOverwrite = kMode == 3;
   constexpr bool kPrecise = kKind != 0, kF16 = kKind == 2;
   constexpr int mode = kMode;
 
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   // Let the next launch of the stream start at once: before its own griddepcontrol.wait it only
   // reads index metadata and lora slabs, which no kernel of this library writes, so its weight
   // traffic overlaps this kernel's compute and keeps HBM busy across launch boundaries.
-  if (p.use_pdl) griddep_launch_dependents();
+  if (p.use_pdl && !kF32Out) griddep_launch_dependents();
   // ---- bucket metadata (uniform across the cluster); barrier set-up overlaps the loads
   // Extra cluster e looks after multiple m = (e + 1) * window of the window inside the sorted rows: if m lies behind the
   // first row of a bucket [start, start + cnt), it is the i-th such multiple there, and the cluster takes the bucket's i-th
@@ -226,6 +228,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
     // of the stream: a launch that ended before its predecessor would let the launch behind it
     // pass its own wait too early.
     if (p.use_pdl && (kOverwrite || (kMode == 1 && p.zero_rows) || (blockIdx.y == 0 && c == 0))) griddep_wait();
+    if (p.use_pdl && kF32Out) griddep_launch_dependents();
     if (kMode == 1 && p.zero_rows) bgmv_zero_rows_without_adapter(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvThreads);
     if (kOverwrite)  // an idle cluster still does its share of the -0.0 rows
       bgmv_fill_rows_without_delta(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvThreads);
@@ -250,7 +253,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   // Shrink work of the cluster: either the rank rows are split over the CTAs (each takes all K parts of
   // its rows, the bf16 results are all-gathered), or - long input rows - the K parts are dealt over the
   // CTAs (each takes all rank rows of its K parts, the fp32 partial sums are exchanged and added).
-  const bool ksplit = (kMode == 0 || kMode == 3) && p.ksplit != 0;
+  const bool ksplit = (kMode == 0 || kMode >= 3) && p.ksplit != 0;
   const int Rc = ksplit ? Q : ((((Q + C - 1) >> p.c_shift) + 7) & ~7);  // rows owned per CTA
   const int q_lo = ksplit ? 0 : min(c * Rc, Q);
   const int rows_c = mode == 2 ? 0 : min(q_lo + Rc, Q) - q_lo;   // multiple of 8, may be 0 (expand only: no shrink rows)
@@ -277,7 +280,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   // bytes a pass delivers into this CTA: 16 token rows of all Q stacked rank rows, as bf16 once
   // (all-gather) or as fp32 from every CTA of the cluster (K split)
   const uint32_t gather_bytes = ksplit ? (uint32_t)(C * kBgmvTok * Q * 4) : (uint32_t)(kBgmvTok * Q * (kPrecise ? 4 : 2));
-  if (tid == 0 && (mode == 0 || mode == 3)) {
+  if (tid == 0 && (mode == 0 || mode >= 3)) {
     mbar_arrive_expect_tx(tmp_ready_bars, gather_bytes);                      // pass 0
     if (npass > 1) mbar_arrive_expect_tx(tmp_ready_bars + 8u, gather_bytes);  // pass 1
   }
@@ -449,6 +452,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   const uint32_t it_roff = (uint32_t)(it_tok * p.pitchR + it_q) * 4u;  // K split: the item inside one sender's block
 
   if (p.use_pdl) griddep_wait();  // x and y of this launch are final from here on
+  if (p.use_pdl && kF32Out) griddep_launch_dependents();
   if (kOverwrite) bgmv_fill_rows_without_delta(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvConsumers);
   if (kMode == 1 && p.zero_rows) bgmv_zero_rows_without_adapter(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvConsumers);
   B200_TRACE_POINT(4)
@@ -560,7 +564,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
     // ===== cross-warp reduction of the K slices, scale, bf16, all-gather =====
     // the barrier of pass + 1 is armed one pass ahead (passes 0 and 1 at start-up): every local wait on
     // its previous phase is over, and no peer sends for pass + 1 before it has this pass from this CTA
-    if (tid == 0 && pass >= 1 && pass + 1 < npass && (mode == 0 || mode == 3))
+    if (tid == 0 && pass >= 1 && pass + 1 < npass && (mode == 0 || mode >= 3))
       mbar_arrive_expect_tx(tmp_ready_bars + 8u * (uint32_t)((pass + 1) & 1), gather_bytes);
     named_bar_sync(1, kBgmvConsumers);
     if (pass == 0) {
@@ -674,7 +678,7 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
     // kinds 1 and 2: y of the next tile is requested while this one is multiplied (the first one here, behind the wait)
     uint4 y_next[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
     auto load_y = [&](int e) {
-      if (e >= tiles_exp || (kMode == 2 && p.no_add)) return;
+      if (e >= tiles_exp || kF32Out || (kMode == 2 && p.no_add)) return;
       const int2 te = etab[e];
       if (y_col >= (te.y & 0xffff) || !B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) return;
       if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + te.x);
@@ -710,6 +714,18 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
         for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.z, ahi.z, alo.w, ahi.w, w[j].z, w[j].w);
       }
       if (y_col < (te.y & 0xffff) && B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) {
+        if (kF32Out) {
+          float* const yf = reinterpret_cast<float*>(p.y) + te.x + y_col;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int tok = h ? tok_hi : tok_lo;
+            if (tok < 0) continue;
+            float4* const dst = reinterpret_cast<float4*>(yf + (int64_t)tok * p.y_ld);
+            dst[0] = make_float4(d[0][2 * h], d[0][2 * h + 1], d[1][2 * h], d[1][2 * h + 1]);
+            dst[1] = make_float4(d[2][2 * h], d[2][2 * h + 1], d[3][2 * h], d[3][2 * h + 1]);
+          }
+          return;
+        }
         if (kPrecise) {
           if (tok_lo >= 0)
             stg128(ylo_p + te.x, make_uint4(add_16x2<kF16>(y_lo.x, d[0][0], d[0][1]), add_16x2<kF16>(y_lo.y, d[1][0], d[1][1]),
@@ -810,6 +826,7 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
     return false;
   }
   if (b.kind != 0 && b.mode == 3) { *why = "overwrite mode is for bf16 with r_max a multiple of 32"; return false; }
+  if (b.kind == 2 && b.mode == 4) { *why = "the fp32 form is for bf16"; return false; }
   if (b.in_dim % 32 != 0) { *why = "in_dim must be a multiple of 32"; return false; }
   if (b.x_ld % 8 != 0 || b.y_ld % 8 != 0) { *why = "row strides must be multiples of 8 elements"; return false; }
   if (!aligned16(b.x) || !aligned16(b.y)) { *why = "x / y must be 16-byte aligned"; return false; }
@@ -848,7 +865,7 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   // K split: at least one K part (1024 columns) per CTA of the cluster and all rank rows in one CTA;
   // the shrink-only / expand-only pair of the tensor-parallel exchange keeps the row split
   const int nkp_all = ceil_div_i(b.in_dim, kBgmvKP);
-  const bool ksplit = bgmv_options().ksplit && C > 1 && (b.mode == 0 || b.mode == 3) && nkp_all >= C && Q <= kBgmvMaxRc &&
+  const bool ksplit = bgmv_options().ksplit && C > 1 && (b.mode == 0 || b.mode >= 3) && nkp_all >= C && Q <= kBgmvMaxRc &&
                       2 * C * kBgmvTok * (Q + 4) * 4 <= 40 * 1024;  // (received partial sums: more would cost the second CTA per SM)
   if (!ksplit)
     while (C < 8 && round_up_i(ceil_div_i(Q, C), 8) > kBgmvMaxRc) C *= 2;
@@ -936,7 +953,8 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
   (const void*)bgmv_fused_kernel<M, false, K, false>, (const void*)bgmv_fused_kernel<M, true, K, false>,                     \
       (const void*)bgmv_fused_kernel<M, false, K, true>, (const void*)bgmv_fused_kernel<M, true, K, true>
     const void* kernels[] = {B200_BGMV_ALL(0, 0), B200_BGMV_ALL(1, 0), B200_BGMV_ALL(2, 0), B200_BGMV_ALL(3, 0), B200_BGMV_ALL(0, 1), B200_BGMV_ALL(0, 2), B200_BGMV_ALL(1, 1),
-                             B200_BGMV_ALL(1, 2), B200_BGMV_ALL(2, 1), B200_BGMV_ALL(2, 2)};
+                             B200_BGMV_ALL(1, 2), B200_BGMV_ALL(2, 1), B200_BGMV_ALL(2, 2), B200_BGMV_ALL(4, 0),
+                             B200_BGMV_ALL(4, 1)};
 #undef B200_BGMV_ALL
     for (const void* k : kernels) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kBgmvSmemMax);
@@ -969,16 +987,18 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
                            : cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, false, K, false>, p)) \
                : (p.full_k ? cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, true, K, true>, p)    \
                            : cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, false, K, true>, p)))
-  switch (4 * p.kind + p.mode) {
+  switch (8 * p.kind + p.mode) {
     case 1: e = B200_BGMV_LAUNCH(1, 0); break;
     case 2: e = B200_BGMV_LAUNCH(2, 0); break;
     case 3: e = B200_BGMV_LAUNCH(3, 0); break;
-    case 4: e = B200_BGMV_LAUNCH(0, 1); break;
-    case 5: e = B200_BGMV_LAUNCH(1, 1); break;
-    case 6: e = B200_BGMV_LAUNCH(2, 1); break;
-    case 8: e = B200_BGMV_LAUNCH(0, 2); break;
-    case 9: e = B200_BGMV_LAUNCH(1, 2); break;
-    case 10: e = B200_BGMV_LAUNCH(2, 2); break;
+    case 4: e = B200_BGMV_LAUNCH(4, 0); break;
+    case 8: e = B200_BGMV_LAUNCH(0, 1); break;
+    case 9: e = B200_BGMV_LAUNCH(1, 1); break;
+    case 10: e = B200_BGMV_LAUNCH(2, 1); break;
+    case 12: e = B200_BGMV_LAUNCH(4, 1); break;
+    case 16: e = B200_BGMV_LAUNCH(0, 2); break;
+    case 17: e = B200_BGMV_LAUNCH(1, 2); break;
+    case 18: e = B200_BGMV_LAUNCH(2, 2); break;
     default: e = B200_BGMV_LAUNCH(0, 0); break;
   }
 #undef B200_BGMV_LAUNCH

@@ -1,0 +1,514 @@
+// Kernels of a decode step's layer chain for small batches (up to 128 rows): base GEMM, attention and the glue between them,
+// built so that the chain is short.
+//
+// A decode step of a small model is a chain of dependent launches, each bound by latency: with library GEMMs, the LoRA add
+// behind each of them, split-KV attention and separate glue kernels a layer of a 1024-wide decoder took 94 us (64 rows),
+// against 12 us of HBM time for its weights. Here
+//   * the base product and the LoRA delta of a projection run side by side: the fused decode kernel writes its delta (fp32)
+//     into one plane of a buffer [planes, T, out], decode_gemm_kernel its K parts into the others. The delta kernel lets its
+//     successor start once it has passed its own wait (everything before is complete then), so the GEMM needs no wait
+//     for x; it waits for the delta kernel before it ends, and what follows is ordered behind both;
+//   * the consumer of a projection (add + norm, RoPE + attention, SiLU * up) adds the planes in fp32: no rounding of the base
+//     output, no pass of its own;
+//   * RoPE, the cache store and attention are one kernel per (request, kv head).
+// All are launched as programmatic dependents; weights are requested before the wait.
+#pragma once
+
+#include "bgmv_fused.cuh"
+#include "glue.cuh"
+#include "tc_common.cuh"
+
+namespace b200lora {
+
+constexpr int kDecMaxRows = 128;
+constexpr int kDecMaxPlanes = 9;      // 8 K parts + the LoRA delta
+
+// ============================================================================ base GEMM
+// part[p][t][o] = sum over K part p of x[t][k] W[o][k], as D^T = W . x^T on tcgen05: 128 weight rows are the M operand, the
+// tokens the N operand. CTA = (weight row tile, K part).
+constexpr int kDecGemmThreads = 192;  // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
+constexpr int kDecGemmStages = 4;
+constexpr int kDecBK = 64;
+
+struct DecGemmArgs {
+  float* part;
+  int T, in_dim, out, n_pad;  // n_pad: T rounded up to 16
+  int k_part;                 // columns of a K part (multiple of 64)
+  int after_delta;            // the launch before this one is the delta kernel of the same projection (see above)
+  // the plane of the delta kernel: rows without a delta are zeroed here (a cluster of that kernel that has no rows exits at once)
+  float* delta;
+  const int32_t *token_to_slot, *rank_per_slot;
+  int S;
+};
+struct DecGemmMaps {
+  CUtensorMap w;  // [out, in], box 128 x 64
+  CUtensorMap x;  // [T, in], box n_pad x 64
+};
+
+__global__ void __launch_bounds__(kDecGemmThreads, 1)
+decode_gemm_kernel(const __grid_constant__ DecGemmMaps maps, const DecGemmArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(8) uint64_t bars[2 * kDecGemmStages + 1];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ volatile int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;
+  constexpr uint32_t kW = 128 * kDecBK * 2;
+  const uint32_t x_bytes = (uint32_t)a.n_pad * kDecBK * 2, stage = kW + ((x_bytes + 1023u) & ~1023u);
+  const uint32_t bar0 = smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * (uint32_t)s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (uint32_t)(kDecGemmStages + s); };
+  const uint32_t acc_full = bar0 + 8u * (2 * kDecGemmStages);
+  int tmem_cols = 32;
+  while (tmem_cols < a.n_pad) tmem_cols *= 2;
+  if (tid == 0) {
+    for (int s = 0; s < kDecGemmStages; ++s) { mbar_init(full_bar(s), 2); mbar_init(empty_bar(s), 1); }  // full: W and x
+    mbar_init(acc_full, 1);
+    abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&tmem_base_s), (uint32_t)tmem_cols);
+    tc_fence_before_sync();
+  }
+  __syncthreads();
+  griddep_launch_dependents();  // (after this CTA holds its tensor memory)
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_s;
+  const int row0 = blockIdx.x * 128, k0 = blockIdx.y * a.k_part;
+  const int nk = (min(a.k_part, a.in_dim - k0) + kDecBK - 1) / kDecBK;
+  if (warp == 0) {
+    const uint32_t leader = elect_one();
+    if (leader) { tma_prefetch_desc(&maps.w); tma_prefetch_desc(&maps.x); }
+    const int ahead = min(nk, kDecGemmStages);
+    auto load_w = [&](int kc, int st) {
+      if (leader) {
+        mbar_arrive_expect_tx(full_bar(st), kW);
+        tma_load_2d(smem_base + (uint32_t)st * stage, &maps.w, k0 + kc * kDecBK, row0, full_bar(st));
+      }
+      __syncwarp();
+    };
+    for (int kc = 0; kc < ahead; ++kc) load_w(kc, kc);  // weights depend on nothing
+    if (!a.after_delta) griddep_wait();
+    int st = 0, round = 0;
+    for (int kc = 0; kc < nk; ++kc) {
+      if (round > 0) {
+        mbar_wait_bounded(empty_bar(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
+        load_w(kc, st);
+      }
+      if (leader) {
+        mbar_arrive_expect_tx(full_bar(st), x_bytes);
+        tma_load_2d(smem_base + (uint32_t)st * stage + kW, &maps.x, k0 + kc * kDecBK, 0, full_bar(st));
+      }
+      __syncwarp();
+      if (++st == kDecGemmStages) { st = 0; ++round; }
+    }
+  } else if (warp == 1) {
+    const uint32_t leader = elect_one();
+    const uint64_t desc0 = umma_smem_desc(smem_base, 128);
+    const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0, idesc = umma_idesc_bf16(128, a.n_pad);
+    int st = 0, round = 0;
+    for (int kc = 0; kc < nk; ++kc) {
+      mbar_wait_bounded(full_bar(st), (uint32_t)(round & 1), &abort_flag);
+      tc_fence_after_sync();
+      const uint32_t w = lo0 + ((uint32_t)st * stage >> 4), xr = w + (kW >> 4);
+#pragma unroll
+      for (int k4 = 0; k4 < kDecBK / 16; ++k4) umma_elected(tmem_base, w + 2u * k4, xr + 2u * k4, hi, idesc, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
+      umma_commit_elected(empty_bar(st), leader);
+      if (++st == kDecGemmStages) { st = 0; ++round; }
+    }
+    umma_commit_elected(acc_full, leader);
+  } else {
+    const int quarter = warp & 3, o = row0 + quarter * 32 + lane;
+    float* dst = a.part + (int64_t)blockIdx.y * a.T * a.out + o;
+    if (a.delta != nullptr && blockIdx.y == 0) {  // (32 rows at a time: one by one the lookups took 12 us)
+      for (int t0 = 0; t0 < a.T; t0 += 32) {
+        bool dead = false;
+        if (t0 + lane < a.T) {
+          const int sl = a.token_to_slot[t0 + lane];
+          dead = sl < 0 || sl >= a.S || (a.rank_per_slot != nullptr && a.rank_per_slot[sl] <= 0);
+        }
+        for (unsigned rows = __ballot_sync(0xffffffffu, dead); rows != 0; rows &= rows - 1)
+          if (o < a.out) a.delta[(int64_t)(t0 + __ffs((int)rows) - 1) * a.out + o] = 0.f;
+      }
+    }
+    mbar_wait_bounded(acc_full, 0u, &abort_flag);
+    tc_fence_after_sync();
+    for (int c = 0; c < a.T; c += 16) {
+      uint32_t v[16];
+      tmem_ld_32x16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c, v);
+      tmem_ld_wait();
+      if (o < a.out) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+          if (c + e < a.T) dst[(int64_t)(c + e) * a.out] = __uint_as_float(v[e]);
+      }
+    }
+    tc_fence_before_sync();
+  }
+  griddep_wait();  // the delta kernel (or whatever came before) is complete before this launch is
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)tmem_cols);
+  if (tid == 0 && abort_flag != 0) atomicOr(&g_b200_status, kStatusWaitGaveUp);
+}
+
+// K parts of a projection: about 128 CTAs, at most 8 parts of at least one 64-column step
+inline int decode_gemm_parts(int in_dim, int out) {
+  const int tiles = ceil_div_i(out, 128), steps = ceil_div_i(in_dim, kDecBK);
+  int parts = 1;
+  while (parts < 8 && tiles * parts * 2 <= 148 && ceil_div_i(steps, 2 * parts) * (2 * parts - 1) < steps) parts *= 2;
+  return parts;
+}
+
+template <typename... Params, typename... Args>
+inline int launch_dependent(void (*kernel)(Params...), const char* name, dim3 grid, int threads, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = bgmv_options().pdl ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(B200_LORA_ECUDA, "%s launch: %s", name, cudaGetErrorString(e));
+  }
+  return B200_LORA_OK;
+}
+
+inline int decode_gemm_launch(float* part, const void* x, int64_t x_ld, int T, int in_dim, const void* w, int64_t w_ld, int out, float* delta,
+                              const int32_t* token_to_slot, const int32_t* rank_per_slot, int S, cudaStream_t stream) {
+  DecGemmArgs a;
+  DecGemmMaps maps;
+  const int parts = decode_gemm_parts(in_dim, out);
+  a.part = part; a.T = T; a.in_dim = in_dim; a.out = out; a.n_pad = round_up_i(T, 16); a.after_delta = delta != nullptr;
+  a.delta = delta; a.token_to_slot = token_to_slot; a.rank_per_slot = rank_per_slot; a.S = S;
+  a.k_part = round_up_i(ceil_div_i(in_dim, parts), kDecBK);
+  if (int rc = make_tmap_2d(&maps.w, w, (uint64_t)out, (uint64_t)in_dim, (uint64_t)w_ld, 128, kDecBK)) return rc;
+  if (int rc = make_tmap_2d(&maps.x, x, (uint64_t)T, (uint64_t)in_dim, (uint64_t)x_ld, (uint32_t)a.n_pad, kDecBK)) return rc;
+  const size_t smem = (size_t)kDecGemmStages * (128 * kDecBK * 2 + round_up_i(a.n_pad * kDecBK * 2, 1024)) + 1024;
+  const cudaError_t e = cudaFuncSetAttribute(decode_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return fail(B200_LORA_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  return launch_dependent(decode_gemm_kernel, "decode_gemm_kernel", dim3((unsigned)ceil_div_i(out, 128), (unsigned)parts), kDecGemmThreads, smem,
+                          stream, maps, a);
+}
+
+// ============================================================================ glue over planes
+// Eight consecutive columns of a row of a projection's result: the planes [planes, T, ld] added in fp32.
+__device__ __forceinline__ void planes_load8(const float* part, int planes, int64_t plane, int64_t at, float (&v)[8]) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) v[e] = 0.f;
+#pragma unroll
+  for (int p = 0; p < kDecMaxPlanes; ++p) {
+    if (p < planes) {
+      const float4* src = reinterpret_cast<const float4*>(part + p * plane + at);
+      const float4 a = __ldcg(src), b = __ldcg(src + 1);
+      v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+      v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+    }
+  }
+}
+
+// hidden_out = residual + sum of planes (bf16); normed = rms_norm(hidden_out) * weight. One CTA per row, one 8-column vector per
+// thread: a row's loads are all in flight at once.
+__global__ void __launch_bounds__(512) decode_add_rmsnorm_kernel(__nv_bfloat16* __restrict__ normed, __nv_bfloat16* hidden_out,
+                                                                 const float* part, int planes, const __nv_bfloat16* residual,
+                                                                 const __nv_bfloat16* __restrict__ weight, int T, int H, float eps) {
+  __shared__ float sums[16];
+  griddep_launch_dependents();
+  const int row = blockIdx.x, v8 = threadIdx.x * 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Vec8<__nv_bfloat16> w, res, h;
+  const bool live = v8 < H;
+  if (live) w.raw = *reinterpret_cast<const uint4*>(weight + v8);
+  griddep_wait();
+  float v[8], ss = 0.f;
+  if (live) {
+    res.raw = *reinterpret_cast<const uint4*>(residual + (int64_t)row * H + v8);
+    planes_load8(part, planes, (int64_t)T * H, (int64_t)row * H + v8, v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      h.set(e, res.get(e) + v[e]);
+      v[e] = h.get(e);  // the norm sees the rounded sum
+      ss += v[e] * v[e];
+    }
+    *reinterpret_cast<uint4*>(hidden_out + (int64_t)row * H + v8) = h.raw;
+  }
+  ss = warp_sum(ss);
+  if (lane == 0) sums[warp] = ss;
+  __syncthreads();
+  ss = 0.f;
+  for (int i = 0; i < (int)(blockDim.x >> 5); ++i) ss += sums[i];
+  if (!live) return;
+  const float rstd = rsqrtf(ss / (float)H + eps);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) h.set(e, v[e] * rstd * w.get(e));
+  *reinterpret_cast<uint4*>(normed + (int64_t)row * H + v8) = h.raw;
+}
+
+// out = silu(gate) * up of the summed planes [planes, T, 2 I]
+__global__ void __launch_bounds__(256) decode_silu_mul_kernel(__nv_bfloat16* __restrict__ out, const float* part, int planes, int T, int I) {
+  griddep_launch_dependents();
+  griddep_wait();
+  const int nvec = I >> 3, total = T * nvec;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+    const int row = i / nvec, v8 = (i - row * nvec) * 8;
+    float g[8], u[8];
+    const int64_t at = (int64_t)row * 2 * I + v8;
+    planes_load8(part, planes, (int64_t)T * 2 * I, at, g);
+    planes_load8(part, planes, (int64_t)T * 2 * I, at + I, u);
+    Vec8<__nv_bfloat16> o;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o.set(e, g[e] / (1.f + expf(-g[e])) * u[e]);
+    *reinterpret_cast<uint4*>(out + (int64_t)row * I + v8) = o.raw;
+  }
+}
+
+// ============================================================================ attention
+// One CTA per (kv head, request): sums the planes of the request's q heads of that kv head, k and v, rotates q and k, stores k
+// and v to the paged cache and attends over the cached tokens. The K and V rows of a chunk of tokens are requested with
+// cp.async, those of earlier steps before the wait; eight warps take 16 tokens each in turn (mma.sync m16n8k16 with the up
+// to 16 q heads as rows, online softmax per warp, merged at the end).
+constexpr int kDecAttnThreads = 256;
+constexpr int kDecAttnWarps = 8;
+
+struct DecAttnArgs {
+  const float* part; int planes, ld;       // [planes, T, (Hq + 2 Hk) D]
+  int T, Hq, Hk;
+  const int64_t* positions;
+  const void* cos; const void* sin;        // [max_pos, D / 2] or [max_pos, D]
+  int table_dim, table_dtype, max_pos;
+  __nv_bfloat16 *k_cache, *v_cache;        // [blocks, block_size, Hk, D]
+  const int32_t* block_tables; int max_blocks, block_size;
+  const int32_t* context_lens;             // tokens to attend to, the new one included
+  const int64_t* slot_mapping;             // where the new token's k and v go (< 0: nowhere)
+  __nv_bfloat16* out;                      // [T, Hq D]
+  float scale;
+  int early;                               // everything before the launch pair of the projection is complete at the start
+};
+
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int D>
+__host__ __device__ constexpr int dec_attn_chunk() { return D == 64 ? 384 : 192; }  // tokens in shared memory at a time (two CTAs per SM)
+template <int D>
+__host__ __device__ constexpr int dec_attn_smem() {
+  const int kv = 2 * dec_attn_chunk<D>() * (D * 2 + 16), merge = kDecAttnWarps * 16 * (D + 2) * 4;
+  return (kv > merge ? kv : merge) + 16 * (D * 2 + 16);
+}
+
+template <int D>
+__global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const DecAttnArgs a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  constexpr int kPitch = D * 2 + 16, kChunk = dec_attn_chunk<D>(), kHalf = D / 2;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int kvh = blockIdx.x, req = blockIdx.y, group = a.Hq / a.Hk;
+  griddep_launch_dependents();
+  const uint32_t q_u32 = smem_u32(smem), k_u32 = q_u32 + 16 * kPitch, v_u32 = k_u32 + kChunk * kPitch;
+  if (!a.early) griddep_wait();
+  const int ctx = a.context_lens[req];
+  const int32_t* table = a.block_tables + (int64_t)req * a.max_blocks;
+  const int n_old = max(ctx - 1, 0);  // tokens whose k and v are in the cache already
+
+  // rows [c0, c0 + n) of the cache into the chunk buffers; the last row of all is the new token's (written below), rows up
+  // to the next multiple of 16 are zero (their probabilities are zero, their values must be finite)
+  auto load_chunk = [&](int c0, int n) {
+    const int rows = (n + 15) & ~15;
+    constexpr int kPieces = D / 8;
+    for (int i = tid; i < rows * kPieces; i += kDecAttnThreads) {
+      const int r = i / kPieces, p = i - r * kPieces, tok = c0 + r;
+      if (tok == n_old && r < n) continue;
+      const bool live = r < n;
+      int64_t at = 0;
+      if (live) at = ((int64_t)table[tok / a.block_size] * a.block_size + tok % a.block_size) * a.Hk * D + (int64_t)kvh * D + p * 8;
+      const uint32_t off = (uint32_t)(r * kPitch + p * 16);
+      cp_async_16(k_u32 + off, a.k_cache + at, live ? 16u : 0u);
+      cp_async_16(v_u32 + off, a.v_cache + at, live ? 16u : 0u);
+    }
+  };
+  if (ctx > 0) load_chunk(0, min(ctx, kChunk));
+  if (a.early) griddep_wait();
+
+  // ---- q, k, v of the new token
+  int64_t pos = a.positions[req];
+  pos = pos < 0 ? 0 : (pos >= a.max_pos ? a.max_pos - 1 : pos);
+  const int64_t slot = a.slot_mapping[req];
+  const int64_t plane = (int64_t)a.T * a.ld, row_at = (int64_t)req * a.ld;
+  const int hi_off = a.table_dim == D ? kHalf : 0;
+  uint8_t* const k_new = smem + 16 * kPitch + (n_old % kChunk) * kPitch;
+  uint8_t* const v_new = k_new + kChunk * kPitch;
+  const bool new_in_first = n_old < kChunk;
+  __shared__ __align__(16) __nv_bfloat16 kv_new[2][D];
+  for (int i = tid; i < (group + 2) * kHalf; i += kDecAttnThreads) {
+    const int head = i / kHalf, j = i - head * kHalf;  // heads 0 .. group - 1: q; group: k; group + 1: v
+    const int64_t col = head < group ? (int64_t)(kvh * group + head) * D : (int64_t)(a.Hq + (head - group) * a.Hk + kvh) * D;
+    float x1 = 0.f, x2 = 0.f;
+#pragma unroll
+    for (int p = 0; p < kDecMaxPlanes; ++p) {
+      if (p < a.planes) {
+        x1 += __ldcg(a.part + p * plane + row_at + col + j);
+        x2 += __ldcg(a.part + p * plane + row_at + col + kHalf + j);
+      }
+    }
+    if (head <= group) {
+      const int64_t tb = pos * a.table_dim + j;
+      const float c1 = table_at(a.cos, a.table_dtype, tb), s1 = table_at(a.sin, a.table_dtype, tb);
+      const float c2 = table_at(a.cos, a.table_dtype, tb + hi_off), s2 = table_at(a.sin, a.table_dtype, tb + hi_off);
+      const float y1 = __fadd_rn(__fmul_rn(x1, c1), __fmul_rn(-x2, s1)), y2 = __fadd_rn(__fmul_rn(x2, c2), __fmul_rn(x1, s2));
+      x1 = y1; x2 = y2;
+    }
+    __nv_bfloat16* dst = head < group ? reinterpret_cast<__nv_bfloat16*>(smem + head * kPitch) : kv_new[head - group];
+    dst[j] = __float2bfloat16_rn(x1);
+    dst[kHalf + j] = __float2bfloat16_rn(x2);
+  }
+  for (int i = tid; i < (16 - group) * D; i += kDecAttnThreads)  // unused rows of the q tile
+    reinterpret_cast<__nv_bfloat16*>(smem + (group + i / D) * kPitch)[i % D] = __float2bfloat16_rn(0.f);
+  __syncthreads();
+  if (tid < 2 * (D / 8)) {
+    const int which = tid / (D / 8), p = tid - which * (D / 8);
+    const uint4 piece = *reinterpret_cast<const uint4*>(&kv_new[which][8 * p]);
+    if (slot >= 0) *reinterpret_cast<uint4*>((which ? a.v_cache : a.k_cache) + slot * a.Hk * D + (int64_t)kvh * D + 8 * p) = piece;
+    if (new_in_first && ctx > 0) *reinterpret_cast<uint4*>((which ? v_new : k_new) + 16 * p) = piece;
+  }
+
+  uint32_t qf[D / 16][4];
+  {
+    const uint32_t addr = q_u32 + (uint32_t)((lane & 15) * kPitch + (lane >> 4) * 16);
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k) ldsm_x4(addr + 32u * k, qf[k]);
+  }
+  float o[D / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int d = 0; d < D / 8; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
+  const float sc = a.scale * 1.4426950408889634f;  // scores in units of log2(e)
+
+  for (int c0 = 0; c0 < ctx; c0 += kChunk) {
+    const int n = min(ctx - c0, kChunk);
+    if (c0 > 0) {
+      __syncthreads();  // the previous chunk has been read
+      load_chunk(c0, n);
+      if (n_old >= c0 && n_old < c0 + n && tid < 2 * (D / 8)) {
+        const int which = tid / (D / 8), p = tid - which * (D / 8);
+        *reinterpret_cast<uint4*>((which ? v_new : k_new) + 16 * p) = *reinterpret_cast<const uint4*>(&kv_new[which][8 * p]);
+      }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    for (int b = warp * 16; b < n; b += kDecAttnWarps * 16) {
+      float s[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) s[h][0] = s[h][1] = s[h][2] = s[h][3] = 0.f;
+      // matrices: tokens 0-7 / dims 0-7, tokens 0-7 / dims 8-15, tokens 8-15 / dims 0-7, tokens 8-15 / dims 8-15
+      const uint32_t ka = k_u32 + (uint32_t)((b + (lane & 7) + ((lane >> 4) << 3)) * kPitch + ((lane >> 3) & 1) * 16);
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k) {
+        uint32_t kf[4];
+        ldsm_x4(ka + 32u * k, kf);
+        mma_bf16_16816(s[0], qf[k][0], qf[k][1], qf[k][2], qf[k][3], kf[0], kf[1]);
+        mma_bf16_16816(s[1], qf[k][0], qf[k][1], qf[k][2], qf[k][3], kf[2], kf[3]);
+      }
+      float mx[2] = {m[0], m[1]};
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool live = b + 8 * h + 2 * t + (e & 1) < n;
+          s[h][e] = live ? s[h][e] * sc : -INFINITY;
+          mx[e >> 1] = fmaxf(mx[e >> 1], s[h][e]);
+        }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], 1));
+        mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], 2));
+        const float f = exp2f(m[q] - mx[q]);  // (token b of the tile is live, so mx is finite)
+        m[q] = mx[q];
+        l[q] *= f;
+#pragma unroll
+        for (int d = 0; d < D / 8; ++d) { o[d][2 * q] *= f; o[d][2 * q + 1] *= f; }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s[h][e] = exp2f(s[h][e] - m[e >> 1]);
+          l[e >> 1] += s[h][e];
+        }
+      const uint32_t p0 = pack_bf16x2(s[0][0], s[0][1]), p1 = pack_bf16x2(s[0][2], s[0][3]);
+      const uint32_t p2 = pack_bf16x2(s[1][0], s[1][1]), p3 = pack_bf16x2(s[1][2], s[1][3]);
+      const uint32_t va = v_u32 + (uint32_t)((b + (lane & 15)) * kPitch + (lane >> 4) * 16);
+#pragma unroll
+      for (int d = 0; d < D / 16; ++d) {
+        uint32_t vf[4];
+        ldsm_x4_t(va + 32u * d, vf);
+        mma_bf16_16816(o[2 * d], p0, p1, p2, p3, vf[0], vf[1]);
+        mma_bf16_16816(o[2 * d + 1], p0, p1, p2, p3, vf[2], vf[3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    l[q] += __shfl_xor_sync(0xffffffffu, l[q], 1);
+    l[q] += __shfl_xor_sync(0xffffffffu, l[q], 2);
+  }
+  // ---- merge the warps: [warp][head][D] sums, then m and l
+  __syncthreads();
+  float* acc = reinterpret_cast<float*>(smem + 16 * kPitch);
+  float* ml = acc + kDecAttnWarps * 16 * D;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int head = g + 8 * q;
+    if (head < group) {
+#pragma unroll
+      for (int d = 0; d < D / 8; ++d)
+        *reinterpret_cast<float2*>(acc + (warp * 16 + head) * D + 8 * d + 2 * t) = make_float2(o[d][2 * q], o[d][2 * q + 1]);
+      if (t == 0) { ml[(warp * 16 + head) * 2] = m[q]; ml[(warp * 16 + head) * 2 + 1] = l[q]; }
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < group * D / 2; i += kDecAttnThreads) {
+    const int head = i / (D / 2), d = (i - head * (D / 2)) * 2;
+    float top = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kDecAttnWarps; ++w) top = fmaxf(top, ml[(w * 16 + head) * 2]);
+    float total = 0.f, x = 0.f, y = 0.f;
+#pragma unroll
+    for (int w = 0; w < kDecAttnWarps; ++w) {
+      const float mw = ml[(w * 16 + head) * 2];
+      const float f = mw == -INFINITY ? 0.f : exp2f(mw - top);
+      const float2 v = *reinterpret_cast<const float2*>(acc + (w * 16 + head) * D + d);
+      total += f * ml[(w * 16 + head) * 2 + 1];
+      x += f * v.x;
+      y += f * v.y;
+    }
+    const float inv = total > 0.f ? 1.f / total : 0.f;
+    *reinterpret_cast<uint32_t*>(a.out + (int64_t)req * a.Hq * D + (int64_t)(kvh * group + head) * D + d) = pack_bf16x2(x * inv, y * inv);
+  }
+}
+
+// ------------------------------------------------------------------ host side
+inline int decode_attention_launch(const DecAttnArgs& a, int D, cudaStream_t stream) {
+  const dim3 grid((unsigned)a.Hk, (unsigned)a.T);
+#define B200_DEC_ATTN(DIM)                                                                                                          \
+  {                                                                                                                                 \
+    const cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_attn_smem<DIM>()); \
+    if (e != cudaSuccess) return fail(B200_LORA_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));                          \
+    return launch_dependent(decode_attention_kernel<DIM>, "decode_attention_kernel", grid, kDecAttnThreads, dec_attn_smem<DIM>(), stream, a); \
+  }
+  if (D == 64) B200_DEC_ATTN(64)
+  B200_DEC_ATTN(128)
+#undef B200_DEC_ATTN
+}
+
+}  // namespace b200lora
