@@ -382,8 +382,9 @@ int lora_b200_debug_trace(long long* out, int32_t n_values);
  * lora_b200_decode_silu_mul: out = silu(gate) * up of planes [n, T, 2 * intermediate].
  * lora_b200_decode_attention: q, k, v = sum of planes [n, T, (heads + 2 kv_heads) * head_dim]; rotates q and k, stores k and v at
  *   slot_mapping (int64, < 0 = nowhere) and attends over the context_lens[t] first tokens of the request's block table, the
- *   new one being the last of them. head_dim 64 or 128, at most 16 q heads per kv head. after_delta: the planes come from a
- *   lora_b200_decode_linear with adapters directly before this call.
+ *   new one being the last of them. head_dim 64 or 128, at most 16 q heads per kv head.
+ * Start a chain with an ordinary launch (one that waits for the stream): within it the cache rows of earlier steps, weights and
+ * index arrays are read before the launches ahead are complete.
  */
 int lora_b200_decode_planes(int32_t in_dim, int32_t out);
 int lora_b200_decode_linear(float* planes, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight,
@@ -402,7 +403,7 @@ int lora_b200_decode_attention(void* out, const float* planes, int32_t n_planes,
                                const void* sin_table, int32_t table_dim, int32_t table_dtype, int32_t max_position,
                                void* k_cache, void* v_cache, const int32_t* block_tables, int32_t max_blocks,
                                int32_t block_size, const int32_t* context_lens, const int64_t* slot_mapping, float scale,
-                               int32_t after_delta, void* stream);
+                               void* stream);
 
 #ifdef __cplusplus
 }

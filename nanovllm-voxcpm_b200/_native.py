@@ -105,7 +105,7 @@ _SIGNATURES = {
     "lora_b200_decode_attention": (
         c_int32,
         [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
-         c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_float, c_int32, c_void_p],
+         c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_float, c_void_p],
     ),
     "lora_b200_tp_allreduce": (
         c_int32, [c_void_p, c_void_p, c_int32, POINTER(c_void_p), c_int32, c_int32, c_int32, c_void_p],

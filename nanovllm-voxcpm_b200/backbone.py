@@ -221,7 +221,7 @@ class Decoder(nn.Module):
         return True
 
     def _decode_chain(self, embeds, positions, step: AttentionStep):
-        """One decode step as nine dependent launches per layer whose projections leave their parts to the consumer."""
+        """One decode step as seven dependent launches per layer whose projections leave their parts to the consumer."""
         cfg, T, dev = self.cfg, embeds.size(0), embeds.device
         heads, kv_heads, dim, inter, eps = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.intermediate_size, cfg.rms_norm_eps
         lib, stream = N.lib(), N.current_stream(dev)
@@ -272,7 +272,7 @@ class Decoder(nn.Module):
                     attn.data_ptr(), planes.data_ptr(), n, T, heads, kv_heads, dim, positions.data_ptr(), self.cos.data_ptr(),
                     self.sin.data_ptr(), self.cos.size(1), N.dtype_code(self.cos.dtype), self.cos.size(0), sa.k_cache.data_ptr(),
                     sa.v_cache.data_ptr(), step.block_tables.data_ptr(), step.block_tables.size(1), cfg.kv_block_size,
-                    step.context_lens.data_ptr(), step.slot_mapping.data_ptr(), dim ** -0.5, 1 if with_lora else 0, stream))
+                    step.context_lens.data_ptr(), step.slot_mapping.data_ptr(), dim ** -0.5, stream))
                 add_norm(linear(sa.o_proj, attn), layer.post_attention_layernorm)
                 n = linear(layer.mlp.gate_up_proj, normed)
                 N.check(lib.lora_b200_decode_silu_mul(act.data_ptr(), planes.data_ptr(), n, T, inter, stream))

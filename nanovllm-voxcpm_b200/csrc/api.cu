@@ -181,9 +181,9 @@ int lora_b200_decode_linear(float* planes, const void* x, int64_t x_ld, int32_t 
       !aligned16(weight))
     return fail(B200_LORA_EUNSUPPORTED, "decode_linear: in_dim must be a multiple of 64, out of 8, rows 16-byte aligned");
   cudaStream_t st_ = static_cast<cudaStream_t>(stream);
+  BgmvProblem bp = {};
   if (n_slices > 0) {
     if (out_sizes == nullptr || col_offsets == nullptr || token_to_slot == nullptr) return fail(B200_LORA_EINVAL, "decode_linear: null slice or slot array");
-    BgmvProblem bp = {};
     if (int rc = fill_slices(bp.st, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, true, true)) return rc;
     int covered = 0;
     for (int s = 0; s < bp.st.n; ++s) {
@@ -200,10 +200,8 @@ int lora_b200_decode_linear(float* planes, const void* x, int64_t x_ld, int32_t 
     if (sorted_idx == nullptr || slot_ids == nullptr || counts == nullptr || offsets == nullptr)
       return fail(B200_LORA_EINVAL, "decode_linear: needs the bucket arrays");
     if (!bgmv_supported(bp, &why)) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: %s", why);
-    if (int rc = bgmv_launch(bp, st_)) return rc;
   }
-  float* delta = n_slices > 0 ? planes + (size_t)decode_gemm_parts(in_dim, out_total) * T * out_total : nullptr;
-  return decode_gemm_launch(planes, x, x_ld, T, in_dim, weight, w_ld, out_total, delta, token_to_slot, rank_per_slot, S, st_);
+  return decode_linear_launch(planes, x, x_ld, T, in_dim, weight, w_ld, out_total, n_slices > 0 ? &bp : nullptr, st_);
 }
 
 int lora_b200_decode_add_rmsnorm(void* normed, void* hidden_out, const float* planes, int32_t n_planes, const void* residual,
@@ -232,7 +230,7 @@ int lora_b200_decode_attention(void* out, const float* planes, int32_t n_planes,
                                int32_t head_dim, const int64_t* positions, const void* cos_table, const void* sin_table,
                                int32_t table_dim, int32_t table_dtype, int32_t max_position, void* k_cache, void* v_cache,
                                const int32_t* block_tables, int32_t max_blocks, int32_t block_size, const int32_t* context_lens,
-                               const int64_t* slot_mapping, float scale, int32_t after_delta, void* stream) {
+                               const int64_t* slot_mapping, float scale, void* stream) {
   if (T < 1 || T > 65535 || num_kv_heads < 1 || num_heads % num_kv_heads != 0 || num_heads / num_kv_heads > 16 || (head_dim != 64 && head_dim != 128))
     return fail(B200_LORA_EUNSUPPORTED, "decode_attention: T=%d heads=%d / %d of %d", T, num_heads, num_kv_heads, head_dim);
   if (n_planes < 1 || n_planes > kDecMaxPlanes || max_blocks < 1 || block_size < 1 || max_position < 1)
@@ -247,7 +245,7 @@ int lora_b200_decode_attention(void* out, const float* planes, int32_t n_planes,
   a.positions = positions; a.cos = cos_table; a.sin = sin_table; a.table_dim = table_dim; a.table_dtype = table_dtype; a.max_pos = max_position;
   a.k_cache = static_cast<__nv_bfloat16*>(k_cache); a.v_cache = static_cast<__nv_bfloat16*>(v_cache);
   a.block_tables = block_tables; a.max_blocks = max_blocks; a.block_size = block_size; a.context_lens = context_lens; a.slot_mapping = slot_mapping;
-  a.out = static_cast<__nv_bfloat16*>(out); a.scale = scale; a.early = after_delta;
+  a.out = static_cast<__nv_bfloat16*>(out); a.scale = scale;
   return decode_attention_launch(a, head_dim, static_cast<cudaStream_t>(stream));
 }
 

@@ -77,14 +77,14 @@ struct BgmvProblem {
   // 3 = overwrite: y[t, cols] = delta for rows with an adapter and -0.0 for every other row (y is not
   // read); a base GEMM that then accumulates into y (beta = 1) gives base + delta, and x + (-0.0) == x
   // keeps rows without adapter bit-identical to the base result.
-  // 4 = y = delta in fp32 [T, y_ld], rows with an adapter only: one of the planes that decode_step.cuh adds up. Its
-  // successor in the stream may start when this launch has passed its own wait, and need not wait for what came before.
+  // 4 = y = delta in fp32 [T, y_ld], rows with an adapter only: one of the planes that decode_step.cuh adds up.
   int mode = 0;
   // Precision of the rank-r intermediate and of the update. 0 (bf16, r_max % 32 == 0): tmp rounded to bf16, the delta
   // rounded to bf16 and added at the L2. 1 (bf16) / 2 (fp16): tmp kept as the sum of two 16-bit numbers, y read, added to
   // in fp32 and rounded once; modes 0, 1 and 2, r_max % 16 == 0. What the per-token kernel computes, which these sizes and
   // types used to take (a 37-row batch of rank-16 adapters: 45 us per projection there, 3 us here).
   int kind = 0;
+  int beside = 0;          // other CTAs in the launch, at two per SM
   void* tmp_io = nullptr;  // [n_slices, T, r_max], fp32 or (io16) values of the activations' type
   int io16 = 0;
   int zero_rows = 0;       // mode 1: rows without adapter are written as zeros (token_to_slot tells which)
@@ -98,7 +98,7 @@ struct BgmvParams {
   SliceTable st;  // active slices only
   const int32_t* rank_per_slot; const float* scale_per_slot;
   const int32_t *sorted_idx, *slot_ids, *counts, *offsets;
-  int n_buckets; float scaling;
+  int n_buckets, n_live; float scaling;  // n_live: clusters for first windows (a bucket each, or a bucket that holds rows each)
   int window;       // tokens per cluster (multiple of 16)
   int c_shift;      // cluster size C = 1 << c_shift
   int KP, nkp;      // columns per shrink tile (min(in, 1024)) and number of K parts
@@ -167,11 +167,11 @@ __device__ __forceinline__ void bgmv_zero_rows_without_adapter(const BgmvParams&
 // kFullK = every K part has all 1024 columns (in_dim a multiple of 1024): no column checks in the shrink
 // kKind = BgmvProblem::kind; kWide = r_max > 32: output tiles are less than 256 rows high and a step of the expand takes
 // several (the general step costs 12 % where a tile is a step)
+// block_y / blocks_y: this CTA's bucket index and their number (a launch may carry other work beside the buckets)
 template <int kMode, bool kFullK, int kKind, bool kWide>
-__global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kernel(const __grid_constant__ BgmvParams p) {
-  extern __shared__ __align__(1024) uint8_t smem[];
+__device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, const int block_y, const int blocks_y) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  int bucket = blockIdx.y;
+  int bucket = block_y;
   const int C = 1 << p.c_shift;
   const int c = (int)cluster_ctarank();
   const int NS = p.NS;
@@ -183,15 +183,34 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   // Let the next launch of the stream start at once: before its own griddepcontrol.wait it only
   // reads index metadata and lora slabs, which no kernel of this library writes, so its weight
   // traffic overlaps this kernel's compute and keeps HBM busy across launch boundaries.
-  if (p.use_pdl && !kF32Out) griddep_launch_dependents();
+  if (p.use_pdl) griddep_launch_dependents();
   // ---- bucket metadata (uniform across the cluster); barrier set-up overlaps the loads
   // Extra cluster e looks after multiple m = (e + 1) * window of the window inside the sorted rows: if m lies behind the
   // first row of a bucket [start, start + cnt), it is the i-th such multiple there, and the cluster takes the bucket's i-th
   // window. (A bucket of cnt rows has ceil(cnt / window) - 1 windows beyond its first and at least that many multiples.)
   int window_no = 0;
-  if (bucket >= p.n_buckets) {
+  if (bucket < p.n_live) {
+    // Fewer rows than buckets (graph buffers carry a bucket for every slot): the launch has a cluster per row, and cluster i
+    // takes the i-th bucket that holds rows. (A cluster per bucket cost 64 rows over 128 adapters two waves of idle CTAs.)
+    if (p.n_live < p.n_buckets) {
+      int seen = 0;
+      bucket = -1;
+      for (int b0 = 0; b0 < p.n_buckets && bucket < 0; b0 += 128) {
+        int held[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) held[i] = b0 + 32 * i + lane < p.n_buckets ? p.counts[b0 + 32 * i + lane] : 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const unsigned live = __ballot_sync(0xffffffffu, held[i] > 0);
+          const unsigned mine = __ballot_sync(0xffffffffu, held[i] > 0 && seen + __popc(live & ((1u << lane) - 1u)) == block_y);
+          if (mine != 0) bucket = b0 + 32 * i + __ffs((int)mine) - 1;
+          seen += __popc(live);
+        }
+      }
+    }
+  } else {
     volatile int* owner = reinterpret_cast<volatile int*>(smem + p.off_bar + 8 * (2 * kBgmvMaxStages + 2)) + 1;  // behind the abort flag
-    const int m = (bucket - p.n_buckets + 1) * p.window;
+    const int m = (bucket - p.n_live + 1) * p.window;
     if (tid == 0) *owner = -1;
     __syncthreads();
     for (int b = tid; b < p.n_buckets; b += kBgmvThreads) {
@@ -227,11 +246,10 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
     // An idle cluster holds nothing, but one CTA of every launch must outlive the previous launch
     // of the stream: a launch that ended before its predecessor would let the launch behind it
     // pass its own wait too early.
-    if (p.use_pdl && (kOverwrite || (kMode == 1 && p.zero_rows) || (blockIdx.y == 0 && c == 0))) griddep_wait();
-    if (p.use_pdl && kF32Out) griddep_launch_dependents();
-    if (kMode == 1 && p.zero_rows) bgmv_zero_rows_without_adapter(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvThreads);
+    if (p.use_pdl && (kOverwrite || (kMode == 1 && p.zero_rows) || (block_y == 0 && c == 0))) griddep_wait();
+    if (kMode == 1 && p.zero_rows) bgmv_zero_rows_without_adapter(p, block_y * C + c, blocks_y * C, tid, kBgmvThreads);
     if (kOverwrite)  // an idle cluster still does its share of the -0.0 rows
-      bgmv_fill_rows_without_delta(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvThreads);
+      bgmv_fill_rows_without_delta(p, block_y * C + c, blocks_y * C, tid, kBgmvThreads);
     return;
   }
   if (tid < NS) {
@@ -452,9 +470,8 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   const uint32_t it_roff = (uint32_t)(it_tok * p.pitchR + it_q) * 4u;  // K split: the item inside one sender's block
 
   if (p.use_pdl) griddep_wait();  // x and y of this launch are final from here on
-  if (p.use_pdl && kF32Out) griddep_launch_dependents();
-  if (kOverwrite) bgmv_fill_rows_without_delta(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvConsumers);
-  if (kMode == 1 && p.zero_rows) bgmv_zero_rows_without_adapter(p, (int)blockIdx.y * C + c, (int)gridDim.y * C, tid, kBgmvConsumers);
+  if (kOverwrite) bgmv_fill_rows_without_delta(p, block_y * C + c, blocks_y * C, tid, kBgmvConsumers);
+  if (kMode == 1 && p.zero_rows) bgmv_zero_rows_without_adapter(p, block_y * C + c, blocks_y * C, tid, kBgmvConsumers);
   B200_TRACE_POINT(4)
 
   int c_stage = 0;
@@ -788,6 +805,12 @@ __global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kerne
   if (tid == 0 && *abort_flag != 0) atomicOr(&g_b200_status, kStatusWaitGaveUp);
 }
 
+template <int kMode, bool kFullK, int kKind, bool kWide>
+__global__ void __launch_bounds__(kBgmvThreads, BGMV_MINBLOCKS) bgmv_fused_kernel(const __grid_constant__ BgmvParams p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  bgmv_body<kMode, kFullK, kKind, kWide>(p, smem, (int)blockIdx.y, (int)gridDim.y);
+}
+
 // ------------------------------------------------------------------ host side
 struct BgmvOptions {
   int cluster = 0;   // 0 = auto
@@ -847,7 +870,10 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
     // 4, 7.0 with 2, 6.8 with 8.
     const double nb = (double)b.n_buckets;
     const double in_use = nb * (1.0 - std::exp(-(double)std::max(b.T, 1) / nb));
-    C = in_use <= 56.0 ? 4 : (in_use <= 112.0 ? 2 : 1);
+    // Other CTAs in the launch (decode_step.cuh's GEMM) leave fewer places: 128 of them beside 50 buckets in use, 1024-wide,
+    // rank 32: 442 us a step with 2, 500 with 4, 548 with 1; beside 16 buckets of 100 rows 383 with 2, 368 with 4.
+    const double resident = 2.0 * 148 - b.beside, half = 0.38 * resident;
+    C = in_use * 2 <= half ? 4 : (in_use <= half ? 2 : 1);
     // A CTA streams its share of the slabs at 25 - 30 GB/s (loads, multiplication and exchange take turns): large adapters
     // want more CTAs, as far as those are resident together or their streams are long. Measured, us per projection with
     // clusters of 4 / 8: one row of 4096-wide layers, rank 64: 23.1 / 9.8; 64 rows over 32 adapters of 2048-wide layers, rank
@@ -857,7 +883,6 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
     // CTA per bucket, 19.7 with 2, 19.0 with 4.
     int64_t bucket_bytes = 0;
     for (int s = 0; s < st.n; ++s) bucket_bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + st.out[s]);
-    const double resident = 2.0 * 148;
     while (C < 4 && (bucket_bytes / C > 512 * 1024 || (bucket_bytes / C > 256 * 1024 && in_use * C * 2 <= resident))) C *= 2;
     const double clusters = in_use + (b.T - 1) / kBgmvTok;
     if (C == 4 && ((bucket_bytes / 4 > 128 * 1024 && clusters * 8 <= resident) || (bucket_bytes / 4 >= 256 * 1024 && in_use * 8 <= resident))) C = 8;
@@ -879,7 +904,7 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   p.T = b.T; p.in_dim = b.in_dim; p.S = b.S; p.r_max = b.r_max; p.st = st;
   p.rank_per_slot = b.rank_per_slot; p.scale_per_slot = b.scale_per_slot;
   p.sorted_idx = b.sorted_idx; p.slot_ids = b.slot_ids; p.counts = b.counts; p.offsets = b.offsets;
-  p.n_buckets = b.n_buckets; p.scaling = b.scaling;
+  p.n_buckets = b.n_buckets; p.n_live = std::min(b.n_buckets, std::max(b.T, 1)); p.scaling = b.scaling;
   p.c_shift = log2_exact(C);
   p.KP = std::min(b.in_dim, kBgmvKP);
   p.nkp = ceil_div_i(b.in_dim, p.KP);
@@ -953,8 +978,7 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
   (const void*)bgmv_fused_kernel<M, false, K, false>, (const void*)bgmv_fused_kernel<M, true, K, false>,                     \
       (const void*)bgmv_fused_kernel<M, false, K, true>, (const void*)bgmv_fused_kernel<M, true, K, true>
     const void* kernels[] = {B200_BGMV_ALL(0, 0), B200_BGMV_ALL(1, 0), B200_BGMV_ALL(2, 0), B200_BGMV_ALL(3, 0), B200_BGMV_ALL(0, 1), B200_BGMV_ALL(0, 2), B200_BGMV_ALL(1, 1),
-                             B200_BGMV_ALL(1, 2), B200_BGMV_ALL(2, 1), B200_BGMV_ALL(2, 2), B200_BGMV_ALL(4, 0),
-                             B200_BGMV_ALL(4, 1)};
+                             B200_BGMV_ALL(1, 2), B200_BGMV_ALL(2, 1), B200_BGMV_ALL(2, 2)};
 #undef B200_BGMV_ALL
     for (const void* k : kernels) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kBgmvSmemMax);
@@ -963,7 +987,7 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
     configured_device = dev;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(1u << p.c_shift, (unsigned)(p.n_buckets + (p.T - 1) / p.window), 1);
+  cfg.gridDim = dim3(1u << p.c_shift, (unsigned)(p.n_live + (p.T - 1) / p.window), 1);
   cfg.blockDim = dim3(kBgmvThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -987,15 +1011,13 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
                            : cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, false, K, false>, p)) \
                : (p.full_k ? cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, true, K, true>, p)    \
                            : cudaLaunchKernelEx(&cfg, bgmv_fused_kernel<M, false, K, true>, p)))
-  switch (8 * p.kind + p.mode) {
+  switch (8 * p.kind + p.mode) {  // (mode 4: decode_step.cuh)
     case 1: e = B200_BGMV_LAUNCH(1, 0); break;
     case 2: e = B200_BGMV_LAUNCH(2, 0); break;
     case 3: e = B200_BGMV_LAUNCH(3, 0); break;
-    case 4: e = B200_BGMV_LAUNCH(4, 0); break;
     case 8: e = B200_BGMV_LAUNCH(0, 1); break;
     case 9: e = B200_BGMV_LAUNCH(1, 1); break;
     case 10: e = B200_BGMV_LAUNCH(2, 1); break;
-    case 12: e = B200_BGMV_LAUNCH(4, 1); break;
     case 16: e = B200_BGMV_LAUNCH(0, 2); break;
     case 17: e = B200_BGMV_LAUNCH(1, 2); break;
     case 18: e = B200_BGMV_LAUNCH(2, 2); break;

@@ -4,10 +4,8 @@
 // A decode step of a small model is a chain of dependent launches, each bound by latency: with library GEMMs, the LoRA add
 // behind each of them, split-KV attention and separate glue kernels a layer of a 1024-wide decoder took 94 us (64 rows),
 // against 12 us of HBM time for its weights. Here
-//   * the base product and the LoRA delta of a projection run side by side: the fused decode kernel writes its delta (fp32)
-//     into one plane of a buffer [planes, T, out], decode_gemm_kernel its K parts into the others. The delta kernel lets its
-//     successor start once it has passed its own wait (everything before is complete then), so the GEMM needs no wait
-//     for x; it waits for the delta kernel before it ends, and what follows is ordered behind both;
+//   * the base product and the LoRA delta of a projection are one launch: clusters of the fused decode kernel write their delta
+//     (fp32) into one plane of a buffer [planes, T, out], GEMM CTAs beside them the K parts into the others;
 //   * the consumer of a projection (add + norm, RoPE + attention, SiLU * up) adds the planes in fp32: no rounding of the base
 //     output, no pass of its own;
 //   * RoPE, the cache store and attention are one kernel per (request, kv head).
@@ -23,19 +21,19 @@ namespace b200lora {
 constexpr int kDecMaxRows = 128;
 constexpr int kDecMaxPlanes = 9;      // 8 K parts + the LoRA delta
 
-// ============================================================================ base GEMM
+// ============================================================================ projection
 // part[p][t][o] = sum over K part p of x[t][k] W[o][k], as D^T = W . x^T on tcgen05: 128 weight rows are the M operand, the
 // tokens the N operand. CTA = (weight row tile, K part).
-constexpr int kDecGemmThreads = 192;  // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
-constexpr int kDecGemmStages = 4;
+constexpr int kDecGemmMaxStages = 4;
 constexpr int kDecBK = 64;
+constexpr int kDecGemmBars = 128;  // bytes of the barriers and flags in front of the ring
 
 struct DecGemmArgs {
   float* part;
   int T, in_dim, out, n_pad;  // n_pad: T rounded up to 16
-  int k_part;                 // columns of a K part (multiple of 64)
-  int after_delta;            // the launch before this one is the delta kernel of the same projection (see above)
-  // the plane of the delta kernel: rows without a delta are zeroed here (a cluster of that kernel that has no rows exits at once)
+  int tiles, parts, k_part;   // weight row tiles, K parts and their columns (multiple of 64)
+  int stages;
+  // the plane of the delta: rows without one are zeroed here (a cluster of the delta kernel that has no rows exits at once)
   float* delta;
   const int32_t *token_to_slot, *rank_per_slot;
   int S;
@@ -45,42 +43,49 @@ struct DecGemmMaps {
   CUtensorMap x;  // [T, in], box n_pad x 64
 };
 
-__global__ void __launch_bounds__(kDecGemmThreads, 1)
-decode_gemm_kernel(const __grid_constant__ DecGemmMaps maps, const DecGemmArgs a) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ __align__(8) uint64_t bars[2 * kDecGemmStages + 1];
-  __shared__ uint32_t tmem_base_s;
-  __shared__ volatile int abort_flag;
+// One GEMM CTA of kBgmvThreads threads: warp 8 TMA, warp 0 MMA, warps 4-7 epilogue.
+__device__ __forceinline__ void decode_gemm_body(const DecGemmMaps& maps, const DecGemmArgs& a, uint8_t* smem, int unit) {
+  // barriers, TMEM base and abort flag in the first bytes, the ring behind them (no static shared memory: with it two CTAs of
+  // the delta kernel would no longer fit on an SM)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+  volatile uint32_t& tmem_base_s = *reinterpret_cast<volatile uint32_t*>(smem + 8 * (2 * kDecGemmMaxStages + 1));
+  volatile int& abort_flag = *reinterpret_cast<volatile int*>(smem + 8 * (2 * kDecGemmMaxStages + 1) + 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;
+  if (unit >= a.tiles * a.parts) {
+    griddep_launch_dependents();
+    griddep_wait();
+    return;
+  }
+  const uint32_t smem_base = (smem_u32(smem) + kDecGemmBars + 1023u) & ~1023u;
   constexpr uint32_t kW = 128 * kDecBK * 2;
   const uint32_t x_bytes = (uint32_t)a.n_pad * kDecBK * 2, stage = kW + ((x_bytes + 1023u) & ~1023u);
   const uint32_t bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * (uint32_t)s; };
-  auto empty_bar = [&](int s) { return bar0 + 8u * (uint32_t)(kDecGemmStages + s); };
-  const uint32_t acc_full = bar0 + 8u * (2 * kDecGemmStages);
+  auto empty_bar = [&](int s) { return bar0 + 8u * (uint32_t)(kDecGemmMaxStages + s); };
+  const uint32_t acc_full = bar0 + 8u * (2 * kDecGemmMaxStages);
+  const int NS = a.stages;
   int tmem_cols = 32;
   while (tmem_cols < a.n_pad) tmem_cols *= 2;
   if (tid == 0) {
-    for (int s = 0; s < kDecGemmStages; ++s) { mbar_init(full_bar(s), 2); mbar_init(empty_bar(s), 1); }  // full: W and x
+    for (int s = 0; s < NS; ++s) { mbar_init(full_bar(s), 2); mbar_init(empty_bar(s), 1); }  // full: W and x
     mbar_init(acc_full, 1);
     abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_base_s), (uint32_t)tmem_cols);
+  if (warp == 0) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(&tmem_base_s)), (uint32_t)tmem_cols);
     tc_fence_before_sync();
   }
   __syncthreads();
   griddep_launch_dependents();  // (after this CTA holds its tensor memory)
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
-  const int row0 = blockIdx.x * 128, k0 = blockIdx.y * a.k_part;
+  const int tile = unit / a.parts, part = unit - tile * a.parts;
+  const int row0 = tile * 128, k0 = part * a.k_part;
   const int nk = (min(a.k_part, a.in_dim - k0) + kDecBK - 1) / kDecBK;
-  if (warp == 0) {
+  if (warp == kBgmvWarps) {
     const uint32_t leader = elect_one();
     if (leader) { tma_prefetch_desc(&maps.w); tma_prefetch_desc(&maps.x); }
-    const int ahead = min(nk, kDecGemmStages);
     auto load_w = [&](int kc, int st) {
       if (leader) {
         mbar_arrive_expect_tx(full_bar(st), kW);
@@ -88,8 +93,8 @@ decode_gemm_kernel(const __grid_constant__ DecGemmMaps maps, const DecGemmArgs a
       }
       __syncwarp();
     };
-    for (int kc = 0; kc < ahead; ++kc) load_w(kc, kc);  // weights depend on nothing
-    if (!a.after_delta) griddep_wait();
+    for (int kc = 0; kc < min(nk, NS); ++kc) load_w(kc, kc);  // weights depend on nothing
+    griddep_wait();
     int st = 0, round = 0;
     for (int kc = 0; kc < nk; ++kc) {
       if (round > 0) {
@@ -101,9 +106,9 @@ decode_gemm_kernel(const __grid_constant__ DecGemmMaps maps, const DecGemmArgs a
         tma_load_2d(smem_base + (uint32_t)st * stage + kW, &maps.x, k0 + kc * kDecBK, 0, full_bar(st));
       }
       __syncwarp();
-      if (++st == kDecGemmStages) { st = 0; ++round; }
+      if (++st == NS) { st = 0; ++round; }
     }
-  } else if (warp == 1) {
+  } else if (warp == 0) {
     const uint32_t leader = elect_one();
     const uint64_t desc0 = umma_smem_desc(smem_base, 128);
     const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0, idesc = umma_idesc_bf16(128, a.n_pad);
@@ -115,13 +120,14 @@ decode_gemm_kernel(const __grid_constant__ DecGemmMaps maps, const DecGemmArgs a
 #pragma unroll
       for (int k4 = 0; k4 < kDecBK / 16; ++k4) umma_elected(tmem_base, w + 2u * k4, xr + 2u * k4, hi, idesc, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
       umma_commit_elected(empty_bar(st), leader);
-      if (++st == kDecGemmStages) { st = 0; ++round; }
+      if (++st == NS) { st = 0; ++round; }
     }
     umma_commit_elected(acc_full, leader);
-  } else {
+  } else if (warp >= 4 && warp < 8) {
     const int quarter = warp & 3, o = row0 + quarter * 32 + lane;
-    float* dst = a.part + (int64_t)blockIdx.y * a.T * a.out + o;
-    if (a.delta != nullptr && blockIdx.y == 0) {  // (32 rows at a time: one by one the lookups took 12 us)
+    float* dst = a.part + (int64_t)part * a.T * a.out + o;
+    griddep_wait();  // the previous launch may still read the planes
+    if (a.delta != nullptr && part == 0) {  // (32 rows at a time: one by one the lookups took 12 us)
       for (int t0 = 0; t0 < a.T; t0 += 32) {
         bool dead = false;
         if (t0 + lane < a.T) {
@@ -146,10 +152,23 @@ decode_gemm_kernel(const __grid_constant__ DecGemmMaps maps, const DecGemmArgs a
     }
     tc_fence_before_sync();
   }
-  griddep_wait();  // the delta kernel (or whatever came before) is complete before this launch is
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)tmem_cols);
+  if (warp == 0) tmem_dealloc(tmem_base, (uint32_t)tmem_cols);
   if (tid == 0 && abort_flag != 0) atomicOr(&g_b200_status, kStatusWaitGaveUp);
+}
+
+// GEMM CTAs first (they are all in use), then the buckets of the delta kernel, in clusters of one size.
+template <bool kFullK, int kKind, bool kWide>
+__global__ void __launch_bounds__(kBgmvThreads, 2)
+decode_linear_kernel(const __grid_constant__ DecGemmMaps maps, const DecGemmArgs g, const __grid_constant__ BgmvParams p, const int gemm_rows) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if ((int)blockIdx.y < gemm_rows) decode_gemm_body(maps, g, smem, (int)blockIdx.y * (int)gridDim.x + (int)blockIdx.x);
+  else bgmv_body<4, kFullK, kKind, kWide>(p, smem, (int)blockIdx.y - gemm_rows, (int)gridDim.y - gemm_rows);
+}
+__global__ void __launch_bounds__(kBgmvThreads, 2)
+decode_gemm_kernel(const __grid_constant__ DecGemmMaps maps, const DecGemmArgs g) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  decode_gemm_body(maps, g, smem, (int)blockIdx.x);
 }
 
 // K parts of a projection: about 128 CTAs, at most 8 parts of at least one 64-column step
@@ -180,21 +199,68 @@ inline int launch_dependent(void (*kernel)(Params...), const char* name, dim3 gr
   return B200_LORA_OK;
 }
 
-inline int decode_gemm_launch(float* part, const void* x, int64_t x_ld, int T, int in_dim, const void* w, int64_t w_ld, int out, float* delta,
-                              const int32_t* token_to_slot, const int32_t* rank_per_slot, int S, cudaStream_t stream) {
-  DecGemmArgs a;
+// planes of x . W^T, and (lora != nullptr) the delta in the plane behind them
+inline int decode_linear_launch(float* planes, const void* x, int64_t x_ld, int T, int in_dim, const void* w, int64_t w_ld, int out,
+                                BgmvProblem* lora, cudaStream_t stream) {
+  DecGemmArgs a = {};
   DecGemmMaps maps;
-  const int parts = decode_gemm_parts(in_dim, out);
-  a.part = part; a.T = T; a.in_dim = in_dim; a.out = out; a.n_pad = round_up_i(T, 16); a.after_delta = delta != nullptr;
-  a.delta = delta; a.token_to_slot = token_to_slot; a.rank_per_slot = rank_per_slot; a.S = S;
-  a.k_part = round_up_i(ceil_div_i(in_dim, parts), kDecBK);
+  a.part = planes; a.T = T; a.in_dim = in_dim; a.out = out; a.n_pad = round_up_i(T, 16);
+  a.parts = decode_gemm_parts(in_dim, out); a.tiles = ceil_div_i(out, 128);
+  a.k_part = round_up_i(ceil_div_i(in_dim, a.parts), kDecBK);
+  const int stage = 128 * kDecBK * 2 + round_up_i(a.n_pad * kDecBK * 2, 1024);
+  a.stages = std::min(kDecGemmMaxStages, 98 * 1024 / stage);
   if (int rc = make_tmap_2d(&maps.w, w, (uint64_t)out, (uint64_t)in_dim, (uint64_t)w_ld, 128, kDecBK)) return rc;
   if (int rc = make_tmap_2d(&maps.x, x, (uint64_t)T, (uint64_t)in_dim, (uint64_t)x_ld, (uint32_t)a.n_pad, kDecBK)) return rc;
-  const size_t smem = (size_t)kDecGemmStages * (128 * kDecBK * 2 + round_up_i(a.n_pad * kDecBK * 2, 1024)) + 1024;
-  const cudaError_t e = cudaFuncSetAttribute(decode_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return fail(B200_LORA_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  return launch_dependent(decode_gemm_kernel, "decode_gemm_kernel", dim3((unsigned)ceil_div_i(out, 128), (unsigned)parts), kDecGemmThreads, smem,
-                          stream, maps, a);
+  size_t smem = (size_t)a.stages * stage + 1024 + kDecGemmBars;
+  if (lora == nullptr) {
+    const cudaError_t e = cudaFuncSetAttribute(decode_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(B200_LORA_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    return launch_dependent(decode_gemm_kernel, "decode_gemm_kernel", dim3((unsigned)(a.tiles * a.parts)), kBgmvThreads, smem, stream, maps, a);
+  }
+  a.delta = planes + (size_t)a.parts * T * out;
+  a.token_to_slot = lora->token_to_slot; a.rank_per_slot = lora->rank_per_slot; a.S = lora->S;
+  lora->beside = std::min(a.tiles * a.parts, 148);
+  BgmvParams p;
+  const char* why = nullptr;
+  if (!bgmv_plan(*lora, &p, &why)) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: %s", why);
+  smem = std::max(smem, (size_t)p.off_bar + 256);
+  const int C = 1 << p.c_shift, gemm_rows = ceil_div_i(a.tiles * a.parts, C);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)C, (unsigned)(gemm_rows + p.n_live + (T - 1) / p.window), 1);
+  cfg.blockDim = dim3(kBgmvThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = (unsigned)C;
+  attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = p.use_pdl ? 2 : 1;
+  cudaError_t e = cudaSuccess;
+#define B200_DEC_LINEAR(F, K, W)                                                                                              \
+  {                                                                                                                           \
+    e = cudaFuncSetAttribute(decode_linear_kernel<F, K, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBgmvSmemMax); \
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, decode_linear_kernel<F, K, W>, maps, a, p, gemm_rows);                 \
+  }
+  const int which = (p.full_k ? 4 : 0) + (p.kind ? 2 : 0) + (p.ER == 256 ? 0 : 1);
+  switch (which) {
+    case 0: B200_DEC_LINEAR(false, 0, false) break;
+    case 1: B200_DEC_LINEAR(false, 0, true) break;
+    case 2: B200_DEC_LINEAR(false, 1, false) break;
+    case 3: B200_DEC_LINEAR(false, 1, true) break;
+    case 4: B200_DEC_LINEAR(true, 0, false) break;
+    case 5: B200_DEC_LINEAR(true, 0, true) break;
+    case 6: B200_DEC_LINEAR(true, 1, false) break;
+    default: B200_DEC_LINEAR(true, 1, true) break;
+  }
+#undef B200_DEC_LINEAR
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(B200_LORA_ECUDA, "decode_linear_kernel launch: %s", cudaGetErrorString(e));
+  }
+  return B200_LORA_OK;
 }
 
 // ============================================================================ glue over planes
@@ -287,7 +353,6 @@ struct DecAttnArgs {
   const int64_t* slot_mapping;             // where the new token's k and v go (< 0: nowhere)
   __nv_bfloat16* out;                      // [T, Hq D]
   float scale;
-  int early;                               // everything before the launch pair of the projection is complete at the start
 };
 
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
@@ -317,7 +382,7 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
   const int kvh = blockIdx.x, req = blockIdx.y, group = a.Hq / a.Hk;
   griddep_launch_dependents();
   const uint32_t q_u32 = smem_u32(smem), k_u32 = q_u32 + 16 * kPitch, v_u32 = k_u32 + kChunk * kPitch;
-  if (!a.early) griddep_wait();
+  // (the cache rows of earlier steps were written before this chain of dependent launches began: see the header)
   const int ctx = a.context_lens[req];
   const int32_t* table = a.block_tables + (int64_t)req * a.max_blocks;
   const int n_old = max(ctx - 1, 0);  // tokens whose k and v are in the cache already
@@ -339,7 +404,7 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
     }
   };
   if (ctx > 0) load_chunk(0, min(ctx, kChunk));
-  if (a.early) griddep_wait();
+  griddep_wait();
 
   // ---- q, k, v of the new token
   int64_t pos = a.positions[req];
