@@ -94,6 +94,24 @@ int launch_generic_expand(void* y, int64_t y_ld, const void* tmp, int T_rows, co
 
 }  // namespace
 
+namespace {
+
+// Whether a bf16 batch is large enough for the prefill kernels (at least 11 us for the pair, the adapters read once per 128
+// rows) rather than the bucket kernel (3 to 5 us, the adapters read once per 16 rows): from 512 rows on, by the adapter bytes
+// that the bucket kernel would read. us per projection, bucket / prefill kernels, six prompts of different adapters: 1024-wide,
+// rank 32, 900 rows, qkv (16 MB) 6.7 / 13.5, gate_up (37 MB) 8.9 / 15.1, 1500 rows 11.5 / 13.8 and (61 MB) 18.6 / 20.4;
+// 2048-wide, rank 32, 900 rows, gate_up (59 MB) 19.0 / 19.1, 1500 rows (98 MB) 32.9 / 24.7, qkv (52 MB) 16.4 / 16.3; rank 64,
+// 900 rows, qkv (63 MB) 18.8 / 17.0, 1500 rows 33.2 / 19.3.
+constexpr int64_t kPrefillMinBytes = 50ll * 1000 * 1000;
+inline bool prefill_sized(int32_t T, const SliceTable& st, int32_t r_max, int32_t in_dim, bool expand) {
+  int64_t bytes = 0;
+  for (int s = 0; s < st.n; ++s)
+    if (st.out[s] > 0 || !expand) bytes += 2 * (int64_t)r_max * (in_dim + (expand ? st.out[s] : 0));
+  return T >= kSgmvAutoMinTokens && ceil_div_i(T, kBgmvTok) * bytes > kPrefillMinBytes;
+}
+
+}  // namespace
+
 extern "C" {
 
 int lora_b200_version(void) { return B200_LORA_ABI_VERSION; }
@@ -212,7 +230,7 @@ int lora_b200_decode_add_rmsnorm(void* normed, void* hidden_out, const float* pl
   if (!aligned16(normed) || !aligned16(hidden_out) || !aligned16(planes) || !aligned16(residual) || !aligned16(weight))
     return fail(B200_LORA_EUNSUPPORTED, "decode_add_rmsnorm: rows must be 16-byte aligned");
   using B = __nv_bfloat16;
-  return launch_dependent(decode_add_rmsnorm_kernel, "decode_add_rmsnorm_kernel", dim3((unsigned)T), round_up_i(hidden / 8, 32), 0,
+  return launch_dependent(decode_add_rmsnorm_kernel, "decode_add_rmsnorm_kernel", dim3((unsigned)T), round_up_i(hidden / 4, 32), 0,
                           static_cast<cudaStream_t>(stream), static_cast<B*>(normed), static_cast<B*>(hidden_out), planes, n_planes,
                           static_cast<const B*>(residual), static_cast<const B*>(weight), T, hidden, eps);
 }
@@ -221,7 +239,7 @@ int lora_b200_decode_silu_mul(void* out, const float* planes, int32_t n_planes, 
   if (T < 1 || intermediate < 8 || intermediate % 8 != 0) return fail(B200_LORA_EUNSUPPORTED, "decode_silu_mul: bad shape T=%d I=%d", T, intermediate);
   if (n_planes < 1 || n_planes > kDecMaxPlanes) return fail(B200_LORA_EINVAL, "decode_silu_mul: %d planes", n_planes);
   if (!out || !planes || !aligned16(out) || !aligned16(planes)) return fail(B200_LORA_EINVAL, "decode_silu_mul: null or misaligned pointer");
-  const int ctas = std::min(2 * 148, ceil_div_i(T * (intermediate / 8), 256));
+  const int ctas = std::min(4 * 148, ceil_div_i(T * (intermediate / 4), 256));
   return launch_dependent(decode_silu_mul_kernel, "decode_silu_mul_kernel", dim3((unsigned)ctas), 256, 0, static_cast<cudaStream_t>(stream),
                           static_cast<__nv_bfloat16*>(out), planes, n_planes, T, intermediate);
 }
@@ -435,7 +453,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     bp.kind = 0;
     bp.mode = 3;
     bp.token_to_slot = token_to_slot;
-    const bool decode_like = T < kSgmvAutoMinTokens || T < 32 * n_buckets;
+    const bool decode_like = T < 32 * n_buckets || !prefill_sized(T, st, r_max, in_dim, true);
     if (dtype == B200_LORA_BF16 && have_buckets &&
         (impl == B200_LORA_IMPL_BGMV || (impl == B200_LORA_IMPL_AUTO && decode_like)) && bgmv_supported(bp, nullptr))
       return bgmv_launch(bp, st_);
@@ -465,7 +483,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     // want request-contiguous rows: with bucket arrays at hand, fewer than 32 rows per bucket on
     // average means a decode-like batch (slots scattered over the rows) and goes to the bucket kernel.
     const bool scattered = bgmv_ok && T < 32 * n_buckets;
-    if (dtype == B200_LORA_BF16 && T >= kSgmvAutoMinTokens && !scattered && sgmv_supported(sp, nullptr) &&
+    if (dtype == B200_LORA_BF16 && !scattered && (!bgmv_ok ? T >= kSgmvAutoMinTokens : prefill_sized(T, st, r_max, in_dim, true)) && sgmv_supported(sp, nullptr) &&
         workspace != nullptr && workspace_bytes >= sgmv_workspace_bytes(T, n_act, r_max))
       impl = B200_LORA_IMPL_SGMV;
     else if (bgmv_ok && !(grouped_preferred(gp) && workspace != nullptr && workspace_bytes >= grouped_workspace_bytes(T, n_act, r_max) &&
@@ -547,22 +565,21 @@ int lora_b200_shrink_buckets(void* out, int32_t out_dtype, const void* x, int64_
   if (int rc = fill_slices(st, n_slices, a_slabs, nullptr, nullptr, nullptr, true, false)) return rc;
   cudaStream_t st_ = static_cast<cudaStream_t>(stream);
   // With bucket arrays: the shrink half of the fused decode kernel (same sums as the per-token kernel, which reads an
-  // adapter again for every row), except for long batches of contiguous rows, which the tensor-core shrink takes.
+  // adapter again for every row). Batches of prefill size go to the tensor-core shrink if their rows are contiguous: with
+  // bucket arrays the two are launched together and look for themselves (rows_scattered).
   const bool buckets = sorted_idx && slot_ids && counts && offsets && n_buckets > 0;
-  const bool contiguous = T >= kSgmvAutoMinTokens && !(buckets && T < 32 * n_buckets);
-  if (buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && !(dtype == B200_LORA_BF16 && out_dtype == B200_LORA_BF16 && contiguous)) {
-    BgmvProblem bp = {};
-    bp.y = nullptr; bp.y_ld = 8; bp.x = x; bp.x_ld = x_ld; bp.T = T; bp.in_dim = in_dim; bp.st = st; bp.S = S; bp.r_max = r_max;
-    for (int s = 0; s < st.n; ++s) bp.st.out[s] = 8;  // (no output columns here)
-    bp.rank_per_slot = nullptr; bp.scale_per_slot = nullptr;
-    bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets;
-    bp.n_buckets = n_buckets; bp.scaling = scaling; bp.mode = 1; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
-    bp.tmp_io = out; bp.io16 = out_dtype != B200_LORA_F32; bp.zero_rows = 1; bp.token_to_slot = token_to_slot;
-    if (aligned16(out) && bgmv_supported(bp, nullptr)) return bgmv_launch(bp, st_);
-  }
-  if (dtype == B200_LORA_BF16 && out_dtype == B200_LORA_BF16 && contiguous) {
+  BgmvProblem bp = {};
+  bp.y = nullptr; bp.y_ld = 8; bp.x = x; bp.x_ld = x_ld; bp.T = T; bp.in_dim = in_dim; bp.st = st; bp.S = S; bp.r_max = r_max;
+  for (int s = 0; s < st.n; ++s) bp.st.out[s] = 8;  // (no output columns here)
+  bp.rank_per_slot = nullptr; bp.scale_per_slot = nullptr;
+  bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets;
+  bp.n_buckets = n_buckets; bp.scaling = scaling; bp.mode = 1; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
+  bp.tmp_io = out; bp.io16 = out_dtype != B200_LORA_F32; bp.zero_rows = 1; bp.token_to_slot = token_to_slot;
+  const bool by_bucket = buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && aligned16(out) && bgmv_supported(bp, nullptr);
+  const bool prefill = by_bucket ? T >= 32 * n_buckets && prefill_sized(T, st, r_max, in_dim, false) : T >= kSgmvAutoMinTokens;
+  if (dtype == B200_LORA_BF16 && out_dtype == B200_LORA_BF16 && prefill) {
     // prefill-sized bf16 batches: the tensor-core shrink (rows without adapter are written as zeros, as the
-    // per-token kernel does); anything it does not take falls through to the per-token kernel
+    // per-token kernel does); anything it does not take falls through
     SgmvProblem sp;
     sp.y = nullptr; sp.y_ld = 0; sp.x = x; sp.x_ld = x_ld; sp.T = T; sp.in_dim = in_dim; sp.S = S; sp.r_max = r_max;
     sp.st = st; sp.scale_per_slot = nullptr; sp.token_to_slot = token_to_slot; sp.scaling = scaling;
@@ -571,9 +588,13 @@ int lora_b200_shrink_buckets(void* out, int32_t out_dtype, const void* x, int64_
       SgmvArgs sa;
       if (int rc = sgmv_prepare_tmp(sp, out, (uint64_t)st.n * T, true, false, &sm, &sa)) return rc;
       sa.zero_fill = 1;
-      return sgmv_launch_shrink(sm, sa, st_);
+      sa.gate = by_bucket ? 1 : 0;
+      const int rc = sgmv_launch_shrink(sm, sa, st_);
+      if (rc != B200_LORA_OK || !by_bucket) return rc;
+      bp.gate = 1;
     }
   }
+  if (by_bucket) return bgmv_launch(bp, st_);
 #define B200_SHRINK(TT)                                                                              \
   (out_dtype == B200_LORA_F32 && dtype != B200_LORA_F32)                                             \
       ? launch_generic_shrink<TT, float>(out, x, x_ld, T, in_dim, st, S, r_max, token_to_slot, scaling, st_) \
@@ -602,29 +623,25 @@ int lora_b200_expand_buckets(void* y, int64_t y_ld, const void* tmp, int32_t tmp
   for (int s = 0; s < st.n; ++s)
     if (y_ld < (int64_t)st.col[s] + st.out[s]) return fail(B200_LORA_EINVAL, "y_ld smaller than slice end");
   cudaStream_t st_ = static_cast<cudaStream_t>(stream);
+  // (as in the shrink: one of two launches for prefill-sized batches with bucket arrays)
   const bool buckets = sorted_idx && slot_ids && counts && offsets && n_buckets > 0;
-  const bool contiguous = T >= kSgmvAutoMinTokens && !(buckets && T < 32 * n_buckets);
-  if (buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) &&
-      !(dtype == B200_LORA_BF16 && tmp_dtype == B200_LORA_BF16 && add_inputs && contiguous)) {
-    bool dense = true;  // tmp is indexed by slice position
-    for (int s = 0; s < st.n; ++s) dense = dense && st.out[s] > 0;
-    BgmvProblem bp = {};
-    bp.y = y; bp.y_ld = y_ld; bp.x = nullptr; bp.x_ld = 32; bp.T = T; bp.in_dim = 32; bp.st = st; bp.S = S; bp.r_max = r_max;
-    bp.rank_per_slot = nullptr; bp.scale_per_slot = nullptr;
-    bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets;
-    bp.n_buckets = n_buckets; bp.scaling = 1.0f; bp.mode = 2; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
-    bp.tmp_io = const_cast<void*>(tmp); bp.io16 = tmp_dtype != B200_LORA_F32; bp.no_add = add_inputs ? 0 : 1;
-    if (dense && aligned16(tmp) && bgmv_supported(bp, nullptr)) return bgmv_launch(bp, st_);
-  }
-  if (dtype == B200_LORA_BF16 && tmp_dtype == B200_LORA_BF16 && add_inputs && contiguous) {
+  bool dense = true;  // no zero-width slice: tmp is indexed by slice position
+  for (int s = 0; s < st.n; ++s) dense = dense && st.out[s] > 0;
+  BgmvProblem bp = {};
+  bp.y = y; bp.y_ld = y_ld; bp.x = nullptr; bp.x_ld = 32; bp.T = T; bp.in_dim = 32; bp.st = st; bp.S = S; bp.r_max = r_max;
+  bp.rank_per_slot = nullptr; bp.scale_per_slot = nullptr;
+  bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets;
+  bp.n_buckets = n_buckets; bp.scaling = 1.0f; bp.mode = 2; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
+  bp.tmp_io = const_cast<void*>(tmp); bp.io16 = tmp_dtype != B200_LORA_F32; bp.no_add = add_inputs ? 0 : 1; bp.token_to_slot = token_to_slot;
+  const bool by_bucket = buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && dense && aligned16(tmp) && bgmv_supported(bp, nullptr);
+  const bool prefill = by_bucket ? T >= 32 * n_buckets && prefill_sized(T, st, r_max, 0, true) : T >= kSgmvAutoMinTokens;
+  if (dtype == B200_LORA_BF16 && tmp_dtype == B200_LORA_BF16 && add_inputs && prefill) {
     // prefill-sized bf16 batches: the tensor-core expand (reduce-add tile kernel when the slices tile the
     // columns they cover in 64-column units, run-based kernel otherwise)
     int first = -1;
     for (int s = 0; s < st.n; ++s)
       if (st.out[s] > 0 && (first < 0 || st.col[s] < first)) first = st.col[s];
-    bool dense = first >= 0;  // no zero-width slice in between: tmp is indexed by slice position
-    for (int s = 0; s < st.n; ++s) dense = dense && st.out[s] > 0;
-    if (dense && first % 8 == 0) {
+    if (dense && first >= 0 && first % 8 == 0) {
       SgmvProblem sp;
       sp.y = static_cast<char*>(y) + (size_t)first * 2; sp.y_ld = y_ld; sp.x = nullptr; sp.x_ld = 0; sp.T = T; sp.in_dim = 0;
       sp.S = S; sp.r_max = r_max; sp.st = st; sp.scale_per_slot = nullptr; sp.token_to_slot = token_to_slot; sp.scaling = 1.0f;
@@ -633,18 +650,24 @@ int lora_b200_expand_buckets(void* y, int64_t y_ld, const void* tmp, int32_t tmp
         SgmvMaps sm;
         SgmvArgs sa;
         if (int rc = sgmv_prepare_tmp(sp, const_cast<void*>(tmp), (uint64_t)st.n * T, false, true, &sm, &sa)) return rc;
+        sa.gate = by_bucket ? 1 : 0;
+        int rc;
         if (tc_expand_fast_path_ok(sa)) {
           int n_total = 0;
           for (int s = 0; s < sa.n; ++s) n_total = std::max(n_total, sa.col[s] + sa.out[s]);
           GemmMaps gm;
           GemmArgs ga;
-          if (int rc = tc_tile_prepare(sm, sa, nullptr, 0, n_total, nullptr, true, true, &gm, &ga, false, false)) return rc;
-          return tc_tile_launch(gm, ga, st_);
+          if (int rc2 = tc_tile_prepare(sm, sa, nullptr, 0, n_total, nullptr, true, true, &gm, &ga, false, false)) return rc2;
+          rc = tc_tile_launch(gm, ga, st_);
+        } else {
+          rc = sgmv_launch_expand(sm, sa, st_);
         }
-        return sgmv_launch_expand(sm, sa, st_);
+        if (rc != B200_LORA_OK || !by_bucket) return rc;
+        bp.gate = 1;
       }
     }
   }
+  if (by_bucket) return bgmv_launch(bp, st_);
 #define B200_EXPAND(TT)                                                                               \
   (tmp_dtype == B200_LORA_F32 && dtype != B200_LORA_F32)                                              \
       ? launch_generic_expand<TT, float>(y, y_ld, tmp, T, st, S, r_max, token_to_slot, add_inputs, st_) \

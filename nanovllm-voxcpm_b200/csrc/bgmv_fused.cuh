@@ -89,7 +89,8 @@ struct BgmvProblem {
   int io16 = 0;
   int zero_rows = 0;       // mode 1: rows without adapter are written as zeros (token_to_slot tells which)
   int no_add = 0;          // mode 2, kinds 1 and 2: y = delta in rows with an adapter instead of y += delta
-  const int32_t* token_to_slot = nullptr;  // mode 3: which rows have no adapter
+  int gate = 0;            // modes 1, 2: leave batches of contiguous rows to another kernel (rows_scattered)
+  const int32_t* token_to_slot = nullptr;  // modes 1 and 3: which rows have no adapter; gate
 };
 
 struct BgmvParams {
@@ -98,7 +99,8 @@ struct BgmvParams {
   SliceTable st;  // active slices only
   const int32_t* rank_per_slot; const float* scale_per_slot;
   const int32_t *sorted_idx, *slot_ids, *counts, *offsets;
-  int n_buckets, n_live; float scaling;  // n_live: clusters for first windows (a bucket each, or a bucket that holds rows each)
+  int n_buckets; float scaling;
+  int clusters, by_window;  // clusters of the launch; by_window: cluster i takes the i-th window of the batch
   int window;       // tokens per cluster (multiple of 16)
   int c_shift;      // cluster size C = 1 << c_shift
   int KP, nkp;      // columns per shrink tile (min(in, 1024)) and number of K parts
@@ -119,7 +121,7 @@ struct BgmvParams {
   int use_pdl;
   int mode;         // 0 fused, 1 shrink only (tmp_io written), 2 expand only (tmp_io read), 3 overwrite y
   void* tmp_io;
-  int io16, zero_rows, no_add;
+  int io16, zero_rows, no_add, gate;
   const int32_t* token_to_slot;
 };
 
@@ -184,33 +186,46 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   // reads index metadata and lora slabs, which no kernel of this library writes, so its weight
   // traffic overlaps this kernel's compute and keeps HBM busy across launch boundaries.
   if (p.use_pdl) griddep_launch_dependents();
+  if ((kMode == 1 || kMode == 2) && p.gate && !rows_scattered(p.token_to_slot, p.T)) {
+    if (p.use_pdl && block_y == 0 && c == 0) griddep_wait();
+    return;
+  }
   // ---- bucket metadata (uniform across the cluster); barrier set-up overlaps the loads
   // Extra cluster e looks after multiple m = (e + 1) * window of the window inside the sorted rows: if m lies behind the
   // first row of a bucket [start, start + cnt), it is the i-th such multiple there, and the cluster takes the bucket's i-th
   // window. (A bucket of cnt rows has ceil(cnt / window) - 1 windows beyond its first and at least that many multiples.)
   int window_no = 0;
-  if (bucket < p.n_live) {
-    // Fewer rows than buckets (graph buffers carry a bucket for every slot): the launch has a cluster per row, and cluster i
-    // takes the i-th bucket that holds rows. (A cluster per bucket cost 64 rows over 128 adapters two waves of idle CTAs.)
-    if (p.n_live < p.n_buckets) {
-      int seen = 0;
-      bucket = -1;
-      for (int b0 = 0; b0 < p.n_buckets && bucket < 0; b0 += 128) {
-        int held[4];
+  if (p.by_window) {
+    // Fewer rows than buckets (graph buffers carry a bucket for every slot): the launch has a cluster for every window that T
+    // rows can make, and cluster i takes the i-th one. (A cluster per bucket cost 64 rows over 128 adapters two waves of CTAs
+    // that only found no rows.)
+    int seen = 0;
+    bucket = -1;
+    for (int b0 = 0; b0 < p.n_buckets && bucket < 0; b0 += 128) {
+      int held[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) held[i] = b0 + 32 * i + lane < p.n_buckets ? p.counts[b0 + 32 * i + lane] : 0;
+      for (int i = 0; i < 4; ++i) held[i] = b0 + 32 * i + lane < p.n_buckets ? p.counts[b0 + 32 * i + lane] : 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const unsigned live = __ballot_sync(0xffffffffu, held[i] > 0);
-          const unsigned mine = __ballot_sync(0xffffffffu, held[i] > 0 && seen + __popc(live & ((1u << lane) - 1u)) == block_y);
-          if (mine != 0) bucket = b0 + 32 * i + __ffs((int)mine) - 1;
-          seen += __popc(live);
+      for (int i = 0; i < 4; ++i) {
+        const int windows = held[i] > 0 && held[i] <= p.T ? (held[i] + p.window - 1) / p.window : 0;
+        int upto = windows;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+          const int v = __shfl_up_sync(0xffffffffu, upto, d);
+          if (lane >= d) upto += v;
         }
+        const int first = seen + upto - windows;
+        const unsigned mine = __ballot_sync(0xffffffffu, block_y >= first && block_y < first + windows);
+        if (mine != 0) {
+          bucket = b0 + 32 * i + __ffs((int)mine) - 1;
+          window_no = block_y - __shfl_sync(0xffffffffu, first, __ffs((int)mine) - 1);
+        }
+        seen = __shfl_sync(0xffffffffu, seen + upto, 31);
       }
     }
-  } else {
+  } else if (bucket >= p.n_buckets) {
     volatile int* owner = reinterpret_cast<volatile int*>(smem + p.off_bar + 8 * (2 * kBgmvMaxStages + 2)) + 1;  // behind the abort flag
-    const int m = (bucket - p.n_live + 1) * p.window;
+    const int m = (bucket - p.n_buckets + 1) * p.window;
     if (tid == 0) *owner = -1;
     __syncthreads();
     for (int b = tid; b < p.n_buckets; b += kBgmvThreads) {
@@ -885,7 +900,7 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
     for (int s = 0; s < st.n; ++s) bucket_bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + st.out[s]);
     while (C < 4 && (bucket_bytes / C > 512 * 1024 || (bucket_bytes / C > 256 * 1024 && in_use * C * 2 <= resident))) C *= 2;
     const double clusters = in_use + (b.T - 1) / kBgmvTok;
-    if (C == 4 && ((bucket_bytes / 4 > 128 * 1024 && clusters * 8 <= resident) || (bucket_bytes / 4 >= 256 * 1024 && in_use * 8 <= resident))) C = 8;
+    if (C == 4 && ((bucket_bytes / 4 > 128 * 1024 && clusters * 8 <= resident && b.beside == 0) || (bucket_bytes / 4 >= 256 * 1024 && in_use * 8 <= resident))) C = 8;
   }
   // K split: at least one K part (1024 columns) per CTA of the cluster and all rank rows in one CTA;
   // the shrink-only / expand-only pair of the tensor-parallel exchange keeps the row split
@@ -899,12 +914,17 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
 
   BgmvParams p;
   p.window = kBgmvTok;
+  // (a bucket of n rows has 1 + (n - 1) / window windows, the most with as many buckets in use as there are rows)
+  const int in_use_max = std::min(b.n_buckets, std::max(b.T, 1));
+  p.clusters = b.n_buckets + (b.T - 1) / p.window;
+  p.by_window = in_use_max + (b.T - in_use_max) / p.window < p.clusters && in_use_max < b.n_buckets ? 1 : 0;
+  if (p.by_window) p.clusters = in_use_max + (b.T - in_use_max) / p.window;
   p.y = static_cast<__nv_bfloat16*>(b.y); p.y_ld = b.y_ld;
   p.x = static_cast<const __nv_bfloat16*>(b.x); p.x_ld = b.x_ld;
   p.T = b.T; p.in_dim = b.in_dim; p.S = b.S; p.r_max = b.r_max; p.st = st;
   p.rank_per_slot = b.rank_per_slot; p.scale_per_slot = b.scale_per_slot;
   p.sorted_idx = b.sorted_idx; p.slot_ids = b.slot_ids; p.counts = b.counts; p.offsets = b.offsets;
-  p.n_buckets = b.n_buckets; p.n_live = std::min(b.n_buckets, std::max(b.T, 1)); p.scaling = b.scaling;
+  p.n_buckets = b.n_buckets; p.scaling = b.scaling;
   p.c_shift = log2_exact(C);
   p.KP = std::min(b.in_dim, kBgmvKP);
   p.nkp = ceil_div_i(b.in_dim, p.KP);
@@ -955,7 +975,7 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   for (int s = 0; s < st.n; ++s) p.y_cols = std::max(p.y_cols, st.col[s] + st.out[s]);
   p.use_pdl = bgmv_options().pdl ? 1 : 0;
   p.mode = b.mode;
-  p.tmp_io = b.tmp_io; p.io16 = b.io16; p.zero_rows = b.zero_rows; p.no_add = b.no_add;
+  p.tmp_io = b.tmp_io; p.io16 = b.io16; p.zero_rows = b.zero_rows; p.no_add = b.no_add; p.gate = b.gate;
   p.token_to_slot = b.token_to_slot;
   if ((b.mode == 1 || b.mode == 2) && b.tmp_io == nullptr) { *why = "shrink-only / expand-only need the tmp array"; return false; }
   if (b.mode == 3 && b.token_to_slot == nullptr) { *why = "overwrite mode needs token_to_slot"; return false; }
@@ -987,7 +1007,7 @@ inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
     configured_device = dev;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(1u << p.c_shift, (unsigned)(p.n_live + (p.T - 1) / p.window), 1);
+  cfg.gridDim = dim3(1u << p.c_shift, (unsigned)p.clusters, 1);
   cfg.blockDim = dim3(kBgmvThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;

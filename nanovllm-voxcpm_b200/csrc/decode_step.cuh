@@ -125,7 +125,6 @@ __device__ __forceinline__ void decode_gemm_body(const DecGemmMaps& maps, const 
     umma_commit_elected(acc_full, leader);
   } else if (warp >= 4 && warp < 8) {
     const int quarter = warp & 3, o = row0 + quarter * 32 + lane;
-    float* dst = a.part + (int64_t)part * a.T * a.out + o;
     griddep_wait();  // the previous launch may still read the planes
     if (a.delta != nullptr && part == 0) {  // (32 rows at a time: one by one the lookups took 12 us)
       for (int t0 = 0; t0 < a.T; t0 += 32) {
@@ -140,15 +139,23 @@ __device__ __forceinline__ void decode_gemm_body(const DecGemmMaps& maps, const 
     }
     mbar_wait_bounded(acc_full, 0u, &abort_flag);
     tc_fence_after_sync();
+    // Through shared memory (the ring is free: every MMA has read it), then one bulk copy per token: with a store per thread
+    // and token the 64 tokens of a tile took 2.8 us.
     for (int c = 0; c < a.T; c += 16) {
       uint32_t v[16];
       tmem_ld_32x16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c, v);
       tmem_ld_wait();
-      if (o < a.out) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e)
-          if (c + e < a.T) dst[(int64_t)(c + e) * a.out] = __uint_as_float(v[e]);
-      }
+      for (int e = 0; e < 16; ++e)  // (the rows up to n_pad exist in the ring)
+        sts32(smem_base + (uint32_t)((c + e) * 512 + (quarter * 32 + lane) * 4), v[e]);
+    }
+    fence_proxy_async_smem();
+    named_bar_sync(2, 128);
+    const int token = tid - 128;
+    if (token < a.T) {
+      bulk_s2g(a.part + ((int64_t)part * a.T + token) * a.out + row0, smem_base + (uint32_t)token * 512u, (uint32_t)min(128, a.out - row0) * 4u);
+      bulk_commit_group();
+      bulk_wait_all();
     }
     tc_fence_before_sync();
   }
@@ -226,7 +233,7 @@ inline int decode_linear_launch(float* planes, const void* x, int64_t x_ld, int 
   smem = std::max(smem, (size_t)p.off_bar + 256);
   const int C = 1 << p.c_shift, gemm_rows = ceil_div_i(a.tiles * a.parts, C);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)C, (unsigned)(gemm_rows + p.n_live + (T - 1) / p.window), 1);
+  cfg.gridDim = dim3((unsigned)C, (unsigned)(gemm_rows + p.clusters), 1);
   cfg.blockDim = dim3(kBgmvThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -264,72 +271,89 @@ inline int decode_linear_launch(float* planes, const void* x, int64_t x_ld, int 
 }
 
 // ============================================================================ glue over planes
-// Eight consecutive columns of a row of a projection's result: the planes [planes, T, ld] added in fp32.
-__device__ __forceinline__ void planes_load8(const float* part, int planes, int64_t plane, int64_t at, float (&v)[8]) {
+// Four consecutive columns of a row of a projection's result, N of them: the planes [planes, T, ld] added in fp32. All loads
+// of a thread are issued before the first sum waits, hence the unrolled forms (up to kP planes; the last plane is read again
+// in place of the missing ones and left out of the sum).
+template <int N, int kP>
+__device__ __forceinline__ void planes_load4_upto(const float* part, int planes, int64_t plane, const int64_t (&at)[N], float (&v)[N][4]) {
+  float4 got[kP][N];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) v[e] = 0.f;
+  for (int p = 0; p < kP; ++p)
 #pragma unroll
-  for (int p = 0; p < kDecMaxPlanes; ++p) {
-    if (p < planes) {
-      const float4* src = reinterpret_cast<const float4*>(part + p * plane + at);
-      const float4 a = __ldcg(src), b = __ldcg(src + 1);
-      v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-      v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+    for (int n = 0; n < N; ++n) got[p][n] = __ldcg(reinterpret_cast<const float4*>(part + min(p, planes - 1) * plane + at[n]));
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    v[n][0] = v[n][1] = v[n][2] = v[n][3] = 0.f;
+#pragma unroll
+    for (int p = 0; p < kP; ++p) {
+      const bool live = p < planes;
+      v[n][0] += live ? got[p][n].x : 0.f; v[n][1] += live ? got[p][n].y : 0.f;
+      v[n][2] += live ? got[p][n].z : 0.f; v[n][3] += live ? got[p][n].w : 0.f;
     }
   }
 }
+template <int N>
+__device__ __forceinline__ void planes_load4(const float* part, int planes, int64_t plane, const int64_t (&at)[N], float (&v)[N][4]) {
+  if (planes <= 2) planes_load4_upto<N, 2>(part, planes, plane, at, v);
+  else if (planes == 3) planes_load4_upto<N, 3>(part, planes, plane, at, v);
+  else if (planes <= 5) planes_load4_upto<N, 5>(part, planes, plane, at, v);
+  else planes_load4_upto<N, kDecMaxPlanes>(part, planes, plane, at, v);
+}
+__device__ __forceinline__ uint2 pack4(const float (&v)[4]) { return make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])); }
+__device__ __forceinline__ void unpack4(uint2 r, float (&v)[4]) {
+  const float2 a = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&r.x)), b = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&r.y));
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
 
-// hidden_out = residual + sum of planes (bf16); normed = rms_norm(hidden_out) * weight. One CTA per row, one 8-column vector per
+// hidden_out = residual + sum of planes (bf16); normed = rms_norm(hidden_out) * weight. One CTA per row, four columns per
 // thread: a row's loads are all in flight at once.
-__global__ void __launch_bounds__(512) decode_add_rmsnorm_kernel(__nv_bfloat16* __restrict__ normed, __nv_bfloat16* hidden_out,
-                                                                 const float* part, int planes, const __nv_bfloat16* residual,
-                                                                 const __nv_bfloat16* __restrict__ weight, int T, int H, float eps) {
-  __shared__ float sums[16];
+__global__ void __launch_bounds__(1024) decode_add_rmsnorm_kernel(__nv_bfloat16* __restrict__ normed, __nv_bfloat16* hidden_out,
+                                                                  const float* part, int planes, const __nv_bfloat16* residual,
+                                                                  const __nv_bfloat16* __restrict__ weight, int T, int H, float eps) {
+  __shared__ float sums[32];
   griddep_launch_dependents();
-  const int row = blockIdx.x, v8 = threadIdx.x * 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  Vec8<__nv_bfloat16> w, res, h;
-  const bool live = v8 < H;
-  if (live) w.raw = *reinterpret_cast<const uint4*>(weight + v8);
+  const int row = blockIdx.x, col = threadIdx.x * 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float w[4], res[4], v[1][4], ss = 0.f;
+  const bool live = col < H;
+  if (live) unpack4(*reinterpret_cast<const uint2*>(weight + col), w);
   griddep_wait();
-  float v[8], ss = 0.f;
   if (live) {
-    res.raw = *reinterpret_cast<const uint4*>(residual + (int64_t)row * H + v8);
-    planes_load8(part, planes, (int64_t)T * H, (int64_t)row * H + v8, v);
+    const int64_t at[1] = {(int64_t)row * H + col};
+    const uint2 old = *reinterpret_cast<const uint2*>(residual + at[0]);
+    planes_load4<1>(part, planes, (int64_t)T * H, at, v);
+    unpack4(old, res);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      h.set(e, res.get(e) + v[e]);
-      v[e] = h.get(e);  // the norm sees the rounded sum
-      ss += v[e] * v[e];
-    }
-    *reinterpret_cast<uint4*>(hidden_out + (int64_t)row * H + v8) = h.raw;
+    for (int e = 0; e < 4; ++e) v[0][e] += res[e];
+    const uint2 sum = pack4(v[0]);
+    *reinterpret_cast<uint2*>(hidden_out + at[0]) = sum;
+    unpack4(sum, v[0]);  // the norm sees the rounded sum
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ss += v[0][e] * v[0][e];
   }
   ss = warp_sum(ss);
   if (lane == 0) sums[warp] = ss;
   __syncthreads();
-  ss = 0.f;
-  for (int i = 0; i < (int)(blockDim.x >> 5); ++i) ss += sums[i];
+  ss = warp_sum(lane < (int)(blockDim.x >> 5) ? sums[lane] : 0.f);
   if (!live) return;
   const float rstd = rsqrtf(ss / (float)H + eps);
 #pragma unroll
-  for (int e = 0; e < 8; ++e) h.set(e, v[e] * rstd * w.get(e));
-  *reinterpret_cast<uint4*>(normed + (int64_t)row * H + v8) = h.raw;
+  for (int e = 0; e < 4; ++e) v[0][e] *= rstd * w[e];
+  *reinterpret_cast<uint2*>(normed + (int64_t)row * H + col) = pack4(v[0]);
 }
 
 // out = silu(gate) * up of the summed planes [planes, T, 2 I]
 __global__ void __launch_bounds__(256) decode_silu_mul_kernel(__nv_bfloat16* __restrict__ out, const float* part, int planes, int T, int I) {
   griddep_launch_dependents();
   griddep_wait();
-  const int nvec = I >> 3, total = T * nvec;
+  const int nvec = I >> 2, total = T * nvec;
   for (int i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
-    const int row = i / nvec, v8 = (i - row * nvec) * 8;
-    float g[8], u[8];
-    const int64_t at = (int64_t)row * 2 * I + v8;
-    planes_load8(part, planes, (int64_t)T * 2 * I, at, g);
-    planes_load8(part, planes, (int64_t)T * 2 * I, at + I, u);
-    Vec8<__nv_bfloat16> o;
+    const int row = i / nvec, col = (i - row * nvec) * 4;
+    float v[2][4], o[4];
+    const int64_t gate = (int64_t)row * 2 * I + col, at[2] = {gate, gate + I};
+    planes_load4<2>(part, planes, (int64_t)T * 2 * I, at, v);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) o.set(e, g[e] / (1.f + expf(-g[e])) * u[e]);
-    *reinterpret_cast<uint4*>(out + (int64_t)row * I + v8) = o.raw;
+    for (int e = 0; e < 4; ++e) o[e] = v[0][e] / (1.f + expf(-v[0][e])) * v[1][e];
+    *reinterpret_cast<uint2*>(out + (int64_t)row * I + col) = pack4(o);
   }
 }
 
@@ -367,7 +391,7 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint3
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <int D>
-__host__ __device__ constexpr int dec_attn_chunk() { return D == 64 ? 384 : 192; }  // tokens in shared memory at a time (two CTAs per SM)
+__host__ __device__ constexpr int dec_attn_chunk() { return D == 64 ? 368 : 192; }  // tokens in shared memory at a time (two CTAs per SM)
 template <int D>
 __host__ __device__ constexpr int dec_attn_smem() {
   const int kv = 2 * dec_attn_chunk<D>() * (D * 2 + 16), merge = kDecAttnWarps * 16 * (D + 2) * 4;
@@ -376,7 +400,7 @@ __host__ __device__ constexpr int dec_attn_smem() {
 
 template <int D>
 __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const DecAttnArgs a) {
-  extern __shared__ __align__(128) uint8_t smem[];
+  extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int kPitch = D * 2 + 16, kChunk = dec_attn_chunk<D>(), kHalf = D / 2;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int kvh = blockIdx.x, req = blockIdx.y, group = a.Hq / a.Hk;
@@ -386,27 +410,36 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
   const int ctx = a.context_lens[req];
   const int32_t* table = a.block_tables + (int64_t)req * a.max_blocks;
   const int n_old = max(ctx - 1, 0);  // tokens whose k and v are in the cache already
+  __shared__ int64_t cache_row[kChunk];
 
   // rows [c0, c0 + n) of the cache into the chunk buffers; the last row of all is the new token's (written below), rows up
   // to the next multiple of 16 are zero (their probabilities are zero, their values must be finite)
   auto load_chunk = [&](int c0, int n) {
     const int rows = (n + 15) & ~15;
     constexpr int kPieces = D / 8;
-    for (int i = tid; i < rows * kPieces; i += kDecAttnThreads) {
-      const int r = i / kPieces, p = i - r * kPieces, tok = c0 + r;
-      if (tok == n_old && r < n) continue;
+    // where each row lies first (a look-up and a division per row, not per piece: those took 4 us)
+    for (int r = tid; r < n; r += kDecAttnThreads) {
+      const int tok = c0 + r;
+      const int blk = table[tok / a.block_size];
+      cache_row[r] = blk * (int64_t)a.block_size + tok % a.block_size;
+    }
+    __syncthreads();
+    const int p = tid % kPieces;
+    const uint32_t off0 = (uint32_t)(p * 16);
+    const int64_t at0 = (int64_t)kvh * D + p * 8, row_ld = (int64_t)a.Hk * D;
+#pragma unroll 4
+    for (int r = tid / kPieces; r < rows; r += kDecAttnThreads / kPieces) {
+      if (c0 + r == n_old && r < n) continue;
       const bool live = r < n;
-      int64_t at = 0;
-      if (live) at = ((int64_t)table[tok / a.block_size] * a.block_size + tok % a.block_size) * a.Hk * D + (int64_t)kvh * D + p * 8;
-      const uint32_t off = (uint32_t)(r * kPitch + p * 16);
+      const int64_t at = live ? cache_row[r] * row_ld + at0 : 0;
+      const uint32_t off = (uint32_t)(r * kPitch) + off0;
       cp_async_16(k_u32 + off, a.k_cache + at, live ? 16u : 0u);
       cp_async_16(v_u32 + off, a.v_cache + at, live ? 16u : 0u);
     }
   };
   if (ctx > 0) load_chunk(0, min(ctx, kChunk));
-  griddep_wait();
 
-  // ---- q, k, v of the new token
+  // ---- q, k, v of the new token: a thread takes four pairs (j, j + D / 2) of a head
   int64_t pos = a.positions[req];
   pos = pos < 0 ? 0 : (pos >= a.max_pos ? a.max_pos - 1 : pos);
   const int64_t slot = a.slot_mapping[req];
@@ -416,27 +449,36 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
   uint8_t* const v_new = k_new + kChunk * kPitch;
   const bool new_in_first = n_old < kChunk;
   __shared__ __align__(16) __nv_bfloat16 kv_new[2][D];
-  for (int i = tid; i < (group + 2) * kHalf; i += kDecAttnThreads) {
-    const int head = i / kHalf, j = i - head * kHalf;  // heads 0 .. group - 1: q; group: k; group + 1: v
-    const int64_t col = head < group ? (int64_t)(kvh * group + head) * D : (int64_t)(a.Hq + (head - group) * a.Hk + kvh) * D;
-    float x1 = 0.f, x2 = 0.f;
+  bool waited = false;
+  for (int i = tid; i < (group + 2) * (kHalf / 4) || !waited; i += kDecAttnThreads) {
+    const int head = i / (kHalf / 4), j = (i - head * (kHalf / 4)) * 4;  // heads 0 .. group - 1: q; group: k; group + 1: v
+    const bool item = head < group + 2, turned = head <= group;
+    float c1[4], s1[4], c2[4], s2[4];
 #pragma unroll
-    for (int p = 0; p < kDecMaxPlanes; ++p) {
-      if (p < a.planes) {
-        x1 += __ldcg(a.part + p * plane + row_at + col + j);
-        x2 += __ldcg(a.part + p * plane + row_at + col + kHalf + j);
+    for (int e = 0; e < 4; ++e) {
+      c1[e] = c2[e] = 1.f;
+      s1[e] = s2[e] = 0.f;
+      if (turned) {
+        const int64_t tb = pos * a.table_dim + j + e;
+        c1[e] = table_at(a.cos, a.table_dtype, tb); s1[e] = table_at(a.sin, a.table_dtype, tb);
+        c2[e] = table_at(a.cos, a.table_dtype, tb + hi_off); s2[e] = table_at(a.sin, a.table_dtype, tb + hi_off);
       }
     }
-    if (head <= group) {
-      const int64_t tb = pos * a.table_dim + j;
-      const float c1 = table_at(a.cos, a.table_dtype, tb), s1 = table_at(a.sin, a.table_dtype, tb);
-      const float c2 = table_at(a.cos, a.table_dtype, tb + hi_off), s2 = table_at(a.sin, a.table_dtype, tb + hi_off);
-      const float y1 = __fadd_rn(__fmul_rn(x1, c1), __fmul_rn(-x2, s1)), y2 = __fadd_rn(__fmul_rn(x2, c2), __fmul_rn(x1, s2));
-      x1 = y1; x2 = y2;
+    if (!waited) griddep_wait();  // (tables, positions and the cache do not depend on the launches ahead)
+    waited = true;
+    if (!item) break;
+    const int64_t col = head < group ? (int64_t)(kvh * group + head) * D : (int64_t)(a.Hq + (head - group) * a.Hk + kvh) * D;
+    const int64_t at[2] = {row_at + col + j, row_at + col + kHalf + j};
+    float x[2][4], lo[4], hi[4];
+    planes_load4<2>(a.part, a.planes, plane, at, x);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      lo[e] = turned ? __fadd_rn(__fmul_rn(x[0][e], c1[e]), __fmul_rn(-x[1][e], s1[e])) : x[0][e];
+      hi[e] = turned ? __fadd_rn(__fmul_rn(x[1][e], c2[e]), __fmul_rn(x[0][e], s2[e])) : x[1][e];
     }
     __nv_bfloat16* dst = head < group ? reinterpret_cast<__nv_bfloat16*>(smem + head * kPitch) : kv_new[head - group];
-    dst[j] = __float2bfloat16_rn(x1);
-    dst[kHalf + j] = __float2bfloat16_rn(x2);
+    *reinterpret_cast<uint2*>(dst + j) = pack4(lo);
+    *reinterpret_cast<uint2*>(dst + kHalf + j) = pack4(hi);
   }
   for (int i = tid; i < (16 - group) * D; i += kDecAttnThreads)  // unused rows of the q tile
     reinterpret_cast<__nv_bfloat16*>(smem + (group + i / D) * kPitch)[i % D] = __float2bfloat16_rn(0.f);

@@ -57,6 +57,7 @@ struct GemmArgs {
   //     GEMM of the first tiles, overlap it.
   // 0 = unknown predecessor: the first load of anything waits.
   int after_shrink;
+  int gate;                        // leave batches of scattered rows to another kernel (rows_scattered)
   __nv_bfloat16* y; int64_t y_ld;  // plain view of the output beside its tensor map (L2 prefetch of the rows a reduce-add will touch)
 };
 
@@ -141,6 +142,10 @@ tc_tile_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a) {
   // the next kernel of the stream, if it was launched as a programmatic dependent (this library's shrink and decode
   // kernels are), may set itself up now; those kernels wait for this one before they touch activations or scratch
   griddep_launch_dependents();
+  if (a.gate && rows_scattered(a.token_to_slot, a.T)) {
+    griddep_wait();
+    return;
+  }
   // Persistent schedule: the output tiles, numbered row block major (id = blk * ntile_all + j), are
   // dealt to the CTAs in equal contiguous ranges, so every SM gets the same number of tiles and a CTA
   // changes row block at most kTileMaxSeg - 1 times.
@@ -465,7 +470,7 @@ inline int tc_tile_prepare(const SgmvMaps& sm, const SgmvArgs& sa, const void* w
   a.expand_mode = expand_mode ? 1 : 0;
   a.lora = lora ? 1 : 0;
   a.overwrite = overwrite ? 1 : 0;
-  a.y = sa.y; a.y_ld = sa.y_ld;
+  a.y = sa.y; a.y_ld = sa.y_ld; a.gate = sa.gate;
   a.after_shrink = (lora && after_shrink) ? 1 : 0;  // the caller has just launched the shrink that writes tmp (else: unknown predecessor)
   maps->x = sm.x; maps->t = sm.t;
   for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) maps->b[s] = sm.b[s];

@@ -35,6 +35,7 @@ struct SgmvArgs {
   const float* scale_per_slot; float scaling;
   int zero_fill;                            // shrink: write zero rows for tokens without adapter
   int skip_clean;                           // expand: leave blocks in which every row has an adapter to tc_tile_kernel
+  int gate;                                 // leave batches of scattered rows to another kernel (rows_scattered)
   int shrink_gmax;                          // shrink: runs of a block whose K loops share one pass over x (set by the launch)
   int shrink_ring_bytes;                    // shrink: bytes of the TMA ring (set by the launch)
   int shrink_ck;                            // shrink: CTAs of a cluster = parts of K (set by the launch)
@@ -131,6 +132,10 @@ sgmv_shrink_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
   const int blk = (int)blockIdx.x / CK;
   const int r = a.r_max, n = a.n, width = n * r;
   B200_SHRINK_TRACE_CTA(0)
+  if (a.gate && rows_scattered(a.token_to_slot, a.T)) {
+    griddep_wait();
+    return;
+  }
   const uint32_t a_tile_bytes = (uint32_t)r * kSgmvBK * 2;
   const uint32_t x_tile_bytes = kSgmvBM * kSgmvBK * 2;
   const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;  // swizzled tiles need 1024-byte alignment
@@ -353,6 +358,7 @@ sgmv_expand_kernel(const __grid_constant__ SgmvMaps maps, const SgmvArgs a) {
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int blk = blockIdx.x, z = blockIdx.y, Z = gridDim.y;
+  if (a.gate && rows_scattered(a.token_to_slot, a.T)) return;
   const int r = a.r_max, n = a.n;
   const uint32_t t_tile_bytes = (uint32_t)kSgmvBM * r * 2;
   const uint32_t b_tile_bytes = (uint32_t)kSgmvBN * r * 2;
@@ -537,7 +543,7 @@ inline int sgmv_prepare_tmp(const SgmvProblem& b, void* tmp, uint64_t tmp_rows, 
   a.tmp = static_cast<__nv_bfloat16*>(tmp);
   a.T = b.T; a.in_dim = b.in_dim; a.S = b.S; a.r_max = b.r_max;
   a.token_to_slot = b.token_to_slot; a.scale_per_slot = b.scale_per_slot; a.scaling = b.scaling;
-  a.zero_fill = 0;
+  a.zero_fill = a.gate = 0;
   if (int rc = make_tmap_2d(&maps->t, a.tmp, tmp_rows, (uint64_t)b.r_max, (uint64_t)b.r_max, kSgmvBM, (uint32_t)b.r_max)) return rc;
   if (with_x) {
     if (int rc = make_tmap_2d(&maps->x, b.x, (uint64_t)b.T, (uint64_t)b.in_dim, (uint64_t)b.x_ld, kSgmvBM, kSgmvBK)) return rc;

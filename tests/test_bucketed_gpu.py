@@ -102,3 +102,28 @@ def test_operators_with_bucket_arrays_match_oracle(case, dtype):
         assert_lora_close(y2, want, what="expand, overwriting")
         assert not y2.cpu()[:, : p.col_offsets[k]].any()
     assert N.device_status(reset=True) == 0
+
+
+@pytest.mark.parametrize("contiguous", [True, False], ids=["prompts", "scattered"])
+def test_operators_choose_the_kernel_by_the_order_of_the_rows(contiguous):
+    """Batches of prefill size, where each call launches a kernel for contiguous and one for scattered rows and one of them does
+    the work: once, whatever the order."""
+    T, outs, S, r = 1100, [2048, 2048, 2048], 4, 64
+    slots = None
+    if contiguous:
+        slots = torch.repeat_interleave(torch.tensor([2, -1, 0, 3, 2], dtype=torch.int32), torch.tensor([300, 129, 1, 500, 170]))
+    p = W.make_projection(400, T, 2048, outs, S, r, token_to_slot=slots)
+    d = p.to_device(DEV)
+    km = LoRAKernelMeta.make(S, T, DEV)
+    km.prepare_tensors(d.token_to_slot)
+    args = km.meta_args(T, specialize_active_lora=True)
+    tmp = torch.full((3, T, r), 3.0, device=DEV, dtype=torch.bfloat16)
+    lora_shrink(d.x, d.a_slabs, tmp, *args, 0.5)
+    assert_lora_close(tmp, O.shrink(p.x, p.a_slabs, p.token_to_slot, 0.5), what="shrink")
+    y = d.y.clone()
+    lora_expand(tmp, d.b_slabs, y, *args, offset_start=0, add_inputs=True)
+    assert_lora_close(y, O.expand(p.y, tmp.float().cpu(), p.b_slabs, p.token_to_slot), what="expand")
+    none = p.token_to_slot < 0
+    assert not tmp.cpu()[:, none].any()
+    assert torch.equal(y.cpu()[none].view(torch.int16), p.y[none].view(torch.int16))
+    assert N.device_status(reset=True) == 0
