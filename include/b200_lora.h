@@ -370,6 +370,16 @@ int lora_b200_debug_trace(long long* out, int32_t n_values);
 #endif
 
 /*
+ * Causal attention over packed prompts: q | k | v are the columns of qkv [T, (num_heads + 2 num_kv_heads) * head_dim] (bf16,
+ * rotated already), prompt i the rows [cu_seqlens[i], cu_seqlens[i + 1]), none longer than max_seqlen; out [T, num_heads *
+ * head_dim]. head_dim 64 or 128. Counterpart in the reference: flash_attn_varlen_func in Attention.forward
+ * (nanovllm_voxcpm/layers/attention.py:70-79).
+ */
+int lora_b200_prefill_attention(void* out, int64_t out_ld, const void* qkv, int64_t qkv_ld, int32_t T, int32_t num_heads,
+                                int32_t num_kv_heads, int32_t head_dim, const int32_t* cu_seqlens, int32_t n_seqs,
+                                int32_t max_seqlen, float scale, void* stream);
+
+/*
  * A decode step's layer chain for small batches (bf16, T <= 128): the result of a projection is left as fp32 planes
  * [n, T, out] that its consumer adds up - the K parts of the base product and, last, the LoRA delta - so that base product
  * and delta run side by side and no pass reads or rounds the sum in between. Counterpart in the reference: F.linear + add_lora

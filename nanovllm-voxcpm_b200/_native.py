@@ -92,6 +92,10 @@ _SIGNATURES = {
     ),
     "lora_b200_glue_silu_mul": (c_int32, [c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32, c_int32, c_void_p]),
     "lora_b200_decode_planes": (c_int32, [c_int32, c_int32]),
+    "lora_b200_prefill_attention": (
+        c_int32,
+        [c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32, c_int32, c_int32, c_void_p, c_int32, c_int32, c_float, c_void_p],
+    ),
     "lora_b200_decode_linear": (
         c_int32,
         [c_void_p, c_void_p, c_int64, c_int32, c_int32, c_void_p, c_int64, c_int32, c_int32, POINTER(c_void_p), POINTER(c_void_p),

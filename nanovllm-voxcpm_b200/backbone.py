@@ -280,8 +280,47 @@ class Decoder(nn.Module):
                 add_norm(linear(layer.mlp.down_proj, act), following)
         return normed
 
+    def _prefill_native(self, embeds, positions, step: AttentionStep) -> torch.Tensor | None:
+        """An eager prefill step through ``prefill_layers`` (``csrc/binding.cpp``): the launches of all layers in one call. None
+        for steps and layers that it does not cover (decode rows in the batch, tensor parallelism, biases, other types)."""
+        cfg = self.cfg
+        if not step.is_prefill or step.n_decode or step.cu_seqlens is None or embeds.dtype != torch.bfloat16:
+            return None
+        backend = LORA.get_backend()
+        if not isinstance(backend, LORA.B200LoRABackend) or backend.impl != N.IMPL_AUTO or L.FUSED_LINEAR or L.LORA_FIRST:
+            return None
+        ctx = get_lora_context()
+        if ctx.parts:
+            return None
+        capture = torch.cuda.is_current_stream_capturing()
+        with_lora = ctx.token_to_slot is not None and not ctx.no_lora_flag
+        if with_lora and ctx.token_to_slot.numel() != embeds.size(0):
+            return None
+        layers, meta = [], None
+        for layer in self.layers:
+            sa, mlp = layer.self_attn, layer.mlp
+            projections = []
+            for mod in (sa.qkv_proj, sa.o_proj, mlp.gate_up_proj, mlp.down_proj):
+                if mod.bias is not None or mod.tp_size != 1 or mod.lora_domain != LM_LORA_DOMAIN:
+                    return None
+                lora = with_lora and mod.supports_lora and (capture or any(mod._effective_lora_rank_values))
+                if lora and meta is None:
+                    meta = mod._runtime_metadata()
+                projections.append(mod._native_projection(lora))
+            layers.append((layer.input_layernorm, layer.post_attention_layernorm, sa.k_cache, sa.v_cache, *projections))
+        got = N.native().prefill_layers(
+            embeds, positions, step.cu_seqlens, step.max_seqlen, step.slot_mapping, self.cos, self.sin, layers, self.norm,
+            meta, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.intermediate_size, cfg.rms_norm_eps)
+        if got is None:
+            return None
+        N.check(got[0])
+        return got[1]
+
     def forward(self, embeds, positions, step: AttentionStep):
         if self.fused_glue:
+            out = self._prefill_native(embeds, positions, step)
+            if out is not None:
+                return out
             if self._decode_chain_ok(embeds, positions, step):
                 return self._decode_chain(embeds, positions, step)
             return self._forward_fused(embeds, positions, step)

@@ -11,6 +11,7 @@
 #include "gemm_tc.cuh"
 #include "grouped_tc.cuh"
 #include "decode_step.cuh"
+#include "prefill_attention.cuh"
 
 using namespace b200lora;
 
@@ -265,6 +266,25 @@ int lora_b200_decode_attention(void* out, const float* planes, int32_t n_planes,
   a.block_tables = block_tables; a.max_blocks = max_blocks; a.block_size = block_size; a.context_lens = context_lens; a.slot_mapping = slot_mapping;
   a.out = static_cast<__nv_bfloat16*>(out); a.scale = scale;
   return decode_attention_launch(a, head_dim, static_cast<cudaStream_t>(stream));
+}
+
+int lora_b200_prefill_attention(void* out, int64_t out_ld, const void* qkv, int64_t qkv_ld, int32_t T, int32_t num_heads,
+                                int32_t num_kv_heads, int32_t head_dim, const int32_t* cu_seqlens, int32_t n_seqs,
+                                int32_t max_seqlen, float scale, void* stream) {
+  if (T < 0 || n_seqs < 0 || max_seqlen < 0) return fail(B200_LORA_EINVAL, "prefill_attention: bad sizes");
+  if (T == 0 || n_seqs == 0 || max_seqlen == 0) return B200_LORA_OK;
+  if (num_kv_heads < 1 || num_heads < 1 || num_heads % num_kv_heads != 0 || (head_dim != 64 && head_dim != 128) || n_seqs > 65535 ||
+      max_seqlen > (1 << 19))
+    return fail(B200_LORA_EUNSUPPORTED, "prefill_attention: heads=%d / %d of %d, %d sequences", num_heads, num_kv_heads, head_dim, n_seqs);
+  if (!out || !qkv || !cu_seqlens) return fail(B200_LORA_EINVAL, "prefill_attention: null pointer");
+  const int width = (num_heads + 2 * num_kv_heads) * head_dim;
+  if (qkv_ld < width || out_ld < num_heads * head_dim) return fail(B200_LORA_EINVAL, "prefill_attention: row stride smaller than row");
+  if (!aligned16(qkv) || qkv_ld % 8 != 0 || out_ld % 2 != 0 || (reinterpret_cast<uintptr_t>(out) & 3u))
+    return fail(B200_LORA_EUNSUPPORTED, "prefill_attention: rows must be 16-byte aligned");
+  PreAttnArgs a = {};
+  a.qkv = static_cast<const __nv_bfloat16*>(qkv); a.ld = qkv_ld; a.out = static_cast<__nv_bfloat16*>(out); a.out_ld = out_ld;
+  a.cu_seqlens = cu_seqlens; a.Hq = num_heads; a.Hk = num_kv_heads; a.T = T; a.scale = scale;
+  return prefill_attention_launch(a, head_dim, n_seqs, max_seqlen, static_cast<cudaStream_t>(stream));
 }
 
 size_t lora_b200_tp_exchange_bytes(int32_t tp, int32_t capacity) { return tp_exchange_bytes(tp, capacity); }

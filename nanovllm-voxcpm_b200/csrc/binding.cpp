@@ -12,6 +12,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/core/LegacyTypeDispatch.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Device.h>
@@ -19,6 +20,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <vector>
 
@@ -35,8 +37,9 @@ decltype(&lora_b200_glue_silu_mul) p_silu = nullptr;
 decltype(&lora_b200_glue_rope_kv_store) p_rope = nullptr;
 decltype(&lora_b200_shrink_buckets) p_shrink = nullptr;
 decltype(&lora_b200_expand_buckets) p_expand = nullptr;
+decltype(&lora_b200_prefill_attention) p_attention = nullptr;
 PyObject* scratch_for = nullptr;  // lora.scratch_for(device, bytes)
-PyObject *s_tts, *s_sorted, *s_ids, *s_counts, *s_offsets, *s_num_active;
+PyObject *s_weight, *s_lora_a, *s_tts, *s_sorted, *s_ids, *s_counts, *s_offsets, *s_num_active;
 
 inline const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
 
@@ -511,6 +514,170 @@ PyObject* rope_kv_store(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+// One projection of a decoder layer: (parameters dict of the module, lora_B names | None, widths, columns, rank buffer).
+// lora_A is one parameter, stacked [slices, S, r, in] or a single [S, r, in].
+struct Projection {
+  const at::Tensor* w = nullptr;
+  Slices sl;
+  const void* rank = nullptr;
+
+  bool read(PyObject* o, int64_t in, int64_t out, int dev) {
+    if (!PyTuple_CheckExact(o) || PyTuple_GET_SIZE(o) != 5 || !PyDict_Check(PyTuple_GET_ITEM(o, 0))) return false;
+    PyObject* params = PyTuple_GET_ITEM(o, 0);
+    auto parameter = [&](PyObject* name) {
+      PyObject* v = PyDict_GetItemWithError(params, name);
+      return v == nullptr ? nullptr : tensor_of(v);
+    };
+    w = parameter(s_weight);
+    if (w == nullptr || w->dim() != 2 || w->scalar_type() != at::kBFloat16 || !on(*w, dev) || !w->is_contiguous() || w->size(0) != out ||
+        w->size(1) != in)
+      return false;
+    if (PyTuple_GET_ITEM(o, 1) == Py_None) return true;
+    PyObject **names, **wi, **ci;
+    const Py_ssize_t n = items(PyTuple_GET_ITEM(o, 1), &names);
+    if (n < 1 || n > B200_LORA_MAX_SLICES || items(PyTuple_GET_ITEM(o, 2), &wi) != n || items(PyTuple_GET_ITEM(o, 3), &ci) != n) return false;
+    const at::Tensor* a = parameter(s_lora_a);
+    if (a == nullptr || a->scalar_type() != at::kBFloat16 || !on(*a, dev) || !a->is_contiguous() || a->dim() < 3 || a->dim() > 4 ||
+        (a->dim() == 4 ? a->size(0) : 1) != n || a->size(-1) != in || a->size(-3) > INT32_MAX)
+      return false;
+    sl.S = a->size(-3); sl.r = a->size(-2); sl.in = in;
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      const int64_t width = PyLong_AsLongLong(wi[i]), column = PyLong_AsLongLong(ci[i]);
+      if (PyErr_Occurred()) { PyErr_Clear(); return false; }
+      if (width == 0) continue;
+      const at::Tensor* b = parameter(names[i]);
+      if (b == nullptr || b->scalar_type() != at::kBFloat16 || !on(*b, dev) || !b->is_contiguous() || b->dim() != 3 || b->size(0) != sl.S ||
+          b->size(1) != width || b->size(2) != sl.r || column < 0 || column + width > out)
+        return false;
+      sl.a[sl.n] = static_cast<const char*>(a->data_ptr()) + i * sl.S * sl.r * in * 2;
+      sl.b[sl.n] = b->data_ptr();
+      sl.out[sl.n] = (int32_t)width;
+      sl.col[sl.n++] = (int32_t)column;
+    }
+    return sl.n == 0 || optional_vector(PyTuple_GET_ITEM(o, 4), at::kInt, sl.S, dev, &rank);
+  }
+};
+
+// prefill_layers(embeds, positions, cu_seqlens, max_seqlen, slot_mapping, cos, sin, layers, final_norm, metadata | None, heads,
+//                kv_heads, head_dim, intermediate, eps) -> (status, normed), or None
+// All layers of an eager bf16 prefill step. `layers`: (norm weight, norm weight, k_cache, v_cache, qkv, o, gate_up, down) with
+// projections as above. (Layer by layer from Python a step of 400 rows took 270 us of host time per layer, for 86 us of kernels.)
+PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 15) { PyErr_SetString(PyExc_TypeError, "prefill_layers takes 15 arguments"); return nullptr; }
+  const at::Tensor* x = tensor_of(args[0]);
+  if (x == nullptr || !x->is_cuda() || x->dim() != 2 || !x->is_contiguous() || x->scalar_type() != at::kBFloat16) return not_handled();
+  const int dev = x->get_device();
+  const at::Tensor* t[6];
+  const int where[6] = {1, 2, 4, 5, 6, 8};
+  for (int i = 0; i < 6; ++i) {
+    t[i] = tensor_of(args[where[i]]);
+    if (t[i] == nullptr || !on(*t[i], dev) || !t[i]->is_contiguous()) return not_handled();
+  }
+  const at::Tensor slots = t[2]->scalar_type() == at::kLong ? t[2]->to(at::kInt) : *t[2];  // (the store kernel takes int32)
+  const at::Tensor &pos = *t[0], &cu = *t[1], &cos = *t[3], &sin = *t[4], &last = *t[5];
+  const int64_t max_len = PyLong_AsLongLong(args[3]), hq = PyLong_AsLongLong(args[10]), hk = PyLong_AsLongLong(args[11]),
+                d = PyLong_AsLongLong(args[12]), inter = PyLong_AsLongLong(args[13]);
+  const double eps = PyFloat_AsDouble(args[14]);
+  if (PyErr_Occurred()) { PyErr_Clear(); return not_handled(); }
+  const int64_t T = x->size(0), H = x->size(1), q_size = hq * d, kv = hk * d, qkv_width = q_size + 2 * kv;
+  const int table = dtype_code(cos.scalar_type());
+  if (dev != c10::cuda::current_device() || T < 1 || T > INT32_MAX || hq < 1 || hk < 1 || (d != 64 && d != 128) || hq % hk || inter < 8 || inter % 8 ||
+      H % 8 || H > 4096 || max_len < 1 || max_len > T || table < 0)
+    return not_handled();
+  if (pos.scalar_type() != at::kLong || pos.numel() != T || cu.scalar_type() != at::kInt || cu.numel() < 2 || cu.numel() > 65536 ||
+      slots.scalar_type() != at::kInt || slots.numel() != T || cos.dim() != 2 || cos.sizes() != sin.sizes() ||
+      sin.scalar_type() != cos.scalar_type() || (cos.size(1) != d && cos.size(1) != d / 2) || last.scalar_type() != at::kBFloat16 || last.numel() != H)
+    return not_handled();
+  PyObject** it;
+  const Py_ssize_t n_layers = items(args[7], &it);
+  if (n_layers < 1) return not_handled();
+  struct Layer {
+    const at::Tensor *ln1, *ln2, *k, *v;
+    Projection p[4];
+  };
+  std::vector<Layer> layers((size_t)n_layers);
+  const int64_t in[4] = {H, q_size, H, inter}, out[4] = {qkv_width, H, 2 * inter, H};
+  size_t need = 0;
+  for (Py_ssize_t i = 0; i < n_layers; ++i) {
+    if (!PyTuple_CheckExact(it[i]) || PyTuple_GET_SIZE(it[i]) != 8) return not_handled();
+    Layer& l = layers[(size_t)i];
+    const at::Tensor** part[4] = {&l.ln1, &l.ln2, &l.k, &l.v};
+    for (int j = 0; j < 4; ++j) {
+      *part[j] = tensor_of(PyTuple_GET_ITEM(it[i], j));
+      if (*part[j] == nullptr || !on(**part[j], dev) || !(*part[j])->is_contiguous() || (*part[j])->scalar_type() != at::kBFloat16) return not_handled();
+    }
+    if (l.ln1->numel() != H || l.ln2->numel() != H || l.k->numel() % kv || l.v->numel() % kv) return not_handled();
+    for (int j = 0; j < 4; ++j) {
+      if (!l.p[j].read(PyTuple_GET_ITEM(it[i], 4 + j), in[j], out[j], dev)) return not_handled();
+      const Slices& sl = l.p[j].sl;
+      if (sl.n > 0) need = std::max(need, p_workspace_bytes((int)T, sl.n, (int)sl.r));
+    }
+  }
+  Buckets b = {};
+  if (args[9] != Py_None && !read_metadata(args[9], T, dev, &b)) return not_handled();
+  PyObject* keep;
+  void* ws;
+  size_t ws_bytes;
+  if (!workspace(Py_None, *x, need, &keep, &ws, &ws_bytes)) return nullptr;
+
+  at::AutoDispatchBelowADInplaceOrView no_autograd;
+  void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const auto opt = x->options();
+  at::Tensor normed = at::empty({T, H}, opt), hidden = at::empty({T, H}, opt), qkv = at::empty({T, qkv_width}, opt), attn = at::empty({T, q_size}, opt),
+             y = at::empty({T, H}, opt), gate_up = at::empty({T, 2 * inter}, opt), act = at::empty({T, inter}, opt);
+  int rc = p_rmsnorm(normed.data_ptr(), H, nullptr, H, x->data_ptr(), H, nullptr, 0, layers[0].ln1->data_ptr(), (int)T, (int)H, (float)eps, 1,
+                     B200_LORA_BF16, stream);
+  const void* residual = x->data_ptr();
+  auto project = [&](const Projection& p, at::Tensor& dst, const at::Tensor& src) {
+    if (rc != B200_LORA_OK) return;
+    const Slices& sl = p.sl;
+    const bool lora = sl.n > 0 && b.tts != nullptr;
+    const int K = (int)src.size(1), N = (int)dst.size(1);
+    // Base product and delta in one kernel once its 128 x 256 tiles come near the number of SMs: it then saves the pass over y
+    // and a launch, with fewer tiles cuBLAS's smaller ones win. Whole steps, us, fused / separate: 4001 rows of 1024, 4 layers
+    // 935 / 1120; 2000 rows of 2048, 3 layers 883 / 957; 1000 rows of 2048 (gate_up 384 tiles, the others 64 to 80) 582 / 609;
+    // 1000 rows of 1024 (256, the others 32 to 40) 416 / 367.
+    const int64_t tiles = (T + 127) / 128 * ((N + 255) / 256);
+    if (lora && tiles >= 100 && K % 64 == 0 && (sl.r == 16 || sl.r == 32 || sl.r == 64)) {
+      rc = p_linear(dst.data_ptr(), N, src.data_ptr(), K, (int)T, K, p.w->data_ptr(), K, N, nullptr, sl.n, sl.a, sl.b, sl.out, sl.col, (int)sl.S,
+                    (int)sl.r, nullptr, b.tts, 1.0f, ws, ws_bytes, stream);
+      return;
+    }
+    at::mm_out(dst, src, p.w->t());
+    if (lora)
+      rc = p_add(dst.data_ptr(), N, src.data_ptr(), K, (int)T, K, sl.n, sl.a, sl.b, sl.out, sl.col, (int)sl.S, (int)sl.r,
+                 static_cast<const int32_t*>(p.rank), nullptr, b.tts, b.sorted, b.ids, b.counts, b.offsets, b.n, 1.0f, B200_LORA_BF16,
+                 B200_LORA_IMPL_AUTO, ws, ws_bytes, stream);
+  };
+  auto add_norm = [&](const at::Tensor& weight) {
+    if (rc != B200_LORA_OK) return;
+    rc = p_rmsnorm(normed.data_ptr(), H, hidden.data_ptr(), H, y.data_ptr(), H, residual, H, weight.data_ptr(), (int)T, (int)H, (float)eps, 1,
+                   B200_LORA_BF16, stream);
+    residual = hidden.data_ptr();
+  };
+  for (size_t i = 0; i < layers.size(); ++i) {
+    const Layer& l = layers[i];
+    project(l.p[0], qkv, normed);
+    if (rc == B200_LORA_OK)
+      rc = p_rope(qkv.data_ptr(), qkv_width, (int)T, (int)hq, (int)hk, (int)d, pos.data_ptr<int64_t>(), cos.data_ptr(), sin.data_ptr(),
+                  (int)cos.size(1), table, (int)cos.size(0), l.k->data_ptr(), l.v->data_ptr(), slots.data_ptr<int32_t>(), B200_LORA_BF16, stream);
+    if (rc == B200_LORA_OK)
+      rc = p_attention(attn.data_ptr(), q_size, qkv.data_ptr(), qkv_width, (int)T, (int)hq, (int)hk, (int)d, cu.data_ptr<int32_t>(),
+                       (int)cu.numel() - 1, (int)max_len, 1.0f / std::sqrt((float)d), stream);
+    project(l.p[1], y, attn);
+    add_norm(*l.ln2);
+    project(l.p[2], gate_up, normed);
+    if (rc == B200_LORA_OK)
+      rc = p_silu(act.data_ptr(), inter, gate_up.data_ptr(), 2 * inter, (int)T, (int)inter, B200_LORA_BF16, stream);
+    project(l.p[3], y, act);
+    add_norm(i + 1 < layers.size() ? *layers[i + 1].ln1 : last);
+  }
+  Py_XDECREF(keep);
+  return Py_BuildValue("(iN)", rc, THPVariable_Wrap(normed));
+  END_HANDLE_TH_ERRORS
+}
+
 // An int of a list or tuple; false (error cleared) if the item is none or does not fit.
 inline bool as_int32(PyObject* o, int32_t* v) {
   if (!PyLong_CheckExact(o)) return false;
@@ -618,6 +785,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   B200_BIND(p_silu, lora_b200_glue_silu_mul)
   B200_BIND(p_shrink, lora_b200_shrink_buckets)
   B200_BIND(p_expand, lora_b200_expand_buckets)
+  B200_BIND(p_attention, lora_b200_prefill_attention)
   B200_BIND(p_rope, lora_b200_glue_rope_kv_store)
 #undef B200_BIND
   Py_INCREF(args[1]);
@@ -628,12 +796,14 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 #define B200_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {B200_METHOD(add), B200_METHOD(shrink), B200_METHOD(expand), B200_METHOD(linear), B200_METHOD(add_rms_norm), B200_METHOD(silu_mul),
-                         B200_METHOD(rope_kv_store), B200_METHOD(bucket_lists), B200_METHOD(pack_lists), B200_METHOD(bind), {nullptr, nullptr, 0, nullptr}};
+                         B200_METHOD(rope_kv_store), B200_METHOD(prefill_layers), B200_METHOD(bucket_lists), B200_METHOD(pack_lists), B200_METHOD(bind), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "b200lora_binding", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 
 PyMODINIT_FUNC PyInit_b200lora_binding(void) {
+  s_weight = PyUnicode_InternFromString("weight");
+  s_lora_a = PyUnicode_InternFromString("lora_A");
   s_tts = PyUnicode_InternFromString("token_to_slot");
   s_sorted = PyUnicode_InternFromString("token_indices_sorted_by_slot");
   s_ids = PyUnicode_InternFromString("active_slot_ids");

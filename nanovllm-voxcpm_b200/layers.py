@@ -104,6 +104,18 @@ class _LoRALayerBase(nn.Module):
         self.__dict__["_slices_plan"] = (key, slices)
         return slices
 
+    def _native_projection(self, with_lora: bool) -> tuple:
+        """This projection as ``prefill_layers`` takes it: the parameters by name, so that nothing can be stale, and the fixed
+        layout of its slices."""
+        if not with_lora:
+            return self._parameters, None, None, None, None
+        layout = self.__dict__.get("_native_layout")
+        if layout is None:
+            targets = getattr(self, "lora_targets", None)
+            names = ["lora_B"] if "lora_B" in self._parameters else [f"lora_B_{t}" for t in targets]
+            layout = self.__dict__["_native_layout"] = (names, *self._slice_layout())
+        return (self._parameters, *layout, self._buffers["effective_lora_rank"])
+
     @property
     def lora_enabled(self) -> bool:
         return self.supports_lora
