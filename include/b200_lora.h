@@ -143,6 +143,15 @@ int lora_b200_linear_lora(void* y, int64_t y_ld, const void* x, int64_t x_ld, in
                           const int32_t* out_sizes, const int32_t* col_offsets, int32_t S,
                           int32_t r_max, const float* scale_per_slot, const int32_t* token_to_slot,
                           float scaling, void* workspace, size_t workspace_bytes, void* stream);
+/* The same for a [gate | up] projection of out_total rows, followed by the activation: y [T, out_total / 2] =
+ * silu(gate) * up in fp32, one rounding (`SiluAndMul` behind the merged projection, nanovllm_voxcpm/layers/activation.py:11-14).
+ * out_total a multiple of 64, slice widths and columns of 32. */
+int lora_b200_linear_lora_silu(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight,
+                               int64_t w_ld, int32_t out_total, int32_t n_slices, const void* const* a_slabs,
+                               const void* const* b_slabs, const int32_t* out_sizes, const int32_t* col_offsets, int32_t S,
+                               int32_t r_max, const float* scale_per_slot, const int32_t* token_to_slot, float scaling,
+                               void* workspace, size_t workspace_bytes, void* stream);
+
 
 /* Bytes of device scratch that B200_LORA_IMPL_SGMV needs for a batch of T tokens (the
  * [n_slices, T, r_max] shrink result in bf16, plus alignment slack). The reference allocates this

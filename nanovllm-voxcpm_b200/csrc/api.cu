@@ -9,6 +9,7 @@
 #include "glue.cuh"
 #include "sgmv_tc.cuh"
 #include "gemm_tc.cuh"
+#include "linear_pair.cuh"
 #include "grouped_tc.cuh"
 #include "decode_step.cuh"
 #include "prefill_attention.cuh"
@@ -316,7 +317,7 @@ int lora_b200_device_status(int32_t* status, int32_t reset) {
   return B200_LORA_OK;
 }
 
-int lora_b200_linear_lora(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,
+static int linear_lora_checked(bool silu, void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,
                           const void* weight, int64_t w_ld, int32_t out_total, const void* bias, int32_t n_slices,
                           const void* const* a_slabs, const void* const* b_slabs, const int32_t* out_sizes,
                           const int32_t* col_offsets, int32_t S, int32_t r_max, const float* scale_per_slot,
@@ -325,9 +326,9 @@ int lora_b200_linear_lora(void* y, int64_t y_ld, const void* x, int64_t x_ld, in
   if (T < 0 || in_dim < 1 || out_total < 1) return fail(B200_LORA_EINVAL, "bad sizes T=%d in=%d out=%d", T, in_dim, out_total);
   if (T == 0) return B200_LORA_OK;
   if (y == nullptr || x == nullptr || weight == nullptr) return fail(B200_LORA_EINVAL, "null y / x / weight");
-  if (y_ld < out_total || x_ld < in_dim || w_ld < in_dim) return fail(B200_LORA_EINVAL, "row stride smaller than row");
+  if (y_ld < (silu ? out_total / 2 : out_total) || x_ld < in_dim || w_ld < in_dim) return fail(B200_LORA_EINVAL, "row stride smaller than row");
   LinearProblem lp;
-  lp.weight = weight; lp.w_ld = w_ld; lp.n_total = out_total; lp.bias = bias;
+  lp.weight = weight; lp.w_ld = w_ld; lp.n_total = out_total; lp.bias = bias; lp.silu = silu;
   SliceTable st;
   st.n = 0;
   for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) { st.a[s] = st.b[s] = nullptr; st.out[s] = st.col[s] = 0; }
@@ -342,6 +343,22 @@ int lora_b200_linear_lora(void* y, int64_t y_ld, const void* x, int64_t x_ld, in
   lp.lora.S = S; lp.lora.r_max = r_max; lp.lora.st = st; lp.lora.scale_per_slot = scale_per_slot;
   lp.lora.token_to_slot = token_to_slot; lp.lora.scaling = scaling;
   return linear_lora_launch(lp, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+int lora_b200_linear_lora(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight, int64_t w_ld, int32_t out_total,
+                          const void* bias, int32_t n_slices, const void* const* a_slabs, const void* const* b_slabs, const int32_t* out_sizes,
+                          const int32_t* col_offsets, int32_t S, int32_t r_max, const float* scale_per_slot, const int32_t* token_to_slot,
+                          float scaling, void* workspace, size_t workspace_bytes, void* stream) {
+  return linear_lora_checked(false, y, y_ld, x, x_ld, T, in_dim, weight, w_ld, out_total, bias, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, S,
+                             r_max, scale_per_slot, token_to_slot, scaling, workspace, workspace_bytes, stream);
+}
+
+int lora_b200_linear_lora_silu(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight, int64_t w_ld, int32_t out_total,
+                          int32_t n_slices, const void* const* a_slabs, const void* const* b_slabs, const int32_t* out_sizes,
+                          const int32_t* col_offsets, int32_t S, int32_t r_max, const float* scale_per_slot, const int32_t* token_to_slot,
+                          float scaling, void* workspace, size_t workspace_bytes, void* stream) {
+  return linear_lora_checked(true, y, y_ld, x, x_ld, T, in_dim, weight, w_ld, out_total, nullptr, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, S,
+                             r_max, scale_per_slot, token_to_slot, scaling, workspace, workspace_bytes, stream);
 }
 
 size_t lora_b200_workspace_bytes(int32_t T, int32_t n_slices, int32_t r_max) {

@@ -32,6 +32,7 @@ decltype(&lora_b200_add) p_add = nullptr;
 decltype(&lora_b200_delta) p_delta = nullptr;
 decltype(&lora_b200_workspace_bytes) p_workspace_bytes = nullptr;
 decltype(&lora_b200_linear_lora) p_linear = nullptr;
+decltype(&lora_b200_linear_lora_silu) p_linear_silu = nullptr;
 decltype(&lora_b200_glue_add_rmsnorm) p_rmsnorm = nullptr;
 decltype(&lora_b200_glue_silu_mul) p_silu = nullptr;
 decltype(&lora_b200_glue_rope_kv_store) p_rope = nullptr;
@@ -558,6 +559,8 @@ struct Projection {
   }
 };
 
+constexpr int64_t kFusedTiles = 100;  // (see `project` below)
+
 // prefill_layers(embeds, positions, cu_seqlens, max_seqlen, slot_mapping, cos, sin, layers, final_norm, metadata | None, heads,
 //                kv_heads, head_dim, intermediate, eps) -> (status, normed), or None
 // All layers of an eager bf16 prefill step. `layers`: (norm weight, norm weight, k_cache, v_cache, qkv, o, gate_up, down) with
@@ -639,7 +642,7 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     // 935 / 1120; 2000 rows of 2048, 3 layers 883 / 957; 1000 rows of 2048 (gate_up 384 tiles, the others 64 to 80) 582 / 609;
     // 1000 rows of 1024 (256, the others 32 to 40) 416 / 367.
     const int64_t tiles = (T + 127) / 128 * ((N + 255) / 256);
-    if (lora && tiles >= 100 && K % 64 == 0 && (sl.r == 16 || sl.r == 32 || sl.r == 64)) {
+    if (lora && tiles >= kFusedTiles && K % 64 == 0 && (sl.r == 16 || sl.r == 32 || sl.r == 64)) {
       rc = p_linear(dst.data_ptr(), N, src.data_ptr(), K, (int)T, K, p.w->data_ptr(), K, N, nullptr, sl.n, sl.a, sl.b, sl.out, sl.col, (int)sl.S,
                     (int)sl.r, nullptr, b.tts, 1.0f, ws, ws_bytes, stream);
       return;
@@ -649,6 +652,14 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       rc = p_add(dst.data_ptr(), N, src.data_ptr(), K, (int)T, K, sl.n, sl.a, sl.b, sl.out, sl.col, (int)sl.S, (int)sl.r,
                  static_cast<const int32_t*>(p.rank), nullptr, b.tts, b.sorted, b.ids, b.counts, b.offsets, b.n, 1.0f, B200_LORA_BF16,
                  B200_LORA_IMPL_AUTO, ws, ws_bytes, stream);
+  };
+  // gate_up with the activation in its epilogue, by the same line (128 + 128 columns make a tile)
+  auto silu_in_linear = [&](const Slices& sl) {
+    if ((T + 127) / 128 * ((2 * inter + 255) / 256) < kFusedTiles || H % 64 || inter % 32) return false;
+    if (sl.n > 0 && b.tts != nullptr && sl.r != 16 && sl.r != 32 && sl.r != 64) return false;
+    for (int q = 0; q < sl.n; ++q)
+      if (sl.out[q] % 32 || sl.col[q] % 32) return false;
+    return true;
   };
   auto add_norm = [&](const at::Tensor& weight) {
     if (rc != B200_LORA_OK) return;
@@ -667,6 +678,15 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
                        (int)cu.numel() - 1, (int)max_len, 1.0f / std::sqrt((float)d), stream);
     project(l.p[1], y, attn);
     add_norm(*l.ln2);
+    if (rc == B200_LORA_OK && silu_in_linear(l.p[2].sl)) {
+      const Slices& sl = l.p[2].sl;
+      rc = p_linear_silu(act.data_ptr(), inter, normed.data_ptr(), H, (int)T, (int)H, l.p[2].w->data_ptr(), H, (int)(2 * inter),
+                         b.tts != nullptr ? sl.n : 0, sl.a, sl.b, sl.out, sl.col, (int)std::max<int64_t>(sl.S, 1), (int)std::max<int64_t>(sl.r, 16),
+                         nullptr, b.tts, 1.0f, ws, ws_bytes, stream);
+      project(l.p[3], y, act);
+      add_norm(i + 1 < layers.size() ? *layers[i + 1].ln1 : last);
+      continue;
+    }
     project(l.p[2], gate_up, normed);
     if (rc == B200_LORA_OK)
       rc = p_silu(act.data_ptr(), inter, gate_up.data_ptr(), 2 * inter, (int)T, (int)inter, B200_LORA_BF16, stream);
@@ -781,6 +801,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   B200_BIND(p_delta, lora_b200_delta)
   B200_BIND(p_workspace_bytes, lora_b200_workspace_bytes)
   B200_BIND(p_linear, lora_b200_linear_lora)
+  B200_BIND(p_linear_silu, lora_b200_linear_lora_silu)
   B200_BIND(p_rmsnorm, lora_b200_glue_add_rmsnorm)
   B200_BIND(p_silu, lora_b200_glue_silu_mul)
   B200_BIND(p_shrink, lora_b200_shrink_buckets)

@@ -545,43 +545,4 @@ inline int prefill_add_launch(const SgmvProblem& b, void* workspace, size_t work
   return sgmv_launch_expand(sm, sa, stream);
 }
 
-struct LinearProblem {
-  SgmvProblem lora;          // y, x, slabs, token_to_slot (null token_to_slot or no slice: plain linear)
-  const void* weight; int64_t w_ld; int n_total; const void* bias;
-};
-
-// y = x . W^T (+ bias) + LoRA delta, the delta accumulated into the GEMM's TMEM accumulator.
-inline int linear_lora_launch(const LinearProblem& p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-  const SgmvProblem& b = p.lora;
-  if (b.in_dim % kSgmvBK != 0) return fail(B200_LORA_EUNSUPPORTED, "fused linear: in_dim must be a multiple of 64");
-  if (p.n_total % 8 != 0 || p.w_ld % 8 != 0 || b.x_ld % 8 != 0 || b.y_ld % 8 != 0)
-    return fail(B200_LORA_EUNSUPPORTED, "fused linear: widths and row strides must be multiples of 8");
-  if ((reinterpret_cast<uintptr_t>(p.weight) & 15u) || (reinterpret_cast<uintptr_t>(b.x) & 15u) ||
-      (reinterpret_cast<uintptr_t>(b.y) & 15u) || (reinterpret_cast<uintptr_t>(p.bias) & 1u))
-    return fail(B200_LORA_EUNSUPPORTED, "fused linear: pointers must be 16-byte aligned");
-  bool any = false;
-  for (int s = 0; s < b.st.n; ++s) any = any || b.st.out[s] > 0;
-  const bool with_lora = any && b.token_to_slot != nullptr;
-  SgmvMaps sm;
-  SgmvArgs sa = {};
-  if (with_lora) {
-    if (int rc = sgmv_prepare(b, workspace, workspace_bytes, &sm, &sa)) return rc;
-    if (int rc = sgmv_launch_shrink(sm, sa, stream)) return rc;
-  } else {
-    // no adapter work: only the x and y views are needed
-    sa.y = static_cast<__nv_bfloat16*>(b.y); sa.y_ld = b.y_ld; sa.T = b.T; sa.in_dim = b.in_dim; sa.S = 1; sa.r_max = 16;
-    sa.n = 0; sa.token_to_slot = nullptr;
-    if (int rc = make_tmap_2d(&sm.x, b.x, (uint64_t)b.T, (uint64_t)b.in_dim, (uint64_t)b.x_ld, kSgmvBM, kSgmvBK)) return rc;
-    sm.t = sm.x;
-    for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) { sm.a[s] = sm.x; sm.b[s] = sm.x; }
-  }
-  const bool fuse = with_lora && tc_lora_stage_ok(sa);
-  GemmMaps gm;
-  GemmArgs ga;
-  if (int rc = tc_tile_prepare(sm, sa, p.weight, p.w_ld, p.n_total, p.bias, false, fuse, &gm, &ga)) return rc;
-  if (int rc = tc_tile_launch(gm, ga, stream)) return rc;
-  if (!with_lora || fuse) return B200_LORA_OK;
-  return sgmv_launch_expand(sm, sa, stream);  // slices not 16-column aligned: delta in a second pass
-}
-
 }  // namespace b200lora
