@@ -103,13 +103,14 @@ namespace {
 // that the bucket kernel would read. us per projection, bucket / prefill kernels, six prompts of different adapters: 1024-wide,
 // rank 32, 900 rows, qkv (16 MB) 6.7 / 13.5, gate_up (37 MB) 8.9 / 15.1, 1500 rows 11.5 / 13.8 and (61 MB) 18.6 / 20.4;
 // 2048-wide, rank 32, 900 rows, gate_up (59 MB) 19.0 / 19.1, 1500 rows (98 MB) 32.9 / 24.7, qkv (52 MB) 16.4 / 16.3; rank 64,
-// 900 rows, qkv (63 MB) 18.8 / 17.0, 1500 rows 33.2 / 19.3.
+// 900 rows, qkv (63 MB) 18.8 / 17.0, 1500 rows 33.2 / 19.3. Above rank 32 the line stays at 512 rows: rank 64, 600 rows, the
+// mean of the four projections 17.0 / 16.1, 900 rows 20.4 / 17.8.
 constexpr int64_t kPrefillMinBytes = 50ll * 1000 * 1000;
 inline bool prefill_sized(int32_t T, const SliceTable& st, int32_t r_max, int32_t in_dim, bool expand) {
   int64_t bytes = 0;
   for (int s = 0; s < st.n; ++s)
     if (st.out[s] > 0 || !expand) bytes += 2 * (int64_t)r_max * (in_dim + (expand ? st.out[s] : 0));
-  return T >= kSgmvAutoMinTokens && ceil_div_i(T, kBgmvTok) * bytes > kPrefillMinBytes;
+  return T >= kSgmvAutoMinTokens && (r_max > 32 || ceil_div_i(T, kBgmvTok) * bytes > kPrefillMinBytes);
 }
 
 }  // namespace

@@ -639,7 +639,7 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const int K = (int)src.size(1), N = (int)dst.size(1);
     // Base product and delta in one kernel once its 128 x 256 tiles come near the number of SMs: it then saves the pass over y
     // and a launch, with fewer tiles cuBLAS's smaller ones win. Whole steps, us, fused / separate: 4001 rows of 1024, 4 layers
-    // 935 / 1120; 2000 rows of 2048, 3 layers 883 / 957; 1000 rows of 2048 (gate_up 384 tiles, the others 64 to 80) 582 / 609;
+    // 888 / 1120; 2000 rows of 2048, 3 layers 831 / 957; 1000 rows of 2048 (gate_up 384 tiles, the others 64 to 80) 582 / 609;
     // 1000 rows of 1024 (256, the others 32 to 40) 416 / 367.
     const int64_t tiles = (T + 127) / 128 * ((N + 255) / 256);
     if (lora && tiles >= kFusedTiles && K % 64 == 0 && (sl.r == 16 || sl.r == 32 || sl.r == 64)) {

@@ -1,15 +1,16 @@
 // Fused linear for large batches: y = x . W^T (+ bias) + LoRA delta with CTA pairs (tcgen05 cta_group::2).
 //
 // What bounds it: a 128 x 256 tile per CTA (tc_tile_kernel) takes 48 KB from the L2 for 512 cycles of MMA, 94 bytes per cycle
-// and SM - the L2 limit, not the tensor cores, and power the tensor cores could use. Here two CTAs share a 256 x 256 tile:
-// each loads its own 128 rows of x and HALF of the weight tile (32 KB for the same 512 cycles), the pair's MMA reads the other
-// half from the peer's shared memory. Everything else is as in tc_tile_kernel: persistent CTAs over equal contiguous ranges of
-// tiles, two accumulators of 256 TMEM columns, LoRA stages (masked rows of tmp, lora_B tile) behind the K loop of a tile,
-// output through swizzled shared memory and TMA stores.
+// and SM. Here two CTAs share a 256 x 256 tile: each loads its own 128 rows of x and HALF of the weight tile (32 KB for the
+// same 512 cycles), the pair's MMA reads the other half from the peer's shared memory. Everything else is as in
+// tc_tile_kernel: persistent CTAs over equal contiguous ranges of tiles, two accumulators of 256 TMEM columns, LoRA steps
+// (masked rows of tmp, lora_B tile) behind the K loop of a tile, output through swizzled shared memory and TMA stores.
+// 8172 rows, without adapters, us, tile / pair kernel / cuBLAS: 2048 -> 12288 302 / 281 / 264 (all zeros: 262 / 225 / 222, the
+// power cap is the difference), 6144 -> 2048 155 / 147 / 127; with rank-32 adapters 316 / 294 and 156 / 153.
 //
-// The LoRA operands have two buffers of their own, filled and masked by two warps of their own while the K loop runs: load,
+// The LoRA operands have buffers of their own, filled and masked by two warps of their own while the K loop runs: load,
 // mask and the arrival at the leader are a chain of 2 us, and in the stages of the K loop, 1 us ahead of the MMAs, every tile
-// waited for it (2048 -> 12288 of 8172 rows, rank 32: 360 us against 281 without adapters).
+// waited for it (2048 -> 12288 of 8172 rows, rank 32: 361 us against 281 without adapters; 316 with two buffers, 294 with four).
 //
 // Who waits for whom: loads of a base stage by both CTAs count on the LEADER's full barrier (rank 0 issues all MMAs); the
 // operands of a LoRA step count on a barrier of the CTA that loaded them, whose mask warp then arrives at the leader's masked
@@ -24,16 +25,17 @@ constexpr int kPairThreads = 256;  // warp 0 TMA, warp 1 MMA (rank 0) + TMEM, wa
 constexpr int kPairMaxStages = 5;
 constexpr int kPairStageBytes = 2 * kSgmvBM * kSgmvBK * 2;  // 32 KB: 128 rows of x, 128 rows of W
 constexpr int kPairOutBufs = 2;
-constexpr int kPairLoraBufs = 2;
+constexpr int kPairMaxLoraBufs = 4;
 constexpr int kPairMaxSeg = 2;                              // 256-row blocks that a pair's tile range may touch
 constexpr int kPairRuns = 2 * kSgmvBM;
 constexpr int kPairRunBytes = kPairRuns * 4;                // slot (int16), first and end row of this CTA's half (uint8 each)
 // Dynamic shared memory: ring, LoRA buffers, output buffers, run tables; 1 KB of the 227 is left to static shared memory.
 constexpr int kPairFixed = kPairOutBufs * kGemmOutBufBytes + kPairMaxSeg * kPairRunBytes;
 __host__ __device__ constexpr int pair_lora_bytes(int r) { return 2 * kSgmvBM * r * 2; }  // tmp tile and half a lora_B tile
+__host__ __device__ constexpr int pair_lora_bufs(int r) { return r > 32 ? 2 : 4; }
 __host__ __device__ constexpr int pair_stages(int r) {
-  const int fit = (kBgmvSmemMax - 1024 - kPairFixed - kPairLoraBufs * pair_lora_bytes(r)) / kPairStageBytes;
-  return fit < kPairMaxStages ? fit : kPairMaxStages;  // 4 at rank 64, else 5
+  const int fit = (kBgmvSmemMax - 1024 - kPairFixed - pair_lora_bufs(r) * pair_lora_bytes(r)) / kPairStageBytes;
+  return fit < kPairMaxStages ? fit : kPairMaxStages;  // 5 at rank 16, else 4
 }
 
 // ---- cta_group::2 forms
@@ -120,7 +122,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ int f_n[2], seg_nruns[kPairMaxSeg];
-  __shared__ __align__(8) uint64_t bars[2 * kPairMaxStages + 3 * kPairLoraBufs + 5];
+  __shared__ __align__(8) uint64_t bars[2 * kPairMaxStages + 3 * kPairMaxLoraBufs + 5];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_flag;
 
@@ -134,10 +136,10 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
   const int blk_first = t_begin / ntile_all;
   const int nseg = t_end > t_begin ? (t_end - 1) / ntile_all - blk_first + 1 : 0;  // <= kPairMaxSeg (host)
   const uint32_t smem_base = smem_u32(smem);  // 1024-byte aligned by the declaration: static shared memory is padded to it
-  const int NS = pair_stages(r);
+  const int NS = pair_stages(r), LB = pair_lora_bufs(r);
   const uint32_t lora_bytes = (uint32_t)pair_lora_bytes(r), lora_base = smem_base + (uint32_t)(NS * kPairStageBytes);
-  const uint32_t out_base = lora_base + kPairLoraBufs * lora_bytes;
-  uint8_t* const out_ptr = smem + NS * kPairStageBytes + kPairLoraBufs * lora_bytes;
+  const uint32_t out_base = lora_base + (uint32_t)LB * lora_bytes;
+  uint8_t* const out_ptr = smem + NS * kPairStageBytes + LB * lora_bytes;
   uint8_t* const tables = out_ptr + kPairOutBufs * kGemmOutBufBytes;
   // (while the tables are made, in the output buffers)
   int16_t* const f_slot = reinterpret_cast<int16_t*>(out_ptr);
@@ -151,17 +153,17 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
   auto full_bar = [&](int s) { return bar0 + 8u * (uint32_t)s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (uint32_t)(kPairMaxStages + s); };
   auto lora_bar = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + b); };
-  auto masked_bar = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + kPairLoraBufs + b); };
-  auto lora_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 2 * kPairLoraBufs + b); };
-  auto acc_full = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 3 * kPairLoraBufs + b); };
-  auto acc_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 3 * kPairLoraBufs + 2 + b); };
+  auto masked_bar = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + kPairMaxLoraBufs + b); };
+  auto lora_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 2 * kPairMaxLoraBufs + b); };
+  auto acc_full = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 3 * kPairMaxLoraBufs + b); };
+  auto acc_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 3 * kPairMaxLoraBufs + 2 + b); };
   constexpr int tmem_cols = 2 * kSgmvBN;
   const uint32_t tables_bar = acc_empty(2);
   const bool aligned = (smem_base & 1023u) == 0;  // (the same in both CTAs)
 
   if (tid == 0) {
     for (int s = 0; s < kPairMaxStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int b = 0; b < kPairLoraBufs; ++b) {
+    for (int b = 0; b < kPairMaxLoraBufs; ++b) {
       mbar_init(lora_bar(b), 1);
       mbar_init(masked_bar(b), 2);  // the mask warps of both CTAs
       mbar_init(lora_empty(b), 1);
@@ -255,7 +257,7 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
               tma_load_2d(base + t_tile_bytes, &maps.b[s], 0, slot * a.out[s] + (lo - a.col[s]) + rank * ((hi - lo) >> 1), lora_bar(b));
             }
             __syncwarp();
-            if (++b == kPairLoraBufs) { b = 0; ++round; }
+            if (++b == LB) { b = 0; ++round; }
           }
         }
     }
@@ -287,7 +289,7 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
             }
             __syncwarp();
             if (lane == 0) mbar_arrive_remote_release(masked0 + 8u * (uint32_t)b);
-            if (++b == kPairLoraBufs) { b = 0; ++round; }
+            if (++b == LB) { b = 0; ++round; }
           }
         }
     }
@@ -335,7 +337,7 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
               if (16 * k4 < r)
                 umma_pair_elected(d_tmem + (uint32_t)d, tl + 2u * k4, bl + 2u * k4, hi_t, idesc, 1u, leader);
             umma_commit_pair_elected(lora_empty(lb), leader);
-            if (++lb == kPairLoraBufs) { lb = 0; ++lround; }
+            if (++lb == LB) { lb = 0; ++lround; }
           }
         }
         umma_commit_pair_elected(acc_full(buf), leader);
@@ -392,7 +394,9 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
 #pragma unroll
               for (int q = 0; q < 32; ++q) {
                 const float g = __uint_as_float(v[q]);
-                v[q] = __float_as_uint(g / (1.f + expf(-g)) * __uint_as_float(up[q]));
+                // (__fdividef, good to 2 ulp: with the correctly rounded division and its branch the elements of a thread took
+                // turns, 390 cycles each, and the kernel 189 us instead of the projection's 64)
+                v[q] = __float_as_uint(__fdividef(g, 1.f + expf(-g)) * __uint_as_float(up[q]));
               }
             } else {
               tmem_ld_wait();
@@ -473,7 +477,7 @@ inline int linear_pair_launch(const SgmvMaps& sm, const SgmvArgs& sa, const void
   int pairs = std::min(kTileSMs / 2, total);
   const int max_per = (kPairMaxSeg - 1) * ntile;  // a range of that many tiles touches at most kPairMaxSeg blocks
   if ((total + pairs - 1) / pairs > max_per) pairs = (total + max_per - 1) / max_per;
-  const int smem = pair_stages(sa.r_max) * kPairStageBytes + kPairLoraBufs * pair_lora_bytes(sa.r_max) + kPairFixed;
+  const int smem = pair_stages(sa.r_max) * kPairStageBytes + pair_lora_bufs(sa.r_max) * pair_lora_bytes(sa.r_max) + kPairFixed;
   if (int rc = sgmv_set_smem(reinterpret_cast<const void*>(silu ? linear_pair_kernel<true> : linear_pair_kernel<false>), smem)) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
@@ -496,10 +500,10 @@ inline int linear_pair_launch(const SgmvMaps& sm, const SgmvArgs& sa, const void
   return B200_LORA_OK;
 }
 
-#ifndef B200_PAIR_MIN
-#define B200_PAIR_MIN 128
-#endif
-constexpr int64_t kPairMinTiles = B200_PAIR_MIN;
+// Pair tiles (256 x 256) from which the pair kernel takes a projection; with fewer, the 74 pairs are filled unevenly and
+// tc_tile_kernel's 128 x 256 tiles are as fast. us, pair / tile kernel, rank 32: 2048 -> 2048, 3000 rows (96 tiles) 32.7 / 35.3;
+// 2048 -> 2560, 2000 rows (80) 38.9 / 38.4; 1024 -> 1024, 4001 rows (64) 20.4 / 18.9; 1024 -> 8192, 4001 rows (512) 53.9 / 60.9.
+constexpr int64_t kPairMinTiles = 96;
 struct LinearProblem {
   SgmvProblem lora;          // y, x, slabs, token_to_slot (null token_to_slot or no slice: plain linear)
   const void* weight; int64_t w_ld; int n_total; const void* bias;
