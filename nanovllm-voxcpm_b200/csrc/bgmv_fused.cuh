@@ -224,17 +224,34 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
       }
     }
   } else if (bucket >= p.n_buckets) {
-    volatile int* owner = reinterpret_cast<volatile int*>(smem + p.off_bar + 8 * (2 * kBgmvMaxStages + 2)) + 1;  // behind the abort flag
+    // (every warp looks for itself: most of these clusters find nothing, and the sooner they leave, the sooner the next launch
+    // has their place)
     const int m = (bucket - p.n_buckets + 1) * p.window;
-    if (tid == 0) *owner = -1;
-    __syncthreads();
-    for (int b = tid; b < p.n_buckets; b += kBgmvThreads) {
-      const int lo = p.offsets[b];
-      if (lo < m && m - lo < p.counts[b]) *owner = b;
+    bucket = -1;
+    for (int b0 = 0; b0 < p.n_buckets && bucket < 0; b0 += 128) {
+      int lo[4], cnt4[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int b = b0 + 32 * i + lane;
+        lo[i] = b < p.n_buckets ? p.offsets[b] : m;
+        cnt4[i] = b < p.n_buckets ? p.counts[b] : 0;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const unsigned mine = __ballot_sync(0xffffffffu, lo[i] < m && m - lo[i] < cnt4[i]);
+        if (mine != 0) {
+          const int owner = __ffs((int)mine) - 1;
+          bucket = b0 + 32 * i + owner;
+          window_no = m / p.window - __shfl_sync(0xffffffffu, lo[i], owner) / p.window;
+        }
+      }
     }
-    __syncthreads();
-    bucket = *owner;
-    if (bucket >= 0) window_no = m / p.window - p.offsets[bucket] / p.window;
+    if (bucket < 0) {
+      if (p.use_pdl && (kOverwrite || (kMode == 1 && p.zero_rows))) griddep_wait();
+      if (kMode == 1 && p.zero_rows) bgmv_zero_rows_without_adapter(p, block_y * C + c, blocks_y * C, tid, kBgmvThreads);
+      if (kOverwrite) bgmv_fill_rows_without_delta(p, block_y * C + c, blocks_y * C, tid, kBgmvThreads);
+      return;
+    }
   }
   const int slot = bucket >= 0 ? p.slot_ids[bucket] : -1;
   const int rows_all = bucket >= 0 ? p.counts[bucket] : 0, start_all = bucket >= 0 ? p.offsets[bucket] : 0;
