@@ -63,18 +63,24 @@ class SlotLoader:
             raise ValueError("the model has no LoRA-enabled module")
         self.device = next(iter(self.modules.values())).weight.device
         self._loaded: dict[int, list[str]] = {}   # slot -> modules its occupant populated
-        self._host: torch.Tensor | None = None    # pinned staging (grow-only)
+        # two pinned staging buffers in turn (grow-only), each free again once its event has passed: an admission is prepared
+        # and queued while the copy of the one before still runs (with one buffer the host link idled 25 us in between)
+        self._host: list[torch.Tensor | None] = [None, None]
+        self._copied: list[torch.cuda.Event | None] = [None, None]
+        self._turn = 0
         self._dev: torch.Tensor | None = None
-        self._copied: torch.cuda.Event | None = None  # the staging buffer is free again once this has passed
         self._plans: dict[tuple[int, tuple[str, ...]], _Plan] = {}
 
     # ------------------------------------------------------------------ staging
-    def _buffers(self, nbytes: int) -> tuple[torch.Tensor, torch.Tensor]:
-        if self._host is None or self._host.numel() < nbytes:
-            cap = max(nbytes, 1 << 20)
-            self._host = torch.empty(cap, dtype=torch.uint8).pin_memory()
-            self._dev = torch.empty(cap, dtype=torch.uint8, device=self.device)
-        return self._host, self._dev
+    def _buffers(self, host_bytes: int, dev_bytes: int) -> tuple[torch.Tensor, torch.Tensor]:
+        turn = self._turn
+        if self._copied[turn] is not None:
+            self._copied[turn].synchronize()  # the copy that last used this pinned buffer
+        if self._host[turn] is None or self._host[turn].numel() < host_bytes:
+            self._host[turn] = torch.empty(max(host_bytes, 1 << 18), dtype=torch.uint8).pin_memory()
+        if self._dev is None or self._dev.numel() < dev_bytes:
+            self._dev = torch.empty(max(dev_bytes, 1 << 20), dtype=torch.uint8, device=self.device)
+        return self._host[turn], self._dev
 
     def _guard(self) -> int:
         return next(iter(self.modules.values()))._a_slices()[0].data_ptr()
@@ -192,9 +198,7 @@ class SlotLoader:
         table["dst"] += plan.slot_stride * np.uint64(slot_id)
         table["src_offset"] += np.where(plan.src_kind == _SRC_ARENA, arena_base,
                                         np.where(plan.src_kind == _SRC_BLOB, table_bytes, 0)).astype(np.int64)
-        if self._copied is not None:
-            self._copied.synchronize()  # the previous admission's copy still reads the pinned buffer until then
-        host, dev = self._buffers(arena_base + arena_bytes)
+        host, dev = self._buffers(table_bytes + plan.blob_bytes, arena_base + arena_bytes)
         host[:table_bytes].copy_(torch.from_numpy(table.view(np.uint8).reshape(-1)))
         for off, src in plan.blobs:
             n = src.numel() * src.element_size()
@@ -205,8 +209,10 @@ class SlotLoader:
             if arena_bytes:
                 # asynchronous when the arena is pinned; the payload must stay unchanged until the copy has run
                 dev[arena_base: arena_base + arena_bytes].copy_(plan.arena, non_blocking=True)
-            self._copied = torch.cuda.Event()
-            self._copied.record()
+            if self._copied[self._turn] is None:
+                self._copied[self._turn] = torch.cuda.Event()
+            self._copied[self._turn].record()
+            self._turn ^= 1
             N.check(N.lib().lora_b200_load_slot(dev.data_ptr(), n_desc, plan.max_elems, N.current_stream(self.device)))
         # host mirrors of the layers (the kernel wrote the device buffers)
         for module, rank, scaling in plan.mirrors:

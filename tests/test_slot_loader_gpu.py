@@ -145,3 +145,22 @@ def test_checkpoint_payload_is_admitted_from_its_arena(tmp_path):
         else:
             assert torch.equal(got[key], want[key]), key
     assert N.device_status() == 0
+
+
+@pytest.mark.parametrize("rank,payload_rank,dtype", [(3, 8, torch.float32), (13, 16, torch.bfloat16), (20, 24, torch.float16),
+                                                     (5, 5, torch.float32), (32, 32, torch.bfloat16)])
+def test_slot_load_at_the_edges_of_its_vectors(rank, payload_rank, dtype):
+    """Data corners that end inside a vector of eight, and payload rows that no vector load can take; two admissions in
+    a row from the two staging buffers, the second over the first."""
+    _, model = _model()
+    ref = copy.deepcopy(model)
+    loader = SlotLoader(model)
+    payloads = [_adapter(model, 32, 1.5, seed=7), _adapter(model, rank, 0.75, seed=8, payload_rank=payload_rank, dtype=dtype),
+                _adapter(model, rank, 1.25, seed=9, payload_rank=payload_rank, dtype=dtype)]
+    for slot, p in ((2, payloads[0]), (2, payloads[1]), (0, payloads[2])):
+        loader.load_slot(slot, p)
+        _load_by_module(ref, slot, p)
+    torch.cuda.synchronize()
+    got, want = _state(model), _state(ref)
+    for key in want:
+        assert got[key] == want[key] if key.endswith(".host") else torch.equal(got[key], want[key]), key
