@@ -1,11 +1,12 @@
-// Fused decode multi-LoRA kernel (bf16): shrink + expand in ONE launch.
+// Fused decode multi-LoRA kernel (bf16, fp16): shrink + expand in ONE launch.
 //
 // Work decomposition
-//   grid = (C, n_buckets + extra), thread-block cluster = (C, 1, 1): one cluster per slot
-//   bucket of the batch (bucket g = tokens sorted_idx[offsets[g] .. +counts[g]) that
+//   grid = (C, clusters), thread-block cluster = (C, 1, 1): one cluster per slot
+//   bucket of the batch (or, with fewer rows than buckets, per window that holds rows) (bucket g = tokens sorted_idx[offsets[g] .. +counts[g]) that
 //   all use adapter slot slot_ids[g]); buckets with id -1 or no tokens exit at once.
-//   A cluster takes at most `window` tokens (16, one pass, unless the GPU is full); the
-//   rest of a popular bucket goes to the extra clusters, window by window.
+//   A cluster takes at most `window` tokens (16, one pass); the rest of a popular bucket
+//   goes to the extra clusters, window by window (windows of 32: 256 rows over 32 adapters
+//   of skewed popularity, four layers of 1024, 94 -> 133 us).
 //   Inside a cluster the adapter's weights are split so that every byte of
 //   lora_A[slot] and lora_B[slot] is pulled from HBM by exactly one CTA:
 //     shrink : the n*r stacked rank rows are split across the C CTAs (full K each)
@@ -161,7 +162,7 @@ __device__ __forceinline__ void bgmv_zero_rows_without_adapter(const BgmvParams&
 }
 
 // Two CTAs per SM: the CTAs of the next launch of the stream become resident while this launch still
-// runs, so their weight copies and L2 prefetches overlap this launch's dependent chain.
+// runs, so their weight copies overlap this launch's dependent chain.
 #ifndef BGMV_MINBLOCKS
 #define BGMV_MINBLOCKS 2
 #endif

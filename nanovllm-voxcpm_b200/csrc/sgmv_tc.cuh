@@ -636,12 +636,4 @@ inline int sgmv_launch_expand(const SgmvMaps& maps, const SgmvArgs& a, cudaStrea
   return check_launch("sgmv_expand_kernel");
 }
 
-inline int sgmv_launch(const SgmvProblem& b, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-  SgmvMaps maps;
-  SgmvArgs args;
-  if (int rc = sgmv_prepare(b, workspace, workspace_bytes, &maps, &args)) return rc;
-  if (int rc = sgmv_launch_shrink(maps, args, stream)) return rc;
-  return sgmv_launch_expand(maps, args, stream);
-}
-
 }  // namespace b200lora

@@ -681,3 +681,38 @@ def test_device_metadata_feeds_the_decode_kernel_and_reports_bad_ids():
                          torch.empty(20000, dtype=torch.int32, device=DEV), None, cnt, off, None)
     with pytest.raises(RuntimeError, match="CUDA tensors only"):
         N.build_metadata(torch.zeros(4, dtype=torch.int32), 2, N.META_GRAPH, srt, None, cnt, off, None)
+
+
+@pytest.mark.parametrize("S", [1, 5, 1023, 1024])
+@pytest.mark.parametrize("T", [1, 63, 255, 256, 257])
+def test_metadata_build_around_the_line_of_the_ranked_form(T, S):
+    """Both forms of the device build (ranked up to 256 rows and 1023 slots, sorted beyond) in the three conventions."""
+    gen = torch.Generator().manual_seed(T * 7 + S)
+    for slots in (torch.randint(-1, S, (T,), generator=gen, dtype=torch.int32), torch.full((T,), -1, dtype=torch.int32),
+                  torch.full((T,), S - 1, dtype=torch.int32)):
+        order = torch.sort(slots, stable=True).indices.to(torch.int32)
+        none = int((slots < 0).sum())
+        for mode in (N.META_GRAPH, N.META_KERNEL, N.META_EAGER):
+            srt = torch.full((T,), -7, dtype=torch.int32, device=DEV)
+            ids, cnt = (torch.full((S + 1,), -7, dtype=torch.int32, device=DEV) for _ in range(2))
+            off, info = torch.full((S + 2,), -7, dtype=torch.int32, device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
+            N.build_metadata(slots.to(DEV), S, mode, srt, ids, cnt, off, info)
+            per = torch.bincount(slots.long() + 1, minlength=S + 1)
+            rows = order if mode == N.META_KERNEL else order[none:]
+            if mode == N.META_KERNEL and none == T:
+                rows, per = order[:0], torch.zeros_like(per)
+            if mode != N.META_KERNEL:
+                per[0] = 0
+            assert torch.equal(srt.cpu()[: rows.numel()], rows) and bool((srt.cpu()[rows.numel():] == -7).all())
+            if mode == N.META_GRAPH:
+                want_ids, want_cnt = torch.arange(-1, S), per
+                want_off = torch.cat([torch.zeros(1, dtype=torch.long), per.cumsum(0)])
+            else:
+                used = per.nonzero().flatten()
+                k = used.numel()
+                want_ids, want_cnt, want_off = torch.full((S + 1,), -1), torch.zeros(S + 1), torch.zeros(S + 2)
+                want_ids[:k], want_cnt[:k], want_off[1: k + 1] = used - 1, per[used].float(), per[used].cumsum(0).float()
+                assert int(info[0]) == k
+            assert torch.equal(ids.cpu().long(), want_ids.long()) and torch.equal(cnt.cpu().long(), want_cnt.long())
+            assert torch.equal(off.cpu().long(), want_off.long())
+            assert int(info[1]) == T - none and int(info[2]) == 0
