@@ -736,7 +736,7 @@ def run_prefill_arm(args, emit=True):
                      "unit": "TFLOP/s", "gpu_launches": 2 * len(names) * args.steps,
                      "roofline": {"bound": "tensor", "achieved": ach, "peak": tf_peak, "unit": "TFLOP/s",
                                   "frac": ach / tf_peak, "traffic": None, "peak_kind": f"of {tkind}",
-                                  "kernel": "tc_tile_kernel", "algorithmic_flops_per_step": base_flops + lora_flops,
+                                  "kernel": "linear_pair_kernel", "algorithmic_flops_per_step": base_flops + lora_flops,
                                   # the step runs back to back for longer than a burst; with sw_power_cap active
                                   # the sustained cuBLAS figure is the comparable one
                                   "frac_of_sustained_peak": (ach / tf_sustained) if tf_sustained else None,
