@@ -90,9 +90,9 @@ const char* lora_b200_last_error(void);
  *                  conventions: eager plan, graph buffers with a leading -1 bucket,
  *                  vLLM-style with a counted -1 bucket). With the bucket arrays NULL
  *                  only the generic kernel can run.
- *  workspace       device scratch for B200_LORA_IMPL_SGMV (see lora_b200_workspace_bytes); may be
- *                  NULL otherwise. With B200_LORA_IMPL_AUTO the prefill kernels are chosen only
- *                  when enough scratch is passed.
+ *  workspace       device scratch for B200_LORA_IMPL_SGMV and _GROUPED (see lora_b200_workspace_bytes); may
+ *                  be NULL otherwise. With B200_LORA_IMPL_AUTO those kernels are chosen only when
+ *                  enough scratch is passed.
  */
 int lora_b200_add(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,
                   int32_t n_slices, const void* const* a_slabs, const void* const* b_slabs,
@@ -153,10 +153,14 @@ int lora_b200_linear_lora_silu(void* y, int64_t y_ld, const void* x, int64_t x_l
                                void* workspace, size_t workspace_bytes, void* stream);
 
 
-/* Bytes of device scratch that B200_LORA_IMPL_SGMV needs for a batch of T tokens (the
- * [n_slices, T, r_max] shrink result in bf16, plus alignment slack). The reference allocates this
+/* Bytes of device scratch with which every kernel that lora_b200_add may choose for a batch of T tokens can run: the
+ * [n_slices, T, r_max] shrink result of B200_LORA_IMPL_SGMV in bf16, or the fp32 partial sums of
+ * B200_LORA_IMPL_GROUPED, whichever is more, plus alignment slack. The reference allocates this
  * intermediate itself on every call (nanovllm_voxcpm/lora.py:302). */
 size_t lora_b200_workspace_bytes(int32_t T, int32_t n_slices, int32_t r_max);
+/* What B200_LORA_IMPL_GROUPED takes of it for one projection and its number of buckets (0 for ranks that it does not run).
+ * With less, B200_LORA_IMPL_AUTO takes the fused decode kernel. No counterpart in the reference. */
+size_t lora_b200_grouped_workspace_bytes(int32_t T, int32_t in_dim, int32_t n_slices, int32_t r_max, int32_t n_buckets);
 
 /*
  * out[s, t, 0:r_max] = scaling * x[t] . A_s[slot_t]^T for slot_t >= 0, and 0 for

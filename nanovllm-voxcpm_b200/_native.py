@@ -66,6 +66,7 @@ _SIGNATURES = {
          POINTER(c_int32), c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p],
     ),
     "lora_b200_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
+    "lora_b200_grouped_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32, c_int32, c_int32]),
     "lora_b200_linear_lora": (
         c_int32,
         [c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32, c_void_p, c_int64, c_int32, c_void_p, c_int32,

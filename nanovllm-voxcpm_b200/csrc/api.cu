@@ -367,6 +367,15 @@ size_t lora_b200_workspace_bytes(int32_t T, int32_t n_slices, int32_t r_max) {
   return std::max(sgmv_workspace_bytes(T, n_slices, r_max), grouped_workspace_bytes(T, n_slices, r_max));
 }
 
+size_t lora_b200_grouped_workspace_bytes(int32_t T, int32_t in_dim, int32_t n_slices, int32_t r_max, int32_t n_buckets) {
+  if (T < 0 || in_dim < 1 || n_slices < 1 || n_slices > B200_LORA_MAX_SLICES || n_buckets < 1 || (r_max != 16 && r_max != 32 && r_max != 64)) return 0;
+  GroupedProblem b = {};
+  b.T = T; b.in_dim = in_dim; b.r_max = r_max; b.n_buckets = n_buckets; b.st.n = n_slices;
+  for (int s = 0; s < n_slices; ++s) b.st.out[s] = 8;
+  int parts;
+  return grouped_need(b, &parts);
+}
+
 int lora_b200_shrink_allreduce_expand(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,
                                       int32_t n_slices, const void* const* a_slabs, const void* const* b_slabs,
                                       const int32_t* out_sizes, const int32_t* col_offsets, int32_t S, int32_t r_max,
@@ -514,7 +523,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
   if (impl == B200_LORA_IMPL_AUTO) {
     // Long batches (prefill) go to the tensor-core kernels when scratch memory was supplied, decode
     // batches to the fused kernel, everything else (other dtypes, odd shapes) to the generic one.
-    int n_act = 0;
+    int n_act = 0, parts;
     for (int s = 0; s < st.n; ++s) n_act += st.out[s] > 0;
     const bool bgmv_ok = is16 && have_buckets && bgmv_supported(bp, nullptr);
     // The prefill kernels tile rows in token order and pay one stage per run of equal slot, so they
@@ -524,11 +533,11 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     if (dtype == B200_LORA_BF16 && !scattered && (!bgmv_ok ? T >= kSgmvAutoMinTokens : prefill_sized(T, st, r_max, in_dim, true)) && sgmv_supported(sp, nullptr) &&
         workspace != nullptr && workspace_bytes >= sgmv_workspace_bytes(T, n_act, r_max))
       impl = B200_LORA_IMPL_SGMV;
-    else if (bgmv_ok && !(grouped_preferred(gp) && workspace != nullptr && workspace_bytes >= grouped_workspace_bytes(T, n_act, r_max) &&
-                          grouped_supported(gp, nullptr)))
-      impl = B200_LORA_IMPL_BGMV;
-    else if (bgmv_ok)
+    else if (bgmv_ok && grouped_preferred(gp) && grouped_supported(gp, nullptr) && workspace != nullptr &&
+             workspace_bytes >= grouped_need(gp, &parts))
       impl = B200_LORA_IMPL_GROUPED;
+    else if (bgmv_ok)
+      impl = B200_LORA_IMPL_BGMV;
     else
       impl = B200_LORA_IMPL_GENERIC;
   }

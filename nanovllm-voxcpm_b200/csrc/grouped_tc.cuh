@@ -665,9 +665,12 @@ inline int grouped_parts(int chunks, int groups, int in_dim) {
   return ceil_div_i(in_dim, round_up_i(ceil_div_i(in_dim, parts), kGrpBK));
 }
 
-// (a batch of T rows has at least T / 64 chunks, which bounds the parts)
+// Scratch of the largest split that a batch of T rows can get: it has at least T / 32 chunks in use and any number above
+// that. More chunks do not always mean fewer parts (one round of items up to half the SMs, six rounds above), so the bound is
+// the larger of the two sides of that line.
 inline size_t grouped_workspace_bytes(int T, int n_slices, int r_max) {
-  return (size_t)grouped_parts(std::max(1, T / kGrpTok), 1, INT32_MAX / 2) * n_slices * T * r_max * 4 + 256;
+  const int chunks = std::max(T / kGrpTok, kGrpSMs / 2 + 1);
+  return (size_t)std::min(kGrpMaxSplit, ceil_div_i(6 * kGrpSMs, chunks)) * n_slices * T * r_max * 4 + 256;
 }
 
 inline bool grouped_supported(const GroupedProblem& b, const char** why, bool with_x = true, bool with_y = true) {
@@ -838,17 +841,23 @@ inline int grouped_expand_launch(const GroupedProblem& b, const void* tmp, int t
   return grouped_launch(grouped_expand_kernel, "grouped_expand_kernel", kGrpSMs, kGrpExpandThreads, smem, maps, a, stream);
 }
 
-inline int grouped_add_launch(const GroupedProblem& b, void* workspace, size_t workspace_bytes, int round_delta, cudaStream_t stream) {
-  const char* why = nullptr;
-  if (!grouped_supported(b, &why)) return fail(B200_LORA_EUNSUPPORTED, "grouped kernels: %s", why);
+// K parts of this batch's shrink and the scratch that its partial sums take
+inline size_t grouped_need(const GroupedProblem& b, int* parts) {
   int n = 0;
   for (int s = 0; s < b.st.n; ++s) n += b.st.out[s] > 0;
   const int groups = ceil_div_i(n, std::max(1, std::min(n, kGrpRows / b.r_max)));
-  int parts = grouped_parts(grouped_expected_chunks(b), groups, b.in_dim);
-  uintptr_t ws = (reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255;
-  const size_t need = (size_t)parts * n * b.T * b.r_max * 4;
-  if (workspace == nullptr || ws + need > reinterpret_cast<uintptr_t>(workspace) + workspace_bytes)
-    return fail(B200_LORA_EWORKSPACE, "grouped kernels need %zu bytes of scratch, got %zu", need + 256, workspace_bytes);
+  *parts = grouped_parts(grouped_expected_chunks(b), groups, b.in_dim);
+  return (size_t)*parts * n * b.T * b.r_max * 4 + 256;
+}
+
+inline int grouped_add_launch(const GroupedProblem& b, void* workspace, size_t workspace_bytes, int round_delta, cudaStream_t stream) {
+  const char* why = nullptr;
+  if (!grouped_supported(b, &why)) return fail(B200_LORA_EUNSUPPORTED, "grouped kernels: %s", why);
+  int parts;
+  const size_t need = grouped_need(b, &parts);  // (256 bytes of it for the alignment)
+  const uintptr_t ws = (reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255;
+  if (workspace == nullptr || workspace_bytes < need)
+    return fail(B200_LORA_EWORKSPACE, "grouped kernels need %zu bytes of scratch, got %zu", need, workspace_bytes);
   if (int rc = grouped_shrink_launch(b, reinterpret_cast<void*>(ws), 0, &parts, nullptr, stream)) return rc;
   return grouped_expand_launch(b, reinterpret_cast<void*>(ws), 0, parts, round_delta, stream);
 }

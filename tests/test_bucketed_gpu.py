@@ -127,3 +127,31 @@ def test_operators_choose_the_kernel_by_the_order_of_the_rows(contiguous):
     assert not tmp.cpu()[:, none].any()
     assert torch.equal(y.cpu()[none].view(torch.int16), p.y[none].view(torch.int16))
     assert N.device_status(reset=True) == 0
+
+
+def test_auto_takes_the_grouped_kernels_with_the_scratch_that_the_query_names():
+    """A batch over many large adapters: ``lora_b200_workspace_bytes`` of scratch is enough for the kernel that IMPL_AUTO
+    chooses, and one that does not get what this batch needs runs on the fused decode kernel instead of failing."""
+    T, in_dim, outs, S, r = 640, 14336, [4096], 60, 64
+    p = W.make_projection(500, T, in_dim, outs, S, r, p_none=0.0)
+    d = p.to_device(DEV)
+    meta = metadata_for(p.token_to_slot, "graph", S)
+    need = N.lib().lora_b200_grouped_workspace_bytes(T, in_dim, len(outs), r, S + 1)
+    given = N.workspace_bytes(T, len(outs), r)
+    assert need <= given
+
+    def run(impl, nbytes):
+        y, ws = d.y.clone(), torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+        LORA.launch_add(y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, meta, 1.0, impl=impl, workspace=ws)
+        torch.cuda.synchronize()
+        assert N.device_status(reset=True) == 0
+        return y
+
+    grouped, fused = run(N.IMPL_GROUPED, need), run(N.IMPL_BGMV, need)
+    assert torch.equal(run(N.IMPL_AUTO, given), grouped) and not torch.equal(grouped, fused)
+    assert torch.equal(run(N.IMPL_AUTO, need - 1), fused)
+    with pytest.raises(RuntimeError, match="scratch"):
+        run(N.IMPL_GROUPED, need - 1)
+    # one rounding of the sum to bf16 (and of the delta): outputs of size 4 to 8 have steps of 2^-5
+    ref = O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets)
+    assert_lora_close(grouped, ref, max_abs=2 * ref.abs().max().item() * 2 ** -8, what="grouped")
