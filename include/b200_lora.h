@@ -401,6 +401,8 @@ int lora_b200_prefill_attention(void* out, int64_t out_ld, const void* qkv, int6
  *
  * lora_b200_decode_planes: planes of an [in -> out] projection with adapters (one less without).
  * lora_b200_decode_linear: fills them (n_slices = 0: base product only). The slices must cover the output.
+ * lora_b200_decode_linear_check: the status that lora_b200_decode_linear would return for a projection before any launch (rows
+ *   of x dense and aligned); a caller asks it before it commits a step to the chain. Host code only.
  * lora_b200_decode_add_rmsnorm: hidden_out = residual + sum, normed = rms_norm(hidden_out) * weight; hidden_out may be residual.
  * lora_b200_decode_silu_mul: out = silu(gate) * up of planes [n, T, 2 * intermediate].
  * lora_b200_decode_attention: q, k, v = sum of planes [n, T, (heads + 2 kv_heads) * head_dim]; rotates q and k, stores k and v at
@@ -410,6 +412,10 @@ int lora_b200_prefill_attention(void* out, int64_t out_ld, const void* qkv, int6
  * index arrays are read before the launches ahead are complete.
  */
 int lora_b200_decode_planes(int32_t in_dim, int32_t out);
+int lora_b200_decode_linear_check(int32_t T, int32_t in_dim, const void* weight, int64_t w_ld, int32_t out_total,
+                                  int32_t n_slices, const void* const* a_slabs, const void* const* b_slabs,
+                                  const int32_t* out_sizes, const int32_t* col_offsets, int32_t S, int32_t r_max,
+                                  int32_t n_buckets);
 int lora_b200_decode_linear(float* planes, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight,
                             int64_t w_ld, int32_t out_total, int32_t n_slices, const void* const* a_slabs,
                             const void* const* b_slabs, const int32_t* out_sizes, const int32_t* col_offsets, int32_t S,

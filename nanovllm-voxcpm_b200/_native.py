@@ -109,6 +109,10 @@ _SIGNATURES = {
          POINTER(c_int32), POINTER(c_int32), c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32,
          c_void_p],
     ),
+    "lora_b200_decode_linear_check": (
+        c_int32, [c_int32, c_int32, c_void_p, c_int64, c_int32, c_int32, POINTER(c_void_p), POINTER(c_void_p), POINTER(c_int32),
+                  POINTER(c_int32), c_int32, c_int32, c_int32],
+    ),
     "lora_b200_decode_add_rmsnorm": (
         c_int32, [c_void_p, c_void_p, c_void_p, c_int32, c_void_p, c_void_p, c_int32, c_int32, c_float, c_void_p],
     ),

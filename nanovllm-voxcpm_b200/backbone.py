@@ -209,15 +209,43 @@ class Decoder(nn.Module):
         if ctx.parts or (with_lora and (ctx.token_to_slot.numel() != T or ctx.token_indices_sorted_by_slot is None
                                         or ctx.active_slot_ids is None or ctx.num_tokens_per_slot is None or ctx.slot_start_offsets is None)):
             return False
+        if any(layer.self_attn.k_cache is None or layer.self_attn.k_cache.dtype != torch.bfloat16 for layer in self.layers):
+            return False
+        return self._chain_projections_ok(T, self._chain_buckets(ctx) if with_lora else None)
+
+    @staticmethod
+    def _chain_buckets(ctx: LoRAContext) -> int:
+        n = min(ctx.active_slot_ids.numel(), ctx.num_tokens_per_slot.numel(), ctx.slot_start_offsets.numel() - 1)
+        return min(n, ctx.num_active_loras) if ctx.num_active_loras > 0 else n
+
+    def _chain_projections_ok(self, T: int, n_buckets: int | None) -> bool:
+        """Whether ``lora_b200_decode_linear`` takes every projection (``n_buckets`` None: without adapters). What ranks, widths
+        and slices it takes is the library's to say; it is asked once per form of projection."""
+        asked: set[tuple] = set()
         for layer in self.layers:
-            for mod in (layer.self_attn.qkv_proj, layer.self_attn.o_proj, layer.mlp.gate_up_proj, layer.mlp.down_proj):
-                if mod.bias is not None or mod.tp_size != 1 or mod.weight.dtype != torch.bfloat16 or mod.lora_domain != LM_LORA_DOMAIN:
+            sa, mlp = layer.self_attn, layer.mlp
+            for mod in (sa.qkv_proj, sa.o_proj, mlp.gate_up_proj, mlp.down_proj):
+                params = mod._parameters  # (module attribute look-ups are what this loop costs)
+                w = params["weight"]
+                if params.get("bias") is not None or mod.tp_size != 1 or w.dtype != torch.bfloat16 or mod.lora_domain != LM_LORA_DOMAIN:
                     return False
-                if with_lora and (not mod.supports_lora or mod.max_lora_rank % 16 or mod.max_lora_rank > 256
-                                  or sum(mod._active_slices()[2]) != mod.weight.size(0)):
+                a, b, widths, cols = mod._active_slices() if n_buckets is not None and mod.supports_lora else ([], [], [], [])
+                if n_buckets is not None and not a:
                     return False
-            if layer.self_attn.k_cache is None or layer.self_attn.k_cache.dtype != torch.bfloat16:
-                return False
+                at = w.data_ptr()
+                for t in (*a, *b):
+                    if t.dtype != torch.bfloat16 or not t.is_contiguous():
+                        return False
+                    at |= t.data_ptr()
+                form = (w.shape, w.stride(), at & 15, *widths, *cols, a[0].shape if a else None)
+                if form in asked:
+                    continue
+                S, r = a[0].shape[:2] if a else (0, 0)
+                if w.stride(1) != 1 or N.lib().lora_b200_decode_linear_check(
+                        T, w.size(1), w.data_ptr(), w.stride(0), w.size(0), len(a), N.ptr_array(a), N.ptr_array(b), N.int_array(widths),
+                        N.int_array(cols), S, r, n_buckets or 0) != 0:
+                    return False
+                asked.add(form)
         return True
 
     def _decode_chain(self, embeds, positions, step: AttentionStep):
@@ -228,11 +256,7 @@ class Decoder(nn.Module):
         ctx = get_lora_context()
         with_lora = ctx.token_to_slot is not None and not ctx.no_lora_flag
         meta = self.layers[0].self_attn.qkv_proj._runtime_metadata() if with_lora else None
-        n_buckets = 0
-        if with_lora:
-            n_buckets = min(meta.active_slot_ids.numel(), meta.num_tokens_per_slot.numel(), meta.slot_start_offsets.numel() - 1)
-            if meta.num_active_loras > 0:
-                n_buckets = min(n_buckets, meta.num_active_loras)
+        n_buckets = self._chain_buckets(ctx) if with_lora else 0
         shapes = [(m.weight.size(1), m.weight.size(0)) for m in (
             self.layers[0].self_attn.qkv_proj, self.layers[0].self_attn.o_proj, self.layers[0].mlp.gate_up_proj, self.layers[0].mlp.down_proj)]
         planes_of = {s: lib.lora_b200_decode_planes(*s) - (0 if with_lora else 1) for s in shapes}

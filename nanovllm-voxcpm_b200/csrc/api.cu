@@ -190,39 +190,63 @@ int lora_b200_decode_planes(int32_t in_dim, int32_t out) {
   return decode_gemm_parts(in_dim, out) + 1;
 }
 
+// Argument checks of a projection of the decode chain, and the adapters' part of the launch (*bp). Reads no pointer.
+static int decode_linear_problem(BgmvProblem* bp, float* planes, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight,
+                                 int64_t w_ld, int32_t out_total, int32_t n_slices, const void* const* a_slabs,
+                                 const void* const* b_slabs, const int32_t* out_sizes, const int32_t* col_offsets, int32_t S,
+                                 int32_t r_max, const int32_t* rank_per_slot, const int32_t* token_to_slot,
+                                 const int32_t* sorted_idx, const int32_t* slot_ids, const int32_t* counts, const int32_t* offsets,
+                                 int32_t n_buckets) {
+  if (T < 1 || T > kDecMaxRows || in_dim < 1 || out_total < 1) return fail(B200_LORA_EINVAL, "decode_linear: bad sizes T=%d in=%d out=%d", T, in_dim, out_total);
+  if (planes == nullptr || x == nullptr || weight == nullptr) return fail(B200_LORA_EINVAL, "decode_linear: null pointer");
+  if (in_dim % 64 != 0 || x_ld % 8 != 0 || w_ld % 8 != 0 || x_ld < in_dim || w_ld < in_dim || out_total % 8 != 0 || !aligned16(planes) || !aligned16(x) ||
+      !aligned16(weight))
+    return fail(B200_LORA_EUNSUPPORTED, "decode_linear: in_dim must be a multiple of 64, out of 8, rows 16-byte aligned");
+  if (n_slices <= 0) return B200_LORA_OK;
+  if (out_sizes == nullptr || col_offsets == nullptr || token_to_slot == nullptr) return fail(B200_LORA_EINVAL, "decode_linear: null slice or slot array");
+  if (int rc = fill_slices(bp->st, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, true, true)) return rc;
+  int covered = 0;
+  for (int s = 0; s < bp->st.n; ++s) {
+    if (bp->st.col[s] + bp->st.out[s] > out_total) return fail(B200_LORA_EINVAL, "slice %d exceeds the output width", s);
+    covered += bp->st.out[s];
+  }
+  if (covered != out_total) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: the slices must cover the output");
+  const int parts = decode_gemm_parts(in_dim, out_total);
+  bp->y = planes + (size_t)parts * T * out_total; bp->y_ld = out_total;
+  bp->x = x; bp->x_ld = x_ld; bp->T = T; bp->in_dim = in_dim; bp->S = S; bp->r_max = r_max;
+  bp->rank_per_slot = rank_per_slot; bp->scale_per_slot = nullptr;
+  bp->sorted_idx = sorted_idx; bp->slot_ids = slot_ids; bp->counts = counts; bp->offsets = offsets; bp->n_buckets = n_buckets;
+  bp->scaling = 1.0f; bp->mode = 4; bp->kind = r_max % 32 != 0 ? 1 : 0; bp->token_to_slot = token_to_slot;
+  bp->beside = std::min(ceil_div_i(out_total, 128) * parts, 148);
+  if (S < 1 || r_max < 1) return fail(B200_LORA_EINVAL, "decode_linear: bad sizes S=%d r_max=%d", S, r_max);
+  if (sorted_idx == nullptr || slot_ids == nullptr || counts == nullptr || offsets == nullptr)
+    return fail(B200_LORA_EINVAL, "decode_linear: needs the bucket arrays");
+  const char* why = nullptr;
+  if (!bgmv_supported(*bp, &why)) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: %s", why);
+  return B200_LORA_OK;
+}
+
+int lora_b200_decode_linear_check(int32_t T, int32_t in_dim, const void* weight, int64_t w_ld, int32_t out_total, int32_t n_slices,
+                                  const void* const* a_slabs, const void* const* b_slabs, const int32_t* out_sizes,
+                                  const int32_t* col_offsets, int32_t S, int32_t r_max, int32_t n_buckets) {
+  BgmvProblem bp = {};
+  float* const some = reinterpret_cast<float*>(uintptr_t(256));  // (stands for the arrays of a step; not read)
+  const int32_t* const index = reinterpret_cast<const int32_t*>(some);
+  return decode_linear_problem(&bp, some, some, in_dim, T, in_dim, weight, w_ld, out_total, n_slices, a_slabs, b_slabs, out_sizes, col_offsets,
+                               S, r_max, nullptr, index, index, index, index, index, n_buckets);
+}
+
 int lora_b200_decode_linear(float* planes, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight, int64_t w_ld,
                             int32_t out_total, int32_t n_slices, const void* const* a_slabs, const void* const* b_slabs,
                             const int32_t* out_sizes, const int32_t* col_offsets, int32_t S, int32_t r_max,
                             const int32_t* rank_per_slot, const int32_t* token_to_slot, const int32_t* sorted_idx,
                             const int32_t* slot_ids, const int32_t* counts, const int32_t* offsets, int32_t n_buckets,
                             void* stream) {
-  if (T < 1 || T > kDecMaxRows || in_dim < 1 || out_total < 1) return fail(B200_LORA_EINVAL, "decode_linear: bad sizes T=%d in=%d out=%d", T, in_dim, out_total);
-  if (planes == nullptr || x == nullptr || weight == nullptr) return fail(B200_LORA_EINVAL, "decode_linear: null pointer");
-  if (in_dim % 64 != 0 || x_ld % 8 != 0 || w_ld % 8 != 0 || x_ld < in_dim || w_ld < in_dim || out_total % 8 != 0 || !aligned16(planes) || !aligned16(x) ||
-      !aligned16(weight))
-    return fail(B200_LORA_EUNSUPPORTED, "decode_linear: in_dim must be a multiple of 64, out of 8, rows 16-byte aligned");
-  cudaStream_t st_ = static_cast<cudaStream_t>(stream);
   BgmvProblem bp = {};
-  if (n_slices > 0) {
-    if (out_sizes == nullptr || col_offsets == nullptr || token_to_slot == nullptr) return fail(B200_LORA_EINVAL, "decode_linear: null slice or slot array");
-    if (int rc = fill_slices(bp.st, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, true, true)) return rc;
-    int covered = 0;
-    for (int s = 0; s < bp.st.n; ++s) {
-      if (bp.st.col[s] + bp.st.out[s] > out_total) return fail(B200_LORA_EINVAL, "slice %d exceeds the output width", s);
-      covered += bp.st.out[s];
-    }
-    if (covered != out_total) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: the slices must cover the output");
-    bp.y = planes + (size_t)decode_gemm_parts(in_dim, out_total) * T * out_total; bp.y_ld = out_total;
-    bp.x = x; bp.x_ld = x_ld; bp.T = T; bp.in_dim = in_dim; bp.S = S; bp.r_max = r_max;
-    bp.rank_per_slot = rank_per_slot; bp.scale_per_slot = nullptr;
-    bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets; bp.n_buckets = n_buckets;
-    bp.scaling = 1.0f; bp.mode = 4; bp.kind = r_max % 32 != 0 ? 1 : 0; bp.token_to_slot = token_to_slot;
-    const char* why = nullptr;
-    if (sorted_idx == nullptr || slot_ids == nullptr || counts == nullptr || offsets == nullptr)
-      return fail(B200_LORA_EINVAL, "decode_linear: needs the bucket arrays");
-    if (!bgmv_supported(bp, &why)) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: %s", why);
-  }
-  return decode_linear_launch(planes, x, x_ld, T, in_dim, weight, w_ld, out_total, n_slices > 0 ? &bp : nullptr, st_);
+  if (int rc = decode_linear_problem(&bp, planes, x, x_ld, T, in_dim, weight, w_ld, out_total, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, S,
+                                     r_max, rank_per_slot, token_to_slot, sorted_idx, slot_ids, counts, offsets, n_buckets))
+    return rc;
+  return decode_linear_launch(planes, x, x_ld, T, in_dim, weight, w_ld, out_total, n_slices > 0 ? &bp : nullptr, static_cast<cudaStream_t>(stream));
 }
 
 int lora_b200_decode_add_rmsnorm(void* normed, void* hidden_out, const float* planes, int32_t n_planes, const void* residual,

@@ -208,7 +208,7 @@ inline int launch_dependent(void (*kernel)(Params...), const char* name, dim3 gr
 
 // planes of x . W^T, and (lora != nullptr) the delta in the plane behind them
 inline int decode_linear_launch(float* planes, const void* x, int64_t x_ld, int T, int in_dim, const void* w, int64_t w_ld, int out,
-                                BgmvProblem* lora, cudaStream_t stream) {
+                                const BgmvProblem* lora, cudaStream_t stream) {
   DecGemmArgs a = {};
   DecGemmMaps maps;
   a.part = planes; a.T = T; a.in_dim = in_dim; a.out = out; a.n_pad = round_up_i(T, 16);
@@ -226,7 +226,6 @@ inline int decode_linear_launch(float* planes, const void* x, int64_t x_ld, int 
   }
   a.delta = planes + (size_t)a.parts * T * out;
   a.token_to_slot = lora->token_to_slot; a.rank_per_slot = lora->rank_per_slot; a.S = lora->S;
-  lora->beside = std::min(a.tiles * a.parts, 148);
   BgmvParams p;
   const char* why = nullptr;
   if (!bgmv_plan(*lora, &p, &why)) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: %s", why);

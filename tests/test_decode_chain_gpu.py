@@ -100,3 +100,33 @@ def test_chain_matches_the_layer_by_layer_step(case, with_lora):
         assert torch.equal(out[none], base[none]), "rows without adapter differ from the decoder without adapters"
         assert T == 1 or not torch.equal(out[~none], base[~none])
     assert N.device_status(reset=True) == 0
+
+
+def test_step_at_a_rank_that_the_chain_does_not_take():
+    """Rank 176 in three slices is more than a cluster holds: the step runs layer by layer."""
+    T, S, hidden = 5, 3, 256
+    cfg = BB.DecoderConfig(hidden_size=hidden, num_heads=4, num_kv_heads=2, head_dim=64, intermediate_size=128, num_layers=2,
+                           max_position=64, max_loras=S, max_lora_rank=176)
+    with torch.device(DEV):
+        model = BB.Decoder(cfg).to(torch.bfloat16)
+    model.init_random_(0)
+    model.fill_adapter_slots_(S, 176, seed=1)
+    model.allocate_kv_cache(T)
+    lens = torch.arange(3, 3 + T, device=DEV)
+    tables = torch.arange(T, dtype=torch.int32, device=DEV).view(T, 1)
+    step = BB.AttentionStep(False, tables[:, 0].long() * cfg.kv_block_size + lens, context_lens=(lens + 1).to(torch.int32), block_tables=tables)
+    embeds = torch.randn(T, hidden, generator=torch.Generator().manual_seed(0)).to(DEV, torch.bfloat16)
+    bufs = GraphLoRABuffers.make(T, S, device=DEV)
+    bufs.load_token_to_slot_on_device(torch.tensor([0, 1, -1, 2, 0], dtype=torch.int32, device=DEV))
+    set_lora_context(bufs.context(T))
+    try:
+        with torch.inference_mode():
+            model.fused_glue = True
+            assert not model._decode_chain_ok(embeds, lens, step)
+            got = model(embeds, lens, step)
+            model.fused_glue = False
+            want = model(embeds, lens, step)
+    finally:
+        reset_lora_context()
+    torch.testing.assert_close(got.float(), want.float(), atol=4e-2, rtol=4e-2)
+    assert N.device_status(reset=True) == 0
