@@ -190,26 +190,41 @@ class Decoder(nn.Module):
         rows on one GPU, adapters (if any) on every output of every projection, and contexts short enough that one CTA
         per request and kv head is the faster attention."""
         cfg, T = self.cfg, embeds.size(0)
-        if step.is_prefill or not 1 <= T <= 128 or not embeds.is_cuda or embeds.dtype != torch.bfloat16 or not embeds.is_contiguous():
+        if step.is_prefill or not 1 <= T <= 128 or not embeds.is_cuda:
             return False
-        if cfg.head_dim not in (64, 128) or cfg.num_heads % cfg.num_kv_heads or cfg.num_heads // cfg.num_kv_heads > 16:
+
+        def dense(t, dtype, *shape) -> bool:  # (the chain passes addresses on: a strided or foreign array would be misread)
+            return t is not None and t.dtype == dtype and t.shape == shape and t.is_contiguous() and t.device == embeds.device
+
+        heads, kv_heads, dim = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
+        if dim not in (64, 128) or heads % kv_heads or heads // kv_heads > 16:
             return False
-        if cfg.hidden_size % 64 or cfg.hidden_size > 4096 or cfg.intermediate_size % 64 or (cfg.num_heads * cfg.head_dim) % 64:
+        if cfg.hidden_size % 64 or cfg.hidden_size > 4096 or cfg.intermediate_size % 64 or (heads * dim) % 64:
             return False
-        if step.block_tables.size(1) * cfg.kv_block_size > 4096 or not step.block_tables.is_contiguous():
+        if step.block_tables is None or step.block_tables.dim() != 2 or step.block_tables.size(1) * cfg.kv_block_size > 4096:
             return False
-        if step.context_lens.dtype != torch.int32 or step.block_tables.dtype != torch.int32 or step.slot_mapping.dtype != torch.int64 \
-                or positions.dtype != torch.int64:
+        if not (dense(embeds, torch.bfloat16, T, cfg.hidden_size) and dense(positions, torch.int64, T) and dense(step.slot_mapping, torch.int64, T)
+                and dense(step.context_lens, torch.int32, T) and dense(step.block_tables, torch.int32, T, step.block_tables.size(1))):
+            return False
+        if not (dense(self.cos, self.cos.dtype, *self.cos.shape) and dense(self.sin, self.cos.dtype, *self.cos.shape)):
             return False
         backend = LORA.get_backend()
         if not isinstance(backend, LORA.B200LoRABackend) or backend.impl != N.IMPL_AUTO:
             return False
         ctx = get_lora_context()
         with_lora = ctx.token_to_slot is not None and not ctx.no_lora_flag
-        if ctx.parts or (with_lora and (ctx.token_to_slot.numel() != T or ctx.token_indices_sorted_by_slot is None
-                                        or ctx.active_slot_ids is None or ctx.num_tokens_per_slot is None or ctx.slot_start_offsets is None)):
+        if ctx.parts or (with_lora and not dense(ctx.token_to_slot, torch.int32, T)):
             return False
-        if any(layer.self_attn.k_cache is None or layer.self_attn.k_cache.dtype != torch.bfloat16 for layer in self.layers):
+        if with_lora and any(t is None or t.dim() != 1 or not dense(t, torch.int32, t.numel()) for t in (
+                ctx.token_indices_sorted_by_slot, ctx.active_slot_ids, ctx.num_tokens_per_slot, ctx.slot_start_offsets)):
+            return False
+        norms = [self.norm]
+        for layer in self.layers:
+            norms += (layer.input_layernorm, layer.post_attention_layernorm)
+            for cache in (layer.self_attn.k_cache, layer.self_attn.v_cache):
+                if cache is None or cache.dim() != 4 or not dense(cache, torch.bfloat16, cache.size(0), cfg.kv_block_size, kv_heads, dim):
+                    return False
+        if not all(dense(w, torch.bfloat16, cfg.hidden_size) for w in norms):
             return False
         return self._chain_projections_ok(T, self._chain_buckets(ctx) if with_lora else None)
 

@@ -130,3 +130,75 @@ def test_step_at_a_rank_that_the_chain_does_not_take():
         reset_lora_context()
     torch.testing.assert_close(got.float(), want.float(), atol=4e-2, rtol=4e-2)
     assert N.device_status(reset=True) == 0
+
+
+def _strided(t):
+    """The same values with a gap behind each."""
+    wide = torch.zeros(*t.shape, 2, dtype=t.dtype, device=t.device)
+    wide[..., 0] = t
+    return wide[..., 0]
+
+
+@pytest.mark.parametrize("what", ["positions", "slot_mapping", "context_lens", "block_tables", "k_cache", "block size", "norm", "token_to_slot",
+                                  "counts", "embeds"])
+def test_forms_that_the_chain_would_misread_run_layer_by_layer(what):
+    T, S, hidden = 5, 3, 256
+    cfg = BB.DecoderConfig(hidden_size=hidden, num_heads=4, num_kv_heads=2, head_dim=64, intermediate_size=128, num_layers=1,
+                           max_position=64, max_loras=S, max_lora_rank=16)
+    with torch.device(DEV):
+        model = BB.Decoder(cfg).to(torch.bfloat16)
+    model.fused_glue = True
+    model.allocate_kv_cache(2 * T)
+    lens = torch.arange(3, 3 + T, device=DEV)
+    tables = torch.arange(2 * T, dtype=torch.int32, device=DEV).view(T, 2)
+    step = BB.AttentionStep(False, tables[:, 0].long() * cfg.kv_block_size + lens, context_lens=(lens + 1).to(torch.int32), block_tables=tables)
+    embeds = torch.randn(T, hidden, device=DEV, dtype=torch.bfloat16)
+    bufs = GraphLoRABuffers.make(T, S, device=DEV)
+    bufs.load_token_to_slot_on_device(torch.tensor([0, 1, -1, 2, 0], dtype=torch.int32, device=DEV))
+    ctx = bufs.context(T)
+    set_lora_context(ctx)
+    try:
+        assert model._decode_chain_ok(embeds, lens, step)
+        sa = model.layers[0].self_attn
+        if what == "positions":
+            lens = _strided(lens)
+        elif what in ("slot_mapping", "context_lens", "block_tables"):
+            setattr(step, what, _strided(getattr(step, what)))
+        elif what == "k_cache":
+            sa.k_cache = _strided(sa.k_cache)
+        elif what == "block size":
+            sa.k_cache = sa.k_cache.view(-1, cfg.kv_block_size * 2, 2, 64)
+        elif what == "norm":
+            model.norm.data = model.norm.data.float()
+        elif what == "token_to_slot":
+            ctx.token_to_slot = _strided(ctx.token_to_slot)
+        elif what == "counts":
+            ctx.num_tokens_per_slot = ctx.num_tokens_per_slot.long()
+        else:
+            embeds = _strided(embeds)
+        assert not model._decode_chain_ok(embeds, lens, step)
+    finally:
+        reset_lora_context()
+
+
+def test_strided_slot_mapping_gives_the_same_step():
+    """A form that the layer-by-layer step takes (it converts the map)."""
+    T, hidden = 5, 256
+    cfg = BB.DecoderConfig(hidden_size=hidden, num_heads=4, num_kv_heads=2, head_dim=64, intermediate_size=128, num_layers=1,
+                           max_position=64, max_loras=2, max_lora_rank=16)
+    with torch.device(DEV):
+        model = BB.Decoder(cfg).to(torch.bfloat16)
+    model.fused_glue = True
+    model.init_random_(0)
+    lens = torch.arange(3, 3 + T, device=DEV)
+    tables = torch.arange(T, dtype=torch.int32, device=DEV).view(T, 1)
+    at = tables[:, 0].long() * cfg.kv_block_size + lens
+    embeds = torch.randn(T, hidden, device=DEV, dtype=torch.bfloat16)
+    out = []
+    for slots in (at, _strided(at)):
+        model.allocate_kv_cache(T)
+        step = BB.AttentionStep(False, slots, context_lens=(lens + 1).to(torch.int32), block_tables=tables)
+        with torch.inference_mode():
+            out.append((model(embeds, lens, step).float(), model.layers[0].self_attn.k_cache.float()))
+    torch.testing.assert_close(out[1][0], out[0][0], atol=4e-2, rtol=4e-2)
+    torch.testing.assert_close(out[1][1], out[0][1], atol=4e-2, rtol=4e-2)
