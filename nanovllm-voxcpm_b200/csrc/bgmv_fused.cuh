@@ -1,19 +1,20 @@
 // Fused decode multi-LoRA kernel (bf16, fp16): shrink + expand in ONE launch.
 //
 // Work decomposition
-//   grid = (C, clusters), thread-block cluster = (C, 1, 1): one cluster per slot
-//   bucket of the batch (or, with fewer rows than buckets, per window that holds rows) (bucket g = tokens sorted_idx[offsets[g] .. +counts[g]) that
-//   all use adapter slot slot_ids[g]); buckets with id -1 or no tokens exit at once.
-//   A cluster takes at most `window` tokens (16, one pass); the rest of a popular bucket
-//   goes to the extra clusters, window by window (windows of 32: 256 rows over 32 adapters
-//   of skewed popularity, four layers of 1024, 94 -> 133 us).
+//   grid = (C, clusters), thread-block cluster = (C, 1, 1). Bucket g of the batch is the tokens
+//   sorted_idx[offsets[g] .. +counts[g]), which all use adapter slot slot_ids[g]; it is cut into
+//   windows of 16 tokens (one MMA M tile), and a cluster takes one window. There is a cluster per
+//   bucket, for its first window, and extra ones for the further windows of popular buckets
+//   (clusters of two passes: 256 rows over 32 adapters of skewed popularity, four layers of 1024,
+//   94 -> 133 us); with fewer rows than buckets there is one per window that the rows can make.
+//   Clusters without rows exit at once.
 //   Inside a cluster the adapter's weights are split so that every byte of
 //   lora_A[slot] and lora_B[slot] is pulled from HBM by exactly one CTA:
 //     shrink : the n*r stacked rank rows are split across the C CTAs (full K each)
 //     expand : each slice's output rows are split across the C CTAs
 //   and the rank-r intermediate tmp[16 tokens, n*r] (bf16) is all-gathered through
-//   distributed shared memory between the two phases (stores into every peer's buffer,
-//   then one remote mbarrier arrive per peer; the buffer is double-buffered by pass).
+//   distributed shared memory between the two phases (st.async: the data and their byte
+//   count on the receiver's mbarrier in one operation).
 //
 // Roles
 //   warp 8      producer: walks the CTA's tile list and issues 1-D bulk async copies
@@ -24,7 +25,7 @@
 //               depend on the previous kernel of the stream, so under programmatic
 //               dependent launch they are requested before griddepcontrol.wait.
 //   warps 0-7   consumers: mma.sync m16n8k16 bf16 -> fp32 with tokens as the 16-row
-//               operand (a pass handles 16 tokens of the bucket) and weight rows as the
+//               operand and weight rows as the
 //               8-column operand. Activations are read straight into MMA fragments
 //               (16-byte global loads, once per 1024-column part); y is read one tile
 //               ahead and written back with 16-byte stores.
@@ -46,7 +47,7 @@ namespace b200lora {
 constexpr int kBgmvWarps = 8;                       // consumer warps
 constexpr int kBgmvConsumers = kBgmvWarps * 32;
 constexpr int kBgmvThreads = kBgmvConsumers + 32;   // + producer warp
-constexpr int kBgmvTok = 16;           // tokens per pass (one MMA M tile)
+constexpr int kBgmvTok = 16;           // tokens per cluster: a window of a bucket (one MMA M tile)
 constexpr int kBgmvMaxRc = 64;         // stacked rank rows per CTA
 constexpr int kBgmvKP = 1024;          // columns per shrink tile
 constexpr int kBgmvXBlocks = kBgmvKP / 32 / kBgmvWarps;  // 32-column blocks per warp and tile
@@ -102,7 +103,6 @@ struct BgmvParams {
   const int32_t *sorted_idx, *slot_ids, *counts, *offsets;
   int n_buckets; float scaling;
   int clusters, by_window;  // clusters of the launch; by_window: cluster i takes the i-th window of the batch
-  int window;       // tokens per cluster (multiple of 16)
   int c_shift;      // cluster size C = 1 << c_shift
   int KP, nkp;      // columns per shrink tile (min(in, 1024)) and number of K parts
   int pitchA;       // bytes between rows of a shrink tile (KP*2, +64 when rows are copied one by one)
@@ -113,12 +113,11 @@ struct BgmvParams {
   int pitchT;       // bytes per token row of tmp
   int lo_off;       // kinds 1, 2: bytes from a token's high halves to its low halves
   int kind;
-  int tmp_bytes;    // bytes of one tmp buffer
   int off_red, off_tmp, off_tab, off_bar;
   int full_k;       // every K part has all 1024 columns
   int y_cols;       // columns of y that the slices may touch (largest column end)
   int ksplit;       // 1: the K parts (not the rank rows) are dealt over the CTAs of a cluster
-  int pitchR, recv_bytes, off_recv;  // K split: floats per token row / bytes of one buffer of received partial sums
+  int pitchR, off_recv;  // K split: floats per token row of the received partial sums
   int use_pdl;
   int mode;         // 0 fused, 1 shrink only (tmp_io written), 2 expand only (tmp_io read), 3 overwrite y
   void* tmp_io;
@@ -192,9 +191,9 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     return;
   }
   // ---- bucket metadata (uniform across the cluster); barrier set-up overlaps the loads
-  // Extra cluster e looks after multiple m = (e + 1) * window of the window inside the sorted rows: if m lies behind the
+  // Extra cluster e looks after multiple m = (e + 1) * 16 inside the sorted rows: if m lies behind the
   // first row of a bucket [start, start + cnt), it is the i-th such multiple there, and the cluster takes the bucket's i-th
-  // window. (A bucket of cnt rows has ceil(cnt / window) - 1 windows beyond its first and at least that many multiples.)
+  // window. (A bucket of cnt rows has ceil(cnt / 16) - 1 windows beyond its first and at least that many multiples.)
   int window_no = 0;
   if (p.by_window) {
     // Fewer rows than buckets (graph buffers carry a bucket for every slot): the launch has a cluster for every window that T
@@ -208,7 +207,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
       for (int i = 0; i < 4; ++i) held[i] = b0 + 32 * i + lane < p.n_buckets ? p.counts[b0 + 32 * i + lane] : 0;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int windows = held[i] > 0 && held[i] <= p.T ? (held[i] + p.window - 1) / p.window : 0;
+        const int windows = held[i] > 0 && held[i] <= p.T ? (held[i] + kBgmvTok - 1) / kBgmvTok : 0;
         int upto = windows;
 #pragma unroll
         for (int d = 1; d < 32; d *= 2) {
@@ -227,7 +226,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   } else if (bucket >= p.n_buckets) {
     // (every warp looks for itself: most of these clusters find nothing, and the sooner they leave, the sooner the next launch
     // has their place)
-    const int m = (bucket - p.n_buckets + 1) * p.window;
+    const int m = (bucket - p.n_buckets + 1) * kBgmvTok;
     bucket = -1;
     for (int b0 = 0; b0 < p.n_buckets && bucket < 0; b0 += 128) {
       int lo[4], cnt4[4];
@@ -243,7 +242,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
         if (mine != 0) {
           const int owner = __ffs((int)mine) - 1;
           bucket = b0 + 32 * i + owner;
-          window_no = m / p.window - __shfl_sync(0xffffffffu, lo[i], owner) / p.window;
+          window_no = m / kBgmvTok - __shfl_sync(0xffffffffu, lo[i], owner) / kBgmvTok;
         }
       }
     }
@@ -256,17 +255,16 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   }
   const int slot = bucket >= 0 ? p.slot_ids[bucket] : -1;
   const int rows_all = bucket >= 0 ? p.counts[bucket] : 0, start_all = bucket >= 0 ? p.offsets[bucket] : 0;
-  const int cnt = min(p.window, rows_all - window_no * p.window);
-  const int start = start_all + window_no * p.window;
+  const int cnt = min(kBgmvTok, rows_all - window_no * kBgmvTok);
+  const int start = start_all + window_no * kBgmvTok;
 
   float* red = reinterpret_cast<float*>(smem + p.off_red);
   uint8_t* tmp_base = smem + p.off_tmp;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.off_bar);  // full[], empty[], tmp_ready[2]
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kBgmvMaxStages + 2);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.off_bar);  // full[], empty[], tmp_ready
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kBgmvMaxStages + 1);
   const uint32_t bar_base = smem_u32(bars);
   const uint32_t ring_base = smem_u32(smem);
-  // one barrier per tmp buffer: pass p uses barrier p & 1 in phase (p >> 1) & 1
-  const uint32_t tmp_ready_bars = bar_base + 8u * (uint32_t)(2 * kBgmvMaxStages);
+  const uint32_t tmp_ready_bar = bar_base + 8u * (uint32_t)(2 * kBgmvMaxStages);
   auto full_bar = [&](int s) { return bar_base + 8u * (uint32_t)s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (uint32_t)(kBgmvMaxStages + s); };
 
@@ -289,8 +287,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     mbar_init(full_bar(tid), 1);
     mbar_init(empty_bar(tid), kBgmvWarps);
     if (tid == 0) {
-      mbar_init(tmp_ready_bars, 1u);  // completed by byte count (st.async from every CTA of the cluster)
-      mbar_init(tmp_ready_bars + 8u, 1u);
+      mbar_init(tmp_ready_bar, 1u);  // completed by byte count (st.async from every CTA of the cluster)
       *abort_flag = 0;
     }
     mbar_fence_init();
@@ -326,15 +323,11 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
       tiles_exp += e_tiles[s];
     }
   }
-  const int npass = (cnt + kBgmvTok - 1) >> 4;
-  const int total = (shrink_tiles + tiles_exp) * npass;
-  // bytes a pass delivers into this CTA: 16 token rows of all Q stacked rank rows, as bf16 once
+  const int total = shrink_tiles + tiles_exp;
+  // bytes delivered into this CTA: 16 token rows of all Q stacked rank rows, as bf16 once
   // (all-gather) or as fp32 from every CTA of the cluster (K split)
-  const uint32_t gather_bytes = ksplit ? (uint32_t)(C * kBgmvTok * Q * 4) : (uint32_t)(kBgmvTok * Q * (kPrecise ? 4 : 2));
-  if (tid == 0 && (mode == 0 || mode >= 3)) {
-    mbar_arrive_expect_tx(tmp_ready_bars, gather_bytes);                      // pass 0
-    if (npass > 1) mbar_arrive_expect_tx(tmp_ready_bars + 8u, gather_bytes);  // pass 1
-  }
+  if (tid == 0 && (mode == 0 || mode >= 3))
+    mbar_arrive_expect_tx(tmp_ready_bar, ksplit ? (uint32_t)(C * kBgmvTok * Q * 4) : (uint32_t)(kBgmvTok * Q * (kPrecise ? 4 : 2)));
 
   __syncthreads();  // barriers initialised
   B200_TRACE_POINT(2)
@@ -387,20 +380,17 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
         if (i_qr >= r_eff) { i_qr = 0; ++i_qs; }
         if (i_j == nt_c) {
           i_j = 0; i_qs = q0_s; i_qr = q0_r;
-          // (shrink-only launches have no expand tiles: the next pass starts with shrink tiles again)
-          if (++i_kp == nkp_c) { i_kp = 0; i_shrink = tiles_exp > 0 ? 0 : 1; i_s = 0; i_et = 0; }
+          if (++i_kp == nkp_c) i_shrink = 0;
         }
       } else {
 #pragma unroll
         for (int s = 0; s < B200_LORA_MAX_SLICES - 1; ++s)  // skip slices this CTA has no tiles of
           if (i_s == s && i_et >= e_tiles[s]) { i_s = s + 1; i_et = 0; }
-        int lo = 0, en = 0, out = 0, left = 0;
+        int lo = 0, en = 0, out = 0;
         const void* bptr = nullptr;
 #pragma unroll
-        for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) {
-          if (s == i_s) { lo = e_lo[s]; en = e_n[s]; out = p.st.out[s]; bptr = p.st.b[s]; left = e_tiles[s]; }
-          if (s > i_s) left += e_tiles[s];
-        }
+        for (int s = 0; s < B200_LORA_MAX_SLICES; ++s)
+          if (s == i_s) { lo = e_lo[s]; en = e_n[s]; out = p.st.out[s]; bptr = p.st.b[s]; }
         const int r0 = i_et << p.er_shift;
         const int nrows = min(ER, en - r0);
         if (!B200_IN_BOUNDS(bptr != nullptr && nrows > 0 && lo + r0 + nrows <= out && p_stage < NS &&
@@ -415,12 +405,6 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
           bulk_g2s(sbase, src, bytes, fb);
         }
         ++i_et;
-        // `left` = tiles of this and later slices; after the last one the next pass starts
-        // with its shrink tiles again
-        if (i_et >= left) {
-          i_shrink = shrink_tiles > 0 ? 1 : 0;
-          i_kp = 0; i_j = 0; i_qs = q0_s; i_qr = q0_r; i_s = 0; i_et = 0;
-        }
       }
       __syncwarp();
       if (++p_stage == NS) { p_stage = 0; ++p_round; }
@@ -438,12 +422,12 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   // token rows, the table of this CTA's expand tiles, thread-constant address pieces and L2 prefetches of x
   // (a prefetch never creates stale data: L2 is the point of coherence). What runs after the wait is
   // the dependent chain activations -> shrink -> all-gather -> expand, kept as short as possible.
-  int tok0_lo = -1, tok0_hi = -1;
-  if (g < cnt) tok0_lo = p.sorted_idx[start + g];
-  if (g + 8 < cnt) tok0_hi = p.sorted_idx[start + g + 8];
-  (void)B200_IN_BOUNDS(tok0_lo < p.T && tok0_hi < p.T && tok0_lo >= -1 && tok0_hi >= -1);
-  if (tok0_lo >= p.T) tok0_lo = -1;
-  if (tok0_hi >= p.T) tok0_hi = -1;
+  int tok_lo = -1, tok_hi = -1;
+  if (g < cnt) tok_lo = p.sorted_idx[start + g];
+  if (g + 8 < cnt) tok_hi = p.sorted_idx[start + g + 8];
+  (void)B200_IN_BOUNDS(tok_lo < p.T && tok_hi < p.T && tok_lo >= -1 && tok_hi >= -1);
+  if (tok_lo >= p.T) tok_lo = -1;
+  if (tok_hi >= p.T) tok_hi = -1;
 
   // expand tile e of this CTA (ring order): x = first y column, y = rows | slice << 16
   int2* etab = reinterpret_cast<int2*>(smem + p.off_tab);
@@ -474,8 +458,8 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
       const int k0 = (kp0 + ikp * kstep) * KP;
 #pragma unroll 1
       for (int kc = k0 + x_col; kc < min(k0 + KP, in_dim); kc += kBgmvWarps * 32) {
-        if (tok0_lo >= 0) prefetch_l2(p.x + (int64_t)tok0_lo * p.x_ld + kc);
-        if (tok0_hi >= 0) prefetch_l2(p.x + (int64_t)tok0_hi * p.x_ld + kc);
+        if (tok_lo >= 0) prefetch_l2(p.x + (int64_t)tok_lo * p.x_ld + kc);
+        if (tok_hi >= 0) prefetch_l2(p.x + (int64_t)tok_hi * p.x_ld + kc);
       }
     }
   }
@@ -499,8 +483,6 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   const float* const red_rd = red + (size_t)it_tok * p.red_pitch + (it_q - q_lo);
   const uint32_t it_off = (uint32_t)(it_tok * p.pitchT + it_q * 2);
   const uint32_t tmp_u32 = smem_u32(tmp_base);
-  const uint32_t recv_u32 = smem_u32(smem + p.off_recv);
-  const uint32_t it_roff = (uint32_t)(it_tok * p.pitchR + it_q) * 4u;  // K split: the item inside one sender's block
 
   if (p.use_pdl) griddep_wait();  // x and y of this launch are final from here on
   if (kOverwrite) bgmv_fill_rows_without_delta(p, block_y * C + c, blocks_y * C, tid, kBgmvConsumers);
@@ -514,205 +496,177 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     if (++c_stage == NS) { c_stage = 0; c_parity ^= 1u; stage_addr = ring_base; }
   };
 
-#pragma unroll 1
-  for (int pass = 0; pass < npass; ++pass) {
-    int tok_lo = tok0_lo, tok_hi = tok0_hi;
-    if (pass > 0) {
-      tok_lo = tok_hi = -1;
-      if (pass * kBgmvTok + g < cnt) tok_lo = p.sorted_idx[start + pass * kBgmvTok + g];
-      if (pass * kBgmvTok + g + 8 < cnt) tok_hi = p.sorted_idx[start + pass * kBgmvTok + g + 8];
-      (void)B200_IN_BOUNDS(tok_lo < p.T && tok_hi < p.T && tok_lo >= -1 && tok_hi >= -1);
-      if (tok_lo >= p.T) tok_lo = -1;
-      if (tok_hi >= p.T) tok_hi = -1;
-    }
-    const __nv_bfloat16* const xlo_p = p.x + (int64_t)max(tok_lo, 0) * p.x_ld + x_col;
-    const __nv_bfloat16* const xhi_p = p.x + (int64_t)max(tok_hi, 0) * p.x_ld + x_col;
-    __nv_bfloat16* const ylo_p = p.y + (int64_t)max(tok_lo, 0) * p.y_ld + y_col;
-    __nv_bfloat16* const yhi_p = p.y + (int64_t)max(tok_hi, 0) * p.y_ld + y_col;
+  const __nv_bfloat16* const xlo_p = p.x + (int64_t)max(tok_lo, 0) * p.x_ld + x_col;
+  const __nv_bfloat16* const xhi_p = p.x + (int64_t)max(tok_hi, 0) * p.x_ld + x_col;
 
-    // ===== shrink: red[warp][tok][row] = x[16 tok, K blocks of this warp] . A_rows^T =====
+  // ===== shrink: red[warp][tok][row] = x[16 tok, K blocks of this warp] . A_rows^T =====
 #pragma unroll 1
-    for (int kp = 0; kp < (rows_c > 0 ? nkp_c : 0); ++kp) {
-      const int k0 = (kp0 + kp * kstep) * KP;
-      // activation fragments of this warp's 32-column blocks, kept for all row tiles
-      uint4 xlo[kBgmvXBlocks], xhi[kBgmvXBlocks];
+  for (int kp = 0; kp < (rows_c > 0 ? nkp_c : 0); ++kp) {
+    const int k0 = (kp0 + kp * kstep) * KP;
+    // activation fragments of this warp's 32-column blocks, kept for all row tiles
+    uint4 xlo[kBgmvXBlocks], xhi[kBgmvXBlocks];
+#pragma unroll
+    for (int i = 0; i < kBgmvXBlocks; ++i) {
+      xlo[i] = xhi[i] = make_uint4(0, 0, 0, 0);
+      if (kFullK || (x_col + 256 * i < KP && k0 + x_col + 256 * i < in_dim)) {
+        if (tok_lo >= 0) xlo[i] = ldg128_nc(xlo_p + k0 + 256 * i);
+        if (tok_hi >= 0) xhi[i] = ldg128_nc(xhi_p + k0 + 256 * i);
+      }
+    }
+    // kTiles (1 or 2) 8-row tiles of the ring against the warp's activation fragments: all loads
+    // first, then the independent MMA chains of both tiles, then the stores; sums of the K blocks go
+    // to the warp's rows of the reduction buffer (added to what earlier K parts left there)
+    auto shrink_tiles_fn = [&](auto n_tiles, int j, uint32_t addr0, uint32_t addr1) {
+      constexpr int kTiles = decltype(n_tiles)::value;
+      float acc[kTiles][2][4];
+#pragma unroll
+      for (int u = 0; u < kTiles; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) acc[u][h][0] = acc[u][h][1] = acc[u][h][2] = acc[u][h][3] = 0.f;
 #pragma unroll
       for (int i = 0; i < kBgmvXBlocks; ++i) {
-        xlo[i] = xhi[i] = make_uint4(0, 0, 0, 0);
-        if (kFullK || (x_col + 256 * i < KP && k0 + x_col + 256 * i < in_dim)) {
-          if (tok_lo >= 0) xlo[i] = ldg128_nc(xlo_p + k0 + 256 * i);
-          if (tok_hi >= 0) xhi[i] = ldg128_nc(xhi_p + k0 + 256 * i);
-        }
-      }
-      // kTiles (1 or 2) 8-row tiles of the ring against the warp's activation fragments: all loads
-      // first, then the independent MMA chains of both tiles, then the stores; sums of the K blocks go
-      // to the warp's rows of the reduction buffer (added to what earlier K parts left there)
-      auto shrink_tiles_fn = [&](auto n_tiles, int j, uint32_t addr0, uint32_t addr1) {
-        constexpr int kTiles = decltype(n_tiles)::value;
-        float acc[kTiles][2][4];
+        uint4 w[kTiles];
 #pragma unroll
-        for (int u = 0; u < kTiles; ++u)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) acc[u][h][0] = acc[u][h][1] = acc[u][h][2] = acc[u][h][3] = 0.f;
-#pragma unroll
-        for (int i = 0; i < kBgmvXBlocks; ++i) {
-          uint4 w[kTiles];
-#pragma unroll
-          for (int u = 0; u < kTiles; ++u) {
-            w[u] = make_uint4(0, 0, 0, 0);
-            if (kFullK || (x_col + 256 * i < KP && k0 + x_col + 256 * i < in_dim))
-              w[u] = lds128((u == 0 ? addr0 : addr1) + a_off + 512u * i);
-          }
-#pragma unroll
-          for (int u = 0; u < kTiles; ++u) {
-            mma_16816<kF16>(acc[u][0], xlo[i].x, xhi[i].x, xlo[i].y, xhi[i].y, w[u].x, w[u].y);
-            mma_16816<kF16>(acc[u][1], xlo[i].z, xhi[i].z, xlo[i].w, xhi[i].w, w[u].z, w[u].w);
-          }
+        for (int u = 0; u < kTiles; ++u) {
+          w[u] = make_uint4(0, 0, 0, 0);
+          if (kFullK || (x_col + 256 * i < KP && k0 + x_col + 256 * i < in_dim))
+            w[u] = lds128((u == 0 ? addr0 : addr1) + a_off + 512u * i);
         }
 #pragma unroll
         for (int u = 0; u < kTiles; ++u) {
-          // acc holds (tok g | g+8, rank rows 8(j+u)+2t, 8(j+u)+2t+1)
-          float2* r0 = reinterpret_cast<float2*>(red_wr + 8 * (j + u));
-          float2* r1 = reinterpret_cast<float2*>(red_wr + 8 * p.red_pitch + 8 * (j + u));
-          float2 a = make_float2(0.f, 0.f), b = a;
-          if (kp != 0) { a = *r0; b = *r1; }
-          *r0 = make_float2(a.x + acc[u][0][0] + acc[u][1][0], a.y + acc[u][0][1] + acc[u][1][1]);
-          *r1 = make_float2(b.x + acc[u][0][2] + acc[u][1][2], b.y + acc[u][0][3] + acc[u][1][3]);
-        }
-      };
-      int j = 0;
-#pragma unroll 1
-      for (; j + 1 < nt_c; j += 2) {
-        const int s0 = c_stage;
-        const uint32_t a0 = stage_addr;
-        mbar_wait_bounded(full_bar(s0), c_parity, abort_flag);
-        if (kp == 0 && j == 0 && pass == 0) { B200_TRACE_POINT(5) }
-        advance();
-        const int s1 = c_stage;
-        const uint32_t a1 = stage_addr;
-        mbar_wait_bounded(full_bar(s1), c_parity, abort_flag);
-        advance();
-        shrink_tiles_fn(std::integral_constant<int, 2>{}, j, a0, a1);
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive_relaxed(empty_bar(s0));
-          mbar_arrive_relaxed(empty_bar(s1));
+          mma_16816<kF16>(acc[u][0], xlo[i].x, xhi[i].x, xlo[i].y, xhi[i].y, w[u].x, w[u].y);
+          mma_16816<kF16>(acc[u][1], xlo[i].z, xhi[i].z, xlo[i].w, xhi[i].w, w[u].z, w[u].w);
         }
       }
-#pragma unroll 1
-      for (; j < nt_c; ++j) {
-        mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
-        if (kp == 0 && j == 0 && pass == 0) { B200_TRACE_POINT(5) }
-        shrink_tiles_fn(std::integral_constant<int, 1>{}, j, stage_addr, stage_addr);
-        __syncwarp();
-        if (lane == 0) mbar_arrive_relaxed(empty_bar(c_stage));
-        advance();
-      }
-    }
-    if (pass == 0) { B200_TRACE_POINT(6) }
-
-    // ===== cross-warp reduction of the K slices, scale, bf16, all-gather =====
-    // the barrier of pass + 1 is armed one pass ahead (passes 0 and 1 at start-up): every local wait on
-    // its previous phase is over, and no peer sends for pass + 1 before it has this pass from this CTA
-    if (tid == 0 && pass >= 1 && pass + 1 < npass && (mode == 0 || mode >= 3))
-      mbar_arrive_expect_tx(tmp_ready_bars + 8u * (uint32_t)((pass + 1) & 1), gather_bytes);
-    named_bar_sync(1, kBgmvConsumers);
-    if (pass == 0) {
-      B200_TRACE_POINT(7)
-      cluster_wait();  // start-up barrier: peers run and their barriers are initialised
-    }
-    const uint32_t tmp_cur = tmp_u32 + (uint32_t)((pass & 1) * p.tmp_bytes);
-    const uint32_t tmp_ready_bar = tmp_ready_bars + 8u * (uint32_t)(pass & 1);
-    if (mode == 2) {
-      // expand only: tmp of this pass comes from global memory (fp32 [n, T, r_max], summed over the
-      // tensor-parallel ranks) and is rounded to bf16 into this CTA's own buffer
-      uint8_t* tmp_full = tmp_base + (size_t)(pass & 1) * p.tmp_bytes;
-      const int tok = tid >> 4;
-      int trow = -1;
-      if (pass * kBgmvTok + tok < cnt) trow = p.sorted_idx[start + pass * kBgmvTok + tok];
-      if (trow >= p.T) trow = -1;
-#pragma unroll 1
-      for (int pr = tid & 15; pr < (Q >> 1); pr += 16) {
-        const int q = 2 * pr, s = q / r_eff, rr = q - s * r_eff;
-        const int64_t at = ((int64_t)s * p.T + trow) * p.r_max + rr;
-        uint32_t* const dst = reinterpret_cast<uint32_t*>(tmp_full + (size_t)tok * p.pitchT + (size_t)q * 2);
-        if (p.io16) {
-          *dst = trow >= 0 ? *reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(p.tmp_io) + at) : 0u;
-          if (kPrecise) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(dst) + p.lo_off) = 0u;
-        } else {
-          float2 v = make_float2(0.f, 0.f);
-          if (trow >= 0) v = *reinterpret_cast<const float2*>(static_cast<const float*>(p.tmp_io) + at);
-          const uint32_t h = pack_16x2<kF16>(v.x, v.y);
-          *dst = h;
-          if (kPrecise) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(dst) + p.lo_off) = pack_rest<kF16>(v.x, v.y, h);
-        }
-      }
-      named_bar_sync(1, kBgmvConsumers);
-    } else {
-      if (has_item) {
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int w = 0; w < kBgmvWarps; ++w) {
-          const float4 v = *reinterpret_cast<const float4*>(red_rd + (size_t)w * kBgmvTok * p.red_pitch);
-          a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
-        }
-        if (mode == 1) {
-          // shrink only: fp32 result of this CTA's rank rows straight to global memory
-          int trow = -1;
-          if (pass * kBgmvTok + it_tok < cnt) trow = p.sorted_idx[start + pass * kBgmvTok + it_tok];
-          if (trow >= 0 && trow < p.T) {
-            const int s = it_q / r_eff, rr = it_q - s * r_eff;
-            const int64_t at = ((int64_t)s * p.T + trow) * p.r_max + rr;
-            if (p.io16) {
-              *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.tmp_io) + at) =
-                  make_uint2(pack_16x2<kF16>(a.x * sc, a.y * sc), pack_16x2<kF16>(a.z * sc, a.w * sc));
-            } else {
-              float2* dst = reinterpret_cast<float2*>(static_cast<float*>(p.tmp_io) + at);
-              dst[0] = make_float2(a.x * sc, a.y * sc);
-              dst[1] = make_float2(a.z * sc, a.w * sc);
-            }
-          }
-        } else if (ksplit) {
-          // to every CTA of the cluster (this one included): this CTA's fp32 partial sums over its K parts,
-          // into the block the receiver keeps for this sender
-          const uint32_t dst = recv_u32 + (uint32_t)(((pass & 1) * C + c) * (kBgmvTok * p.pitchR * 4)) + it_roff;
+      for (int u = 0; u < kTiles; ++u) {
+        // acc holds (tok g | g+8, rank rows 8(j+u)+2t, 8(j+u)+2t+1)
+        float2* r0 = reinterpret_cast<float2*>(red_wr + 8 * (j + u));
+        float2* r1 = reinterpret_cast<float2*>(red_wr + 8 * p.red_pitch + 8 * (j + u));
+        float2 a = make_float2(0.f, 0.f), b = a;
+        if (kp != 0) { a = *r0; b = *r1; }
+        *r0 = make_float2(a.x + acc[u][0][0] + acc[u][1][0], a.y + acc[u][0][1] + acc[u][1][1]);
+        *r1 = make_float2(b.x + acc[u][0][2] + acc[u][1][2], b.y + acc[u][0][3] + acc[u][1][3]);
+      }
+    };
+    int j = 0;
 #pragma unroll 1
-          for (int rc = 0; rc < C; ++rc)
-            st_async_f32x4(mapa_shared(dst, (uint32_t)rc), a, mapa_shared(tmp_ready_bar, (uint32_t)rc));
-        } else {
-          // to every CTA of the cluster (this one included): 8 bytes of tmp + their count on the
-          // receiver's barrier in one operation
-          const uint32_t v0 = pack_16x2<kF16>(a.x * sc, a.y * sc), v1 = pack_16x2<kF16>(a.z * sc, a.w * sc);
-          const uint32_t l0 = kPrecise ? pack_rest<kF16>(a.x * sc, a.y * sc, v0) : 0u, l1 = kPrecise ? pack_rest<kF16>(a.z * sc, a.w * sc, v1) : 0u;
+    for (; j + 1 < nt_c; j += 2) {
+      const int s0 = c_stage;
+      const uint32_t a0 = stage_addr;
+      mbar_wait_bounded(full_bar(s0), c_parity, abort_flag);
+      if (kp == 0 && j == 0) { B200_TRACE_POINT(5) }
+      advance();
+      const int s1 = c_stage;
+      const uint32_t a1 = stage_addr;
+      mbar_wait_bounded(full_bar(s1), c_parity, abort_flag);
+      advance();
+      shrink_tiles_fn(std::integral_constant<int, 2>{}, j, a0, a1);
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive_relaxed(empty_bar(s0));
+        mbar_arrive_relaxed(empty_bar(s1));
+      }
+    }
 #pragma unroll 1
-          for (int rc = 0; rc < C; ++rc) {
-            st_async_b32x2(mapa_shared(tmp_cur + it_off, (uint32_t)rc), v0, v1, mapa_shared(tmp_ready_bar, (uint32_t)rc));
-            if (kPrecise)
-              st_async_b32x2(mapa_shared(tmp_cur + it_off + (uint32_t)p.lo_off, (uint32_t)rc), l0, l1, mapa_shared(tmp_ready_bar, (uint32_t)rc));
-          }
-        }
+    for (; j < nt_c; ++j) {
+      mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
+      if (kp == 0 && j == 0) { B200_TRACE_POINT(5) }
+      shrink_tiles_fn(std::integral_constant<int, 1>{}, j, stage_addr, stage_addr);
+      __syncwarp();
+      if (lane == 0) mbar_arrive_relaxed(empty_bar(c_stage));
+      advance();
+    }
+  }
+  B200_TRACE_POINT(6)
+
+  // ===== cross-warp reduction of the K slices, scale, bf16, all-gather =====
+  named_bar_sync(1, kBgmvConsumers);
+  B200_TRACE_POINT(7)
+  cluster_wait();  // start-up barrier: peers run and their barriers are initialised
+  if (mode == 2) {
+    // expand only: tmp comes from global memory (fp32 [n, T, r_max], summed over the
+    // tensor-parallel ranks) and is rounded to bf16 into this CTA's own buffer
+    const int tok = tid >> 4;
+    int trow = -1;
+    if (tok < cnt) trow = p.sorted_idx[start + tok];
+    if (trow >= p.T) trow = -1;
+#pragma unroll 1
+    for (int pr = tid & 15; pr < (Q >> 1); pr += 16) {
+      const int q = 2 * pr, s = q / r_eff, rr = q - s * r_eff;
+      const int64_t at = ((int64_t)s * p.T + trow) * p.r_max + rr;
+      uint32_t* const dst = reinterpret_cast<uint32_t*>(tmp_base + (size_t)tok * p.pitchT + (size_t)q * 2);
+      if (p.io16) {
+        *dst = trow >= 0 ? *reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(p.tmp_io) + at) : 0u;
+        if (kPrecise) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(dst) + p.lo_off) = 0u;
+      } else {
+        float2 v = make_float2(0.f, 0.f);
+        if (trow >= 0) v = *reinterpret_cast<const float2*>(static_cast<const float*>(p.tmp_io) + at);
+        const uint32_t h = pack_16x2<kF16>(v.x, v.y);
+        *dst = h;
+        if (kPrecise) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(dst) + p.lo_off) = pack_rest<kF16>(v.x, v.y, h);
+      }
+    }
+    named_bar_sync(1, kBgmvConsumers);
+  } else {
+    if (has_item) {
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < kBgmvWarps; ++w) {
+        const float4 v = *reinterpret_cast<const float4*>(red_rd + (size_t)w * kBgmvTok * p.red_pitch);
+        a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
       }
       if (mode == 1) {
-        named_bar_sync(1, kBgmvConsumers);  // all warps have read the reduction buffer before the next pass refills it
-        continue;
+        // shrink only: fp32 result of this CTA's rank rows straight to global memory
+        int trow = -1;
+        if (it_tok < cnt) trow = p.sorted_idx[start + it_tok];
+        if (trow >= 0 && trow < p.T) {
+          const int s = it_q / r_eff, rr = it_q - s * r_eff;
+          const int64_t at = ((int64_t)s * p.T + trow) * p.r_max + rr;
+          if (p.io16) {
+            *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.tmp_io) + at) =
+                make_uint2(pack_16x2<kF16>(a.x * sc, a.y * sc), pack_16x2<kF16>(a.z * sc, a.w * sc));
+          } else {
+            float2* dst = reinterpret_cast<float2*>(static_cast<float*>(p.tmp_io) + at);
+            dst[0] = make_float2(a.x * sc, a.y * sc);
+            dst[1] = make_float2(a.z * sc, a.w * sc);
+          }
+        }
+      } else if (ksplit) {
+        // to every CTA of the cluster (this one included): this CTA's fp32 partial sums over its K parts,
+        // into the block the receiver keeps for this sender
+        const uint32_t dst = smem_u32(smem + p.off_recv) + (uint32_t)((c * kBgmvTok + it_tok) * p.pitchR + it_q) * 4u;
+#pragma unroll 1
+        for (int rc = 0; rc < C; ++rc)
+          st_async_f32x4(mapa_shared(dst, (uint32_t)rc), a, mapa_shared(tmp_ready_bar, (uint32_t)rc));
+      } else {
+        // to every CTA of the cluster (this one included): 8 bytes of tmp + their count on the
+        // receiver's barrier in one operation
+        const uint32_t v0 = pack_16x2<kF16>(a.x * sc, a.y * sc), v1 = pack_16x2<kF16>(a.z * sc, a.w * sc);
+        const uint32_t l0 = kPrecise ? pack_rest<kF16>(a.x * sc, a.y * sc, v0) : 0u, l1 = kPrecise ? pack_rest<kF16>(a.z * sc, a.w * sc, v1) : 0u;
+#pragma unroll 1
+        for (int rc = 0; rc < C; ++rc) {
+          st_async_b32x2(mapa_shared(tmp_u32 + it_off, (uint32_t)rc), v0, v1, mapa_shared(tmp_ready_bar, (uint32_t)rc));
+          if (kPrecise)
+            st_async_b32x2(mapa_shared(tmp_u32 + it_off + (uint32_t)p.lo_off, (uint32_t)rc), l0, l1, mapa_shared(tmp_ready_bar, (uint32_t)rc));
+        }
       }
-      if (pass == 0) { B200_TRACE_POINT(8) }
-      // (the wait also orders the reduction buffer: no warp passes it before every warp of every CTA
-      // of the cluster has summed and sent its items, so the next pass may refill the buffer)
-      mbar_wait_bounded_acquire_cluster(tmp_ready_bar, (uint32_t)((pass >> 1) & 1), abort_flag);
+    }
+    if (mode != 1) {
+      B200_TRACE_POINT(8)
+      mbar_wait_bounded_acquire_cluster(tmp_ready_bar, 0u, abort_flag);
       if (ksplit) {
-        // add the C partial sums of this thread's item, scale, round: tmp of this pass, kept locally
+        // add the C partial sums of this thread's item, scale, round: tmp, kept locally
         if (has_item) {
           float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-          const float* src = reinterpret_cast<const float*>(smem + p.off_recv) + (size_t)(pass & 1) * C * kBgmvTok * p.pitchR +
-                             (size_t)it_tok * p.pitchR + it_q;
+          const float* src = reinterpret_cast<const float*>(smem + p.off_recv) + (size_t)it_tok * p.pitchR + it_q;
 #pragma unroll 1
           for (int rc = 0; rc < C; ++rc) {
             const float4 v = *reinterpret_cast<const float4*>(src + (size_t)rc * kBgmvTok * p.pitchR);
             a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
           }
           const uint32_t v0 = pack_16x2<kF16>(a.x * sc, a.y * sc), v1 = pack_16x2<kF16>(a.z * sc, a.w * sc);
-          uint8_t* dst = tmp_base + (size_t)(pass & 1) * p.tmp_bytes + it_off;
+          uint8_t* dst = tmp_base + it_off;
           *reinterpret_cast<uint2*>(dst) = make_uint2(v0, v1);
           if (kPrecise)
             *reinterpret_cast<uint2*>(dst + p.lo_off) =
@@ -720,120 +674,122 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
         }
         named_bar_sync(1, kBgmvConsumers);
       }
-      if (pass == 0) { B200_TRACE_POINT(9) }
+      B200_TRACE_POINT(9)
     }
-
-    // ===== expand: y[tok, cols] += tmp[16 tok, r] . B_rows^T ======================
-    // Rows of a stage beyond the tile's rows hold stale bytes; their products land in columns that are not written.
-    // kinds 1 and 2: y of the next tile is requested while this one is multiplied (the first one here, behind the wait)
-    uint4 y_next[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-    auto load_y = [&](int e) {
-      if (e >= tiles_exp || kF32Out || (kMode == 2 && p.no_add)) return;
-      const int2 te = etab[e];
-      if (y_col >= (te.y & 0xffff) || !B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) return;
-      if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + te.x);
-      if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + te.x);
-    };
-    if (kPrecise) load_y(sub);
-    auto expand_fn = [&](int e, uint32_t tile_addr) {
-      const int2 te = etab[e];
-      const uint4 y_lo = y_next[0], y_hi = y_next[1];
-      if (kPrecise) load_y(e + U);
-      float d[4][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.f;
-      const uint32_t a_addr = tmp_cur + t_off + (uint32_t)((te.y >> 16) * r_eff * 2);
-      const uint32_t w_addr = tile_addr + w_off;
-#pragma unroll 1
-      for (int kb = 0; kb < kblocks; ++kb) {
-        uint32_t a_kb = a_addr + 64u * kb, w_kb = w_addr + 64u * kb;
-        if (kPrecise) {
-          // this thread's eight columns start at 32 kb + 8 t of [high | low]; a_addr and w_addr already hold 16 t bytes
-          const int at = 32 * kb + 8 * t, low = at >= r_eff;
-          a_kb = a_addr + (uint32_t)(64 * kb + (low ? p.lo_off - 2 * r_eff : 0));
-          w_kb = w_addr + (uint32_t)(64 * kb - (low ? 2 * r_eff : 0));
-        }
-        const uint4 alo = lds128(a_kb);
-        const uint4 ahi = lds128(a_kb + 8u * (uint32_t)p.pitchT);
-        uint4 w[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) w[j] = lds128(w_kb + 2u * j * pitchB);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.x, ahi.x, alo.y, ahi.y, w[j].x, w[j].y);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.z, ahi.z, alo.w, ahi.w, w[j].z, w[j].w);
-      }
-      if (y_col < (te.y & 0xffff) && B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) {
-        if (kF32Out) {
-          float* const yf = reinterpret_cast<float*>(p.y) + te.x + y_col;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int tok = h ? tok_hi : tok_lo;
-            if (tok < 0) continue;
-            float4* const dst = reinterpret_cast<float4*>(yf + (int64_t)tok * p.y_ld);
-            dst[0] = make_float4(d[0][2 * h], d[0][2 * h + 1], d[1][2 * h], d[1][2 * h + 1]);
-            dst[1] = make_float4(d[2][2 * h], d[2][2 * h + 1], d[3][2 * h], d[3][2 * h + 1]);
-          }
-          return;
-        }
-        if (kPrecise) {
-          if (tok_lo >= 0)
-            stg128(ylo_p + te.x, make_uint4(add_16x2<kF16>(y_lo.x, d[0][0], d[0][1]), add_16x2<kF16>(y_lo.y, d[1][0], d[1][1]),
-                                            add_16x2<kF16>(y_lo.z, d[2][0], d[2][1]), add_16x2<kF16>(y_lo.w, d[3][0], d[3][1])));
-          if (tok_hi >= 0)
-            stg128(yhi_p + te.x, make_uint4(add_16x2<kF16>(y_hi.x, d[0][2], d[0][3]), add_16x2<kF16>(y_hi.y, d[1][2], d[1][3]),
-                                            add_16x2<kF16>(y_hi.z, d[2][2], d[2][3]), add_16x2<kF16>(y_hi.w, d[3][2], d[3][3])));
-          return;
-        }
-        const uint4 lo4 = make_uint4(pack_bf16x2(d[0][0], d[0][1]), pack_bf16x2(d[1][0], d[1][1]),
-                                     pack_bf16x2(d[2][0], d[2][1]), pack_bf16x2(d[3][0], d[3][1]));
-        const uint4 hi4 = make_uint4(pack_bf16x2(d[0][2], d[0][3]), pack_bf16x2(d[1][2], d[1][3]),
-                                     pack_bf16x2(d[2][2], d[2][3]), pack_bf16x2(d[3][2], d[3][3]));
-        if (kOverwrite) {
-          if (tok_lo >= 0) stg128(ylo_p + te.x, lo4);
-          if (tok_hi >= 0) stg128(yhi_p + te.x, hi4);
-        } else {
-          // The delta is rounded to bf16 and added to y by one 16-byte reduction at the L2: y never
-          // travels to the SM and nothing waits for it. Each element of y receives exactly one
-          // reduction per launch, so the result does not depend on their order.
-          if (tok_lo >= 0) red_add_bf16x8(ylo_p + te.x, lo4.x, lo4.y, lo4.z, lo4.w);
-          if (tok_hi >= 0) red_add_bf16x8(yhi_p + te.x, hi4.x, hi4.y, hi4.z, hi4.w);
-        }
-      }
-    };
-    if (!kWide) {
-#pragma unroll 1
-      for (int e = 0; e < tiles_exp; ++e) {
-        mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
-        if (pass == 0 && e < 10) { B200_TRACE_POINT(12 + 2 * e) }
-        expand_fn(e, stage_addr);
-        if (pass == 0 && e < 10) { B200_TRACE_POINT(13 + 2 * e) }
-        __syncwarp();
-        if (lane == 0) mbar_arrive_relaxed(empty_bar(c_stage));
-        advance();
-      }
-    } else {
-#pragma unroll 1
-    for (int e = 0; e < tiles_exp; e += U) {
-      // (every warp waits for every tile of the step: a wait that skipped phases of a stage could no longer tell them apart)
-      const int n_here = min(U, tiles_exp - e), stage0 = c_stage;
-      uint32_t mine = 0;
-#pragma unroll 1
-      for (int u = 0; u < n_here; ++u) {
-        mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
-        if (u == sub) mine = stage_addr;
-        advance();
-      }
-      if (sub < n_here) expand_fn(e + sub, mine);
-      __syncwarp();
-      if (lane < n_here) {
-        const int st = stage0 + lane;
-        mbar_arrive_relaxed(empty_bar(st >= NS ? st - NS : st));
-      }
-    }
-    }
-    if (pass == 0) { B200_TRACE_POINT(10) }
   }
+
+  // ===== expand: y[tok, cols] += tmp[16 tok, r] . B_rows^T ======================
+  // Rows of a stage beyond the tile's rows hold stale bytes; their products land in columns that are not written.
+  __nv_bfloat16* const ylo_p = p.y + (int64_t)max(tok_lo, 0) * p.y_ld + y_col;
+  __nv_bfloat16* const yhi_p = p.y + (int64_t)max(tok_hi, 0) * p.y_ld + y_col;
+  // kinds 1 and 2: y of the next tile is requested while this one is multiplied (the first one here, behind the wait)
+  uint4 y_next[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+  auto load_y = [&](int e) {
+    if (e >= tiles_exp || kF32Out || (kMode == 2 && p.no_add)) return;
+    const int2 te = etab[e];
+    if (y_col >= (te.y & 0xffff) || !B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) return;
+    if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + te.x);
+    if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + te.x);
+  };
+  if (kPrecise) load_y(sub);
+  auto expand_fn = [&](int e, uint32_t tile_addr) {
+    const int2 te = etab[e];
+    const uint4 y_lo = y_next[0], y_hi = y_next[1];
+    if (kPrecise) load_y(e + U);
+    float d[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.f;
+    const uint32_t a_addr = tmp_u32 + t_off + (uint32_t)((te.y >> 16) * r_eff * 2);
+    const uint32_t w_addr = tile_addr + w_off;
+#pragma unroll 1
+    for (int kb = 0; kb < kblocks; ++kb) {
+      uint32_t a_kb = a_addr + 64u * kb, w_kb = w_addr + 64u * kb;
+      if (kPrecise) {
+        // this thread's eight columns start at 32 kb + 8 t of [high | low]; a_addr and w_addr already hold 16 t bytes
+        const int at = 32 * kb + 8 * t, low = at >= r_eff;
+        a_kb = a_addr + (uint32_t)(64 * kb + (low ? p.lo_off - 2 * r_eff : 0));
+        w_kb = w_addr + (uint32_t)(64 * kb - (low ? 2 * r_eff : 0));
+      }
+      const uint4 alo = lds128(a_kb);
+      const uint4 ahi = lds128(a_kb + 8u * (uint32_t)p.pitchT);
+      uint4 w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = lds128(w_kb + 2u * j * pitchB);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.x, ahi.x, alo.y, ahi.y, w[j].x, w[j].y);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.z, ahi.z, alo.w, ahi.w, w[j].z, w[j].w);
+    }
+    if (y_col < (te.y & 0xffff) && B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) {
+      if (kF32Out) {
+        float* const yf = reinterpret_cast<float*>(p.y) + te.x + y_col;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int tok = h ? tok_hi : tok_lo;
+          if (tok < 0) continue;
+          float4* const dst = reinterpret_cast<float4*>(yf + (int64_t)tok * p.y_ld);
+          dst[0] = make_float4(d[0][2 * h], d[0][2 * h + 1], d[1][2 * h], d[1][2 * h + 1]);
+          dst[1] = make_float4(d[2][2 * h], d[2][2 * h + 1], d[3][2 * h], d[3][2 * h + 1]);
+        }
+        return;
+      }
+      if (kPrecise) {
+        if (tok_lo >= 0)
+          stg128(ylo_p + te.x, make_uint4(add_16x2<kF16>(y_lo.x, d[0][0], d[0][1]), add_16x2<kF16>(y_lo.y, d[1][0], d[1][1]),
+                                          add_16x2<kF16>(y_lo.z, d[2][0], d[2][1]), add_16x2<kF16>(y_lo.w, d[3][0], d[3][1])));
+        if (tok_hi >= 0)
+          stg128(yhi_p + te.x, make_uint4(add_16x2<kF16>(y_hi.x, d[0][2], d[0][3]), add_16x2<kF16>(y_hi.y, d[1][2], d[1][3]),
+                                          add_16x2<kF16>(y_hi.z, d[2][2], d[2][3]), add_16x2<kF16>(y_hi.w, d[3][2], d[3][3])));
+        return;
+      }
+      const uint4 lo4 = make_uint4(pack_bf16x2(d[0][0], d[0][1]), pack_bf16x2(d[1][0], d[1][1]),
+                                   pack_bf16x2(d[2][0], d[2][1]), pack_bf16x2(d[3][0], d[3][1]));
+      const uint4 hi4 = make_uint4(pack_bf16x2(d[0][2], d[0][3]), pack_bf16x2(d[1][2], d[1][3]),
+                                   pack_bf16x2(d[2][2], d[2][3]), pack_bf16x2(d[3][2], d[3][3]));
+      if (kOverwrite) {
+        if (tok_lo >= 0) stg128(ylo_p + te.x, lo4);
+        if (tok_hi >= 0) stg128(yhi_p + te.x, hi4);
+      } else {
+        // The delta is rounded to bf16 and added to y by one 16-byte reduction at the L2: y never
+        // travels to the SM and nothing waits for it. Each element of y receives exactly one
+        // reduction per launch, so the result does not depend on their order.
+        if (tok_lo >= 0) red_add_bf16x8(ylo_p + te.x, lo4.x, lo4.y, lo4.z, lo4.w);
+        if (tok_hi >= 0) red_add_bf16x8(yhi_p + te.x, hi4.x, hi4.y, hi4.z, hi4.w);
+      }
+    }
+  };
+  if (!kWide) {
+#pragma unroll 1
+    for (int e = 0; e < tiles_exp; ++e) {
+      mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
+      if (e < 10) { B200_TRACE_POINT(12 + 2 * e) }
+      expand_fn(e, stage_addr);
+      if (e < 10) { B200_TRACE_POINT(13 + 2 * e) }
+      __syncwarp();
+      if (lane == 0) mbar_arrive_relaxed(empty_bar(c_stage));
+      advance();
+    }
+  } else {
+#pragma unroll 1
+  for (int e = 0; e < tiles_exp; e += U) {
+    // (every warp waits for every tile of the step: a wait that skipped phases of a stage could no longer tell them apart)
+    const int n_here = min(U, tiles_exp - e), stage0 = c_stage;
+    uint32_t mine = 0;
+#pragma unroll 1
+    for (int u = 0; u < n_here; ++u) {
+      mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
+      if (u == sub) mine = stage_addr;
+      advance();
+    }
+    if (sub < n_here) expand_fn(e + sub, mine);
+    __syncwarp();
+    if (lane < n_here) {
+      const int st = stage0 + lane;
+      mbar_arrive_relaxed(empty_bar(st >= NS ? st - NS : st));
+    }
+  }
+  }
+  B200_TRACE_POINT(10)
   B200_TRACE_POINT(11)
   if (tid == 0 && *abort_flag != 0) atomicOr(&g_b200_status, kStatusWaitGaveUp);
 }
@@ -920,23 +876,23 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
     const double clusters = in_use + (b.T - 1) / kBgmvTok;
     if (C == 4 && ((bucket_bytes / 4 > 128 * 1024 && clusters * 8 <= resident && b.beside == 0) || (bucket_bytes / 4 >= 256 * 1024 && in_use * 8 <= resident))) C = 8;
   }
-  // K split: at least one K part (1024 columns) per CTA of the cluster and all rank rows in one CTA;
-  // the shrink-only / expand-only pair of the tensor-parallel exchange keeps the row split
+  // K split: at least one K part (1024 columns) per CTA of the cluster and all rank rows in one CTA, up to 20 KB of received
+  // partial sums (64 rank rows over 8 CTAs, 35 KB: one layer of 4096, rank 64, 1 / 16 rows 45 / 60 us, with the row split
+  // 40 / 53); the shrink-only / expand-only pair of the tensor-parallel exchange keeps the row split
   const int nkp_all = ceil_div_i(b.in_dim, kBgmvKP);
   const bool ksplit = bgmv_options().ksplit && C > 1 && (b.mode == 0 || b.mode >= 3) && nkp_all >= C && Q <= kBgmvMaxRc &&
-                      2 * C * kBgmvTok * (Q + 4) * 4 <= 40 * 1024;  // (received partial sums: more would cost the second CTA per SM)
+                      C * kBgmvTok * (Q + 4) * 4 <= 20 * 1024;
   if (!ksplit)
     while (C < 8 && round_up_i(ceil_div_i(Q, C), 8) > kBgmvMaxRc) C *= 2;
   const int Rc = ksplit ? Q : round_up_i(ceil_div_i(Q, C), 8);
   if (Rc > kBgmvMaxRc) { *why = "n_slices * r_max too large for one cluster"; return false; }
 
   BgmvParams p;
-  p.window = kBgmvTok;
-  // (a bucket of n rows has 1 + (n - 1) / window windows, the most with as many buckets in use as there are rows)
+  // (a bucket of n rows has 1 + (n - 1) / 16 windows, the most with as many buckets in use as there are rows)
   const int in_use_max = std::min(b.n_buckets, std::max(b.T, 1));
-  p.clusters = b.n_buckets + (b.T - 1) / p.window;
-  p.by_window = in_use_max + (b.T - in_use_max) / p.window < p.clusters && in_use_max < b.n_buckets ? 1 : 0;
-  if (p.by_window) p.clusters = in_use_max + (b.T - in_use_max) / p.window;
+  p.clusters = b.n_buckets + (b.T - 1) / kBgmvTok;
+  p.by_window = in_use_max + (b.T - in_use_max) / kBgmvTok < p.clusters && in_use_max < b.n_buckets ? 1 : 0;
+  if (p.by_window) p.clusters = in_use_max + (b.T - in_use_max) / kBgmvTok;
   p.y = static_cast<__nv_bfloat16*>(b.y); p.y_ld = b.y_ld;
   p.x = static_cast<const __nv_bfloat16*>(b.x); p.x_ld = b.x_ld;
   p.T = b.T; p.in_dim = b.in_dim; p.S = b.S; p.r_max = b.r_max; p.st = st;
@@ -965,7 +921,7 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   p.kind = b.kind;
   p.lo_off = Q * 2;
   p.pitchT = round_up_i(Q * (b.kind != 0 ? 4 : 2), 128) + 64;
-  p.tmp_bytes = round_up_i(kBgmvTok * p.pitchT, 128);
+  const int tmp_bytes = round_up_i(kBgmvTok * p.pitchT, 128);
   const int bar_bytes = 256;
   int exp_tiles = 0;
   for (int s = 0; s < st.n; ++s) exp_tiles += ceil_div_i(p.oc[s], p.ER);
@@ -973,8 +929,8 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   const int tab_bytes = round_up_i(std::max(exp_tiles, 1) * 8, 128);
   p.ksplit = ksplit ? 1 : 0;
   p.pitchR = Q + 4;
-  p.recv_bytes = ksplit ? C * kBgmvTok * p.pitchR * 4 : 0;
-  const int fixed = red_bytes + 2 * p.tmp_bytes + 2 * p.recv_bytes + tab_bytes + bar_bytes;
+  const int recv_bytes = ksplit ? round_up_i(C * kBgmvTok * p.pitchR * 4, 128) : 0;
+  const int fixed = red_bytes + tmp_bytes + recv_bytes + tab_bytes + bar_bytes;
   // ring: what fits beside a second CTA on the SM, unless the caller set a size (up to the whole SM)
   const int ring_bytes = bgmv_options().ring_kb > 0 ? bgmv_options().ring_kb * 1024
                                                     : std::max(kBgmvSmemCoResident - fixed - 256, std::max(2, 256 / p.ER) * p.stage_bytes);
@@ -985,8 +941,8 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   p.NS = NS;
   p.off_red = NS * p.stage_bytes;
   p.off_tmp = p.off_red + red_bytes;
-  p.off_recv = p.off_tmp + 2 * p.tmp_bytes;
-  p.off_tab = p.off_recv + 2 * p.recv_bytes;
+  p.off_recv = p.off_tmp + tmp_bytes;
+  p.off_tab = p.off_recv + recv_bytes;
   p.off_bar = p.off_tab + tab_bytes;
   p.full_k = (p.KP == kBgmvKP && b.in_dim % kBgmvKP == 0) ? 1 : 0;
   p.y_cols = 0;
