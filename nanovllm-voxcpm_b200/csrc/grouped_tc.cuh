@@ -1,23 +1,23 @@
 // Multi-LoRA add for bucketed batches on the Blackwell tensor cores, two launches: shrink (x . A^T, fp32 partial sums to
 // scratch) and expand (tmp . B^T, added to y), both in the weight-stationary form D^T = W . act^T: the adapter's rows are
-// the 128-row operand of tcgen05.mma and the bucket's tokens its N operand (16 .. 64 columns).
+// the 128-row operand of tcgen05.mma and the bucket's tokens its N operand (16 or 32 columns).
 //
-// Why this form. A bucket's weights are fetched once per 64 tokens and the cost of a tile does not depend on how many of
-// the 64 are in use, so a popular adapter (a Zipf batch, or a short prompt of a few hundred rows) costs about as much as a
-// rare one. The fused decode kernel (bgmv_fused.cuh) multiplies 16 tokens at a time and walks a popular bucket pass by
-// pass on the CTAs of one cluster; it stays the kernel of small adapters with few tokens each, where its single launch
-// is shorter than two.
+// Why this form. A bucket's weights are fetched once per 32 tokens, by CTAs that share the tiles of all buckets evenly. The
+// fused decode kernel (bgmv_fused.cuh) gives every 16 tokens a cluster of its own, which fetches the adapter again and takes
+// as long as its slowest cluster; it stays the kernel of most batches, because its single launch is shorter than two
+// (grouped_preferred has the line between them).
 //
-// Both kernels are persistent, one CTA per SM: every CTA builds the list of (bucket, 64-token chunk) pairs in use from the
+// Both kernels are persistent, one CTA per SM: every CTA builds the list of (bucket, 32-token chunk) pairs in use from the
 // index arrays (graph buffers carry one bucket per slot, most of them empty) and takes items of it in turn:
 //   shrink item = (chunk, group of slices whose rank rows fit the 128 rows, K part)
 //   expand item = (chunk, slice, run of 128-row output tiles)
 // Under programmatic dependent launch a CTA builds its list and fills its ring of weight tiles (TMA, 128 / 64 / 32-byte
-// swizzle) before it waits for the previous kernel; 100 KB of shared memory each, so that the CTA of the next launch is
-// resident beside the one that runs.
+// swizzle) before it waits for the previous kernel. Its ring is 84 KB, so that the CTA of the next launch is resident beside
+// it, or 196 KB where a launch streams many bytes (grouped_ring_bytes).
 //
 // Precision: tmp stays fp32 between the launches and is multiplied as the sum of two 16-bit numbers (hi + lo), the K parts
-// are added in fp32, and y is read, added to in fp32 and rounded once - what the per-token kernels compute.
+// are added in fp32, and y is read, added to in fp32 and rounded once - what the per-token kernels compute. Where the fused
+// decode kernel rounds the delta to bf16 and adds it at the L2, the delta is rounded here too (round_delta) and needs hi only.
 #pragma once
 
 #include "bgmv_fused.cuh"
@@ -38,18 +38,15 @@ constexpr int kGrpMaxStages = 12;
 constexpr int kGrpSMs = 148;
 
 struct GroupedArgs {
-  const uint8_t* x; int64_t x_ld;      // 16-bit elements
-  uint8_t* y; int64_t y_ld;
+  uint8_t* y; int64_t y_ld;            // 16-bit elements
   int T, in_dim, S, r, n;
   int out[B200_LORA_MAX_SLICES], col[B200_LORA_MAX_SLICES];
   const int32_t *sorted_idx, *slot_ids, *counts, *offsets;
-  const int32_t* token_to_slot;        // shrink: rows without adapter get zero rows (null: they are left alone)
   const int32_t* rank_per_slot; const float* scale_per_slot;
   int n_buckets;
   float scaling;
   int f16;                             // fp16 instead of bf16
-  void* tmp;                           // shrink result / expand input [parts, n, T, r]
-  int tmp_16bit;                       // tmp holds 16-bit values of the activations' type (one part), else fp32
+  float* tmp;                          // shrink result / expand input [parts, n, T, r]
   int parts, k_part;                   // K parts and their width (multiple of kGrpBK)
   int panels, w_bytes;                 // shrink: 64-column panels per stage, bytes of its lora_A part
   int whole_stage;                     // shrink: one slice per operand, its panels of a stage arrive in one copy (3-D map)
@@ -293,20 +290,6 @@ grouped_shrink_kernel(const __grid_constant__ GroupedMaps maps, const GroupedArg
     // epilogue: lane <-> stacked rank row, column <-> token
     const int quarter = warp & 3, q = quarter * 32 + lane;
     griddep_wait();  // the previous launch may still read the scratch
-    if (a.token_to_slot != nullptr) {
-      // rows without adapter: zero rows in every slice
-      for (int t = blockIdx.x; t < a.T; t += gridDim.x) {
-        const int sl = a.token_to_slot[t];
-        bool dead = sl < 0 || sl >= a.S;
-        if (!dead && a.rank_per_slot != nullptr) dead = a.rank_per_slot[sl] <= 0;
-        if (!dead) continue;
-        for (int e = tid - 64; e < a.n * a.r; e += 128) {
-          const int64_t at = ((int64_t)(e / a.r) * a.T + t) * a.r + e % a.r;
-          if (a.tmp_16bit) static_cast<uint16_t*>(a.tmp)[at] = 0;
-          else static_cast<float*>(a.tmp)[at] = 0.f;
-        }
-      }
-    }
     int job = 0;
     for (int i = blockIdx.x; i < items; i += gridDim.x, ++job) {
       const Item t = item_at(i);
@@ -331,12 +314,7 @@ grouped_shrink_kernel(const __grid_constant__ GroupedMaps maps, const GroupedArg
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
               const int row = __shfl_sync(0xffffffffu, tok, c + e);
-              if (mine && row >= 0 && row < a.T) {
-                const float d = j < rank ? __uint_as_float(v[e]) * sc : 0.f;
-                const int64_t at = (plane + row) * a.r + j;
-                if (a.tmp_16bit) static_cast<uint16_t*>(a.tmp)[at] = to_16bit(d, a.f16);
-                else static_cast<float*>(a.tmp)[at] = d;
-              }
+              if (mine && row >= 0 && row < a.T) a.tmp[(plane + row) * a.r + j] = j < rank ? __uint_as_float(v[e]) * sc : 0.f;
             }
           }
         }
@@ -368,7 +346,7 @@ grouped_expand_kernel(const __grid_constant__ GroupedMaps maps, const GroupedArg
   const uint32_t stage_bytes = (uint32_t)(kGrpRows * row_bytes);
   const uint32_t half_bytes = (uint32_t)(kGrpTok * row_bytes);  // one of hi / lo
   const uint32_t tmp_base = smem_base + (uint32_t)NS * stage_bytes;
-  const int halves = a.tmp_16bit || a.round_delta ? 1 : 2;  // (a delta that is rounded anyway does not need the low half)
+  const int halves = a.round_delta ? 1 : 2;  // (a delta that is rounded anyway does not need the low half)
   const uint32_t bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * (uint32_t)s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (uint32_t)(kGrpMaxStages + s); };
@@ -515,37 +493,27 @@ grouped_expand_kernel(const __grid_constant__ GroupedMaps maps, const GroupedArg
         float v[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = 0.f;
-        uint4 packed = make_uint4(0, 0, 0, 0), rest = packed;
         if (tok >= 0) {
-          if (a.tmp_16bit) {
-            packed = ldg128(static_cast<const uint16_t*>(a.tmp) + ((int64_t)t.s * a.T + tok) * r + 8 * p);
-          } else {
-            for (int part = 0; part < a.parts; ++part) {
-              const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(a.tmp) +
-                                                                  (((int64_t)part * a.n + t.s) * a.T + tok) * r + 8 * p);
-              const float4 f0 = __ldcg(src), f1 = __ldcg(src + 1);
-              v[0] += f0.x; v[1] += f0.y; v[2] += f0.z; v[3] += f0.w;
-              v[4] += f1.x; v[5] += f1.y; v[6] += f1.z; v[7] += f1.w;
-            }
+          for (int part = 0; part < a.parts; ++part) {
+            const float4* src = reinterpret_cast<const float4*>(a.tmp + (((int64_t)part * a.n + t.s) * a.T + tok) * r + 8 * p);
+            const float4 f0 = __ldcg(src), f1 = __ldcg(src + 1);
+            v[0] += f0.x; v[1] += f0.y; v[2] += f0.z; v[3] += f0.w;
+            v[4] += f1.x; v[5] += f1.y; v[6] += f1.z; v[7] += f1.w;
           }
         }
-        if (!a.tmp_16bit) {
-          uint32_t h[4], l[4];
+        uint32_t h[4], l[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint16_t h0 = to_16bit(v[2 * q], a.f16), h1 = to_16bit(v[2 * q + 1], a.f16);
-            const uint16_t l0 = to_16bit(v[2 * q] - from_16bit(h0, a.f16), a.f16), l1 = to_16bit(v[2 * q + 1] - from_16bit(h1, a.f16), a.f16);
-            h[q] = h0 | ((uint32_t)h1 << 16);
-            l[q] = l0 | ((uint32_t)l1 << 16);
-          }
-          packed = make_uint4(h[0], h[1], h[2], h[3]);
-          rest = make_uint4(l[0], l[1], l[2], l[3]);
+        for (int q = 0; q < 4; ++q) {
+          const uint16_t h0 = to_16bit(v[2 * q], a.f16), h1 = to_16bit(v[2 * q + 1], a.f16);
+          const uint16_t l0 = to_16bit(v[2 * q] - from_16bit(h0, a.f16), a.f16), l1 = to_16bit(v[2 * q + 1] - from_16bit(h1, a.f16), a.f16);
+          h[q] = h0 | ((uint32_t)h1 << 16);
+          l[q] = l0 | ((uint32_t)l1 << 16);
         }
         // TMA swizzle of a row of 128 / 64 / 32 bytes: 16-byte piece index XOR address bits 7..9 (8..7, 7)
         const int x = row_bytes == 128 ? (row & 7) : row_bytes == 64 ? ((row >> 1) & 3) : ((row >> 2) & 1);
         const uint32_t at = (uint32_t)(row * row_bytes + ((p ^ x) << 4));
-        sts128(hi + at, packed);
-        if (halves == 2) sts128(lo + at, rest);
+        sts128(hi + at, make_uint4(h[0], h[1], h[2], h[3]));
+        if (halves == 2) sts128(lo + at, make_uint4(l[0], l[1], l[2], l[3]));
       }
       fence_proxy_async_smem();
       mbar_arrive(tmp_full(tb));
@@ -673,7 +641,7 @@ inline size_t grouped_workspace_bytes(int T, int n_slices, int r_max) {
   return (size_t)std::min(kGrpMaxSplit, ceil_div_i(6 * kGrpSMs, chunks)) * n_slices * T * r_max * 4 + 256;
 }
 
-inline bool grouped_supported(const GroupedProblem& b, const char** why, bool with_x = true, bool with_y = true) {
+inline bool grouped_supported(const GroupedProblem& b, const char** why) {
   const char* dummy;
   if (why == nullptr) why = &dummy;
   if (b.dtype != B200_LORA_BF16 && b.dtype != B200_LORA_F16) { *why = "bf16 / fp16 only"; return false; }
@@ -686,14 +654,14 @@ inline bool grouped_supported(const GroupedProblem& b, const char** why, bool wi
     *why = "too many buckets or rows";
     return false;
   }
-  if (with_x && (b.in_dim % 8 != 0 || b.x_ld % 8 != 0 || !aligned16(b.x))) { *why = "x rows must be 16-byte pieces"; return false; }
-  if (with_y && (b.y_ld % 8 != 0 || !aligned16(b.y))) { *why = "y rows must be 16-byte aligned"; return false; }
+  if (b.in_dim % 8 != 0 || b.x_ld % 8 != 0 || !aligned16(b.x)) { *why = "x rows must be 16-byte pieces"; return false; }
+  if (b.y_ld % 8 != 0 || !aligned16(b.y)) { *why = "y rows must be 16-byte aligned"; return false; }
   bool any = false;
   for (int s = 0; s < b.st.n; ++s) {
     if (b.st.out[s] == 0) continue;
     any = true;
-    if (with_y && (b.st.out[s] % 8 != 0 || b.st.col[s] % 8 != 0)) { *why = "slice widths / offsets must be multiples of 8"; return false; }
-    if ((with_x && !aligned16(b.st.a[s])) || (with_y && !aligned16(b.st.b[s]))) { *why = "slabs must be 16-byte aligned"; return false; }
+    if (b.st.out[s] % 8 != 0 || b.st.col[s] % 8 != 0) { *why = "slice widths / offsets must be multiples of 8"; return false; }
+    if (!aligned16(b.st.a[s]) || !aligned16(b.st.b[s])) { *why = "slabs must be 16-byte aligned"; return false; }
   }
   if (!any) { *why = "no active slice"; return false; }
   return true;
@@ -733,7 +701,6 @@ inline int grouped_ring_bytes(const GroupedProblem& b) {
 
 inline GroupedArgs grouped_args(const GroupedProblem& b, SliceTable* active) {
   GroupedArgs a = {};
-  a.x = static_cast<const uint8_t*>(b.x); a.x_ld = b.x_ld;
   a.y = static_cast<uint8_t*>(b.y); a.y_ld = b.y_ld;
   a.T = b.T; a.in_dim = b.in_dim; a.S = b.S; a.r = b.r_max;
   active->n = 0;
@@ -787,14 +754,12 @@ inline int grouped_configure() {
   return B200_LORA_OK;
 }
 
-// tmp = scaling * x . A^T. *parts > 1 leaves up to that many fp32 partial sums (the number is written back); `zero_rows` (a token_to_slot map) also writes
-// zero rows for tokens without adapter.
-inline int grouped_shrink_launch(const GroupedProblem& b, void* tmp, int tmp_16bit, int* parts, const int32_t* zero_rows,
-                                 cudaStream_t stream) {
+// tmp = scaling * x . A^T as up to *parts fp32 partial sums (the number is written back)
+inline int grouped_shrink_launch(const GroupedProblem& b, float* tmp, int* parts, cudaStream_t stream) {
   SliceTable st;
   GroupedArgs a = grouped_args(b, &st);
   GroupedMaps maps;
-  a.tmp = tmp; a.tmp_16bit = tmp_16bit;
+  a.tmp = tmp;
   a.spg = std::min(a.n, kGrpRows / a.r);
   a.m_groups = ceil_div_i(a.n, a.spg);
   a.k_part = round_up_i(ceil_div_i(b.in_dim, *parts), kGrpBK);
@@ -805,7 +770,6 @@ inline int grouped_shrink_launch(const GroupedProblem& b, void* tmp, int tmp_16b
   while (a.panels > 1 && ring / (a.panels * (panel_w + panel_x)) < 4) --a.panels;
   a.k_part = round_up_i(a.k_part, a.panels * kGrpBK);
   *parts = a.parts = ceil_div_i(b.in_dim, a.k_part);
-  a.token_to_slot = zero_rows;
   if (int rc = grouped_configure()) return rc;
   a.whole_stage = a.spg == 1 && b.in_dim % kGrpBK == 0;
   for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) {
@@ -823,11 +787,11 @@ inline int grouped_shrink_launch(const GroupedProblem& b, void* tmp, int tmp_16b
   return grouped_launch(grouped_shrink_kernel, "grouped_shrink_kernel", kGrpSMs, kGrpShrinkThreads, smem, maps, a, stream);
 }
 
-inline int grouped_expand_launch(const GroupedProblem& b, const void* tmp, int tmp_16bit, int parts, int round_delta, cudaStream_t stream) {
+inline int grouped_expand_launch(const GroupedProblem& b, float* tmp, int parts, int round_delta, cudaStream_t stream) {
   SliceTable st;
   GroupedArgs a = grouped_args(b, &st);
   GroupedMaps maps;
-  a.tmp = const_cast<void*>(tmp); a.tmp_16bit = tmp_16bit; a.parts = parts; a.round_delta = round_delta;
+  a.tmp = tmp; a.parts = parts; a.round_delta = round_delta;
   if (int rc = grouped_configure()) return rc;
   for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) {
     if (s >= a.n) { maps.w[s] = maps.w[0]; continue; }
@@ -855,11 +819,11 @@ inline int grouped_add_launch(const GroupedProblem& b, void* workspace, size_t w
   if (!grouped_supported(b, &why)) return fail(B200_LORA_EUNSUPPORTED, "grouped kernels: %s", why);
   int parts;
   const size_t need = grouped_need(b, &parts);  // (256 bytes of it for the alignment)
-  const uintptr_t ws = (reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255;
   if (workspace == nullptr || workspace_bytes < need)
     return fail(B200_LORA_EWORKSPACE, "grouped kernels need %zu bytes of scratch, got %zu", need, workspace_bytes);
-  if (int rc = grouped_shrink_launch(b, reinterpret_cast<void*>(ws), 0, &parts, nullptr, stream)) return rc;
-  return grouped_expand_launch(b, reinterpret_cast<void*>(ws), 0, parts, round_delta, stream);
+  float* const tmp = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255);
+  if (int rc = grouped_shrink_launch(b, tmp, &parts, stream)) return rc;
+  return grouped_expand_launch(b, tmp, parts, round_delta, stream);
 }
 
 }  // namespace b200lora
