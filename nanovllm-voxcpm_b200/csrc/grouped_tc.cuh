@@ -675,17 +675,28 @@ inline int grouped_expected_chunks(const GroupedProblem& b) {
   return std::max(1, (int)(in_use + 0.5) + b.T / kGrpTok);
 }
 
-// Whether these kernels are the faster ones for a batch that the fused decode kernel takes too: once the adapters in use are
-// so large that the fused kernel's clusters no longer fit the GPU at once, what counts is an even deal of the bytes. us per
-// projection, fused / these, for adapters of rank 64 in 4096-wide layers: 222 MB in use (qkv, 384 rows over 96 adapters) 65 /
-// 47; gate_up, 433 MB: 123 / 84; 146 MB (qkv, 100 rows) 30 / 34; 98 MB (o): 30 / 28; down, whose input rows are longer
-// than its outputs, 92 MB (one of four ranks): 30 / 27, 222 MB: 97 / 47.
+// Whether these kernels are the faster ones for a batch that the fused decode kernel takes too: one slice at rank 64 with
+// input rows at least as long as its output (o and down) and large adapters, enough of them in use. There the fused kernel has
+// only 64 stacked rank rows to deal over a cluster and a long row of each to walk. With several slices its single launch is
+// the better choice: it loses up to 20 % where the second wave of its clusters holds few (75 to 110 adapters of even
+// popularity), and gains up to 45 % on skewed popularity, which the host does not see. us per projection, fused / these, for even and
+// for skewed (Zipf 1.1) popularity, bf16, rank 64, at the expected MB of adapters in use:
+//   14336 -> 4096: 95 35 / 30 and 32 / 27, 164 39 / 38 and 35 / 42, 222 70 / 50 and 66 / 47, 393 103 / 73 and 72 / 62, 681 168 /
+//   114 and 105 / 78. 7168 -> 4096: 113 42 / 33 and 25 / 34, 120 44 / 34 and 41 / 36, 166 46 / 41 and 44 / 43.
+//   6144 -> 2048: 106 30 / 32 and 29 / 27, 134 33 / 40 and 32 / 48, 174 54 / 40 and 31 / 37, 203 57 / 45 and 54 / 45, 303 62 / 60
+//   and 55 / 45. 4096 -> 4096: 134 35 / 40 and 33 / 46, 174 56 / 42 and 32 / 39, 303 64 / 61 and 57 / 48.
+//   2048 -> 2048 (0.5 MB an adapter): 151 28 / 39 and 24 / 33.
+//   Three slices, 4096 -> 6144: 184 50 / 45 and 29 / 53, 222 54 / 49 and 53 / 52, 296 58 / 61 and 56 / 59, 393 81 / 78 and 57 / 78.
+//   Two, 4096 -> 28672: 369 88 / 77 and 51 / 82, 445 96 / 90 and 94 / 91, 593 104 / 115 and 99 / 124, 785 147 / 139 and 100 / 121.
+//   Rank 32, 14336 -> 4096: 111 33 / 41 and 33 / 35, 229 51 / 67 and 50 / 55, 352 82 / 98 and 73 / 97.
 inline bool grouped_preferred(const GroupedProblem& b) {
   int64_t bytes = 0, out = 0;
+  int n = 0;
   for (int s = 0; s < b.st.n; ++s)
-    if (b.st.out[s] > 0) { bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + b.st.out[s]); out += b.st.out[s]; }
+    if (b.st.out[s] > 0) { bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + b.st.out[s]); out += b.st.out[s]; ++n; }
+  if (n != 1 || b.r_max != 64 || b.in_dim < out || bytes < 1000 * 1000) return false;
   const double nb = (double)b.n_buckets, in_use = nb * (1.0 - std::exp(-(double)b.T / nb));
-  return in_use * bytes >= (b.in_dim > out ? 85e6 : 150e6);
+  return in_use * bytes >= (bytes >= 1400 * 1000 ? 85e6 : 170e6);
 }
 
 // Shared memory of one CTA. Small batches: half an SM, so that the CTA of the next launch is resident beside the one that
