@@ -559,7 +559,19 @@ struct Projection {
   }
 };
 
-constexpr int64_t kFusedTiles = 100;  // (see `project` below)
+// Whether base product and delta of a prefill projection go in one kernel (csrc/linear_pair.cuh) instead of cuBLAS and the add
+// behind it. It saves the pass over y and a launch (with `silu`, the activation behind gate_up, a second pass and launch) and
+// needs tiles for the SMs: with fewer than 100, cuBLAS's smaller ones win. Whole steps, us, fused / separate: 4001 rows of 1024, 4 layers 888 /
+// 1120; 2000 rows of 2048, 3 layers 831 / 957; 1000 rows of 2048 (gate_up 384 tiles, the others 64 to 80) 582 / 609; 1000 rows
+// of 1024 (256, the others 32 to 40) 416 / 367.
+// Long products are bound by the power cap, and there it takes more energy per operation than cuBLAS, which outweighs the pass
+// from 4096 input columns on. us per layer of whole steps, everything separate / only this projection fused, 4096-wide: 4000
+// rows gate_up with the activation (940 GFLOP) 2131 / 2318, down (470) 2131 / 2244, o (134) 2131 / 2186; 2000 rows 1020 / 1093,
+// 1020 / 1063, 1029 / 1048; 1000 rows 540 / 516 (235), 540 / 547 (118), 540 / 541 (34). 2048-wide down (6144 columns): 4000 rows
+// (101) 692 / 705, 2000 rows (50) 355 / 348; its gate_up (2048 columns, 201 and 101) 692 / 651 and 355 / 323.
+inline bool fused_linear_wins(int64_t T, int64_t K, int64_t N, bool silu) {
+  return (T + 127) / 128 * ((N + 255) / 256) >= 100 && (K < 4096 || 2.0 * (double)T * (double)K * (double)N < (silu ? 300e9 : 60e9));
+}
 
 // prefill_layers(embeds, positions, cu_seqlens, max_seqlen, slot_mapping, cos, sin, layers, final_norm, metadata | None, heads,
 //                kv_heads, head_dim, intermediate, eps) -> (status, normed), or None
@@ -637,12 +649,7 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const Slices& sl = p.sl;
     const bool lora = sl.n > 0 && b.tts != nullptr;
     const int K = (int)src.size(1), N = (int)dst.size(1);
-    // Base product and delta in one kernel once its 128 x 256 tiles come near the number of SMs: it then saves the pass over y
-    // and a launch, with fewer tiles cuBLAS's smaller ones win. Whole steps, us, fused / separate: 4001 rows of 1024, 4 layers
-    // 888 / 1120; 2000 rows of 2048, 3 layers 831 / 957; 1000 rows of 2048 (gate_up 384 tiles, the others 64 to 80) 582 / 609;
-    // 1000 rows of 1024 (256, the others 32 to 40) 416 / 367.
-    const int64_t tiles = (T + 127) / 128 * ((N + 255) / 256);
-    if (lora && tiles >= kFusedTiles && K % 64 == 0 && (sl.r == 16 || sl.r == 32 || sl.r == 64)) {
+    if (lora && fused_linear_wins(T, K, N, false) && K % 64 == 0 && (sl.r == 16 || sl.r == 32 || sl.r == 64)) {
       rc = p_linear(dst.data_ptr(), N, src.data_ptr(), K, (int)T, K, p.w->data_ptr(), K, N, nullptr, sl.n, sl.a, sl.b, sl.out, sl.col, (int)sl.S,
                     (int)sl.r, nullptr, b.tts, 1.0f, ws, ws_bytes, stream);
       return;
@@ -655,7 +662,7 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   };
   // gate_up with the activation in its epilogue, by the same line (128 + 128 columns make a tile)
   auto silu_in_linear = [&](const Slices& sl) {
-    if ((T + 127) / 128 * ((2 * inter + 255) / 256) < kFusedTiles || H % 64 || inter % 32) return false;
+    if (!fused_linear_wins(T, H, 2 * inter, true) || H % 64 || inter % 32) return false;
     if (sl.n > 0 && b.tts != nullptr && sl.r != 16 && sl.r != 32 && sl.r != 64) return false;
     for (int q = 0; q < sl.n; ++q)
       if (sl.out[q] % 32 || sl.col[q] % 32) return false;
