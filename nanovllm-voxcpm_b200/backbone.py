@@ -319,6 +319,33 @@ class Decoder(nn.Module):
                 add_norm(linear(layer.mlp.down_proj, act), following)
         return normed
 
+    def _flash_is_faster(self, T: int, max_seqlen: int) -> bool:
+        """Which attention a native prefill step takes. The own kernel (``csrc/prefill_attention.cuh``) is built for few rows and
+        short, ragged prompts; a batch that keeps the GPU busy for long is bound by its ``mma.sync`` rate, and flash_attn has
+        the higher one. us, own / flash_attn, heads / kv heads x head dim: 16 / 2 x 64: 12 prompts of 330 rows 23 / 34, 8 of 1000
+        76 / 96, one of 4000 135 / 153, 6000 271 / 273, 8000 465 / 451, 12000 1020 / 908, 4 of 4000 471 / 434; 32 / 8 x 64: 24 of
+        330 76 / 124, one of 4000 242 / 245, 5000 371 / 357, 6000 525 / 473. 16 / 2 x 128: 12 of 330 39 / 49, one of 4000 237 /
+        261, 6000 505 / 496, 8 of 1000 139 / 131, one of 8000 874 / 811, 4 of 3000 519 / 458; 32 / 8 x 128: 12 of 330 75 / 88, 24
+        of 330 150 / 165, 16 of 450 158 / 167, 11 of 700 209 / 201, 4 of 1000 142 / 133, 3000 264 / 266, 8000 1724 / 1438."""
+        rows = self.cfg.num_heads * T
+        return rows * max_seqlen >= 600_000_000 if self.cfg.head_dim == 64 else rows >= 128_000 and max_seqlen > 500
+
+    def _flash_attend(self, step: AttentionStep):
+        try:
+            from flash_attn import flash_attn_varlen_func
+        except ImportError:
+            return None  # the own kernel takes every length
+
+        heads, kv_heads, dim = self.cfg.num_heads, self.cfg.num_kv_heads, self.cfg.head_dim
+
+        def attend(qkv: torch.Tensor) -> torch.Tensor:
+            q, k, v = qkv.view(-1, heads + 2 * kv_heads, dim).split([heads, kv_heads, kv_heads], dim=1)
+            out = flash_attn_varlen_func(q, k, v, step.cu_seqlens, step.cu_seqlens, step.max_seqlen, step.max_seqlen,
+                                         softmax_scale=dim ** -0.5, causal=True)
+            return out.view(-1, heads * dim)
+
+        return attend
+
     def _prefill_native(self, embeds, positions, step: AttentionStep) -> torch.Tensor | None:
         """An eager prefill step through ``prefill_layers`` (``csrc/binding.cpp``): the launches of all layers in one call. None
         for steps and layers that it does not cover (decode rows in the batch, tensor parallelism, biases, other types)."""
@@ -349,7 +376,8 @@ class Decoder(nn.Module):
             layers.append((layer.input_layernorm, layer.post_attention_layernorm, sa.k_cache, sa.v_cache, *projections))
         got = N.native().prefill_layers(
             embeds, positions, step.cu_seqlens, step.max_seqlen, step.slot_mapping, self.cos, self.sin, layers, self.norm,
-            meta, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.intermediate_size, cfg.rms_norm_eps)
+            meta, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.intermediate_size, cfg.rms_norm_eps,
+            self._flash_attend(step) if self._flash_is_faster(embeds.size(0), step.max_seqlen) else None)
         if got is None:
             return None
         N.check(got[0])

@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <optional>
 #include <vector>
 
 #include "../../include/b200_lora.h"
@@ -521,6 +522,7 @@ struct Projection {
   const at::Tensor* w = nullptr;
   Slices sl;
   const void* rank = nullptr;
+  at::Tensor held[2 + B200_LORA_MAX_SLICES];  // (attention may be a Python call, during which another thread may replace a parameter)
 
   bool read(PyObject* o, int64_t in, int64_t out, int dev) {
     if (!PyTuple_CheckExact(o) || PyTuple_GET_SIZE(o) != 5 || !PyDict_Check(PyTuple_GET_ITEM(o, 0))) return false;
@@ -533,6 +535,8 @@ struct Projection {
     if (w == nullptr || w->dim() != 2 || w->scalar_type() != at::kBFloat16 || !on(*w, dev) || !w->is_contiguous() || w->size(0) != out ||
         w->size(1) != in)
       return false;
+    held[0] = *w;
+    w = &held[0];
     if (PyTuple_GET_ITEM(o, 1) == Py_None) return true;
     PyObject **names, **wi, **ci;
     const Py_ssize_t n = items(PyTuple_GET_ITEM(o, 1), &names);
@@ -541,6 +545,7 @@ struct Projection {
     if (a == nullptr || a->scalar_type() != at::kBFloat16 || !on(*a, dev) || !a->is_contiguous() || a->dim() < 3 || a->dim() > 4 ||
         (a->dim() == 4 ? a->size(0) : 1) != n || a->size(-1) != in || a->size(-3) > INT32_MAX)
       return false;
+    held[1] = *a;
     sl.S = a->size(-3); sl.r = a->size(-2); sl.in = in;
     for (Py_ssize_t i = 0; i < n; ++i) {
       const int64_t width = PyLong_AsLongLong(wi[i]), column = PyLong_AsLongLong(ci[i]);
@@ -551,6 +556,7 @@ struct Projection {
           b->size(1) != width || b->size(2) != sl.r || column < 0 || column + width > out)
         return false;
       sl.a[sl.n] = static_cast<const char*>(a->data_ptr()) + i * sl.S * sl.r * in * 2;
+      held[2 + sl.n] = *b;
       sl.b[sl.n] = b->data_ptr();
       sl.out[sl.n] = (int32_t)width;
       sl.col[sl.n++] = (int32_t)column;
@@ -574,12 +580,13 @@ inline bool fused_linear_wins(int64_t T, int64_t K, int64_t N, bool silu) {
 }
 
 // prefill_layers(embeds, positions, cu_seqlens, max_seqlen, slot_mapping, cos, sin, layers, final_norm, metadata | None, heads,
-//                kv_heads, head_dim, intermediate, eps) -> (status, normed), or None
-// All layers of an eager bf16 prefill step. `layers`: (norm weight, norm weight, k_cache, v_cache, qkv, o, gate_up, down) with
+//                kv_heads, head_dim, intermediate, eps, attend | None) -> (status, normed), or None
+// All layers of an eager bf16 prefill step. attend: what to call for attention, attend(qkv) -> [T, heads * head_dim], or None for
+// lora_b200_prefill_attention. `layers`: (norm weight, norm weight, k_cache, v_cache, qkv, o, gate_up, down) with
 // projections as above. (Layer by layer from Python a step of 400 rows took 270 us of host time per layer, for 86 us of kernels.)
 PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 15) { PyErr_SetString(PyExc_TypeError, "prefill_layers takes 15 arguments"); return nullptr; }
+  if (nargs != 16) { PyErr_SetString(PyExc_TypeError, "prefill_layers takes 16 arguments"); return nullptr; }
   const at::Tensor* x = tensor_of(args[0]);
   if (x == nullptr || !x->is_cuda() || x->dim() != 2 || !x->is_contiguous() || x->scalar_type() != at::kBFloat16) return not_handled();
   const int dev = x->get_device();
@@ -636,7 +643,7 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   size_t ws_bytes;
   if (!workspace(Py_None, *x, need, &keep, &ws, &ws_bytes)) return nullptr;
 
-  at::AutoDispatchBelowADInplaceOrView no_autograd;
+  std::optional<at::AutoDispatchBelowADInplaceOrView> no_autograd(std::in_place);
   void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   const auto opt = x->options();
   at::Tensor normed = at::empty({T, H}, opt), hidden = at::empty({T, H}, opt), qkv = at::empty({T, qkv_width}, opt), attn = at::empty({T, q_size}, opt),
@@ -680,9 +687,26 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (rc == B200_LORA_OK)
       rc = p_rope(qkv.data_ptr(), qkv_width, (int)T, (int)hq, (int)hk, (int)d, pos.data_ptr<int64_t>(), cos.data_ptr(), sin.data_ptr(),
                   (int)cos.size(1), table, (int)cos.size(0), l.k->data_ptr(), l.v->data_ptr(), slots.data_ptr<int32_t>(), B200_LORA_BF16, stream);
-    if (rc == B200_LORA_OK)
+    if (rc == B200_LORA_OK && args[15] != Py_None) {
+      no_autograd.reset();  // (the callee dispatches as from Python)
+      PyObject* rows = THPVariable_Wrap(qkv);
+      PyObject* got = rows == nullptr ? nullptr : PyObject_CallOneArg(args[15], rows);
+      Py_XDECREF(rows);
+      const at::Tensor* t = got == nullptr ? nullptr : tensor_of(got);
+      if (t == nullptr || !on(*t, dev) || t->scalar_type() != at::kBFloat16 || t->dim() != 2 || t->size(0) != T || t->size(1) != q_size ||
+          !t->is_contiguous()) {
+        if (got != nullptr) PyErr_SetString(PyExc_TypeError, "attend must return contiguous bf16 rows of all heads");
+        Py_XDECREF(got);
+        Py_XDECREF(keep);
+        return nullptr;
+      }
+      attn = *t;
+      Py_DECREF(got);
+      no_autograd.emplace();
+    } else if (rc == B200_LORA_OK) {
       rc = p_attention(attn.data_ptr(), q_size, qkv.data_ptr(), qkv_width, (int)T, (int)hq, (int)hk, (int)d, cu.data_ptr<int32_t>(),
                        (int)cu.numel() - 1, (int)max_len, 1.0f / std::sqrt((float)d), stream);
+    }
     project(l.p[1], y, attn);
     add_norm(*l.ln2);
     if (rc == B200_LORA_OK && silu_in_linear(l.p[2].sl)) {

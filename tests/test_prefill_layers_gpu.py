@@ -43,10 +43,12 @@ def test_prefill_attention_matches_reference(heads, kv, dim, lens):
         at += n
 
 
-# rows from below to above the lines between the bucket, prefill and fused-linear kernels
+# rows from below to above the lines between the bucket, prefill and fused-linear kernels; attention by either kernel
+@pytest.mark.parametrize("flash", [False, True], ids=["own", "flash"])
 @pytest.mark.parametrize("with_lora", [True, False], ids=["lora", "base"])
 @pytest.mark.parametrize("dim,lens,r", [(64, [40, 1, 90], 16), (128, [300, 333], 32), (64, [700, 500, 3], 32)])
-def test_native_prefill_step_matches_layer_by_layer(dim, lens, r, with_lora):
+def test_native_prefill_step_matches_layer_by_layer(dim, lens, r, with_lora, flash, monkeypatch):
+    monkeypatch.setattr(BB.Decoder, "_flash_is_faster", lambda *a: flash)
     S, hidden, T = 5, 512, sum(lens)
     cfg = BB.DecoderConfig(hidden_size=hidden, num_heads=8, num_kv_heads=2, head_dim=dim, intermediate_size=768, num_layers=2,
                            max_position=1024, max_loras=S, max_lora_rank=r)
@@ -86,3 +88,26 @@ def test_native_prefill_step_matches_layer_by_layer(dim, lens, r, with_lora):
     assert ((got - want).float().norm() / want.float().norm()).item() < 1e-2
     for a, b in zip(got_caches, want_caches):
         assert ((a - b).float().norm() / b.float().norm()).item() < 1e-2
+
+
+def test_attention_callable_is_checked(monkeypatch):
+    cfg = BB.DecoderConfig(hidden_size=128, num_heads=2, num_kv_heads=1, head_dim=64, intermediate_size=128, num_layers=1, max_position=64,
+                           max_loras=2, max_lora_rank=16)
+    with torch.device(DEV):
+        model = BB.Decoder(cfg).to(torch.bfloat16)
+    model.allocate_kv_cache(1)
+    reset_lora_context()
+    step = BB.AttentionStep(True, torch.arange(4, device=DEV), cu_seqlens=torch.tensor([0, 4], dtype=torch.int32, device=DEV), max_seqlen=4)
+    embeds, positions = torch.zeros(4, 128, device=DEV, dtype=torch.bfloat16), torch.arange(4, device=DEV)
+    monkeypatch.setattr(BB.Decoder, "_flash_is_faster", lambda *a: True)
+    for bad in (lambda qkv: qkv, lambda qkv: qkv[:, :128], lambda qkv: None, lambda qkv: qkv[:, :128].float().contiguous()):
+        monkeypatch.setattr(BB.Decoder, "_flash_attend", lambda self, s, bad=bad: bad)
+        with pytest.raises(TypeError, match="attend"):
+            model._prefill_native(embeds, positions, step)
+
+    def fails(qkv):
+        raise KeyError("out of blocks")
+
+    monkeypatch.setattr(BB.Decoder, "_flash_attend", lambda self, s: fails)
+    with pytest.raises(KeyError, match="out of blocks"):
+        model._prefill_native(embeds, positions, step)
