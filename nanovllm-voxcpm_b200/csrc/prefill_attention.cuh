@@ -6,7 +6,7 @@
 // of eight warps keeps 16 rows (mma.sync m16n8k16, online softmax in registers, as in Dao, "FlashAttention-2", 2023). The
 // blocks with the longest key ranges are launched first. mma.sync and not tcgen05: for 4001 rows of 12 prompts the arithmetic
 // is 4 GFLOP, the time is latency of loads and of the softmax chain. Measured (16 / 2 heads of 64): 12 prompts of 330 rows 23 us,
-// one of 4000 135 us, one of 8000 465 us = 141 TFLOP/s of the causal half, which is what mma.sync with two 64-key stages gives; a
+// one of 4000 135 us, one of 8000 465 us = 282 TFLOP/s of the causal half, which is what mma.sync with two 64-key stages gives; a
 // caller with a faster kernel for long prompts takes that (backbone.py has the line and both sides of it).
 #pragma once
 
