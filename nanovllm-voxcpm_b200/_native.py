@@ -144,13 +144,13 @@ class NativeLibraryError(RuntimeError):
     pass
 
 
-def _load() -> ctypes.CDLL:
+def _load(kind=ctypes.CDLL) -> ctypes.CDLL:
     if not os.path.exists(LIB_PATH):
         raise NativeLibraryError(
             f"{LIB_PATH} is missing: build it with `python -m nanovllm_voxcpm_b200.build` "
             "(nvcc, sm_100a). This package has no fallback path."
         )
-    lib = ctypes.CDLL(LIB_PATH)
+    lib = kind(LIB_PATH)
     for name, (restype, argtypes) in _SIGNATURES.items():
         fn = getattr(lib, name)  # AttributeError if the build is stale
         fn.restype = restype
@@ -169,6 +169,18 @@ def lib() -> ctypes.CDLL:
     if _LIB is None:
         _LIB = _load()
     return _LIB
+
+
+_ATOMIC_LIB: ctypes.PyDLL | None = None
+
+
+def atomic_lib() -> ctypes.PyDLL:
+    """The same library with the GIL held during a call: for calls that launch several kernels around one shared scratch
+    buffer, between which another thread's call on the same stream must not come."""
+    global _ATOMIC_LIB
+    if _ATOMIC_LIB is None:
+        _ATOMIC_LIB = _load(ctypes.PyDLL)
+    return _ATOMIC_LIB
 
 
 BINDING_PATH = os.path.join(_HERE, "lib", "b200lora_binding.so")
@@ -267,6 +279,10 @@ def current_stream(device: torch.device) -> int:
     if _RAW_STREAM is not None:
         return _RAW_STREAM(device.index if device.index is not None else torch.cuda.current_device())
     return torch.cuda.current_stream(device).cuda_stream
+
+
+def with_index(device: torch.device) -> torch.device:
+    return device if device.index is not None or device.type != "cuda" else torch.device("cuda", torch.cuda.current_device())
 
 
 def on_device(device: torch.device):

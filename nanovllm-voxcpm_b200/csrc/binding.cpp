@@ -150,21 +150,27 @@ inline bool optional_vector(PyObject* o, at::ScalarType dt, int64_t S, int dev, 
   return true;
 }
 
-// Scratch of the tensor-core kernels: the caller's tensor, or the package's per-device buffer. That buffer only grows and an
-// outgrown one stays allocated, so the last one seen per device is asked again only when it is too small (asking costs 1 us).
+// Scratch of the tensor-core kernels: the caller's tensor, or the package's buffer of the current stream. That buffer only grows
+// and an outgrown one stays allocated, so the last one seen per device is asked again only when the stream is another one or it
+// is too small (asking costs 1 us). Calls that use it keep the GIL over their launches: another thread's on the same stream
+// must not come between them.
 // Returns a new reference in *keep (may be null); false with a Python error set.
 constexpr int kMaxDevices = 64;
-PyObject* scratch_seen[kMaxDevices] = {};
+struct ScratchSeen {
+  PyObject* buffer = nullptr;
+  void* stream = nullptr;
+} scratch_seen[kMaxDevices];
 bool workspace(PyObject* given, const at::Tensor& x, size_t need, PyObject** keep, void** ptr, size_t* bytes) {
   *keep = nullptr; *ptr = nullptr; *bytes = 0;
   PyObject* o = given;
   if (o == Py_None) {
     if (need == 0) return true;
     const int dev = x.get_device();
-    PyObject* seen = dev < kMaxDevices ? scratch_seen[dev] : nullptr;
-    if (seen != nullptr && (size_t)THPVariable_Unpack(seen).nbytes() >= need) {
-      Py_INCREF(seen);
-      *keep = seen;
+    void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+    ScratchSeen none, &seen = dev < kMaxDevices ? scratch_seen[dev] : none;
+    if (seen.buffer != nullptr && seen.stream == stream && (size_t)THPVariable_Unpack(seen.buffer).nbytes() >= need) {
+      Py_INCREF(seen.buffer);
+      *keep = seen.buffer;
     } else {
       PyObject* device = THPDevice_New(x.device());
       if (device == nullptr) return false;
@@ -173,7 +179,8 @@ bool workspace(PyObject* given, const at::Tensor& x, size_t need, PyObject** kee
       if (*keep == nullptr) return false;
       if (dev < kMaxDevices && THPVariable_Check(*keep)) {
         Py_INCREF(*keep);
-        Py_XSETREF(scratch_seen[dev], *keep);
+        seen.stream = stream;
+        Py_XSETREF(seen.buffer, *keep);
       }
     }
     o = *keep;
@@ -238,12 +245,9 @@ PyObject* add(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (!workspace(args[11], *x, scratch ? p_workspace_bytes((int)T, sl.n, (int)sl.r) : 0, &keep, &ws, &ws_bytes)) return nullptr;
   void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   const auto fn = args[12] == Py_True ? p_delta : p_add;
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = fn(y->data_ptr(), y->stride(0), x->data_ptr(), x->stride(0), (int)T, (int)sl.in, sl.n, sl.a, sl.b, sl.out, sl.col,
-          (int)sl.S, (int)sl.r, static_cast<const int32_t*>(rank), static_cast<const float*>(scale), k.tts, k.sorted, k.ids,
-          k.counts, k.offsets, k.n, (float)scaling, code, (int)impl, ws, ws_bytes, stream);
-  Py_END_ALLOW_THREADS
+  const int rc = fn(y->data_ptr(), y->stride(0), x->data_ptr(), x->stride(0), (int)T, (int)sl.in, sl.n, sl.a, sl.b, sl.out, sl.col,
+                    (int)sl.S, (int)sl.r, static_cast<const int32_t*>(rank), static_cast<const float*>(scale), k.tts, k.sorted, k.ids,
+                    k.counts, k.offsets, k.n, (float)scaling, code, (int)impl, ws, ws_bytes, stream);
   Py_XDECREF(keep);
   return PyLong_FromLong(rc);
   END_HANDLE_TH_ERRORS
@@ -409,12 +413,9 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   size_t ws_bytes;
   if (!workspace(Py_None, *x, p_workspace_bytes((int)T, sl.n, (int)sl.r), &keep, &ws, &ws_bytes)) return nullptr;
   void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = p_linear(out->data_ptr(), out->stride(0), x->data_ptr(), x->stride(0), (int)T, (int)in, w->data_ptr(), w->stride(0),
-                (int)out_total, bias, sl.n, sl.a, sl.b, sl.out, sl.col, (int)sl.S, (int)sl.r, static_cast<const float*>(scale),
-                static_cast<const int32_t*>(tts->data_ptr()), (float)scaling, ws, ws_bytes, stream);
-  Py_END_ALLOW_THREADS
+  const int rc = p_linear(out->data_ptr(), out->stride(0), x->data_ptr(), x->stride(0), (int)T, (int)in, w->data_ptr(), w->stride(0),
+                          (int)out_total, bias, sl.n, sl.a, sl.b, sl.out, sl.col, (int)sl.S, (int)sl.r, static_cast<const float*>(scale),
+                          static_cast<const int32_t*>(tts->data_ptr()), (float)scaling, ws, ws_bytes, stream);
   Py_XDECREF(keep);
   if (args[10] != Py_None) return Py_BuildValue("(iO)", rc, args[10]);
   return Py_BuildValue("(iN)", rc, THPVariable_Wrap(fresh));

@@ -102,32 +102,40 @@ def _i32(t: torch.Tensor | None, name: str) -> torch.Tensor | None:
 #: batches of at least this many rows use the tensor-core prefill kernels under IMPL_AUTO
 SGMV_MIN_TOKENS = 512
 
-_SCRATCH: dict[torch.device, torch.Tensor] = {}
+#: per (device, stream)
+_SCRATCH: dict[tuple[torch.device, int], torch.Tensor] = {}
+_SCRATCH_FLOOR: dict[torch.device, int] = {}
 #: buffers that were replaced by a larger one: a CUDA graph captured earlier may still write through their
 #: addresses, so they are kept for the life of the process instead of going back to the allocator
 _RETIRED_SCRATCH: list[torch.Tensor] = []
 
 
 def reserve_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Sizes the per-device scratch buffer up front (e.g. from ``max_num_batched_tokens`` x slices x
-    ``max_lora_rank`` before CUDA graphs are captured), so that it never has to grow later."""
-    return scratch_for(torch.device(device), int(nbytes))
+    """Sizes the scratch buffers of ``device`` up front (e.g. from ``max_num_batched_tokens`` x slices x
+    ``max_lora_rank`` before CUDA graphs are captured), so that they never have to grow later. Returns that of the
+    current stream; other streams get theirs, as large, with their first call."""
+    device = N.with_index(torch.device(device))
+    _SCRATCH_FLOOR[device] = max(int(nbytes), _SCRATCH_FLOOR.get(device, 0))
+    return scratch_for(device, int(nbytes))
 
 
 def scratch_for(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Per-device scratch buffer for the prefill kernels' rank-r intermediate.
+    """Scratch buffer of the current stream of ``device`` for the rank-r intermediate of the kernels that take two launches
+    (prefill batches, decode batches over many large adapters).
 
-    The reference allocates this intermediate on every call (``lora.py:302``); here one buffer per device
+    The reference allocates this intermediate on every call (``lora.py:302``); here one buffer per device and stream
     is reused, so steady-state calls (and CUDA-graph replays) allocate nothing. The buffer only grows, and a
-    buffer that is outgrown is never freed: its address may be baked into a captured graph. One buffer per
-    device means one stream at a time may run calls that use it (the runner's single stream); callers that
-    overlap streams pass their own ``workspace``."""
-    buf = _SCRATCH.get(device)
+    buffer that is outgrown is never freed: its address may be baked into a captured graph. Calls on different streams
+    may overlap; graphs captured on one stream share its buffer, so replays of two of them may not (or their calls pass
+    ``workspace``)."""
+    device = N.with_index(device)
+    key = (device, N.current_stream(device))
+    buf = _SCRATCH.get(key)
     if buf is None or buf.numel() < nbytes:
         if buf is not None:
             _RETIRED_SCRATCH.append(buf)
-        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _SCRATCH[device] = buf
+        buf = torch.empty(max(nbytes, _SCRATCH_FLOOR.get(device, 0), 1 << 20), dtype=torch.uint8, device=device)
+        _SCRATCH[key] = buf
     return buf
 
 
@@ -187,7 +195,8 @@ def launch_add(
     if workspace is None and x.dtype != torch.float32 and impl in (N.IMPL_AUTO, N.IMPL_SGMV, N.IMPL_GROUPED):
         workspace = scratch_for(x.device, N.workspace_bytes(T, len(a_slabs), r_max))
     with N.on_device(x.device):
-        rc = (N.lib().lora_b200_delta if overwrite else N.lib().lora_b200_add)(
+        lib = N.atomic_lib()  # (two launches around one scratch buffer)
+        rc = (lib.lora_b200_delta if overwrite else lib.lora_b200_add)(
             y_packed.data_ptr(), y_packed.stride(0), x.data_ptr(), x.stride(0), T, in_dim, len(a_slabs),
             N.ptr_array(a_slabs), N.ptr_array(b_slabs), N.int_array(out_sizes), N.int_array(col_offsets),
             S, r_max, N.ptr(rank_per_slot), N.ptr(scale_per_slot), tts.data_ptr(), N.ptr(srt), N.ptr(ids),
@@ -252,7 +261,7 @@ def linear_lora(
             )
         workspace = scratch_for(x.device, N.workspace_bytes(T, n, r_max))
     with N.on_device(x.device):
-        rc = N.lib().lora_b200_linear_lora(
+        rc = N.atomic_lib().lora_b200_linear_lora(
             out.data_ptr(), out.stride(0), x.data_ptr(), x.stride(0), T, in_dim, weight.data_ptr(), weight.stride(0),
             out_total, N.ptr(bias), n, N.ptr_array(a_slabs[:n]) if n else None, N.ptr_array(b_slabs[:n]) if n else None,
             N.int_array(out_sizes[:n]) if n else None, N.int_array(col_offsets[:n]) if n else None, S, r_max,

@@ -100,7 +100,7 @@ def shrink_allreduce_expand(y, x, a_slabs, b_slabs, out_sizes, col_offsets, meta
     tmp = exchange._tmp if exchange is not None and n * T * r_max <= exchange.capacity else scratch_for(x.device, n * T * r_max * 4 + 256)
     tmp_ptr = (tmp.data_ptr() + 255) & ~255
     with N.on_device(x.device):
-        N.check(N.lib().lora_b200_shrink_allreduce_expand(
+        N.check(N.atomic_lib().lora_b200_shrink_allreduce_expand(
             y.data_ptr(), y.stride(0), x.data_ptr(), x.stride(0), T, in_dim, n, N.ptr_array(a_slabs), N.ptr_array(b_slabs),
             N.int_array(out_sizes), N.int_array(col_offsets), S, r_max, N.ptr(_i32(rank_per_slot, "rank_per_slot")),
             N.ptr(scale_per_slot), N.ptr(_i32(tts, "token_to_slot")), N.ptr(_i32(srt, "sorted")), N.ptr(_i32(ids, "slot ids")),

@@ -3,6 +3,8 @@ CPU oracle at the edges of their tiles - one token, 16- and 32-token chunks and 
 tiles, K tails and K parts, every rank, popular buckets, mixed ranks, slots of rank 0 - through ``lora_b200_add`` with the
 kernel asked for by name."""
 
+from concurrent.futures import ThreadPoolExecutor
+
 import pytest
 import torch
 
@@ -155,3 +157,29 @@ def test_auto_takes_the_grouped_kernels_with_the_scratch_that_the_query_names():
     # one rounding of the sum to bf16 (and of the delta): outputs of size 4 to 8 have steps of 2^-5
     ref = O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets)
     assert_lora_close(grouped, ref, max_abs=2 * ref.abs().max().item() * 2 ** -8, what="grouped")
+
+
+def test_two_launch_kernels_on_two_streams_at_once():
+    """Calls that keep an intermediate in the package's scratch, from two threads on streams of their own and then on one stream."""
+    T, S, r, rounds = 96, 6, 64, 30
+    p = [W.make_projection(600 + i, T, 2048, [2048], S, r, p_none=0.0) for i in range(2)]
+    d = [q.to_device(DEV) for q in p]
+    meta = [metadata_for(q.token_to_slot, "graph", S) for q in p]
+
+    def run(i, stream):
+        y = d[i].y.clone()
+        with torch.cuda.stream(stream):
+            stream.wait_stream(torch.cuda.default_stream())
+            for _ in range(rounds):
+                LORA.launch_add(y, d[i].x, d[i].a_slabs, d[i].b_slabs, d[i].out_sizes, d[i].col_offsets, meta[i], 0.01, impl=N.IMPL_GROUPED)
+        stream.synchronize()
+        return y
+
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    want = [run(i, streams[i]) for i in range(2)]
+    with ThreadPoolExecutor(2) as pool:
+        for pair in (streams, [streams[0]] * 2):
+            got = list(pool.map(run, range(2), pair))
+            for i in range(2):
+                assert torch.equal(got[i], want[i])
+    assert N.device_status(reset=True) == 0
