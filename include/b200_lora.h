@@ -218,8 +218,8 @@ int lora_b200_expand_buckets(void* y, int64_t y_ld, const void* tmp, int32_t tmp
  * allocates that intermediate with torch.empty on every call.
  *
  * Limits and rules:
- *  - the batch must fit the built-in scratch: lora_b200_workspace_bytes(T, active slices,
- *    r_max) <= lora_b200_static_scratch_bytes() (8 MiB); larger batches are rejected with
+ *  - the batch must fit the built-in scratch: (active slices * T + 128) * r_max * 2 + 1024 bytes
+ *    <= lora_b200_static_scratch_bytes() (8 MiB); larger batches are rejected with
  *    B200_LORA_EWORKSPACE and nothing is launched;
  *  - bf16 only, shapes as for B200_LORA_IMPL_SGMV (r_max 16/32/64, in % 64 == 0);
  *  - the first call on each GPU looks up the array's device address (cudaGetSymbolAddress,

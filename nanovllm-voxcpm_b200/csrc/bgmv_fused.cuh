@@ -4,9 +4,10 @@
 //   grid = (C, clusters), thread-block cluster = (C, 1, 1). Bucket g of the batch is the tokens
 //   sorted_idx[offsets[g] .. +counts[g]), which all use adapter slot slot_ids[g]; it is cut into
 //   windows of 16 tokens (one MMA M tile), and a cluster takes one window. There is a cluster per
-//   bucket, for its first window, and extra ones for the further windows of popular buckets
-//   (clusters of two passes: 256 rows over 32 adapters of skewed popularity, four layers of 1024,
-//   94 -> 133 us); with fewer rows than buckets there is one per window that the rows can make.
+//   bucket, for its first window, and extra ones for the further windows of popular buckets (256
+//   rows over 32 adapters of skewed popularity, four layers of 1024: 92 us; with 32 rows per cluster
+//   in two passes 133, with a whole bucket in one cluster 315). With fewer rows than buckets there is
+//   one per window that the rows can make.
 //   Clusters without rows exit at once.
 //   Inside a cluster the adapter's weights are split so that every byte of
 //   lora_A[slot] and lora_B[slot] is pulled from HBM by exactly one CTA:
