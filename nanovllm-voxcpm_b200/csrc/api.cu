@@ -9,6 +9,7 @@
 #include "glue.cuh"
 #include "sgmv_tc.cuh"
 #include "gemm_tc.cuh"
+#include "prefill_cluster.cuh"
 #include "linear_pair.cuh"
 #include "grouped_tc.cuh"
 #include "decode_step.cuh"
@@ -98,19 +99,25 @@ int launch_generic_expand(void* y, int64_t y_ld, const void* tmp, int T_rows, co
 
 namespace {
 
-// Whether a bf16 batch is large enough for the prefill kernels (at least 11 us for the pair, the adapters read once per 128
-// rows) rather than the bucket kernel (3 to 5 us, the adapters read once per 16 rows): from 512 rows on, by the adapter bytes
-// that the bucket kernel would read. us per projection, bucket / prefill kernels, six prompts of different adapters: 1024-wide,
-// rank 32, 900 rows, qkv (16 MB) 6.7 / 13.5, gate_up (37 MB) 8.9 / 15.1, 1500 rows 11.5 / 13.8 and (61 MB) 18.6 / 20.4;
-// 2048-wide, rank 32, 900 rows, gate_up (59 MB) 19.0 / 19.1, 1500 rows (98 MB) 32.9 / 24.7, qkv (52 MB) 16.4 / 16.3; rank 64,
-// 900 rows, qkv (63 MB) 18.8 / 17.0, 1500 rows 33.2 / 19.3. Above rank 32 the line stays at 512 rows: rank 64, 600 rows, the
-// mean of the four projections 17.0 / 16.1, 900 rows 20.4 / 17.8.
-constexpr int64_t kPrefillMinBytes = 50ll * 1000 * 1000;
-inline bool prefill_sized(int32_t T, const SliceTable& st, int32_t r_max, int32_t in_dim, bool expand) {
+// Whether a bf16 batch is large enough for the prefill kernels rather than the bucket kernel (3 to 5 us, an adapter read once per
+// 16 rows of it, in windows of which 74 by 4 CTAs are resident), from 512 rows on, by rows and by the adapter bytes that the
+// bucket kernel would read.
+//   prefill_cluster_kernel (adds): us per projection, bucket / prefill kernel, two to eight prompts. 1024-wide, rank 32: 1000 rows
+//   qkv (18 MB) 7.0 / 10.5, gate_up (41 MB) 9.3 / 13.1, 1300 rows 10 / 10.5 and 15 / 13.1, 2200 rows 14 / 11.7 and 22 / 19;
+//   2048-wide, rank 32: 1000 rows qkv (35 MB) 9.4 / 11.8, gate_up (66 MB) 20 / 16, 1500 rows 16 / 12.7 and 32 / 19; rank 64: 700 rows
+//   qkv (49 MB) 16.7 / 14.1, down (46 MB) 23 / 11.2, o (23 MB) 7.5 / 9.5. Over 900 measured points of 300 to 3200 rows, three
+//   widths and ranks, this line is 1.2 % slower than the better choice each time (the line below: 6.2 %).
+//   sgmv_shrink_kernel and the launch behind it (operators, slices that do not tile the output; at least 11 us for the pair): bucket /
+//   pair, six prompts: 1024-wide, rank 32, 900 rows, qkv (16 MB) 6.7 / 13.5, gate_up (37 MB) 8.9 / 15.1, 1500 rows 11.5 / 13.8 and
+//   (61 MB) 18.6 / 20.4; 2048-wide, rank 32, 900 rows, gate_up (59 MB) 19.0 / 19.1, 1500 rows (98 MB) 32.9 / 24.7; rank 64, 900
+//   rows, qkv (63 MB) 18.8 / 17.0, 1500 rows 33.2 / 19.3.
+inline bool prefill_sized(int32_t T, const SliceTable& st, int32_t r_max, int32_t in_dim, bool expand, bool one_launch) {
   int64_t bytes = 0;
   for (int s = 0; s < st.n; ++s)
     if (st.out[s] > 0 || !expand) bytes += 2 * (int64_t)r_max * (in_dim + (expand ? st.out[s] : 0));
-  return T >= kSgmvAutoMinTokens && (r_max > 32 || ceil_div_i(T, kBgmvTok) * bytes > kPrefillMinBytes);
+  bytes *= ceil_div_i(T, kBgmvTok);
+  if (T < kSgmvAutoMinTokens) return false;
+  return r_max > 32 || (one_launch ? ceil_div_i(T, kBgmvTok) > 74 || bytes > 35 * 1000 * 1000 : bytes > 50 * 1000 * 1000);
 }
 
 }  // namespace
@@ -524,7 +531,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     bp.kind = 0;
     bp.mode = 3;
     bp.token_to_slot = token_to_slot;
-    const bool decode_like = T < 32 * n_buckets || !prefill_sized(T, st, r_max, in_dim, true);
+    const bool decode_like = T < 32 * n_buckets || !prefill_sized(T, st, r_max, in_dim, true, prefill_cluster_add_ok(sp));
     if (dtype == B200_LORA_BF16 && have_buckets &&
         (impl == B200_LORA_IMPL_BGMV || (impl == B200_LORA_IMPL_AUTO && decode_like)) && bgmv_supported(bp, nullptr))
       return bgmv_launch(bp, st_);
@@ -538,7 +545,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
       if (dtype == B200_LORA_BF16 && (impl == B200_LORA_IMPL_SGMV || (impl == B200_LORA_IMPL_AUTO && !decode_like)) &&
           sgmv_supported(sp, nullptr) && prefill_overwrite_ok(st) && workspace != nullptr &&
           workspace_bytes >= sgmv_workspace_bytes(T, n_act, r_max))
-        return prefill_add_launch(sp, workspace, workspace_bytes, st_, true);
+        return prefill_add(sp, workspace, workspace_bytes, st_, true);
     }
     fill_neg_zero_kernel<<<(unsigned)T, 128, 0, st_>>>(y, y_ld, st, dtype == B200_LORA_F32 ? 4 : 2);
     if (int rc = check_launch("fill_neg_zero_kernel")) return rc;
@@ -554,7 +561,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     // want request-contiguous rows: with bucket arrays at hand, fewer than 32 rows per bucket on
     // average means a decode-like batch (slots scattered over the rows) and goes to the bucket kernel.
     const bool scattered = bgmv_ok && T < 32 * n_buckets;
-    if (dtype == B200_LORA_BF16 && !scattered && (!bgmv_ok ? T >= kSgmvAutoMinTokens : prefill_sized(T, st, r_max, in_dim, true)) && sgmv_supported(sp, nullptr) &&
+    if (dtype == B200_LORA_BF16 && !scattered && (!bgmv_ok ? T >= kSgmvAutoMinTokens : prefill_sized(T, st, r_max, in_dim, true, prefill_cluster_add_ok(sp))) && sgmv_supported(sp, nullptr) &&
         workspace != nullptr && workspace_bytes >= sgmv_workspace_bytes(T, n_act, r_max))
       impl = B200_LORA_IMPL_SGMV;
     else if (bgmv_ok && grouped_preferred(gp) && grouped_supported(gp, nullptr) && workspace != nullptr &&
@@ -585,7 +592,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     }
     case B200_LORA_IMPL_SGMV:
       if (dtype != B200_LORA_BF16) return fail(B200_LORA_EUNSUPPORTED, "prefill kernels are bf16 only");
-      return prefill_add_launch(sp, workspace, workspace_bytes, st_);
+      return prefill_add(sp, workspace, workspace_bytes, st_);
     case B200_LORA_IMPL_GROUPED:
       // (where the fused decode kernel takes the batch too, the delta is rounded to bf16 and added at the L2 as there)
       return grouped_add_launch(gp, workspace, workspace_bytes, dtype == B200_LORA_BF16 && r_max % 32 == 0, st_);
@@ -647,7 +654,7 @@ int lora_b200_shrink_buckets(void* out, int32_t out_dtype, const void* x, int64_
   bp.n_buckets = n_buckets; bp.scaling = scaling; bp.mode = 1; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
   bp.tmp_io = out; bp.io16 = out_dtype != B200_LORA_F32; bp.zero_rows = 1; bp.token_to_slot = token_to_slot;
   const bool by_bucket = buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && aligned16(out) && bgmv_supported(bp, nullptr);
-  const bool prefill = by_bucket ? T >= 32 * n_buckets && prefill_sized(T, st, r_max, in_dim, false) : T >= kSgmvAutoMinTokens;
+  const bool prefill = by_bucket ? T >= 32 * n_buckets && prefill_sized(T, st, r_max, in_dim, false, false) : T >= kSgmvAutoMinTokens;
   if (dtype == B200_LORA_BF16 && out_dtype == B200_LORA_BF16 && prefill) {
     // prefill-sized bf16 batches: the tensor-core shrink (rows without adapter are written as zeros, as the
     // per-token kernel does); anything it does not take falls through
@@ -705,7 +712,7 @@ int lora_b200_expand_buckets(void* y, int64_t y_ld, const void* tmp, int32_t tmp
   bp.n_buckets = n_buckets; bp.scaling = 1.0f; bp.mode = 2; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
   bp.tmp_io = const_cast<void*>(tmp); bp.io16 = tmp_dtype != B200_LORA_F32; bp.no_add = add_inputs ? 0 : 1; bp.token_to_slot = token_to_slot;
   const bool by_bucket = buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && dense && aligned16(tmp) && bgmv_supported(bp, nullptr);
-  const bool prefill = by_bucket ? T >= 32 * n_buckets && prefill_sized(T, st, r_max, 0, true) : T >= kSgmvAutoMinTokens;
+  const bool prefill = by_bucket ? T >= 32 * n_buckets && prefill_sized(T, st, r_max, 0, true, false) : T >= kSgmvAutoMinTokens;
   if (dtype == B200_LORA_BF16 && tmp_dtype == B200_LORA_BF16 && add_inputs && prefill) {
     // prefill-sized bf16 batches: the tensor-core expand (reduce-add tile kernel when the slices tile the
     // columns they cover in 64-column units, run-based kernel otherwise)
@@ -845,7 +852,7 @@ int lora_b200_add_prefill_noalloc(void* y, int64_t y_ld, const void* x, int64_t 
   sp.st = st; sp.scale_per_slot = scale_per_slot; sp.token_to_slot = token_to_slot; sp.scaling = scaling;
   void* scratch = nullptr;
   if (int rc = static_scratch_for_current_device(&scratch)) return rc;
-  return prefill_add_launch(sp, scratch, kStaticScratchBytes, static_cast<cudaStream_t>(stream));
+  return prefill_add(sp, scratch, kStaticScratchBytes, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -1,0 +1,607 @@
+// Prefill multi-LoRA in one launch (bf16, tcgen05): a cluster takes a block of rows, shrinks it with K split over its CTAs,
+// and takes the block's output tiles in turn.
+//
+//   ADD    : y[rows, :] += delta (reduce-add), or y = delta
+//   LINEAR : y[rows, :]  = x . W^T (+ bias) + delta
+//
+// What bounds the pair it replaces (sgmv_shrink_kernel, then tc_tile_kernel) is the way between its launches: both fill an SM's
+// shared memory, so the second one's set-up, its wait for the first and the trip of the intermediate through the L2 are all
+// serial with the K loop: 9 to 13 us a shrink of 1000 rows whose loads take 2. Here
+//   * one set-up (barriers, TMEM, run table) and one wait for the launch ahead;
+//   * the CTAs of the cluster add their partial sums in distributed shared memory, and each sends the 16-bit values of its share
+//     straight into the MMA operand tile of every CTA (st.async): no scratch, no barrier of the cluster between the halves;
+//   * the tiles' B operands are on their way before that exchange is over, and y's rows are on their way to the L2;
+//   * eight epilogue warps in two sets, each with two output buffers, and few TMA instructions: 1.35 us a tile of 128 x 256 (2.3).
+// us per projection (qkv, o, gate_up, down), the pair / this kernel: 8172 rows, 2048-wide, rank 64: 40 / 37, 32 / 24, 92 / 91,
+// 49 / 41; 1000 rows of them 18.7 / 15.6, 14.5 / 9.7, 22 / 19, 17 / 12. What is left of gate_up's 91 (HBM time 67): every GPC writes
+// y at 0.39 TB/s, and those with fewer SMs are done after half of the time.
+// Rows of a block may use different slots: the MMA of a run of equal slots updates the rows of that run only (its lane mask), so
+// the operand needs no masked copy per run. Rows without adapter: -0.0 in ADD launches (x + (-0.0) == x bit for bit), the base
+// result in LINEAR ones.
+#pragma once
+
+#include "gemm_tc.cuh"
+
+namespace b200lora {
+
+constexpr int kPcThreads = 320;   // warp 0 TMA, warp 1 MMA + TMEM owner, warps 2-9 epilogue
+constexpr int kPcEpi = 256;
+constexpr int kPcShrinkStages = 12;
+constexpr int kPcTileStages = 4;
+constexpr int kPcSmem = 224 * 1024;
+constexpr int kPcBox = 64;        // rows of a W or lora_B box
+constexpr int kPcLinearStage = kGemmStageBytes;  // x tile and W tile; LINEAR launches shrink in the same ring
+
+struct PcArgs {
+  __nv_bfloat16* y; int64_t y_ld;
+  const __nv_bfloat16* bias;                // LINEAR, may be null
+  int T, in_dim, n_total, S, r, n;
+  int out[B200_LORA_MAX_SLICES], col[B200_LORA_MAX_SLICES];
+  const int32_t* token_to_slot;
+  const float* scale_per_slot; float scaling;
+  int cta_cols, tile_cols;                  // columns of y per CTA and per tile (multiples of 64, a tile at most 256)
+  int overwrite;                            // ADD: store the delta (-0.0 in rows without adapter) instead of adding it
+  int bm, pad_shift, ck;                    // rows of a block (a multiple of 8, 64 to 128), log2 of the next power of two, CTAs of a cluster
+  int gmax;                                 // runs of a block whose K loops share one pass over x
+  int stages, stage_bytes;                  // ring of the tiles: lora_B tiles (LINEAR: or x and W tiles)
+  int out_bufs, off_out, off_tmp;           // output buffers of each epilogue set; byte offsets
+  int part_cols;                            // columns of partial sums exchanged at a time
+};
+struct PcMaps {
+  CUtensorMap x;                            // [T, in]           box bm x 64
+  CUtensorMap w;                            // [n_total, in]     box 64 x 64 (LINEAR)
+  CUtensorMap y;                            // [T, n_total]      box bm x 64
+  CUtensorMap a[B200_LORA_MAX_SLICES];      // [S*r, in]         box r x 64
+  CUtensorMap b[B200_LORA_MAX_SLICES];      // [S*out_s, r]      box 64 x r
+};
+
+// 16-byte piece c of row `row` inside an operand tile with rows of `row_bytes` (the TMA swizzle of that span)
+__device__ __forceinline__ uint32_t swizzled_piece(int row, int c, int row_bytes) {
+  const int x = row_bytes == 128 ? (row & 7) : (row_bytes == 64 ? (row >> 1) & 3 : (row >> 2) & 1);
+  return (uint32_t)(row * row_bytes + ((c ^ x) << 4));
+}
+__device__ __forceinline__ void st_async_b32x4(uint32_t cluster_addr, uint4 v, uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(cluster_addr),
+               "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(cluster_bar)
+               : "memory");
+}
+
+template <bool kLinear>
+__global__ void __launch_bounds__(kPcThreads, 1)
+prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constant__ PcArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ int16_t s_slot[kSgmvBM], run_slot[kSgmvBM];
+  __shared__ uint8_t run_lo[kSgmvBM], run_hi[kSgmvBM];
+  __shared__ int nruns_s;
+  __shared__ __align__(8) uint64_t bar_words[2 * kPcShrinkStages + 2 * kPcTileStages + 9];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ volatile int abort_flag;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int CK = a.ck, ck = CK > 1 ? (int)cluster_ctarank() : 0, blk = (int)blockIdx.x / CK;
+  const int r = a.r, n = a.n, width = n * r, row_bytes = r * 2, bm = a.bm, row0 = blk * bm;
+  const int pad = 1 << a.pad_shift;  // rows of the exchange's buffers
+  griddep_launch_dependents();
+  const uint32_t smem_base = smem_u32(smem);
+  if ((smem_base & 1023u) != 0) {  // (the swizzled tiles need it; the same in every CTA)
+    if (tid == 0) atomicOr(&g_b200_status, kStatusBadSmemBase);
+    return;
+  }
+  const uint32_t bar0 = smem_u32(bar_words);
+  // ring of the shrink (ADD launches), ring of the tiles
+  auto s_full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
+  auto s_empty = [&](int s) { return bar0 + 8u * (uint32_t)(kPcShrinkStages + s); };
+  auto t_full = [&](int s) { return bar0 + 8u * (uint32_t)(2 * kPcShrinkStages + s); };
+  auto t_empty = [&](int s) { return bar0 + 8u * (uint32_t)(2 * kPcShrinkStages + kPcTileStages + s); };
+  const uint32_t bar1 = bar0 + 8u * (2 * kPcShrinkStages + 2 * kPcTileStages);
+  auto acc_full = [&](int b) { return bar1 + 8u * (uint32_t)b; };
+  auto acc_empty = [&](int b) { return bar1 + 16u + 8u * (uint32_t)b; };
+  const uint32_t s_acc_full = bar1 + 32u, s_acc_empty = bar1 + 40u;
+  const uint32_t part_ready = bar1 + 48u, part_done = bar1 + 56u;  // every CTA of the cluster has written / read partial sums
+  const uint32_t tmp_full = bar1 + 64u;                            // every CTA's share of the intermediate has arrived
+
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&tmem_base_s), 512u);
+    tc_fence_before_sync();
+  }
+  if (warp == 0 && elect_one()) {
+    tma_prefetch_desc(&maps.x); tma_prefetch_desc(&maps.y);
+    if (kLinear) tma_prefetch_desc(&maps.w);
+    for (int s = 0; s < n; ++s) { tma_prefetch_desc(&maps.a[s]); tma_prefetch_desc(&maps.b[s]); }
+  }
+  // ---- runs of equal slot inside the block
+  {
+    __shared__ int warp_starts[4];
+    const int i = tid;
+    if (i < kSgmvBM) {
+      int sl = i < bm && row0 + i < a.T ? a.token_to_slot[row0 + i] : -1;
+      (void)B200_IN_BOUNDS(sl >= -1 && sl < a.S);  // ids outside [-1, S) are treated as "no adapter"; the checked build reports them
+      if (sl >= a.S || sl < -1) sl = -1;
+      s_slot[i] = (int16_t)sl;
+    }
+    __syncthreads();
+    bool starts = false, ends = false;
+    unsigned before = 0;
+    if (i < kSgmvBM) {
+      const int sl = s_slot[i];
+      starts = sl >= 0 && (i == 0 || s_slot[i - 1] != sl);
+      ends = sl >= 0 && (i == kSgmvBM - 1 || s_slot[i + 1] != sl);
+      const unsigned mask = __ballot_sync(0xffffffffu, starts);
+      before = __popc(mask & ((2u << (i & 31)) - 1u));  // runs of this warp that start at or before this row
+      if ((i & 31) == 0) warp_starts[i >> 5] = __popc(mask);
+    }
+    __syncthreads();
+    if (i < kSgmvBM) {
+      for (int w = 0; w < i >> 5; ++w) before += (unsigned)warp_starts[w];
+      if (starts) { run_slot[before - 1] = s_slot[i]; run_lo[before - 1] = (uint8_t)i; }
+      if (ends) run_hi[before - 1] = (uint8_t)(i + 1);
+    }
+    const int total = warp_starts[0] + warp_starts[1] + warp_starts[2] + warp_starts[3];
+    if (i == 0) {
+      nruns_s = total;
+      for (int s = 0; s < kPcShrinkStages; ++s) { mbar_init(s_full(s), 1); mbar_init(s_empty(s), 1); }
+      for (int s = 0; s < kPcTileStages; ++s) { mbar_init(t_full(s), 1); mbar_init(t_empty(s), 1); }
+      for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), kPcEpi / 32); }
+      mbar_init(s_acc_full, 1);
+      mbar_init(s_acc_empty, kPcEpi / 32);
+      mbar_init(part_ready, (uint32_t)CK);
+      mbar_init(part_done, (uint32_t)CK);
+      mbar_init(tmp_full, 1);
+      abort_flag = 0;
+      mbar_fence_init();
+      mbar_arrive_expect_tx(tmp_full, (uint32_t)(bm * width * 2));
+    }
+  }
+  __syncthreads();
+  tc_fence_after_sync();
+  if (CK > 1) { cluster_arrive(); cluster_wait(); }  // the barriers of every CTA of the cluster are initialised
+  // Everything above may overlap the previous launch of the stream; x and y are final from here on.
+  griddep_wait();
+
+  const uint32_t tmem_base = tmem_base_s;
+  const int nruns = nruns_s;
+  // This CTA's columns of y and its tiles of up to 256 of them. An ADD launch has nothing to add to a block without any adapter row.
+  const int c_begin = min(ck * a.cta_cols, a.n_total), c_end = min(c_begin + a.cta_cols, a.n_total);
+  const int my_tiles = kLinear || nruns > 0 || a.overwrite ? (c_end - c_begin + a.tile_cols - 1) / a.tile_cols : 0;
+  auto tile_lo = [&](int i) { return c_begin + i * a.tile_cols; };
+  auto tile_hi = [&](int i) { return min(c_begin + (i + 1) * a.tile_cols, c_end); };
+  const uint32_t tmp_base = smem_base + (uint32_t)a.off_tmp, tmp_tile = (uint32_t)(kSgmvBM * row_bytes);
+  // ---- the shrink's passes over x: up to G runs share one
+  const int nk_all = a.in_dim / kSgmvBK, nk_per = (nk_all + CK - 1) / CK;
+  const int kc0 = min(ck * nk_per, nk_all), nk = min(nk_per, nk_all - kc0);  // this CTA's K steps (at least one: see the launch)
+  const int G = min(a.gmax, max(nruns, 1)), npass = (nruns + G - 1) / G;
+  const uint32_t x_tile = (uint32_t)bm * kSgmvBK * 2, a_tile = (uint32_t)r * kSgmvBK * 2;
+  const uint32_t x_span = kSgmvBM * kSgmvBK * 2;  // (the MMA reads 128 rows; those beyond bm give rows that nobody reads)
+  const uint32_t s_stage = kLinear ? (uint32_t)kPcLinearStage : x_span + (uint32_t)(G * n) * a_tile;
+  const int s_stages = kLinear ? a.stages : min(kPcShrinkStages, (int)((uint32_t)a.off_tmp / s_stage));
+  const uint32_t s_tmem = tmem_base + (kLinear ? kSgmvBN : 0);  // (LINEAR: the first tile's sums lie in front)
+  const uint32_t part_base = kLinear ? smem_base + (uint32_t)a.off_out : smem_base + (uint32_t)((a.off_tmp - a.part_cols * pad * 4) & ~1023);
+  const int nk_base = kLinear ? nk_all : 0;
+
+  // slice s inside tile i: its columns [lo, hi) of y
+  auto part_of = [&](int s, int i, int& lo, int& hi) {
+    lo = max(a.col[s], tile_lo(i));
+    hi = min(a.col[s] + a.out[s], tile_hi(i));
+    return lo < hi;
+  };
+
+  if (warp == 0) {
+    // =========================== TMA
+    const uint32_t leader = elect_one();
+    int st = 0, round = 0;
+    for (int pi = 0; pi < npass; ++pi) {
+      // (ADD: the partial sums of a pass lie where the ring is)
+      if (!kLinear && pi > 0) mbar_wait_bounded(s_acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
+      const int u0 = pi * G, g = min(G, nruns - u0);
+      int row[4];  // first lora_A row of each run of the pass (G <= 4)
+#pragma unroll
+      for (int ui = 0; ui < 4; ++ui) row[ui] = uniform(ui < g ? run_slot[u0 + ui] * r : 0);
+      for (int kc = 0; kc < nk; ++kc) {
+        const uint32_t full = kLinear ? t_full(st) : s_full(st), empty = kLinear ? t_empty(st) : s_empty(st);
+        if (round > 0) mbar_wait_bounded(empty, (uint32_t)((round & 1) ^ 1), &abort_flag);
+        if (leader) {
+          const uint32_t base = smem_base + (uint32_t)st * s_stage;
+          mbar_arrive_expect_tx(full, x_tile + (uint32_t)(g * n) * a_tile);
+          tma_load_2d(base, &maps.x, (kc0 + kc) * kSgmvBK, row0, full);
+          uint32_t dst = base + x_span;
+#pragma unroll
+          for (int ui = 0; ui < 4; ++ui)
+            if (ui < g)
+              for (int s = 0; s < n; ++s, dst += a_tile) tma_load_2d(dst, &maps.a[s], (kc0 + kc) * kSgmvBK, row[ui], full);
+        }
+        __syncwarp();
+        if (++st == s_stages) { st = 0; ++round; }
+      }
+    }
+    if (!kLinear) {
+      st = round = 0;
+      if (npass > 0) mbar_wait_bounded(s_acc_full, (uint32_t)((npass - 1) & 1), &abort_flag);  // the ring changes its use
+    }
+    bool exchanged = kLinear;
+    const uint64_t w_policy = l2_policy_evict_last();
+    // The reduce-add reads y at the L2: the rows of a tile are asked for together with its lora_B tiles, as many tiles ahead as the
+    // ring has stages (one tile further ahead 2 to 8 % slower), the first ones while the sums of the shrink are exchanged. By box:
+    // 128 bulk prefetches of a row piece each kept the TMA unit busy for 2.3 us a tile.
+    auto ask_y = [&](int i) {
+      if (kLinear || a.overwrite || !leader || i >= my_tiles) return;
+      for (int c = tile_lo(i); c < tile_hi(i); c += kGemmOutChunk) tma_prefetch_2d(&maps.y, c, row0);
+    };
+    for (int i = 0; i < my_tiles; ++i) {
+      ask_y(i);
+      const int w_boxes = (tile_hi(i) - tile_lo(i) + kPcBox - 1) / kPcBox;
+      for (int kc = 0; kc < nk_base; ++kc) {
+        if (round > 0) mbar_wait_bounded(t_empty(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
+        if (leader) {
+          const uint32_t base = smem_base + (uint32_t)st * kPcLinearStage, full = t_full(st);
+          mbar_arrive_expect_tx(full, x_tile + (uint32_t)(w_boxes * kPcBox * kSgmvBK * 2));
+          tma_load_2d(base, &maps.x, kc * kSgmvBK, row0, full);
+          for (int q = 0; q < w_boxes; ++q)
+            tma_load_2d_hint(base + x_span + (uint32_t)(q * kPcBox * kSgmvBK * 2), &maps.w, kc * kSgmvBK, tile_lo(i) + q * kPcBox, full, w_policy);
+        }
+        __syncwarp();
+        if (++st == a.stages) { st = 0; ++round; }
+      }
+      for (int u = 0; u < nruns; ++u) {
+        const int slot = uniform(run_slot[u]);
+        for (int s = 0; s < n; ++s) {
+          int lo, hi;
+          if (!part_of(s, i, lo, hi)) continue;
+          if (round > 0) mbar_wait_bounded(t_empty(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
+          const uint32_t base = smem_base + (uint32_t)(st * a.stage_bytes), full = t_full(st);
+          // (ADD: a stage that lies where the partial sums are waits until every CTA has read them, that is, has sent its share)
+          if (!exchanged && base + (uint32_t)a.stage_bytes > part_base) {
+            mbar_wait_bounded_acquire_cluster(tmp_full, 0u, &abort_flag);
+            fence_proxy_async_smem();
+            exchanged = true;
+          }
+          if (leader) {
+            const int boxes = (hi - lo + kPcBox - 1) / kPcBox;
+            mbar_arrive_expect_tx(full, (uint32_t)(boxes * kPcBox * row_bytes));
+            for (int q = 0; q < boxes; ++q)
+              tma_load_2d(base + (uint32_t)(q * kPcBox * row_bytes), &maps.b[s], 0, slot * a.out[s] + (lo - a.col[s]) + q * kPcBox, full);
+          }
+          __syncwarp();
+          if (++st == a.stages) { st = 0; ++round; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // =========================== MMA
+    const uint32_t leader = elect_one();
+    const uint64_t desc_x = umma_smem_desc(smem_base, 128), desc_t = umma_smem_desc(smem_base, row_bytes);
+    const uint32_t hi_x = (uint32_t)(desc_x >> 32), hi_t = (uint32_t)(desc_t >> 32), lo0 = (uint32_t)desc_x;
+    const uint32_t idesc_s = umma_idesc_bf16(kSgmvBM, width);
+    int st = 0, round = 0;
+    for (int pi = 0; pi < npass; ++pi) {
+      const int jobs = uniform(min(G, nruns - pi * G));
+      if (pi > 0) mbar_wait_bounded(s_acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
+      tc_fence_after_sync();
+      for (int kc = 0; kc < nk; ++kc) {
+        mbar_wait_bounded(kLinear ? t_full(st) : s_full(st), (uint32_t)(round & 1), &abort_flag);
+        tc_fence_after_sync();
+        const uint32_t xl = lo0 + ((uint32_t)st * s_stage >> 4);
+        uint32_t al = xl + (x_span >> 4), d = s_tmem;
+        for (int q = 0; q < jobs; ++q, al += (uint32_t)n * a_tile >> 4, d += (uint32_t)width) {  // runs of the pass
+#pragma unroll
+          for (int k4 = 0; k4 < kSgmvBK / 16; ++k4) umma_elected(d, xl + 2u * k4, al + 2u * k4, hi_x, idesc_s, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
+        }
+        umma_commit_elected(kLinear ? t_empty(st) : s_empty(st), leader);  // stage reusable once these MMAs have read it
+        if (++st == s_stages) { st = 0; ++round; }
+      }
+      umma_commit_elected(s_acc_full, leader);
+    }
+    if (!kLinear) st = round = 0;
+    bool have_tmp = false;
+    for (int job = 0; job < my_tiles; ++job) {
+      const int buf = job & 1, c_lo = tile_lo(job);
+      const uint32_t idesc_w = umma_idesc_bf16(kSgmvBM, (tile_hi(job) - c_lo + 15) & ~15);
+      const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kSgmvBN);
+      // (the shrink's sums: in LINEAR launches where the second tile's will be, in ADD ones read before the intermediate was sent)
+      if (kLinear && job == 1 && npass > 0) mbar_wait_bounded(s_acc_empty, (uint32_t)((npass - 1) & 1), &abort_flag);
+      if (job >= 2) mbar_wait_bounded(acc_empty(buf), (uint32_t)(((job >> 1) - 1) & 1), &abort_flag);
+      tc_fence_after_sync();
+      for (int kc = 0; kc < nk_base; ++kc) {
+        mbar_wait_bounded(t_full(st), (uint32_t)(round & 1), &abort_flag);
+        tc_fence_after_sync();
+        const uint32_t xl = lo0 + ((uint32_t)st * kPcLinearStage >> 4), wl = xl + (x_span >> 4);
+#pragma unroll
+        for (int k4 = 0; k4 < kSgmvBK / 16; ++k4) umma_elected(d_tmem, xl + 2u * k4, wl + 2u * k4, hi_x, idesc_w, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
+        umma_commit_elected(t_empty(st), leader);
+        if (++st == a.stages) { st = 0; ++round; }
+      }
+      for (int u = 0; u < nruns; ++u) {
+        const int lo_row = uniform(run_lo[u]), hi_row = uniform(run_hi[u]);
+        const uint32_t off[4] = {rows_outside(lo_row, hi_row, 0), rows_outside(lo_row, hi_row, 1), rows_outside(lo_row, hi_row, 2), rows_outside(lo_row, hi_row, 3)};
+        for (int s = 0; s < n; ++s) {
+          int lo, hi;
+          if (!part_of(s, job, lo, hi)) continue;
+          if (!have_tmp) {
+            mbar_wait_bounded_acquire_cluster(tmp_full, 0u, &abort_flag);
+            fence_proxy_async_smem();  // (it came by plain stores)
+            if (!kLinear) mbar_wait_bounded(s_acc_empty, (uint32_t)((npass - 1) & 1), &abort_flag);  // this CTA's own sums have been read
+            have_tmp = true;
+            tc_fence_after_sync();
+          }
+          mbar_wait_bounded(t_full(st), (uint32_t)(round & 1), &abort_flag);
+          tc_fence_after_sync();
+          const uint32_t bl = lo0 + ((uint32_t)(st * a.stage_bytes) >> 4), tl = lo0 + (((uint32_t)a.off_tmp + (uint32_t)s * tmp_tile) >> 4);
+          const uint32_t idesc = umma_idesc_bf16(kSgmvBM, (hi - lo + 15) & ~15);
+#pragma unroll
+          for (int k4 = 0; k4 < 4; ++k4)
+            if (16 * k4 < r)
+              umma_rows_elected(d_tmem + (uint32_t)(lo - c_lo), tl + 2u * k4, bl + 2u * k4, hi_t, idesc, kLinear || k4 > 0 ? 1u : 0u, leader, off);
+          umma_commit_elected(t_empty(st), leader);
+          if (++st == a.stages) { st = 0; ++round; }
+        }
+      }
+      umma_commit_elected(acc_full(buf), leader);
+    }
+  } else {
+    // =========================== epilogue: eight warps; a warp may only touch its own quarter of the 128 TMEM lanes
+    const int quarter = warp & 3, set = (warp - 2) >> 2, etid = tid - 64, row_in_blk = quarter * 32 + lane;
+    // ---- the shrink's sums: added up over the cluster, rounded, sent to every CTA's operand tile
+    int exchange = 0;
+    for (int pi = 0; pi < npass; ++pi) {
+      const int u0 = pi * G, g = min(G, nruns - u0);
+      const int first_row = run_lo[u0], end_row = run_hi[u0 + g - 1];
+      mbar_wait_bounded(s_acc_full, (uint32_t)(pi & 1), &abort_flag);
+      tc_fence_after_sync();
+      for (int c0 = 0; c0 < width; c0 += a.part_cols, ++exchange) {
+        const int cols = min(a.part_cols, width - c0);
+        if (exchange > 0) mbar_wait_bounded_acquire_cluster(part_done, (uint32_t)((exchange - 1) & 1), &abort_flag);
+        // This CTA's partial sums into its own shared memory, as [4 columns][row] pieces of 16 bytes: the lanes of a remote read
+        // then cover consecutive bytes. A row has one run, so the runs of a pass share the buffer. (A TMEM load is a warp-wide
+        // operation on one column range: a warp whose rows straddle two runs reads both runs' columns.)
+        for (int ui = 0; ui < g; ++ui) {
+          const int lo_row = run_lo[u0 + ui], hi_row = run_hi[u0 + ui];
+          if (hi_row <= quarter * 32 || lo_row >= quarter * 32 + 32) continue;  // warp-uniform
+          const bool mine = row_in_blk >= lo_row && row_in_blk < hi_row;
+          for (int c = 16 * set; c < cols; c += 32) {
+            uint32_t v[16];
+            tmem_ld_32x16(s_tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ui * width + c0 + c), v);
+            tmem_ld_wait();
+            if (mine) {
+              const uint32_t dst = part_base + (uint32_t)((c >> 2) * pad + row_in_blk) * 16u;
+#pragma unroll
+              for (int q = 0; q < 4; ++q) sts128(dst + 16u * (uint32_t)(pad * q), make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+            }
+          }
+        }
+        tc_fence_before_sync();
+        named_bar_sync(2, kPcEpi);
+        if (etid < CK) mbar_arrive_remote_release(mapa_shared(part_ready, (uint32_t)etid));
+        mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)(exchange & 1), &abort_flag);
+        // This CTA's share of the (8 columns x row) pieces; those of a thread are all of one row.
+        const int pieces = (cols >> 3) << a.pad_shift, per = (pieces + CK - 1) / CK;
+        const int first = ck * per + etid, last = min((ck + 1) * per, pieces);
+        const int er = first & (pad - 1), slot = s_slot[er];
+        const bool live = slot >= 0 && er >= first_row && er < end_row;
+        const bool zero = slot < 0 && pi == 0 && er < bm;  // rows without adapter
+        const float sc = live ? a.scaling * (a.scale_per_slot != nullptr ? a.scale_per_slot[slot] : 1.0f) : 0.f;
+        auto send = [&](auto parts) {
+          // eight remote reads of 32 bytes in flight per thread: one at a time each costs a round trip of 500 cycles
+          constexpr int kParts = decltype(parts)::value, kBatch = kParts >= 4 ? 8 / kParts : 2;
+          if (!live && !zero) return;
+          for (int e0 = first; e0 < last; e0 += kBatch * kPcEpi) {
+            float4 v[kBatch * kParts][2];
+#pragma unroll
+            for (int q = 0; q < kBatch * kParts; ++q) {
+              const int e = e0 + (q / kParts) * kPcEpi;
+              v[q][0] = v[q][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (live && e < last) {
+                const uint32_t src = mapa_shared(part_base + (uint32_t)(((e >> a.pad_shift) * 2 << a.pad_shift) + er) * 16u, (uint32_t)(q % kParts));
+                v[q][0] = ld_cluster_f32x4(src);
+                v[q][1] = ld_cluster_f32x4(src + 16u * (uint32_t)pad);
+              }
+            }
+#pragma unroll
+            for (int h = 0; h < kBatch; ++h) {
+              const int e = e0 + h * kPcEpi;
+              if (e >= last) continue;
+              float4 s0 = v[h * kParts][0], s1 = v[h * kParts][1];
+#pragma unroll
+              for (int q = 1; q < kParts; ++q) {
+                const float4 w0 = v[h * kParts + q][0], w1 = v[h * kParts + q][1];
+                s0.x += w0.x; s0.y += w0.y; s0.z += w0.z; s0.w += w0.w;
+                s1.x += w1.x; s1.y += w1.y; s1.z += w1.z; s1.w += w1.w;
+              }
+              uint4 packed = make_uint4(0, 0, 0, 0);
+              if (live)
+                packed = make_uint4(pack_bf16x2(s0.x * sc, s0.y * sc), pack_bf16x2(s0.z * sc, s0.w * sc), pack_bf16x2(s1.x * sc, s1.y * sc),
+                                    pack_bf16x2(s1.z * sc, s1.w * sc));
+              const int col = c0 + 8 * (e >> a.pad_shift), s = col / r, c = col - s * r;
+              const uint32_t dst = tmp_base + (uint32_t)s * tmp_tile + swizzled_piece(er, c >> 3, row_bytes);
+              for (int q = 0; q < CK; ++q) st_async_b32x4(mapa_shared(dst, (uint32_t)q), packed, mapa_shared(tmp_full, (uint32_t)q));
+            }
+          }
+        };
+        if (CK == 8) send(std::integral_constant<int, 8>{});
+        else if (CK == 4) send(std::integral_constant<int, 4>{});
+        else if (CK == 2) send(std::integral_constant<int, 2>{});
+        else send(std::integral_constant<int, 1>{});
+        if (pi + 1 < npass || c0 + cols < width) {
+          named_bar_sync(2, kPcEpi);
+          if (etid < CK) mbar_arrive_remote_release(mapa_shared(part_done, (uint32_t)etid));
+        }
+      }
+      // (ADD: the partial sums lie where the ring is: no refill before every CTA has read them)
+      if (!kLinear && pi + 1 < npass) mbar_wait_bounded_acquire_cluster(part_done, (uint32_t)((exchange - 1) & 1), &abort_flag);
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(s_acc_empty);
+    }
+    // ---- the tiles: set 0 takes the first and third 64-column chunk of a tile, set 1 the others
+    const uint32_t out_bytes = (uint32_t)bm * kGemmOutChunk * 2;
+    const uint32_t out_set = smem_base + (uint32_t)a.off_out + (uint32_t)(set * a.out_bufs) * out_bytes;
+    const bool issuer = tid == 64 + 128 * set, in_block = quarter * 32 < bm;
+    const bool neg_zero_row = !kLinear && s_slot[row_in_blk] < 0;
+    int chunk_no = 0;
+    // Every CTA has read the partial sums that lie where the output buffers are. (A CTA without tiles waits too: it may not leave
+    // while a peer still reads from it or sends to it.)
+    if (npass > 0) mbar_wait_bounded_acquire_cluster(tmp_full, 0u, &abort_flag);
+    for (int job = 0; job < my_tiles; ++job) {
+      const int buf = job & 1, c_lo = tile_lo(job), cols = tile_hi(job) - c_lo;
+      mbar_wait_bounded(acc_full(buf), (uint32_t)((job >> 1) & 1), &abort_flag);
+      tc_fence_after_sync();
+      for (int c = kGemmOutChunk * set; c < cols; c += 2 * kGemmOutChunk, ++chunk_no) {
+        const int col0 = c_lo + c;
+        const uint32_t obuf = out_set + (uint32_t)(chunk_no % a.out_bufs) * out_bytes;
+        if (issuer) {  // the store that last used this buffer must have finished reading it
+          if (a.out_bufs == 2) bulk_wait_group_read<1>();
+          else bulk_wait_group_read<0>();
+        }
+        named_bar_sync(3 + (uint32_t)set, 128);
+        if (in_block) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t v[32];
+            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * kSgmvBN + c + 32 * h), v);
+            tmem_ld_wait();
+            if (kLinear && a.bias != nullptr) {
+#pragma unroll
+              for (int q = 0; q < 32; ++q) {
+                const int cc = col0 + 32 * h + q;
+                v[q] = __float_as_uint(__uint_as_float(v[q]) + (cc < a.n_total ? __bfloat162float(a.bias[cc]) : 0.f));
+              }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              uint4 o;
+              o.x = pack_bf16x2(__uint_as_float(v[8 * q + 0]), __uint_as_float(v[8 * q + 1]));
+              o.y = pack_bf16x2(__uint_as_float(v[8 * q + 2]), __uint_as_float(v[8 * q + 3]));
+              o.z = pack_bf16x2(__uint_as_float(v[8 * q + 4]), __uint_as_float(v[8 * q + 5]));
+              o.w = pack_bf16x2(__uint_as_float(v[8 * q + 6]), __uint_as_float(v[8 * q + 7]));
+              if (neg_zero_row) o = make_uint4(0x80008000u, 0x80008000u, 0x80008000u, 0x80008000u);
+              if (row_in_blk < bm) sts128(obuf + swizzled_piece(row_in_blk, 4 * h + q, 128), o);
+            }
+          }
+        }
+        fence_proxy_async_smem();
+        named_bar_sync(3 + (uint32_t)set, 128);
+        if (issuer) {
+          if (!kLinear && !a.overwrite) tma_reduce_add_2d(&maps.y, obuf, col0, row0);
+          else tma_store_2d_hint(&maps.y, obuf, col0, row0, l2_policy_evict_first());
+          bulk_commit_group();
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty(buf));
+    }
+    if (issuer) bulk_wait_group_read<0>();
+  }
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, 512u);
+  if (tid == 0 && abort_flag != 0) atomicOr(&g_b200_status, kStatusWaitGaveUp);
+}
+
+// ------------------------------------------------------------------ host side
+// Clusters of 1, 2, 4 and 8 CTAs with an SM each that are resident at a time (what cudaOccupancyMaxActiveClusters says: the SMs
+// of a cluster lie in one GPC). One cluster more is a second wave.
+inline int clusters_resident(int ck) { return ck == 1 ? 148 : (ck == 2 ? 74 : (ck == 4 ? 33 : 15)); }
+// CTAs of a cluster (as many as are resident at once, every K part at least one K step), then the rows of a block that make as
+// many clusters as are resident (at least 64: every block reads its adapters again).
+inline void prefill_cluster_split(int T, int in_dim, PcArgs* a) {
+  const int nk = in_dim / kSgmvBK;
+  a->ck = 1;
+  while (a->ck < 8 && ceil_div_i(T, kSgmvBM) <= clusters_resident(2 * a->ck) && ceil_div_i(nk, 2 * a->ck) * (2 * a->ck - 1) < nk) a->ck *= 2;
+  a->bm = std::min(kSgmvBM, std::max(64, round_up_i(ceil_div_i(T, clusters_resident(a->ck)), 8)));
+  a->pad_shift = a->bm == 64 ? 6 : 7;
+}
+
+// y += delta or y = delta (weight == nullptr), or y = x . W^T (+ bias) + delta, of a problem that sgmv_supported takes.
+inline int prefill_cluster_launch(const SgmvProblem& b, const void* weight, int64_t w_ld, int n_total, const void* bias, bool overwrite, cudaStream_t stream) {
+  const bool linear = weight != nullptr;
+  PcArgs a = {};
+  PcMaps maps;
+  if (b.S > 32767) return fail(B200_LORA_EUNSUPPORTED, "prefill kernel: more than 32767 adapter slots");
+  prefill_cluster_split(b.T, b.in_dim, &a);
+  a.y = static_cast<__nv_bfloat16*>(b.y); a.y_ld = b.y_ld; a.bias = static_cast<const __nv_bfloat16*>(bias);
+  a.T = b.T; a.in_dim = b.in_dim; a.n_total = n_total; a.S = b.S; a.r = b.r_max;
+  a.token_to_slot = b.token_to_slot; a.scale_per_slot = b.scale_per_slot; a.scaling = b.scaling; a.overwrite = overwrite ? 1 : 0;
+  for (int s = 0; s < b.st.n; ++s) {
+    if (b.st.out[s] == 0) continue;
+    a.out[a.n] = b.st.out[s]; a.col[a.n] = b.st.col[s];
+    if (int rc = make_tmap_2d(&maps.a[a.n], b.st.a[s], (uint64_t)b.S * b.r_max, (uint64_t)b.in_dim, (uint64_t)b.in_dim, (uint32_t)b.r_max, kSgmvBK)) return rc;
+    if (int rc = make_tmap_2d(&maps.b[a.n], b.st.b[s], (uint64_t)b.S * b.st.out[s], (uint64_t)b.r_max, (uint64_t)b.r_max, kPcBox, (uint32_t)b.r_max)) return rc;
+    ++a.n;
+  }
+  for (int s = a.n; s < B200_LORA_MAX_SLICES; ++s) { maps.a[s] = maps.a[0]; maps.b[s] = maps.b[0]; }
+  if (int rc = make_tmap_2d(&maps.x, b.x, (uint64_t)b.T, (uint64_t)b.in_dim, (uint64_t)b.x_ld, (uint32_t)a.bm, kSgmvBK)) return rc;
+  if (int rc = make_tmap_2d(&maps.y, b.y, (uint64_t)b.T, (uint64_t)n_total, (uint64_t)b.y_ld, (uint32_t)a.bm, kGemmOutChunk)) return rc;
+  maps.w = maps.x;
+  if (linear)
+    if (int rc = make_tmap_2d(&maps.w, weight, (uint64_t)n_total, (uint64_t)b.in_dim, (uint64_t)w_ld, kPcBox, kSgmvBK)) return rc;
+  a.cta_cols = round_up_i(ceil_div_i(n_total, a.ck), 64);
+  a.tile_cols = round_up_i(ceil_div_i(a.cta_cols, ceil_div_i(a.cta_cols, kSgmvBN)), 64);
+  // shared memory: ring of the tiles, output buffers, the intermediate as MMA operand; ADD launches shrink through a ring over the
+  // first two
+  const int width = a.n * a.r, tmp_bytes = a.n * kSgmvBM * a.r * 2, out_buf = a.bm * kGemmOutChunk * 2;
+  a.off_tmp = kPcSmem - tmp_bytes;
+  a.stage_bytes = linear ? kPcLinearStage : kSgmvBN * a.r * 2;
+  a.stages = linear ? 3 : kPcTileStages;
+  a.out_bufs = 2;
+  while (a.out_bufs > 0 && a.off_tmp - a.stages * a.stage_bytes < 2 * a.out_bufs * out_buf) {
+    if (!linear && a.stages > 2) --a.stages;
+    else --a.out_bufs;
+  }
+  if (a.out_bufs == 0) return fail(B200_LORA_EUNSUPPORTED, "prefill kernel: too many rank rows");
+  a.off_out = a.stages * a.stage_bytes;
+  a.part_cols = linear ? std::min(width, 2 * a.out_bufs * out_buf / (4 << a.pad_shift) & ~15) : width;
+  a.gmax = 1;
+  for (int g = 2; g <= 4; ++g) {
+    const int stage = kSgmvBM * kSgmvBK * 2 + g * width * kSgmvBK * 2;
+    if (linear ? g * width <= kSgmvBN && stage <= kPcLinearStage : g * width <= 512 && a.off_tmp / stage >= 2) a.gmax = g;
+  }
+  const auto kernel = linear ? prefill_cluster_kernel<true> : prefill_cluster_kernel<false>;
+  if (int rc = sgmv_set_smem(reinterpret_cast<const void*>(kernel), kPcSmem)) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(ceil_div_i(b.T, a.bm) * a.ck), 1, 1);
+  cfg.blockDim = dim3(kPcThreads, 1, 1);
+  cfg.dynamicSmemBytes = kPcSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)a.ck;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = bgmv_options().pdl ? 2 : 1;  // B200_LORA_OPT_PDL = 0: strict stream order
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, a);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(B200_LORA_ECUDA, "prefill_cluster_kernel launch: %s", cudaGetErrorString(e));
+  }
+  return B200_LORA_OK;
+}
+
+// Whether the kernel takes an ADD launch: slices that tile the output in 64-column units, a block of rows per SM at most.
+inline bool prefill_cluster_add_ok(const SgmvProblem& b) {
+  int n = 0, pos = 0;
+  for (int s = 0; s < b.st.n; ++s) {
+    if (b.st.out[s] == 0) continue;
+    if (b.st.col[s] != pos || b.st.out[s] % kGemmOutChunk != 0) return false;
+    pos += b.st.out[s];
+    ++n;
+  }
+  return n * b.r_max <= 256 && ceil_div_i(b.T, kSgmvBM) <= kTileSMs;
+}
+
+// y += LoRA delta for a prefill batch. Callers pass scratch for the launches that the kernel does not take (what needs it is
+// not theirs to know), so it is asked for in any case.
+inline int prefill_add(const SgmvProblem& b, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool overwrite = false) {
+  const char* why = nullptr;
+  if (!prefill_cluster_add_ok(b)) return prefill_add_launch(b, workspace, workspace_bytes, stream, overwrite);
+  if (!sgmv_supported(b, &why)) return fail(B200_LORA_EUNSUPPORTED, "prefill kernels: %s", why);
+  int n = 0, n_total = 0;
+  for (int s = 0; s < b.st.n; ++s) {
+    n += b.st.out[s] > 0;
+    if (b.st.out[s] > 0) n_total = std::max(n_total, b.st.col[s] + b.st.out[s]);
+  }
+  if (int rc = sgmv_workspace_check(b, n, workspace, workspace_bytes)) return rc;
+  return prefill_cluster_launch(b, nullptr, 0, n_total, nullptr, overwrite, stream);
+}
+
+}  // namespace b200lora

@@ -567,13 +567,18 @@ inline int sgmv_prepare_tmp(const SgmvProblem& b, void* tmp, uint64_t tmp_rows, 
   return B200_LORA_OK;
 }
 
+inline int sgmv_workspace_check(const SgmvProblem& b, int n, const void* workspace, size_t workspace_bytes) {
+  const size_t need = sgmv_workspace_bytes(b.T, std::max(n, 1), b.r_max);
+  if (workspace == nullptr || workspace_bytes < need)
+    return fail(B200_LORA_EWORKSPACE, "prefill kernels need %zu bytes of scratch, got %zu", need, workspace_bytes);
+  return B200_LORA_OK;
+}
+
 // Builds the launch arguments and tensor maps shared by the two kernels, the intermediate in caller-provided scratch.
 inline int sgmv_prepare(const SgmvProblem& b, void* workspace, size_t workspace_bytes, SgmvMaps* maps, SgmvArgs* args) {
   int n = 0;
   for (int s = 0; s < b.st.n; ++s) n += b.st.out[s] > 0;
-  const size_t need = sgmv_workspace_bytes(b.T, std::max(n, 1), b.r_max);
-  if (workspace == nullptr || workspace_bytes < need)
-    return fail(B200_LORA_EWORKSPACE, "prefill kernels need %zu bytes of scratch, got %zu", need, workspace_bytes);
+  if (int rc = sgmv_workspace_check(b, n, workspace, workspace_bytes)) return rc;
   uintptr_t ws = (reinterpret_cast<uintptr_t>(workspace) + 1023) & ~(uintptr_t)1023;
   return sgmv_prepare_tmp(b, reinterpret_cast<void*>(ws), (uint64_t)n * b.T + kSgmvBM, true, true, maps, args);
 }

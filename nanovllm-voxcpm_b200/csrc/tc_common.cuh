@@ -91,6 +91,23 @@ __device__ __forceinline__ void umma_elected(uint32_t d_tmem, uint32_t a_lo, uin
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
+// the same, updating only the TMEM lanes (rows of D) whose bit in `off` is clear
+__device__ __forceinline__ void umma_rows_elected(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate,
+                                                  uint32_t leader, const uint32_t (&off)[4]) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, {%7, %8, %9, %10}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(leader), "r"(off[0]), "r"(off[1]), "r"(off[2]), "r"(off[3])
+      : "memory");
+}
+// lanes 32 w .. 32 w + 31 outside rows [lo, hi)
+__device__ __forceinline__ uint32_t rows_outside(int lo, int hi, int w) {
+  const int a = min(max(lo - 32 * w, 0), 32), b = min(max(hi - 32 * w, 0), 32);
+  const uint32_t below_b = b == 32 ? 0xffffffffu : (1u << b) - 1u, below_a = a == 32 ? 0xffffffffu : (1u << a) - 1u;
+  return ~(below_b & ~below_a);
+}
 __device__ __forceinline__ void umma_commit_elected(uint32_t bar, uint32_t leader) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
@@ -125,6 +142,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const CUtensorMap
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(dst_smem), "l"(tmap), "r"(c0), "r"(c1), "r"(bar)
       : "memory");
+}
+// a box of the map to the L2
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* tmap, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(c0), "r"(c1) : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");

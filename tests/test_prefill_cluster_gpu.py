@@ -1,0 +1,68 @@
+"""The one-launch prefill kernel (``csrc/prefill_cluster.cuh``) at the edges of its blocks and clusters: row counts around the
+lines where the cluster size and the rows of a block change, ragged last blocks, K splits with a short last part, many runs in
+a block (several passes), runs that end at block lines, blocks without any adapter, one to four slices, every rank."""
+
+import pytest
+import torch
+
+from helpers import assert_lora_close
+from nanovllm_voxcpm_b200 import _native as N
+from nanovllm_voxcpm_b200 import lora as LORA
+from nanovllm_voxcpm_b200 import workloads as W
+from oracle import lora_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def by_runs(T, S, longest, seed):
+    """Slots of rows in runs of 1 .. longest rows, every fifth run or so without adapter."""
+    gen = torch.Generator().manual_seed(seed)
+    out = []
+    while len(out) < T:
+        slot = int(torch.randint(-S // 4 - 1, S, (1,), generator=gen).clamp(min=-1))
+        out += [slot] * int(torch.randint(1, longest + 1, (1,), generator=gen))
+    return torch.tensor(out[:T], dtype=torch.int32)
+
+
+def metadata(slots):
+    from nanovllm_voxcpm_b200 import batch_plan as BP
+
+    ctx = BP.build_lora_context_from_slot_list(slots.tolist(), device=DEV)
+    return LORA.LoRAMetadata(ctx.token_to_slot, ctx.token_indices_sorted_by_slot, ctx.active_slot_ids, ctx.num_tokens_per_slot,
+                             ctx.slot_start_offsets, ctx.no_lora_flag, ctx.num_active_loras)
+
+
+# T, in, outs, S, r, longest run (0: one run of all rows but a head without adapter)
+CASES = [
+    (1, 64, [64], 1, 16, 1),                     # one row, one K step
+    (64, 1024, [128, 64], 3, 32, 9),             # one block of 64 rows, eight K parts
+    (65, 192, [320], 3, 64, 70),                 # two blocks, K parts of one step
+    (960, 2048, [256, 64, 64], 5, 64, 200),      # 15 clusters of 8: blocks of 64 rows
+    (961, 2048, [256, 64, 64], 5, 64, 30),       # ... of 72, several passes a block
+    (1920, 576, [640], 4, 32, 400),              # 15 of 128; K parts of two steps, the last of one
+    (1921, 1024, [192, 192], 4, 32, 5),          # clusters of 4, blocks of 64, 40 runs a block
+    (4225, 320, [512], 6, 16, 300),              # clusters of 2, ragged
+    (9472, 128, [64, 64, 64, 64], 2, 64, 900),   # 74 clusters of 2, four slices of rank 64
+    (9473, 128, [256], 2, 32, 0),                # one CTA a block
+]
+
+
+@pytest.mark.parametrize("overwrite", [False, True])
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_prefill_add_matches_oracle(case, overwrite):
+    T, in_dim, outs, S, r, longest = CASES[case]
+    slots = by_runs(T, S, longest, case) if longest else torch.cat([torch.full((300,), -1), torch.zeros(T - 300)]).to(torch.int32)
+    slots[0] = 0
+    if T > 1000:
+        slots[200:460] = -1  # at least one block without any adapter
+    p = W.make_projection(700 + case, T, in_dim, outs, S, r, token_to_slot=slots)
+    d = p.to_device(DEV)
+    LORA.launch_add(d.y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata(slots), 0.5, impl=N.IMPL_SGMV, overwrite=overwrite)
+    torch.cuda.synchronize()
+    assert N.device_status(reset=True) == 0
+    base = torch.full_like(p.y, -0.0) if overwrite else p.y
+    # one 16-bit rounding of the intermediate, one of the delta, one of the sum: the tolerance stated for the path
+    assert_lora_close(d.y, O.add_lora(base, p.x, p.a_slabs, p.b_slabs, slots, 0.5, p.col_offsets), what="prefill add")
+    none = slots < 0
+    assert torch.equal(d.y.cpu()[none].view(torch.int16), base[none].view(torch.int16)), "rows without adapter keep their bits"
