@@ -17,7 +17,7 @@
 // barrier; commits arrive at the empty, lora_empty and acc_full barriers of both CTAs.
 #pragma once
 
-#include "gemm_tc.cuh"
+#include "prefill_cluster.cuh"
 
 namespace b200lora {
 
@@ -510,6 +510,29 @@ struct LinearProblem {
   bool silu = false;         // y = silu(gate) * up of the projection's halves, [T, n_total / 2]
 };
 
+// Whether prefill_cluster_kernel takes a fused linear: its CTAs have a contiguous share of a block's columns each, so it is chosen
+// where that share is no more tiles than the CTAs of the other two have (or one more, over at most 1024 columns of x), which then
+// cost a shrink launch more. us, the others / this, rank 32: 1024 -> 1280, 300, 1700, 4001 rows 17.1 / 10.7, 19.0 / 13.3, 26.5 / 19.6;
+// 1024 -> 1024 13.4 / 9.3, 16.3 / 10.8, 18.2 / 13.3; 4096 -> 1024 26.6 / 23.6, 32.2 / 25.0, 38.6 / 35.3; 2048 -> 2048, 1000 and 3000
+// rows 17.5 / 17.2, 36.4 / 33.4. Outside the line: 1024 -> 8192, 1000 rows (4 tiles, 2) 25.6 / 30.8; 2048 -> 2560, 1000 rows (2, 1)
+// 18.9 / 25.7; 6144 -> 2048, 1000 rows (K steps of the shrink ahead of 96 others) 36.2 / 38.4; three slices of rank 64 (a pass over x
+// for every run) 1024 -> 1280, 1300 rows 17.9 / 23.0.
+inline bool prefill_cluster_linear_ok(const LinearProblem& p) {
+  const SgmvProblem& b = p.lora;
+  int n = 0;
+  for (int s = 0; s < b.st.n; ++s) {
+    if (b.st.out[s] == 0) continue;
+    if (b.st.col[s] % 16 != 0 || b.st.out[s] % 16 != 0) return false;  // (the MMAs of a slice would reach into the next one)
+    ++n;
+  }
+  PcArgs a = {};
+  if (ceil_div_i(b.T, kSgmvBM) > kTileSMs || !sgmv_supported(b, nullptr) || !prefill_cluster_plan(b, n, p.n_total, true, &a)) return false;
+  const int nk = b.in_dim / kSgmvBK, tiles = ceil_div_i(a.cta_cols, a.tile_cols), total = ceil_div_i(b.T, kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
+  const int64_t pair_tiles = (int64_t)ceil_div_i(b.T, 2 * kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
+  const int rounds = pair_tiles >= kPairMinTiles ? ceil_div_i((int)pair_tiles, kTileSMs / 2) : ceil_div_i(total, kTileSMs);
+  return n * b.r_max <= 128 && b.in_dim <= 4096 && (tiles <= rounds || (tiles <= 2 && (tiles - rounds) * nk <= 16));
+}
+
 // y = x . W^T (+ bias) + LoRA delta, the delta accumulated into the GEMM's TMEM accumulator.
 inline int linear_lora_launch(const LinearProblem& p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   const SgmvProblem& b = p.lora;
@@ -520,11 +543,15 @@ inline int linear_lora_launch(const LinearProblem& p, void* workspace, size_t wo
   if ((reinterpret_cast<uintptr_t>(p.weight) & 15u) || (reinterpret_cast<uintptr_t>(b.x) & 15u) ||
       (reinterpret_cast<uintptr_t>(b.y) & 15u) || (reinterpret_cast<uintptr_t>(p.bias) & 1u))
     return fail(B200_LORA_EUNSUPPORTED, "fused linear: pointers must be 16-byte aligned");
-  bool any = false;
-  for (int s = 0; s < b.st.n; ++s) any = any || b.st.out[s] > 0;
-  const bool with_lora = any && b.token_to_slot != nullptr;
+  int slices = 0;
+  for (int s = 0; s < b.st.n; ++s) slices += b.st.out[s] > 0;
+  const bool with_lora = slices > 0 && b.token_to_slot != nullptr;
   SgmvMaps sm;
   SgmvArgs sa = {};
+  if (with_lora && !p.silu && prefill_cluster_linear_ok(p)) {
+    if (int rc = sgmv_workspace_check(b, slices, workspace, workspace_bytes)) return rc;
+    return prefill_cluster_launch(b, p.weight, p.w_ld, p.n_total, p.bias, false, stream);
+  }
   if (with_lora) {
     if (int rc = sgmv_prepare(b, workspace, workspace_bytes, &sm, &sa)) return rc;
     if (int rc = sgmv_launch_shrink(sm, sa, stream)) return rc;

@@ -30,7 +30,6 @@ constexpr int kPcShrinkStages = 12;
 constexpr int kPcTileStages = 4;
 constexpr int kPcSmem = 224 * 1024;
 constexpr int kPcBox = 64;        // rows of a W or lora_B box
-constexpr int kPcLinearStage = kGemmStageBytes;  // x tile and W tile; LINEAR launches shrink in the same ring
 
 struct PcArgs {
   __nv_bfloat16* y; int64_t y_ld;
@@ -172,7 +171,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   const int G = min(a.gmax, max(nruns, 1)), npass = (nruns + G - 1) / G;
   const uint32_t x_tile = (uint32_t)bm * kSgmvBK * 2, a_tile = (uint32_t)r * kSgmvBK * 2;
   const uint32_t x_span = kSgmvBM * kSgmvBK * 2;  // (the MMA reads 128 rows; those beyond bm give rows that nobody reads)
-  const uint32_t s_stage = kLinear ? (uint32_t)kPcLinearStage : x_span + (uint32_t)(G * n) * a_tile;
+  const uint32_t s_stage = kLinear ? (uint32_t)a.stage_bytes : x_span + (uint32_t)(G * n) * a_tile;
   const int s_stages = kLinear ? a.stages : min(kPcShrinkStages, (int)((uint32_t)a.off_tmp / s_stage));
   const uint32_t s_tmem = tmem_base + (kLinear ? kSgmvBN : 0);  // (LINEAR: the first tile's sums lie in front)
   const uint32_t part_base = kLinear ? smem_base + (uint32_t)a.off_out : smem_base + (uint32_t)((a.off_tmp - a.part_cols * pad * 4) & ~1023);
@@ -232,7 +231,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
       for (int kc = 0; kc < nk_base; ++kc) {
         if (round > 0) mbar_wait_bounded(t_empty(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
         if (leader) {
-          const uint32_t base = smem_base + (uint32_t)st * kPcLinearStage, full = t_full(st);
+          const uint32_t base = smem_base + (uint32_t)(st * a.stage_bytes), full = t_full(st);
           mbar_arrive_expect_tx(full, x_tile + (uint32_t)(w_boxes * kPcBox * kSgmvBK * 2));
           tma_load_2d(base, &maps.x, kc * kSgmvBK, row0, full);
           for (int q = 0; q < w_boxes; ++q)
@@ -303,7 +302,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
       for (int kc = 0; kc < nk_base; ++kc) {
         mbar_wait_bounded(t_full(st), (uint32_t)(round & 1), &abort_flag);
         tc_fence_after_sync();
-        const uint32_t xl = lo0 + ((uint32_t)st * kPcLinearStage >> 4), wl = xl + (x_span >> 4);
+        const uint32_t xl = lo0 + ((uint32_t)(st * a.stage_bytes) >> 4), wl = xl + (x_span >> 4);
 #pragma unroll
         for (int k4 = 0; k4 < kSgmvBK / 16; ++k4) umma_elected(d_tmem, xl + 2u * k4, wl + 2u * k4, hi_x, idesc_w, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
         umma_commit_elected(t_empty(st), leader);
@@ -510,13 +509,48 @@ inline void prefill_cluster_split(int T, int in_dim, PcArgs* a) {
   a->pad_shift = a->bm == 64 ? 6 : 7;
 }
 
+// Split, tiles and shared memory (ring of the tiles, output buffers, the intermediate as MMA operand; ADD launches shrink through a
+// ring over the first two) of a problem with `n` slices; false: too many rank rows for them.
+inline bool prefill_cluster_plan(const SgmvProblem& b, int n, int n_total, bool linear, PcArgs* a) {
+  prefill_cluster_split(b.T, b.in_dim, a);
+  a->cta_cols = round_up_i(ceil_div_i(n_total, a->ck), 64);
+  a->tile_cols = round_up_i(ceil_div_i(a->cta_cols, ceil_div_i(a->cta_cols, kSgmvBN)), 64);
+  const int width = n * b.r_max, tmp_bytes = n * kSgmvBM * b.r_max * 2, out_buf = a->bm * kGemmOutChunk * 2;
+  a->off_tmp = kPcSmem - tmp_bytes;
+  a->gmax = 1;
+  if (linear) {
+    // stages of an x and a W tile (or, ahead of the tiles, of the lora_A tiles of up to gmax runs), then output buffers
+    a->stages = 3;
+    const int b_tiles = std::max(a->tile_cols, width) * kSgmvBK * 2;
+    while (a->gmax < 4 && (a->gmax + 1) * width <= kSgmvBN && (a->gmax + 1) * width * kSgmvBK * 2 <= b_tiles) ++a->gmax;
+    a->stage_bytes = kSgmvBM * kSgmvBK * 2 + b_tiles;
+    if (a->off_tmp - 4 * a->stage_bytes >= 4 * out_buf) a->stages = 4;
+    const int room = a->off_tmp - a->stages * a->stage_bytes;
+    if (width > kSgmvBN || room < 2 * out_buf) return false;
+    a->out_bufs = std::min(2, room / (2 * out_buf));
+    a->part_cols = std::min(width, 2 * a->out_bufs * out_buf / (4 << a->pad_shift) & ~15);
+  } else {
+    a->stages = kPcTileStages;
+    a->stage_bytes = a->tile_cols * b.r_max * 2;
+    a->out_bufs = 2;
+    while (a->stages > 2 && a->off_tmp - a->stages * a->stage_bytes < 2 * a->out_bufs * out_buf) --a->stages;
+    for (int g = 2; g <= 4; ++g)
+      if (g * width <= 512 && a->off_tmp / (kSgmvBM * kSgmvBK * 2 + g * width * kSgmvBK * 2) >= 2) a->gmax = g;
+    a->part_cols = width;
+  }
+  a->off_out = a->stages * a->stage_bytes;
+  return true;
+}
+
 // y += delta or y = delta (weight == nullptr), or y = x . W^T (+ bias) + delta, of a problem that sgmv_supported takes.
 inline int prefill_cluster_launch(const SgmvProblem& b, const void* weight, int64_t w_ld, int n_total, const void* bias, bool overwrite, cudaStream_t stream) {
   const bool linear = weight != nullptr;
   PcArgs a = {};
   PcMaps maps;
   if (b.S > 32767) return fail(B200_LORA_EUNSUPPORTED, "prefill kernel: more than 32767 adapter slots");
-  prefill_cluster_split(b.T, b.in_dim, &a);
+  int n = 0;
+  for (int s = 0; s < b.st.n; ++s) n += b.st.out[s] > 0;
+  if (!prefill_cluster_plan(b, n, n_total, linear, &a)) return fail(B200_LORA_EUNSUPPORTED, "prefill kernel: too many rank rows");
   a.y = static_cast<__nv_bfloat16*>(b.y); a.y_ld = b.y_ld; a.bias = static_cast<const __nv_bfloat16*>(bias);
   a.T = b.T; a.in_dim = b.in_dim; a.n_total = n_total; a.S = b.S; a.r = b.r_max;
   a.token_to_slot = b.token_to_slot; a.scale_per_slot = b.scale_per_slot; a.scaling = b.scaling; a.overwrite = overwrite ? 1 : 0;
@@ -533,27 +567,6 @@ inline int prefill_cluster_launch(const SgmvProblem& b, const void* weight, int6
   maps.w = maps.x;
   if (linear)
     if (int rc = make_tmap_2d(&maps.w, weight, (uint64_t)n_total, (uint64_t)b.in_dim, (uint64_t)w_ld, kPcBox, kSgmvBK)) return rc;
-  a.cta_cols = round_up_i(ceil_div_i(n_total, a.ck), 64);
-  a.tile_cols = round_up_i(ceil_div_i(a.cta_cols, ceil_div_i(a.cta_cols, kSgmvBN)), 64);
-  // shared memory: ring of the tiles, output buffers, the intermediate as MMA operand; ADD launches shrink through a ring over the
-  // first two
-  const int width = a.n * a.r, tmp_bytes = a.n * kSgmvBM * a.r * 2, out_buf = a.bm * kGemmOutChunk * 2;
-  a.off_tmp = kPcSmem - tmp_bytes;
-  a.stage_bytes = linear ? kPcLinearStage : kSgmvBN * a.r * 2;
-  a.stages = linear ? 3 : kPcTileStages;
-  a.out_bufs = 2;
-  while (a.out_bufs > 0 && a.off_tmp - a.stages * a.stage_bytes < 2 * a.out_bufs * out_buf) {
-    if (!linear && a.stages > 2) --a.stages;
-    else --a.out_bufs;
-  }
-  if (a.out_bufs == 0) return fail(B200_LORA_EUNSUPPORTED, "prefill kernel: too many rank rows");
-  a.off_out = a.stages * a.stage_bytes;
-  a.part_cols = linear ? std::min(width, 2 * a.out_bufs * out_buf / (4 << a.pad_shift) & ~15) : width;
-  a.gmax = 1;
-  for (int g = 2; g <= 4; ++g) {
-    const int stage = kSgmvBM * kSgmvBK * 2 + g * width * kSgmvBK * 2;
-    if (linear ? g * width <= kSgmvBN && stage <= kPcLinearStage : g * width <= 512 && a.off_tmp / stage >= 2) a.gmax = g;
-  }
   const auto kernel = linear ? prefill_cluster_kernel<true> : prefill_cluster_kernel<false>;
   if (int rc = sgmv_set_smem(reinterpret_cast<const void*>(kernel), kPcSmem)) return rc;
   cudaLaunchConfig_t cfg = {};

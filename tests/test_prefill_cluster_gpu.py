@@ -66,3 +66,33 @@ def test_prefill_add_matches_oracle(case, overwrite):
     assert_lora_close(d.y, O.add_lora(base, p.x, p.a_slabs, p.b_slabs, slots, 0.5, p.col_offsets), what="prefill add")
     none = slots < 0
     assert torch.equal(d.y.cpu()[none].view(torch.int16), base[none].view(torch.int16)), "rows without adapter keep their bits"
+
+
+# T, in, outs, S, r, longest run: fused linears of the kernel (the plan's lines: one tile a CTA, one more over 1024 columns of x)
+LINEAR = [
+    (7, 64, [48], 2, 16, 3),                     # less than a tile of columns, some CTAs without any
+    (333, 1024, [1024, 128, 128], 4, 32, 90),    # 1280 columns over eight CTAs
+    (517, 4096, [208, 112], 3, 32, 4),           # slices of 16-column units, 40 runs a block, many passes
+    (961, 320, [1000 - 8], 3, 64, 300),          # ragged columns, blocks of 72 rows
+    (2200, 1024, [640, 640], 4, 64, 500),        # clusters of 4, two tiles a CTA
+    (4300, 128, [512], 4, 16, 128),              # clusters of 2
+]
+
+
+@pytest.mark.parametrize("case", range(len(LINEAR)))
+def test_linear_of_the_cluster_kernel_matches_oracle(case):
+    T, in_dim, outs, S, r, longest = LINEAR[case]
+    slots = by_runs(T, S, longest, 50 + case)
+    slots[0] = 0
+    p = W.make_projection(800 + case, T, in_dim, outs, S, r, token_to_slot=slots, with_weight=True)
+    d = p.to_device(DEV)
+    bias = torch.randn(sum(outs), generator=torch.Generator().manual_seed(2)).to(torch.bfloat16).to(DEV)
+    y = LORA.linear_lora(d.x, d.weight, bias, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, d.token_to_slot, 1.0)
+    plain = LORA.linear_lora(d.x, d.weight, bias, [], [], [], [], None, 1.0)
+    torch.cuda.synchronize()
+    assert N.device_status(reset=True) == 0
+    ref = O.linear_lora(p.x, p.weight, bias.cpu(), p.a_slabs, p.b_slabs, p.col_offsets, slots)
+    # half a unit in the last place of the largest output, on top of the path's tolerance
+    assert_lora_close(y, ref, max_abs=2e-2 + 2.0 ** -8 * float(ref.abs().max()), what="cluster linear")
+    none = slots < 0
+    assert torch.equal(y.cpu()[none].view(torch.int16), plain.cpu()[none].view(torch.int16)), "rows without adapter are the plain linear"
