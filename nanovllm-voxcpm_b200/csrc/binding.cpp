@@ -571,13 +571,15 @@ struct Projection {
 // needs tiles for the SMs: with fewer than 100, cuBLAS's smaller ones win. Whole steps, us, fused / separate: 4001 rows of 1024, 4 layers 888 /
 // 1120; 2000 rows of 2048, 3 layers 831 / 957; 1000 rows of 2048 (gate_up 384 tiles, the others 64 to 80) 582 / 609; 1000 rows
 // of 1024 (256, the others 32 to 40) 416 / 367.
+// Narrow outputs, from 45 tiles on (prefill_cluster_kernel: one launch): us per layer, rank 32, 1024-wide: 1500 rows 135 / 149, 2000
+// rows 168 / 172, 3000 rows 190 / 198; 1000 rows (32 and 40 tiles) 121 / 120; 2048-wide 500 rows (32, 40) 167 / 155, 1000 rows 189 / 188.
 // Long products are bound by the power cap, and there it takes more energy per operation than cuBLAS, which outweighs the pass
 // from 4096 input columns on. us per layer of whole steps, everything separate / only this projection fused, 4096-wide: 4000
 // rows gate_up with the activation (940 GFLOP) 2131 / 2318, down (470) 2131 / 2244, o (134) 2131 / 2186; 2000 rows 1020 / 1093,
 // 1020 / 1063, 1029 / 1048; 1000 rows 540 / 516 (235), 540 / 547 (118), 540 / 541 (34). 2048-wide down (6144 columns): 4000 rows
 // (101) 692 / 705, 2000 rows (50) 355 / 348; its gate_up (2048 columns, 201 and 101) 692 / 651 and 355 / 323.
 inline bool fused_linear_wins(int64_t T, int64_t K, int64_t N, bool silu) {
-  return (T + 127) / 128 * ((N + 255) / 256) >= 100 && (K < 4096 || 2.0 * (double)T * (double)K * (double)N < (silu ? 300e9 : 60e9));
+  return (T + 127) / 128 * ((N + 255) / 256) >= (N <= 1536 ? 45 : 100) && (K < 4096 || 2.0 * (double)T * (double)K * (double)N < (silu ? 300e9 : 60e9));
 }
 
 // prefill_layers(embeds, positions, cu_seqlens, max_seqlen, slot_mapping, cos, sin, layers, final_norm, metadata | None, heads,
