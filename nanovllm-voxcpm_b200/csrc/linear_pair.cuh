@@ -8,27 +8,29 @@
 // 8172 rows, without adapters, us, tile / pair kernel / cuBLAS: 2048 -> 12288 302 / 281 / 264 (all zeros: 262 / 225 / 222, the
 // power cap is the difference), 6144 -> 2048 155 / 147 / 127; with rank-32 adapters 316 / 294 and 156 / 153.
 //
-// The LoRA operands have buffers of their own, filled and masked by two warps of their own while the K loop runs: load,
-// mask and the arrival at the leader are a chain of 2 us, and in the stages of the K loop, 1 us ahead of the MMAs, every tile
-// waited for it (2048 -> 12288 of 8172 rows, rank 32: 361 us against 281 without adapters; 316 with two buffers, 294 with four).
+// The LoRA operands have buffers of their own, filled by a warp of its own while the K loop runs: in the stages of the K loop, 1 us
+// ahead of the MMAs, every tile waited for them (2048 -> 12288 of 8172 rows, rank 32: 361 us against 281 without adapters). The MMA
+// of a run of equal slots updates the rows of that run only (its lane mask).
 //
-// Who waits for whom: loads of a base stage by both CTAs count on the LEADER's full barrier (rank 0 issues all MMAs); the
-// operands of a LoRA step count on a barrier of the CTA that loaded them, whose mask warp then arrives at the leader's masked
-// barrier; commits arrive at the empty, lora_empty and acc_full barriers of both CTAs.
+// Eight epilogue warps in two sets, each with an output buffer: with four, an epilogue was longer than the K loop of the tile behind
+// it from 1024 columns of x down (SiLU form, 4001 rows, 1024 -> 2 x 4096, rank 32: 68 us with four, 56 with eight and the steps below).
+//
+// Who waits for whom: all loads, by both CTAs, count on barriers of the LEADER (rank 0 issues all MMAs); commits arrive at the empty,
+// lora_empty and acc_full barriers of both CTAs.
 #pragma once
 
 #include "prefill_cluster.cuh"
 
 namespace b200lora {
 
-constexpr int kPairThreads = 256;  // warp 0 TMA, warp 1 MMA (rank 0) + TMEM, warps 2-5 epilogue, warp 6 row mask, warp 7 LoRA loads
+constexpr int kPairThreads = 352;  // warp 0 TMA, warp 1 MMA (rank 0) + TMEM, warps 2-9 epilogue, warp 10 LoRA loads
 constexpr int kPairMaxStages = 5;
 constexpr int kPairStageBytes = 2 * kSgmvBM * kSgmvBK * 2;  // 32 KB: 128 rows of x, 128 rows of W
-constexpr int kPairOutBufs = 2;
+constexpr int kPairOutBufs = 2;                             // one of each epilogue set
 constexpr int kPairMaxLoraBufs = 4;
 constexpr int kPairMaxSeg = 2;                              // 256-row blocks that a pair's tile range may touch
 constexpr int kPairRuns = 2 * kSgmvBM;
-constexpr int kPairRunBytes = kPairRuns * 4;                // slot (int16), first and end row of this CTA's half (uint8 each)
+constexpr int kPairRunBytes = kPairRuns * 4;                // slot (int16), first and last row of the 256 (uint8 each)
 // Dynamic shared memory: ring, LoRA buffers, output buffers, run tables; 1 KB of the 227 is left to static shared memory.
 constexpr int kPairFixed = kPairOutBufs * kGemmOutBufBytes + kPairMaxSeg * kPairRunBytes;
 __host__ __device__ constexpr int pair_lora_bytes(int r) { return 2 * kSgmvBM * r * 2; }  // tmp tile and half a lora_B tile
@@ -54,6 +56,18 @@ __device__ __forceinline__ void umma_pair_elected(uint32_t d_tmem, uint32_t a_lo
       "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
       "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, p;\n\t}"
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+// the same, updating only the rows of D whose bit in `off` is clear (rows 0 - 127 in the leader's tensor memory, 128 - 255 in the peer's)
+__device__ __forceinline__ void umma_pair_rows_elected(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                                       uint32_t leader, const uint32_t (&off)[8]) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "setp.eq.b32 p, 0, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, {%6, %7, %8, %9, %10, %11, %12, %13}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(leader), "r"(off[0]), "r"(off[1]), "r"(off[2]), "r"(off[3]), "r"(off[4]),
+      "r"(off[5]), "r"(off[6]), "r"(off[7])
       : "memory");
 }
 // one arrival at the barrier of this offset in both CTAs of the pair
@@ -119,10 +133,11 @@ struct PairMaps {
 // epilogue, in fp32; neither the projection's output nor a pass over it is left (4001 x 2 x 4096: 130 MB, 21 us of its own).
 template <bool kSilu>
 __global__ void __launch_bounds__(kPairThreads, 1)
-linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
+linear_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ GemmArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ int f_n[2], seg_nruns[kPairMaxSeg];
-  __shared__ __align__(8) uint64_t bars[2 * kPairMaxStages + 3 * kPairMaxLoraBufs + 5];
+  __shared__ __align__(8) uint64_t bars[2 * kPairMaxStages + 2 * kPairMaxLoraBufs + 5];
+  __shared__ uint4 jobs[kPairMaxLoraBufs][3];  // column of D and instruction descriptor, then the lane mask, of the step in a buffer
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_flag;
 
@@ -148,15 +163,14 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
   auto f_hi = [&](int h) { return out_ptr + (8 + h) * kSgmvBM; };
   auto run_slot = [&](int sg) { return reinterpret_cast<int16_t*>(tables + sg * kPairRunBytes); };
   auto run_lo = [&](int sg) { return tables + sg * kPairRunBytes + 2 * kPairRuns; };
-  auto run_hi = [&](int sg) { return tables + sg * kPairRunBytes + 3 * kPairRuns; };
+  auto run_last = [&](int sg) { return tables + sg * kPairRunBytes + 3 * kPairRuns; };
   const uint32_t bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * (uint32_t)s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (uint32_t)(kPairMaxStages + s); };
   auto lora_bar = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + b); };
-  auto masked_bar = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + kPairMaxLoraBufs + b); };
-  auto lora_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 2 * kPairMaxLoraBufs + b); };
-  auto acc_full = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 3 * kPairMaxLoraBufs + b); };
-  auto acc_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 3 * kPairMaxLoraBufs + 2 + b); };
+  auto lora_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + kPairMaxLoraBufs + b); };
+  auto acc_full = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 2 * kPairMaxLoraBufs + b); };
+  auto acc_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * kPairMaxStages + 2 * kPairMaxLoraBufs + 2 + b); };
   constexpr int tmem_cols = 2 * kSgmvBN;
   const uint32_t tables_bar = acc_empty(2);
   const bool aligned = (smem_base & 1023u) == 0;  // (the same in both CTAs)
@@ -165,10 +179,9 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
     for (int s = 0; s < kPairMaxStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int b = 0; b < kPairMaxLoraBufs; ++b) {
       mbar_init(lora_bar(b), 1);
-      mbar_init(masked_bar(b), 2);  // the mask warps of both CTAs
       mbar_init(lora_empty(b), 1);
     }
-    for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 8); }  // four epilogue warps of each CTA
+    for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 16); }  // eight epilogue warps of each CTA
     mbar_init(tables_bar, 128);
     abort_flag = 0;
     mbar_fence_init();
@@ -231,9 +244,10 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
         }
       }
     }
-  } else if (warp == 7) {
-    // ---- LoRA loads: this CTA's rows of tmp and half of the lora_B tile, one buffer ahead of the mask warp
-    const uint32_t leader = elect_one();
+  } else if (warp == 10) {
+    // ---- LoRA loads: this CTA's rows of tmp and half of the lora_B tile
+    const uint32_t leader = elect_one(), lora0 = mapa_shared(lora_bar(0), 0);
+    const uint64_t policy = l2_policy_evict_normal();
     if (a.lora) {
       mbar_wait_bounded(tables_bar, 0u, &abort_flag);
       griddep_wait();  // tmp is final from here on
@@ -246,49 +260,28 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
       for (int j = ja; j < jb; ++j)
         for (int u = 0; u < nruns; ++u) {
           const int slot = uniform(run_slot(sg)[u]);
+          // What the MMA warp needs is put beside the operands here, well ahead: between two K loops 30 instructions of one warp
+          // for each run and piece were 0.5 us of an idle tensor pipe.
+          const int lo_row = run_lo(sg)[u], hi_row = run_last(sg)[u] + 1;
+          uint32_t off[8];
+#pragma unroll
+          for (int w = 0; w < 8; ++w) off[w] = rows_outside(lo_row, hi_row, w);
           for (int q = 0; q < n_pieces; ++q) {
             int s, lo, hi, d;
             if (!piece(q, j, s, lo, hi, d)) continue;
             if (round > 0) mbar_wait_bounded(lora_empty(b), (uint32_t)((round & 1) ^ 1), &abort_flag);
             if (leader) {
-              const uint32_t base = lora_base + (uint32_t)b * lora_bytes;
-              mbar_arrive_expect_tx(lora_bar(b), lora_bytes);
-              tma_load_2d(base, &maps.t, 0, s * a.T + row0, lora_bar(b));
-              tma_load_2d(base + t_tile_bytes, &maps.b[s], 0, slot * a.out[s] + (lo - a.col[s]) + rank * ((hi - lo) >> 1), lora_bar(b));
+              const uint32_t base = lora_base + (uint32_t)b * lora_bytes, bar = lora0 + 8u * (uint32_t)b;
+              if (rank == 0) {
+                jobs[b][0] = make_uint4((uint32_t)d, umma_idesc_bf16(2 * kSgmvBM, hi - lo), 0u, 0u);  // (a multiple of 32: see the launch)
+                jobs[b][1] = make_uint4(off[0], off[1], off[2], off[3]);
+                jobs[b][2] = make_uint4(off[4], off[5], off[6], off[7]);
+                mbar_arrive_expect_tx(lora_bar(b), 2 * lora_bytes);  // both CTAs' loads
+              }
+              tma_load_2d_pair(base, &maps.t, 0, s * a.T + row0, bar, policy);
+              tma_load_2d_pair(base + t_tile_bytes, &maps.b[s], 0, slot * a.out[s] + (lo - a.col[s]) + rank * ((hi - lo) >> 1), bar, policy);
             }
             __syncwarp();
-            if (++b == LB) { b = 0; ++round; }
-          }
-        }
-    }
-  } else if (warp == 6) {
-    // ---- mask warp: zero this CTA's tmp rows outside the run, then tell the leader
-    const uint32_t masked0 = mapa_shared(masked_bar(0), 0);
-    if (a.lora) mbar_wait_bounded(tables_bar, 0u, &abort_flag);
-    int b = 0, round = 0;
-    for (int sg = 0; sg < nseg; ++sg) {
-      int blk, ja, jb;
-      seg_range(sg, blk, ja, jb);
-      const int nruns = a.lora ? seg_nruns[sg] : 0;
-      for (int j = ja; j < jb; ++j)
-        for (int u = 0; u < nruns; ++u) {
-          const int lo_row = run_lo(sg)[u], hi_row = run_hi(sg)[u];
-          for (int q = 0; q < n_pieces; ++q) {
-            int s, lo, hi, d;
-            if (!piece(q, j, s, lo, hi, d)) continue;
-            mbar_wait_bounded(lora_bar(b), (uint32_t)(round & 1), &abort_flag);
-            if (lo_row > 0 || hi_row < kSgmvBM) {
-              const uint32_t base = lora_base + (uint32_t)b * lora_bytes;
-              const int chunks = row_bytes >> 4, rows_per_step = 32 / chunks, sub = lane / chunks;
-              const uint32_t piece = (uint32_t)(lane - sub * chunks) * 16u;
-              for (int row = sub; row < lo_row; row += rows_per_step)
-                asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(base + (uint32_t)(row * row_bytes) + piece), "r"(0u) : "memory");
-              for (int row = hi_row + sub; row < kSgmvBM; row += rows_per_step)
-                asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(base + (uint32_t)(row * row_bytes) + piece), "r"(0u) : "memory");
-              fence_proxy_async_smem();
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote_release(masked0 + 8u * (uint32_t)b);
             if (++b == LB) { b = 0; ++round; }
           }
         }
@@ -304,7 +297,7 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
       int blk, ja, jb;
       seg_range(sg, blk, ja, jb);
       ja = uniform(ja); jb = uniform(jb);
-      int nruns = 0;
+      int nruns = 0, steps = 0;  // LoRA steps of a tile
       for (int j = ja; j < jb; ++j, ++job) {
         const int buf = job & 1;
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kSgmvBN);
@@ -319,38 +312,40 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
             umma_pair_elected(d_tmem, xl + 2u * k4, wl + 2u * k4, hi_x, idesc_base, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
           umma_commit_pair_elected(empty_bar(st), leader);
           if (++st == NS) { st = 0; ++round; }
-        }
-        if (a.lora && j == ja) {
-          mbar_wait_bounded(tables_bar, 0u, &abort_flag);
-          nruns = uniform(seg_nruns[sg]);
-        }
-        for (int u = 0; u < nruns; ++u) {
-          for (int q = 0; q < n_pieces; ++q) {
-            int s, lo, hi, d;
-            if (!piece(q, j, s, lo, hi, d)) continue;
-            mbar_wait_bounded_acquire_cluster(masked_bar(lb), (uint32_t)(lround & 1), &abort_flag);
-            tc_fence_after_sync();
-            const uint32_t tl = lt0 + ((uint32_t)lb * lora_bytes >> 4), bl = tl + (t_tile_bytes >> 4);
-            const uint32_t idesc = umma_idesc_bf16(2 * kSgmvBM, hi - lo);  // (a multiple of 32: see the launch)
-#pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4)
-              if (16 * k4 < r)
-                umma_pair_elected(d_tmem + (uint32_t)d, tl + 2u * k4, bl + 2u * k4, hi_t, idesc, 1u, leader);
-            umma_commit_pair_elected(lora_empty(lb), leader);
-            if (++lb == LB) { lb = 0; ++lround; }
+          if (a.lora && kc == min(1, nk - 1)) {  // (while the MMAs of the first steps run)
+            if (j == ja) {
+              mbar_wait_bounded(tables_bar, 0u, &abort_flag);
+              nruns = uniform(seg_nruns[sg]);
+            }
+            steps = 0;
+            for (int q = 0; q < n_pieces; ++q) {
+              int s, lo, hi, d;
+              steps += piece(q, j, s, lo, hi, d) ? nruns : 0;
+            }
           }
+        }
+        for (int k = 0; k < steps; ++k) {
+          mbar_wait_bounded_acquire_cluster(lora_bar(lb), (uint32_t)(lround & 1), &abort_flag);
+          tc_fence_after_sync();
+          const uint32_t tl = lt0 + ((uint32_t)lb * lora_bytes >> 4), bl = tl + (t_tile_bytes >> 4);
+          const uint4 what = jobs[lb][0], m0 = jobs[lb][1], m1 = jobs[lb][2];
+          const uint32_t off[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+          for (int k4 = 0; k4 < 4; ++k4)
+            if (16 * k4 < r) umma_pair_rows_elected(d_tmem + what.x, tl + 2u * k4, bl + 2u * k4, hi_t, what.y, leader, off);
+          umma_commit_pair_elected(lora_empty(lb), leader);
+          if (++lb == LB) { lb = 0; ++lround; }
         }
         umma_commit_pair_elected(acc_full(buf), leader);
       }
     }
-  } else if (warp >= 2 && warp <= 5) {
-    // ---- epilogue: thread <-> row of this CTA's half
-    const int quarter = warp & 3, row_in_blk = quarter * 32 + lane, etid = tid - 64;
+  } else if (warp >= 2 && warp <= 9) {
+    // ---- epilogue: thread <-> row of this CTA's half; the two sets take the 64-column chunks of a tile in turn
+    const int quarter = warp & 3, row_in_blk = quarter * 32 + lane, set = (warp - 2) >> 2, etid = tid - 64 - 128 * set;
     const uint32_t acc_empty0 = mapa_shared(acc_empty(0), 0);
-    int job = 0, chunk_no = 0;
-    if (a.lora) {
-      // Runs of equal slot of every block, first half then second, a run over the middle once: both CTAs walk the same list,
-      // each with the rows of its own half (none: the whole of its tmp tile is masked). Made while the first K loop runs.
+    int job = 0;
+    if (a.lora && set == 0) {
+      // Runs of equal slot of every block, first half then second, a run over the middle once. Made while the first K loop runs.
       for (int sg = 0; sg < nseg; ++sg) {
         pair_find_runs(a.token_to_slot, a.T, a.S, 2 * (blk_first + sg), etid, f_slot, f_run(0), f_lo(0), f_hi(0), f_n);
         const int n0 = f_n[0], n1 = f_n[1];
@@ -358,10 +353,9 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
         const int total = n0 + n1 - joint;
         for (int i = etid; i < total; i += 128) {
           const int k0 = i < n0 ? i : -1, k1 = i >= n0 - joint ? i - n0 + joint : -1;  // entry of the first / second half's list
-          const int mine = rank == 0 ? k0 : k1;
           run_slot(sg)[i] = k0 >= 0 ? f_run(0)[k0] : f_run(1)[k1];
-          run_lo(sg)[i] = mine >= 0 ? f_lo(rank)[mine] : 0;
-          run_hi(sg)[i] = mine >= 0 ? f_hi(rank)[mine] : 0;
+          run_lo(sg)[i] = (uint8_t)(k0 >= 0 ? f_lo(0)[k0] : kSgmvBM + f_lo(1)[k1]);
+          run_last(sg)[i] = (uint8_t)((k1 >= 0 ? kSgmvBM + f_hi(1)[k1] : f_hi(0)[k0]) - 1);
         }
         if (etid == 0) seg_nruns[sg] = total;
         named_bar_sync(2, 128);
@@ -376,12 +370,12 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
         const int buf = job & 1;
         mbar_wait_bounded_acquire_cluster(acc_full(buf), (uint32_t)((job >> 1) & 1), &abort_flag);
         tc_fence_after_sync();
-        for (int c = 0; c < kCols; c += kGemmOutChunk, ++chunk_no) {
+        for (int c = kGemmOutChunk * set; c < kCols; c += 2 * kGemmOutChunk) {
           const int col0 = j * kCols + c;
-          if (col0 >= a.n_total || row0 >= a.T) break;  // uniform over the CTA
-          const uint32_t obuf = out_base + (uint32_t)(chunk_no % kPairOutBufs) * kGemmOutBufBytes;
-          if (etid == 0) bulk_wait_group_read<kPairOutBufs - 1>();  // the store that last used this buffer has read it
-          named_bar_sync(2, 128);
+          if (col0 >= a.n_total || row0 >= a.T) break;  // uniform over the set
+          const uint32_t obuf = out_base + (uint32_t)set * kGemmOutBufBytes;
+          if (etid == 0) bulk_wait_group_read<0>();  // the store that last used this buffer has read it
+          named_bar_sync(3 + (uint32_t)set, 128);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t v[32];
@@ -423,7 +417,7 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const GemmArgs a) {
             }
           }
           fence_proxy_async_smem();
-          named_bar_sync(2, 128);
+          named_bar_sync(3 + (uint32_t)set, 128);
           if (etid == 0) {
             tma_store_2d_hint(&maps.y, obuf, col0, row0, l2_policy_evict_first());
             bulk_commit_group();
@@ -530,7 +524,7 @@ inline bool prefill_cluster_linear_ok(const LinearProblem& p) {
   const int nk = b.in_dim / kSgmvBK, tiles = ceil_div_i(a.cta_cols, a.tile_cols), total = ceil_div_i(b.T, kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
   const int64_t pair_tiles = (int64_t)ceil_div_i(b.T, 2 * kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
   const int rounds = pair_tiles >= kPairMinTiles ? ceil_div_i((int)pair_tiles, kTileSMs / 2) : ceil_div_i(total, kTileSMs);
-  return n * b.r_max <= 128 && b.in_dim <= 4096 && (tiles <= rounds || (tiles <= 2 && (tiles - rounds) * nk <= 16));
+  return n * b.r_max <= 128 && b.in_dim <= 4096 && ((tiles <= rounds && tiles <= 3) || (tiles <= 2 && (tiles - rounds) * nk <= 16));
 }
 
 // y = x . W^T (+ bias) + LoRA delta, the delta accumulated into the GEMM's TMEM accumulator.
