@@ -106,7 +106,9 @@ namespace {
 //   qkv (18 MB) 7.0 / 10.5, gate_up (41 MB) 9.3 / 13.1, 1300 rows 10 / 10.5 and 15 / 13.1, 2200 rows 14 / 11.7 and 22 / 19;
 //   2048-wide, rank 32: 1000 rows qkv (35 MB) 9.4 / 11.8, gate_up (66 MB) 20 / 16, 1500 rows 16 / 12.7 and 32 / 19; rank 64: 700 rows
 //   qkv (49 MB) 16.7 / 14.1, down (46 MB) 23 / 11.2, o (23 MB) 7.5 / 9.5. Over 900 measured points of 300 to 3200 rows, three
-//   widths and ranks, this line is 1.2 % slower than the better choice each time (the line below: 6.2 %).
+//   widths and ranks, this line is 2.1 % slower than the better choice each time (without the line at 75 windows 6.2 %). At 35 MB
+//   it would be 1.2 %, but adapters of mixed ranks cost the bucket kernel less: 962 rows, 1024-wide, ranks 8 to 32, gate_up (40
+//   MB): a layer 24.6 / 29.4.
 //   sgmv_shrink_kernel and the launch behind it (operators, slices that do not tile the output; at least 11 us for the pair): bucket /
 //   pair, six prompts: 1024-wide, rank 32, 900 rows, qkv (16 MB) 6.7 / 13.5, gate_up (37 MB) 8.9 / 15.1, 1500 rows 11.5 / 13.8 and
 //   (61 MB) 18.6 / 20.4; 2048-wide, rank 32, 900 rows, gate_up (59 MB) 19.0 / 19.1, 1500 rows (98 MB) 32.9 / 24.7; rank 64, 900
@@ -117,7 +119,7 @@ inline bool prefill_sized(int32_t T, const SliceTable& st, int32_t r_max, int32_
     if (st.out[s] > 0 || !expand) bytes += 2 * (int64_t)r_max * (in_dim + (expand ? st.out[s] : 0));
   bytes *= ceil_div_i(T, kBgmvTok);
   if (T < kSgmvAutoMinTokens) return false;
-  return r_max > 32 || (one_launch ? ceil_div_i(T, kBgmvTok) > 74 || bytes > 35 * 1000 * 1000 : bytes > 50 * 1000 * 1000);
+  return r_max > 32 || bytes > 50 * 1000 * 1000 || (one_launch && ceil_div_i(T, kBgmvTok) > 74);
 }
 
 }  // namespace
