@@ -497,6 +497,19 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     if (++c_stage == NS) { c_stage = 0; c_parity ^= 1u; stage_addr = ring_base; }
   };
 
+  __nv_bfloat16* const ylo_p = p.y + (int64_t)max(tok_lo, 0) * p.y_ld + y_col;
+  __nv_bfloat16* const yhi_p = p.y + (int64_t)max(tok_hi, 0) * p.y_ld + y_col;
+  // kinds 1 and 2: y of the next tile is requested while this one is multiplied, the first one behind the shrink
+  // (its 0.5 us of latency then lie beside the exchange: 37 rows, rank 16 74.1 -> 70.9 us a layer stack, 64 rows fp16 43.5 -> 40.7; before the
+  // shrink it delays the x loads: 76.0 and 45.0)
+  uint4 y_next[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+  auto load_y = [&](int e) {
+    if (e >= tiles_exp || kF32Out || (kMode == 2 && p.no_add)) return;
+    const int2 te = etab[e];
+    if (y_col >= (te.y & 0xffff) || !B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) return;
+    if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + te.x);
+    if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + te.x);
+  };
   const __nv_bfloat16* const xlo_p = p.x + (int64_t)max(tok_lo, 0) * p.x_ld + x_col;
   const __nv_bfloat16* const xhi_p = p.x + (int64_t)max(tok_hi, 0) * p.x_ld + x_col;
 
@@ -580,6 +593,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     }
   }
   B200_TRACE_POINT(6)
+  if (kPrecise) load_y(sub);
 
   // ===== cross-warp reduction of the K slices, scale, bf16, all-gather =====
   named_bar_sync(1, kBgmvConsumers);
@@ -681,18 +695,6 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
 
   // ===== expand: y[tok, cols] += tmp[16 tok, r] . B_rows^T ======================
   // Rows of a stage beyond the tile's rows hold stale bytes; their products land in columns that are not written.
-  __nv_bfloat16* const ylo_p = p.y + (int64_t)max(tok_lo, 0) * p.y_ld + y_col;
-  __nv_bfloat16* const yhi_p = p.y + (int64_t)max(tok_hi, 0) * p.y_ld + y_col;
-  // kinds 1 and 2: y of the next tile is requested while this one is multiplied (the first one here, behind the wait)
-  uint4 y_next[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-  auto load_y = [&](int e) {
-    if (e >= tiles_exp || kF32Out || (kMode == 2 && p.no_add)) return;
-    const int2 te = etab[e];
-    if (y_col >= (te.y & 0xffff) || !B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) return;
-    if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + te.x);
-    if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + te.x);
-  };
-  if (kPrecise) load_y(sub);
   auto expand_fn = [&](int e, uint32_t tile_addr) {
     const int2 te = etab[e];
     const uint4 y_lo = y_next[0], y_hi = y_next[1];
