@@ -112,7 +112,6 @@ struct BgmvParams {
   int stage_bytes, NS;
   int red_pitch;    // floats per token row of the cross-warp reduction buffer
   int pitchT;       // bytes per token row of tmp
-  int lo_off;       // kinds 1, 2: bytes from a token's high halves to its low halves
   int kind;
   int off_red, off_tmp, off_tab, off_bar;
   int full_k;       // every K part has all 1024 columns
@@ -468,13 +467,13 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   // thread-constant pieces of the shared-memory addresses
   const uint32_t pitchB = (uint32_t)p.r_max * 2u;
   const uint32_t a_off = (uint32_t)(g * pitchA + x_col * 2);                            // shrink tile: row g
-  const uint32_t w_off = (uint32_t)(rb + 8 * (g >> 1) + (g & 1)) * pitchB + (uint32_t)t * 16u;  // expand tile
+  const uint32_t w_off = (uint32_t)(rb + 8 * (g >> 1) + (g & 1)) * pitchB + (uint32_t)t * (kPrecise ? 8u : 16u);  // expand tile
   // MMA column n of n-tile j reads slab row 8*(n/2) + 2j + (n%2) of the warp's 32 rows: thread (g,t)
   // then owns 8 consecutive output columns 8t..8t+7 of the block.
   const uint32_t t_off = (uint32_t)(g * p.pitchT + t * 16);                             // tmp: token row g
   float* const red_wr = red + ((size_t)warp * kBgmvTok + g) * p.red_pitch + 2 * t;      // + 8 * pitch: token g + 8
-  // expand: 32-column blocks of the intermediate; kinds 1 and 2 run through [high halves | low halves], 2 r_eff columns,
-  // against the same weights twice
+  // expand: 32-column blocks of the intermediate; kinds 1 and 2 keep it as groups [four high halves | four low halves], 16 columns
+  // a block, so that a 16-byte fragment is both halves of four columns and the weights are read once
   const int kblocks = kPrecise ? r_eff >> 4 : r_eff >> 5;
   // all-gather item of this thread: one token row x four consecutive rank rows of this CTA
   const int groups = rows_c >> 2;
@@ -482,7 +481,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   const int it_tok = has_item ? tid / max(groups, 1) : 0;
   const int it_q = q_lo + 4 * (has_item ? tid - it_tok * groups : 0);
   const float* const red_rd = red + (size_t)it_tok * p.red_pitch + (it_q - q_lo);
-  const uint32_t it_off = (uint32_t)(it_tok * p.pitchT + it_q * 2);
+  const uint32_t it_off = (uint32_t)(it_tok * p.pitchT + it_q * (kPrecise ? 4 : 2));
   const uint32_t tmp_u32 = smem_u32(tmp_base);
 
   if (p.use_pdl) griddep_wait();  // x and y of this launch are final from here on
@@ -610,16 +609,16 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     for (int pr = tid & 15; pr < (Q >> 1); pr += 16) {
       const int q = 2 * pr, s = q / r_eff, rr = q - s * r_eff;
       const int64_t at = ((int64_t)s * p.T + trow) * p.r_max + rr;
-      uint32_t* const dst = reinterpret_cast<uint32_t*>(tmp_base + (size_t)tok * p.pitchT + (size_t)q * 2);
+      uint32_t* const dst = reinterpret_cast<uint32_t*>(tmp_base + (size_t)tok * p.pitchT + (size_t)(kPrecise ? (q >> 2) * 16 + (q & 3) * 2 : q * 2));
       if (p.io16) {
         *dst = trow >= 0 ? *reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(p.tmp_io) + at) : 0u;
-        if (kPrecise) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(dst) + p.lo_off) = 0u;
+        if (kPrecise) dst[2] = 0u;
       } else {
         float2 v = make_float2(0.f, 0.f);
         if (trow >= 0) v = *reinterpret_cast<const float2*>(static_cast<const float*>(p.tmp_io) + at);
         const uint32_t h = pack_16x2<kF16>(v.x, v.y);
         *dst = h;
-        if (kPrecise) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(dst) + p.lo_off) = pack_rest<kF16>(v.x, v.y, h);
+        if (kPrecise) dst[2] = pack_rest<kF16>(v.x, v.y, h);
       }
     }
     named_bar_sync(1, kBgmvConsumers);
@@ -661,9 +660,8 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
         const uint32_t l0 = kPrecise ? pack_rest<kF16>(a.x * sc, a.y * sc, v0) : 0u, l1 = kPrecise ? pack_rest<kF16>(a.z * sc, a.w * sc, v1) : 0u;
 #pragma unroll 1
         for (int rc = 0; rc < C; ++rc) {
-          st_async_b32x2(mapa_shared(tmp_u32 + it_off, (uint32_t)rc), v0, v1, mapa_shared(tmp_ready_bar, (uint32_t)rc));
-          if (kPrecise)
-            st_async_b32x2(mapa_shared(tmp_u32 + it_off + (uint32_t)p.lo_off, (uint32_t)rc), l0, l1, mapa_shared(tmp_ready_bar, (uint32_t)rc));
+          if (kPrecise) st_async_b32x4(mapa_shared(tmp_u32 + it_off, (uint32_t)rc), make_uint4(v0, v1, l0, l1), mapa_shared(tmp_ready_bar, (uint32_t)rc));
+          else st_async_b32x2(mapa_shared(tmp_u32 + it_off, (uint32_t)rc), v0, v1, mapa_shared(tmp_ready_bar, (uint32_t)rc));
         }
       }
     }
@@ -682,10 +680,10 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
           }
           const uint32_t v0 = pack_16x2<kF16>(a.x * sc, a.y * sc), v1 = pack_16x2<kF16>(a.z * sc, a.w * sc);
           uint8_t* dst = tmp_base + it_off;
-          *reinterpret_cast<uint2*>(dst) = make_uint2(v0, v1);
           if (kPrecise)
-            *reinterpret_cast<uint2*>(dst + p.lo_off) =
-                make_uint2(pack_rest<kF16>(a.x * sc, a.y * sc, v0), pack_rest<kF16>(a.z * sc, a.w * sc, v1));
+            *reinterpret_cast<uint4*>(dst) = make_uint4(v0, v1, pack_rest<kF16>(a.x * sc, a.y * sc, v0), pack_rest<kF16>(a.z * sc, a.w * sc, v1));
+          else
+            *reinterpret_cast<uint2*>(dst) = make_uint2(v0, v1);
         }
         named_bar_sync(1, kBgmvConsumers);
       }
@@ -702,22 +700,23 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     float d[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.f;
-    const uint32_t a_addr = tmp_u32 + t_off + (uint32_t)((te.y >> 16) * r_eff * 2);
+    const uint32_t a_addr = tmp_u32 + t_off + (uint32_t)((te.y >> 16) * r_eff * (kPrecise ? 4 : 2));
     const uint32_t w_addr = tile_addr + w_off;
 #pragma unroll 1
     for (int kb = 0; kb < kblocks; ++kb) {
-      uint32_t a_kb = a_addr + 64u * kb, w_kb = w_addr + 64u * kb;
-      if (kPrecise) {
-        // this thread's eight columns start at 32 kb + 8 t of [high | low]; a_addr and w_addr already hold 16 t bytes
-        const int at = 32 * kb + 8 * t, low = at >= r_eff;
-        a_kb = a_addr + (uint32_t)(64 * kb + (low ? p.lo_off - 2 * r_eff : 0));
-        w_kb = w_addr + (uint32_t)(64 * kb - (low ? 2 * r_eff : 0));
-      }
+      const uint32_t a_kb = a_addr + 64u * kb, w_kb = w_addr + (kPrecise ? 32u : 64u) * kb;
       const uint4 alo = lds128(a_kb);
       const uint4 ahi = lds128(a_kb + 8u * (uint32_t)p.pitchT);
       uint4 w[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = lds128(w_kb + 2u * j * pitchB);
+      for (int j = 0; j < 4; ++j) {
+        if (kPrecise) {
+          const uint2 four = lds64(w_kb + 2u * j * pitchB);
+          w[j] = make_uint4(four.x, four.y, four.x, four.y);
+        } else {
+          w[j] = lds128(w_kb + 2u * j * pitchB);
+        }
+      }
 #pragma unroll
       for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.x, ahi.x, alo.y, ahi.y, w[j].x, w[j].y);
 #pragma unroll
@@ -922,7 +921,6 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   p.red_pitch = (Rc % 16 == 8) ? Rc : Rc + 8;
   const int red_bytes = round_up_i(kBgmvWarps * kBgmvTok * p.red_pitch * 4, 128);
   p.kind = b.kind;
-  p.lo_off = Q * 2;
   p.pitchT = round_up_i(Q * (b.kind != 0 ? 4 : 2), 128) + 64;
   const int tmp_bytes = round_up_i(kBgmvTok * p.pitchT, 128);
   const int bar_bytes = 256;

@@ -59,11 +59,6 @@ __device__ __forceinline__ uint32_t swizzled_piece(int row, int c, int row_bytes
   const int x = row_bytes == 128 ? (row & 7) : (row_bytes == 64 ? (row >> 1) & 3 : (row >> 2) & 1);
   return (uint32_t)(row * row_bytes + ((c ^ x) << 4));
 }
-__device__ __forceinline__ void st_async_b32x4(uint32_t cluster_addr, uint4 v, uint32_t cluster_bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(cluster_addr),
-               "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(cluster_bar)
-               : "memory");
-}
 
 template <bool kLinear>
 __global__ void __launch_bounds__(kPcThreads, 1)
