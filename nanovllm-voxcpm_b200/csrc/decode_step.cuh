@@ -358,12 +358,11 @@ __global__ void __launch_bounds__(256) decode_silu_mul_kernel(__nv_bfloat16* __r
 
 // ============================================================================ attention
 // One CTA per (kv head, request): sums the planes of the request's q heads of that kv head, k and v, rotates q and k, stores k
-// and v to the paged cache and attends over the cached tokens. The K and V rows of a chunk of tokens are requested with
-// cp.async, those of earlier steps before the wait; eight warps take 16 tokens each in turn (mma.sync m16n8k16 with the up
-// to 16 q heads as rows, online softmax per warp, merged at the end).
-constexpr int kDecAttnThreads = 256;
-constexpr int kDecAttnWarps = 8;
-
+// and v to the paged cache and attends over the cached tokens (mma.sync m16n8k16 with the up to 16 q heads as rows, online
+// softmax per warp, merged at the end). Every warp has blocks of 16 tokens of its own and stages of its own for their K and V
+// rows: the first ones are requested (cp.async) before the wait, the next one as soon as a stage is free, and no warp waits for
+// another before the merge. (Chunks of 368 tokens shared by the CTA, one after the other: 64 requests around 352 tokens 8.2 us
+// a layer, around 640 14.4; now 6.9 and 12.0.)
 struct DecAttnArgs {
   const float* part; int planes, ld;       // [planes, T, (Hq + 2 Hk) D]
   int T, Hq, Hk;
@@ -387,56 +386,70 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t (&r)[4]) {
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint32_t bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+constexpr int kDecAttnWarps = 8;
+// A warp's items are the K and V rows of its blocks together (heads of 64), or K and V in turn (128: one and a half blocks are all
+// that fits, two CTAs per SM); slots of an item
 template <int D>
-__host__ __device__ constexpr int dec_attn_chunk() { return D == 64 ? 368 : 192; }  // tokens in shared memory at a time (two CTAs per SM)
+__host__ __device__ constexpr int dec_attn_slots() { return 3; }
 template <int D>
 __host__ __device__ constexpr int dec_attn_smem() {
-  const int kv = 2 * dec_attn_chunk<D>() * (D * 2 + 16), merge = kDecAttnWarps * 16 * (D + 2) * 4;
+  const int kv = kDecAttnWarps * dec_attn_slots<D>() * (D == 64 ? 2 : 1) * 16 * (D * 2 + 16), merge = kDecAttnWarps * 16 * (D + 2) * 4;
   return (kv > merge ? kv : merge) + 16 * (D * 2 + 16);
 }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
 template <int D>
-__global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const DecAttnArgs a) {
+__global__ void __launch_bounds__(kDecAttnWarps * 32) decode_attention_kernel(const DecAttnArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr int kPitch = D * 2 + 16, kChunk = dec_attn_chunk<D>(), kHalf = D / 2;
+  constexpr int kPitch = D * 2 + 16, kHalf = D / 2, kWarps = kDecAttnWarps, kThreads = kWarps * 32, kSlots = dec_attn_slots<D>();
+  constexpr bool kTurn = D == 128;  // K and V in turn
+  constexpr int kRows = 16 * kPitch, kItem = (kTurn ? 1 : 2) * kRows;  // bytes of the K or V rows of a block, of an item
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int kvh = blockIdx.x, req = blockIdx.y, group = a.Hq / a.Hk;
   griddep_launch_dependents();
-  const uint32_t q_u32 = smem_u32(smem), k_u32 = q_u32 + 16 * kPitch, v_u32 = k_u32 + kChunk * kPitch;
+  const uint32_t q_u32 = smem_u32(smem), kv_u32 = q_u32 + kRows + (uint32_t)(warp * kSlots * kItem);  // this warp's slots
   // (the cache rows of earlier steps were written before this chain of dependent launches began: see the header)
   const int ctx = a.context_lens[req];
   const int32_t* table = a.block_tables + (int64_t)req * a.max_blocks;
   const int n_old = max(ctx - 1, 0);  // tokens whose k and v are in the cache already
-  __shared__ int64_t cache_row[kChunk];
+  const int n_blocks = (ctx + 15) >> 4;
 
-  // rows [c0, c0 + n) of the cache into the chunk buffers; the last row of all is the new token's (written below), rows up
-  // to the next multiple of 16 are zero (their probabilities are zero, their values must be finite)
-  auto load_chunk = [&](int c0, int n) {
-    const int rows = (n + 15) & ~15;
-    constexpr int kPieces = D / 8;
-    // where each row lies first (a look-up and a division per row, not per piece: those took 4 us)
-    for (int r = tid; r < n; r += kDecAttnThreads) {
-      const int tok = c0 + r;
-      const int blk = table[tok / a.block_size];
-      cache_row[r] = blk * (int64_t)a.block_size + tok % a.block_size;
-    }
-    __syncthreads();
-    const int p = tid % kPieces;
-    const uint32_t off0 = (uint32_t)(p * 16);
-    const int64_t at0 = (int64_t)kvh * D + p * 8, row_ld = (int64_t)a.Hk * D;
-#pragma unroll 4
-    for (int r = tid / kPieces; r < rows; r += kDecAttnThreads / kPieces) {
-      if (c0 + r == n_old && r < n) continue;
-      const bool live = r < n;
-      const int64_t at = live ? cache_row[r] * row_ld + at0 : 0;
-      const uint32_t off = (uint32_t)(r * kPitch) + off0;
-      cp_async_16(k_u32 + off, a.k_cache + at, live ? 16u : 0u);
-      cp_async_16(v_u32 + off, a.v_cache + at, live ? 16u : 0u);
-    }
+  // A warp's blocks are warp, warp + 8, ... First element of the cache rows of its block j (lane l: row l % 16):
+  auto rows_of = [&](int j) {
+    const int tok = 16 * (warp + j * kWarps) + (lane & 15);
+    if (16 * (warp + j * kWarps) >= n_old || tok >= n_old) return (int64_t)0;
+    const int blk = table[tok / a.block_size];
+    return (blk * (int64_t)a.block_size + tok % a.block_size) * ((int64_t)a.Hk * D) + (int64_t)kvh * D;
   };
-  if (ctx > 0) load_chunk(0, min(ctx, kChunk));
+  // K (which 0), V (1) or both (2) of block j into a slot: cached rows; that of the new token is written below, rows behind the
+  // context are zero (their probabilities are zero, their values must be finite). A group is committed for missing blocks too.
+  auto load_item = [&](int j, int which, uint32_t slot, int64_t at) {
+    const int b = warp + j * kWarps;
+    if (b < n_blocks) {
+      constexpr int kPieces = D / 8;  // 16-byte pieces of a row
+      const int p = lane % kPieces;
+#pragma unroll
+      for (int q = 0; q < kPieces / 2; ++q) {
+        const int r = lane / kPieces + q * (32 / kPieces);
+        const int64_t row = __shfl_sync(0xffffffffu, at, r) + p * 8;
+        if (16 * b + r == n_old && ctx > 0) continue;
+        const bool live = 16 * b + r < n_old;
+        const uint32_t dst = slot + (uint32_t)(r * kPitch + p * 16);
+        if (which != 1) cp_async_16(dst, a.k_cache + (live ? row : 0), live ? 16u : 0u);
+        if (which != 0) cp_async_16(dst + (which == 2 ? (uint32_t)kRows : 0u), a.v_cache + (live ? row : 0), live ? 16u : 0u);
+      }
+    }
+    cp_async_commit();
+  };
+  int64_t at = 0;  // (in turn) of the block whose K was asked for last
+#pragma unroll
+  for (int i = 0; i < kSlots; ++i) {
+    if (!kTurn || (i & 1) == 0) at = rows_of(kTurn ? i >> 1 : i);
+    load_item(kTurn ? i >> 1 : i, kTurn ? i & 1 : 2, kv_u32 + (uint32_t)(i * kItem), at);
+  }
 
   // ---- q, k, v of the new token: a thread takes four pairs (j, j + D / 2) of a head
   int64_t pos = a.positions[req];
@@ -444,12 +457,9 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
   const int64_t slot = a.slot_mapping[req];
   const int64_t plane = (int64_t)a.T * a.ld, row_at = (int64_t)req * a.ld;
   const int hi_off = a.table_dim == D ? kHalf : 0;
-  uint8_t* const k_new = smem + 16 * kPitch + (n_old % kChunk) * kPitch;
-  uint8_t* const v_new = k_new + kChunk * kPitch;
-  const bool new_in_first = n_old < kChunk;
   __shared__ __align__(16) __nv_bfloat16 kv_new[2][D];
   bool waited = false;
-  for (int i = tid; i < (group + 2) * (kHalf / 4) || !waited; i += kDecAttnThreads) {
+  for (int i = tid; i < (group + 2) * (kHalf / 4) || !waited; i += kThreads) {
     const int head = i / (kHalf / 4), j = (i - head * (kHalf / 4)) * 4;  // heads 0 .. group - 1: q; group: k; group + 1: v
     const bool item = head < group + 2, turned = head <= group;
     float c1[4], s1[4], c2[4], s2[4];
@@ -479,14 +489,13 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
     *reinterpret_cast<uint2*>(dst + j) = pack4(lo);
     *reinterpret_cast<uint2*>(dst + kHalf + j) = pack4(hi);
   }
-  for (int i = tid; i < (16 - group) * D; i += kDecAttnThreads)  // unused rows of the q tile
+  for (int i = tid; i < (16 - group) * D; i += kThreads)  // unused rows of the q tile
     reinterpret_cast<__nv_bfloat16*>(smem + (group + i / D) * kPitch)[i % D] = __float2bfloat16_rn(0.f);
   __syncthreads();
   if (tid < 2 * (D / 8)) {
     const int which = tid / (D / 8), p = tid - which * (D / 8);
     const uint4 piece = *reinterpret_cast<const uint4*>(&kv_new[which][8 * p]);
     if (slot >= 0) *reinterpret_cast<uint4*>((which ? a.v_cache : a.k_cache) + slot * a.Hk * D + (int64_t)kvh * D + 8 * p) = piece;
-    if (new_in_first && ctx > 0) *reinterpret_cast<uint4*>((which ? v_new : k_new) + 16 * p) = piece;
   }
 
   uint32_t qf[D / 16][4];
@@ -500,24 +509,31 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
   for (int d = 0; d < D / 8; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
   const float sc = a.scale * 1.4426950408889634f;  // scores in units of log2(e)
 
-  for (int c0 = 0; c0 < ctx; c0 += kChunk) {
-    const int n = min(ctx - c0, kChunk);
-    if (c0 > 0) {
-      __syncthreads();  // the previous chunk has been read
-      load_chunk(c0, n);
-      if (n_old >= c0 && n_old < c0 + n && tid < 2 * (D / 8)) {
-        const int which = tid / (D / 8), p = tid - which * (D / 8);
-        *reinterpret_cast<uint4*>((which ? v_new : k_new) + 16 * p) = *reinterpret_cast<const uint4*>(&kv_new[which][8 * p]);
-      }
+  auto put_new = [&](int b, int which, uint32_t slot) {  // the new token's row
+    if (n_old >> 4 == b && lane < D / 8)
+      sts128(slot + (uint32_t)((n_old & 15) * kPitch + 16 * lane), *reinterpret_cast<const uint4*>(&kv_new[which][8 * lane]));
+  };
+  uint32_t here = kv_u32;  // the slot of the item at hand
+  auto advance = [&]() {
+    here += kItem;
+    if (here == kv_u32 + kSlots * kItem) here = kv_u32;
+  };
+  for (int j = 0, b = warp; b < n_blocks; ++j, b += kWarps) {
+    cp_async_wait_group<kSlots - 1>();
+    const uint32_t k_st = here;
+    if (kTurn) {
+      put_new(b, 0, k_st);
+    } else if (n_old >> 4 == b && lane < 2 * (D / 8)) {
+      const int which = lane / (D / 8), p = lane - which * (D / 8);
+      sts128(k_st + (uint32_t)(which * kRows + (n_old & 15) * kPitch + 16 * p), *reinterpret_cast<const uint4*>(&kv_new[which][8 * p]));
     }
-    cp_async_wait_all();
-    __syncthreads();
-    for (int b = warp * 16; b < n; b += kDecAttnWarps * 16) {
+    __syncwarp();
+    {
       float s[2][4];
 #pragma unroll
       for (int h = 0; h < 2; ++h) s[h][0] = s[h][1] = s[h][2] = s[h][3] = 0.f;
       // matrices: tokens 0-7 / dims 0-7, tokens 0-7 / dims 8-15, tokens 8-15 / dims 0-7, tokens 8-15 / dims 8-15
-      const uint32_t ka = k_u32 + (uint32_t)((b + (lane & 7) + ((lane >> 4) << 3)) * kPitch + ((lane >> 3) & 1) * 16);
+      const uint32_t ka = k_st + (uint32_t)(((lane & 7) + ((lane >> 4) << 3)) * kPitch + ((lane >> 3) & 1) * 16);
 #pragma unroll
       for (int k = 0; k < D / 16; ++k) {
         uint32_t kf[4];
@@ -525,12 +541,17 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
         mma_bf16_16816(s[0], qf[k][0], qf[k][1], qf[k][2], qf[k][3], kf[0], kf[1]);
         mma_bf16_16816(s[1], qf[k][0], qf[k][1], qf[k][2], qf[k][3], kf[2], kf[3]);
       }
+      if (kTurn) {
+        __syncwarp();  // every lane has read the slot: V of the next block goes there
+        load_item(j + 1, 1, here, at);
+        advance();
+      }
       float mx[2] = {m[0], m[1]};
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const bool live = b + 8 * h + 2 * t + (e & 1) < n;
+          const bool live = 16 * b + 8 * h + 2 * t + (e & 1) < ctx;
           s[h][e] = live ? s[h][e] * sc : -INFINITY;
           mx[e >> 1] = fmaxf(mx[e >> 1], s[h][e]);
         }
@@ -553,7 +574,12 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
         }
       const uint32_t p0 = pack_bf16x2(s[0][0], s[0][1]), p1 = pack_bf16x2(s[0][2], s[0][3]);
       const uint32_t p2 = pack_bf16x2(s[1][0], s[1][1]), p3 = pack_bf16x2(s[1][2], s[1][3]);
-      const uint32_t va = v_u32 + (uint32_t)((b + (lane & 15)) * kPitch + (lane >> 4) * 16);
+      if (kTurn) {
+        cp_async_wait_group<kSlots - 1>();
+        put_new(b, 1, here);
+        __syncwarp();
+      }
+      const uint32_t va = (kTurn ? here : k_st + kRows) + (uint32_t)((lane & 15) * kPitch + (lane >> 4) * 16);
 #pragma unroll
       for (int d = 0; d < D / 16; ++d) {
         uint32_t vf[4];
@@ -562,16 +588,20 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
         mma_bf16_16816(o[2 * d + 1], p0, p1, p2, p3, vf[2], vf[3]);
       }
     }
+    __syncwarp();
+    if (kTurn) load_item(j + 2, 0, here, at = rows_of(j + 2));
+    else load_item(j + kSlots, 2, here, rows_of(j + kSlots));
+    advance();
   }
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     l[q] += __shfl_xor_sync(0xffffffffu, l[q], 1);
     l[q] += __shfl_xor_sync(0xffffffffu, l[q], 2);
   }
-  // ---- merge the warps: [warp][head][D] sums, then m and l
+  // ---- merge the warps: [warp][head][D] sums, then m and l (every warp has waited for the copies of its blocks)
   __syncthreads();
   float* acc = reinterpret_cast<float*>(smem + 16 * kPitch);
-  float* ml = acc + kDecAttnWarps * 16 * D;
+  float* ml = acc + kWarps * 16 * D;
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     const int head = g + 8 * q;
@@ -583,14 +613,14 @@ __global__ void __launch_bounds__(kDecAttnThreads) decode_attention_kernel(const
     }
   }
   __syncthreads();
-  for (int i = tid; i < group * D / 2; i += kDecAttnThreads) {
+  for (int i = tid; i < group * D / 2; i += kThreads) {
     const int head = i / (D / 2), d = (i - head * (D / 2)) * 2;
     float top = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < kDecAttnWarps; ++w) top = fmaxf(top, ml[(w * 16 + head) * 2]);
+    for (int w = 0; w < kWarps; ++w) top = fmaxf(top, ml[(w * 16 + head) * 2]);
     float total = 0.f, x = 0.f, y = 0.f;
 #pragma unroll
-    for (int w = 0; w < kDecAttnWarps; ++w) {
+    for (int w = 0; w < kWarps; ++w) {
       const float mw = ml[(w * 16 + head) * 2];
       const float f = mw == -INFINITY ? 0.f : exp2f(mw - top);
       const float2 v = *reinterpret_cast<const float2*>(acc + (w * 16 + head) * D + d);
@@ -610,7 +640,7 @@ inline int decode_attention_launch(const DecAttnArgs& a, int D, cudaStream_t str
   {                                                                                                                                 \
     const cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_attn_smem<DIM>()); \
     if (e != cudaSuccess) return fail(B200_LORA_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));                          \
-    return launch_dependent(decode_attention_kernel<DIM>, "decode_attention_kernel", grid, kDecAttnThreads, dec_attn_smem<DIM>(), stream, a); \
+    return launch_dependent(decode_attention_kernel<DIM>, "decode_attention_kernel", grid, kDecAttnWarps * 32, dec_attn_smem<DIM>(), stream, a); \
   }
   if (D == 64) B200_DEC_ATTN(64)
   B200_DEC_ATTN(128)
