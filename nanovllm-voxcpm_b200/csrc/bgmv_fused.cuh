@@ -854,30 +854,48 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   const int Q = st.n * b.r_max;
   int C = bgmv_options().cluster;
   if (C != 1 && C != 2 && C != 4 && C != 8) {
-    // Buckets expected to hold rows: graph buffers carry one bucket per slot, most of them empty, and a bucket
-    // without rows exits at once. With T rows dealt over nb buckets about nb * (1 - exp(-T / nb)) are in use.
-    // 4 CTAs per bucket while two consecutive launches fit side by side (296 CTAs are resident at two per SM), then
-    // 2, then 1. Measured on a 24-layer decoder step of 64 rows over 129 buckets (about 30 in use): 2.13 ms per step
-    // with clusters of 4, 2.27 with 2, 2.42 with 1, 2.46 with 8; on 256 rows over 33 buckets 4.9 us per launch with
-    // 4, 7.0 with 2, 6.8 with 8.
+    // Buckets expected to hold rows: graph buffers carry one bucket per slot, most of them empty. With T rows dealt over nb buckets
+    // about nb * (1 - exp(-T / nb)) are in use; a skewed popularity uses fewer and gives them more windows, which the host does not
+    // see.
     const double nb = (double)b.n_buckets;
     const double in_use = nb * (1.0 - std::exp(-(double)std::max(b.T, 1) / nb));
-    // Other CTAs in the launch (decode_step.cuh's GEMM) leave fewer places: 128 of them beside 50 buckets in use, 1024-wide,
-    // rank 32: 442 us a step with 2, 500 with 4, 548 with 1; beside 16 buckets of 100 rows 383 with 2, 368 with 4.
-    const double resident = 2.0 * 148 - b.beside, half = 0.38 * resident;
-    C = in_use * 2 <= half ? 4 : (in_use <= half ? 2 : 1);
-    // A CTA streams its share of the slabs at 25 - 30 GB/s (loads, multiplication and exchange take turns): large adapters
-    // want more CTAs, as far as those are resident together or their streams are long. Measured, us per projection with
-    // clusters of 4 / 8: one row of 4096-wide layers, rank 64: 23.1 / 9.8; 64 rows over 32 adapters of 2048-wide layers, rank
-    // 64: 15.3 / 9.3; gate_up of 200 rows over 20 adapters, 2048-wide, rank 32 (262 KB a CTA at 4): 11.0 / 8.0, its o (66 KB):
-    // 4.0 / 4.5; gate_up of 384 rows over 64 adapters, 1024-wide, rank 32, with 2 / 4: 15.2 / 12.3; above about 300 CTAs
-    // only streams of more than 512 KB gain: 32-head decoder, 512 rows over 175 adapters, 4 layers: 20.8 ms a step with one
-    // CTA per bucket, 19.7 with 2, 19.0 with 4.
     int64_t bucket_bytes = 0;
     for (int s = 0; s < st.n; ++s) bucket_bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + st.out[s]);
-    while (C < 4 && (bucket_bytes / C > 512 * 1024 || (bucket_bytes / C > 256 * 1024 && in_use * C * 2 <= resident))) C *= 2;
-    const double clusters = in_use + (b.T - 1) / kBgmvTok;
-    if (C == 4 && ((bucket_bytes / 4 > 128 * 1024 && clusters * 8 <= resident && b.beside == 0) || (bucket_bytes / 4 >= 256 * 1024 && in_use * 8 <= resident))) C = 8;
+    const double kb = (double)bucket_bytes / 1024.0 * std::max(1.0, 32.0 / b.r_max);  // (16 rank rows take as long as 32)
+    if (b.mode == 1 || b.mode == 2) {
+      // A shrink or an expand alone, which take turns: 4 CTAs per bucket while two launches fit side by side (296 CTAs are resident
+      // at two per SM), then 2, then 1; more for large adapters, as far as those are resident together or their streams are long.
+      // 1024-wide, rank 16, 8 rows, gate_up's expand with 4 / 8: 5.0 / 3.2 us; rank 32, 200 rows over 32, the four pairs of a layer
+      // with 4 everywhere 18.1, with 8 for gate_up's expand (8.4 / 6.8 us by itself) 18.5.
+      const double resident = 2.0 * 148, half = 0.38 * resident, clusters = in_use + (b.T - 1) / kBgmvTok;
+      C = in_use * 2 <= half ? 4 : (in_use <= half ? 2 : 1);
+      while (C < 4 && (kb / C > 512 || (kb / C > 256 && in_use * C * 2 <= resident))) C *= 2;
+      if (C == 4 && ((kb / 4 > 128 && clusters * 8 <= resident) || (kb / 4 >= 256 && in_use * 8 <= resident))) C = 8;
+    } else {
+      // The least of what it costs, in units of the time in which a CTA takes 1 KB of adapters (about 15 ns): its share of an adapter;
+      // the CTAs beyond those that are resident (296 at two per SM, of which the CTAs of another kind
+      // in the launch hold their places longer), 25 ns each, clusters without rows at a quarter; the exchange, which grows with the
+      // cluster; and the K split of the shrink where eight CTAs are too many for it. us a launch with clusters of 1 / 2 / 4 / 8:
+      //   adds: 1024-wide, rank 16, 32 rows over 8 adapters, gate_up 18.5 / 10.0 / 5.9 / 4.1; rank 32, 64 rows over 32, o 3.8 / 2.9 /
+      //   2.9 / 4.2, 128 over 128 of skewed popularity, gate_up 20.5 / 11.2 / 9.5 / 15.4; 2048-wide, rank 32, 4 rows, down 14.9 / 7.6 /
+      //   5.5 / 4.1, 384 rows over 32 of skewed popularity, gate_up 28.8 / 22.0 / 12.3 / 16.4, 384 over 128, o 10.4 / 6.9 / 11.0 / 17.3;
+      //   4096-wide, rank 32, 4 rows, gate_up - / - / 15.7 / 8.0, 384 rows over 32, qkv 23.3 / 23.3 / 13.4 / 20.6.
+      //   beside a GEMM (with the launch of the consumer): 1024-wide, rank 32, 64 rows over 64 adapters, qkv 11.4 / 11.4 / 16 / 26, o 6.7 /
+      //   6.1 / 10 / 18, gate_up 22 / 14.8 / 18 / 24, down 13 / 9.5 / 14 / 25; 32 rows over 128, gate_up 20 / 11.9 / 10.3 / 13.8; 8 rows,
+      //   qkv 8.7 / 8.7 / 7.9 / 7.1, gate_up 18 / 10.2 / 7.7 / 7.2; 2048-wide, 64 rows over 128, gate_up 34 / 26 / 19.8 / 26.7.
+      // Against the lines before (56 and 112 buckets in use, fewer with a GEMM beside, and 128 to 512 KB a CTA): 230 layers of adds -2 %
+      // (-20 to +3, two of even popularity and rank 64 +7 and +10), 100 layers of decode steps -2 % (-28 to +2, one +5).
+      const int in_use_most = std::min(b.n_buckets, std::max(b.T, 1));
+      const int launched = std::min(in_use_most < b.n_buckets ? in_use_most + (b.T - in_use_most) / kBgmvTok : 65535, b.n_buckets + (b.T - 1) / kBgmvTok);
+      const double clusters = 0.75 * in_use + 0.25 * launched + (b.T - 1) / (2.0 * kBgmvTok);
+      const int kparts = ceil_div_i(b.in_dim, kBgmvKP);
+      double least = 0.0;
+      for (int c = 1; c <= 8; c *= 2) {
+        double cost = kb / c + 2.0 * std::max(0.0, b.beside + c * clusters - (b.beside > 0 ? 200.0 : 290.0)) + 14.0 * c;
+        if (c == 8 && kparts >= 4 && kparts < 8 && st.n * b.r_max <= kBgmvMaxRc) cost += 20.0;
+        if (c == 1 || cost < least) { least = cost; C = c; }
+      }
+    }
   }
   // K split: at least one K part (1024 columns) per CTA of the cluster and all rank rows in one CTA, up to 20 KB of received
   // partial sums (64 rank rows over 8 CTAs, 35 KB: one layer of 4096, rank 64, 1 / 16 rows 45 / 60 us, with the row split
