@@ -52,6 +52,25 @@ def test_fused_decode_kernel_wide_ranks(r, cluster):
     assert_lora_close(y, O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets), max_abs=6e-2, what=f"r{r}")
 
 
+@pytest.mark.parametrize("T, in_dim, outs, S, r", [
+    (4, 6144, [2048], 8, 32),           # eight CTAs although they lose the K split of six parts
+    (4, 4096, [1024], 8, 32),           # four, with the K split of four parts
+    (37, 1024, [4096, 4096], 16, 16),   # eight, 16 rank rows
+    (64, 1024, [1024], 48, 32),         # four and two, by the clusters that fit
+    (90, 1024, [1024], 100, 32),
+    (384, 1024, [1024], 128, 32),       # one
+])
+def test_fused_decode_kernel_with_the_cluster_it_chooses(T, in_dim, outs, S, r):
+    p = W.make_projection(900 + T, T, in_dim, outs, S, r)
+    d = p.to_device(DEV)
+    y = d.y.clone()
+    LORA.launch_add(y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata_for(p.token_to_slot, "graph", S), 1.0,
+                    impl=N.IMPL_BGMV)
+    torch.cuda.synchronize()
+    assert N.device_status(reset=True) == 0
+    assert_lora_close(y, O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets), what=f"{T} {in_dim} {outs}")
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
 @pytest.mark.parametrize("impl", [N.IMPL_GROUPED, N.IMPL_BGMV], ids=["grouped", "bgmv"])
 @pytest.mark.parametrize("case", range(len(CASES)))

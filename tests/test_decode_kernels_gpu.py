@@ -88,6 +88,9 @@ ATTENTION = [
     (16, 1, 64, 1, False, torch.bfloat16, [5, 300]),
     (8, 2, 128, 5, True, torch.float32, [1, 16, 191, 192, 193, 384, 385, 500]),
     (32, 8, 128, 3, False, torch.float32, [64, 1000]),
+    # a warp's blocks of 16 tokens: the first and last of a round of eight warps, of the three slots of a warp, one token more
+    (16, 2, 64, 9, False, torch.float32, [111, 112, 113, 127, 128, 383, 384, 385, 400, 513]),
+    (16, 2, 128, 9, False, torch.float32, [111, 113, 128, 130, 255, 256, 257, 400]),
 ]
 
 
