@@ -891,7 +891,10 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
       const int kparts = ceil_div_i(b.in_dim, kBgmvKP);
       double least = 0.0;
       for (int c = 1; c <= 8; c *= 2) {
-        double cost = kb / c + 2.0 * std::max(0.0, b.beside + c * clusters - (b.beside > 0 ? 200.0 : 290.0)) + 14.0 * c;
+        // (fewer rows than buckets: eight CTAs of a cluster without rows count in full; 39 rows over 107 adapters of rank 16, 1024-wide, a
+        // layer 19.9 with 4 for gate_up, 23.0 with 8)
+        const double these = c == 8 && in_use_most < b.n_buckets ? std::max(clusters, launched + (b.T - 1) / (2.0 * kBgmvTok)) : clusters;
+        double cost = kb / c + 2.0 * std::max(0.0, b.beside + c * these - (b.beside > 0 ? 200.0 : 290.0)) + 14.0 * c;
         if (c == 8 && kparts >= 4 && kparts < 8 && st.n * b.r_max <= kBgmvMaxRc) cost += 20.0;
         if (c == 1 || cost < least) { least = cost; C = c; }
       }
