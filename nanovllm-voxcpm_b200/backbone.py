@@ -188,13 +188,12 @@ class Decoder(nn.Module):
     def _decode_chain_ok(self, embeds, positions, step: AttentionStep) -> bool:
         """Whether this step can run as the short decode chain (``csrc/decode_step.cuh``): a bf16 decode batch of at most 128
         rows on one GPU, adapters (if any) on every output of every projection, and a block table of at most 4096 tokens
-        (the contexts themselves are on the device). One CTA per request and kv head walks its context in chunks without
-        overlap, which flash_attn's split of the context beats from some length on; the rest of the chain pays for it up to
-        there. us per layer of a step, chain / layer by layer, contexts of 1500, 4000 and 8000 tokens: 1024-wide (2 kv
-        heads of 64) one row 38 / 82, 58 / 85, 92 / 89; 32 rows 48 / 84, 75 / 93, 119 / 109; 64 rows 53 / 87, 81 / 107.
-        2048-wide (2 of 128) one row 60 / 113, 97 / 118, 158 / 126; 64 rows 77 / 126, 121 / 161. 4096-wide (8 of 128) one row
-        115 / 195, 152 / 203, 214 / 207; 32 rows 175 / 234, 255 / 300, 390 / 407; 64 rows 236 / 273, 400 / 401; 128 rows
-        of 1500 341 / 349."""
+        (the contexts themselves are on the device). One CTA per request and kv head walks its context, which flash_attn's
+        split of the context beats from some length on; the rest of the chain pays for it up to there. us per layer of a step,
+        chain / layer by layer, 32 rank-32 adapters, contexts of 1500, 4000 and 8000 tokens: 1024-wide (2 kv heads of 64) one row
+        32 / 81, 47 / 84, 69 / 87; 32 rows 61 / 90, 83 / 98, 117 / 113; 64 rows 62 / 91, 83 / 109, 115 / 137. 2048-wide (2 of
+        128) one row 57 / 113, 85 / 119, 129 / 127; 64 rows 82 / 129, 111 / 163, 155 / 218. 4096-wide (8 of 128) one row 114 /
+        194, 142 / 204, 187 / 207; 32 rows 191 / 241, 246 / 308, 334 / 414; 64 rows 232 / 277, 344 / 411."""
         cfg, T = self.cfg, embeds.size(0)
         if step.is_prefill or not 1 <= T <= 128 or not embeds.is_cuda:
             return False

@@ -13,7 +13,7 @@ from nanovllm_voxcpm_b200.context import reset_lora_context, set_lora_context
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
-# rows, q heads, kv heads, head dim, hidden, intermediate, rank, longest context (chunks hold 368 / 192 tokens)
+# rows, q heads, kv heads, head dim, hidden, intermediate, rank, longest context (a warp takes blocks of 16 tokens, eight warps in turn)
 CASES = [
     (1, 16, 2, 64, 1024, 4096, 32, 40),
     (17, 16, 2, 64, 1024, 4096, 16, 800),

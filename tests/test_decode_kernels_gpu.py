@@ -81,7 +81,7 @@ def test_decode_linear_planes(case, with_lora):
     assert not planes[n - 1][none.to(DEV)].any(), "rows without adapter must have a zero delta"
 
 
-# heads, kv heads, head dim, planes, rotation table of the full or half width, its type, contexts (chunks hold 368 / 192 tokens)
+# heads, kv heads, head dim, planes, rotation table of the full or half width, its type, contexts (a warp takes blocks of 16 tokens, eight warps in turn)
 ATTENTION = [
     (16, 2, 64, 9, False, torch.float32, [1, 2, 15, 16, 17, 129, 367, 368, 369, 800]),
     (4, 4, 64, 2, True, torch.bfloat16, [40, 736, 737]),
