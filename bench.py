@@ -745,10 +745,10 @@ def run_prefill_arm(args, emit=True):
     else:
         ach = bytes_step / (ms_per_step * 1e-3) / 1e9
         line.update({"metric": "multi-LoRA linear GB/s (prefill SGMV, algorithmic bytes)", "value": ach, "unit": "GB/s",
-                     "gpu_launches": 2 * len(names) * args.steps,
+                     "gpu_launches": len(names) * args.steps,
                      "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak,
                                   "traffic": None, "peak_kind": f"of {kind}",
-                                  "kernel": "sgmv_shrink_kernel + tc_tile_kernel",
+                                  "kernel": "prefill_cluster_kernel",
                                   "algorithmic_bytes_per_step": bytes_step},
                      "lora_tflops": lora_flops / (ms_per_step * 1e-3) / 1e12})
     if emit:
