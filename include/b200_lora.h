@@ -161,6 +161,10 @@ size_t lora_b200_workspace_bytes(int32_t T, int32_t n_slices, int32_t r_max);
 /* What B200_LORA_IMPL_GROUPED takes of it for one projection and its number of buckets (0 for ranks that it does not run).
  * With less, B200_LORA_IMPL_AUTO takes the fused decode kernel. No counterpart in the reference. */
 size_t lora_b200_grouped_workspace_bytes(int32_t T, int32_t in_dim, int32_t n_slices, int32_t r_max, int32_t n_buckets);
+/* CTAs per cluster with which B200_LORA_IMPL_BGMV runs an add of aligned operands (beside_gemm = 0) or lora_b200_decode_linear its
+ * delta (1); 0: it does not take the problem. Host code, for tests and tuning. No counterpart in the reference. */
+int32_t lora_b200_bucket_cluster(int32_t T, int32_t in_dim, int32_t n_slices, const int32_t* out_sizes, int32_t r_max, int32_t n_buckets,
+                                 int32_t dtype, int32_t beside_gemm);
 
 /*
  * out[s, t, 0:r_max] = scaling * x[t] . A_s[slot_t]^T for slot_t >= 0, and 0 for

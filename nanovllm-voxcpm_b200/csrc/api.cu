@@ -226,7 +226,7 @@ static int decode_linear_problem(BgmvProblem* bp, float* planes, const void* x, 
   bp->rank_per_slot = rank_per_slot; bp->scale_per_slot = nullptr;
   bp->sorted_idx = sorted_idx; bp->slot_ids = slot_ids; bp->counts = counts; bp->offsets = offsets; bp->n_buckets = n_buckets;
   bp->scaling = 1.0f; bp->mode = 4; bp->kind = r_max % 32 != 0 ? 1 : 0; bp->token_to_slot = token_to_slot;
-  bp->beside = std::min(ceil_div_i(out_total, 128) * parts, 148);
+  bp->beside = decode_gemm_ctas(in_dim, out_total);
   if (S < 1 || r_max < 1) return fail(B200_LORA_EINVAL, "decode_linear: bad sizes S=%d r_max=%d", S, r_max);
   if (sorted_idx == nullptr || slot_ids == nullptr || counts == nullptr || offsets == nullptr)
     return fail(B200_LORA_EINVAL, "decode_linear: needs the bucket arrays");
@@ -407,6 +407,27 @@ size_t lora_b200_grouped_workspace_bytes(int32_t T, int32_t in_dim, int32_t n_sl
   for (int s = 0; s < n_slices; ++s) b.st.out[s] = 8;
   int parts;
   return grouped_need(b, &parts);
+}
+
+int32_t lora_b200_bucket_cluster(int32_t T, int32_t in_dim, int32_t n_slices, const int32_t* out_sizes, int32_t r_max, int32_t n_buckets,
+                                 int32_t dtype, int32_t beside_gemm) {
+  if (T < 1 || in_dim < 1 || r_max < 1 || out_sizes == nullptr || n_slices < 1 || n_slices > B200_LORA_MAX_SLICES ||
+      (dtype != B200_LORA_BF16 && dtype != B200_LORA_F16))
+    return 0;
+  void* const some = reinterpret_cast<void*>(uintptr_t(256));  // (stands for the arrays of a call; not read)
+  BgmvProblem b = {};
+  int out_total = 0;
+  b.st.n = n_slices;
+  for (int s = 0; s < n_slices; ++s) {
+    if (out_sizes[s] < 0) return 0;
+    b.st.a[s] = b.st.b[s] = some; b.st.out[s] = out_sizes[s]; b.st.col[s] = out_total;
+    out_total += out_sizes[s];
+  }
+  b.y = some; b.y_ld = out_total; b.x = some; b.x_ld = in_dim; b.T = T; b.in_dim = in_dim; b.S = 1; b.r_max = r_max; b.n_buckets = n_buckets;
+  b.kind = dtype == B200_LORA_F16 ? 2 : (r_max % 32 != 0 ? 1 : 0);
+  if (beside_gemm) { b.mode = 4; b.beside = decode_gemm_ctas(in_dim, out_total); }
+  BgmvParams p;
+  return bgmv_plan(b, &p, nullptr) ? 1 << p.c_shift : 0;
 }
 
 int lora_b200_shrink_allreduce_expand(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,

@@ -822,84 +822,61 @@ inline bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr
 inline int floor_pow2(int v) { int r = 1; while (r * 2 <= v) r *= 2; return r; }
 inline int log2_exact(int v) { int s = 0; while ((1 << s) < v) ++s; return s; }
 
-// Fills `pp` with the tiling for this problem; returns false (and a reason) when
-// the fused kernel cannot run it.
-inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
-  const char* dummy;
-  if (why == nullptr) why = &dummy;
-  SliceTable st;
-  st.n = 0;
-  for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) { st.a[s] = st.b[s] = nullptr; st.out[s] = st.col[s] = 0; }
-  for (int s = 0; s < b.st.n; ++s) {
-    if (b.st.out[s] == 0) continue;
-    st.a[st.n] = b.st.a[s]; st.b[st.n] = b.st.b[s]; st.out[st.n] = b.st.out[s]; st.col[st.n] = b.st.col[s];
-    ++st.n;
-  }
-  if (st.n == 0) { *why = "no active slice"; return false; }
-  if (b.r_max % (b.kind != 0 ? 16 : 32) != 0 || b.r_max > 256) {
-    *why = b.kind != 0 ? "r_max must be a multiple of 16, <= 256" : "r_max must be a multiple of 32, <= 256";
-    return false;
-  }
-  if (b.kind != 0 && b.mode == 3) { *why = "overwrite mode is for bf16 with r_max a multiple of 32"; return false; }
-  if (b.kind == 2 && b.mode == 4) { *why = "the fp32 form is for bf16"; return false; }
-  if (b.in_dim % 32 != 0) { *why = "in_dim must be a multiple of 32"; return false; }
-  if (b.x_ld % 8 != 0 || b.y_ld % 8 != 0) { *why = "row strides must be multiples of 8 elements"; return false; }
-  if (!aligned16(b.x) || !aligned16(b.y)) { *why = "x / y must be 16-byte aligned"; return false; }
-  for (int s = 0; s < st.n; ++s) {
-    if (st.out[s] % 8 != 0 || st.col[s] % 8 != 0) { *why = "slice widths / offsets must be multiples of 8"; return false; }
-    if (!aligned16(st.a[s]) || !aligned16(st.b[s])) { *why = "slabs must be 16-byte aligned"; return false; }
-  }
-  if (b.n_buckets < 1 || b.n_buckets + b.T / kBgmvTok > 65535) { *why = "n_buckets outside [1, 65535]"; return false; }
-
-  const int Q = st.n * b.r_max;
-  int C = bgmv_options().cluster;
-  if (C != 1 && C != 2 && C != 4 && C != 8) {
-    // Buckets expected to hold rows: graph buffers carry one bucket per slot, most of them empty. With T rows dealt over nb buckets
-    // about nb * (1 - exp(-T / nb)) are in use; a skewed popularity uses fewer and gives them more windows, which the host does not
-    // see.
-    const double nb = (double)b.n_buckets;
-    const double in_use = nb * (1.0 - std::exp(-(double)std::max(b.T, 1) / nb));
-    int64_t bucket_bytes = 0;
-    for (int s = 0; s < st.n; ++s) bucket_bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + st.out[s]);
-    const double kb = (double)bucket_bytes / 1024.0 * std::max(1.0, 32.0 / b.r_max);  // (16 rank rows take as long as 32)
-    if (b.mode == 1 || b.mode == 2) {
-      // A shrink or an expand alone, which take turns: 4 CTAs per bucket while two launches fit side by side (296 CTAs are resident
-      // at two per SM), then 2, then 1; more for large adapters, as far as those are resident together or their streams are long.
-      // 1024-wide, rank 16, 8 rows, gate_up's expand with 4 / 8: 5.0 / 3.2 us; rank 32, 200 rows over 32, the four pairs of a layer
-      // with 4 everywhere 18.1, with 8 for gate_up's expand (8.4 / 6.8 us by itself) 18.5.
-      const double resident = 2.0 * 148, half = 0.38 * resident, clusters = in_use + (b.T - 1) / kBgmvTok;
-      C = in_use * 2 <= half ? 4 : (in_use <= half ? 2 : 1);
-      while (C < 4 && (kb / C > 512 || (kb / C > 256 && in_use * C * 2 <= resident))) C *= 2;
-      if (C == 4 && ((kb / 4 > 128 && clusters * 8 <= resident) || (kb / 4 >= 256 && in_use * 8 <= resident))) C = 8;
-    } else {
-      // The least of what it costs, in units of the time in which a CTA takes 1 KB of adapters (about 15 ns): its share of an adapter;
-      // the CTAs beyond those that are resident (296 at two per SM, of which the CTAs of another kind
-      // in the launch hold their places longer), 25 ns each, clusters without rows at a quarter; the exchange, which grows with the
-      // cluster; and the K split of the shrink where eight CTAs are too many for it. us a launch with clusters of 1 / 2 / 4 / 8:
-      //   adds: 1024-wide, rank 16, 32 rows over 8 adapters, gate_up 18.5 / 10.0 / 5.9 / 4.1; rank 32, 64 rows over 32, o 3.8 / 2.9 /
-      //   2.9 / 4.2, 128 over 128 of skewed popularity, gate_up 20.5 / 11.2 / 9.5 / 15.4; 2048-wide, rank 32, 4 rows, down 14.9 / 7.6 /
-      //   5.5 / 4.1, 384 rows over 32 of skewed popularity, gate_up 28.8 / 22.0 / 12.3 / 16.4, 384 over 128, o 10.4 / 6.9 / 11.0 / 17.3;
-      //   4096-wide, rank 32, 4 rows, gate_up - / - / 15.7 / 8.0, 384 rows over 32, qkv 23.3 / 23.3 / 13.4 / 20.6.
-      //   beside a GEMM (with the launch of the consumer): 1024-wide, rank 32, 64 rows over 64 adapters, qkv 11.4 / 11.4 / 16 / 26, o 6.7 /
-      //   6.1 / 10 / 18, gate_up 22 / 14.8 / 18 / 24, down 13 / 9.5 / 14 / 25; 32 rows over 128, gate_up 20 / 11.9 / 10.3 / 13.8; 8 rows,
-      //   qkv 8.7 / 8.7 / 7.9 / 7.1, gate_up 18 / 10.2 / 7.7 / 7.2; 2048-wide, 64 rows over 128, gate_up 34 / 26 / 19.8 / 26.7.
-      // Against the lines before (56 and 112 buckets in use, fewer with a GEMM beside, and 128 to 512 KB a CTA): 230 layers of adds -2 %
-      // (-20 to +3, two of even popularity and rank 64 +7 and +10), 100 layers of decode steps -2 % (-28 to +2, one +5).
-      const int in_use_most = std::min(b.n_buckets, std::max(b.T, 1));
-      const int launched = std::min(in_use_most < b.n_buckets ? in_use_most + (b.T - in_use_most) / kBgmvTok : 65535, b.n_buckets + (b.T - 1) / kBgmvTok);
-      const double clusters = 0.75 * in_use + 0.25 * launched + (b.T - 1) / (2.0 * kBgmvTok);
-      const int kparts = ceil_div_i(b.in_dim, kBgmvKP);
-      double least = 0.0;
-      for (int c = 1; c <= 8; c *= 2) {
-        // (fewer rows than buckets: eight CTAs of a cluster without rows count in full; 39 rows over 107 adapters of rank 16, 1024-wide, a
-        // layer 19.9 with 4 for gate_up, 23.0 with 8)
-        const double these = c == 8 && in_use_most < b.n_buckets ? std::max(clusters, launched + (b.T - 1) / (2.0 * kBgmvTok)) : clusters;
-        double cost = kb / c + 2.0 * std::max(0.0, b.beside + c * these - (b.beside > 0 ? 200.0 : 290.0)) + 14.0 * c;
-        if (c == 8 && kparts >= 4 && kparts < 8 && st.n * b.r_max <= kBgmvMaxRc) cost += 20.0;
-        if (c == 1 || cost < least) { least = cost; C = c; }
-      }
+// Cluster size of least cost for the active slices `st` of a problem.
+inline int bgmv_cluster(const BgmvProblem& b, const SliceTable& st) {
+  int C = 1;
+  // Buckets expected to hold rows: graph buffers carry one bucket per slot, most of them empty. With T rows dealt over nb buckets
+  // about nb * (1 - exp(-T / nb)) are in use; a skewed popularity uses fewer and gives them more windows, which the host does not
+  // see.
+  const double nb = (double)b.n_buckets;
+  const double in_use = nb * (1.0 - std::exp(-(double)std::max(b.T, 1) / nb));
+  int64_t bucket_bytes = 0;
+  for (int s = 0; s < st.n; ++s) bucket_bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + st.out[s]);
+  const double kb = (double)bucket_bytes / 1024.0 * std::max(1.0, 32.0 / b.r_max);  // (16 rank rows take as long as 32)
+  if (b.mode == 1 || b.mode == 2) {
+    // A shrink or an expand alone, which take turns: 4 CTAs per bucket while two launches fit side by side (296 CTAs are resident
+    // at two per SM), then 2, then 1; more for large adapters, as far as those are resident together or their streams are long.
+    // 1024-wide, rank 16, 8 rows, gate_up's expand with 4 / 8: 5.0 / 3.2 us; rank 32, 200 rows over 32, the four pairs of a layer
+    // with 4 everywhere 18.1, with 8 for gate_up's expand (8.4 / 6.8 us by itself) 18.5.
+    const double resident = 2.0 * 148, half = 0.38 * resident, clusters = in_use + (b.T - 1) / kBgmvTok;
+    C = in_use * 2 <= half ? 4 : (in_use <= half ? 2 : 1);
+    while (C < 4 && (kb / C > 512 || (kb / C > 256 && in_use * C * 2 <= resident))) C *= 2;
+    if (C == 4 && ((kb / 4 > 128 && clusters * 8 <= resident) || (kb / 4 >= 256 && in_use * 8 <= resident))) C = 8;
+  } else {
+    // The least of what it costs, in units of the time in which a CTA takes 1 KB of adapters (about 15 ns): its share of an adapter;
+    // the CTAs beyond those that are resident (296 at two per SM, of which the CTAs of another kind
+    // in the launch hold their places longer), 25 ns each, clusters without rows at a quarter; the exchange, which grows with the
+    // cluster; and the K split of the shrink where eight CTAs are too many for it. us a launch with clusters of 1 / 2 / 4 / 8:
+    //   adds: 1024-wide, rank 16, 32 rows over 8 adapters, gate_up 18.5 / 10.0 / 5.9 / 4.1; rank 32, 64 rows over 32, o 3.8 / 2.9 /
+    //   2.9 / 4.2, 128 over 128 of skewed popularity, gate_up 20.5 / 11.2 / 9.5 / 15.4; 2048-wide, rank 32, 4 rows, down 14.9 / 7.6 /
+    //   5.5 / 4.1, 384 rows over 32 of skewed popularity, gate_up 28.8 / 22.0 / 12.3 / 16.4, 384 over 128, o 10.4 / 6.9 / 11.0 / 17.3;
+    //   4096-wide, rank 32, 4 rows, gate_up - / - / 15.7 / 8.0, 384 rows over 32, qkv 23.3 / 23.3 / 13.4 / 20.6.
+    //   beside a GEMM (with the launch of the consumer): 1024-wide, rank 32, 64 rows over 64 adapters, qkv 11.4 / 11.4 / 16 / 26, o 6.7 /
+    //   6.1 / 10 / 18, gate_up 22 / 14.8 / 18 / 24, down 13 / 9.5 / 14 / 25; 32 rows over 128, gate_up 20 / 11.9 / 10.3 / 13.8; 8 rows,
+    //   qkv 8.7 / 8.7 / 7.9 / 7.1, gate_up 18 / 10.2 / 7.7 / 7.2; 2048-wide, 64 rows over 128, gate_up 34 / 26 / 19.8 / 26.7.
+    // Against the lines before (56 and 112 buckets in use, fewer with a GEMM beside, and 128 to 512 KB a CTA): 230 layers of adds -2 %
+    // (-20 to +3, two of even popularity and rank 64 +7 and +10), 100 layers of decode steps -2 % (-28 to +2, one +5).
+    const int in_use_most = std::min(b.n_buckets, std::max(b.T, 1));
+    const int launched = std::min(in_use_most < b.n_buckets ? in_use_most + (b.T - in_use_most) / kBgmvTok : 65535, b.n_buckets + (b.T - 1) / kBgmvTok);
+    const double clusters = 0.75 * in_use + 0.25 * launched + (b.T - 1) / (2.0 * kBgmvTok);
+    const int kparts = ceil_div_i(b.in_dim, kBgmvKP);
+    double least = 0.0;
+    for (int c = 1; c <= 8; c *= 2) {
+      // (fewer rows than buckets: eight CTAs of a cluster without rows count in full; 39 rows over 107 adapters of rank 16, 1024-wide, a
+      // layer 19.9 with 4 for gate_up, 23.0 with 8)
+      const double these = c == 8 && in_use_most < b.n_buckets ? std::max(clusters, launched + (b.T - 1) / (2.0 * kBgmvTok)) : clusters;
+      double cost = kb / c + 2.0 * std::max(0.0, b.beside + c * these - (b.beside > 0 ? 200.0 : 290.0)) + 14.0 * c;
+      if (c == 8 && kparts >= 4 && kparts < 8 && st.n * b.r_max <= kBgmvMaxRc) cost += 20.0;
+      if (c == 1 || cost < least) { least = cost; C = c; }
     }
   }
+  return C;
+}
+
+// Tiling of a problem with the active slices `st` for clusters of C CTAs (more where the rank rows need them); false (and a
+// reason) when it does not fit a CTA.
+inline bool bgmv_plan_cluster(const BgmvProblem& b, const SliceTable& st, int C, BgmvParams* pp, const char** why) {
+  const int Q = st.n * b.r_max;
   // K split: at least one K part (1024 columns) per CTA of the cluster and all rank rows in one CTA, up to 20 KB of received
   // partial sums (64 rank rows over 8 CTAs, 35 KB: one layer of 4096, rank 64, 1 / 16 rows 45 / 60 us, with the row split
   // 40 / 53); the shrink-only / expand-only pair of the tensor-parallel exchange keeps the row split
@@ -978,6 +955,45 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   if (b.mode == 3 && b.token_to_slot == nullptr) { *why = "overwrite mode needs token_to_slot"; return false; }
   if (pp != nullptr) *pp = p;
   return true;
+}
+
+// Fills `pp` with the tiling for this problem; returns false (and a reason) when
+// the fused kernel cannot run it.
+inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
+  const char* dummy;
+  if (why == nullptr) why = &dummy;
+  SliceTable st;
+  st.n = 0;
+  for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) { st.a[s] = st.b[s] = nullptr; st.out[s] = st.col[s] = 0; }
+  for (int s = 0; s < b.st.n; ++s) {
+    if (b.st.out[s] == 0) continue;
+    st.a[st.n] = b.st.a[s]; st.b[st.n] = b.st.b[s]; st.out[st.n] = b.st.out[s]; st.col[st.n] = b.st.col[s];
+    ++st.n;
+  }
+  if (st.n == 0) { *why = "no active slice"; return false; }
+  if (b.r_max % (b.kind != 0 ? 16 : 32) != 0 || b.r_max > 256) {
+    *why = b.kind != 0 ? "r_max must be a multiple of 16, <= 256" : "r_max must be a multiple of 32, <= 256";
+    return false;
+  }
+  if (b.kind != 0 && b.mode == 3) { *why = "overwrite mode is for bf16 with r_max a multiple of 32"; return false; }
+  if (b.kind == 2 && b.mode == 4) { *why = "the fp32 form is for bf16"; return false; }
+  if (b.in_dim % 32 != 0) { *why = "in_dim must be a multiple of 32"; return false; }
+  if (b.x_ld % 8 != 0 || b.y_ld % 8 != 0) { *why = "row strides must be multiples of 8 elements"; return false; }
+  if (!aligned16(b.x) || !aligned16(b.y)) { *why = "x / y must be 16-byte aligned"; return false; }
+  for (int s = 0; s < st.n; ++s) {
+    if (st.out[s] % 8 != 0 || st.col[s] % 8 != 0) { *why = "slice widths / offsets must be multiples of 8"; return false; }
+    if (!aligned16(st.a[s]) || !aligned16(st.b[s])) { *why = "slabs must be 16-byte aligned"; return false; }
+  }
+  if (b.n_buckets < 1 || b.n_buckets + b.T / kBgmvTok > 65535) { *why = "n_buckets outside [1, 65535]"; return false; }
+
+  const int asked = bgmv_options().cluster;
+  if (asked == 1 || asked == 2 || asked == 4 || asked == 8) return bgmv_plan_cluster(b, st, asked, pp, why);
+  // the cheapest cluster whose CTAs can hold their share; a larger one where that one cannot (outputs of more than 256 tiles a CTA:
+  // 65536 columns at rank 96 in clusters of two)
+  for (int C = bgmv_cluster(b, st);; C *= 2) {
+    if (bgmv_plan_cluster(b, st, C, pp, why)) return true;
+    if (C >= 8) return false;
+  }
 }
 
 inline bool bgmv_supported(const BgmvProblem& b, const char** why) { return bgmv_plan(b, nullptr, why); }

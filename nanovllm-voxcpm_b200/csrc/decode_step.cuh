@@ -185,6 +185,8 @@ inline int decode_gemm_parts(int in_dim, int out) {
   while (parts < 8 && tiles * parts * 2 <= 148 && ceil_div_i(steps, 2 * parts) * (2 * parts - 1) < steps) parts *= 2;
   return parts;
 }
+// ... and the CTAs that it counts beside the clusters of the delta (two to an SM)
+inline int decode_gemm_ctas(int in_dim, int out) { return std::min(ceil_div_i(out, 128) * decode_gemm_parts(in_dim, out), 148); }
 
 template <typename... Params, typename... Args>
 inline int launch_dependent(void (*kernel)(Params...), const char* name, dim3 grid, int threads, size_t smem, cudaStream_t stream, Args&&... args) {
