@@ -822,18 +822,31 @@ inline bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr
 inline int floor_pow2(int v) { int r = 1; while (r * 2 <= v) r *= 2; return r; }
 inline int log2_exact(int v) { int s = 0; while ((1 << s) < v) ++s; return s; }
 
-// Cluster size of least cost for the active slices `st` of a problem.
+// How the CTAs of a cluster share the shrink: the rank rows (rc each, all K), or with input rows of at least one K part (1024
+// columns) per CTA and all rank rows in one CTA the K parts, up to 20 KB of received partial sums (64 rank rows over 8 CTAs, 35
+// KB: one layer of 4096, rank 64, 1 / 16 rows 45 / 60 us, with the row split 40 / 53). The shrink-only / expand-only pair keeps
+// the row split. rc = 0: the rank rows are too many for C CTAs.
+struct BgmvSplit { bool by_k; int rc; };
+inline BgmvSplit bgmv_split(const BgmvProblem& b, int Q, int C) {
+  const bool by_k = bgmv_options().ksplit && C > 1 && (b.mode == 0 || b.mode >= 3) && ceil_div_i(b.in_dim, kBgmvKP) >= C && Q <= kBgmvMaxRc &&
+                    C * kBgmvTok * (Q + 4) * 4 <= 20 * 1024;
+  const int rc = by_k ? Q : round_up_i(ceil_div_i(Q, C), 8);
+  return {by_k, rc <= kBgmvMaxRc ? rc : 0};
+}
+
+// Cluster size for the active slices `st` of a problem.
 inline int bgmv_cluster(const BgmvProblem& b, const SliceTable& st) {
   int C = 1;
+  const int Q = st.n * b.r_max;
   // Buckets expected to hold rows: graph buffers carry one bucket per slot, most of them empty. With T rows dealt over nb buckets
   // about nb * (1 - exp(-T / nb)) are in use; a skewed popularity uses fewer and gives them more windows, which the host does not
   // see.
-  const double nb = (double)b.n_buckets;
-  const double in_use = nb * (1.0 - std::exp(-(double)std::max(b.T, 1) / nb));
-  int64_t bucket_bytes = 0;
-  for (int s = 0; s < st.n; ++s) bucket_bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + st.out[s]);
-  const double kb = (double)bucket_bytes / 1024.0 * std::max(1.0, 32.0 / b.r_max);  // (16 rank rows take as long as 32)
+  const double nb = (double)b.n_buckets, rows = (double)std::max(b.T, 1);
+  const double in_use = nb * (1.0 - std::exp(-rows / nb));
   if (b.mode == 1 || b.mode == 2) {
+    int64_t bucket_bytes = 0;
+    for (int s = 0; s < st.n; ++s) bucket_bytes += 2 * (int64_t)b.r_max * ((int64_t)b.in_dim + st.out[s]);
+    const double kb = (double)bucket_bytes / 1024.0 * std::max(1.0, 32.0 / b.r_max);  // (16 rank rows take as long as 32)
     // A shrink or an expand alone, which take turns: 4 CTAs per bucket while two launches fit side by side (296 CTAs are resident
     // at two per SM), then 2, then 1; more for large adapters, as far as those are resident together or their streams are long.
     // 1024-wide, rank 16, 8 rows, gate_up's expand with 4 / 8: 5.0 / 3.2 us; rank 32, 200 rows over 32, the four pairs of a layer
@@ -842,33 +855,39 @@ inline int bgmv_cluster(const BgmvProblem& b, const SliceTable& st) {
     C = in_use * 2 <= half ? 4 : (in_use <= half ? 2 : 1);
     while (C < 4 && (kb / C > 512 || (kb / C > 256 && in_use * C * 2 <= resident))) C *= 2;
     if (C == 4 && ((kb / 4 > 128 && clusters * 8 <= resident) || (kb / 4 >= 256 && in_use * 8 <= resident))) C = 8;
-  } else {
-    // The least of what it costs, in units of the time in which a CTA takes 1 KB of adapters (about 15 ns): its share of an adapter;
-    // the CTAs beyond those that are resident (296 at two per SM, of which the CTAs of another kind
-    // in the launch hold their places longer), 25 ns each, clusters without rows at a quarter; the exchange, which grows with the
-    // cluster; and the K split of the shrink where eight CTAs are too many for it. us a launch with clusters of 1 / 2 / 4 / 8:
-    //   adds: 1024-wide, rank 16, 32 rows over 8 adapters, gate_up 18.5 / 10.0 / 5.9 / 4.1; rank 32, 64 rows over 32, o 3.8 / 2.9 /
-    //   2.9 / 4.2, 128 over 128 of skewed popularity, gate_up 20.5 / 11.2 / 9.5 / 15.4; 2048-wide, rank 32, 4 rows, down 14.9 / 7.6 /
-    //   5.5 / 4.1, 384 rows over 32 of skewed popularity, gate_up 28.8 / 22.0 / 12.3 / 16.4, 384 over 128, o 10.4 / 6.9 / 11.0 / 17.3;
-    //   4096-wide, rank 32, 4 rows, gate_up - / - / 15.7 / 8.0, 384 rows over 32, qkv 23.3 / 23.3 / 13.4 / 20.6.
-    //   beside a GEMM (with the launch of the consumer): 1024-wide, rank 32, 64 rows over 64 adapters, qkv 11.4 / 11.4 / 16 / 26, o 6.7 /
-    //   6.1 / 10 / 18, gate_up 22 / 14.8 / 18 / 24, down 13 / 9.5 / 14 / 25; 32 rows over 128, gate_up 20 / 11.9 / 10.3 / 13.8; 8 rows,
-    //   qkv 8.7 / 8.7 / 7.9 / 7.1, gate_up 18 / 10.2 / 7.7 / 7.2; 2048-wide, 64 rows over 128, gate_up 34 / 26 / 19.8 / 26.7.
-    // Against the lines before (56 and 112 buckets in use, fewer with a GEMM beside, and 128 to 512 KB a CTA): 230 layers of adds -2 %
-    // (-20 to +3, two of even popularity and rank 64 +7 and +10), 100 layers of decode steps -2 % (-28 to +2, one +5).
-    const int in_use_most = std::min(b.n_buckets, std::max(b.T, 1));
-    const int launched = std::min(in_use_most < b.n_buckets ? in_use_most + (b.T - in_use_most) / kBgmvTok : 65535, b.n_buckets + (b.T - 1) / kBgmvTok);
-    const double clusters = 0.75 * in_use + 0.25 * launched + (b.T - 1) / (2.0 * kBgmvTok);
-    const int kparts = ceil_div_i(b.in_dim, kBgmvKP);
-    double least = 0.0;
-    for (int c = 1; c <= 8; c *= 2) {
-      // (fewer rows than buckets: eight CTAs of a cluster without rows count in full; 39 rows over 107 adapters of rank 16, 1024-wide, a
-      // layer 19.9 with 4 for gate_up, 23.0 with 8)
-      const double these = c == 8 && in_use_most < b.n_buckets ? std::max(clusters, launched + (b.T - 1) / (2.0 * kBgmvTok)) : clusters;
-      double cost = kb / c + 2.0 * std::max(0.0, b.beside + c * these - (b.beside > 0 ? 200.0 : 290.0)) + 14.0 * c;
-      if (c == 8 && kparts >= 4 && kparts < 8 && st.n * b.r_max <= kBgmvMaxRc) cost += 20.0;
-      if (c == 1 || cost < least) { least = cost; C = c; }
-    }
+    return C;
+  }
+  // The least of a sum in KB of lora_B that a CTA could take meanwhile: what it takes of lora_B (rows of 16 ranks count as 32; kinds 1
+  // and 2, which multiply two halves of the intermediate and read y, 1.6 times), of lora_A and of x; the CTAs of the launch that
+  // share an SM, and those that wait for a place (the GEMM's CTAs hold theirs longer); the exchange. The factors are a fit, made for
+  // the least loss against the best size of each point, over 6688 measured points: adds (4512) of 1 to 4000 rows over 6 to 900
+  // adapters, even and skewed, graph and eager index arrays, widths 1024 to 4096, ranks 16 to 128, down of 4 to 7 and 14 K
+  // parts, and projections beside their GEMM (2176) of 1 to 128 rows. Mean loss 0.9 % (adds) and 1.2 %, of which 0.4 and 0.6 is
+  // popularity, which the host does not see: the same rows over the same buckets, 2048-wide, rank 64, 48 over 100, take 55.6 us a
+  // layer with clusters of four and 60.2 with the sizes taken (eight, o four) if even, 49.1 and 35.9 if skewed. Sums of shares unrounded by rank rows and K
+  // parts, with a line at 290 CTAs, lost 2.3 and 1.6 %. us a launch with clusters of 1 / 2 / 4 / 8, the size taken in brackets:
+  //   adds: 1024-wide, rank 16, 8 rows over 32 adapters, gate_up 16.3 / 9.1 / 5.4 / [3.8]; rank 32, 64 over 32, o 3.9 / 2.8 / [2.5] / 3.7, 128 over
+  //   128, gate_up 20.2 / [12.8] / 15.1 / 19.5 (of skewed popularity 20.5 / 11.3 / 9.5 / 15.3), 384 over 128, o 5.2 / [5.0] / 8.0 / 16.8; 4 rows, down of 4 K parts 9.5 / 4.9 /
+  //   [3.1] / 3.3, of 5 11.9 / 7.3 / 5.5 / [3.7], of 6 14.9 / 7.7 / 5.5 / [4.1], of 7 16.7 / 9.6 / 5.4 / [4.4], of 6 and 16 rows a bucket 15.4 / 8.0 / [6.1] /
+  //   7.3; 2048-wide, 384 over 32 of skewed popularity, gate_up 28.5 / 21.8 / [12.3] / 16.3; rank 64, 256 over 32, down 35.3 / 24.8 / 16.4 /
+  //   [12.5], of skewed popularity 34.4 / 24.9 / 16.8 / [19.4]; 4096-wide, 4 over 8, gate_up 54 / 30 / 15.8 / [7.8].
+  //   beside a GEMM (with the launch of the consumer): 1024-wide, rank 32, 64 rows over 64 adapters, qkv 11.4 / [11.4] / 15.9 / 26, o 6.7 /
+  //   [6.1] / 9.9 / 17.6, gate_up 22 / [15.0] / 17.9 / 24, down 13.4 / [9.5] / 13.9 / 25; 24 over 128, gate_up 18.7 / 11.7 / [10.6] / 13.9; 8 over 32, qkv
+  //   8.8 / 8.6 / 7.9 / [7.1], gate_up 17.6 / 10.2 / [7.6] / 7.2; 128 over 128, o [8.2] / 11.4 / 17.9 / 36; 2048-wide, 64 over 128, gate_up 35 /
+  //   27.4 / [27.2] / 35.
+  double least = 0.0;
+  const double windows = in_use + 0.9 * std::max(0.0, rows - 1.0 - 2.0 * in_use) / kBgmvTok, rows_each = std::min((double)kBgmvTok, rows / in_use);
+  const int kparts = ceil_div_i(b.in_dim, kBgmvKP);
+  for (int c = 1, any = 0; c <= 8; c *= 2) {
+    const BgmvSplit split = bgmv_split(b, Q, c);
+    if (split.rc == 0) continue;
+    const double columns = split.by_k ? std::min(ceil_div_i(kparts, c) * kBgmvKP, b.in_dim) : b.in_dim;
+    double b_rows = 0.0;
+    for (int s = 0; s < st.n; ++s) b_rows += round_up_i(ceil_div_i(st.out[s], c), 32);
+    const double share = b_rows * 2.0 * std::max(b.r_max, 32) / 1024.0 * (b.kind != 0 ? 1.6 : 1.0) + (1.9 * split.rc + 0.8 * rows_each) * columns * 2.0 / 1024.0;
+    const double ctas = 2.8 * b.beside + c * windows;
+    const double cost = share + 0.75 * std::max(0.0, ctas - 148.0) + 2.25 * std::max(0.0, ctas - 296.0) + 3.8 * c;
+    if (!any || cost < least) { least = cost; C = c; any = 1; }
   }
   return C;
 }
@@ -877,16 +896,11 @@ inline int bgmv_cluster(const BgmvProblem& b, const SliceTable& st) {
 // reason) when it does not fit a CTA.
 inline bool bgmv_plan_cluster(const BgmvProblem& b, const SliceTable& st, int C, BgmvParams* pp, const char** why) {
   const int Q = st.n * b.r_max;
-  // K split: at least one K part (1024 columns) per CTA of the cluster and all rank rows in one CTA, up to 20 KB of received
-  // partial sums (64 rank rows over 8 CTAs, 35 KB: one layer of 4096, rank 64, 1 / 16 rows 45 / 60 us, with the row split
-  // 40 / 53); the shrink-only / expand-only pair of the tensor-parallel exchange keeps the row split
-  const int nkp_all = ceil_div_i(b.in_dim, kBgmvKP);
-  const bool ksplit = bgmv_options().ksplit && C > 1 && (b.mode == 0 || b.mode >= 3) && nkp_all >= C && Q <= kBgmvMaxRc &&
-                      C * kBgmvTok * (Q + 4) * 4 <= 20 * 1024;
-  if (!ksplit)
-    while (C < 8 && round_up_i(ceil_div_i(Q, C), 8) > kBgmvMaxRc) C *= 2;
-  const int Rc = ksplit ? Q : round_up_i(ceil_div_i(Q, C), 8);
-  if (Rc > kBgmvMaxRc) { *why = "n_slices * r_max too large for one cluster"; return false; }
+  BgmvSplit split = bgmv_split(b, Q, C);
+  while (split.rc == 0 && C < 8) split = bgmv_split(b, Q, C *= 2);
+  if (split.rc == 0) { *why = "n_slices * r_max too large for one cluster"; return false; }
+  const bool ksplit = split.by_k;
+  const int Rc = split.rc;
 
   BgmvParams p;
   // (a bucket of n rows has 1 + (n - 1) / 16 windows, the most with as many buckets in use as there are rows)
