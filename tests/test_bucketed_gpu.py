@@ -3,6 +3,7 @@ CPU oracle at the edges of their tiles - one token, 16- and 32-token chunks and 
 tiles, K tails and K parts, every rank, popular buckets, mixed ranks, slots of rank 0 - through ``lora_b200_add`` with the
 kernel asked for by name."""
 
+import ctypes
 from concurrent.futures import ThreadPoolExecutor
 
 import pytest
@@ -52,15 +53,18 @@ def test_fused_decode_kernel_wide_ranks(r, cluster):
     assert_lora_close(y, O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets), max_abs=6e-2, what=f"r{r}")
 
 
-@pytest.mark.parametrize("T, in_dim, outs, S, r", [
-    (4, 6144, [2048], 8, 32),           # eight CTAs although they lose the K split of six parts
-    (4, 4096, [1024], 8, 32),           # four, with the K split of four parts
-    (37, 1024, [4096, 4096], 16, 16),   # eight, 16 rank rows
-    (64, 1024, [1024], 48, 32),         # four and two, by the clusters that fit
-    (90, 1024, [1024], 100, 32),
-    (384, 1024, [1024], 128, 32),       # one
+@pytest.mark.parametrize("T, in_dim, outs, S, r, cluster", [
+    (4, 6144, [2048], 8, 32, 8),           # eight CTAs although they lose the K split of six parts
+    (4, 5120, [1280], 8, 32, 8),           # ... of five
+    (4, 4096, [1024], 8, 32, 4),           # with the K split of four parts
+    (37, 1024, [4096, 4096], 16, 16, 8),   # 16 rank rows
+    (64, 1024, [1024], 48, 32, 4),         # by the clusters that fit
+    (90, 1024, [1024], 100, 32, 2),
+    (256, 1024, [1024], 300, 32, 1),
 ])
-def test_fused_decode_kernel_with_the_cluster_it_chooses(T, in_dim, outs, S, r):
+def test_fused_decode_kernel_with_the_cluster_it_chooses(T, in_dim, outs, S, r, cluster):
+    widths = (ctypes.c_int32 * len(outs))(*outs)
+    assert N.lib().lora_b200_bucket_cluster(T, in_dim, len(outs), widths, r, S + 1, N.DT_BF16, 0) == cluster
     p = W.make_projection(900 + T, T, in_dim, outs, S, r)
     d = p.to_device(DEV)
     y = d.y.clone()
