@@ -199,13 +199,13 @@ int lora_b200_decode_planes(int32_t in_dim, int32_t out) {
   return decode_gemm_parts(in_dim, out) + 1;
 }
 
-// Argument checks of a projection of the decode chain, and the adapters' part of the launch (*bp). Reads no pointer.
-static int decode_linear_problem(BgmvProblem* bp, float* planes, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight,
-                                 int64_t w_ld, int32_t out_total, int32_t n_slices, const void* const* a_slabs,
-                                 const void* const* b_slabs, const int32_t* out_sizes, const int32_t* col_offsets, int32_t S,
-                                 int32_t r_max, const int32_t* rank_per_slot, const int32_t* token_to_slot,
-                                 const int32_t* sorted_idx, const int32_t* slot_ids, const int32_t* counts, const int32_t* offsets,
-                                 int32_t n_buckets) {
+// Argument checks of a projection of the decode chain, and the plan of the adapters' part of the launch. Reads no pointer.
+static int decode_linear_plan(BgmvParams* plan, float* planes, const void* x, int64_t x_ld, int32_t T, int32_t in_dim, const void* weight,
+                              int64_t w_ld, int32_t out_total, int32_t n_slices, const void* const* a_slabs,
+                              const void* const* b_slabs, const int32_t* out_sizes, const int32_t* col_offsets, int32_t S,
+                              int32_t r_max, const int32_t* rank_per_slot, const int32_t* token_to_slot,
+                              const int32_t* sorted_idx, const int32_t* slot_ids, const int32_t* counts, const int32_t* offsets,
+                              int32_t n_buckets) {
   if (T < 1 || T > kDecMaxRows || in_dim < 1 || out_total < 1) return fail(B200_LORA_EINVAL, "decode_linear: bad sizes T=%d in=%d out=%d", T, in_dim, out_total);
   if (planes == nullptr || x == nullptr || weight == nullptr) return fail(B200_LORA_EINVAL, "decode_linear: null pointer");
   if (in_dim % 64 != 0 || x_ld % 8 != 0 || w_ld % 8 != 0 || x_ld < in_dim || w_ld < in_dim || out_total % 8 != 0 || !aligned16(planes) || !aligned16(x) ||
@@ -213,35 +213,36 @@ static int decode_linear_problem(BgmvProblem* bp, float* planes, const void* x, 
     return fail(B200_LORA_EUNSUPPORTED, "decode_linear: in_dim must be a multiple of 64, out of 8, rows 16-byte aligned");
   if (n_slices <= 0) return B200_LORA_OK;
   if (out_sizes == nullptr || col_offsets == nullptr || token_to_slot == nullptr) return fail(B200_LORA_EINVAL, "decode_linear: null slice or slot array");
-  if (int rc = fill_slices(bp->st, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, true, true)) return rc;
+  BgmvProblem bp = {};
+  if (int rc = fill_slices(bp.st, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, true, true)) return rc;
   int covered = 0;
-  for (int s = 0; s < bp->st.n; ++s) {
-    if (bp->st.col[s] + bp->st.out[s] > out_total) return fail(B200_LORA_EINVAL, "slice %d exceeds the output width", s);
-    covered += bp->st.out[s];
+  for (int s = 0; s < bp.st.n; ++s) {
+    if (bp.st.col[s] + bp.st.out[s] > out_total) return fail(B200_LORA_EINVAL, "slice %d exceeds the output width", s);
+    covered += bp.st.out[s];
   }
   if (covered != out_total) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: the slices must cover the output");
   const int parts = decode_gemm_parts(in_dim, out_total);
-  bp->y = planes + (size_t)parts * T * out_total; bp->y_ld = out_total;
-  bp->x = x; bp->x_ld = x_ld; bp->T = T; bp->in_dim = in_dim; bp->S = S; bp->r_max = r_max;
-  bp->rank_per_slot = rank_per_slot; bp->scale_per_slot = nullptr;
-  bp->sorted_idx = sorted_idx; bp->slot_ids = slot_ids; bp->counts = counts; bp->offsets = offsets; bp->n_buckets = n_buckets;
-  bp->scaling = 1.0f; bp->mode = 4; bp->kind = r_max % 32 != 0 ? 1 : 0; bp->token_to_slot = token_to_slot;
-  bp->beside = decode_gemm_ctas(in_dim, out_total);
+  bp.y = planes + (size_t)parts * T * out_total; bp.y_ld = out_total;
+  bp.x = x; bp.x_ld = x_ld; bp.T = T; bp.in_dim = in_dim; bp.S = S; bp.r_max = r_max;
+  bp.rank_per_slot = rank_per_slot; bp.scale_per_slot = nullptr;
+  bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets; bp.n_buckets = n_buckets;
+  bp.scaling = 1.0f; bp.mode = 4; bp.kind = r_max % 32 != 0 ? 1 : 0; bp.token_to_slot = token_to_slot;
+  bp.beside = decode_gemm_ctas(in_dim, out_total);
   if (S < 1 || r_max < 1) return fail(B200_LORA_EINVAL, "decode_linear: bad sizes S=%d r_max=%d", S, r_max);
   if (sorted_idx == nullptr || slot_ids == nullptr || counts == nullptr || offsets == nullptr)
     return fail(B200_LORA_EINVAL, "decode_linear: needs the bucket arrays");
   const char* why = nullptr;
-  if (!bgmv_supported(*bp, &why)) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: %s", why);
+  if (!bgmv_plan(bp, plan, &why)) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: %s", why);
   return B200_LORA_OK;
 }
 
 int lora_b200_decode_linear_check(int32_t T, int32_t in_dim, const void* weight, int64_t w_ld, int32_t out_total, int32_t n_slices,
                                   const void* const* a_slabs, const void* const* b_slabs, const int32_t* out_sizes,
                                   const int32_t* col_offsets, int32_t S, int32_t r_max, int32_t n_buckets) {
-  BgmvProblem bp = {};
+  BgmvParams plan;
   float* const some = reinterpret_cast<float*>(uintptr_t(256));  // (stands for the arrays of a step; not read)
   const int32_t* const index = reinterpret_cast<const int32_t*>(some);
-  return decode_linear_problem(&bp, some, some, in_dim, T, in_dim, weight, w_ld, out_total, n_slices, a_slabs, b_slabs, out_sizes, col_offsets,
+  return decode_linear_plan(&plan, some, some, in_dim, T, in_dim, weight, w_ld, out_total, n_slices, a_slabs, b_slabs, out_sizes, col_offsets,
                                S, r_max, nullptr, index, index, index, index, index, n_buckets);
 }
 
@@ -251,11 +252,11 @@ int lora_b200_decode_linear(float* planes, const void* x, int64_t x_ld, int32_t 
                             const int32_t* rank_per_slot, const int32_t* token_to_slot, const int32_t* sorted_idx,
                             const int32_t* slot_ids, const int32_t* counts, const int32_t* offsets, int32_t n_buckets,
                             void* stream) {
-  BgmvProblem bp = {};
-  if (int rc = decode_linear_problem(&bp, planes, x, x_ld, T, in_dim, weight, w_ld, out_total, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, S,
-                                     r_max, rank_per_slot, token_to_slot, sorted_idx, slot_ids, counts, offsets, n_buckets))
+  BgmvParams plan;
+  if (int rc = decode_linear_plan(&plan, planes, x, x_ld, T, in_dim, weight, w_ld, out_total, n_slices, a_slabs, b_slabs, out_sizes, col_offsets, S,
+                                  r_max, rank_per_slot, token_to_slot, sorted_idx, slot_ids, counts, offsets, n_buckets))
     return rc;
-  return decode_linear_launch(planes, x, x_ld, T, in_dim, weight, w_ld, out_total, n_slices > 0 ? &bp : nullptr, static_cast<cudaStream_t>(stream));
+  return decode_linear_launch(planes, x, x_ld, T, in_dim, weight, w_ld, out_total, n_slices > 0 ? &plan : nullptr, static_cast<cudaStream_t>(stream));
 }
 
 int lora_b200_decode_add_rmsnorm(void* normed, void* hidden_out, const float* planes, int32_t n_planes, const void* residual,
@@ -473,10 +474,11 @@ int lora_b200_shrink_allreduce_expand(void* y, int64_t y_ld, const void* x, int6
   BgmvProblem shrink_p = bp, expand_p = bp;
   shrink_p.mode = 1;
   expand_p.mode = 2; expand_p.scaling = 1.0f; expand_p.scale_per_slot = nullptr;  // the scale is already in tmp
-  const bool fused_kernels = dtype == B200_LORA_BF16 && have_buckets && bgmv_supported(shrink_p, nullptr) &&
-                             bgmv_supported(expand_p, nullptr);
+  BgmvParams shrink_plan, expand_plan;
+  const bool fused_kernels = dtype == B200_LORA_BF16 && have_buckets && bgmv_plan(shrink_p, &shrink_plan, nullptr) &&
+                             bgmv_plan(expand_p, &expand_plan, nullptr);
   if (fused_kernels) {
-    if (int rc = bgmv_launch(shrink_p, st_)) return rc;
+    if (int rc = bgmv_launch(shrink_plan, st_)) return rc;
   } else {
     // any dtype / shape: one CTA per token; rows without adapter are zero-filled (they are exchanged too)
     if (r_max > 2048) return fail(B200_LORA_EUNSUPPORTED, "generic kernel: r_max=%d > 2048", r_max);
@@ -492,7 +494,7 @@ int lora_b200_shrink_allreduce_expand(void* y, int64_t y_ld, const void* x, int6
   }
   if (tp > 1)
     if (int rc = tp_allreduce_launch(tmp, tmp, count, peer_buffers, rank, tp, capacity, st_)) return rc;
-  if (fused_kernels) return bgmv_launch(expand_p, st_);
+  if (fused_kernels) return bgmv_launch(expand_plan, st_);
   if (dtype == B200_LORA_BF16) return launch_generic_expand<__nv_bfloat16, float>(y, y_ld, tmp, T, st, S, r_max, token_to_slot, 1, st_);
   if (dtype == B200_LORA_F16) return launch_generic_expand<__half, float>(y, y_ld, tmp, T, st, S, r_max, token_to_slot, 1, st_);
   return launch_generic_expand<float, float>(y, y_ld, tmp, T, st, S, r_max, token_to_slot, 1, st_);
@@ -547,6 +549,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
   gp.rank_per_slot = rank_per_slot; gp.scale_per_slot = scale_per_slot; gp.sorted_idx = sorted_idx; gp.slot_ids = slot_ids;
   gp.counts = counts; gp.offsets = offsets; gp.n_buckets = n_buckets; gp.scaling = scaling; gp.dtype = dtype;
 
+  BgmvParams plan;
   if (overwrite) {
     // decode batches: the row-split kernel writes the delta (and the -0.0 rows) itself; everything else
     // fills y with -0.0 first and then adds as usual (-0.0 + d == d)
@@ -556,8 +559,8 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     bp.token_to_slot = token_to_slot;
     const bool decode_like = T < 32 * n_buckets || !prefill_sized(T, st, r_max, in_dim, true, prefill_cluster_add_ok(sp));
     if (dtype == B200_LORA_BF16 && have_buckets &&
-        (impl == B200_LORA_IMPL_BGMV || (impl == B200_LORA_IMPL_AUTO && decode_like)) && bgmv_supported(bp, nullptr))
-      return bgmv_launch(bp, st_);
+        (impl == B200_LORA_IMPL_BGMV || (impl == B200_LORA_IMPL_AUTO && decode_like)) && bgmv_plan(bp, &plan, nullptr))
+      return bgmv_launch(plan, st_);
     bp.mode = 0;
     bp.kind = kind;
     bp.token_to_slot = nullptr;
@@ -574,12 +577,13 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     if (int rc = check_launch("fill_neg_zero_kernel")) return rc;
   }
 
+  bool planned = false;
   if (impl == B200_LORA_IMPL_AUTO) {
     // Long batches (prefill) go to the tensor-core kernels when scratch memory was supplied, decode
     // batches to the fused kernel, everything else (other dtypes, odd shapes) to the generic one.
     int n_act = 0, parts;
     for (int s = 0; s < st.n; ++s) n_act += st.out[s] > 0;
-    const bool bgmv_ok = is16 && have_buckets && bgmv_supported(bp, nullptr);
+    const bool bgmv_ok = planned = is16 && have_buckets && bgmv_plan(bp, &plan, nullptr);
     // The prefill kernels tile rows in token order and pay one stage per run of equal slot, so they
     // want request-contiguous rows: with bucket arrays at hand, fewer than 32 rows per bucket on
     // average means a decode-like batch (slots scattered over the rows) and goes to the bucket kernel.
@@ -610,7 +614,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
       if (!is16) return fail(B200_LORA_EUNSUPPORTED, "fused decode kernel is bf16 / fp16 only");
       if (!have_buckets) return fail(B200_LORA_EINVAL, "fused decode kernel needs the bucket arrays");
       const char* why = nullptr;
-      if (bgmv_supported(bp, &why)) return bgmv_launch(bp, st_);
+      if (planned || bgmv_plan(bp, &plan, &why)) return bgmv_launch(plan, st_);
       return fail(B200_LORA_EUNSUPPORTED, "fused decode kernel: %s", why);
     }
     case B200_LORA_IMPL_SGMV:
@@ -676,7 +680,8 @@ int lora_b200_shrink_buckets(void* out, int32_t out_dtype, const void* x, int64_
   bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets;
   bp.n_buckets = n_buckets; bp.scaling = scaling; bp.mode = 1; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
   bp.tmp_io = out; bp.io16 = out_dtype != B200_LORA_F32; bp.zero_rows = 1; bp.token_to_slot = token_to_slot;
-  const bool by_bucket = buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && aligned16(out) && bgmv_supported(bp, nullptr);
+  BgmvParams plan;
+  const bool by_bucket = buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && aligned16(out) && bgmv_plan(bp, &plan, nullptr);
   const bool prefill = by_bucket ? T >= 32 * n_buckets && prefill_sized(T, st, r_max, in_dim, false, false) : T >= kSgmvAutoMinTokens;
   if (dtype == B200_LORA_BF16 && out_dtype == B200_LORA_BF16 && prefill) {
     // prefill-sized bf16 batches: the tensor-core shrink (rows without adapter are written as zeros, as the
@@ -692,10 +697,10 @@ int lora_b200_shrink_buckets(void* out, int32_t out_dtype, const void* x, int64_
       sa.gate = by_bucket ? 1 : 0;
       const int rc = sgmv_launch_shrink(sm, sa, st_);
       if (rc != B200_LORA_OK || !by_bucket) return rc;
-      bp.gate = 1;
+      plan.gate = 1;
     }
   }
-  if (by_bucket) return bgmv_launch(bp, st_);
+  if (by_bucket) return bgmv_launch(plan, st_);
 #define B200_SHRINK(TT)                                                                              \
   (out_dtype == B200_LORA_F32 && dtype != B200_LORA_F32)                                             \
       ? launch_generic_shrink<TT, float>(out, x, x_ld, T, in_dim, st, S, r_max, token_to_slot, scaling, st_) \
@@ -734,7 +739,8 @@ int lora_b200_expand_buckets(void* y, int64_t y_ld, const void* tmp, int32_t tmp
   bp.sorted_idx = sorted_idx; bp.slot_ids = slot_ids; bp.counts = counts; bp.offsets = offsets;
   bp.n_buckets = n_buckets; bp.scaling = 1.0f; bp.mode = 2; bp.kind = dtype == B200_LORA_F16 ? 2 : 1;
   bp.tmp_io = const_cast<void*>(tmp); bp.io16 = tmp_dtype != B200_LORA_F32; bp.no_add = add_inputs ? 0 : 1; bp.token_to_slot = token_to_slot;
-  const bool by_bucket = buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && dense && aligned16(tmp) && bgmv_supported(bp, nullptr);
+  BgmvParams plan;
+  const bool by_bucket = buckets && (dtype == B200_LORA_BF16 || dtype == B200_LORA_F16) && dense && aligned16(tmp) && bgmv_plan(bp, &plan, nullptr);
   const bool prefill = by_bucket ? T >= 32 * n_buckets && prefill_sized(T, st, r_max, 0, true, false) : T >= kSgmvAutoMinTokens;
   if (dtype == B200_LORA_BF16 && tmp_dtype == B200_LORA_BF16 && add_inputs && prefill) {
     // prefill-sized bf16 batches: the tensor-core expand (reduce-add tile kernel when the slices tile the
@@ -764,11 +770,11 @@ int lora_b200_expand_buckets(void* y, int64_t y_ld, const void* tmp, int32_t tmp
           rc = sgmv_launch_expand(sm, sa, st_);
         }
         if (rc != B200_LORA_OK || !by_bucket) return rc;
-        bp.gate = 1;
+        plan.gate = 1;
       }
     }
   }
-  if (by_bucket) return bgmv_launch(bp, st_);
+  if (by_bucket) return bgmv_launch(plan, st_);
 #define B200_EXPAND(TT)                                                                               \
   (tmp_dtype == B200_LORA_F32 && dtype != B200_LORA_F32)                                              \
       ? launch_generic_expand<TT, float>(y, y_ld, tmp, T, st, S, r_max, token_to_slot, add_inputs, st_) \

@@ -967,7 +967,7 @@ inline bool bgmv_plan_cluster(const BgmvProblem& b, const SliceTable& st, int C,
   p.token_to_slot = b.token_to_slot;
   if ((b.mode == 1 || b.mode == 2) && b.tmp_io == nullptr) { *why = "shrink-only / expand-only need the tmp array"; return false; }
   if (b.mode == 3 && b.token_to_slot == nullptr) { *why = "overwrite mode needs token_to_slot"; return false; }
-  if (pp != nullptr) *pp = p;
+  *pp = p;
   return true;
 }
 
@@ -1010,12 +1010,8 @@ inline bool bgmv_plan(const BgmvProblem& b, BgmvParams* pp, const char** why) {
   }
 }
 
-inline bool bgmv_supported(const BgmvProblem& b, const char** why) { return bgmv_plan(b, nullptr, why); }
-
-inline int bgmv_launch(const BgmvProblem& b, cudaStream_t stream) {
-  BgmvParams p;
-  const char* why = nullptr;
-  if (!bgmv_plan(b, &p, &why)) return fail(B200_LORA_EUNSUPPORTED, "fused decode kernel: %s", why);
+// (the caller has planned it)
+inline int bgmv_launch(const BgmvParams& p, cudaStream_t stream) {
   const size_t smem = (size_t)p.off_bar + 256;
   static thread_local int configured_device = -1;
   int dev = 0;

@@ -210,7 +210,7 @@ inline int launch_dependent(void (*kernel)(Params...), const char* name, dim3 gr
 
 // planes of x . W^T, and (lora != nullptr) the delta in the plane behind them
 inline int decode_linear_launch(float* planes, const void* x, int64_t x_ld, int T, int in_dim, const void* w, int64_t w_ld, int out,
-                                const BgmvProblem* lora, cudaStream_t stream) {
+                                const BgmvParams* lora, cudaStream_t stream) {
   DecGemmArgs a = {};
   DecGemmMaps maps;
   a.part = planes; a.T = T; a.in_dim = in_dim; a.out = out; a.n_pad = round_up_i(T, 16);
@@ -227,10 +227,8 @@ inline int decode_linear_launch(float* planes, const void* x, int64_t x_ld, int 
     return launch_dependent(decode_gemm_kernel, "decode_gemm_kernel", dim3((unsigned)(a.tiles * a.parts)), kBgmvThreads, smem, stream, maps, a);
   }
   a.delta = planes + (size_t)a.parts * T * out;
-  a.token_to_slot = lora->token_to_slot; a.rank_per_slot = lora->rank_per_slot; a.S = lora->S;
-  BgmvParams p;
-  const char* why = nullptr;
-  if (!bgmv_plan(*lora, &p, &why)) return fail(B200_LORA_EUNSUPPORTED, "decode_linear: %s", why);
+  const BgmvParams& p = *lora;
+  a.token_to_slot = p.token_to_slot; a.rank_per_slot = p.rank_per_slot; a.S = p.S;
   smem = std::max(smem, (size_t)p.off_bar + 256);
   const int C = 1 << p.c_shift, gemm_rows = ceil_div_i(a.tiles * a.parts, C);
   cudaLaunchConfig_t cfg = {};

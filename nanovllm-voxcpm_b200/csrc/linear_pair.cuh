@@ -504,14 +504,14 @@ struct LinearProblem {
   bool silu = false;         // y = silu(gate) * up of the projection's halves, [T, n_total / 2]
 };
 
-// Whether prefill_cluster_kernel takes a fused linear: its CTAs have a contiguous share of a block's columns each, so it is chosen
+// Whether prefill_cluster_kernel takes a fused linear (and its plan): its CTAs have a contiguous share of a block's columns each, so it is chosen
 // where that share is no more tiles than the CTAs of the other two have (or one more, over at most 1024 columns of x), which then
 // cost a shrink launch more. us, the others / this, rank 32: 1024 -> 1280, 300, 1700, 4001 rows 17.1 / 10.7, 19.0 / 13.3, 26.5 / 19.6;
 // 1024 -> 1024 13.4 / 9.3, 16.3 / 10.8, 18.2 / 13.3; 4096 -> 1024 26.6 / 23.6, 32.2 / 25.0, 38.6 / 35.3; 2048 -> 2048, 1000 and 3000
 // rows 17.5 / 17.2, 36.4 / 33.4. Outside the line: 1024 -> 8192, 1000 rows (4 tiles, 2) 25.6 / 30.8; 2048 -> 2560, 1000 rows (2, 1)
 // 18.9 / 25.7; 6144 -> 2048, 1000 rows (K steps of the shrink ahead of 96 others) 36.2 / 38.4; three slices of rank 64 (a pass over x
 // for every run) 1024 -> 1280, 1300 rows 17.9 / 23.0.
-inline bool prefill_cluster_linear_ok(const LinearProblem& p) {
+inline bool prefill_cluster_linear_ok(const LinearProblem& p, PcArgs* plan) {
   const SgmvProblem& b = p.lora;
   int n = 0;
   for (int s = 0; s < b.st.n; ++s) {
@@ -519,7 +519,7 @@ inline bool prefill_cluster_linear_ok(const LinearProblem& p) {
     if (b.st.col[s] % 16 != 0 || b.st.out[s] % 16 != 0) return false;  // (the MMAs of a slice would reach into the next one)
     ++n;
   }
-  PcArgs a = {};
+  PcArgs& a = *plan;
   if (ceil_div_i(b.T, kSgmvBM) > kTileSMs || !sgmv_supported(b, nullptr) || !prefill_cluster_plan(b, n, p.n_total, true, &a)) return false;
   const int nk = b.in_dim / kSgmvBK, tiles = ceil_div_i(a.cta_cols, a.tile_cols), total = ceil_div_i(b.T, kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
   const int64_t pair_tiles = (int64_t)ceil_div_i(b.T, 2 * kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
@@ -542,9 +542,10 @@ inline int linear_lora_launch(const LinearProblem& p, void* workspace, size_t wo
   const bool with_lora = slices > 0 && b.token_to_slot != nullptr;
   SgmvMaps sm;
   SgmvArgs sa = {};
-  if (with_lora && !p.silu && prefill_cluster_linear_ok(p)) {
+  PcArgs plan = {};
+  if (with_lora && !p.silu && prefill_cluster_linear_ok(p, &plan)) {
     if (int rc = sgmv_workspace_check(b, slices, workspace, workspace_bytes)) return rc;
-    return prefill_cluster_launch(b, p.weight, p.w_ld, p.n_total, p.bias, false, stream);
+    return prefill_cluster_launch(b, plan, p.weight, p.w_ld, p.n_total, p.bias, false, stream);
   }
   if (with_lora) {
     if (int rc = sgmv_prepare(b, workspace, workspace_bytes, &sm, &sa)) return rc;

@@ -537,15 +537,12 @@ inline bool prefill_cluster_plan(const SgmvProblem& b, int n, int n_total, bool 
   return true;
 }
 
-// y += delta or y = delta (weight == nullptr), or y = x . W^T (+ bias) + delta, of a problem that sgmv_supported takes.
-inline int prefill_cluster_launch(const SgmvProblem& b, const void* weight, int64_t w_ld, int n_total, const void* bias, bool overwrite, cudaStream_t stream) {
+// y += delta or y = delta (weight == nullptr), or y = x . W^T (+ bias) + delta, of a problem that sgmv_supported takes and that
+// prefill_cluster_plan has planned in `a`.
+inline int prefill_cluster_launch(const SgmvProblem& b, PcArgs a, const void* weight, int64_t w_ld, int n_total, const void* bias, bool overwrite, cudaStream_t stream) {
   const bool linear = weight != nullptr;
-  PcArgs a = {};
   PcMaps maps;
   if (b.S > 32767) return fail(B200_LORA_EUNSUPPORTED, "prefill kernel: more than 32767 adapter slots");
-  int n = 0;
-  for (int s = 0; s < b.st.n; ++s) n += b.st.out[s] > 0;
-  if (!prefill_cluster_plan(b, n, n_total, linear, &a)) return fail(B200_LORA_EUNSUPPORTED, "prefill kernel: too many rank rows");
   a.y = static_cast<__nv_bfloat16*>(b.y); a.y_ld = b.y_ld; a.bias = static_cast<const __nv_bfloat16*>(bias);
   a.T = b.T; a.in_dim = b.in_dim; a.n_total = n_total; a.S = b.S; a.r = b.r_max;
   a.token_to_slot = b.token_to_slot; a.scale_per_slot = b.scale_per_slot; a.scaling = b.scaling; a.overwrite = overwrite ? 1 : 0;
@@ -609,7 +606,9 @@ inline int prefill_add(const SgmvProblem& b, void* workspace, size_t workspace_b
     if (b.st.out[s] > 0) n_total = std::max(n_total, b.st.col[s] + b.st.out[s]);
   }
   if (int rc = sgmv_workspace_check(b, n, workspace, workspace_bytes)) return rc;
-  return prefill_cluster_launch(b, nullptr, 0, n_total, nullptr, overwrite, stream);
+  PcArgs a = {};
+  if (!prefill_cluster_plan(b, n, n_total, false, &a)) return fail(B200_LORA_EUNSUPPORTED, "prefill kernel: too many rank rows");
+  return prefill_cluster_launch(b, a, nullptr, 0, n_total, nullptr, overwrite, stream);
 }
 
 }  // namespace b200lora
