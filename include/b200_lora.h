@@ -91,8 +91,9 @@ const char* lora_b200_last_error(void);
  *                  vLLM-style with a counted -1 bucket). With the bucket arrays NULL
  *                  only the generic kernel can run.
  *  workspace       device scratch for B200_LORA_IMPL_SGMV and _GROUPED (see lora_b200_workspace_bytes); may
- *                  be NULL otherwise. With B200_LORA_IMPL_AUTO those kernels are chosen only when
- *                  enough scratch is passed.
+ *                  be NULL otherwise. With B200_LORA_IMPL_AUTO the kernels that use it are chosen only when
+ *                  enough is passed; bf16 batches of up to 18944 rows whose slices tile the output in units of 64
+ *                  columns take a prefill kernel that uses none.
  */
 int lora_b200_add(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,
                   int32_t n_slices, const void* const* a_slabs, const void* const* b_slabs,

@@ -549,6 +549,13 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
   gp.rank_per_slot = rank_per_slot; gp.scale_per_slot = scale_per_slot; gp.sorted_idx = sorted_idx; gp.slot_ids = slot_ids;
   gp.counts = counts; gp.offsets = offsets; gp.n_buckets = n_buckets; gp.scaling = scaling; gp.dtype = dtype;
 
+  // Scratch of the prefill pair. The one-launch kernel uses none: AUTO takes it without, a call that asks for the prefill kernels by
+  // name is refused without (which of them runs is not the caller's to know).
+  int n_act = 0;
+  for (int s = 0; s < st.n; ++s) n_act += st.out[s] > 0;
+  const bool one_launch = prefill_cluster_add_ok(sp), auto_impl = impl == B200_LORA_IMPL_AUTO;
+  const bool scratch_ok = (auto_impl && one_launch) || (workspace != nullptr && workspace_bytes >= sgmv_workspace_bytes(T, n_act, r_max));
+
   BgmvParams plan;
   if (overwrite) {
     // decode batches: the row-split kernel writes the delta (and the -0.0 rows) itself; everything else
@@ -557,39 +564,33 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     bp.kind = 0;
     bp.mode = 3;
     bp.token_to_slot = token_to_slot;
-    const bool decode_like = T < 32 * n_buckets || !prefill_sized(T, st, r_max, in_dim, true, prefill_cluster_add_ok(sp));
+    const bool decode_like = T < 32 * n_buckets || !prefill_sized(T, st, r_max, in_dim, true, one_launch);
     if (dtype == B200_LORA_BF16 && have_buckets &&
-        (impl == B200_LORA_IMPL_BGMV || (impl == B200_LORA_IMPL_AUTO && decode_like)) && bgmv_plan(bp, &plan, nullptr))
+        (impl == B200_LORA_IMPL_BGMV || (auto_impl && decode_like)) && bgmv_plan(bp, &plan, nullptr))
       return bgmv_launch(plan, st_);
     bp.mode = 0;
     bp.kind = kind;
     bp.token_to_slot = nullptr;
-    // prefill batches: the tile kernel stores the delta tiles instead of reduce-adding them
-    {
-      int n_act = 0;
-      for (int s = 0; s < st.n; ++s) n_act += st.out[s] > 0;
-      if (dtype == B200_LORA_BF16 && (impl == B200_LORA_IMPL_SGMV || (impl == B200_LORA_IMPL_AUTO && !decode_like)) &&
-          sgmv_supported(sp, nullptr) && prefill_overwrite_ok(st) && workspace != nullptr &&
-          workspace_bytes >= sgmv_workspace_bytes(T, n_act, r_max))
-        return prefill_add(sp, workspace, workspace_bytes, st_, true);
-    }
+    // prefill batches: the tiles of the delta are stored instead of reduce-added
+    if (dtype == B200_LORA_BF16 && (impl == B200_LORA_IMPL_SGMV || (auto_impl && !decode_like)) && sgmv_supported(sp, nullptr) &&
+        prefill_overwrite_ok(st) && scratch_ok)
+      return prefill_add(sp, workspace, workspace_bytes, st_, true);
     fill_neg_zero_kernel<<<(unsigned)T, 128, 0, st_>>>(y, y_ld, st, dtype == B200_LORA_F32 ? 4 : 2);
     if (int rc = check_launch("fill_neg_zero_kernel")) return rc;
   }
 
   bool planned = false;
-  if (impl == B200_LORA_IMPL_AUTO) {
-    // Long batches (prefill) go to the tensor-core kernels when scratch memory was supplied, decode
+  if (auto_impl) {
+    // Long batches (prefill) go to the tensor-core kernels, where they have the scratch they use, decode
     // batches to the fused kernel, everything else (other dtypes, odd shapes) to the generic one.
-    int n_act = 0, parts;
-    for (int s = 0; s < st.n; ++s) n_act += st.out[s] > 0;
+    int parts;
     const bool bgmv_ok = planned = is16 && have_buckets && bgmv_plan(bp, &plan, nullptr);
     // The prefill kernels tile rows in token order and pay one stage per run of equal slot, so they
     // want request-contiguous rows: with bucket arrays at hand, fewer than 32 rows per bucket on
     // average means a decode-like batch (slots scattered over the rows) and goes to the bucket kernel.
     const bool scattered = bgmv_ok && T < 32 * n_buckets;
-    if (dtype == B200_LORA_BF16 && !scattered && (!bgmv_ok ? T >= kSgmvAutoMinTokens : prefill_sized(T, st, r_max, in_dim, true, prefill_cluster_add_ok(sp))) && sgmv_supported(sp, nullptr) &&
-        workspace != nullptr && workspace_bytes >= sgmv_workspace_bytes(T, n_act, r_max))
+    if (dtype == B200_LORA_BF16 && !scattered && (!bgmv_ok ? T >= kSgmvAutoMinTokens : prefill_sized(T, st, r_max, in_dim, true, one_launch)) && sgmv_supported(sp, nullptr) &&
+        scratch_ok)
       impl = B200_LORA_IMPL_SGMV;
     else if (bgmv_ok && grouped_preferred(gp) && grouped_supported(gp, nullptr) && workspace != nullptr &&
              workspace_bytes >= grouped_need(gp, &parts))
@@ -619,6 +620,8 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     }
     case B200_LORA_IMPL_SGMV:
       if (dtype != B200_LORA_BF16) return fail(B200_LORA_EUNSUPPORTED, "prefill kernels are bf16 only");
+      if (!scratch_ok && sgmv_supported(sp, nullptr))
+        if (int rc = sgmv_workspace_check(sp, n_act, workspace, workspace_bytes)) return rc;
       return prefill_add(sp, workspace, workspace_bytes, st_);
     case B200_LORA_IMPL_GROUPED:
       // (where the fused decode kernel takes the batch too, the delta is rounded to bf16 and added at the L2 as there)

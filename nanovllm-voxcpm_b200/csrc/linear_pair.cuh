@@ -544,6 +544,7 @@ inline int linear_lora_launch(const LinearProblem& p, void* workspace, size_t wo
   SgmvArgs sa = {};
   PcArgs plan = {};
   if (with_lora && !p.silu && prefill_cluster_linear_ok(p, &plan)) {
+    // (uses none; the entry point's contract is the same for every shape)
     if (int rc = sgmv_workspace_check(b, slices, workspace, workspace_bytes)) return rc;
     return prefill_cluster_launch(b, plan, p.weight, p.w_ld, p.n_total, p.bias, false, stream);
   }

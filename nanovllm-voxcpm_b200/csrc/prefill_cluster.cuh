@@ -594,8 +594,7 @@ inline bool prefill_cluster_add_ok(const SgmvProblem& b) {
   return n * b.r_max <= 256 && ceil_div_i(b.T, kSgmvBM) <= kTileSMs;
 }
 
-// y += LoRA delta for a prefill batch. Callers pass scratch for the launches that the kernel does not take (what needs it is
-// not theirs to know), so it is asked for in any case.
+// y += LoRA delta for a prefill batch (overwrite: y = delta). Scratch is for the two launches of what the kernel does not take.
 inline int prefill_add(const SgmvProblem& b, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool overwrite = false) {
   const char* why = nullptr;
   if (!prefill_cluster_add_ok(b)) return prefill_add_launch(b, workspace, workspace_bytes, stream, overwrite);
@@ -605,7 +604,6 @@ inline int prefill_add(const SgmvProblem& b, void* workspace, size_t workspace_b
     n += b.st.out[s] > 0;
     if (b.st.out[s] > 0) n_total = std::max(n_total, b.st.col[s] + b.st.out[s]);
   }
-  if (int rc = sgmv_workspace_check(b, n, workspace, workspace_bytes)) return rc;
   PcArgs a = {};
   if (!prefill_cluster_plan(b, n, n_total, false, &a)) return fail(B200_LORA_EUNSUPPORTED, "prefill kernel: too many rank rows");
   return prefill_cluster_launch(b, a, nullptr, 0, n_total, nullptr, overwrite, stream);

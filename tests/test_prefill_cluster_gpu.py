@@ -68,6 +68,28 @@ def test_prefill_add_matches_oracle(case, overwrite):
     assert torch.equal(d.y.cpu()[none].view(torch.int16), base[none].view(torch.int16)), "rows without adapter keep their bits"
 
 
+@pytest.mark.parametrize("overwrite", [False, True])
+def test_auto_needs_no_scratch_for_the_one_launch_kernel(overwrite):
+    T, in_dim, outs, S, r = 1300, 1024, [1024, 128, 128], 4, 64
+    slots = torch.arange(T, dtype=torch.int32) // 400
+    p = W.make_projection(720, T, in_dim, outs, S, r, token_to_slot=slots)
+    d = p.to_device(DEV)
+    none = torch.empty(0, dtype=torch.uint8, device=DEV)
+
+    def run(impl, workspace=None):
+        y = d.y.clone()
+        LORA.launch_add(y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata(slots), 0.5, impl=impl, overwrite=overwrite,
+                        workspace=workspace)
+        torch.cuda.synchronize()
+        assert N.device_status(reset=True) == 0
+        return y
+
+    prefill, bucket = run(N.IMPL_SGMV), run(N.IMPL_BGMV)
+    assert torch.equal(run(N.IMPL_AUTO, none), prefill) and not torch.equal(prefill, bucket)
+    with pytest.raises(RuntimeError, match="scratch"):
+        run(N.IMPL_SGMV, none)
+
+
 # T, in, outs, S, r, longest run: fused linears of the kernel (the plan's lines: one tile a CTA, one more over 1024 columns of x)
 LINEAR = [
     (7, 64, [48], 2, 16, 3),                     # less than a tile of columns, some CTAs without any
