@@ -102,9 +102,25 @@ def test_delta_on_the_other_paths():
 
 
 @pytest.mark.parametrize("name", ["qkv", "o", "gate_up", "down"])
-def test_prefill_delta_is_stored_by_the_tile_kernel(name):
+def test_prefill_delta_matches_oracle(name):
     p = W.prefill_projection(name, seed=2)
     check_delta(p, run_delta(p, N.IMPL_AUTO, "eager", pad=64), f"prefill {name}")
+
+
+@pytest.mark.parametrize("T", [148 * 128, 148 * 128 + 1, 20000])  # as many row blocks as SMs: the one-launch kernel; more: the pair
+def test_delta_and_add_of_many_rows(T):
+    """Batches of more row blocks than SMs are shrunk by one kernel and stored or added by the tile kernel."""
+    slots = torch.full((T,), -1, dtype=torch.int32)
+    slots[:9000], slots[9100:18000], slots[18900:] = 0, 2, 1  # a block without adapter, runs that end inside blocks
+    p = W.make_projection(31, T, 64, [128, 64], 3, 16, token_to_slot=slots.tolist())
+    for impl in (N.IMPL_AUTO, N.IMPL_SGMV):
+        check_delta(p, run_delta(p, impl, "eager", pad=8), f"{T} rows")
+        d = p.to_device(DEV)
+        LORA.launch_add(d.y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata_for(d.token_to_slot, "eager", 3), 1.0, impl=impl)
+        want = O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets)
+        assert_lora_close(d.y.cpu(), want, what=f"add of {T} rows")
+        none = p.token_to_slot < 0
+        assert torch.equal(d.y.cpu()[none].view(torch.int16), p.y[none].view(torch.int16))
 
 
 def test_prefill_delta_mixed_blocks_and_rows_without_adapter():
