@@ -812,7 +812,8 @@ int lora_b200_expand(void* y, int64_t y_ld, const void* tmp, int32_t tmp_dtype, 
 // running inside an already captured or replaying CUDA graph, plug-ins that are handed
 // input / output buffers by a host framework and are forbidden to call the allocator, and
 // latency-critical loops that must not touch cudaMalloc (it synchronises the device). For them
-// the same two kernels run on a fixed scratch array that is part of the library image.
+// the same kernels run on a fixed scratch array that is part of the library image (the one-launch kernel uses
+// none of it; what is refused depends on the sizes alone).
 //
 // The array is one per GPU (every device that loads this library carries these bytes until
 // the process exits) and is shared by every call on that GPU: it still holds the previous

@@ -87,7 +87,7 @@ struct BgmvProblem {
   // in fp32 and rounded once; modes 0, 1 and 2, r_max % 16 == 0. What the per-token kernel computes, which these sizes and
   // types used to take (a 37-row batch of rank-16 adapters: 45 us per projection there, 3 us here).
   int kind = 0;
-  int beside = 0;          // other CTAs in the launch, at two per SM
+  int beside = 0;          // CTAs of another kind in the launch
   void* tmp_io = nullptr;  // [n_slices, T, r_max], fp32 or (io16) values of the activations' type
   int io16 = 0;
   int zero_rows = 0;       // mode 1: rows without adapter are written as zeros (token_to_slot tells which)
@@ -857,24 +857,26 @@ inline int bgmv_cluster(const BgmvProblem& b, const SliceTable& st) {
     if (C == 4 && ((kb / 4 > 128 && clusters * 8 <= resident) || (kb / 4 >= 256 && in_use * 8 <= resident))) C = 8;
     return C;
   }
-  // The least of a sum in KB of lora_B that a CTA could take meanwhile: what it takes of lora_B (rows of 16 ranks count as 32; kinds 1
-  // and 2, which multiply two halves of the intermediate and read y, 1.6 times), of lora_A and of x; the CTAs of the launch that
-  // share an SM, and those that wait for a place (the GEMM's CTAs hold theirs longer); the exchange. The factors are a fit, made for
-  // the least loss against the best size of each point, over 6688 measured points: adds (4512) of 1 to 4000 rows over 6 to 900
-  // adapters, even and skewed, graph and eager index arrays, widths 1024 to 4096, ranks 16 to 128, down of 4 to 7 and 14 K
-  // parts, and projections beside their GEMM (2176) of 1 to 128 rows. Mean loss 0.9 % (adds) and 1.2 %, of which 0.4 and 0.6 is
-  // popularity, which the host does not see: the same rows over the same buckets, 2048-wide, rank 64, 48 over 100, take 55.6 us a
-  // layer with clusters of four and 60.2 with the sizes taken (eight, o four) if even, 49.1 and 35.9 if skewed. Sums of shares unrounded by rank rows and K
-  // parts, with a line at 290 CTAs, lost 2.3 and 1.6 %. us a launch with clusters of 1 / 2 / 4 / 8, the size taken in brackets:
-  //   adds: 1024-wide, rank 16, 8 rows over 32 adapters, gate_up 16.3 / 9.1 / 5.4 / [3.8]; rank 32, 64 over 32, o 3.9 / 2.8 / [2.5] / 3.7, 128 over
-  //   128, gate_up 20.2 / [12.8] / 15.1 / 19.5 (of skewed popularity 20.5 / 11.3 / 9.5 / 15.3), 384 over 128, o 5.2 / [5.0] / 8.0 / 16.8; 4 rows, down of 4 K parts 9.5 / 4.9 /
-  //   [3.1] / 3.3, of 5 11.9 / 7.3 / 5.5 / [3.7], of 6 14.9 / 7.7 / 5.5 / [4.1], of 7 16.7 / 9.6 / 5.4 / [4.4], of 6 and 16 rows a bucket 15.4 / 8.0 / [6.1] /
-  //   7.3; 2048-wide, 384 over 32 of skewed popularity, gate_up 28.5 / 21.8 / [12.3] / 16.3; rank 64, 256 over 32, down 35.3 / 24.8 / 16.4 /
-  //   [12.5], of skewed popularity 34.4 / 24.9 / 16.8 / [19.4]; 4096-wide, 4 over 8, gate_up 54 / 30 / 15.8 / [7.8].
-  //   beside a GEMM (with the launch of the consumer): 1024-wide, rank 32, 64 rows over 64 adapters, qkv 11.4 / [11.4] / 15.9 / 26, o 6.7 /
-  //   [6.1] / 9.9 / 17.6, gate_up 22 / [15.0] / 17.9 / 24, down 13.4 / [9.5] / 13.9 / 25; 24 over 128, gate_up 18.7 / 11.7 / [10.6] / 13.9; 8 over 32, qkv
-  //   8.8 / 8.6 / 7.9 / [7.1], gate_up 17.6 / 10.2 / [7.6] / 7.2; 128 over 128, o [8.2] / 11.4 / 17.9 / 36; 2048-wide, 64 over 128, gate_up 35 /
-  //   27.4 / [27.2] / 35.
+  // The least of a sum in KB of lora_B that a CTA could take meanwhile: what it takes of lora_B (rows of 16 ranks count as 32;
+  // kinds 1 and 2, which multiply two halves of the intermediate and read y, 1.6 times), of lora_A and of x; the CTAs of the
+  // launch that share an SM, and those that wait for a place (the GEMM's CTAs hold theirs longer); the exchange. The factors are
+  // a fit, made for the least loss against the best size of each point, over 6688 measured points: adds (4512) of 1 to 4000 rows
+  // over 6 to 900 adapters, even and skewed, graph and eager index arrays, widths 1024 to 4096, ranks 16 to 128, down of 4 to 7
+  // and 14 K parts, and projections beside their GEMM (2176) of 1 to 128 rows. Mean loss 1.0 % (adds) and 1.3 %, of which 0.4 and
+  // 0.6 is popularity, which the host does not see: the same rows over the same buckets, 2048-wide, rank 64, 48 over 100, take
+  // 55.6 us a layer with clusters of four and 60.2 with the sizes taken (eight, o four) if even, 49.1 and 35.9 if skewed. Sums of
+  // shares unrounded by rank rows and K parts, with a line at 290 CTAs, lost 2.3 and 1.6 %. us a launch with clusters of 1 / 2 /
+  // 4 / 8, the size taken in brackets:
+  //   adds: 1024-wide, rank 16, 8 rows over 32 adapters, gate_up 16.3 / 9.1 / 5.4 / [3.8]; rank 32, 64 over 32, o 3.9 / 2.8 /
+  //   [2.5] / 3.7, 128 over 128, gate_up 20.2 / [12.8] / 15.1 / 19.5 (of skewed popularity 20.5 / 11.3 / 9.5 / 15.3), 384 over
+  //   128, o 5.2 / [5.0] / 8.0 / 16.8; 4 rows, down of 4 K parts 9.5 / 4.9 / [3.1] / 3.3, of 5 11.9 / 7.3 / 5.5 / [3.7], of 6
+  //   14.9 / 7.7 / 5.5 / [4.1], of 7 16.7 / 9.6 / 5.4 / [4.4], of 6 and 16 rows a bucket 15.4 / 8.0 / [6.1] / 7.3; 2048-wide, 384
+  //   over 32 of skewed popularity, gate_up 28.5 / 21.8 / [12.3] / 16.3; rank 64, 256 over 32, down 35.3 / 24.8 / 16.4 / [12.5],
+  //   of skewed popularity 34.4 / 24.9 / 16.8 / [19.4]; 4096-wide, 4 over 8, gate_up 54 / 30 / 15.8 / [7.8].
+  //   beside a GEMM (with the launch of the consumer): 1024-wide, rank 32, 64 rows over 64 adapters, qkv 11.4 / [11.4] / 15.9 /
+  //   26, o 6.7 / [6.1] / 9.9 / 17.6, gate_up 22 / [15.0] / 17.9 / 24, down 13.4 / [9.5] / 13.9 / 25; 24 over 128, gate_up 18.7 /
+  //   11.7 / [10.6] / 13.9; 8 over 32, qkv 8.8 / 8.6 / 7.9 / [7.1], gate_up 17.6 / 10.2 / [7.6] / 7.2; 128 over 128, o [8.2] /
+  //   11.4 / 17.9 / 36; 2048-wide, 64 over 128, gate_up 35 / 27.4 / [27.2] / 35.
   double least = 0.0;
   const double windows = in_use + 0.9 * std::max(0.0, rows - 1.0 - 2.0 * in_use) / kBgmvTok, rows_each = std::min((double)kBgmvTok, rows / in_use);
   const int kparts = ceil_div_i(b.in_dim, kBgmvKP);
@@ -884,7 +886,8 @@ inline int bgmv_cluster(const BgmvProblem& b, const SliceTable& st) {
     const double columns = split.by_k ? std::min(ceil_div_i(kparts, c) * kBgmvKP, b.in_dim) : b.in_dim;
     double b_rows = 0.0;
     for (int s = 0; s < st.n; ++s) b_rows += round_up_i(ceil_div_i(st.out[s], c), 32);
-    const double share = b_rows * 2.0 * std::max(b.r_max, 32) / 1024.0 * (b.kind != 0 ? 1.6 : 1.0) + (1.9 * split.rc + 0.8 * rows_each) * columns * 2.0 / 1024.0;
+    const double share_b = b_rows * 2.0 * std::max(b.r_max, 32) / 1024.0 * (b.kind != 0 ? 1.6 : 1.0);
+    const double share = share_b + (1.9 * split.rc + 0.8 * rows_each) * columns * 2.0 / 1024.0;
     const double ctas = 2.8 * b.beside + c * windows;
     const double cost = share + 0.75 * std::max(0.0, ctas - 148.0) + 2.25 * std::max(0.0, ctas - 296.0) + 3.8 * c;
     if (!any || cost < least) { least = cost; C = c; any = 1; }

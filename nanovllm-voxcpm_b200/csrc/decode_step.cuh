@@ -361,8 +361,10 @@ __global__ void __launch_bounds__(256) decode_silu_mul_kernel(__nv_bfloat16* __r
 // and v to the paged cache and attends over the cached tokens (mma.sync m16n8k16 with the up to 16 q heads as rows, online
 // softmax per warp, merged at the end). Every warp has blocks of 16 tokens of its own and stages of its own for their K and V
 // rows: the first ones are requested (cp.async) before the wait, the next one as soon as a stage is free, and no warp waits for
-// another before the merge. (Chunks of 368 tokens shared by the CTA, one after the other: 64 requests around 352 tokens 8.2 us
-// a layer, around 640 14.4; now 6.9 and 12.0.)
+// another before the merge. us a launch in a chain of its own, chunks of 368 tokens shared by the CTA / this, 64 requests around 200,
+// 352 and 640 tokens: 2 kv heads of 64, 4.6 / 4.8, 6.7 / 6.5 and 11.7 / 10.1; of 128, 7.3 / 7.6, 10.7 / 9.9 and 17.6 / 14.4; one
+// request around 200 3.3 / 3.6: short contexts lose 3 to 7 % to what long ones gain. Beyond 368 tokens a block's probabilities are
+// rounded to bf16 against the running maximum of its own warp, not of the CTA's chunk: the same widths, other last bits.
 struct DecAttnArgs {
   const float* part; int planes, ld;       // [planes, T, (Hq + 2 Hk) D]
   int T, Hq, Hk;

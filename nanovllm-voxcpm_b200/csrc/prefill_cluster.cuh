@@ -13,8 +13,9 @@
 //   * the tiles' B operands are on their way before that exchange is over, and y's rows are on their way to the L2;
 //   * eight epilogue warps in two sets, each with two output buffers, and few TMA instructions: 1.35 us a tile of 128 x 256 (2.3).
 // us per projection (qkv, o, gate_up, down), the pair / this kernel: 8172 rows, 2048-wide, rank 64: 40 / 37, 32 / 24, 92 / 91,
-// 49 / 41; 1000 rows of them 18.7 / 15.6, 14.5 / 9.7, 22 / 19, 17 / 12. What is left of gate_up's 91 (HBM time 67): every GPC writes
-// y at 0.39 TB/s, and those with fewer SMs are done after half of the time.
+// 49 / 41; 1000 rows of them 18.7 / 15.6, 14.5 / 9.7, 22 / 19, 17 / 12. What is left of gate_up's 91 (HBM time 67), from
+// the end of every CTA of one launch, 86 us: a block a cluster, and the median of them ends at 75; the 13 of 73 blocks that hold a
+// request boundary end at 82 (68 to 86), the others at 74 (58 to 83), and the smallest GPC (10 SMs) is done first (58 to 68).
 // Rows of a block may use different slots: the MMA of a run of equal slots updates the rows of that run only (its lane mask), so
 // the operand needs no masked copy per run. Rows without adapter: -0.0 in ADD launches (x + (-0.0) == x bit for bit), the base
 // result in LINEAR ones.
