@@ -167,8 +167,8 @@ __device__ __forceinline__ void bgmv_zero_rows_without_adapter(const BgmvParams&
 #endif
 // kMode = BgmvParams::mode, compiled separately so that no path carries the branches of another;
 // kFullK = every K part has all 1024 columns (in_dim a multiple of 1024): no column checks in the shrink
-// kKind = BgmvProblem::kind; kWide = r_max > 32: output tiles are less than 256 rows high and a step of the expand takes
-// several (the general step costs 12 % where a tile is a step)
+// kKind = BgmvProblem::kind; kWide = r_max > 32: output tiles are less than 256 rows high (in kind 0 the intermediate of a slice
+// has more than one block of 32 columns)
 // block_y / blocks_y: this CTA's bucket index and their number (a launch may carry other work beside the buckets)
 template <int kMode, bool kFullK, int kKind, bool kWide>
 __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, const int block_y, const int blocks_y) {
@@ -429,7 +429,11 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   if (tok_lo >= p.T) tok_lo = -1;
   if (tok_hi >= p.T) tok_hi = -1;
 
-  // expand tile e of this CTA (ring order): x = first y column, y = rows | slice << 16
+  // Expand tile e of this CTA (ring order): x = first y column, y = rows | slice << 16 | first warp << 20. A warp takes 32 rows
+  // of a tile. The tiles are dealt to the warps one behind the other, so that tiles of fewer than 256 rows are multiplied side by
+  // side; with all tiles from warp 0 on, k and v cost a step each while seven warps waited (us a launch, before / now: 1024-wide,
+  // rank 32, qkv of 256 rows over 32 adapters 4.58 / 4.24, of 4 rows 2.96 / 2.57; rank 64, a step of two tiles with every warp
+  // waiting for both: 2048-wide, 48 over 64, gate_up 12.4 / 11.7; 4096-wide, 512 over 88, o 29.5 / 25.2).
   int2* etab = reinterpret_cast<int2*>(smem + p.off_tab);
 #pragma unroll 1
   for (int e = tid; e < tiles_exp; e += kBgmvConsumers) {
@@ -437,21 +441,22 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
 #pragma unroll
     for (int s = 0; s < B200_LORA_MAX_SLICES - 1; ++s)
       if (s_e == s && et >= e_tiles[s]) { et -= e_tiles[s]; s_e = s + 1; }
-    int lo = 0, en = 0, cb = 0;
+    int lo = 0, en = 0, cb = 0, blocks = 0;
 #pragma unroll
-    for (int s = 0; s < B200_LORA_MAX_SLICES; ++s)
+    for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) {
+      if (s < s_e) blocks += (e_n[s] + 31) >> 5;
       if (s == s_e) { lo = e_lo[s]; en = e_n[s]; cb = p.st.col[s]; }
+    }
     const int r0 = et << p.er_shift;
-    etab[e] = make_int2(cb + lo + r0, min(ER, en - r0) | (s_e << 16));
+    blocks += r0 >> 5;
+    etab[e] = make_int2(cb + lo + r0, min(ER, en - r0) | (s_e << 16) | ((blocks & (kBgmvWarps - 1)) << 20));
   }
+  if (tid == 0) etab[tiles_exp] = make_int2(0, 0);  // (nobody has rows of the one behind the last)
   named_bar_sync(1, kBgmvConsumers);  // table complete
 
-  // expand: a step takes U tiles of ER rows, 256 rows in all, one 32-row block per warp: this warp's tile of the step and
-  // its rows inside that tile. (With one tile per step half of the warps had no rows at rank 64, and read past the stage.)
-  const int U = kWide ? (kBgmvWarps * 32) >> p.er_shift : 1, sub = kWide ? (warp * 32) >> p.er_shift : 0;
-  const int rb = kWide ? (warp * 32) & (ER - 1) : warp * 32;
+  // expand: first row of this warp's block of a tile; it has one if that row is one of the tile's
+  auto block_row = [&](int2 te) { return ((warp - (te.y >> 20)) & (kBgmvWarps - 1)) * 32; };
   const int x_col = warp * 32 + t * 8;  // shrink: first column of the thread inside a K part (block i adds 256)
-  const int y_col = rb + 8 * t;         // expand: first of the thread's 8 output columns inside a tile
   if (p.use_pdl) {
 #pragma unroll 1
     for (int ikp = 0; ikp < (rows_c > 0 ? nkp_c : 0); ++ikp) {
@@ -467,7 +472,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   // thread-constant pieces of the shared-memory addresses
   const uint32_t pitchB = (uint32_t)p.r_max * 2u;
   const uint32_t a_off = (uint32_t)(g * pitchA + x_col * 2);                            // shrink tile: row g
-  const uint32_t w_off = (uint32_t)(rb + 8 * (g >> 1) + (g & 1)) * pitchB + (uint32_t)t * (kPrecise ? 8u : 16u);  // expand tile
+  const uint32_t w_off = (uint32_t)(8 * (g >> 1) + (g & 1)) * pitchB + (uint32_t)t * (kPrecise ? 8u : 16u);  // expand tile
   // MMA column n of n-tile j reads slab row 8*(n/2) + 2j + (n%2) of the warp's 32 rows: thread (g,t)
   // then owns 8 consecutive output columns 8t..8t+7 of the block.
   const uint32_t t_off = (uint32_t)(g * p.pitchT + t * 16);                             // tmp: token row g
@@ -501,19 +506,21 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     if (++c_stage == NS) { c_stage = 0; c_parity ^= 1u; stage_addr = ring_base; }
   };
 
-  __nv_bfloat16* const ylo_p = p.y + (int64_t)max(tok_lo, 0) * p.y_ld + y_col;
-  __nv_bfloat16* const yhi_p = p.y + (int64_t)max(tok_hi, 0) * p.y_ld + y_col;
+  __nv_bfloat16* const ylo_p = p.y + (int64_t)max(tok_lo, 0) * p.y_ld + 8 * t;  // + first column of the warp's block
+  __nv_bfloat16* const yhi_p = p.y + (int64_t)max(tok_hi, 0) * p.y_ld + 8 * t;
   // kinds 1 and 2: y of the next tile is requested while this one is multiplied, the first one behind the shrink
   // (its 0.5 us of latency then lie beside the exchange: 37 rows, rank 16 74.1 -> 70.9 us a layer stack, 64 rows fp16 43.5 -> 40.7; before the
   // shrink it delays the x loads: 76.0 and 45.0)
   uint4 y_next[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-  auto load_y = [&](int e) {
-    if (e >= tiles_exp || kF32Out || (kMode == 2 && p.no_add)) return;
-    const int2 te = etab[e];
-    if (y_col >= (te.y & 0xffff) || !B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) return;
-    if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + te.x);
-    if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + te.x);
+  auto load_y = [&](int2 te) {
+    if (kF32Out || (kMode == 2 && p.no_add)) return;
+    const int row = block_row(te), c0 = te.x + row;
+    if (row + 8 * t >= (te.y & 0xffff) || !B200_IN_BOUNDS(c0 >= 0 && c0 + 8 * t + 8 <= p.y_cols)) return;
+    if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + c0);
+    if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + c0);
   };
+  int2 tile_next = make_int2(0, 0);  // kinds 1 and 2: looked up a tile ahead, for its y
+  if (kPrecise) tile_next = etab[0];
   const __nv_bfloat16* const xlo_p = p.x + (int64_t)max(tok_lo, 0) * p.x_ld + x_col;
   const __nv_bfloat16* const xhi_p = p.x + (int64_t)max(tok_hi, 0) * p.x_ld + x_col;
 
@@ -597,7 +604,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     }
   }
   B200_TRACE_POINT(6)
-  if (kPrecise) load_y(sub);
+  if (kPrecise) load_y(tile_next);
 
   // ===== cross-warp reduction of the K slices, scale, bf16, all-gather =====
   named_bar_sync(1, kBgmvConsumers);
@@ -693,104 +700,104 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   }
 
   // ===== expand: y[tok, cols] += tmp[16 tok, r] . B_rows^T ======================
-  // Rows of a stage beyond the tile's rows hold stale bytes; their products land in columns that are not written.
-  auto expand_fn = [&](int e, uint32_t tile_addr) {
-    const int2 te = etab[e];
-    const uint4 y_lo = y_next[0], y_hi = y_next[1];
-    if (kPrecise) load_y(e + U);
+  // Rows of a block beyond the tile's rows hold stale bytes; their products land in columns that are not written.
+  uint4 a_lo = make_uint4(0, 0, 0, 0), a_hi = a_lo;  // kind 0, ranks up to 32: the intermediate's fragments of the slice at hand
+  int a_slice = -1;
+  auto expand_fn = [&](const int2 te, const int row, const uint4 y_lo, const uint4 y_hi) {
+    const int slice = (te.y >> 16) & 15;
     float d[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.f;
-    const uint32_t a_addr = tmp_u32 + t_off + (uint32_t)((te.y >> 16) * r_eff * (kPrecise ? 4 : 2));
-    const uint32_t w_addr = tile_addr + w_off;
+    const uint32_t a_addr = tmp_u32 + t_off + (uint32_t)(slice * r_eff * (kPrecise ? 4 : 2));
+    const uint32_t w_addr = stage_addr + w_off + (uint32_t)row * pitchB;
+    if constexpr (!kWide && !kPrecise) {
+      uint4 w[4];  // (r_eff = r_max = 32: one block)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = lds128(w_addr + 2u * j * pitchB);
+      if (slice != a_slice) {
+        a_slice = slice;
+        a_lo = lds128(a_addr);
+        a_hi = lds128(a_addr + 8u * (uint32_t)p.pitchT);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], a_lo.x, a_hi.x, a_lo.y, a_hi.y, w[j].x, w[j].y);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], a_lo.z, a_hi.z, a_lo.w, a_hi.w, w[j].z, w[j].w);
+    } else {
 #pragma unroll 1
-    for (int kb = 0; kb < kblocks; ++kb) {
-      const uint32_t a_kb = a_addr + 64u * kb, w_kb = w_addr + (kPrecise ? 32u : 64u) * kb;
-      const uint4 alo = lds128(a_kb);
-      const uint4 ahi = lds128(a_kb + 8u * (uint32_t)p.pitchT);
-      uint4 w[4];
+      for (int kb = 0; kb < kblocks; ++kb) {
+        const uint32_t a_kb = a_addr + 64u * kb, w_kb = w_addr + (kPrecise ? 32u : 64u) * kb;
+        const uint4 alo = lds128(a_kb);
+        const uint4 ahi = lds128(a_kb + 8u * (uint32_t)p.pitchT);
+        uint4 w[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (kPrecise) {
-          const uint2 four = lds64(w_kb + 2u * j * pitchB);
-          w[j] = make_uint4(four.x, four.y, four.x, four.y);
-        } else {
-          w[j] = lds128(w_kb + 2u * j * pitchB);
+        for (int j = 0; j < 4; ++j) {
+          if (kPrecise) {
+            const uint2 four = lds64(w_kb + 2u * j * pitchB);
+            w[j] = make_uint4(four.x, four.y, four.x, four.y);
+          } else {
+            w[j] = lds128(w_kb + 2u * j * pitchB);
+          }
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.x, ahi.x, alo.y, ahi.y, w[j].x, w[j].y);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.z, ahi.z, alo.w, ahi.w, w[j].z, w[j].w);
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.x, ahi.x, alo.y, ahi.y, w[j].x, w[j].y);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.z, ahi.z, alo.w, ahi.w, w[j].z, w[j].w);
     }
-    if (y_col < (te.y & 0xffff) && B200_IN_BOUNDS(te.x >= 0 && te.x + y_col + 8 <= p.y_cols)) {
-      if (kF32Out) {
-        float* const yf = reinterpret_cast<float*>(p.y) + te.x + y_col;
+    const int c0 = te.x + row;
+    if (row + 8 * t >= (te.y & 0xffff) || !B200_IN_BOUNDS(c0 >= 0 && c0 + 8 * t + 8 <= p.y_cols)) return;
+    if (kF32Out) {
+      float* const yf = reinterpret_cast<float*>(p.y) + c0 + 8 * t;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int tok = h ? tok_hi : tok_lo;
-          if (tok < 0) continue;
-          float4* const dst = reinterpret_cast<float4*>(yf + (int64_t)tok * p.y_ld);
-          dst[0] = make_float4(d[0][2 * h], d[0][2 * h + 1], d[1][2 * h], d[1][2 * h + 1]);
-          dst[1] = make_float4(d[2][2 * h], d[2][2 * h + 1], d[3][2 * h], d[3][2 * h + 1]);
-        }
-        return;
+      for (int h = 0; h < 2; ++h) {
+        const int tok = h ? tok_hi : tok_lo;
+        if (tok < 0) continue;
+        float4* const dst = reinterpret_cast<float4*>(yf + (int64_t)tok * p.y_ld);
+        dst[0] = make_float4(d[0][2 * h], d[0][2 * h + 1], d[1][2 * h], d[1][2 * h + 1]);
+        dst[1] = make_float4(d[2][2 * h], d[2][2 * h + 1], d[3][2 * h], d[3][2 * h + 1]);
       }
-      if (kPrecise) {
-        if (tok_lo >= 0)
-          stg128(ylo_p + te.x, make_uint4(add_16x2<kF16>(y_lo.x, d[0][0], d[0][1]), add_16x2<kF16>(y_lo.y, d[1][0], d[1][1]),
-                                          add_16x2<kF16>(y_lo.z, d[2][0], d[2][1]), add_16x2<kF16>(y_lo.w, d[3][0], d[3][1])));
-        if (tok_hi >= 0)
-          stg128(yhi_p + te.x, make_uint4(add_16x2<kF16>(y_hi.x, d[0][2], d[0][3]), add_16x2<kF16>(y_hi.y, d[1][2], d[1][3]),
-                                          add_16x2<kF16>(y_hi.z, d[2][2], d[2][3]), add_16x2<kF16>(y_hi.w, d[3][2], d[3][3])));
-        return;
-      }
-      const uint4 lo4 = make_uint4(pack_bf16x2(d[0][0], d[0][1]), pack_bf16x2(d[1][0], d[1][1]),
-                                   pack_bf16x2(d[2][0], d[2][1]), pack_bf16x2(d[3][0], d[3][1]));
-      const uint4 hi4 = make_uint4(pack_bf16x2(d[0][2], d[0][3]), pack_bf16x2(d[1][2], d[1][3]),
-                                   pack_bf16x2(d[2][2], d[2][3]), pack_bf16x2(d[3][2], d[3][3]));
-      if (kOverwrite) {
-        if (tok_lo >= 0) stg128(ylo_p + te.x, lo4);
-        if (tok_hi >= 0) stg128(yhi_p + te.x, hi4);
-      } else {
-        // The delta is rounded to bf16 and added to y by one 16-byte reduction at the L2: y never
-        // travels to the SM and nothing waits for it. Each element of y receives exactly one
-        // reduction per launch, so the result does not depend on their order.
-        if (tok_lo >= 0) red_add_bf16x8(ylo_p + te.x, lo4.x, lo4.y, lo4.z, lo4.w);
-        if (tok_hi >= 0) red_add_bf16x8(yhi_p + te.x, hi4.x, hi4.y, hi4.z, hi4.w);
-      }
+      return;
+    }
+    if (kPrecise) {
+      if (tok_lo >= 0)
+        stg128(ylo_p + c0, make_uint4(add_16x2<kF16>(y_lo.x, d[0][0], d[0][1]), add_16x2<kF16>(y_lo.y, d[1][0], d[1][1]),
+                                      add_16x2<kF16>(y_lo.z, d[2][0], d[2][1]), add_16x2<kF16>(y_lo.w, d[3][0], d[3][1])));
+      if (tok_hi >= 0)
+        stg128(yhi_p + c0, make_uint4(add_16x2<kF16>(y_hi.x, d[0][2], d[0][3]), add_16x2<kF16>(y_hi.y, d[1][2], d[1][3]),
+                                      add_16x2<kF16>(y_hi.z, d[2][2], d[2][3]), add_16x2<kF16>(y_hi.w, d[3][2], d[3][3])));
+      return;
+    }
+    const uint4 lo4 = make_uint4(pack_bf16x2(d[0][0], d[0][1]), pack_bf16x2(d[1][0], d[1][1]),
+                                 pack_bf16x2(d[2][0], d[2][1]), pack_bf16x2(d[3][0], d[3][1]));
+    const uint4 hi4 = make_uint4(pack_bf16x2(d[0][2], d[0][3]), pack_bf16x2(d[1][2], d[1][3]),
+                                 pack_bf16x2(d[2][2], d[2][3]), pack_bf16x2(d[3][2], d[3][3]));
+    if (kOverwrite) {
+      if (tok_lo >= 0) stg128(ylo_p + c0, lo4);
+      if (tok_hi >= 0) stg128(yhi_p + c0, hi4);
+    } else {
+      // The delta is rounded to bf16 and added to y by one 16-byte reduction at the L2: y never
+      // travels to the SM and nothing waits for it. Each element of y receives exactly one
+      // reduction per launch, so the result does not depend on their order.
+      if (tok_lo >= 0) red_add_bf16x8(ylo_p + c0, lo4.x, lo4.y, lo4.z, lo4.w);
+      if (tok_hi >= 0) red_add_bf16x8(yhi_p + c0, hi4.x, hi4.y, hi4.z, hi4.w);
     }
   };
-  if (!kWide) {
 #pragma unroll 1
-    for (int e = 0; e < tiles_exp; ++e) {
-      mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
-      if (e < 10) { B200_TRACE_POINT(12 + 2 * e) }
-      expand_fn(e, stage_addr);
-      if (e < 10) { B200_TRACE_POINT(13 + 2 * e) }
-      __syncwarp();
-      if (lane == 0) mbar_arrive_relaxed(empty_bar(c_stage));
-      advance();
-    }
-  } else {
-#pragma unroll 1
-  for (int e = 0; e < tiles_exp; e += U) {
-    // (every warp waits for every tile of the step: a wait that skipped phases of a stage could no longer tell them apart)
-    const int n_here = min(U, tiles_exp - e), stage0 = c_stage;
-    uint32_t mine = 0;
-#pragma unroll 1
-    for (int u = 0; u < n_here; ++u) {
-      mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
-      if (u == sub) mine = stage_addr;
-      advance();
-    }
-    if (sub < n_here) expand_fn(e + sub, mine);
+  for (int e = 0; e < tiles_exp; ++e) {
+    // (every warp waits for every tile: a wait that skipped phases of a stage could no longer tell them apart)
+    const int2 te = kPrecise ? tile_next : etab[e];
+    const int row = block_row(te);
+    const uint4 y_lo = y_next[0], y_hi = y_next[1];
+    if (kPrecise) tile_next = etab[e + 1];
+    mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
+    if (e < 10) { B200_TRACE_POINT(12 + 2 * e) }
+    if (kPrecise) load_y(tile_next);
+    if (row < (te.y & 0xffff)) expand_fn(te, row, y_lo, y_hi);
+    if (e < 10) { B200_TRACE_POINT(13 + 2 * e) }
     __syncwarp();
-    if (lane < n_here) {
-      const int st = stage0 + lane;
-      mbar_arrive_relaxed(empty_bar(st >= NS ? st - NS : st));
-    }
-  }
+    if (lane == 0) mbar_arrive_relaxed(empty_bar(c_stage));
+    advance();
   }
   B200_TRACE_POINT(10)
   B200_TRACE_POINT(11)
@@ -943,7 +950,7 @@ inline bool bgmv_plan_cluster(const BgmvProblem& b, const SliceTable& st, int C,
   int exp_tiles = 0;
   for (int s = 0; s < st.n; ++s) exp_tiles += ceil_div_i(p.oc[s], p.ER);
   if (exp_tiles > kBgmvMaxExpandTiles) { *why = "too many expand tiles per CTA"; return false; }
-  const int tab_bytes = round_up_i(std::max(exp_tiles, 1) * 8, 128);
+  const int tab_bytes = round_up_i((exp_tiles + 1) * 8, 128);
   p.ksplit = ksplit ? 1 : 0;
   p.pitchR = Q + 4;
   const int recv_bytes = ksplit ? round_up_i(C * kBgmvTok * p.pitchR * 4, 128) : 0;

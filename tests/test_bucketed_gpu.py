@@ -53,6 +53,25 @@ def test_fused_decode_kernel_wide_ranks(r, cluster):
     assert_lora_close(y, O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets), max_abs=6e-2, what=f"r{r}")
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("cluster", [1, 2, 8])
+@pytest.mark.parametrize("outs, r", [([160, 200, 72], 32), ([8, 296, 256, 264], 16), ([520, 40], 64), ([264, 32, 8], 48)])
+def test_output_tiles_dealt_over_the_warps(outs, r, cluster, dtype):
+    """Slices of partial tiles: a tile's rows begin at any warp and may run over the last one to the first."""
+    p = W.make_projection(800 + r, 19, 1024, outs, 2, r, dtype=dtype)
+    d = p.to_device(DEV)
+    y = d.y.clone()
+    N.set_option(N.OPT_CLUSTER, cluster)
+    try:
+        LORA.launch_add(y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata_for(p.token_to_slot, "graph", 2), 1.0,
+                        impl=N.IMPL_BGMV)
+        torch.cuda.synchronize()
+    finally:
+        N.set_option(N.OPT_CLUSTER, 0)
+    assert N.device_status(reset=True) == 0
+    assert_lora_close(y, O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets), what=f"{outs} r{r}")
+
+
 @pytest.mark.parametrize("T, in_dim, outs, S, r, cluster", [
     (4, 6144, [2048], 8, 32, 8),           # eight CTAs although they lose the K split of six parts
     (4, 5120, [1280], 8, 32, 8),           # ... of five
