@@ -1084,4 +1084,25 @@ inline int bgmv_launch(const BgmvParams& p, cudaStream_t stream) {
   return B200_LORA_OK;
 }
 
+// A kernel that waits for the launch ahead itself (griddepcontrol.wait in every CTA): it may become resident while that one runs.
+template <typename... Params, typename... Args>
+inline int launch_dependent(void (*kernel)(Params...), const char* name, dim3 grid, int threads, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = bgmv_options().pdl ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(B200_LORA_ECUDA, "%s launch: %s", name, cudaGetErrorString(e));
+  }
+  return B200_LORA_OK;
+}
+
 }  // namespace b200lora

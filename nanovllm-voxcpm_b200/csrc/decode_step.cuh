@@ -188,26 +188,6 @@ inline int decode_gemm_parts(int in_dim, int out) {
 // ... and the CTAs that it counts beside the clusters of the delta (two to an SM)
 inline int decode_gemm_ctas(int in_dim, int out) { return std::min(ceil_div_i(out, 128) * decode_gemm_parts(in_dim, out), 148); }
 
-template <typename... Params, typename... Args>
-inline int launch_dependent(void (*kernel)(Params...), const char* name, dim3 grid, int threads, size_t smem, cudaStream_t stream, Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = bgmv_options().pdl ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(B200_LORA_ECUDA, "%s launch: %s", name, cudaGetErrorString(e));
-  }
-  return B200_LORA_OK;
-}
-
 // planes of x . W^T, and (lora != nullptr) the delta in the plane behind them
 inline int decode_linear_launch(float* planes, const void* x, int64_t x_ld, int T, int in_dim, const void* w, int64_t w_ld, int out,
                                 const BgmvParams* lora, cudaStream_t stream) {

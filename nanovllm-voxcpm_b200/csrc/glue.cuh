@@ -17,6 +17,15 @@ namespace b200lora {
 constexpr int kGlueThreads = 256;
 constexpr int kNormMaxVec = 16;  // 16-byte vectors per lane kept in registers: rows up to 32 * 16 * 8 = 4096 wide
 
+// The kernels below are programmatic dependents themselves: their CTAs are resident when the launch ahead ends. Only behind the wait
+// do they let the launch that follows start (a multi-LoRA launch fetches its weights, decode attention its cache rows, before
+// waiting in turn): what lies ahead of a glue launch is complete then, rotated rows in the cache among it.
+// (A prefill step of 4001 rows, four layers of 1024: 775 -> 761 us.)
+__device__ __forceinline__ void glue_enter() {
+  griddep_wait();
+  griddep_launch_dependents();
+}
+
 // Flat indexes over (row, item) fit 32 bits with room for one more stride of the grid. (With 64-bit ones the division per item
 // was a third of the instructions: SiLU of 4001 x 4096 took 21.8 us, rotation and store of 4001 rows 9.7 us.)
 inline bool glue_index_fits(int64_t rows, int64_t items) { return rows * items < (1ll << 31); }
@@ -37,9 +46,7 @@ __global__ void __launch_bounds__(kGlueThreads) add_rmsnorm_kernel(T* __restrict
                                                                    int64_t x_ld, const T* residual, int64_t res_ld,
                                                                    const T* __restrict__ weight, int T_rows, int H,
                                                                    float eps, int norm_of_rounded_sum) {
-  // a multi-LoRA launch that follows in the stream may start its weight fetch now (it waits for this
-  // kernel's completion before it touches activations)
-  griddep_launch_dependents();
+  glue_enter();
   const int row = blockIdx.x * (kGlueThreads / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= T_rows) return;
@@ -92,16 +99,15 @@ inline int add_rmsnorm_launch_t(void* normed, int64_t normed_ld, void* hidden_ou
   const int rows_per_cta = kGlueThreads / 32;
   const dim3 grid((unsigned)((T_rows + rows_per_cta - 1) / rows_per_cta));
   const int nv = (H / 8 + 31) / 32;
-#define B200_NORM_CASE(NV)                                                                                              \
-  add_rmsnorm_kernel<T, NV><<<grid, kGlueThreads, 0, stream>>>(                                                         \
-      static_cast<T*>(normed), normed_ld, static_cast<T*>(hidden_out), hidden_ld, static_cast<const T*>(x), x_ld,       \
-      static_cast<const T*>(residual), res_ld, static_cast<const T*>(weight), T_rows, H, eps, rounded)
+#define B200_NORM_CASE(NV)                                                                                                      \
+  return launch_dependent(add_rmsnorm_kernel<T, NV>, "add_rmsnorm_kernel", grid, kGlueThreads, 0, stream, static_cast<T*>(normed), normed_ld, \
+                          static_cast<T*>(hidden_out), hidden_ld, static_cast<const T*>(x), x_ld, static_cast<const T*>(residual), res_ld,    \
+                          static_cast<const T*>(weight), T_rows, H, eps, rounded)
   if (nv <= 2) B200_NORM_CASE(2);
-  else if (nv <= 4) B200_NORM_CASE(4);
-  else if (nv <= 8) B200_NORM_CASE(8);
-  else B200_NORM_CASE(16);
+  if (nv <= 4) B200_NORM_CASE(4);
+  if (nv <= 8) B200_NORM_CASE(8);
+  B200_NORM_CASE(16);
 #undef B200_NORM_CASE
-  return check_launch("add_rmsnorm_kernel");
 }
 
 inline int add_rmsnorm_launch(void* normed, int64_t normed_ld, void* hidden_out, int64_t hidden_ld, const void* x,
@@ -169,7 +175,7 @@ constexpr int kRopeThreads = 256;
 
 template <typename T, typename Index>
 __global__ void __launch_bounds__(kRopeThreads) rope_kv_store_kernel(const RopeKvParams p) {
-  griddep_launch_dependents();
+  glue_enter();
   const int half = p.D >> 1, vec_per_half = half >> 3;
   const int q_size = p.Hq * p.D, kv_size = p.Hk * p.D, kv_vecs = kv_size >> 3;
   const int rot_items = p.apply_rope ? (p.Hq + p.Hk) * vec_per_half : 0;
@@ -249,11 +255,12 @@ inline int rope_kv_store_launch(const RopeKvParams& p, int dtype, cudaStream_t s
   const int64_t want = ((int64_t)p.T * per_tok + kRopeThreads - 1) / kRopeThreads;
   const unsigned grid = (unsigned)std::min<int64_t>(want, 148 * 16);
   const bool narrow = glue_index_fits(p.T, per_tok);
-  if (dtype == B200_LORA_BF16 && narrow) rope_kv_store_kernel<__nv_bfloat16, uint32_t><<<grid, kRopeThreads, 0, stream>>>(p);
-  else if (dtype == B200_LORA_BF16) rope_kv_store_kernel<__nv_bfloat16, uint64_t><<<grid, kRopeThreads, 0, stream>>>(p);
-  else if (narrow) rope_kv_store_kernel<__half, uint32_t><<<grid, kRopeThreads, 0, stream>>>(p);
-  else rope_kv_store_kernel<__half, uint64_t><<<grid, kRopeThreads, 0, stream>>>(p);
-  return check_launch("rope_kv_store_kernel");
+#define B200_ROPE(TT, IX) return launch_dependent(rope_kv_store_kernel<TT, IX>, "rope_kv_store_kernel", dim3(grid), kRopeThreads, 0, stream, p)
+  if (dtype == B200_LORA_BF16 && narrow) B200_ROPE(__nv_bfloat16, uint32_t);
+  if (dtype == B200_LORA_BF16) B200_ROPE(__nv_bfloat16, uint64_t);
+  if (narrow) B200_ROPE(__half, uint32_t);
+  B200_ROPE(__half, uint64_t);
+#undef B200_ROPE
 }
 
 // ------------------------------------------------------------------------------------------ SiLU * up
@@ -261,7 +268,7 @@ inline int rope_kv_store_launch(const RopeKvParams& p, int dtype, cudaStream_t s
 template <typename T, typename Index>
 __global__ void __launch_bounds__(kGlueThreads) silu_mul_kernel(T* __restrict__ out, int64_t out_ld,
                                                                 const T* __restrict__ x, int64_t x_ld, int T_rows, int I) {
-  griddep_launch_dependents();
+  glue_enter();
   const int nvec = I >> 3;
   const Index total = (Index)T_rows * (Index)nvec;
   for (Index i = (Index)blockIdx.x * kGlueThreads + threadIdx.x; i < total; i += (Index)gridDim.x * kGlueThreads) {
@@ -290,14 +297,14 @@ inline int silu_mul_launch(void* out, int64_t out_ld, const void* x, int64_t x_l
   const int64_t want = (total + kGlueThreads - 1) / kGlueThreads;
   const unsigned grid = (unsigned)std::min<int64_t>(want, 148 * 16);  // a multiple of the SM count when the batch is large
   const bool narrow = glue_index_fits(T_rows, I / 8);
-#define B200_SILU(TT, IX) \
-  silu_mul_kernel<TT, IX><<<grid, kGlueThreads, 0, stream>>>(static_cast<TT*>(out), out_ld, static_cast<const TT*>(x), x_ld, T_rows, I)
+#define B200_SILU(TT, IX)                                                                                                                  \
+  return launch_dependent(silu_mul_kernel<TT, IX>, "silu_mul_kernel", dim3(grid), kGlueThreads, 0, stream, static_cast<TT*>(out), out_ld, \
+                          static_cast<const TT*>(x), x_ld, T_rows, I)
   if (dtype == B200_LORA_BF16 && narrow) B200_SILU(__nv_bfloat16, uint32_t);
-  else if (dtype == B200_LORA_BF16) B200_SILU(__nv_bfloat16, uint64_t);
-  else if (narrow) B200_SILU(__half, uint32_t);
-  else B200_SILU(__half, uint64_t);
+  if (dtype == B200_LORA_BF16) B200_SILU(__nv_bfloat16, uint64_t);
+  if (narrow) B200_SILU(__half, uint32_t);
+  B200_SILU(__half, uint64_t);
 #undef B200_SILU
-  return check_launch("silu_mul_kernel");
 }
 
 }  // namespace b200lora

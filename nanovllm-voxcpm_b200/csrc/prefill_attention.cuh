@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(kPreAttnThreads, D == 64 ? 2 : 1) prefill_atte
   const int heads = 1 << a.h_shift, per_cta = kPreAttnRows >> a.h_shift, group = a.Hq / a.Hk;
   const int head0 = (int)blockIdx.x << a.h_shift, kvh = head0 / group, req = blockIdx.y;
   const int q0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * per_cta;
+  glue_enter();
   const int begin = a.cu_seqlens[req], len = a.cu_seqlens[req + 1] - begin;
   if (q0 >= len || begin < 0 || begin + len > a.T) return;
   const int n_keys = min(len, q0 + per_cta), n_tiles = (n_keys + kPreAttnKeys - 1) / kPreAttnKeys;
@@ -173,8 +174,7 @@ inline int prefill_attention_launch(PreAttnArgs a, int D, int n_req, int max_seq
   {                                                                                                                                     \
     const cudaError_t e = cudaFuncSetAttribute(prefill_attention_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre_attn_smem<DIM>()); \
     if (e != cudaSuccess) return fail(B200_LORA_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));                              \
-    prefill_attention_kernel<DIM><<<grid, kPreAttnThreads, pre_attn_smem<DIM>(), stream>>>(a);                                          \
-    return check_launch("prefill_attention_kernel");                                                                                    \
+    return launch_dependent(prefill_attention_kernel<DIM>, "prefill_attention_kernel", grid, kPreAttnThreads, pre_attn_smem<DIM>(), stream, a); \
   }
   if (D == 64) B200_PRE_ATTN(64)
   B200_PRE_ATTN(128)
