@@ -155,11 +155,14 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
 
   const uint32_t tmem_base = tmem_base_s;
   const int nruns = nruns_s;
-  // This CTA's columns of y and its tiles of up to 256 of them. An ADD launch has nothing to add to a block without any adapter row.
+  // This CTA's columns of y and its tiles of up to 256 of them: a range in LINEAR launches; in ADD ones the tiles are dealt to the
+  // CTAs in turn, so that a cluster updates neighbouring pieces of the same rows (8172 rows, 2048-wide, rank 64, a layer 192.1 ->
+  // 190.7 us). An ADD launch has nothing to add to a block without any adapter row.
   const int c_begin = min(ck * a.cta_cols, a.n_total), c_end = min(c_begin + a.cta_cols, a.n_total);
-  const int my_tiles = kLinear || nruns > 0 || a.overwrite ? (c_end - c_begin + a.tile_cols - 1) / a.tile_cols : 0;
-  auto tile_lo = [&](int i) { return c_begin + i * a.tile_cols; };
-  auto tile_hi = [&](int i) { return min(c_begin + (i + 1) * a.tile_cols, c_end); };
+  const int all_tiles = (a.n_total + a.tile_cols - 1) / a.tile_cols;
+  const int my_tiles = kLinear ? (c_end - c_begin + a.tile_cols - 1) / a.tile_cols : nruns > 0 || a.overwrite ? (all_tiles - ck + CK - 1) / CK : 0;
+  auto tile_lo = [&](int i) { return kLinear ? c_begin + i * a.tile_cols : (i * CK + ck) * a.tile_cols; };
+  auto tile_hi = [&](int i) { return kLinear ? min(c_begin + (i + 1) * a.tile_cols, c_end) : min((i * CK + ck + 1) * a.tile_cols, a.n_total); };
   const uint32_t tmp_base = smem_base + (uint32_t)a.off_tmp, tmp_tile = (uint32_t)(kSgmvBM * row_bytes);
   // ---- the shrink's passes over x: up to G runs share one
   const int nk_all = a.in_dim / kSgmvBK, nk_per = (nk_all + CK - 1) / CK;
