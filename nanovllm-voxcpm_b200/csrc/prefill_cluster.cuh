@@ -1,5 +1,5 @@
-// Prefill multi-LoRA in one launch (bf16, tcgen05): a cluster takes a block of rows, shrinks it with K split over its CTAs,
-// and takes the block's output tiles in turn.
+// Prefill multi-LoRA in one launch (bf16, tcgen05): a cluster takes a block of rows and a range of the columns, shrinks the rows (for
+// the slices in its range) with K split over its CTAs, and takes its output tiles in turn.
 //
 //   ADD    : y[rows, :] += delta (reduce-add), or y = delta
 //   LINEAR : y[rows, :]  = x . W^T (+ bias) + delta
@@ -8,14 +8,16 @@
 // shared memory, so the second one's set-up, its wait for the first and the trip of the intermediate through the L2 are all
 // serial with the K loop: 9 to 13 us a shrink of 1000 rows whose loads take 2. Here
 //   * one set-up (barriers, TMEM, run table) and one wait for the launch ahead;
-//   * the CTAs of the cluster add their partial sums in distributed shared memory, and each sends the 16-bit values of its share
-//     straight into the MMA operand tile of every CTA (st.async): no scratch, no barrier of the cluster between the halves;
+//   * partial sums go straight from tensor memory to the CTA that owns their columns, which sends the 16-bit values straight into
+//     the MMA operand tile of every CTA (st.async both times): no scratch, no barrier of the cluster between the halves;
+//   * lora_A is asked for ahead of the wait for the launch ahead;
 //   * the tiles' B operands are on their way before that exchange is over, and y's rows are on their way to the L2;
 //   * eight epilogue warps in two sets, each with two output buffers, and few TMA instructions: 1.35 us a tile of 128 x 256 (2.3).
-// us per projection (qkv, o, gate_up, down), the pair / this kernel: 8172 rows, 2048-wide, rank 64: 40 / 37, 32 / 24, 92 / 91,
-// 49 / 41; 1000 rows of them 18.7 / 15.6, 14.5 / 9.7, 22 / 19, 17 / 12. What is left of gate_up's 91 (HBM time 67), from
-// the end of every CTA of one launch, 86 us: a block a cluster, and the median of them ends at 75; the 13 of 73 blocks that hold a
-// request boundary end at 82 (68 to 86), the others at 74 (58 to 83), and the smallest GPC (10 SMs) is done first (58 to 68).
+// us per projection (qkv, o, gate_up, down), the pair / this kernel: 8000 rows, 2048-wide, rank 64: 40 / 38, 32 / 22, 92 / 86,
+// 49 / 38; 1000 rows of them 18.7 / 15.6, 14.5 / 9.9, 22 / 18.1, 17 / 12.5. What is left of gate_up's 86 (HBM time 66): a kernel that only
+// reads, adds to and writes these rows takes 73 to 80, and the blocks that hold a request boundary end 8 us after the others. Of the 9.9
+// of o: 1.4 from the end of the launch before to its first CTA's wait, 1.3 more to the last CTA's, K loop 2.4, exchange 2.5, tile and
+// store 2.
 // Rows of a block may use different slots: the MMA of a run of equal slots updates the rows of that run only (its lane mask), so
 // the operand needs no masked copy per run. Rows without adapter: -0.0 in ADD launches (x + (-0.0) == x bit for bit), the base
 // result in LINEAR ones.
@@ -39,13 +41,14 @@ struct PcArgs {
   int out[B200_LORA_MAX_SLICES], col[B200_LORA_MAX_SLICES];
   const int32_t* token_to_slot;
   const float* scale_per_slot; float scaling;
+  int groups, group_cols;                   // clusters of a block of rows, each with a range of the columns (a multiple of 64)
   int cta_cols, tile_cols;                  // columns of y per CTA and per tile (multiples of 64, a tile at most 256)
   int overwrite;                            // ADD: store the delta (-0.0 in rows without adapter) instead of adding it
-  int bm, pad_shift, ck;                    // rows of a block (a multiple of 8, 64 to 128), log2 of the next power of two, CTAs of a cluster
+  int bm, ck;                               // rows of a block (a multiple of 8, 64 to 128), CTAs of a cluster
   int gmax;                                 // runs of a block whose K loops share one pass over x
   int stages, stage_bytes;                  // ring of the tiles: lora_B tiles (LINEAR: or x and W tiles)
   int out_bufs, off_out, off_tmp;           // output buffers of each epilogue set; byte offsets
-  int part_cols;                            // columns of partial sums exchanged at a time
+  int part_cols, off_part;                  // columns of partial sums exchanged at a time, where they arrive
 };
 struct PcMaps {
   CUtensorMap x;                            // [T, in]           box bm x 64
@@ -73,9 +76,16 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   __shared__ volatile int abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int CK = a.ck, ck = CK > 1 ? (int)cluster_ctarank() : 0, blk = (int)blockIdx.x / CK;
-  const int r = a.r, n = a.n, width = n * r, row_bytes = r * 2, bm = a.bm, row0 = blk * bm;
-  const int pad = 1 << a.pad_shift;  // rows of the exchange's buffers
+  const int CK = a.ck, ck = CK > 1 ? (int)cluster_ctarank() : 0, blk = (int)blockIdx.x / (CK * a.groups);
+  // This cluster's columns, and the slices that they touch: n of them from s0 on
+  const int g_lo = ((int)blockIdx.x / CK - blk * a.groups) * a.group_cols, g_hi = min(g_lo + a.group_cols, a.n_total);
+  int s0 = 0, n = a.n;
+  if (a.groups > 1) {  // (the slices lie one behind the other)
+    while (a.col[s0] + a.out[s0] <= g_lo) ++s0;
+    n = 1;
+    while (s0 + n < a.n && a.col[s0 + n] < g_hi) ++n;
+  }
+  const int r = a.r, width = n * r, row_bytes = r * 2, bm = a.bm, row0 = blk * bm;
   griddep_launch_dependents();
   const uint32_t smem_base = smem_u32(smem);
   if ((smem_base & 1023u) != 0) {  // (the swizzled tiles need it; the same in every CTA)
@@ -92,7 +102,8 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   auto acc_full = [&](int b) { return bar1 + 8u * (uint32_t)b; };
   auto acc_empty = [&](int b) { return bar1 + 16u + 8u * (uint32_t)b; };
   const uint32_t s_acc_full = bar1 + 32u, s_acc_empty = bar1 + 40u;
-  const uint32_t part_ready = bar1 + 48u, part_done = bar1 + 56u;  // every CTA of the cluster has written / read partial sums
+  const uint32_t part_ready = bar1 + 48u;                          // every CTA of the cluster has room for partial sums
+  const uint32_t part_full = bar1 + 56u;                           // the partial sums of this CTA's columns have arrived
   const uint32_t tmp_full = bar1 + 64u;                            // every CTA's share of the intermediate has arrived
 
   if (warp == 1) {
@@ -102,7 +113,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   if (warp == 0 && elect_one()) {
     tma_prefetch_desc(&maps.x); tma_prefetch_desc(&maps.y);
     if (kLinear) tma_prefetch_desc(&maps.w);
-    for (int s = 0; s < n; ++s) { tma_prefetch_desc(&maps.a[s]); tma_prefetch_desc(&maps.b[s]); }
+    for (int s = s0; s < s0 + n; ++s) { tma_prefetch_desc(&maps.a[s]); tma_prefetch_desc(&maps.b[s]); }
   }
   // ---- runs of equal slot inside the block
   {
@@ -140,7 +151,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
       mbar_init(s_acc_full, 1);
       mbar_init(s_acc_empty, kPcEpi / 32);
       mbar_init(part_ready, (uint32_t)CK);
-      mbar_init(part_done, (uint32_t)CK);
+      mbar_init(part_full, 1);
       mbar_init(tmp_full, 1);
       abort_flag = 0;
       mbar_fence_init();
@@ -150,19 +161,19 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   if (CK > 1) { cluster_arrive(); cluster_wait(); }  // the barriers of every CTA of the cluster are initialised
-  // Everything above may overlap the previous launch of the stream; x and y are final from here on.
-  griddep_wait();
+  // Everything above may overlap the previous launch of the stream; x and y are final from here on. (Warp 0 asks for lora_A first.)
+  if (warp != 0) griddep_wait();
 
   const uint32_t tmem_base = tmem_base_s;
   const int nruns = nruns_s;
   // This CTA's columns of y and its tiles of up to 256 of them: a range in LINEAR launches; in ADD ones the tiles are dealt to the
   // CTAs in turn, so that a cluster updates neighbouring pieces of the same rows (8172 rows, 2048-wide, rank 64, a layer 192.1 ->
   // 190.7 us). An ADD launch has nothing to add to a block without any adapter row.
-  const int c_begin = min(ck * a.cta_cols, a.n_total), c_end = min(c_begin + a.cta_cols, a.n_total);
-  const int all_tiles = (a.n_total + a.tile_cols - 1) / a.tile_cols;
+  const int c_begin = min(g_lo + ck * a.cta_cols, g_hi), c_end = min(c_begin + a.cta_cols, g_hi);
+  const int all_tiles = (g_hi - g_lo + a.tile_cols - 1) / a.tile_cols;
   const int my_tiles = kLinear ? (c_end - c_begin + a.tile_cols - 1) / a.tile_cols : nruns > 0 || a.overwrite ? (all_tiles - ck + CK - 1) / CK : 0;
-  auto tile_lo = [&](int i) { return kLinear ? c_begin + i * a.tile_cols : (i * CK + ck) * a.tile_cols; };
-  auto tile_hi = [&](int i) { return kLinear ? min(c_begin + (i + 1) * a.tile_cols, c_end) : min((i * CK + ck + 1) * a.tile_cols, a.n_total); };
+  auto tile_lo = [&](int i) { return kLinear ? c_begin + i * a.tile_cols : g_lo + (i * CK + ck) * a.tile_cols; };
+  auto tile_hi = [&](int i) { return kLinear ? min(c_begin + (i + 1) * a.tile_cols, c_end) : min(g_lo + (i * CK + ck + 1) * a.tile_cols, g_hi); };
   const uint32_t tmp_base = smem_base + (uint32_t)a.off_tmp, tmp_tile = (uint32_t)(kSgmvBM * row_bytes);
   // ---- the shrink's passes over x: up to G runs share one
   const int nk_all = a.in_dim / kSgmvBK, nk_per = (nk_all + CK - 1) / CK;
@@ -171,9 +182,11 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   const uint32_t x_tile = (uint32_t)bm * kSgmvBK * 2, a_tile = (uint32_t)r * kSgmvBK * 2;
   const uint32_t x_span = kSgmvBM * kSgmvBK * 2;  // (the MMA reads 128 rows; those beyond bm give rows that nobody reads)
   const uint32_t s_stage = kLinear ? (uint32_t)a.stage_bytes : x_span + (uint32_t)(G * n) * a_tile;
-  const int s_stages = kLinear ? a.stages : min(kPcShrinkStages, (int)((uint32_t)a.off_tmp / s_stage));
+  // ADD: the partial sums have a place of their own where that leaves the K loop enough stages
+  const bool apart = kLinear || a.off_part / (int)s_stage >= min(nk_per, 4);
+  const int s_stages = kLinear ? a.stages : min(kPcShrinkStages, (apart ? a.off_part : a.off_tmp) / (int)s_stage);
   const uint32_t s_tmem = tmem_base + (kLinear ? kSgmvBN : 0);  // (LINEAR: the first tile's sums lie in front)
-  const uint32_t part_base = kLinear ? smem_base + (uint32_t)a.off_out : smem_base + (uint32_t)((a.off_tmp - a.part_cols * pad * 4) & ~1023);
+  const uint32_t part_base = smem_base + (uint32_t)a.off_part;
   const int nk_base = kLinear ? nk_all : 0;
 
   // slice s inside tile i: its columns [lo, hi) of y
@@ -187,6 +200,9 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
     // =========================== TMA
     const uint32_t leader = elect_one();
     int st = 0, round = 0;
+    // lora_A of the first stages is asked for ahead of the wait: no kernel that lets others start early writes slabs. (LINEAR launches
+    // of more than 1920 rows: x first, us with lora_A / x first, 1024 -> 1024 of 2500 rows 12.8 / 12.4, of 300 8.2 / 8.5.)
+    const int early = npass > 0 && (!kLinear || CK == 8) ? min(s_stages, nk) : 0;
     for (int pi = 0; pi < npass; ++pi) {
       // (ADD: the partial sums of a pass lie where the ring is)
       if (!kLinear && pi > 0) mbar_wait_bounded(s_acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
@@ -194,23 +210,33 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
       int row[4];  // first lora_A row of each run of the pass (G <= 4)
 #pragma unroll
       for (int ui = 0; ui < 4; ++ui) row[ui] = uniform(ui < g ? run_slot[u0 + ui] * r : 0);
+      auto load_a = [&](int kc, int stage) {
+        const uint32_t full = kLinear ? t_full(stage) : s_full(stage);
+        mbar_arrive_expect_tx(full, x_tile + (uint32_t)(g * n) * a_tile);
+        uint32_t dst = smem_base + (uint32_t)stage * s_stage + x_span;
+#pragma unroll
+        for (int ui = 0; ui < 4; ++ui)
+          if (ui < g)
+            for (int s = 0; s < n; ++s, dst += a_tile) tma_load_2d(dst, &maps.a[s0 + s], (kc0 + kc) * kSgmvBK, row[ui], full);
+      };
+      if (pi == 0) {
+        if (leader)
+          for (int kc = 0; kc < early; ++kc) load_a(kc, kc);
+        __syncwarp();
+        griddep_wait();
+      }
       for (int kc = 0; kc < nk; ++kc) {
         const uint32_t full = kLinear ? t_full(st) : s_full(st), empty = kLinear ? t_empty(st) : s_empty(st);
         if (round > 0) mbar_wait_bounded(empty, (uint32_t)((round & 1) ^ 1), &abort_flag);
         if (leader) {
-          const uint32_t base = smem_base + (uint32_t)st * s_stage;
-          mbar_arrive_expect_tx(full, x_tile + (uint32_t)(g * n) * a_tile);
-          tma_load_2d(base, &maps.x, (kc0 + kc) * kSgmvBK, row0, full);
-          uint32_t dst = base + x_span;
-#pragma unroll
-          for (int ui = 0; ui < 4; ++ui)
-            if (ui < g)
-              for (int s = 0; s < n; ++s, dst += a_tile) tma_load_2d(dst, &maps.a[s], (kc0 + kc) * kSgmvBK, row[ui], full);
+          if (pi > 0 || kc >= early) load_a(kc, st);
+          tma_load_2d(smem_base + (uint32_t)st * s_stage, &maps.x, (kc0 + kc) * kSgmvBK, row0, full);
         }
         __syncwarp();
         if (++st == s_stages) { st = 0; ++round; }
       }
     }
+    if (npass == 0) griddep_wait();
     if (!kLinear) {
       st = round = 0;
       if (npass > 0) mbar_wait_bounded(s_acc_full, (uint32_t)((npass - 1) & 1), &abort_flag);  // the ring changes its use
@@ -241,7 +267,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
       }
       for (int u = 0; u < nruns; ++u) {
         const int slot = uniform(run_slot[u]);
-        for (int s = 0; s < n; ++s) {
+        for (int s = s0; s < s0 + n; ++s) {
           int lo, hi;
           if (!part_of(s, i, lo, hi)) continue;
           if (round > 0) mbar_wait_bounded(t_empty(st), (uint32_t)((round & 1) ^ 1), &abort_flag);
@@ -310,7 +336,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
       for (int u = 0; u < nruns; ++u) {
         const int lo_row = uniform(run_lo[u]), hi_row = uniform(run_hi[u]);
         const uint32_t off[4] = {rows_outside(lo_row, hi_row, 0), rows_outside(lo_row, hi_row, 1), rows_outside(lo_row, hi_row, 2), rows_outside(lo_row, hi_row, 3)};
-        for (int s = 0; s < n; ++s) {
+        for (int s = s0; s < s0 + n; ++s) {
           int lo, hi;
           if (!part_of(s, job, lo, hi)) continue;
           if (!have_tmp) {
@@ -322,7 +348,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
           }
           mbar_wait_bounded(t_full(st), (uint32_t)(round & 1), &abort_flag);
           tc_fence_after_sync();
-          const uint32_t bl = lo0 + ((uint32_t)(st * a.stage_bytes) >> 4), tl = lo0 + (((uint32_t)a.off_tmp + (uint32_t)s * tmp_tile) >> 4);
+          const uint32_t bl = lo0 + ((uint32_t)(st * a.stage_bytes) >> 4), tl = lo0 + (((uint32_t)a.off_tmp + (uint32_t)(s - s0) * tmp_tile) >> 4);
           const uint32_t idesc = umma_idesc_bf16(kSgmvBM, (hi - lo + 15) & ~15);
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4)
@@ -337,97 +363,107 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   } else {
     // =========================== epilogue: eight warps; a warp may only touch its own quarter of the 128 TMEM lanes
     const int quarter = warp & 3, set = (warp - 2) >> 2, etid = tid - 64, row_in_blk = quarter * 32 + lane;
-    // ---- the shrink's sums: added up over the cluster, rounded, sent to every CTA's operand tile
+    // ---- the shrink's sums: every CTA sends its partial sums to the CTA that owns their columns (eight at a time are a piece, the
+    // pieces are dealt in ranges), which adds them up, rounds and sends the values to every CTA's operand tile. Everything travels by
+    // st.async: with plain remote stores and an arrival that releases them a layer of 300 to 5000 rows takes 4 to 10 % longer, the
+    // release alone 1 us. (Before: written to shared memory, read by the owners across the cluster behind a barrier.)
     int exchange = 0;
+    const int my_slot = s_slot[row_in_blk];
+    const float my_scale = my_slot < 0 ? 0.f : a.scaling * (a.scale_per_slot != nullptr ? a.scale_per_slot[my_slot] : 1.0f);
+    const uint32_t row_off = (uint32_t)row_in_blk * 16u, quad = (uint32_t)bm * 16u;  // [sender][piece][half of it][row] of 16 bytes
     for (int pi = 0; pi < npass; ++pi) {
       const int u0 = pi * G, g = min(G, nruns - u0);
-      const int first_row = run_lo[u0], end_row = run_hi[u0 + g - 1];
+      int rows = 0;  // with an adapter, in this pass
+      for (int ui = 0; ui < g; ++ui) rows += run_hi[u0 + ui] - run_lo[u0 + ui];
+      const bool live = my_slot >= 0 && row_in_blk >= run_lo[u0] && row_in_blk < run_hi[u0 + g - 1];
+      const bool zero = my_slot < 0 && pi == 0 && row_in_blk < bm;  // rows without adapter
       mbar_wait_bounded(s_acc_full, (uint32_t)(pi & 1), &abort_flag);
       tc_fence_after_sync();
       for (int c0 = 0; c0 < width; c0 += a.part_cols, ++exchange) {
-        const int cols = min(a.part_cols, width - c0);
-        if (exchange > 0) mbar_wait_bounded_acquire_cluster(part_done, (uint32_t)((exchange - 1) & 1), &abort_flag);
-        // This CTA's partial sums into its own shared memory, as [4 columns][row] pieces of 16 bytes: the lanes of a remote read
-        // then cover consecutive bytes. A row has one run, so the runs of a pass share the buffer. (A TMEM load is a warp-wide
-        // operation on one column range: a warp whose rows straddle two runs reads both runs' columns.)
+        const int cols = min(a.part_cols, width - c0), pieces = cols >> 3, per = (pieces + CK - 1) / CK;
+        const int mine = min(max(pieces - ck * per, 0), per);
+        if (etid == 0) mbar_arrive_expect_tx(part_full, (uint32_t)((CK - 1) * rows * mine * 32));
+        // Room for them: the K loop whose ring lies there is over; behind the first exchange, the sums of the one before have been read.
+        if (!apart || exchange > 0) {
+          if (exchange > 0) named_bar_sync(2, kPcEpi);
+          if (etid < CK) mbar_arrive_remote_relaxed(mapa_shared(part_ready, (uint32_t)etid));  // (nothing to publish: what lay there has been read)
+          mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)((exchange - (apart ? 1 : 0)) & 1), &abort_flag);
+        }
+        // (A TMEM load is a warp-wide operation on one column range: a warp whose rows straddle two runs reads both runs' columns.)
         for (int ui = 0; ui < g; ++ui) {
           const int lo_row = run_lo[u0 + ui], hi_row = run_hi[u0 + ui];
           if (hi_row <= quarter * 32 || lo_row >= quarter * 32 + 32) continue;  // warp-uniform
-          const bool mine = row_in_blk >= lo_row && row_in_blk < hi_row;
+          const bool here = row_in_blk >= lo_row && row_in_blk < hi_row;
           for (int c = 16 * set; c < cols; c += 32) {
             uint32_t v[16];
             tmem_ld_32x16(s_tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ui * width + c0 + c), v);
             tmem_ld_wait();
-            if (mine) {
-              const uint32_t dst = part_base + (uint32_t)((c >> 2) * pad + row_in_blk) * 16u;
+            if (here) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) sts128(dst + 16u * (uint32_t)(pad * q), make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+              for (int h = 0; h < 2; ++h) {
+                const int p = (c >> 3) + h, owner = p / per;
+                const uint32_t at = part_base + (uint32_t)((ck * per + p - owner * per) * 2) * quad + row_off;
+                const uint4 v0 = make_uint4(v[8 * h], v[8 * h + 1], v[8 * h + 2], v[8 * h + 3]);
+                const uint4 v1 = make_uint4(v[8 * h + 4], v[8 * h + 5], v[8 * h + 6], v[8 * h + 7]);
+                if (owner == ck) {  // (this thread reads them again)
+                  sts128(at, v0);
+                  sts128(at + quad, v1);
+                } else {
+                  const uint32_t dst = mapa_shared(at, (uint32_t)owner), bar = mapa_shared(part_full, (uint32_t)owner);
+                  st_async_b32x4(dst, v0, bar);
+                  st_async_b32x4(dst + quad, v1, bar);
+                }
+              }
             }
           }
         }
         tc_fence_before_sync();
-        named_bar_sync(2, kPcEpi);
-        if (etid < CK) mbar_arrive_remote_release(mapa_shared(part_ready, (uint32_t)etid));
-        mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)(exchange & 1), &abort_flag);
-        // This CTA's share of the (8 columns x row) pieces; those of a thread are all of one row.
-        const int pieces = (cols >> 3) << a.pad_shift, per = (pieces + CK - 1) / CK;
-        const int first = ck * per + etid, last = min((ck + 1) * per, pieces);
-        const int er = first & (pad - 1), slot = s_slot[er];
-        const bool live = slot >= 0 && er >= first_row && er < end_row;
-        const bool zero = slot < 0 && pi == 0 && er < bm;  // rows without adapter
-        const float sc = live ? a.scaling * (a.scale_per_slot != nullptr ? a.scale_per_slot[slot] : 1.0f) : 0.f;
-        auto send = [&](auto parts) {
-          // eight remote reads of 32 bytes in flight per thread: one at a time each costs a round trip of 500 cycles
-          constexpr int kParts = decltype(parts)::value, kBatch = kParts >= 4 ? 8 / kParts : 2;
+        if (kLinear && c0 + cols == width) {  // the second tile's sums may go where these were
+          __syncwarp();
+          if (lane == 0) mbar_arrive(s_acc_empty);
+        }
+        mbar_wait_bounded_acquire_cluster(part_full, (uint32_t)(exchange & 1), &abort_flag);
+        auto add_up = [&](auto parts) {
+          constexpr int kParts = decltype(parts)::value;
           if (!live && !zero) return;
-          for (int e0 = first; e0 < last; e0 += kBatch * kPcEpi) {
-            float4 v[kBatch * kParts][2];
+          for (int lp = 0; lp < mine; ++lp) {
+            if ((((ck * per + lp) >> 1) & 1) != set) continue;
+            uint4 packed = make_uint4(0, 0, 0, 0);
+            if (live) {
+              uint4 w[kParts][2];
 #pragma unroll
-            for (int q = 0; q < kBatch * kParts; ++q) {
-              const int e = e0 + (q / kParts) * kPcEpi;
-              v[q][0] = v[q][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (live && e < last) {
-                const uint32_t src = mapa_shared(part_base + (uint32_t)(((e >> a.pad_shift) * 2 << a.pad_shift) + er) * 16u, (uint32_t)(q % kParts));
-                v[q][0] = ld_cluster_f32x4(src);
-                v[q][1] = ld_cluster_f32x4(src + 16u * (uint32_t)pad);
+              for (int q = 0; q < kParts; ++q)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) w[q][h] = lds128(part_base + (uint32_t)((q * per + lp) * 2 + h) * quad + row_off);
+              float sum[2][4];
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                sum[h][0] = __uint_as_float(w[0][h].x); sum[h][1] = __uint_as_float(w[0][h].y);
+                sum[h][2] = __uint_as_float(w[0][h].z); sum[h][3] = __uint_as_float(w[0][h].w);
+#pragma unroll
+                for (int q = 1; q < kParts; ++q) {
+                  sum[h][0] += __uint_as_float(w[q][h].x); sum[h][1] += __uint_as_float(w[q][h].y);
+                  sum[h][2] += __uint_as_float(w[q][h].z); sum[h][3] += __uint_as_float(w[q][h].w);
+                }
               }
+              packed = make_uint4(pack_bf16x2(sum[0][0] * my_scale, sum[0][1] * my_scale), pack_bf16x2(sum[0][2] * my_scale, sum[0][3] * my_scale),
+                                  pack_bf16x2(sum[1][0] * my_scale, sum[1][1] * my_scale), pack_bf16x2(sum[1][2] * my_scale, sum[1][3] * my_scale));
             }
-#pragma unroll
-            for (int h = 0; h < kBatch; ++h) {
-              const int e = e0 + h * kPcEpi;
-              if (e >= last) continue;
-              float4 s0 = v[h * kParts][0], s1 = v[h * kParts][1];
-#pragma unroll
-              for (int q = 1; q < kParts; ++q) {
-                const float4 w0 = v[h * kParts + q][0], w1 = v[h * kParts + q][1];
-                s0.x += w0.x; s0.y += w0.y; s0.z += w0.z; s0.w += w0.w;
-                s1.x += w1.x; s1.y += w1.y; s1.z += w1.z; s1.w += w1.w;
-              }
-              uint4 packed = make_uint4(0, 0, 0, 0);
-              if (live)
-                packed = make_uint4(pack_bf16x2(s0.x * sc, s0.y * sc), pack_bf16x2(s0.z * sc, s0.w * sc), pack_bf16x2(s1.x * sc, s1.y * sc),
-                                    pack_bf16x2(s1.z * sc, s1.w * sc));
-              const int col = c0 + 8 * (e >> a.pad_shift), s = col / r, c = col - s * r;
-              const uint32_t dst = tmp_base + (uint32_t)s * tmp_tile + swizzled_piece(er, c >> 3, row_bytes);
-              for (int q = 0; q < CK; ++q) st_async_b32x4(mapa_shared(dst, (uint32_t)q), packed, mapa_shared(tmp_full, (uint32_t)q));
-            }
+            const int col = c0 + 8 * (ck * per + lp), s = col / r, c = col - s * r;
+            const uint32_t dst = tmp_base + (uint32_t)s * tmp_tile + swizzled_piece(row_in_blk, c >> 3, row_bytes);
+            for (int q = 0; q < CK; ++q) st_async_b32x4(mapa_shared(dst, (uint32_t)q), packed, mapa_shared(tmp_full, (uint32_t)q));
           }
         };
-        if (CK == 8) send(std::integral_constant<int, 8>{});
-        else if (CK == 4) send(std::integral_constant<int, 4>{});
-        else if (CK == 2) send(std::integral_constant<int, 2>{});
-        else send(std::integral_constant<int, 1>{});
-        if (pi + 1 < npass || c0 + cols < width) {
-          named_bar_sync(2, kPcEpi);
-          if (etid < CK) mbar_arrive_remote_release(mapa_shared(part_done, (uint32_t)etid));
-        }
+        if (CK == 8) add_up(std::integral_constant<int, 8>{});
+        else if (CK == 4) add_up(std::integral_constant<int, 4>{});
+        else if (CK == 2) add_up(std::integral_constant<int, 2>{});
+        else add_up(std::integral_constant<int, 1>{});
       }
-      // (ADD: the partial sums lie where the ring is: no refill before every CTA has read them)
-      if (!kLinear && pi + 1 < npass) mbar_wait_bounded_acquire_cluster(part_done, (uint32_t)((exchange - 1) & 1), &abort_flag);
-      fence_proxy_async_smem();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(s_acc_empty);
+      if (!kLinear) {
+        fence_proxy_async_smem();  // the ring is filled again where the partial sums were
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_acc_empty);
+      }
     }
     // ---- the tiles: set 0 takes the first and third 64-column chunk of a tile, set 1 the others
     const uint32_t out_bytes = (uint32_t)bm * kGemmOutChunk * 2;
@@ -505,16 +541,74 @@ inline void prefill_cluster_split(int T, int in_dim, PcArgs* a) {
   a->ck = 1;
   while (a->ck < 8 && ceil_div_i(T, kSgmvBM) <= clusters_resident(2 * a->ck) && ceil_div_i(nk, 2 * a->ck) * (2 * a->ck - 1) < nk) a->ck *= 2;
   a->bm = std::min(kSgmvBM, std::max(64, round_up_i(ceil_div_i(T, clusters_resident(a->ck)), 8)));
-  a->pad_shift = a->bm == 64 ? 6 : 7;
+  a->groups = 1;
 }
+
+// Slices (of those in a) that a range of the columns touches, at most
+inline int prefill_cluster_need(const PcArgs& a, int n, int group_cols, int groups) {
+  int most = 1;
+  for (int g = 0; g < groups; ++g) {
+    int here = 0;
+    for (int s = 0; s < n; ++s) here += a.col[s] < (g + 1) * group_cols && a.col[s] + a.out[s] > g * group_cols;
+    most = std::max(most, here);
+  }
+  return most;
+}
+
+// ADD launches: runs of a block that share a pass over x (`width` rank rows each): sums in 512 TMEM columns, two stages of the ring
+inline int prefill_cluster_runs(int width, int ring) {
+  int runs = 1;
+  for (int g = 2; g <= 4; ++g)
+    if (g * width <= 512 && ring / (kSgmvBM * kSgmvBK * 2 + g * width * kSgmvBK * 2) >= 2) runs = g;
+  return runs;
+}
+
+// ADD launches: K parts (the CTAs of a cluster), groups of columns and rows of a block, out of those whose clusters are resident at
+// once. The least of a sum in us: the K loop at 70 KB a us, the exchange, the output tiles, less than half of the SMs (the launch
+// behind then sets itself up beside this one), passes over x that fewer than four runs can share. A fit to 210 measured points (15
+// projections, 1024- and 2048-wide, rank 16 to 64; 200 to 11000 rows of up to eight prompts, every K split with 1 to 16 groups): it
+// loses 0.9 % to the best split of each, at most 17; one group and the largest K split 10.3. us, that / the split taken: 2048 ->
+// 2 x 6144, rank 64, 300, 700, 2000, 4000 rows 22.5 / 13.6, 22.0 / 15.1, 29.5 / 27.9, 51.9 / 47.2; 2048 -> 2560 300 and 700 20.0 / 12.6,
+// 19.4 / 15.4; 1024 -> 1024, rank 32, 300 and 2000 7.9 / 7.4, 8.8 / 8.8. (A CTA's tiles, 1.1 us each, were half of the time where a
+// block had one cluster: with groups a block can be 128 rows high and its columns still go to 16 CTAs and more.)
+inline void prefill_cluster_add_split(int T, int in_dim, int n, int n_total, int r, PcArgs* a) {
+  const int nk = in_dim / kSgmvBK;
+  double least = 0.0;
+  a->ck = 0;
+  for (int ck = 1; ck <= 8; ck *= 2) {
+    if (ck > 1 && ceil_div_i(nk, ck) * (ck - 1) >= nk) break;  // every K part at least one step
+    for (int groups = 1; groups <= clusters_resident(ck) && 64 * ck * groups <= std::max(n_total, 64 * ck); ++groups) {
+      const int group_cols = round_up_i(ceil_div_i(n_total, groups), 64);
+      if (group_cols * (groups - 1) >= n_total) continue;
+      const int bm = std::max(64, round_up_i(ceil_div_i(T, clusters_resident(ck) / groups), 8)), rows = std::min(bm, kSgmvBM);
+      if (bm > kSgmvBM && (ck > 1 || groups > 1)) break;
+      const int width = prefill_cluster_need(*a, n, group_cols, groups) * r, cols = round_up_i(ceil_div_i(group_cols, ck), 64);
+      const double cost = ceil_div_i(nk, ck) * (rows + width) * (kSgmvBK * 2 / 70e3) + 0.05 * rows * width * 4 / 1024 + 0.35 * ceil_div_i(cols, kSgmvBN) +
+                          0.1 * cols / kSgmvBN + (ck * groups * ceil_div_i(T, rows) > 74 ? 0.3 : 0.0) +
+                          3.0 * (4 - prefill_cluster_runs(width, kPcSmem - width * kSgmvBM * 2));
+      if (a->ck == 0 || cost < least) {
+        least = cost;
+        a->ck = ck; a->groups = groups; a->bm = rows;
+      }
+    }
+  }
+}
+
+// bytes of the partial sums that a CTA gets of `cols` columns
+inline int prefill_cluster_part_bytes(const PcArgs& a, int cols) { return a.ck * ceil_div_i(cols / 8, a.ck) * 8 * a.bm * 4; }
 
 // Split, tiles and shared memory (ring of the tiles, output buffers, the intermediate as MMA operand; ADD launches shrink through a
 // ring over the first two) of a problem with `n` slices; false: too many rank rows for them.
 inline bool prefill_cluster_plan(const SgmvProblem& b, int n, int n_total, bool linear, PcArgs* a) {
-  prefill_cluster_split(b.T, b.in_dim, a);
-  a->cta_cols = round_up_i(ceil_div_i(n_total, a->ck), 64);
+  for (int s = 0, k = 0; s < b.st.n; ++s)
+    if (b.st.out[s] > 0) { a->out[k] = b.st.out[s]; a->col[k] = b.st.col[s]; ++k; }
+  if (linear) prefill_cluster_split(b.T, b.in_dim, a);
+  else prefill_cluster_add_split(b.T, b.in_dim, n, n_total, b.r_max, a);
+  a->group_cols = a->groups > 1 ? round_up_i(ceil_div_i(n_total, a->groups), 64) : n_total;
+  const int need = a->groups > 1 ? prefill_cluster_need(*a, n, a->group_cols, a->groups) : n;
+  a->cta_cols = round_up_i(ceil_div_i(a->group_cols, a->ck), 64);
   a->tile_cols = round_up_i(ceil_div_i(a->cta_cols, ceil_div_i(a->cta_cols, kSgmvBN)), 64);
-  const int width = n * b.r_max, tmp_bytes = n * kSgmvBM * b.r_max * 2, out_buf = a->bm * kGemmOutChunk * 2;
+  const int width = need * b.r_max, tmp_bytes = need * kSgmvBM * b.r_max * 2, out_buf = a->bm * kGemmOutChunk * 2;
   a->off_tmp = kPcSmem - tmp_bytes;
   a->gmax = 1;
   if (linear) {
@@ -527,17 +621,18 @@ inline bool prefill_cluster_plan(const SgmvProblem& b, int n, int n_total, bool 
     const int room = a->off_tmp - a->stages * a->stage_bytes;
     if (width > kSgmvBN || room < 2 * out_buf) return false;
     a->out_bufs = std::min(2, room / (2 * out_buf));
-    a->part_cols = std::min(width, 2 * a->out_bufs * out_buf / (4 << a->pad_shift) & ~15);
+    a->part_cols = width;
+    while (prefill_cluster_part_bytes(*a, a->part_cols) > 2 * a->out_bufs * out_buf) a->part_cols -= 16;  // (16 always fit)
   } else {
     a->stages = kPcTileStages;
     a->stage_bytes = a->tile_cols * b.r_max * 2;
     a->out_bufs = 2;
     while (a->stages > 2 && a->off_tmp - a->stages * a->stage_bytes < 2 * a->out_bufs * out_buf) --a->stages;
-    for (int g = 2; g <= 4; ++g)
-      if (g * width <= 512 && a->off_tmp / (kSgmvBM * kSgmvBK * 2 + g * width * kSgmvBK * 2) >= 2) a->gmax = g;
+    a->gmax = prefill_cluster_runs(width, a->off_tmp);
     a->part_cols = width;
   }
   a->off_out = a->stages * a->stage_bytes;
+  a->off_part = linear ? a->off_out : (a->off_tmp - prefill_cluster_part_bytes(*a, width)) & ~1023;
   return true;
 }
 
@@ -552,7 +647,6 @@ inline int prefill_cluster_launch(const SgmvProblem& b, PcArgs a, const void* we
   a.token_to_slot = b.token_to_slot; a.scale_per_slot = b.scale_per_slot; a.scaling = b.scaling; a.overwrite = overwrite ? 1 : 0;
   for (int s = 0; s < b.st.n; ++s) {
     if (b.st.out[s] == 0) continue;
-    a.out[a.n] = b.st.out[s]; a.col[a.n] = b.st.col[s];
     if (int rc = make_tmap_2d(&maps.a[a.n], b.st.a[s], (uint64_t)b.S * b.r_max, (uint64_t)b.in_dim, (uint64_t)b.in_dim, (uint32_t)b.r_max, kSgmvBK)) return rc;
     if (int rc = make_tmap_2d(&maps.b[a.n], b.st.b[s], (uint64_t)b.S * b.st.out[s], (uint64_t)b.r_max, (uint64_t)b.r_max, kPcBox, (uint32_t)b.r_max)) return rc;
     ++a.n;
@@ -566,7 +660,7 @@ inline int prefill_cluster_launch(const SgmvProblem& b, PcArgs a, const void* we
   const auto kernel = linear ? prefill_cluster_kernel<true> : prefill_cluster_kernel<false>;
   if (int rc = sgmv_set_smem(reinterpret_cast<const void*>(kernel), kPcSmem)) return rc;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(ceil_div_i(b.T, a.bm) * a.ck), 1, 1);
+  cfg.gridDim = dim3((unsigned)(ceil_div_i(b.T, a.bm) * a.groups * a.ck), 1, 1);
   cfg.blockDim = dim3(kPcThreads, 1, 1);
   cfg.dynamicSmemBytes = kPcSmem;
   cfg.stream = stream;

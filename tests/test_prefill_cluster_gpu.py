@@ -37,14 +37,20 @@ def metadata(slots):
 CASES = [
     (1, 64, [64], 1, 16, 1),                     # one row, one K step
     (64, 1024, [128, 64], 3, 32, 9),             # one block of 64 rows, eight K parts
-    (65, 192, [320], 3, 64, 70),                 # two blocks, K parts of one step
-    (960, 2048, [256, 64, 64], 5, 64, 200),      # 15 clusters of 8: blocks of 64 rows
-    (961, 2048, [256, 64, 64], 5, 64, 30),       # ... of 72, several passes a block
-    (1920, 576, [640], 4, 32, 400),              # 15 of 128; K parts of two steps, the last of one
+    (65, 192, [320], 3, 64, 70),                 # two blocks, two groups of columns
+    (960, 2048, [256, 64, 64], 5, 64, 200),      # groups that straddle slices
+    (961, 2048, [256, 64, 64], 5, 64, 30),       # ... more blocks, several passes a block
+    (1920, 576, [640], 4, 32, 400),              # K parts of five and four steps
     (1921, 1024, [192, 192], 4, 32, 5),          # clusters of 4, blocks of 64, 40 runs a block
     (4225, 320, [512], 6, 16, 300),              # clusters of 2, ragged
-    (9472, 128, [64, 64, 64, 64], 2, 64, 900),   # 74 clusters of 2, four slices of rank 64
+    (9472, 128, [64, 64, 64, 64], 2, 64, 900),   # two groups of one CTA, four slices of rank 64
     (9473, 128, [256], 2, 32, 0),                # one CTA a block
+    (300, 1024, [448, 128, 192], 5, 64, 60),     # three groups, of one and of two slices
+    (900, 256, [1536, 1600], 4, 32, 200),        # nine groups, the last one narrower
+    (130, 64, [320, 64, 512, 128], 4, 64, 9),    # sixteen groups of one CTA, a tile each
+    (300, 64, [4032], 3, 16, 7),                 # 21 groups, many runs a block
+    (700, 1024, [1024, 128, 128], 6, 64, 150),   # ten groups of columns
+    (2100, 1024, [1024, 128, 128], 4, 64, 40),   # rank rows of three slices in a block: partial sums where the K loop's ring was
 ]
 
 
