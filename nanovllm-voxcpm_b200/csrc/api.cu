@@ -99,27 +99,30 @@ int launch_generic_expand(void* y, int64_t y_ld, const void* tmp, int T_rows, co
 
 namespace {
 
-// Whether a bf16 batch is large enough for the prefill kernels rather than the bucket kernel (3 to 5 us, an adapter read once per
-// 16 rows of it, in windows of which 74 by 4 CTAs are resident), from 512 rows on, by rows and by the adapter bytes that the
-// bucket kernel would read.
-//   prefill_cluster_kernel (adds): us per projection, bucket / prefill kernel, two to eight prompts. 1024-wide, rank 32: 1000 rows
-//   qkv (18 MB) 7.0 / 10.5, gate_up (41 MB) 9.3 / 13.1, 1300 rows 10 / 10.5 and 15 / 13.1, 2200 rows 14 / 11.7 and 22 / 19;
-//   2048-wide, rank 32: 1000 rows qkv (35 MB) 9.4 / 11.8, gate_up (66 MB) 20 / 16, 1500 rows 16 / 12.7 and 32 / 19; rank 64: 700 rows
-//   qkv (49 MB) 16.7 / 14.1, down (46 MB) 23 / 11.2, o (23 MB) 7.5 / 9.5. Over 900 measured points of 300 to 3200 rows, three
-//   widths and ranks, this line is 2.1 % slower than the better choice each time (without the line at 75 windows 6.2 %). At 35 MB
-//   it would be 1.2 %, but adapters of mixed ranks cost the bucket kernel less: 962 rows, 1024-wide, ranks 8 to 32, gate_up (40
-//   MB): a layer 24.6 / 29.4.
+// Whether a bf16 batch is large enough for the prefill kernels rather than the bucket kernel (an adapter read once per 16 rows of it),
+// by the adapter bytes that the bucket kernel would read; 16 rank rows take it as long as 32.
+//   prefill_cluster_kernel (adds): us per projection, bucket / prefill kernel, eight prompts: 1024-wide, rank 32: 1000 rows, qkv (18
+//   MB) 6.7 / 10.1, gate_up (41 MB) 9.5 / 12.0, 2000 rows, qkv (35 MB) 8.0 / 11.3, 2500 (44 MB) 12.9 / 11.6, o (21 MB) 6.2 / 9.0;
+//   2048-wide, rank 32: 1000 rows, qkv (35 MB) 9.1 / 12.3, 1200 (42 MB) 14.5 / 12.7; rank 64: gate_up of 400 rows (52 MB) 12.7 / 13.0,
+//   of 511 (67 MB) 20 / 14; 4096-wide, rank 64, gate_up of 200 rows (61 MB) 21.9 / 17.6. Over 1440 measured points (200 to 3300 rows of two
+//   to eight prompts, two widths, ranks 16 to 64, equal and mixed) the line is 2.9 % slower than the better choice each time, one at 75
+//   windows and 50 MB 6.5. Adapters of rank 16 that went to the bucket kernel, which keeps their intermediate as two numbers, still
+//   do: up to 1184 rows and 50 MB.
 //   sgmv_shrink_kernel and the launch behind it (operators, slices that do not tile the output; at least 11 us for the pair): bucket /
 //   pair, six prompts: 1024-wide, rank 32, 900 rows, qkv (16 MB) 6.7 / 13.5, gate_up (37 MB) 8.9 / 15.1, 1500 rows 11.5 / 13.8 and
 //   (61 MB) 18.6 / 20.4; 2048-wide, rank 32, 900 rows, gate_up (59 MB) 19.0 / 19.1, 1500 rows (98 MB) 32.9 / 24.7; rank 64, 900
 //   rows, qkv (63 MB) 18.8 / 17.0, 1500 rows 33.2 / 19.3.
 inline bool prefill_sized(int32_t T, const SliceTable& st, int32_t r_max, int32_t in_dim, bool expand, bool one_launch) {
+  constexpr int64_t kMB = 1000 * 1000;
+  const int windows = ceil_div_i(T, kBgmvTok);
   int64_t bytes = 0;
   for (int s = 0; s < st.n; ++s)
     if (st.out[s] > 0 || !expand) bytes += 2 * (int64_t)r_max * (in_dim + (expand ? st.out[s] : 0));
-  bytes *= ceil_div_i(T, kBgmvTok);
-  if (T < kSgmvAutoMinTokens) return false;
-  return r_max > 32 || bytes > 50 * 1000 * 1000 || (one_launch && ceil_div_i(T, kBgmvTok) > 74);
+  bytes *= windows;
+  const bool pair_sized = T >= kSgmvAutoMinTokens && (r_max > 32 || bytes > 50 * kMB);
+  if (pair_sized || !one_launch) return pair_sized;
+  if (r_max <= 16 && windows <= 74) return false;
+  return bytes * (r_max <= 16 ? 2 : 1) > (T < kSgmvAutoMinTokens ? 52 : 38) * kMB || windows > 240;
 }
 
 }  // namespace

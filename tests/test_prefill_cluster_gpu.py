@@ -96,6 +96,29 @@ def test_auto_needs_no_scratch_for_the_one_launch_kernel(overwrite):
         run(N.IMPL_SGMV, none)
 
 
+@pytest.mark.parametrize("T, in_dim, outs, r, prefill", [
+    (2000, 1024, [1024, 128, 128], 32, False), (2500, 1024, [1024, 128, 128], 32, True),   # 35 and 44 MB of adapters for the bucket kernel
+    (400, 2048, [2048, 256, 256], 64, False), (480, 2048, [6144, 6144], 64, True),         # 28 and 63 MB, fewer than 512 rows
+    (1000, 1024, [4096, 4096], 16, False), (1300, 1024, [4096, 4096], 16, True),           # rank 16: as before up to 1184 rows
+    (1300, 1024, [1024], 16, False), (3840, 256, [256], 32, False), (3841, 256, [256], 32, True),
+])
+def test_auto_takes_the_kernel_of_the_line(T, in_dim, outs, r, prefill):
+    slots = torch.arange(T, dtype=torch.int32) * 4 // T
+    p = W.make_projection(740, T, in_dim, outs, 4, r, token_to_slot=slots)
+    d = p.to_device(DEV)
+
+    def run(impl):
+        y = d.y.clone()
+        LORA.launch_add(y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata(slots), 0.5, impl=impl)
+        torch.cuda.synchronize()
+        assert N.device_status(reset=True) == 0
+        return y
+
+    by_name = {True: run(N.IMPL_SGMV), False: run(N.IMPL_BGMV)}
+    assert not torch.equal(by_name[True], by_name[False])
+    assert torch.equal(run(N.IMPL_AUTO), by_name[prefill])
+
+
 # T, in, outs, S, r, longest run: fused linears of the kernel (the plan's lines: one tile a CTA, one more over 1024 columns of x)
 LINEAR = [
     (7, 64, [48], 2, 16, 3),                     # less than a tile of columns, some CTAs without any
