@@ -382,10 +382,12 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
       for (int c0 = 0; c0 < width; c0 += a.part_cols, ++exchange) {
         const int cols = min(a.part_cols, width - c0), pieces = cols >> 3, per = (pieces + CK - 1) / CK;
         const int mine = min(max(pieces - ck * per, 0), per);
+        // (Not before every thread has seen the exchange before complete: one of no bytes is complete at once, and a wait that is two
+        // phases behind takes the parity for that of the phase to come.)
+        if (exchange > 0) named_bar_sync(2, kPcEpi);
         if (etid == 0) mbar_arrive_expect_tx(part_full, (uint32_t)((CK - 1) * rows * mine * 32));
         // Room for them: the K loop whose ring lies there is over; behind the first exchange, the sums of the one before have been read.
         if (!apart || exchange > 0) {
-          if (exchange > 0) named_bar_sync(2, kPcEpi);
           if (etid < CK) mbar_arrive_remote_relaxed(mapa_shared(part_ready, (uint32_t)etid));  // (nothing to publish: what lay there has been read)
           mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)((exchange - (apart ? 1 : 0)) & 1), &abort_flag);
         }

@@ -127,6 +127,7 @@ LINEAR = [
     (961, 320, [1000 - 8], 3, 64, 300),          # ragged columns, blocks of 72 rows
     (2200, 1024, [640, 640], 4, 64, 500),        # clusters of 4, two tiles a CTA
     (4300, 128, [512], 4, 16, 128),              # clusters of 2
+    (517, 1024, [320], 3, 16, 4),                # many passes, CTAs that own no rank columns
 ]
 
 
