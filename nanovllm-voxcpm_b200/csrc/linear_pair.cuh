@@ -504,13 +504,14 @@ struct LinearProblem {
   bool silu = false;         // y = silu(gate) * up of the projection's halves, [T, n_total / 2]
 };
 
-// Whether prefill_cluster_kernel takes a fused linear (and its plan): its CTAs have a contiguous share of a block's columns each, so it is chosen
-// where that share is no more tiles than the CTAs of the other two have (or one more, over at most 1024 columns of x), which then
-// cost a shrink launch more. us, the others / this, rank 32: 1024 -> 1280, 300, 1700, 4001 rows 17.1 / 10.7, 19.0 / 13.3, 26.5 / 19.6;
-// 1024 -> 1024 13.4 / 9.3, 16.3 / 10.8, 18.2 / 13.3; 4096 -> 1024 26.6 / 23.6, 32.2 / 25.0, 38.6 / 35.3; 2048 -> 2048, 1000 and 3000
-// rows 17.5 / 17.2, 36.4 / 33.4. Outside the line: 1024 -> 8192, 1000 rows (4 tiles, 2) 25.6 / 30.8; 2048 -> 2560, 1000 rows (2, 1)
-// 18.9 / 25.7; 6144 -> 2048, 1000 rows (K steps of the shrink ahead of 96 others) 36.2 / 38.4; three slices of rank 64 (a pass over x
-// for every run) 1024 -> 1280, 1300 rows 17.9 / 23.0.
+// Whether prefill_cluster_kernel takes a fused linear (and its plan): where its expected time is less than that of the shrink launch and
+// the kernel behind it, the latter a regression over 149 measured points that it meets within 9 %: launches and tile rounds, K steps of
+// the pair or the tile kernel with few and with all SMs busy, of the shrink; and for up to 128 rank rows and 4096 columns of x where a
+// CTA of an ungrouped cluster has no more tiles than the CTAs of the other two, or one more over at most 1024 columns of x. Over 156 points (12
+// projections, 64 to 4500 rows of up to eight prompts) the choice of kernel and split loses 2.1 % to the best, the tiles alone, without groups of
+// columns, 12. us, the others / this: 2048 -> 2560, rank 64, 64, 300 rows 18.7 / 12.9, 19.6 / 17.7; 6144 -> 2048 64, 300 and 600 rows 40 / 27, 40 / 32,
+// 40 / 36; 1024 -> 8192, rank 32, 64, 300, 1000 rows 13.3 / 10.0, 15.5 / 13.2, 24.8 / 21.9; 4096 -> 1024 300, 1700, 4001 rows 26.6 / 22.3, 32.2 / 26,
+// 38.6 / 35.8. The others keep 2048 -> 12288, rank 64 (of 2000 rows 89 / 117) and 6144 -> 2048 from 1000 rows on.
 inline bool prefill_cluster_linear_ok(const LinearProblem& p, PcArgs* plan) {
   const SgmvProblem& b = p.lora;
   int n = 0;
@@ -519,12 +520,20 @@ inline bool prefill_cluster_linear_ok(const LinearProblem& p, PcArgs* plan) {
     if (b.st.col[s] % 16 != 0 || b.st.out[s] % 16 != 0) return false;  // (the MMAs of a slice would reach into the next one)
     ++n;
   }
-  PcArgs& a = *plan;
-  if (ceil_div_i(b.T, kSgmvBM) > kTileSMs || !sgmv_supported(b, nullptr) || !prefill_cluster_plan(b, n, p.n_total, true, &a)) return false;
-  const int nk = b.in_dim / kSgmvBK, tiles = ceil_div_i(a.cta_cols, a.tile_cols), total = ceil_div_i(b.T, kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
-  const int64_t pair_tiles = (int64_t)ceil_div_i(b.T, 2 * kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
-  const int rounds = pair_tiles >= kPairMinTiles ? ceil_div_i((int)pair_tiles, kTileSMs / 2) : ceil_div_i(total, kTileSMs);
-  return n * b.r_max <= 128 && b.in_dim <= 4096 && ((tiles <= rounds && tiles <= 3) || (tiles <= 2 && (tiles - rounds) * nk <= 16));
+  double here;
+  if (ceil_div_i(b.T, kSgmvBM) > kTileSMs || !sgmv_supported(b, nullptr) || !prefill_cluster_plan(b, n, p.n_total, true, plan, &here)) return false;
+  const int nk = b.in_dim / kSgmvBK, blocks = ceil_div_i(b.T, kSgmvBM), tiles = blocks * ceil_div_i(p.n_total, kSgmvBN);
+  const int pair_tiles = ceil_div_i(b.T, 2 * kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
+  const bool pairs = pair_tiles >= kPairMinTiles;
+  const int rounds = pairs ? ceil_div_i(pair_tiles, kTileSMs / 2) : ceil_div_i(tiles, kTileSMs);
+  int parts = 1;  // K parts of the shrink
+  while (parts < 8 && blocks * parts * 2 <= kTileSMs && ceil_div_i(nk, 2 * parts) * (2 * parts - 1) < nk) parts *= 2;
+  const double busy = pairs ? ceil_div_i(pair_tiles, rounds) / (kTileSMs / 2.0) : ceil_div_i(tiles, rounds) / (double)kTileSMs;
+  const double others = 7.4 + rounds * (1.25 + nk * (pairs ? 0.243 + 0.146 * busy : 0.223 + 0.262 * busy)) + 0.2 * ceil_div_i(nk, parts) + 0.02 * n * b.r_max;
+  int ck = 1;  // the cluster without groups: tiles of its CTAs
+  while (ck < 8 && blocks <= clusters_resident(2 * ck) && ceil_div_i(nk, 2 * ck) * (2 * ck - 1) < nk) ck *= 2;
+  const int own = ceil_div_i(ceil_div_i(p.n_total, 64 * ck), kSgmvBN / 64);
+  return here < 0.95 * others || (n * b.r_max <= 128 && b.in_dim <= 4096 && ((own <= rounds && own <= 3) || (own <= 2 && (own - rounds) * nk <= 16)));
 }
 
 // y = x . W^T (+ bias) + LoRA delta, the delta accumulated into the GEMM's TMEM accumulator.

@@ -30,7 +30,8 @@ namespace b200lora {
 constexpr int kPcThreads = 320;   // warp 0 TMA, warp 1 MMA + TMEM owner, warps 2-9 epilogue
 constexpr int kPcEpi = 256;
 constexpr int kPcShrinkStages = 12;
-constexpr int kPcTileStages = 4;
+constexpr int kPcTileStages = 4;   // ADD
+constexpr int kPcMaxTileStages = 8;
 constexpr int kPcSmem = 224 * 1024;
 constexpr int kPcBox = 64;        // rows of a W or lora_B box
 
@@ -71,7 +72,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   __shared__ int16_t s_slot[kSgmvBM], run_slot[kSgmvBM];
   __shared__ uint8_t run_lo[kSgmvBM], run_hi[kSgmvBM];
   __shared__ int nruns_s;
-  __shared__ __align__(8) uint64_t bar_words[2 * kPcShrinkStages + 2 * kPcTileStages + 9];
+  __shared__ __align__(8) uint64_t bar_words[2 * kPcShrinkStages + 2 * kPcMaxTileStages + 9];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_flag;
 
@@ -97,8 +98,8 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   auto s_full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
   auto s_empty = [&](int s) { return bar0 + 8u * (uint32_t)(kPcShrinkStages + s); };
   auto t_full = [&](int s) { return bar0 + 8u * (uint32_t)(2 * kPcShrinkStages + s); };
-  auto t_empty = [&](int s) { return bar0 + 8u * (uint32_t)(2 * kPcShrinkStages + kPcTileStages + s); };
-  const uint32_t bar1 = bar0 + 8u * (2 * kPcShrinkStages + 2 * kPcTileStages);
+  auto t_empty = [&](int s) { return bar0 + 8u * (uint32_t)(2 * kPcShrinkStages + kPcMaxTileStages + s); };
+  const uint32_t bar1 = bar0 + 8u * (2 * kPcShrinkStages + 2 * kPcMaxTileStages);
   auto acc_full = [&](int b) { return bar1 + 8u * (uint32_t)b; };
   auto acc_empty = [&](int b) { return bar1 + 16u + 8u * (uint32_t)b; };
   const uint32_t s_acc_full = bar1 + 32u, s_acc_empty = bar1 + 40u;
@@ -146,7 +147,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
     if (i == 0) {
       nruns_s = total;
       for (int s = 0; s < kPcShrinkStages; ++s) { mbar_init(s_full(s), 1); mbar_init(s_empty(s), 1); }
-      for (int s = 0; s < kPcTileStages; ++s) { mbar_init(t_full(s), 1); mbar_init(t_empty(s), 1); }
+      for (int s = 0; s < kPcMaxTileStages; ++s) { mbar_init(t_full(s), 1); mbar_init(t_empty(s), 1); }
       for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), kPcEpi / 32); }
       mbar_init(s_acc_full, 1);
       mbar_init(s_acc_empty, kPcEpi / 32);
@@ -201,8 +202,9 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
     const uint32_t leader = elect_one();
     int st = 0, round = 0;
     // lora_A of the first stages is asked for ahead of the wait: no kernel that lets others start early writes slabs. (LINEAR launches
-    // of more than 1920 rows: x first, us with lora_A / x first, 1024 -> 1024 of 2500 rows 12.8 / 12.4, of 300 8.2 / 8.5.)
-    const int early = npass > 0 && (!kLinear || CK == 8) ? min(s_stages, nk) : 0;
+    // of more than 96 rows a block or fewer than eight K parts: x first, us with lora_A / x first, 1024 -> 1024 of 2500 rows 12.8 / 12.4, of 300
+    // 8.2 / 8.5.)
+    const int early = npass > 0 && (!kLinear || (CK == 8 && bm < 96)) ? min(s_stages, nk) : 0;
     for (int pi = 0; pi < npass; ++pi) {
       // (ADD: the partial sums of a pass lie where the ring is)
       if (!kLinear && pi > 0) mbar_wait_bounded(s_acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
@@ -536,93 +538,125 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
 // Clusters of 1, 2, 4 and 8 CTAs with an SM each that are resident at a time (what cudaOccupancyMaxActiveClusters says: the SMs
 // of a cluster lie in one GPC). One cluster more is a second wave.
 inline int clusters_resident(int ck) { return ck == 1 ? 148 : (ck == 2 ? 74 : (ck == 4 ? 33 : 15)); }
-// CTAs of a cluster (as many as are resident at once, every K part at least one K step), then the rows of a block that make as
-// many clusters as are resident (at least 64: every block reads its adapters again).
-inline void prefill_cluster_split(int T, int in_dim, PcArgs* a) {
-  const int nk = in_dim / kSgmvBK;
-  a->ck = 1;
-  while (a->ck < 8 && ceil_div_i(T, kSgmvBM) <= clusters_resident(2 * a->ck) && ceil_div_i(nk, 2 * a->ck) * (2 * a->ck - 1) < nk) a->ck *= 2;
-  a->bm = std::min(kSgmvBM, std::max(64, round_up_i(ceil_div_i(T, clusters_resident(a->ck)), 8)));
-  a->groups = 1;
-}
-
-// Slices (of those in a) that a range of the columns touches, at most
-inline int prefill_cluster_need(const PcArgs& a, int n, int group_cols, int groups) {
+// Slices that one of the groups of `group_cols` columns touches, at most (a group with more than one holds the first column of one)
+inline int prefill_cluster_need(const PcArgs& a, int n, int group_cols) {
   int most = 1;
-  for (int g = 0; g < groups; ++g) {
+  for (int k = 1; k < n; ++k) {
+    const int lo = a.col[k] / group_cols * group_cols, hi = lo + group_cols;
     int here = 0;
-    for (int s = 0; s < n; ++s) here += a.col[s] < (g + 1) * group_cols && a.col[s] + a.out[s] > g * group_cols;
+    for (int s = 0; s < n; ++s) here += a.col[s] < hi && a.col[s] + a.out[s] > lo;
     most = std::max(most, here);
   }
   return most;
 }
 
-// ADD launches: runs of a block that share a pass over x (`width` rank rows each): sums in 512 TMEM columns, two stages of the ring
-inline int prefill_cluster_runs(int width, int ring) {
+// Runs of a block that share a pass over x (`width` rank rows each). ADD: sums in 512 TMEM columns, two stages of the ring; LINEAR: in
+// 256, lora_A tiles where a stage has its W tile.
+inline int prefill_cluster_runs(bool linear, int width, int room) {
   int runs = 1;
   for (int g = 2; g <= 4; ++g)
-    if (g * width <= 512 && ring / (kSgmvBM * kSgmvBK * 2 + g * width * kSgmvBK * 2) >= 2) runs = g;
+    if (linear ? g * width <= kSgmvBN && g * width * kSgmvBK * 2 <= room : g * width <= 512 && room / (kSgmvBM * kSgmvBK * 2 + g * width * kSgmvBK * 2) >= 2)
+      runs = g;
   return runs;
 }
 
-// ADD launches: K parts (the CTAs of a cluster), groups of columns and rows of a block, out of those whose clusters are resident at
-// once. The least of a sum in us: the K loop at 70 KB a us, the exchange, the output tiles, less than half of the SMs (the launch
-// behind then sets itself up beside this one), passes over x that fewer than four runs can share. A fit to 210 measured points (15
-// projections, 1024- and 2048-wide, rank 16 to 64; 200 to 11000 rows of up to eight prompts, every K split with 1 to 16 groups): it
-// loses 0.9 % to the best split of each, at most 17; one group and the largest K split 10.3. us, that / the split taken: 2048 ->
-// 2 x 6144, rank 64, 300, 700, 2000, 4000 rows 22.5 / 13.6, 22.0 / 15.1, 29.5 / 27.9, 51.9 / 47.2; 2048 -> 2560 300 and 700 20.0 / 12.6,
-// 19.4 / 15.4; 1024 -> 1024, rank 32, 300 and 2000 7.9 / 7.4, 8.8 / 8.8. (A CTA's tiles, 1.1 us each, were half of the time where a
-// block had one cluster: with groups a block can be 128 rows high and its columns still go to 16 CTAs and more.)
-inline void prefill_cluster_add_split(int T, int in_dim, int n, int n_total, int r, PcArgs* a) {
+// LINEAR: bytes of a stage and stages of its ring (of which at least three and one output buffer of each epilogue set must fit; 0 if not)
+inline int prefill_cluster_linear_stages(int tile_cols, int width, int off_tmp, int out_buf, int* stage_bytes) {
+  *stage_bytes = kSgmvBM * kSgmvBK * 2 + std::max(tile_cols, width) * kSgmvBK * 2;
+  if (width > kSgmvBN || off_tmp - 3 * *stage_bytes < 2 * out_buf) return 0;
+  int stages = 3;
+  while (stages < kPcMaxTileStages && off_tmp - (stages + 1) * *stage_bytes >= 4 * out_buf) ++stages;
+  return stages;
+}
+
+// K parts (the CTAs of a cluster), groups of columns and rows of a block: of those splits whose clusters are resident at once, the one
+// of the least time in us, which is returned (negative: none fits). `in_groups`: the slices lie one behind the other.
+//   ADD: a sum of the K loop at 70 KB a us, the exchange, the output tiles, less than half of the SMs (the launch behind then sets itself
+//   up beside this one), passes over x that fewer than four runs can share. A fit to 210 measured points (15 projections, 1024- and
+//   2048-wide, rank 16 to 64; 200 to 11000 rows of up to eight prompts, every K split with 1 to 16 groups): it loses 0.9 % to the best
+//   split of each, at most 17; one group and the largest K split 7.1. us, that / the split taken: 2048 -> 2 x 6144, rank 64, 300, 700, 2000,
+//   4000 rows 22.5 / 13.6, 22.0 / 15.1, 29.5 / 27.9, 51.9 / 47.2; 2048 -> 2560 300 and 700 20.0 / 12.6, 19.4 / 15.4; 1024 -> 1024, rank 32,
+//   300 and 2000 7.9 / 7.4, 8.8 / 8.8. (A CTA's tiles, 1.1 us each, were half of the time where a block had one cluster: with groups a
+//   block can be 128 rows high and its columns still go to 16 CTAs and more.)
+//   LINEAR: set-up, the shrink's steps (more where one or two runs share a pass), the base product's (their latency over the stages of
+//   the ring, then the bytes that all CTAs take), the exchange, the tiles: a regression over 3820 measured splits (12 projections as
+//   above, 64 to 4500 rows) that meets them within 8 %. Below that the sum does not tell, so the most K parts with one group stay
+//   unless another split promises 13 % less.
+inline double prefill_cluster_split(bool linear, bool in_groups, int T, int in_dim, int n, int n_total, int r, PcArgs* a) {
   const int nk = in_dim / kSgmvBK;
-  double least = 0.0;
-  a->ck = 0;
+  double least = -1.0, one_group = -1.0;
+  int one_group_ck = 0, one_group_bm = 0;
   for (int ck = 1; ck <= 8; ck *= 2) {
-    if (ck > 1 && ceil_div_i(nk, ck) * (ck - 1) >= nk) break;  // every K part at least one step
-    for (int groups = 1; groups <= clusters_resident(ck) && 64 * ck * groups <= std::max(n_total, 64 * ck); ++groups) {
-      const int group_cols = round_up_i(ceil_div_i(n_total, groups), 64);
-      if (group_cols * (groups - 1) >= n_total) continue;
+    const int nk_part = ceil_div_i(nk, ck);
+    if (ck > 1 && nk_part * (ck - 1) >= nk) break;  // every K part at least one step
+    // columns of a CTA in units of 64: all, then fewer and fewer, in about ten sizes
+    int last = 0;
+    for (int unit = ceil_div_i(n_total, 64 * ck); unit >= 1; unit = unit > 4 ? (unit + 1) * 3 / 4 : unit - 1) {
+      const int groups = unit * ck * 64 >= n_total ? 1 : ceil_div_i(n_total, unit * ck * 64);
+      if (groups == last) continue;
+      if (groups > clusters_resident(ck) || (groups > 1 && !in_groups)) break;
+      last = groups;
       const int bm = std::max(64, round_up_i(ceil_div_i(T, clusters_resident(ck) / groups), 8)), rows = std::min(bm, kSgmvBM);
       if (bm > kSgmvBM && (ck > 1 || groups > 1)) break;
-      const int width = prefill_cluster_need(*a, n, group_cols, groups) * r, cols = round_up_i(ceil_div_i(group_cols, ck), 64);
-      const double cost = ceil_div_i(nk, ck) * (rows + width) * (kSgmvBK * 2 / 70e3) + 0.05 * rows * width * 4 / 1024 + 0.35 * ceil_div_i(cols, kSgmvBN) +
-                          0.1 * cols / kSgmvBN + (ck * groups * ceil_div_i(T, rows) > 74 ? 0.3 : 0.0) +
-                          3.0 * (4 - prefill_cluster_runs(width, kPcSmem - width * kSgmvBM * 2));
-      if (a->ck == 0 || cost < least) {
+      const int group_cols = groups > 1 ? round_up_i(ceil_div_i(n_total, groups), 64) : n_total;
+      if (group_cols * (groups - 1) >= n_total) continue;
+      const int width = (groups > 1 ? prefill_cluster_need(*a, n, group_cols) : n) * r, off_tmp = kPcSmem - width * kSgmvBM * 2;
+      const int cols = round_up_i(ceil_div_i(group_cols, ck), 64), tiles = ceil_div_i(cols, kSgmvBN), tile_cols = round_up_i(ceil_div_i(cols, tiles), 64);
+      const int ctas = ck * groups * ceil_div_i(T, rows);
+      const double exchange = rows * width * 4 / 1024.0;
+      double cost;
+      if (linear) {
+        int stage;
+        const int stages = prefill_cluster_linear_stages(tile_cols, width, off_tmp, rows * kGemmOutChunk * 2, &stage);
+        if (stages == 0) continue;
+        const int runs = prefill_cluster_runs(true, width, std::max(tile_cols, width) * kSgmvBK * 2);
+        const double high = (double)rows / kSgmvBM, kb = (rows + tile_cols) * 0.128;
+        cost = 3.6 + nk_part * (0.27 + high * (0.06 + (runs == 1 ? 0.44 : runs == 2 ? 0.1 : 0.0))) +
+               tiles * nk * (0.042 + 0.87 / stages + kb * (0.0009 + 0.0015 * ctas / 148)) + 0.044 * exchange + tiles * (0.28 + 0.65 * tile_cols / kSgmvBN * high);
+      } else {
+        cost = nk_part * (rows + width) * (kSgmvBK * 2 / 70e3) + 0.05 * exchange + 0.35 * tiles + 0.1 * cols / kSgmvBN + (ctas > 74 ? 0.3 : 0.0) +
+               3.0 * (4 - prefill_cluster_runs(false, width, off_tmp));
+      }
+      if (groups == 1) { one_group = cost; one_group_ck = ck; one_group_bm = rows; }  // (the most K parts come last)
+      if (least < 0.0 || cost < least) {
         least = cost;
-        a->ck = ck; a->groups = groups; a->bm = rows;
+        a->ck = ck; a->groups = groups; a->bm = rows; a->group_cols = group_cols;
       }
     }
   }
+  if (linear && one_group >= 0.0 && least > 0.87 * one_group) {
+    least = one_group;
+    a->ck = one_group_ck; a->groups = 1; a->bm = one_group_bm; a->group_cols = n_total;
+  }
+  return least;
 }
 
 // bytes of the partial sums that a CTA gets of `cols` columns
 inline int prefill_cluster_part_bytes(const PcArgs& a, int cols) { return a.ck * ceil_div_i(cols / 8, a.ck) * 8 * a.bm * 4; }
 
 // Split, tiles and shared memory (ring of the tiles, output buffers, the intermediate as MMA operand; ADD launches shrink through a
-// ring over the first two) of a problem with `n` slices; false: too many rank rows for them.
-inline bool prefill_cluster_plan(const SgmvProblem& b, int n, int n_total, bool linear, PcArgs* a) {
-  for (int s = 0, k = 0; s < b.st.n; ++s)
-    if (b.st.out[s] > 0) { a->out[k] = b.st.out[s]; a->col[k] = b.st.col[s]; ++k; }
-  if (linear) prefill_cluster_split(b.T, b.in_dim, a);
-  else prefill_cluster_add_split(b.T, b.in_dim, n, n_total, b.r_max, a);
-  a->group_cols = a->groups > 1 ? round_up_i(ceil_div_i(n_total, a->groups), 64) : n_total;
-  const int need = a->groups > 1 ? prefill_cluster_need(*a, n, a->group_cols, a->groups) : n;
+// ring over the first two) of a problem with `n` slices; false: too many rank rows for them. `time`: what the split is expected to take.
+inline bool prefill_cluster_plan(const SgmvProblem& b, int n, int n_total, bool linear, PcArgs* a, double* time = nullptr) {
+  bool in_groups = true;  // slices that cover the columns one behind the other
+  for (int s = 0, k = 0, pos = 0; s < b.st.n; ++s)
+    if (b.st.out[s] > 0) {
+      in_groups = in_groups && b.st.col[s] == pos;
+      pos += b.st.out[s];
+      a->out[k] = b.st.out[s]; a->col[k] = b.st.col[s]; ++k;
+      if (k == n) in_groups = in_groups && pos == n_total;
+    }
+  const double cost = prefill_cluster_split(linear, in_groups, b.T, b.in_dim, n, n_total, b.r_max, a);
+  if (cost < 0.0) return false;
+  if (time != nullptr) *time = cost;
   a->cta_cols = round_up_i(ceil_div_i(a->group_cols, a->ck), 64);
   a->tile_cols = round_up_i(ceil_div_i(a->cta_cols, ceil_div_i(a->cta_cols, kSgmvBN)), 64);
-  const int width = need * b.r_max, tmp_bytes = need * kSgmvBM * b.r_max * 2, out_buf = a->bm * kGemmOutChunk * 2;
-  a->off_tmp = kPcSmem - tmp_bytes;
-  a->gmax = 1;
+  const int width = (a->groups > 1 ? prefill_cluster_need(*a, n, a->group_cols) : n) * b.r_max, out_buf = a->bm * kGemmOutChunk * 2;
+  a->off_tmp = kPcSmem - width * kSgmvBM * 2;
   if (linear) {
     // stages of an x and a W tile (or, ahead of the tiles, of the lora_A tiles of up to gmax runs), then output buffers
-    a->stages = 3;
-    const int b_tiles = std::max(a->tile_cols, width) * kSgmvBK * 2;
-    while (a->gmax < 4 && (a->gmax + 1) * width <= kSgmvBN && (a->gmax + 1) * width * kSgmvBK * 2 <= b_tiles) ++a->gmax;
-    a->stage_bytes = kSgmvBM * kSgmvBK * 2 + b_tiles;
-    if (a->off_tmp - 4 * a->stage_bytes >= 4 * out_buf) a->stages = 4;
-    const int room = a->off_tmp - a->stages * a->stage_bytes;
-    if (width > kSgmvBN || room < 2 * out_buf) return false;
-    a->out_bufs = std::min(2, room / (2 * out_buf));
+    a->stages = prefill_cluster_linear_stages(a->tile_cols, width, a->off_tmp, out_buf, &a->stage_bytes);
+    a->gmax = prefill_cluster_runs(true, width, a->stage_bytes - kSgmvBM * kSgmvBK * 2);
+    a->out_bufs = std::min(2, (a->off_tmp - a->stages * a->stage_bytes) / (2 * out_buf));
     a->part_cols = width;
     while (prefill_cluster_part_bytes(*a, a->part_cols) > 2 * a->out_bufs * out_buf) a->part_cols -= 16;  // (16 always fit)
   } else {
@@ -630,7 +664,7 @@ inline bool prefill_cluster_plan(const SgmvProblem& b, int n, int n_total, bool 
     a->stage_bytes = a->tile_cols * b.r_max * 2;
     a->out_bufs = 2;
     while (a->stages > 2 && a->off_tmp - a->stages * a->stage_bytes < 2 * a->out_bufs * out_buf) --a->stages;
-    a->gmax = prefill_cluster_runs(width, a->off_tmp);
+    a->gmax = prefill_cluster_runs(false, width, a->off_tmp);
     a->part_cols = width;
   }
   a->off_out = a->stages * a->stage_bytes;

@@ -128,13 +128,17 @@ LINEAR = [
     (2200, 1024, [640, 640], 4, 64, 500),        # clusters of 4, two tiles a CTA
     (4300, 128, [512], 4, 16, 128),              # clusters of 2
     (517, 1024, [320], 3, 16, 4),                # many passes, CTAs that own no rank columns
+    (70, 512, [1024, 320, 192], 3, 64, 20),      # groups of columns, of one to three slices
+    (40, 2048, [960, 960], 4, 32, 9),            # four groups, a tile of 64 columns a CTA, seven stages
+    (200, 1024, [2048, 1088], 4, 32, 60),        # four groups, the last one narrower
+    (64, 1024, [1008], 2, 16, 0),                # ragged columns, partial sums of one piece
 ]
 
 
 @pytest.mark.parametrize("case", range(len(LINEAR)))
 def test_linear_of_the_cluster_kernel_matches_oracle(case):
     T, in_dim, outs, S, r, longest = LINEAR[case]
-    slots = by_runs(T, S, longest, 50 + case)
+    slots = by_runs(T, S, longest, 50 + case) if longest else torch.ones(T, dtype=torch.int32)
     slots[0] = 0
     p = W.make_projection(800 + case, T, in_dim, outs, S, r, token_to_slot=slots, with_weight=True)
     d = p.to_device(DEV)
