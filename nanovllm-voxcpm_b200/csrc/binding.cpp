@@ -578,13 +578,13 @@ struct Projection {
 // rows gate_up with the activation (940 GFLOP) 2131 / 2318, down (470) 2131 / 2244, o (134) 2131 / 2186; 2000 rows 1020 / 1093,
 // 1020 / 1063, 1029 / 1048; 1000 rows 540 / 516 (235), 540 / 547 (118), 540 / 541 (34). 2048-wide down (6144 columns): 4000 rows
 // (101) 692 / 705, 2000 rows (50) 355 / 348; its gate_up (2048 columns, 201 and 101) 692 / 651 and 355 / 323.
-// Up to 1024 input columns one launch (prefill_cluster_kernel with groups of columns) wins at every number of rows: us, cuBLAS + add /
+// Around 1024 input columns one launch (prefill_cluster_kernel with groups of columns) wins from 128 rows on (fewer not measured): us, cuBLAS + add /
 // fused, rank 32: 1024 -> 1280 of 128, 300, 1100, 2700 rows 9.3 / 9.1, 11.0 / 9.4, 14.5 / 11.9, 22.9 / 15.9; 1024 -> 1024 8.4 / 7.6, 8.9 / 7.9, 10.7 /
 // 10.1, 17.1 / 12.8; 1024 -> 8192 13.0 / 11.4, 16.4 / 13.6, 34.2 / 23.1; steps of 3 layers of 1024, 128, 300, 1000 rows 251 / 229, 274 / 237, 329 / 310.
 // (2048 -> 2048 12.1 / 12.5, 13.1 / 14.7, 17.3 / 19.1; 4096 -> 1024 14.9 / 19.5, 15.5 / 21.3, 20.1 / 24.) Not rank 16, whose intermediate the
 // add of a small batch keeps as two numbers.
 inline bool fused_linear_wins(int64_t T, int64_t K, int64_t N, int64_t r, bool silu) {
-  if (!silu && K <= 1024 && r > 16) return true;
+  if (!silu && K >= 768 && K <= 1024 && T >= 128 && r > 16) return true;
   return (T + 127) / 128 * ((N + 255) / 256) >= (N <= 1536 ? 45 : 100) && (K < 4096 || 2.0 * (double)T * (double)K * (double)N < (silu ? 300e9 : 60e9));
 }
 
