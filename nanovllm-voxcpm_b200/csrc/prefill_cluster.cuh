@@ -573,7 +573,7 @@ inline int prefill_cluster_linear_stages(int tile_cols, int width, int off_tmp, 
 // of the least time in us, which is returned (negative: none fits). `in_groups`: the slices lie one behind the other.
 //   ADD: a sum of the K loop at 70 KB a us, the exchange, the output tiles, less than half of the SMs (the launch behind then sets itself
 //   up beside this one), passes over x that fewer than four runs can share. A fit to 210 measured points (15 projections, 1024- and
-//   2048-wide, rank 16 to 64; 200 to 11000 rows of up to eight prompts, every K split with 1 to 16 groups): it loses 0.9 % to the best
+//   2048-wide, rank 16 to 64; 200 to 11000 rows of up to eight prompts, every K split with 1 to 16 groups): it loses 1.0 % to the best
 //   split of each, at most 17; one group and the largest K split 7.1. us, that / the split taken: 2048 -> 2 x 6144, rank 64, 300, 700, 2000,
 //   4000 rows 22.5 / 13.6, 22.0 / 15.1, 29.5 / 27.9, 51.9 / 47.2; 2048 -> 2560 300 and 700 20.0 / 12.6, 19.4 / 15.4; 1024 -> 1024, rank 32,
 //   300 and 2000 7.9 / 7.4, 8.8 / 8.8. (A CTA's tiles, 1.1 us each, were half of the time where a block had one cluster: with groups a
