@@ -567,7 +567,10 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     bp.kind = 0;
     bp.mode = 3;
     bp.token_to_slot = token_to_slot;
-    const bool decode_like = T < 32 * n_buckets || !prefill_sized(T, st, r_max, in_dim, true, one_launch);
+    // (Without bucket arrays, or at rank 16, which the bucket kernel cannot overwrite, a batch that is its own takes a fill and an add.)
+    const bool bucket_form = have_buckets && r_max % 32 == 0;
+    const bool prefill = prefill_sized(T, st, r_max, in_dim, true, one_launch) || (!bucket_form && one_launch && ceil_div_i(T, kBgmvTok) > 74);
+    const bool decode_like = T < 32 * n_buckets || !prefill;
     if (dtype == B200_LORA_BF16 && have_buckets &&
         (impl == B200_LORA_IMPL_BGMV || (auto_impl && decode_like)) && bgmv_plan(bp, &plan, nullptr))
       return bgmv_launch(plan, st_);

@@ -119,6 +119,19 @@ def test_auto_takes_the_kernel_of_the_line(T, in_dim, outs, r, prefill):
     assert torch.equal(run(N.IMPL_AUTO), by_name[prefill])
 
 
+def test_auto_overwrites_with_the_prefill_kernel_at_rank_16():
+    """1300 rows: an add of this size is the bucket kernel's, which cannot overwrite at rank 16."""
+    T, outs = 1300, [1024]
+    slots = torch.arange(T, dtype=torch.int32) * 4 // T
+    p = W.make_projection(750, T, 1024, outs, 4, 16, token_to_slot=slots)
+    d = p.to_device(DEV)
+    y = [d.y.clone(), d.y.clone()]
+    for out, impl in zip(y, (N.IMPL_AUTO, N.IMPL_SGMV)):
+        LORA.launch_add(out, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata(slots), 0.5, impl=impl, overwrite=True)
+    torch.cuda.synchronize()
+    assert N.device_status(reset=True) == 0 and torch.equal(*y)
+
+
 # T, in, outs, S, r, longest run: fused linears of the kernel (the plan's lines: one tile a CTA, one more over 1024 columns of x)
 LINEAR = [
     (7, 64, [48], 2, 16, 3),                     # less than a tile of columns, some CTAs without any
