@@ -54,7 +54,7 @@ constexpr int kBgmvKP = 1024;          // columns per shrink tile
 constexpr int kBgmvXBlocks = kBgmvKP / 32 / kBgmvWarps;  // 32-column blocks per warp and tile
 constexpr int kBgmvSmemMax = 232448;   // 227 KB opt-in maximum per CTA
 constexpr int kBgmvMaxStages = 12;
-constexpr int kBgmvMaxExpandTiles = 256;  // expand tiles of one CTA (entries of its tile table)
+constexpr int kBgmvMaxExpandTiles = 256;  // expand tiles of one CTA (its table has up to eight blocks of each)
 
 
 // Optional phase timeline (SM clock) of rank-0 CTAs, compiled in only for tuning builds.
@@ -429,33 +429,46 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   if (tok_lo >= p.T) tok_lo = -1;
   if (tok_hi >= p.T) tok_hi = -1;
 
-  // Expand tile e of this CTA (ring order): x = first y column, y = rows | slice << 16 | first warp << 20. A warp takes 32 rows
-  // of a tile. The tiles are dealt to the warps one behind the other, so that tiles of fewer than 256 rows are multiplied side by
-  // side; with all tiles from warp 0 on, k and v cost a step each while seven warps waited (us a launch, before / now: 1024-wide,
-  // rank 32, qkv of 256 rows over 32 adapters 4.58 / 4.24, of 4 rows 2.96 / 2.57; rank 64, a step of two tiles with every warp
-  // waiting for both: 2048-wide, 48 over 64, gate_up 12.4 / 11.7; 4096-wide, 512 over 88, o 29.5 / 25.2).
+  // Expand rows of this CTA in blocks of 32 (ring order), dealt to the warps in turn: warp w multiplies blocks w, w + 8, ..., so that
+  // tiles of fewer than 256 rows are multiplied side by side. (With every tile from warp 0 on, k and v cost a step each while seven
+  // warps waited; us a launch, before / now: 1024-wide, rank 32, qkv of 256 rows over 32 adapters 4.58 / 4.24, of 4 rows 2.96 / 2.57;
+  // rank 64, a step of two tiles with every warp waiting for both: 2048-wide, 48 over 64, gate_up 12.4 / 11.7; 4096-wide, 512 over
+  // 88, o 29.5 / 25.2.)
+  // Kind 0: a table of the tiles, x = first y column, y = rows | slice << 16 | warp of the first block << 20. Kinds 1 and 2 ask for a
+  // block's y while they multiply the block before, which may lie several tiles back: a table of the blocks, x = first y column, y =
+  // rows | slice << 8 | block of its tile << 12 | tile << 16. (Asked for a tile ahead, the y of narrow slices, at ranks above 32 all
+  // of it, came late: us a layer, by tile / by block: fp16, rank 64, 128 rows over 32 adapters, 1024-wide 36.8 / 34.5, 4096-wide 90.5
+  // / 83.7; bf16, rank 48, 256 rows 34.6 / 30.5; rank 16, 37 rows 13.3 / 12.8. Kind 0 with the longer table loses up to 1 %.)
   int2* etab = reinterpret_cast<int2*>(smem + p.off_tab);
+  int entries = tiles_exp;
+  if (kPrecise) {
+    entries = 0;
+#pragma unroll
+    for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) entries += (e_n[s] + 31) >> 5;
+  }
 #pragma unroll 1
-  for (int e = tid; e < tiles_exp; e += kBgmvConsumers) {
-    int s_e = 0, et = e;
+  for (int i = tid; i < entries; i += kBgmvConsumers) {
+    int s_e = 0, r0 = kPrecise ? i << 5 : i << p.er_shift, tile = 0, blocks = 0;  // slice, first row in it; tiles and blocks of those before
 #pragma unroll
     for (int s = 0; s < B200_LORA_MAX_SLICES - 1; ++s)
-      if (s_e == s && et >= e_tiles[s]) { et -= e_tiles[s]; s_e = s + 1; }
-    int lo = 0, en = 0, cb = 0, blocks = 0;
+      if (s_e == s && r0 >= e_n[s]) {
+        r0 -= kPrecise ? (e_n[s] + 31) & ~31 : e_tiles[s] << p.er_shift;
+        tile += e_tiles[s];
+        blocks += (e_n[s] + 31) >> 5;
+        s_e = s + 1;
+      }
+    int lo = 0, en = 0, cb = 0;
 #pragma unroll
-    for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) {
-      if (s < s_e) blocks += (e_n[s] + 31) >> 5;
+    for (int s = 0; s < B200_LORA_MAX_SLICES; ++s)
       if (s == s_e) { lo = e_lo[s]; en = e_n[s]; cb = p.st.col[s]; }
-    }
-    const int r0 = et << p.er_shift;
-    blocks += r0 >> 5;
-    etab[e] = make_int2(cb + lo + r0, min(ER, en - r0) | (s_e << 16) | ((blocks & (kBgmvWarps - 1)) << 20));
+    if (kPrecise)
+      etab[i] = make_int2(cb + lo + r0, min(32, en - r0) | (s_e << 8) | (((r0 & (ER - 1)) >> 5) << 12) | ((tile + (r0 >> p.er_shift)) << 16));
+    else
+      etab[i] = make_int2(cb + lo + r0, min(ER, en - r0) | (s_e << 16) | (((blocks + (r0 >> 5)) & (kBgmvWarps - 1)) << 20));
   }
-  if (tid == 0) etab[tiles_exp] = make_int2(0, 0);  // (nobody has rows of the one behind the last)
+  if (kPrecise && tid < kBgmvWarps) etab[entries + tid] = make_int2(0, -65536);  // (no rows, of no tile: behind the last block of a warp)
   named_bar_sync(1, kBgmvConsumers);  // table complete
 
-  // expand: first row of this warp's block of a tile; it has one if that row is one of the tile's
-  auto block_row = [&](int2 te) { return ((warp - (te.y >> 20)) & (kBgmvWarps - 1)) * 32; };
   const int x_col = warp * 32 + t * 8;  // shrink: first column of the thread inside a K part (block i adds 256)
   if (p.use_pdl) {
 #pragma unroll 1
@@ -508,19 +521,19 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
 
   __nv_bfloat16* const ylo_p = p.y + (int64_t)max(tok_lo, 0) * p.y_ld + 8 * t;  // + first column of the warp's block
   __nv_bfloat16* const yhi_p = p.y + (int64_t)max(tok_hi, 0) * p.y_ld + 8 * t;
-  // kinds 1 and 2: y of the next tile is requested while this one is multiplied, the first one behind the shrink
+  // kinds 1 and 2: y of a warp's next block is requested while it multiplies the one before, the first one behind the shrink
   // (its 0.5 us of latency then lie beside the exchange: 37 rows, rank 16 74.1 -> 70.9 us a layer stack, 64 rows fp16 43.5 -> 40.7; before the
   // shrink it delays the x loads: 76.0 and 45.0)
   uint4 y_next[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-  auto load_y = [&](int2 te) {
+  auto load_y = [&](int2 block) {
     if (kF32Out || (kMode == 2 && p.no_add)) return;
-    const int row = block_row(te), c0 = te.x + row;
-    if (row + 8 * t >= (te.y & 0xffff) || !B200_IN_BOUNDS(c0 >= 0 && c0 + 8 * t + 8 <= p.y_cols)) return;
-    if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + c0);
-    if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + c0);
+    if (8 * t >= (block.y & 0xff) || !B200_IN_BOUNDS(block.x >= 0 && block.x + 8 * t + 8 <= p.y_cols)) return;
+    if (tok_lo >= 0) y_next[0] = ldg128(ylo_p + block.x);
+    if (tok_hi >= 0) y_next[1] = ldg128(yhi_p + block.x);
   };
-  int2 tile_next = make_int2(0, 0);  // kinds 1 and 2: looked up a tile ahead, for its y
-  if (kPrecise) tile_next = etab[0];
+  const int2* block_at = etab + warp;
+  int2 block_next = make_int2(0, 0);  // of this warp
+  if (kPrecise) block_next = *block_at;
   const __nv_bfloat16* const xlo_p = p.x + (int64_t)max(tok_lo, 0) * p.x_ld + x_col;
   const __nv_bfloat16* const xhi_p = p.x + (int64_t)max(tok_hi, 0) * p.x_ld + x_col;
 
@@ -604,7 +617,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     }
   }
   B200_TRACE_POINT(6)
-  if (kPrecise) load_y(tile_next);
+  if (kPrecise) load_y(block_next);
 
   // ===== cross-warp reduction of the K slices, scale, bf16, all-gather =====
   named_bar_sync(1, kBgmvConsumers);
@@ -703,8 +716,8 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   // Rows of a block beyond the tile's rows hold stale bytes; their products land in columns that are not written.
   uint4 a_lo = make_uint4(0, 0, 0, 0), a_hi = a_lo;  // kind 0, ranks up to 32: the intermediate's fragments of the slice at hand
   int a_slice = -1;
-  auto expand_fn = [&](const int2 te, const int row, const uint4 y_lo, const uint4 y_hi) {
-    const int slice = (te.y >> 16) & 15;
+  // this warp's `rows` rows of slice `slice`, from row `row` of the tile on, into y from column c0 on
+  auto expand_fn = [&](const int c0, const int rows, const int slice, const int row, const uint4 y_lo, const uint4 y_hi) {
     float d[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.f;
@@ -745,8 +758,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
         for (int j = 0; j < 4; ++j) mma_16816<kF16>(d[j], alo.z, ahi.z, alo.w, ahi.w, w[j].z, w[j].w);
       }
     }
-    const int c0 = te.x + row;
-    if (row + 8 * t >= (te.y & 0xffff) || !B200_IN_BOUNDS(c0 >= 0 && c0 + 8 * t + 8 <= p.y_cols)) return;
+    if (8 * t >= rows || !B200_IN_BOUNDS(c0 >= 0 && c0 + 8 * t + 8 <= p.y_cols)) return;
     if (kF32Out) {
       float* const yf = reinterpret_cast<float*>(p.y) + c0 + 8 * t;
 #pragma unroll
@@ -786,14 +798,18 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
 #pragma unroll 1
   for (int e = 0; e < tiles_exp; ++e) {
     // (every warp waits for every tile: a wait that skipped phases of a stage could no longer tell them apart)
-    const int2 te = kPrecise ? tile_next : etab[e];
-    const int row = block_row(te);
+    const int2 te = kPrecise ? block_next : etab[e];
+    const int row = kPrecise ? ((te.y >> 12) & 7) * 32 : ((warp - (te.y >> 20)) & (kBgmvWarps - 1)) * 32;
+    const bool mine = kPrecise ? te.y >> 16 == e : row < (te.y & 0xffff);
     const uint4 y_lo = y_next[0], y_hi = y_next[1];
-    if (kPrecise) tile_next = etab[e + 1];
+    if (kPrecise && mine) block_next = *(block_at += kBgmvWarps);
     mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
     if (e < 10) { B200_TRACE_POINT(12 + 2 * e) }
-    if (kPrecise) load_y(tile_next);
-    if (row < (te.y & 0xffff)) expand_fn(te, row, y_lo, y_hi);
+    if (mine) {
+      if (kPrecise) load_y(block_next);
+      if (kPrecise) expand_fn(te.x, te.y & 0xff, (te.y >> 8) & 15, row, y_lo, y_hi);
+      else expand_fn(te.x + row, (te.y & 0xffff) - row, (te.y >> 16) & 15, row, y_lo, y_hi);
+    }
     if (e < 10) { B200_TRACE_POINT(13 + 2 * e) }
     __syncwarp();
     if (lane == 0) mbar_arrive_relaxed(empty_bar(c_stage));
@@ -947,10 +963,13 @@ inline bool bgmv_plan_cluster(const BgmvProblem& b, const SliceTable& st, int C,
   p.pitchT = round_up_i(Q * (b.kind != 0 ? 4 : 2), 128) + 64;
   const int tmp_bytes = round_up_i(kBgmvTok * p.pitchT, 128);
   const int bar_bytes = 256;
-  int exp_tiles = 0;
-  for (int s = 0; s < st.n; ++s) exp_tiles += ceil_div_i(p.oc[s], p.ER);
+  int exp_tiles = 0, exp_blocks = 0;
+  for (int s = 0; s < st.n; ++s) {
+    exp_tiles += ceil_div_i(p.oc[s], p.ER);
+    exp_blocks += p.oc[s] / 32;
+  }
   if (exp_tiles > kBgmvMaxExpandTiles) { *why = "too many expand tiles per CTA"; return false; }
-  const int tab_bytes = round_up_i((exp_tiles + 1) * 8, 128);
+  const int tab_bytes = round_up_i((b.kind != 0 ? exp_blocks + kBgmvWarps : exp_tiles) * 8, 128);
   p.ksplit = ksplit ? 1 : 0;
   p.pitchR = Q + 4;
   const int recv_bytes = ksplit ? round_up_i(C * kBgmvTok * p.pitchR * 4, 128) : 0;

@@ -72,6 +72,35 @@ def test_output_tiles_dealt_over_the_warps(outs, r, cluster, dtype):
     assert_lora_close(y, O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets), what=f"{outs} r{r}")
 
 
+@pytest.mark.parametrize("r, dtype", [(64, torch.float16), (128, torch.float16), (256, torch.float16), (48, torch.bfloat16), (80, torch.bfloat16)])
+@pytest.mark.parametrize("cluster", [2, 8])
+def test_a_warps_next_block_lies_several_tiles_ahead(r, dtype, cluster):
+    """Adds and expands that read y (fp16, bf16 at ranks that are no multiple of 32, ``lora_expand``) where tiles are 128, 64 and 32 rows
+    high: y of a warp's next block is asked for while it multiplies the one before, tiles of other warps lying between."""
+    T, S, outs = 21, 3, [1184, 96, 8]
+    p = W.make_projection(850 + r, T, 512, outs, S, r, dtype=dtype)
+    d = p.to_device(DEV)
+    y, y2 = d.y.clone(), d.y.clone()
+    km = LoRAKernelMeta.make(S, T, DEV)
+    km.prepare_tensors(d.token_to_slot)
+    args = km.meta_args(T, specialize_active_lora=True)
+    tmp = torch.zeros(len(outs), T, r, device=DEV, dtype=torch.float32)
+    N.set_option(N.OPT_CLUSTER, cluster)
+    try:
+        # (three slices of 256 ranks make 96 rank rows a CTA in clusters of eight, the kernel takes 64: one slice less)
+        k = 2 if r == 256 else 3
+        LORA.launch_add(y, d.x, d.a_slabs[:k], d.b_slabs[:k], d.out_sizes[:k], d.col_offsets[:k], metadata_for(p.token_to_slot, "graph", S), 1.0,
+                        impl=N.IMPL_BGMV)
+        lora_shrink(d.x, d.a_slabs, tmp, *args, 1.0)
+        lora_expand(tmp, d.b_slabs, y2, *args, offset_start=0, add_inputs=True)
+        torch.cuda.synchronize()
+    finally:
+        N.set_option(N.OPT_CLUSTER, 0)
+    assert N.device_status(reset=True) == 0
+    assert_lora_close(y, O.add_lora(p.y, p.x, p.a_slabs[:k], p.b_slabs[:k], p.token_to_slot, 1.0, p.col_offsets[:k]), what=f"add r{r}")
+    assert_lora_close(y2, O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, p.token_to_slot, 1.0, p.col_offsets), what=f"expand r{r}")
+
+
 @pytest.mark.parametrize("T, in_dim, outs, S, r, cluster", [
     (4, 6144, [2048], 8, 32, 8),           # eight CTAs although they lose the K split of six parts
     (4, 5120, [1280], 8, 32, 8),           # ... of five
