@@ -389,8 +389,9 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
         if (exchange > 0) named_bar_sync(2, kPcEpi);
         if (etid == 0) mbar_arrive_expect_tx(part_full, (uint32_t)((CK - 1) * rows * mine * 32));
         // Room for them: the K loop whose ring lies there is over; behind the first exchange, the sums of the one before have been read.
+        // (The arrival releases: a peer's stores may go there only behind these reads, which it learns of by acquiring.)
         if (!apart || exchange > 0) {
-          if (etid < CK) mbar_arrive_remote_relaxed(mapa_shared(part_ready, (uint32_t)etid));  // (nothing to publish: what lay there has been read)
+          if (etid < CK) mbar_arrive_remote_release(mapa_shared(part_ready, (uint32_t)etid));
           mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)((exchange - (apart ? 1 : 0)) & 1), &abort_flag);
         }
         // (A TMEM load is a warp-wide operation on one column range: a warp whose rows straddle two runs reads both runs' columns.)

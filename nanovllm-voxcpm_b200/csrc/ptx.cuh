@@ -39,12 +39,10 @@ __device__ __forceinline__ void mbar_arrive_relaxed(uint32_t bar) {
   asm volatile("mbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Arrive on an mbarrier of another CTA of the cluster (address from mapa_shared); the
-// release at cluster scope publishes this CTA's earlier distributed-shared-memory stores.
+// release at cluster scope publishes this CTA's earlier distributed-shared-memory stores, and orders its earlier reads
+// before what the other CTA writes once it has seen the arrival.
 __device__ __forceinline__ void mbar_arrive_remote_release(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_remote_relaxed(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;

@@ -165,3 +165,42 @@ def test_linear_of_the_cluster_kernel_matches_oracle(case):
     assert_lora_close(y, ref, max_abs=2e-2 + 2.0 ** -8 * float(ref.abs().max()), what="cluster linear")
     none = slots < 0
     assert torch.equal(y.cpu()[none].view(torch.int16), plain.cpu()[none].view(torch.int16)), "rows without adapter are the plain linear"
+
+
+# T, in, outs, r, longest run: eight K parts; the place of the partial sums is written again by every pass of a block (and by every
+# part of one)
+REPEATED = [
+    (995, 4096, [1024], 64, 5),                  # adds: sums where the K loop's ring was
+    (197, 2048, [2048, 256, 256], 32, 4),
+    (300, 2048, [1024], 32, 3),
+    (412, 1024, [1024, 128, 128], 64, 6),        # fused linear: rank rows in two parts a pass
+    (333, 1024, [1024, 128, 128], 32, 5),
+]
+
+
+@pytest.mark.parametrize("case", range(len(REPEATED)))
+def test_partial_sums_of_many_passes_are_the_same_every_time(case):
+    T, in_dim, outs, r, longest = REPEATED[case]
+    linear = case >= 3
+    slots = by_runs(T, 9, longest, 90 + case)
+    slots[0] = 0
+    p = W.make_projection(900 + case, T, in_dim, outs, 9, r, token_to_slot=slots, with_weight=linear)
+    d = p.to_device(DEV)
+    meta = metadata(slots)
+
+    def run():
+        if linear:
+            return LORA.linear_lora(d.x, d.weight, None, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, d.token_to_slot, 1.0)
+        y = d.y.clone()
+        LORA.launch_add(y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, meta, 1.0, impl=N.IMPL_SGMV)
+        return y
+
+    got = [run() for _ in range(30)]
+    torch.cuda.synchronize()
+    assert N.device_status(reset=True) == 0
+    for y in got[1:]:
+        assert torch.equal(y.view(torch.int16), got[0].view(torch.int16))
+    ref = (O.linear_lora(p.x, p.weight, None, p.a_slabs, p.b_slabs, p.col_offsets, slots) if linear
+           else O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, slots, 1.0, p.col_offsets))
+    # half a unit in the last place of the largest output, on top of the path's tolerance
+    assert_lora_close(got[0], ref, max_abs=2e-2 + 2.0 ** -8 * float(ref.abs().max()), what="many passes")
