@@ -65,6 +65,15 @@ __device__ __forceinline__ uint32_t swizzled_piece(int row, int c, int row_bytes
   return (uint32_t)(row * row_bytes + ((c ^ x) << 4));
 }
 
+// one arrival, when the MMAs issued so far are complete, at the barrier of this offset in each of the cluster's CTAs in `ctas`
+__device__ __forceinline__ void umma_commit_cluster_elected(uint32_t bar, uint16_t ctas, uint32_t leader) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t}"
+      ::"r"(bar), "r"(leader), "h"(ctas)
+      : "memory");
+}
+
 template <bool kLinear>
 __global__ void __launch_bounds__(kPcThreads, 1)
 prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constant__ PcArgs a) {
@@ -185,6 +194,10 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   const uint32_t s_stage = kLinear ? (uint32_t)a.stage_bytes : x_span + (uint32_t)(G * n) * a_tile;
   // ADD: the partial sums have a place of their own where that leaves the K loop enough stages
   const bool apart = kLinear || a.off_part / (int)s_stage >= min(nk_per, 4);
+  // ADD: the MMAs of a pass read its K loop's ring and begin when this CTA has read the sums of the pass before, so their completion tells
+  // the cluster that this CTA has room for sums. (Told by the epilogue, whose arrival has to release those reads: qkv of 4300 to 8000 rows,
+  // rank 64, 1024-wide 18.5 / 18.1 us, 2048-wide 32.1 / 31.4.) Not where nobody would wait for it: a CTA may leave before its peers arrive.
+  const bool told = !kLinear && CK > 1 && (!apart || npass > 1);
   const int s_stages = kLinear ? a.stages : min(kPcShrinkStages, (apart ? a.off_part : a.off_tmp) / (int)s_stage);
   const uint32_t s_tmem = tmem_base + (kLinear ? kSgmvBN : 0);  // (LINEAR: the first tile's sums lie in front)
   const uint32_t part_base = smem_base + (uint32_t)a.off_part;
@@ -315,6 +328,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
         if (++st == s_stages) { st = 0; ++round; }
       }
       umma_commit_elected(s_acc_full, leader);
+      if (told) umma_commit_cluster_elected(part_ready, (uint16_t)((1 << CK) - 1), leader);
     }
     if (!kLinear) st = round = 0;
     bool have_tmp = false;
@@ -388,12 +402,14 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
         // phases behind takes the parity for that of the phase to come.)
         if (exchange > 0) named_bar_sync(2, kPcEpi);
         if (etid == 0) mbar_arrive_expect_tx(part_full, (uint32_t)((CK - 1) * rows * mine * 32));
-        // Room for them: the K loop whose ring lies there is over; behind the first exchange, the sums of the one before have been read.
-        // (The arrival releases: a peer's stores may go there only behind these reads, which it learns of by acquiring.)
-        if (!apart || exchange > 0) {
+        // Room for them in every CTA: the K loop whose ring lies there is over, the sums of the exchange before have been read.
+        // LINEAR: nothing lies there ahead of the first one; the arrival releases, since peers may write only behind these reads.
+        if (kLinear && exchange > 0) {
           if (etid < CK) mbar_arrive_remote_release(mapa_shared(part_ready, (uint32_t)etid));
-          mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)((exchange - (apart ? 1 : 0)) & 1), &abort_flag);
+          mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)((exchange - 1) & 1), &abort_flag);
         }
+        const bool ahead = !apart || pi > 0;  // of the sends
+        if (told && ahead) mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)(pi & 1), &abort_flag);
         // (A TMEM load is a warp-wide operation on one column range: a warp whose rows straddle two runs reads both runs' columns.)
         for (int ui = 0; ui < g; ++ui) {
           const int lo_row = run_lo[u0 + ui], hi_row = run_hi[u0 + ui];
@@ -428,6 +444,9 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
           if (lane == 0) mbar_arrive(s_acc_empty);
         }
         mbar_wait_bounded_acquire_cluster(part_full, (uint32_t)(exchange & 1), &abort_flag);
+        // (Every phase is waited for, ahead of the arrival that lets this CTA's next pass begin: the next phase may be complete soon after
+        // that, and its parity is the one of the phase before.)
+        if (told && !ahead) mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)(pi & 1), &abort_flag);
         auto add_up = [&](auto parts) {
           constexpr int kParts = decltype(parts)::value;
           if (!live && !zero) return;
