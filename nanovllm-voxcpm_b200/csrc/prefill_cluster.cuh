@@ -10,7 +10,6 @@
 //   * one set-up (barriers, TMEM, run table) and one wait for the launch ahead;
 //   * partial sums go straight from tensor memory to the CTA that owns their columns, which sends the 16-bit values straight into
 //     the MMA operand tile of every CTA (st.async both times): no scratch, no barrier of the cluster between the halves;
-//   * lora_A is asked for ahead of the wait for the launch ahead;
 //   * the tiles' B operands are on their way before that exchange is over, and y's rows are on their way to the L2;
 //   * eight epilogue warps in two sets, each with two output buffers, and few TMA instructions: 1.35 us a tile of 128 x 256 (2.3).
 // us per projection (qkv, o, gate_up, down), the pair / this kernel: 8000 rows, 2048-wide, rank 64: 40 / 38, 32 / 22, 92 / 86,
@@ -171,7 +170,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   if (CK > 1) { cluster_arrive(); cluster_wait(); }  // the barriers of every CTA of the cluster are initialised
-  // Everything above may overlap the previous launch of the stream; x and y are final from here on. (Warp 0 asks for lora_A first.)
+  // Everything above may overlap the previous launch of the stream; x and y are final from here on. (Warp 0 waits ahead of its first load.)
   if (warp != 0) griddep_wait();
 
   const uint32_t tmem_base = tmem_base_s;
@@ -214,10 +213,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
     // =========================== TMA
     const uint32_t leader = elect_one();
     int st = 0, round = 0;
-    // lora_A of the first stages is asked for ahead of the wait: no kernel that lets others start early writes slabs. (LINEAR launches
-    // of more than 96 rows a block or fewer than eight K parts: x first, us with lora_A / x first, 1024 -> 1024 of 2500 rows 12.8 / 12.4, of 300
-    // 8.2 / 8.5.)
-    const int early = npass > 0 && (!kLinear || (CK == 8 && bm < 96)) ? min(s_stages, nk) : 0;
+    if (npass == 0) griddep_wait();
     for (int pi = 0; pi < npass; ++pi) {
       // (ADD: the partial sums of a pass lie where the ring is)
       if (!kLinear && pi > 0) mbar_wait_bounded(s_acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
@@ -225,33 +221,27 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
       int row[4];  // first lora_A row of each run of the pass (G <= 4)
 #pragma unroll
       for (int ui = 0; ui < 4; ++ui) row[ui] = uniform(ui < g ? run_slot[u0 + ui] * r : 0);
-      auto load_a = [&](int kc, int stage) {
-        const uint32_t full = kLinear ? t_full(stage) : s_full(stage);
-        mbar_arrive_expect_tx(full, x_tile + (uint32_t)(g * n) * a_tile);
-        uint32_t dst = smem_base + (uint32_t)stage * s_stage + x_span;
-#pragma unroll
-        for (int ui = 0; ui < 4; ++ui)
-          if (ui < g)
-            for (int s = 0; s < n; ++s, dst += a_tile) tma_load_2d(dst, &maps.a[s0 + s], (kc0 + kc) * kSgmvBK, row[ui], full);
-      };
-      if (pi == 0) {
-        if (leader)
-          for (int kc = 0; kc < early; ++kc) load_a(kc, kc);
-        __syncwarp();
-        griddep_wait();
-      }
+      // (lora_A of the first stages asked for ahead of this wait puts x behind it: us a launch, with / without, means over 1072 adds of 64 to
+      // 8000 rows: up to 450 rows 5.99 / 5.99, to 800 8.65 / 8.50, to 2112 11.45 / 11.17, to 4224 18.3 / 17.9, to 4736 24.6 / 23.9, to 8000
+      // 29.0 / 28.5; slabs that are not in the L2 the same way; fused linears 0 to 1 %.)
+      if (pi == 0) griddep_wait();
       for (int kc = 0; kc < nk; ++kc) {
         const uint32_t full = kLinear ? t_full(st) : s_full(st), empty = kLinear ? t_empty(st) : s_empty(st);
         if (round > 0) mbar_wait_bounded(empty, (uint32_t)((round & 1) ^ 1), &abort_flag);
         if (leader) {
-          if (pi > 0 || kc >= early) load_a(kc, st);
-          tma_load_2d(smem_base + (uint32_t)st * s_stage, &maps.x, (kc0 + kc) * kSgmvBK, row0, full);
+          uint32_t dst = smem_base + (uint32_t)st * s_stage;
+          mbar_arrive_expect_tx(full, x_tile + (uint32_t)(g * n) * a_tile);
+          tma_load_2d(dst, &maps.x, (kc0 + kc) * kSgmvBK, row0, full);
+          dst += x_span;
+#pragma unroll
+          for (int ui = 0; ui < 4; ++ui)
+            if (ui < g)
+              for (int s = 0; s < n; ++s, dst += a_tile) tma_load_2d(dst, &maps.a[s0 + s], (kc0 + kc) * kSgmvBK, row[ui], full);
         }
         __syncwarp();
         if (++st == s_stages) { st = 0; ++round; }
       }
     }
-    if (npass == 0) griddep_wait();
     if (!kLinear) {
       st = round = 0;
       if (npass > 0) mbar_wait_bounded(s_acc_full, (uint32_t)((npass - 1) & 1), &abort_flag);  // the ring changes its use
