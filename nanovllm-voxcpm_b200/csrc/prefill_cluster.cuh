@@ -175,14 +175,18 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
 
   const uint32_t tmem_base = tmem_base_s;
   const int nruns = nruns_s;
-  // This CTA's columns of y and its tiles of up to 256 of them: a range in LINEAR launches; in ADD ones the tiles are dealt to the
-  // CTAs in turn, so that a cluster updates neighbouring pieces of the same rows (8172 rows, 2048-wide, rank 64, a layer 192.1 ->
-  // 190.7 us). An ADD launch has nothing to add to a block without any adapter row.
+  // This CTA's columns of y and its tiles of up to 256 of them: a range, or, in ADD launches, tiles dealt to the CTAs in turn, so that a
+  // cluster updates neighbouring pieces of the same rows (8172 rows, 2048-wide, rank 64, a layer 192.1 -> 190.7 us). Not an odd number
+  // of tiles to two CTAs, of which one would have more columns than by range (1024 -> 1280, 4300 to 8000 rows, in turn / by range: rank
+  // 16 13.1 / 12.6 us, rank 64 17.7 / 17.3). Ten tiles to four CTAs stay dealt (2048 -> 2560, rank 64, 3300 rows 20.1 / 20.7). An ADD
+  // launch has nothing to add to a block without any adapter row.
   const int c_begin = min(g_lo + ck * a.cta_cols, g_hi), c_end = min(c_begin + a.cta_cols, g_hi);
   const int all_tiles = (g_hi - g_lo + a.tile_cols - 1) / a.tile_cols;
-  const int my_tiles = kLinear ? (c_end - c_begin + a.tile_cols - 1) / a.tile_cols : nruns > 0 || a.overwrite ? (all_tiles - ck + CK - 1) / CK : 0;
-  auto tile_lo = [&](int i) { return kLinear ? c_begin + i * a.tile_cols : g_lo + (i * CK + ck) * a.tile_cols; };
-  auto tile_hi = [&](int i) { return kLinear ? min(c_begin + (i + 1) * a.tile_cols, c_end) : min(g_lo + (i * CK + ck + 1) * a.tile_cols, g_hi); };
+  const bool in_turn = !kLinear && (CK != 2 || all_tiles % 2 == 0);
+  const int my_tiles = !kLinear && nruns == 0 && !a.overwrite ? 0 : in_turn ? (all_tiles - ck + CK - 1) / CK : (c_end - c_begin + a.tile_cols - 1) / a.tile_cols;
+  const int t_lo = in_turn ? g_lo + ck * a.tile_cols : c_begin, t_hi = in_turn ? g_hi : c_end, t_step = in_turn ? CK * a.tile_cols : a.tile_cols;
+  auto tile_lo = [&](int i) { return t_lo + i * t_step; };
+  auto tile_hi = [&](int i) { return min(t_lo + i * t_step + a.tile_cols, t_hi); };
   const uint32_t tmp_base = smem_base + (uint32_t)a.off_tmp, tmp_tile = (uint32_t)(kSgmvBM * row_bytes);
   // ---- the shrink's passes over x: up to G runs share one
   const int nk_all = a.in_dim / kSgmvBK, nk_per = (nk_all + CK - 1) / CK;

@@ -204,3 +204,18 @@ def test_partial_sums_of_many_passes_are_the_same_every_time(case):
            else O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, slots, 1.0, p.col_offsets))
     # half a unit in the last place of the largest output, on top of the path's tolerance
     assert_lora_close(got[0], ref, max_abs=2e-2 + 2.0 ** -8 * float(ref.abs().max()), what="many passes")
+
+
+@pytest.mark.parametrize("overwrite", [False, True])
+@pytest.mark.parametrize("T, in_dim, outs, r", [(4300, 128, [1024, 256], 32), (4290, 192, [1024, 192], 16), (4736, 128, [640], 64)])
+def test_two_ctas_take_an_odd_number_of_tiles_by_range(T, in_dim, outs, r, overwrite):
+    """Clusters of two whose CTAs have 640 columns each (the second 640, 576), or 320: tiles of 256, 256, 128 and of 192, 128."""
+    slots = by_runs(T, 4, 700, 60)
+    slots[0] = 0
+    p = W.make_projection(760, T, in_dim, outs, 4, r, token_to_slot=slots)
+    d = p.to_device(DEV)
+    LORA.launch_add(d.y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata(slots), 1.0, impl=N.IMPL_SGMV, overwrite=overwrite)
+    torch.cuda.synchronize()
+    assert N.device_status(reset=True) == 0
+    base = torch.full_like(p.y, -0.0) if overwrite else p.y
+    assert_lora_close(d.y, O.add_lora(base, p.x, p.a_slabs, p.b_slabs, slots, 1.0, p.col_offsets), what="by range")
