@@ -68,6 +68,7 @@ _SIGNATURES = {
     "lora_b200_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
     "lora_b200_grouped_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32, c_int32, c_int32]),
     "lora_b200_bucket_cluster": (c_int32, [c_int32, c_int32, c_int32, POINTER(c_int32), c_int32, c_int32, c_int32, c_int32]),
+    "lora_b200_prefill_plan": (c_int32, [c_int32, c_int32, c_int32, POINTER(c_int32), c_int32, c_int32, POINTER(c_int32)]),
     "lora_b200_linear_lora": (
         c_int32,
         [c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32, c_void_p, c_int64, c_int32, c_void_p, c_int32,

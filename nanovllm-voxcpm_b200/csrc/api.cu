@@ -434,6 +434,43 @@ int32_t lora_b200_bucket_cluster(int32_t T, int32_t in_dim, int32_t n_slices, co
   return bgmv_plan(b, &p, nullptr) ? 1 << p.c_shift : 0;
 }
 
+int32_t lora_b200_prefill_plan(int32_t T, int32_t in_dim, int32_t n_slices, const int32_t* out_sizes, int32_t r_max, int32_t form, int32_t* split) {
+  if (T < 1 || in_dim < 1 || r_max < 1 || out_sizes == nullptr || n_slices < 1 || n_slices > B200_LORA_MAX_SLICES || form < 0 || form > 2 || split == nullptr)
+    return 0;
+  void* const some = reinterpret_cast<void*>(uintptr_t(256));  // (stands for the arrays of a call; not read)
+  LinearProblem p = {};
+  SgmvProblem& b = p.lora;
+  int n = 0;
+  b.st.n = n_slices;
+  for (int s = 0; s < n_slices; ++s) {
+    if (out_sizes[s] < 0) return 0;
+    b.st.a[s] = b.st.b[s] = some; b.st.out[s] = out_sizes[s]; b.st.col[s] = p.n_total;
+    p.n_total += out_sizes[s];
+    n += out_sizes[s] > 0;
+  }
+  b.y = some; b.x = some; b.y_ld = p.n_total; b.x_ld = in_dim; b.T = T; b.in_dim = in_dim; b.S = 1; b.r_max = r_max;
+  p.silu = form == 2;
+  if (!sgmv_supported(b, nullptr)) return 0;
+  PcArgs a = {};
+  int kernel;
+  if (form == 0) {
+    if (!prefill_cluster_add_ok(b)) return kLinearTiles;
+    if (!prefill_cluster_plan(b, n, p.n_total, false, &a)) return 0;
+    kernel = kLinearCluster;
+  } else {
+    kernel = linear_kernel(p, true, &a);
+  }
+  if (kernel != kLinearCluster) return kernel;
+  const int width = (a.groups > 1 ? prefill_cluster_need(a, n, a.group_cols) : n) * r_max, nk_part = ceil_div_i(in_dim / kSgmvBK, a.ck);
+  split[0] = a.ck; split[1] = a.groups; split[2] = a.bm;
+  split[3] = form == 0 ? ceil_div_i(ceil_div_i(a.group_cols, a.tile_cols), a.ck) : ceil_div_i(std::min(a.cta_cols, a.group_cols), a.tile_cols);
+  split[4] = a.gmax; split[5] = ceil_div_i(width, a.part_cols); split[6] = a.stages;
+  split[7] = 0;
+  for (int g = 1; g <= a.gmax; ++g)
+    if (form != 0 || a.off_part / (kSgmvBM * kSgmvBK * 2 + g * width * kSgmvBK * 2) >= std::min(nk_part, 4)) split[7] = g;
+  return kernel;
+}
+
 int lora_b200_shrink_allreduce_expand(void* y, int64_t y_ld, const void* x, int64_t x_ld, int32_t T, int32_t in_dim,
                                       int32_t n_slices, const void* const* a_slabs, const void* const* b_slabs,
                                       const int32_t* out_sizes, const int32_t* col_offsets, int32_t S, int32_t r_max,

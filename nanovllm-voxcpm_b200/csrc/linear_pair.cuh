@@ -442,9 +442,9 @@ linear_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant_
 
 // ------------------------------------------------------------------ host side
 // LoRA stages are MMAs over a column range of which each CTA holds one half: a multiple of 32 columns.
-inline bool linear_pair_lora_ok(const SgmvArgs& a) {
-  for (int s = 0; s < a.n; ++s)
-    if (a.col[s] % 32 != 0 || a.out[s] % 32 != 0) return false;
+inline bool linear_pair_lora_ok(const SliceTable& st) {
+  for (int s = 0; s < st.n; ++s)
+    if (st.out[s] > 0 && (st.col[s] % 32 != 0 || st.out[s] % 32 != 0)) return false;
   return true;
 }
 
@@ -536,6 +536,14 @@ inline bool prefill_cluster_linear_ok(const LinearProblem& p, PcArgs* plan) {
   return here < 0.95 * others || (n * b.r_max <= 128 && b.in_dim <= 4096 && ((own <= rounds && own <= 3) || (own <= 2 && (own - rounds) * nk <= 16)));
 }
 
+// What a fused linear runs: prefill_cluster_kernel (`plan`), or, behind the shrink if it has a delta, CTA pairs or 128 x 256 tiles.
+enum LinearKernel { kLinearCluster = 1, kLinearPairs = 2, kLinearTiles = 3 };
+inline LinearKernel linear_kernel(const LinearProblem& p, bool with_lora, PcArgs* plan) {
+  if (with_lora && !p.silu && prefill_cluster_linear_ok(p, plan)) return kLinearCluster;
+  const int64_t pair_tiles = (int64_t)ceil_div_i(p.lora.T, 2 * kSgmvBM) * ceil_div_i(p.n_total, kSgmvBN);
+  return (p.silu || pair_tiles >= kPairMinTiles) && (!with_lora || linear_pair_lora_ok(p.lora.st)) ? kLinearPairs : kLinearTiles;
+}
+
 // y = x . W^T (+ bias) + LoRA delta, the delta accumulated into the GEMM's TMEM accumulator.
 inline int linear_lora_launch(const LinearProblem& p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   const SgmvProblem& b = p.lora;
@@ -552,7 +560,8 @@ inline int linear_lora_launch(const LinearProblem& p, void* workspace, size_t wo
   SgmvMaps sm;
   SgmvArgs sa = {};
   PcArgs plan = {};
-  if (with_lora && !p.silu && prefill_cluster_linear_ok(p, &plan)) {
+  const LinearKernel kernel = linear_kernel(p, with_lora, &plan);
+  if (kernel == kLinearCluster) {
     // (uses none; the entry point's contract is the same for every shape)
     if (int rc = sgmv_workspace_check(b, slices, workspace, workspace_bytes)) return rc;
     return prefill_cluster_launch(b, plan, p.weight, p.w_ld, p.n_total, p.bias, false, stream);
@@ -568,8 +577,7 @@ inline int linear_lora_launch(const LinearProblem& p, void* workspace, size_t wo
     sm.t = sm.x;
     for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) { sm.a[s] = sm.x; sm.b[s] = sm.x; }
   }
-  const int64_t pair_tiles = (int64_t)((b.T + 2 * kSgmvBM - 1) / (2 * kSgmvBM)) * ((p.n_total + kSgmvBN - 1) / kSgmvBN);
-  if ((p.silu || pair_tiles >= kPairMinTiles) && (!with_lora || linear_pair_lora_ok(sa))) {
+  if (kernel == kLinearPairs) {
     const void* slab_b[B200_LORA_MAX_SLICES];
     int n = 0;
     for (int s = 0; s < b.st.n; ++s)
