@@ -598,6 +598,12 @@ inline int prefill_cluster_linear_stages(int tile_cols, int width, int off_tmp, 
 //   unless another split promises 13 % less.
 inline double prefill_cluster_split(bool linear, bool in_groups, int T, int in_dim, int n, int n_total, int r, PcArgs* a) {
   const int nk = in_dim / kSgmvBK;
+  // Rows that are too many for clusters of four and fill the chip with 64-row blocks of clusters of two, and a y that is updated at the rate
+  // of the HBM: blocks of 128 rows in two groups of columns are slower, although the sum has them equal. us, two groups / one, 24 points
+  // of 4300 to 4700 rows 43.4 / 40.6: 1024 -> 8192, rank 32, 35.7 / 32.5, 2048 -> 12288, rank 64, 51.6 / 47.0. (A y of less than half of the L2
+  // keeps its groups: 1024 -> 4096, rank 32, 15.0 / 17.3.)
+  const bool one_group_only = !linear && ceil_div_i(T, kSgmvBM) > clusters_resident(4) && ceil_div_i(T, 64) <= clusters_resident(2) &&
+                              2 * (int64_t)T * n_total > 56 * 1000 * 1000;
   double least = -1.0, one_group = -1.0;
   int one_group_ck = 0, one_group_bm = 0;
   for (int ck = 1; ck <= 8; ck *= 2) {
@@ -608,7 +614,7 @@ inline double prefill_cluster_split(bool linear, bool in_groups, int T, int in_d
     for (int unit = ceil_div_i(n_total, 64 * ck); unit >= 1; unit = unit > 4 ? (unit + 1) * 3 / 4 : unit - 1) {
       const int groups = unit * ck * 64 >= n_total ? 1 : ceil_div_i(n_total, unit * ck * 64);
       if (groups == last) continue;
-      if (groups > clusters_resident(ck) || (groups > 1 && !in_groups)) break;
+      if (groups > clusters_resident(ck) || (groups > 1 && (!in_groups || one_group_only))) break;
       last = groups;
       const int bm = std::max(64, round_up_i(ceil_div_i(T, clusters_resident(ck) / groups), 8)), rows = std::min(bm, kSgmvBM);
       if (bm > kSgmvBM && (ck > 1 || groups > 1)) break;

@@ -69,6 +69,15 @@ def test_a_split_is_resident_and_covers_the_problem():
                         assert (in_dim // 64 + ck - 1) // ck * (ck - 1) < in_dim // 64  # every K part has a step
 
 
+@pytest.mark.parametrize("T, in_dim, outs, split", [
+    (4225, 1024, [4096, 4096], (2, 1, 64)), (4736, 2048, [6144, 6144], (2, 1, 64)), (4500, 4096, [3584, 3584], (2, 1, 64)),
+    (4300, 1024, [4096], (2, 2, 120)), (4736, 1024, [4096], (2, 2, 128)),   # y of less than half of the L2
+    (4737, 1024, [4096, 4096], (2, 1, 72)),                                  # one 64-row block more than clusters of two
+])
+def test_wide_outputs_of_as_many_blocks_as_clusters_of_two(T, in_dim, outs, split):
+    assert plan(T, in_dim, outs, 64, ADD)[:4] == (CLUSTER, *split)
+
+
 # T, in, outs, S, r, longest run; kernel, CTAs of a cluster, groups, rows of a block
 ADDS = [
     (960, 1024, [1024], 5, 32, 9, (CLUSTER, 8, 1, 64)),               # fifteen clusters of eight, several passes a block
