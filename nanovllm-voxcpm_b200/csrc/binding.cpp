@@ -578,13 +578,19 @@ struct Projection {
 // rows gate_up with the activation (940 GFLOP) 2131 / 2318, down (470) 2131 / 2244, o (134) 2131 / 2186; 2000 rows 1020 / 1093,
 // 1020 / 1063, 1029 / 1048; 1000 rows 540 / 516 (235), 540 / 547 (118), 540 / 541 (34). 2048-wide down (6144 columns): 4000 rows
 // (101) 692 / 705, 2000 rows (50) 355 / 348; its gate_up (2048 columns, 201 and 101) 692 / 651 and 355 / 323.
-// Around 1024 input columns one launch (prefill_cluster_kernel with groups of columns) wins from 128 rows on (fewer not measured): us, cuBLAS + add /
-// fused, rank 32: 1024 -> 1280 of 128, 300, 1100, 2700 rows 9.3 / 9.1, 11.0 / 9.4, 14.5 / 11.9, 22.9 / 15.9; 1024 -> 1024 8.4 / 7.6, 8.9 / 7.9, 10.7 /
-// 10.1, 17.1 / 12.8; 1024 -> 8192 13.0 / 11.4, 16.4 / 13.6, 34.2 / 23.1; steps of 3 layers of 1024, 128, 300, 1000 rows 251 / 229, 274 / 237, 329 / 310.
-// (2048 -> 2048 12.1 / 12.5, 13.1 / 14.7, 17.3 / 19.1; 4096 -> 1024 14.9 / 19.5, 15.5 / 21.3, 20.1 / 24.) Not rank 16, whose intermediate the
-// add of a small batch keeps as two numbers.
-inline bool fused_linear_wins(int64_t T, int64_t K, int64_t N, int64_t r, bool silu) {
-  if (!silu && K >= 768 && K <= 1024 && T >= 128 && r > 16) return true;
+// Around 1024 input columns one launch (prefill_cluster_kernel with groups of columns) wins: us, cuBLAS + add / fused, rank 32: 1024 ->
+// 1280 of 128, 300, 1100, 2700 rows 9.3 / 9.1, 11.0 / 9.4, 14.5 / 11.9, 22.9 / 15.9; 1024 -> 1024 8.4 / 7.6, 8.9 / 7.9, 10.7 / 10.1, 17.1 / 12.8; 1024 ->
+// 8192 13.0 / 11.4, 16.4 / 13.6, 34.2 / 23.1; steps of 3 layers of 1024, one prompt of 128, 256, 1000 rows 248 / 225, 265 / 240, 393 / 364. (2048 -> 2048
+// 12.1 / 12.5, 13.1 / 14.7, 17.3 / 19.1; 4096 -> 1024 14.9 / 19.5, 15.5 / 21.3, 20.1 / 24.) Narrower models and fewer rows would gain too (one prompt,
+// a step of 3 layers of 512, 128 rows 241 / 157, of 1024, 32 rows 245 / 205); they keep cuBLAS and the add, and with it the two roundings that
+// the step has layer by layer: a comparison of the two forms of a 256-wide step, not a time, set these two lines.
+// Not batches of short prompts: a block of rows reads x again for every one to four runs of it, while the add of so small a batch
+// goes by bucket. Steps as above, every prompt an adapter of its own, separate / fused, 128 to 1024 rows: prompts of 4 rows, rank 32, 265 / 469 (128
+// rows), 359 / 610 (256); rank 64 306 / 666 and 336 / 638; by rows a prompt, ratio of the two at rank 32 and 64: 24 rows 0.94, 0.92; 32 0.97, 0.98; 40
+// 1.01, 1.01; 48 1.02, 1.03; 64 1.03, 1.04; 96 1.06, 1.10.
+// Not rank 16, whose intermediate the add of a small batch keeps as two numbers.
+inline bool fused_linear_wins(int64_t T, int64_t K, int64_t N, int64_t r, int64_t prompts, bool silu) {
+  if (!silu && K >= 768 && K <= 1024 && T >= 128 && T >= 48 * prompts && r > 16) return true;
   return (T + 127) / 128 * ((N + 255) / 256) >= (N <= 1536 ? 45 : 100) && (K < 4096 || 2.0 * (double)T * (double)K * (double)N < (silu ? 300e9 : 60e9));
 }
 
@@ -612,6 +618,7 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const double eps = PyFloat_AsDouble(args[14]);
   if (PyErr_Occurred()) { PyErr_Clear(); return not_handled(); }
   const int64_t T = x->size(0), H = x->size(1), q_size = hq * d, kv = hk * d, qkv_width = q_size + 2 * kv;
+  const int64_t prompts = cu.numel() - 1;
   const int table = dtype_code(cos.scalar_type());
   if (dev != c10::cuda::current_device() || T < 1 || T > INT32_MAX || hq < 1 || hk < 1 || (d != 64 && d != 128) || hq % hk || inter < 8 || inter % 8 ||
       H % 8 || H > 4096 || max_len < 1 || max_len > T || table < 0)
@@ -665,7 +672,7 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const Slices& sl = p.sl;
     const bool lora = sl.n > 0 && b.tts != nullptr;
     const int K = (int)src.size(1), N = (int)dst.size(1);
-    if (lora && fused_linear_wins(T, K, N, sl.r, false) && K % 64 == 0 && (sl.r == 16 || sl.r == 32 || sl.r == 64)) {
+    if (lora && fused_linear_wins(T, K, N, sl.r, prompts, false) && K % 64 == 0 && (sl.r == 16 || sl.r == 32 || sl.r == 64)) {
       rc = p_linear(dst.data_ptr(), N, src.data_ptr(), K, (int)T, K, p.w->data_ptr(), K, N, nullptr, sl.n, sl.a, sl.b, sl.out, sl.col, (int)sl.S,
                     (int)sl.r, nullptr, b.tts, 1.0f, ws, ws_bytes, stream);
       return;
@@ -678,7 +685,7 @@ PyObject* prefill_layers(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   };
   // gate_up with the activation in its epilogue, by the same line (128 + 128 columns make a tile)
   auto silu_in_linear = [&](const Slices& sl) {
-    if (!fused_linear_wins(T, H, 2 * inter, sl.r, true) || H % 64 || inter % 32) return false;
+    if (!fused_linear_wins(T, H, 2 * inter, sl.r, prompts, true) || H % 64 || inter % 32) return false;
     if (sl.n > 0 && b.tts != nullptr && sl.r != 16 && sl.r != 32 && sl.r != 64) return false;
     for (int q = 0; q < sl.n; ++q)
       if (sl.out[q] % 32 || sl.col[q] % 32) return false;

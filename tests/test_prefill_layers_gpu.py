@@ -111,3 +111,35 @@ def test_attention_callable_is_checked(monkeypatch):
     monkeypatch.setattr(BB.Decoder, "_flash_attend", lambda self, s: fails)
     with pytest.raises(KeyError, match="out of blocks"):
         model._prefill_native(embeds, positions, step)
+
+
+@pytest.mark.parametrize("lens,fused", [([4] * 32, False), ([47] * 3, False), ([48] * 3, True), ([200, 56], True)])
+def test_projections_of_short_prompts_are_not_fused(lens, fused):
+    """1024 input columns, rank 32: fewer than 48 rows a prompt go to cuBLAS and the add, as layer by layer (the same bits of v in the
+    first layer's cache); the fused linear, which rounds the sum once, takes the others."""
+    T, S = sum(lens), 6
+    cfg = BB.DecoderConfig(hidden_size=1024, num_heads=8, num_kv_heads=2, head_dim=64, intermediate_size=256, num_layers=1, max_position=256,
+                           max_loras=S, max_lora_rank=32)
+    with torch.device(DEV):
+        model = BB.Decoder(cfg).to(torch.bfloat16)
+    model.init_random_(1)
+    model.fill_adapter_slots_(S, 32, seed=2)
+    model.fused_glue = True
+    model.allocate_kv_cache(T // cfg.kv_block_size + 1)
+    embeds = torch.randn(T, 1024, generator=torch.Generator().manual_seed(4)).to(DEV, torch.bfloat16)
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device=DEV)
+    step = BB.AttentionStep(True, torch.arange(T, device=DEV), cu_seqlens=cu, max_seqlen=max(lens))
+    positions = torch.cat([torch.arange(n) for n in lens]).to(DEV)
+    native, caches = model._prefill_native, []
+    for take in (native, lambda *a: None):
+        model._prefill_native = take
+        try:
+            with torch.no_grad():
+                set_lora_context(build_lora_context_from_slot_list([i % S for i, n in enumerate(lens) for _ in range(n)]))
+                model(embeds, positions, step)
+        finally:
+            reset_lora_context()
+        caches.append(model.layers[0].self_attn.v_cache.clone())
+    assert N.device_status(reset=True) == 0
+    torch.testing.assert_close(caches[0], caches[1], rtol=1e-2, atol=2e-2)
+    assert torch.equal(*caches) != fused
