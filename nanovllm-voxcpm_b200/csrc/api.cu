@@ -606,7 +606,9 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     bp.token_to_slot = token_to_slot;
     // (Without bucket arrays, or at rank 16, which the bucket kernel cannot overwrite, a batch that is its own takes a fill and an add.)
     const bool bucket_form = have_buckets && r_max % 32 == 0;
-    const bool prefill = prefill_sized(T, st, r_max, in_dim, true, one_launch) || (!bucket_form && one_launch && ceil_div_i(T, kBgmvTok) > 74);
+    // (What the prefill kernels refuse is no batch of theirs, however large: one bucket launch instead of a fill and an add.)
+    const bool prefill = sgmv_supported(sp, nullptr) && scratch_ok &&
+                         (prefill_sized(T, st, r_max, in_dim, true, one_launch) || (!bucket_form && one_launch && ceil_div_i(T, kBgmvTok) > 74));
     const bool decode_like = T < 32 * n_buckets || !prefill;
     if (dtype == B200_LORA_BF16 && have_buckets &&
         (impl == B200_LORA_IMPL_BGMV || (auto_impl && decode_like)) && bgmv_plan(bp, &plan, nullptr))

@@ -169,3 +169,35 @@ def test_layers_lora_first_order(kind):
     none = slots < 0
     assert torch.equal(first[none].view(torch.int16), base[none].view(torch.int16))
     torch.testing.assert_close(first[none].float(), after[none].float(), atol=1e-2, rtol=1e-2)
+
+
+def launches(run) -> int:
+    """Kernel launches of ``run``, counted in a captured graph."""
+    from cuda.bindings import runtime
+
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        run()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        run()
+    err, _, n = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()))
+    assert err == runtime.cudaError_t.cudaSuccess
+    return n
+
+
+# T, in, outs, r: more adapter bytes than the line between bucket and prefill kernel, and what the prefill kernels refuse or not
+@pytest.mark.parametrize("T, in_dim, outs, r, n", [
+    (500, 1024, [1024, 1024], 128, 1), (300, 2048, [2048, 2048], 96, 1), (700, 1056, [1024, 1024], 32, 1), (1300, 1024, [1024], 96, 1),
+    (480, 2048, [6144, 6144], 64, 1),        # prefill kernel, overwriting
+    (700, 1024, [1000, 1000], 64, 3),        # slices that do not tile the output: fill, shrink, expand
+])
+def test_a_delta_that_the_prefill_kernels_refuse_is_one_bucket_launch(T, in_dim, outs, r, n):
+    slots = torch.arange(T, dtype=torch.int32) * 3 // T
+    slots[5:9] = -1
+    p = W.make_projection(640, T, in_dim, outs, 3, r, token_to_slot=slots)
+    check_delta(p, run_delta(p, N.IMPL_AUTO, "graph"), f"r{r}")
+    d = p.to_device(DEV)
+    meta = metadata_for(d.token_to_slot, "graph", 3)
+    assert launches(lambda: LORA.launch_add(d.y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, meta, 1.0, overwrite=True)) == n
