@@ -506,12 +506,16 @@ struct LinearProblem {
 
 // Whether prefill_cluster_kernel takes a fused linear (and its plan): where its expected time is less than that of the shrink launch and
 // the kernel behind it, the latter a regression over 149 measured points that it meets within 9 %: launches and tile rounds, K steps of
-// the pair or the tile kernel with few and with all SMs busy, of the shrink; and for up to 128 rank rows and 4096 columns of x where a
-// CTA of an ungrouped cluster has no more tiles than the CTAs of the other two, or one more over at most 1024 columns of x. Over 156 points (12
-// projections, 64 to 4500 rows of up to eight prompts) the choice of kernel and split loses 2.1 % to the best, the tiles alone, without groups of
-// columns, 12. us, the others / this: 2048 -> 2560, rank 64, 64, 300 rows 18.7 / 12.9, 19.6 / 17.7; 6144 -> 2048 64, 300 and 600 rows 40 / 27, 40 / 32,
-// 40 / 36; 1024 -> 8192, rank 32, 64, 300, 1000 rows 13.3 / 10.0, 15.5 / 13.2, 24.8 / 21.9; 4096 -> 1024 300, 1700, 4001 rows 26.6 / 22.3, 32.2 / 26,
-// 38.6 / 35.8. The others keep 2048 -> 12288, rank 64 (of 2000 rows 89 / 117) and 6144 -> 2048 from 1000 rows on.
+// the pair or the tile kernel with few and with all SMs busy, of the shrink. Over 156 points (12 projections, 64 to 4500 rows of up to eight
+// prompts) the choice of kernel and split loses 2.1 % to the best, the tiles alone, without groups of columns, 12. us, the others / this: 2048 ->
+// 2560, rank 64, 64, 300 rows 18.7 / 12.9, 19.6 / 17.7; 6144 -> 2048 64, 300 and 600 rows 40 / 27, 40 / 32, 40 / 36; 1024 -> 8192, rank 32, 64, 300,
+// 1000 rows 13.3 / 10.0, 15.5 / 13.2, 24.8 / 21.9. The others keep 2048 -> 12288, rank 64 (of 2000 rows 89 / 117) and 6144 -> 2048 from 1000 rows on.
+// And, as the sums put the two too close to each other (this kernel up to 20 % too high), for up to 128 rank rows where a CTA of a cluster
+// without groups has one tile or, over up to 2048 columns of x, no more tiles than the CTAs of the other two (over 1024 one more). 150 points that
+// the sums alone leave to the others, all ranks, the others / this: one tile 4096 -> 1024, 2200 to 3700 rows 34.3 / 31.4, 4096 -> 512, 3200 to 9000
+// rows 39.6 / 36.6, 1024 -> 1280, 3200 rows 18.8 / 16.7; two 2048 -> 2048, 2200 to 4200 rows 33.2 / 30.0, 2048 -> 1024, 5000 to 9000 rows 36.1 / 32.6. Two
+// tiles over more columns: 4096 -> 4096, 1700 rows 52.7 / 60.7, 4096 -> 2048, 3200 rows 53.8 / 61.4, 4096 -> 1024, 5000 rows 57.7 / 60.6. (A second tile
+// has all K steps again, and x with them.) The rule loses 0.2 % to the best of these points; with two tiles over 4096 columns 3.1.
 inline bool prefill_cluster_linear_ok(const LinearProblem& p, PcArgs* plan) {
   const SgmvProblem& b = p.lora;
   int n = 0;
@@ -533,7 +537,7 @@ inline bool prefill_cluster_linear_ok(const LinearProblem& p, PcArgs* plan) {
   int ck = 1;  // the cluster without groups: tiles of its CTAs
   while (ck < 8 && blocks <= clusters_resident(2 * ck) && ceil_div_i(nk, 2 * ck) * (2 * ck - 1) < nk) ck *= 2;
   const int own = ceil_div_i(ceil_div_i(p.n_total, 64 * ck), kSgmvBN / 64);
-  return here < 0.95 * others || (n * b.r_max <= 128 && b.in_dim <= 4096 && ((own <= rounds && own <= 3) || (own <= 2 && (own - rounds) * nk <= 16)));
+  return here < 0.95 * others || (n * b.r_max <= 128 && b.in_dim <= (own > 1 ? 2048 : 4096) && ((own <= rounds && own <= 3) || (own <= 2 && (own - rounds) * nk <= 16)));
 }
 
 // What a fused linear runs: prefill_cluster_kernel (`plan`), or, behind the shrink if it has a delta, CTA pairs or 128 x 256 tiles.

@@ -78,6 +78,16 @@ def test_wide_outputs_of_as_many_blocks_as_clusters_of_two(T, in_dim, outs, spli
     assert plan(T, in_dim, outs, 64, ADD)[:4] == (CLUSTER, *split)
 
 
+@pytest.mark.parametrize("T, in_dim, outs, kernel", [
+    (3700, 4096, [1024], CLUSTER), (8000, 4096, [512], CLUSTER),          # a tile a CTA
+    (3700, 2048, [2048], CLUSTER), (9000, 2048, [1024], CLUSTER),         # two, no more than the others have
+    (1700, 4096, [4096], PAIRS), (3700, 4096, [2048], PAIRS), (6000, 4096, [1024], PAIRS), (12000, 4096, [512], TILES),  # two over 4096 columns
+    (2000, 2048, [6144, 6144], PAIRS), (1000, 6144, [2048], TILES),
+])
+def test_kernel_of_a_fused_linear(T, in_dim, outs, kernel):
+    assert plan(T, in_dim, outs, 32, LINEAR)[0] == kernel
+
+
 # T, in, outs, S, r, longest run; kernel, CTAs of a cluster, groups, rows of a block
 ADDS = [
     (960, 1024, [1024], 5, 32, 9, (CLUSTER, 8, 1, 64)),               # fifteen clusters of eight, several passes a block
