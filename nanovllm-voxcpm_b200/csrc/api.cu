@@ -102,12 +102,14 @@ namespace {
 // Whether a bf16 batch is large enough for the prefill kernels rather than the bucket kernel (an adapter read once per 16 rows of it),
 // by the adapter bytes that the bucket kernel would read; 16 rank rows take it as long as 32.
 //   prefill_cluster_kernel (adds): us per projection, bucket / prefill kernel, eight prompts: 1024-wide, rank 32: 1000 rows, qkv (18
-//   MB) 6.7 / 10.1, gate_up (41 MB) 9.5 / 12.0, 2000 rows, qkv (35 MB) 8.0 / 11.3, 2500 (44 MB) 12.9 / 11.6, o (21 MB) 6.2 / 9.0;
-//   2048-wide, rank 32: 1000 rows, qkv (35 MB) 9.1 / 12.3, 1200 (42 MB) 14.5 / 12.7; rank 64: gate_up of 400 rows (52 MB) 12.7 / 13.0,
-//   of 511 (67 MB) 20 / 14; 4096-wide, rank 64, gate_up of 200 rows (61 MB) 21.9 / 17.6. Over 1440 measured points (200 to 3300 rows of two
-//   to eight prompts, two widths, ranks 16 to 64, equal and mixed) the line is 2.9 % slower than the better choice each time, one at 75
-//   windows and 50 MB 6.5. Adapters of rank 16 that went to the bucket kernel, which keeps their intermediate as two numbers, still
-//   do: up to 1184 rows and 50 MB.
+//   MB) 6.9 / 10.1, gate_up (41 MB) 9.4 / 11.9, 2048 rows, qkv (36 MB) 8.2 / 11.5, 2400 (42 MB) 12.7 / 11.1, o (20 MB) 6.2 / 8.6;
+//   2048-wide, rank 32: 1000 rows, qkv (35 MB) 9.1 / 12.1, 1200 (42 MB) 14.9 / 12.9; rank 64: gate_up of 400 rows (52 MB) 12.7 / 13.0,
+//   of 511 (67 MB) 21.4 / 13.5. The bucket kernel's time goes up in steps, a wave of clusters each, so that some batches lie on the
+//   wrong side of any line by bytes (the 41 MB above). Over 1560 measured points (200 to 3300 rows of one to eight prompts, three widths,
+//   ranks 16 to 64) the line is 2.4 % slower than the better choice each time, one at 75 windows and 50 MB 5.2. Adapters of rank 16 that
+//   went to the bucket kernel, which keeps their intermediate as two numbers, still do: up to 1184 rows and 50 MB. Rank 64 is not
+//   asked for its bytes from 512 rows on, as it never was: 5.3 % behind the better choice there, most with few bytes (1024 -> 1024,
+//   512 rows, 8 MB 4.8 / 7.9; 2048 -> 2048, 724 rows, 24 MB 7.9 / 9.4).
 //   sgmv_shrink_kernel and the launch behind it (operators, slices that do not tile the output; at least 11 us for the pair): bucket /
 //   pair, six prompts: 1024-wide, rank 32, 900 rows, qkv (16 MB) 6.7 / 13.5, gate_up (37 MB) 8.9 / 15.1, 1500 rows 11.5 / 13.8 and
 //   (61 MB) 18.6 / 20.4; 2048-wide, rank 32, 900 rows, gate_up (59 MB) 19.0 / 19.1, 1500 rows (98 MB) 32.9 / 24.7; rank 64, 900

@@ -872,8 +872,8 @@ inline int bgmv_cluster(const BgmvProblem& b, const SliceTable& st) {
     const double kb = (double)bucket_bytes / 1024.0 * std::max(1.0, 32.0 / b.r_max);  // (16 rank rows take as long as 32)
     // A shrink or an expand alone, which take turns: 4 CTAs per bucket while two launches fit side by side (296 CTAs are resident
     // at two per SM), then 2, then 1; more for large adapters, as far as those are resident together or their streams are long.
-    // 1024-wide, rank 16, 8 rows, gate_up's expand with 4 / 8: 5.0 / 3.2 us; rank 32, 200 rows over 32, the four pairs of a layer
-    // with 4 everywhere 18.1, with 8 for gate_up's expand (8.4 / 6.8 us by itself) 18.5.
+    // 1024-wide, rank 16, 8 rows, gate_up's expand with 4 / 8: 5.7 / 4.2 us; rank 32, 200 rows over 32 (bf16 intermediate, from a graph),
+    // the eight launches of a layer with 1 / 2 / 4 / 8 everywhere 60 / 43 / 30 / 40, gate_up's expand by itself 21 / 12.9 / 8.8 / 7.2.
     const double resident = 2.0 * 148, half = 0.38 * resident, clusters = in_use + (b.T - 1) / kBgmvTok;
     C = in_use * 2 <= half ? 4 : (in_use <= half ? 2 : 1);
     while (C < 4 && (kb / C > 512 || (kb / C > 256 && in_use * C * 2 <= resident))) C *= 2;
@@ -890,12 +890,14 @@ inline int bgmv_cluster(const BgmvProblem& b, const SliceTable& st) {
   // 55.6 us a layer with clusters of four and 60.2 with the sizes taken (eight, o four) if even, 49.1 and 35.9 if skewed. Sums of
   // shares unrounded by rank rows and K parts, with a line at 290 CTAs, lost 2.3 and 1.6 %. us a launch with clusters of 1 / 2 /
   // 4 / 8, the size taken in brackets:
-  //   adds: 1024-wide, rank 16, 8 rows over 32 adapters, gate_up 16.3 / 9.1 / 5.4 / [3.8]; rank 32, 64 over 32, o 3.9 / 2.8 /
-  //   [2.5] / 3.7, 128 over 128, gate_up 20.2 / [12.8] / 15.1 / 19.5 (of skewed popularity 20.5 / 11.3 / 9.5 / 15.3), 384 over
-  //   128, o 5.2 / [5.0] / 8.0 / 16.8; 4 rows, down of 4 K parts 9.5 / 4.9 / [3.1] / 3.3, of 5 11.9 / 7.3 / 5.5 / [3.7], of 6
-  //   14.9 / 7.7 / 5.5 / [4.1], of 7 16.7 / 9.6 / 5.4 / [4.4], of 6 and 16 rows a bucket 15.4 / 8.0 / [6.1] / 7.3; 2048-wide, 384
-  //   over 32 of skewed popularity, gate_up 28.5 / 21.8 / [12.3] / 16.3; rank 64, 256 over 32, down 35.3 / 24.8 / 16.4 / [12.5],
-  //   of skewed popularity 34.4 / 24.9 / 16.8 / [19.4]; 4096-wide, 4 over 8, gate_up 54 / 30 / 15.8 / [7.8].
+  //   adds: 1024-wide, rank 16, 8 rows over 32 adapters, gate_up 16.2 / 9.0 / 5.4 / [3.8]; rank 32, 64 over 32, o 3.7 / 2.9 /
+  //   [2.5] / 3.6, 128 over 128, gate_up 19.7 / [12.6] / 14.9 / 19.7 (of skewed popularity 20.3 / 11.0 / 9.5 / 15.5), 384 over
+  //   128, o 5.1 / [5.0] / 8.1 / 16.8; 4 rows, down of 4 K parts 9.3 / 4.8 / [3.0] / 3.2, of 5 11.9 / 7.3 / 5.5 / [3.7], of 6
+  //   14.9 / 7.7 / 5.5 / [4.1], of 7 16.7 / 9.6 / 5.4 / [4.4], of 6 and 16 rows a bucket 15.3 / 8.0 / [6.0] / 7.4; 2048-wide, 384
+  //   over 32 of skewed popularity, gate_up 28.3 / 21.6 / [12.2] / 16.3; rank 64, 256 over 32, down 33.8 / 22.8 / 15.9 / [12.5],
+  //   of skewed popularity 32.8 / 23.0 / 16.3 / [19.1], 64 over 64, gate_up 32 / 32 / 18.3 / [21.5]; 4096-wide, 4 over 8, gate_up 55 / 28 /
+  //   15.2 / [7.6]. (The fit, the points, and here the down of 5 to 7 K parts and what lies beside a GEMM are of the kernel before
+  //   output tiles were dealt over the warps; the others, measured since, moved by 0 to 8 %, none to another order but near ties.)
   //   beside a GEMM (with the launch of the consumer): 1024-wide, rank 32, 64 rows over 64 adapters, qkv 11.4 / [11.4] / 15.9 /
   //   26, o 6.7 / [6.1] / 9.9 / 17.6, gate_up 22 / [15.0] / 17.9 / 24, down 13.4 / [9.5] / 13.9 / 25; 24 over 128, gate_up 18.7 /
   //   11.7 / [10.6] / 13.9; 8 over 32, qkv 8.8 / 8.6 / 7.9 / [7.1], gate_up 17.6 / 10.2 / [7.6] / 7.2; 128 over 128, o [8.2] /
@@ -974,13 +976,14 @@ inline bool bgmv_plan_cluster(const BgmvProblem& b, const SliceTable& st, int C,
   p.pitchR = Q + 4;
   const int recv_bytes = ksplit ? round_up_i(C * kBgmvTok * p.pitchR * 4, 128) : 0;
   const int fixed = red_bytes + tmp_bytes + recv_bytes + tab_bytes + bar_bytes;
-  // ring: what fits beside a second CTA on the SM, unless the caller set a size (up to the whole SM)
+  // ring: what fits beside a second CTA on the SM, unless the caller set a size (up to the whole SM), and as many stages as hold 256
+  // rows of lora_B (two of 128 up to eight of 32; fewer in flight not measured)
   const int ring_bytes = bgmv_options().ring_kb > 0 ? bgmv_options().ring_kb * 1024
                                                     : std::max(kBgmvSmemCoResident - fixed - 256, std::max(2, 256 / p.ER) * p.stage_bytes);
   int NS = std::min(std::max(tiles, std::max(2, 256 / p.ER)), (kBgmvSmemMax - fixed - 256) / p.stage_bytes);
   NS = std::min(NS, kBgmvMaxStages);
   NS = std::min(NS, std::max(std::max(2, 256 / p.ER), ring_bytes / p.stage_bytes));
-  if (NS < std::max(2, 256 / p.ER)) { *why = "shared memory too small for the stages of a step"; return false; }
+  if (NS < std::max(2, 256 / p.ER)) { *why = "shared memory too small for the stages of 256 rows"; return false; }
   p.NS = NS;
   p.off_red = NS * p.stage_bytes;
   p.off_tmp = p.off_red + red_bytes;

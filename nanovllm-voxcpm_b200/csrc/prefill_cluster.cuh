@@ -12,8 +12,8 @@
 //     the MMA operand tile of every CTA (st.async both times): no scratch, no barrier of the cluster between the halves;
 //   * the tiles' B operands are on their way before that exchange is over, and y's rows are on their way to the L2;
 //   * eight epilogue warps in two sets, each with two output buffers, and few TMA instructions: 1.35 us a tile of 128 x 256 (2.3).
-// us per projection (qkv, o, gate_up, down), the pair / this kernel: 8000 rows, 2048-wide, rank 64: 40 / 38, 32 / 22, 92 / 86,
-// 49 / 38; 1000 rows of them 18.7 / 15.6, 14.5 / 9.9, 22 / 18.1, 17 / 12.5. What is left of gate_up's 86 (HBM time 66): a kernel that only
+// us per projection (qkv, o, gate_up, down), the pair / this kernel: 8000 rows of 14 prompts, 2048-wide, rank 64: 40 / 38, 32 / 23, 92 / 88,
+// 49 / 39; 1000 rows of them 18.7 / 16.8, 14.5 / 10.4, 22 / 17.5, 17 / 12.9. What is left of gate_up's 88 (HBM time 66): a kernel that only
 // reads, adds to and writes these rows takes 73 to 80, and the blocks that hold a request boundary end 8 us after the others. Of the 9.9
 // of o: 1.4 from the end of the launch before to its first CTA's wait, 1.3 more to the last CTA's, K loop 2.4, exchange 2.5, tile and
 // store 2.
@@ -588,7 +588,7 @@ inline int prefill_cluster_linear_stages(int tile_cols, int width, int off_tmp, 
 //   ADD: a sum of the K loop at 70 KB a us, the exchange, the output tiles, less than half of the SMs (the launch behind then sets itself
 //   up beside this one), passes over x that fewer than four runs can share. A fit to 210 measured points (15 projections, 1024- and
 //   2048-wide, rank 16 to 64; 200 to 11000 rows of up to eight prompts, every K split with 1 to 16 groups): it loses 1.0 % to the best
-//   split of each, at most 17; one group and the largest K split 7.1. us, that / the split taken: 2048 -> 2 x 6144, rank 64, 300, 700, 2000,
+//   split of each, at most 17; one group and the largest K split 7.1; over 465 later points (1000 to 8000 rows, three widths) 0.7. us, that / the split taken: 2048 -> 2 x 6144, rank 64, 300, 700, 2000,
 //   4000 rows 22.5 / 13.6, 22.0 / 15.1, 29.5 / 27.9, 51.9 / 47.2; 2048 -> 2560 300 and 700 20.0 / 12.6, 19.4 / 15.4; 1024 -> 1024, rank 32,
 //   300 and 2000 7.9 / 7.4, 8.8 / 8.8. (A CTA's tiles, 1.1 us each, were half of the time where a block had one cluster: with groups a
 //   block can be 128 rows high and its columns still go to 16 CTAs and more.)
