@@ -179,6 +179,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   const int NS = p.NS;
   constexpr bool kF32Out = kMode == 4, kOverwrite = kMode == 3;
   constexpr bool kPrecise = kKind != 0, kF16 = kKind == 2;
+  constexpr bool kBlocks = kPrecise && !kF32Out;  // adds that read y
   constexpr int mode = kMode;
 
   B200_TRACE_POINT(0)
@@ -434,25 +435,27 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   // warps waited; us a launch, before / now: 1024-wide, rank 32, qkv of 256 rows over 32 adapters 4.58 / 4.24, of 4 rows 2.96 / 2.57;
   // rank 64, a step of two tiles with every warp waiting for both: 2048-wide, 48 over 64, gate_up 12.4 / 11.7; 4096-wide, 512 over
   // 88, o 29.5 / 25.2.)
-  // Kind 0: a table of the tiles, x = first y column, y = rows | slice << 16 | warp of the first block << 20. Kinds 1 and 2 ask for a
+  // Kind 0, and mode 4: a table of the tiles, x = first y column, y = rows | slice << 16 | warp of the first block << 20. Kinds 1 and 2 ask for a
   // block's y while they multiply the block before, which may lie several tiles back: a table of the blocks, x = first y column, y =
   // rows | slice << 8 | block of its tile << 12 | tile << 16. (Asked for a tile ahead, the y of narrow slices, at ranks above 32 all
   // of it, came late: us a layer, by tile / by block: fp16, rank 64, 128 rows over 32 adapters, 1024-wide 36.8 / 34.5, 4096-wide 90.5
-  // / 83.7; bf16, rank 48, 256 rows 34.6 / 30.5; rank 16, 37 rows 13.3 / 12.8. Kind 0 with the longer table loses up to 1 %.)
+  // / 83.7; bf16, rank 48, 256 rows 34.6 / 30.5; rank 16, 37 rows 13.3 / 12.8. Kind 0 with the longer table loses up to 1 %, and
+  // so do projections beside a GEMM of kind 1, which read no y: a step of four layers at rank 16, 128 rows over 100 adapters, by block / by
+  // tile, 1024-wide 241.3 / 237.2, 2048-wide 359.7 / 353.9.)
   int2* etab = reinterpret_cast<int2*>(smem + p.off_tab);
   int entries = tiles_exp;
-  if (kPrecise) {
+  if (kBlocks) {
     entries = 0;
 #pragma unroll
     for (int s = 0; s < B200_LORA_MAX_SLICES; ++s) entries += (e_n[s] + 31) >> 5;
   }
 #pragma unroll 1
   for (int i = tid; i < entries; i += kBgmvConsumers) {
-    int s_e = 0, r0 = kPrecise ? i << 5 : i << p.er_shift, tile = 0, blocks = 0;  // slice, first row in it; tiles and blocks of those before
+    int s_e = 0, r0 = kBlocks ? i << 5 : i << p.er_shift, tile = 0, blocks = 0;  // slice, first row in it; tiles and blocks of those before
 #pragma unroll
     for (int s = 0; s < B200_LORA_MAX_SLICES - 1; ++s)
       if (s_e == s && r0 >= e_n[s]) {
-        r0 -= kPrecise ? (e_n[s] + 31) & ~31 : e_tiles[s] << p.er_shift;
+        r0 -= kBlocks ? (e_n[s] + 31) & ~31 : e_tiles[s] << p.er_shift;
         tile += e_tiles[s];
         blocks += (e_n[s] + 31) >> 5;
         s_e = s + 1;
@@ -461,12 +464,12 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
 #pragma unroll
     for (int s = 0; s < B200_LORA_MAX_SLICES; ++s)
       if (s == s_e) { lo = e_lo[s]; en = e_n[s]; cb = p.st.col[s]; }
-    if (kPrecise)
+    if (kBlocks)
       etab[i] = make_int2(cb + lo + r0, min(32, en - r0) | (s_e << 8) | (((r0 & (ER - 1)) >> 5) << 12) | ((tile + (r0 >> p.er_shift)) << 16));
     else
       etab[i] = make_int2(cb + lo + r0, min(ER, en - r0) | (s_e << 16) | (((blocks + (r0 >> 5)) & (kBgmvWarps - 1)) << 20));
   }
-  if (kPrecise && tid < kBgmvWarps) etab[entries + tid] = make_int2(0, -65536);  // (no rows, of no tile: behind the last block of a warp)
+  if (kBlocks && tid < kBgmvWarps) etab[entries + tid] = make_int2(0, -65536);  // (no rows, of no tile: behind the last block of a warp)
   named_bar_sync(1, kBgmvConsumers);  // table complete
 
   const int x_col = warp * 32 + t * 8;  // shrink: first column of the thread inside a K part (block i adds 256)
@@ -533,7 +536,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
   };
   const int2* block_at = etab + warp;
   int2 block_next = make_int2(0, 0);  // of this warp
-  if (kPrecise) block_next = *block_at;
+  if (kBlocks) block_next = *block_at;
   const __nv_bfloat16* const xlo_p = p.x + (int64_t)max(tok_lo, 0) * p.x_ld + x_col;
   const __nv_bfloat16* const xhi_p = p.x + (int64_t)max(tok_hi, 0) * p.x_ld + x_col;
 
@@ -617,7 +620,7 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
     }
   }
   B200_TRACE_POINT(6)
-  if (kPrecise) load_y(block_next);
+  if (kBlocks) load_y(block_next);
 
   // ===== cross-warp reduction of the K slices, scale, bf16, all-gather =====
   named_bar_sync(1, kBgmvConsumers);
@@ -798,16 +801,16 @@ __device__ __forceinline__ void bgmv_body(const BgmvParams& p, uint8_t* smem, co
 #pragma unroll 1
   for (int e = 0; e < tiles_exp; ++e) {
     // (every warp waits for every tile: a wait that skipped phases of a stage could no longer tell them apart)
-    const int2 te = kPrecise ? block_next : etab[e];
-    const int row = kPrecise ? ((te.y >> 12) & 7) * 32 : ((warp - (te.y >> 20)) & (kBgmvWarps - 1)) * 32;
-    const bool mine = kPrecise ? te.y >> 16 == e : row < (te.y & 0xffff);
+    const int2 te = kBlocks ? block_next : etab[e];
+    const int row = kBlocks ? ((te.y >> 12) & 7) * 32 : ((warp - (te.y >> 20)) & (kBgmvWarps - 1)) * 32;
+    const bool mine = kBlocks ? te.y >> 16 == e : row < (te.y & 0xffff);
     const uint4 y_lo = y_next[0], y_hi = y_next[1];
-    if (kPrecise && mine) block_next = *(block_at += kBgmvWarps);
+    if (kBlocks && mine) block_next = *(block_at += kBgmvWarps);
     mbar_wait_bounded(full_bar(c_stage), c_parity, abort_flag);
     if (e < 10) { B200_TRACE_POINT(12 + 2 * e) }
     if (mine) {
-      if (kPrecise) load_y(block_next);
-      if (kPrecise) expand_fn(te.x, te.y & 0xff, (te.y >> 8) & 15, row, y_lo, y_hi);
+      if (kBlocks) load_y(block_next);
+      if (kBlocks) expand_fn(te.x, te.y & 0xff, (te.y >> 8) & 15, row, y_lo, y_hi);
       else expand_fn(te.x + row, (te.y & 0xffff) - row, (te.y >> 16) & 15, row, y_lo, y_hi);
     }
     if (e < 10) { B200_TRACE_POINT(13 + 2 * e) }
@@ -971,7 +974,7 @@ inline bool bgmv_plan_cluster(const BgmvProblem& b, const SliceTable& st, int C,
     exp_blocks += p.oc[s] / 32;
   }
   if (exp_tiles > kBgmvMaxExpandTiles) { *why = "too many expand tiles per CTA"; return false; }
-  const int tab_bytes = round_up_i((b.kind != 0 ? exp_blocks + kBgmvWarps : exp_tiles) * 8, 128);
+  const int tab_bytes = round_up_i((b.kind != 0 && b.mode != 4 ? exp_blocks + kBgmvWarps : exp_tiles) * 8, 128);
   p.ksplit = ksplit ? 1 : 0;
   p.pitchR = Q + 4;
   const int recv_bytes = ksplit ? round_up_i(C * kBgmvTok * p.pitchR * 4, 128) : 0;

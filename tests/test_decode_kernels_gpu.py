@@ -147,3 +147,11 @@ def test_decode_attention(case):
         bound = 2 ** -8 * (mag + ref.abs()) + 1e-4 * mag
         assert ((out[t].double() - ref).abs() <= 1.01 * bound).all(), f"context {ctx[t]}"
     assert N.device_status(reset=True) == 0
+
+
+@pytest.mark.parametrize("shape", [(64, 1024, [1024, 128, 128], 16), (50, 512, [4096, 4096], 16), (90, 512, [1184, 96, 8], 48), (128, 2048, [2048], 80)],
+                         ids=lambda s: f"{s[0]}x{s[1]}-r{s[3]}")
+def test_planes_of_an_intermediate_of_two_numbers(shape, monkeypatch):
+    """Ranks that are no multiple of 32 beside a GEMM: several output tiles a CTA, narrow ones among them."""
+    monkeypatch.setitem(globals(), "LINEAR", [shape])
+    test_decode_linear_planes(0, True)
