@@ -168,8 +168,8 @@ int32_t lora_b200_bucket_cluster(int32_t T, int32_t in_dim, int32_t n_slices, co
                                  int32_t dtype, int32_t beside_gemm);
 /* What the prefill kernels run for aligned operands whose slices lie one behind the other. form: 0 an add, 1 lora_b200_linear_lora, 2
  * lora_b200_linear_lora_silu. Returns 1: prefill_cluster_kernel, 2: a shrink and CTA pairs, 3: a shrink and 128 x 256 tiles, 0: refused.
- * With 1, split[8] = CTAs of a cluster, clusters of a block of rows, rows of a block, output tiles of a CTA, runs of equal slot that
- * share a pass over x, exchanges of partial sums a pass, stages of the tiles, and the most runs of a pass beside whose K loop the
+ * With 1, split[8] = CTAs of a cluster, clusters of a block of rows, rows of a block, output tiles of a CTA, slots of a block
+ * that share a pass over x, exchanges of partial sums a pass, stages of the tiles, and the most slots of a pass beside whose K loop the
  * partial sums have room (0: they lie where its ring was). Host code, for tests and tuning. No counterpart in the reference. */
 int32_t lora_b200_prefill_plan(int32_t T, int32_t in_dim, int32_t n_slices, const int32_t* out_sizes, int32_t r_max, int32_t form,
                                int32_t* split);

@@ -127,6 +127,12 @@ inline bool prefill_sized(int32_t T, const SliceTable& st, int32_t r_max, int32_
   return bytes * (r_max <= 16 ? 2 : 1) > (T < kSgmvAutoMinTokens ? 52 : 38) * kMB || windows > 240;
 }
 
+// Rows a bucket from which a batch may be one of whole prompts. The prefill kernels take the rows of a block's slots apart (the one-launch
+// kernel wherever they lie, the pair run by run), so a decode batch that is taken for one costs a pass over x for every one to four
+// slots of a block. Batches of fewer than 512 rows are more often that: at 64 rows a bucket rows that lie scattered cost adds of rank 64
+// (2048- and 4096-wide) 0.63 to 1.08 of the bucket kernel's time a layer, of rank 32 (4096-wide) up to 1.18, at 32 up to 1.9; whole prompts 0.7.
+inline bool rows_for_prefill(int32_t T, int32_t n_buckets) { return T >= (T < kSgmvAutoMinTokens ? 64 : 32) * (int64_t)n_buckets; }
+
 }  // namespace
 
 extern "C" {
@@ -611,7 +617,7 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     // (What the prefill kernels refuse is no batch of theirs, however large: one bucket launch instead of a fill and an add.)
     const bool prefill = sgmv_supported(sp, nullptr) && scratch_ok &&
                          (prefill_sized(T, st, r_max, in_dim, true, one_launch) || (!bucket_form && one_launch && ceil_div_i(T, kBgmvTok) > 74));
-    const bool decode_like = T < 32 * n_buckets || !prefill;
+    const bool decode_like = !rows_for_prefill(T, n_buckets) || !prefill;
     if (dtype == B200_LORA_BF16 && have_buckets &&
         (impl == B200_LORA_IMPL_BGMV || (auto_impl && decode_like)) && bgmv_plan(bp, &plan, nullptr))
       return bgmv_launch(plan, st_);
@@ -632,10 +638,9 @@ static int add_or_delta(void* y, int64_t y_ld, const void* x, int64_t x_ld, int3
     // batches to the fused kernel, everything else (other dtypes, odd shapes) to the generic one.
     int parts;
     const bool bgmv_ok = planned = is16 && have_buckets && bgmv_plan(bp, &plan, nullptr);
-    // The prefill kernels tile rows in token order and pay one stage per run of equal slot, so they
-    // want request-contiguous rows: with bucket arrays at hand, fewer than 32 rows per bucket on
-    // average means a decode-like batch (slots scattered over the rows) and goes to the bucket kernel.
-    const bool scattered = bgmv_ok && T < 32 * n_buckets;
+    // The prefill kernels take the rows in token order: with bucket arrays at hand, few rows a bucket on average mean a decode-like
+    // batch (slots scattered over the rows), which goes to the bucket kernel.
+    const bool scattered = bgmv_ok && !rows_for_prefill(T, n_buckets);
     if (dtype == B200_LORA_BF16 && !scattered && (!bgmv_ok ? T >= kSgmvAutoMinTokens : prefill_sized(T, st, r_max, in_dim, true, one_launch)) && sgmv_supported(sp, nullptr) &&
         scratch_ok)
       impl = B200_LORA_IMPL_SGMV;

@@ -7,7 +7,7 @@
 // What bounds the pair it replaces (sgmv_shrink_kernel, then tc_tile_kernel) is the way between its launches: both fill an SM's
 // shared memory, so the second one's set-up, its wait for the first and the trip of the intermediate through the L2 are all
 // serial with the K loop: 9 to 13 us a shrink of 1000 rows whose loads take 2. Here
-//   * one set-up (barriers, TMEM, run table) and one wait for the launch ahead;
+//   * one set-up (barriers, TMEM, table of the slots) and one wait for the launch ahead;
 //   * partial sums go straight from tensor memory to the CTA that owns their columns, which sends the 16-bit values straight into
 //     the MMA operand tile of every CTA (st.async both times): no scratch, no barrier of the cluster between the halves;
 //   * the tiles' B operands are on their way before that exchange is over, and y's rows are on their way to the L2;
@@ -17,8 +17,8 @@
 // reads, adds to and writes these rows takes 73 to 80, and the blocks that hold a request boundary end 8 us after the others. Of the 9.9
 // of o: 1.4 from the end of the launch before to its first CTA's wait, 1.3 more to the last CTA's, K loop 2.4, exchange 2.5, tile and
 // store 2.
-// Rows of a block may use different slots: the MMA of a run of equal slots updates the rows of that run only (its lane mask), so
-// the operand needs no masked copy per run. Rows without adapter: -0.0 in ADD launches (x + (-0.0) == x bit for bit), the base
+// Rows of a block may use different slots: the MMA of the rows of one slot updates these rows only (its lane mask), so
+// the operand needs no masked copy per slot. Rows without adapter: -0.0 in ADD launches (x + (-0.0) == x bit for bit), the base
 // result in LINEAR ones.
 #pragma once
 
@@ -45,7 +45,7 @@ struct PcArgs {
   int cta_cols, tile_cols;                  // columns of y per CTA and per tile (multiples of 64, a tile at most 256)
   int overwrite;                            // ADD: store the delta (-0.0 in rows without adapter) instead of adding it
   int bm, ck;                               // rows of a block (a multiple of 8, 64 to 128), CTAs of a cluster
-  int gmax;                                 // runs of a block whose K loops share one pass over x
+  int gmax;                                 // lots (slots of a block) whose K loops share one pass over x
   int stages, stage_bytes;                  // ring of the tiles: lora_B tiles (LINEAR: or x and W tiles)
   int out_bufs, off_out, off_tmp;           // output buffers of each epilogue set; byte offsets
   int part_cols, off_part;                  // columns of partial sums exchanged at a time, where they arrive
@@ -77,9 +77,9 @@ template <bool kLinear>
 __global__ void __launch_bounds__(kPcThreads, 1)
 prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constant__ PcArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ int16_t s_slot[kSgmvBM], run_slot[kSgmvBM];
-  __shared__ uint8_t run_lo[kSgmvBM], run_hi[kSgmvBM];
-  __shared__ int nruns_s;
+  __shared__ int16_t s_slot[kSgmvBM], lot_slot[kSgmvBM];
+  __shared__ uint8_t row_lot[kSgmvBM];  // the lot of a row (255: no adapter)
+  __shared__ int nlots_s;
   __shared__ __align__(8) uint64_t bar_words[2 * kPcShrinkStages + 2 * kPcMaxTileStages + 9];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_flag;
@@ -124,48 +124,54 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
     if (kLinear) tma_prefetch_desc(&maps.w);
     for (int s = s0; s < s0 + n; ++s) { tma_prefetch_desc(&maps.a[s]); tma_prefetch_desc(&maps.b[s]); }
   }
-  // ---- runs of equal slot inside the block
-  {
-    __shared__ int warp_starts[4];
-    const int i = tid;
-    if (i < kSgmvBM) {
-      int sl = i < bm && row0 + i < a.T ? a.token_to_slot[row0 + i] : -1;
-      (void)B200_IN_BOUNDS(sl >= -1 && sl < a.S);  // ids outside [-1, S) are treated as "no adapter"; the checked build reports them
-      if (sl >= a.S || sl < -1) sl = -1;
-      s_slot[i] = (int16_t)sl;
+  if (warp == 2) {
+    // ---- lots: the block's rows of one slot each, wherever they lie, in the order of their first rows. (By runs of equal slot, every row
+    // of a decode batch over few adapters, which the host cannot tell from whole prompts, was a run, and every one to four runs a pass
+    // over x: an add of 333 rows over 8 adapters, 4096-wide, rank 64, took 352 us a layer, by lots 86. One warp finds them by itself: a
+    // table of runs that four warps made between barriers kept a launch of 500 to 6000 rows 0.2 to 0.7 us, fused linears 0.1 to 0.5.)
+    int slot[4], lot[4], n_lots = 0;  // of rows lane, 32 + lane, ...
+    unsigned left[4];                 // rows that have none yet
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const int i = 32 * w + lane;
+      slot[w] = i < bm && row0 + i < a.T ? a.token_to_slot[row0 + i] : -1;
+      (void)B200_IN_BOUNDS(slot[w] >= -1 && slot[w] < a.S);  // ids outside [-1, S) are treated as "no adapter"; the checked build reports them
+      if (slot[w] >= a.S || slot[w] < -1) slot[w] = -1;
+      lot[w] = 255;
     }
-    __syncthreads();
-    bool starts = false, ends = false;
-    unsigned before = 0;
-    if (i < kSgmvBM) {
-      const int sl = s_slot[i];
-      starts = sl >= 0 && (i == 0 || s_slot[i - 1] != sl);
-      ends = sl >= 0 && (i == kSgmvBM - 1 || s_slot[i + 1] != sl);
-      const unsigned mask = __ballot_sync(0xffffffffu, starts);
-      before = __popc(mask & ((2u << (i & 31)) - 1u));  // runs of this warp that start at or before this row
-      if ((i & 31) == 0) warp_starts[i >> 5] = __popc(mask);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) left[w] = __ballot_sync(0xffffffffu, slot[w] >= 0);
+    while ((left[0] | left[1] | left[2] | left[3]) != 0) {
+      const int w = left[0] != 0 ? 0 : left[1] != 0 ? 1 : left[2] != 0 ? 2 : 3;
+      const unsigned rows = w == 0 ? left[0] : w == 1 ? left[1] : w == 2 ? left[2] : left[3];
+      const int v = __shfl_sync(0xffffffffu, w == 0 ? slot[0] : w == 1 ? slot[1] : w == 2 ? slot[2] : slot[3], __ffs(rows) - 1);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (slot[q] == v) lot[q] = n_lots;
+        left[q] &= ~__ballot_sync(0xffffffffu, slot[q] == v);
+      }
+      if (lane == 0) lot_slot[n_lots] = (int16_t)v;
+      ++n_lots;
     }
-    __syncthreads();
-    if (i < kSgmvBM) {
-      for (int w = 0; w < i >> 5; ++w) before += (unsigned)warp_starts[w];
-      if (starts) { run_slot[before - 1] = s_slot[i]; run_lo[before - 1] = (uint8_t)i; }
-      if (ends) run_hi[before - 1] = (uint8_t)(i + 1);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      s_slot[32 * w + lane] = (int16_t)slot[w];
+      row_lot[32 * w + lane] = (uint8_t)lot[w];
     }
-    const int total = warp_starts[0] + warp_starts[1] + warp_starts[2] + warp_starts[3];
-    if (i == 0) {
-      nruns_s = total;
-      for (int s = 0; s < kPcShrinkStages; ++s) { mbar_init(s_full(s), 1); mbar_init(s_empty(s), 1); }
-      for (int s = 0; s < kPcMaxTileStages; ++s) { mbar_init(t_full(s), 1); mbar_init(t_empty(s), 1); }
-      for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), kPcEpi / 32); }
-      mbar_init(s_acc_full, 1);
-      mbar_init(s_acc_empty, kPcEpi / 32);
-      mbar_init(part_ready, (uint32_t)CK);
-      mbar_init(part_full, 1);
-      mbar_init(tmp_full, 1);
-      abort_flag = 0;
-      mbar_fence_init();
-      mbar_arrive_expect_tx(tmp_full, (uint32_t)(bm * width * 2));
-    }
+    if (lane == 0) nlots_s = n_lots;
+  }
+  if (warp == 3 && elect_one()) {
+    for (int s = 0; s < kPcShrinkStages; ++s) { mbar_init(s_full(s), 1); mbar_init(s_empty(s), 1); }
+    for (int s = 0; s < kPcMaxTileStages; ++s) { mbar_init(t_full(s), 1); mbar_init(t_empty(s), 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), kPcEpi / 32); }
+    mbar_init(s_acc_full, 1);
+    mbar_init(s_acc_empty, kPcEpi / 32);
+    mbar_init(part_ready, (uint32_t)CK);
+    mbar_init(part_full, 1);
+    mbar_init(tmp_full, 1);
+    abort_flag = 0;
+    mbar_fence_init();
+    mbar_arrive_expect_tx(tmp_full, (uint32_t)(bm * width * 2));
   }
   __syncthreads();
   tc_fence_after_sync();
@@ -174,7 +180,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   if (warp != 0) griddep_wait();
 
   const uint32_t tmem_base = tmem_base_s;
-  const int nruns = nruns_s;
+  const int nlots = nlots_s;
   // This CTA's columns of y and its tiles of up to 256 of them: a range, or, in ADD launches, tiles dealt to the CTAs in turn, so that a
   // cluster updates neighbouring pieces of the same rows (8172 rows, 2048-wide, rank 64, a layer 192.1 -> 190.7 us). Not an odd number
   // of tiles to two CTAs, of which one would have more columns than by range (1024 -> 1280, 4300 to 8000 rows, in turn / by range: rank
@@ -183,15 +189,15 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
   const int c_begin = min(g_lo + ck * a.cta_cols, g_hi), c_end = min(c_begin + a.cta_cols, g_hi);
   const int all_tiles = (g_hi - g_lo + a.tile_cols - 1) / a.tile_cols;
   const bool in_turn = !kLinear && (CK != 2 || all_tiles % 2 == 0);
-  const int my_tiles = !kLinear && nruns == 0 && !a.overwrite ? 0 : in_turn ? (all_tiles - ck + CK - 1) / CK : (c_end - c_begin + a.tile_cols - 1) / a.tile_cols;
+  const int my_tiles = !kLinear && nlots == 0 && !a.overwrite ? 0 : in_turn ? (all_tiles - ck + CK - 1) / CK : (c_end - c_begin + a.tile_cols - 1) / a.tile_cols;
   const int t_lo = in_turn ? g_lo + ck * a.tile_cols : c_begin, t_hi = in_turn ? g_hi : c_end, t_step = in_turn ? CK * a.tile_cols : a.tile_cols;
   auto tile_lo = [&](int i) { return t_lo + i * t_step; };
   auto tile_hi = [&](int i) { return min(t_lo + i * t_step + a.tile_cols, t_hi); };
   const uint32_t tmp_base = smem_base + (uint32_t)a.off_tmp, tmp_tile = (uint32_t)(kSgmvBM * row_bytes);
-  // ---- the shrink's passes over x: up to G runs share one
+  // ---- the shrink's passes over x: up to G lots share one
   const int nk_all = a.in_dim / kSgmvBK, nk_per = (nk_all + CK - 1) / CK;
   const int kc0 = min(ck * nk_per, nk_all), nk = min(nk_per, nk_all - kc0);  // this CTA's K steps (at least one: see the launch)
-  const int G = min(a.gmax, max(nruns, 1)), npass = (nruns + G - 1) / G;
+  const int G = min(a.gmax, max(nlots, 1)), npass = (nlots + G - 1) / G;
   const uint32_t x_tile = (uint32_t)bm * kSgmvBK * 2, a_tile = (uint32_t)r * kSgmvBK * 2;
   const uint32_t x_span = kSgmvBM * kSgmvBK * 2;  // (the MMA reads 128 rows; those beyond bm give rows that nobody reads)
   const uint32_t s_stage = kLinear ? (uint32_t)a.stage_bytes : x_span + (uint32_t)(G * n) * a_tile;
@@ -221,10 +227,10 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
     for (int pi = 0; pi < npass; ++pi) {
       // (ADD: the partial sums of a pass lie where the ring is)
       if (!kLinear && pi > 0) mbar_wait_bounded(s_acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
-      const int u0 = pi * G, g = min(G, nruns - u0);
-      int row[4];  // first lora_A row of each run of the pass (G <= 4)
+      const int u0 = pi * G, g = min(G, nlots - u0);
+      int row[4];  // first lora_A row of each lot of the pass (G <= 4)
 #pragma unroll
-      for (int ui = 0; ui < 4; ++ui) row[ui] = uniform(ui < g ? run_slot[u0 + ui] * r : 0);
+      for (int ui = 0; ui < 4; ++ui) row[ui] = uniform(ui < g ? lot_slot[u0 + ui] * r : 0);
       // (lora_A of the first stages asked for ahead of this wait puts x behind it: us a launch, with / without, means over 1072 adds of 64 to
       // 8000 rows: up to 450 rows 5.99 / 5.99, to 800 8.65 / 8.50, to 2112 11.45 / 11.17, to 4224 18.3 / 17.9, to 4736 24.6 / 23.9, to 8000
       // 29.0 / 28.5; slabs that are not in the L2 the same way; fused linears 0 to 1 %.)
@@ -274,8 +280,8 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
         __syncwarp();
         if (++st == a.stages) { st = 0; ++round; }
       }
-      for (int u = 0; u < nruns; ++u) {
-        const int slot = uniform(run_slot[u]);
+      for (int u = 0; u < nlots; ++u) {
+        const int slot = uniform(lot_slot[u]);
         for (int s = s0; s < s0 + n; ++s) {
           int lo, hi;
           if (!part_of(s, i, lo, hi)) continue;
@@ -306,7 +312,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
     const uint32_t idesc_s = umma_idesc_bf16(kSgmvBM, width);
     int st = 0, round = 0;
     for (int pi = 0; pi < npass; ++pi) {
-      const int jobs = uniform(min(G, nruns - pi * G));
+      const int jobs = uniform(min(G, nlots - pi * G));
       if (pi > 0) mbar_wait_bounded(s_acc_empty, (uint32_t)((pi - 1) & 1), &abort_flag);
       tc_fence_after_sync();
       for (int kc = 0; kc < nk; ++kc) {
@@ -314,7 +320,7 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
         tc_fence_after_sync();
         const uint32_t xl = lo0 + ((uint32_t)st * s_stage >> 4);
         uint32_t al = xl + (x_span >> 4), d = s_tmem;
-        for (int q = 0; q < jobs; ++q, al += (uint32_t)n * a_tile >> 4, d += (uint32_t)width) {  // runs of the pass
+        for (int q = 0; q < jobs; ++q, al += (uint32_t)n * a_tile >> 4, d += (uint32_t)width) {  // lots of the pass
 #pragma unroll
           for (int k4 = 0; k4 < kSgmvBK / 16; ++k4) umma_elected(d, xl + 2u * k4, al + 2u * k4, hi_x, idesc_s, (kc > 0 || k4 > 0) ? 1u : 0u, leader);
         }
@@ -326,6 +332,9 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
     }
     if (!kLinear) st = round = 0;
     bool have_tmp = false;
+    int my_lot[4];  // of rows lane, 32 + lane, ...
+#pragma unroll
+    for (int w = 0; w < 4; ++w) my_lot[w] = row_lot[32 * w + lane];
     for (int job = 0; job < my_tiles; ++job) {
       const int buf = job & 1, c_lo = tile_lo(job);
       const uint32_t idesc_w = umma_idesc_bf16(kSgmvBM, (tile_hi(job) - c_lo + 15) & ~15);
@@ -343,9 +352,10 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
         umma_commit_elected(t_empty(st), leader);
         if (++st == a.stages) { st = 0; ++round; }
       }
-      for (int u = 0; u < nruns; ++u) {
-        const int lo_row = uniform(run_lo[u]), hi_row = uniform(run_hi[u]);
-        const uint32_t off[4] = {rows_outside(lo_row, hi_row, 0), rows_outside(lo_row, hi_row, 1), rows_outside(lo_row, hi_row, 2), rows_outside(lo_row, hi_row, 3)};
+      for (int u = 0; u < nlots; ++u) {
+        uint32_t off[4];  // lanes that are not of the lot
+#pragma unroll
+        for (int w = 0; w < 4; ++w) off[w] = __ballot_sync(0xffffffffu, my_lot[w] != u);
         for (int s = s0; s < s0 + n; ++s) {
           int lo, hi;
           if (!part_of(s, job, lo, hi)) continue;
@@ -378,14 +388,18 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
     // st.async: with plain remote stores and an arrival that releases them a layer of 300 to 5000 rows takes 4 to 10 % longer, the
     // release alone 1 us. (Before: written to shared memory, read by the owners across the cluster behind a barrier.)
     int exchange = 0;
-    const int my_slot = s_slot[row_in_blk];
+    const int my_slot = s_slot[row_in_blk], my_lot = row_lot[row_in_blk];
     const float my_scale = my_slot < 0 ? 0.f : a.scaling * (a.scale_per_slot != nullptr ? a.scale_per_slot[my_slot] : 1.0f);
     const uint32_t row_off = (uint32_t)row_in_blk * 16u, quad = (uint32_t)bm * 16u;  // [sender][piece][half of it][row] of 16 bytes
     for (int pi = 0; pi < npass; ++pi) {
-      const int u0 = pi * G, g = min(G, nruns - u0);
-      int rows = 0;  // with an adapter, in this pass
-      for (int ui = 0; ui < g; ++ui) rows += run_hi[u0 + ui] - run_lo[u0 + ui];
-      const bool live = my_slot >= 0 && row_in_blk >= run_lo[u0] && row_in_blk < run_hi[u0 + g - 1];
+      const int u0 = pi * G, g = min(G, nlots - u0);
+      int rows = 0;  // of this pass
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const int of = row_lot[32 * w + lane];
+        rows += __popc(__ballot_sync(0xffffffffu, of >= u0 && of < u0 + g));
+      }
+      const bool live = my_lot >= u0 && my_lot < u0 + g;
       const bool zero = my_slot < 0 && pi == 0 && row_in_blk < bm;  // rows without adapter
       mbar_wait_bounded(s_acc_full, (uint32_t)(pi & 1), &abort_flag);
       tc_fence_after_sync();
@@ -404,11 +418,10 @@ prefill_cluster_kernel(const __grid_constant__ PcMaps maps, const __grid_constan
         }
         const bool ahead = !apart || pi > 0;  // of the sends
         if (told && ahead) mbar_wait_bounded_acquire_cluster(part_ready, (uint32_t)(pi & 1), &abort_flag);
-        // (A TMEM load is a warp-wide operation on one column range: a warp whose rows straddle two runs reads both runs' columns.)
+        // (A TMEM load is a warp-wide operation on one column range: a warp with rows of two lots reads both lots' columns.)
         for (int ui = 0; ui < g; ++ui) {
-          const int lo_row = run_lo[u0 + ui], hi_row = run_hi[u0 + ui];
-          if (hi_row <= quarter * 32 || lo_row >= quarter * 32 + 32) continue;  // warp-uniform
-          const bool here = row_in_blk >= lo_row && row_in_blk < hi_row;
+          const bool here = my_lot == u0 + ui;
+          if (!__any_sync(0xffffffffu, here)) continue;
           for (int c = 16 * set; c < cols; c += 32) {
             uint32_t v[16];
             tmem_ld_32x16(s_tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ui * width + c0 + c), v);
@@ -564,14 +577,14 @@ inline int prefill_cluster_need(const PcArgs& a, int n, int group_cols) {
   return most;
 }
 
-// Runs of a block that share a pass over x (`width` rank rows each). ADD: sums in 512 TMEM columns, two stages of the ring; LINEAR: in
+// Lots (the rows of a slot) of a block that share a pass over x (`width` rank rows each). ADD: sums in 512 TMEM columns, two stages of the ring; LINEAR: in
 // 256, lora_A tiles where a stage has its W tile.
-inline int prefill_cluster_runs(bool linear, int width, int room) {
-  int runs = 1;
+inline int prefill_cluster_lots(bool linear, int width, int room) {
+  int lots = 1;
   for (int g = 2; g <= 4; ++g)
     if (linear ? g * width <= kSgmvBN && g * width * kSgmvBK * 2 <= room : g * width <= 512 && room / (kSgmvBM * kSgmvBK * 2 + g * width * kSgmvBK * 2) >= 2)
-      runs = g;
-  return runs;
+      lots = g;
+  return lots;
 }
 
 // LINEAR: bytes of a stage and stages of its ring (of which at least three and one output buffer of each epilogue set must fit; 0 if not)
@@ -586,13 +599,13 @@ inline int prefill_cluster_linear_stages(int tile_cols, int width, int off_tmp, 
 // K parts (the CTAs of a cluster), groups of columns and rows of a block: of those splits whose clusters are resident at once, the one
 // of the least time in us, which is returned (negative: none fits). `in_groups`: the slices lie one behind the other.
 //   ADD: a sum of the K loop at 70 KB a us, the exchange, the output tiles, less than half of the SMs (the launch behind then sets itself
-//   up beside this one), passes over x that fewer than four runs can share. A fit to 210 measured points (15 projections, 1024- and
+//   up beside this one), passes over x that fewer than four lots can share. A fit to 210 measured points (15 projections, 1024- and
 //   2048-wide, rank 16 to 64; 200 to 11000 rows of up to eight prompts, every K split with 1 to 16 groups): it loses 1.0 % to the best
 //   split of each, at most 17; one group and the largest K split 7.1; over 465 later points (1000 to 8000 rows, three widths) 0.7. us, that / the split taken: 2048 -> 2 x 6144, rank 64, 300, 700, 2000,
 //   4000 rows 22.5 / 13.6, 22.0 / 15.1, 29.5 / 27.9, 51.9 / 47.2; 2048 -> 2560 300 and 700 20.0 / 12.6, 19.4 / 15.4; 1024 -> 1024, rank 32,
 //   300 and 2000 7.9 / 7.4, 8.8 / 8.8. (A CTA's tiles, 1.1 us each, were half of the time where a block had one cluster: with groups a
 //   block can be 128 rows high and its columns still go to 16 CTAs and more.)
-//   LINEAR: set-up, the shrink's steps (more where one or two runs share a pass), the base product's (their latency over the stages of
+//   LINEAR: set-up, the shrink's steps (more where one or two lots share a pass), the base product's (their latency over the stages of
 //   the ring, then the bytes that all CTAs take), the exchange, the tiles: a regression over 3820 measured splits (12 projections as
 //   above, 64 to 4500 rows) that meets them within 8 %. Below that the sum does not tell, so the most K parts with one group stay
 //   unless another split promises 13 % less.
@@ -629,13 +642,13 @@ inline double prefill_cluster_split(bool linear, bool in_groups, int T, int in_d
         int stage;
         const int stages = prefill_cluster_linear_stages(tile_cols, width, off_tmp, rows * kGemmOutChunk * 2, &stage);
         if (stages == 0) continue;
-        const int runs = prefill_cluster_runs(true, width, std::max(tile_cols, width) * kSgmvBK * 2);
+        const int lots = prefill_cluster_lots(true, width, std::max(tile_cols, width) * kSgmvBK * 2);
         const double high = (double)rows / kSgmvBM, kb = (rows + tile_cols) * 0.128;
-        cost = 3.6 + nk_part * (0.27 + high * (0.06 + (runs == 1 ? 0.44 : runs == 2 ? 0.1 : 0.0))) +
+        cost = 3.6 + nk_part * (0.27 + high * (0.06 + (lots == 1 ? 0.44 : lots == 2 ? 0.1 : 0.0))) +
                tiles * nk * (0.042 + 0.87 / stages + kb * (0.0009 + 0.0015 * ctas / 148)) + 0.044 * exchange + tiles * (0.28 + 0.65 * tile_cols / kSgmvBN * high);
       } else {
         cost = nk_part * (rows + width) * (kSgmvBK * 2 / 70e3) + 0.05 * exchange + 0.35 * tiles + 0.1 * cols / kSgmvBN + (ctas > 74 ? 0.3 : 0.0) +
-               3.0 * (4 - prefill_cluster_runs(false, width, off_tmp));
+               3.0 * (4 - prefill_cluster_lots(false, width, off_tmp));
       }
       if (groups == 1) { one_group = cost; one_group_ck = ck; one_group_bm = rows; }  // (the most K parts come last)
       if (least < 0.0 || cost < least) {
@@ -673,9 +686,9 @@ inline bool prefill_cluster_plan(const SgmvProblem& b, int n, int n_total, bool 
   const int width = (a->groups > 1 ? prefill_cluster_need(*a, n, a->group_cols) : n) * b.r_max, out_buf = a->bm * kGemmOutChunk * 2;
   a->off_tmp = kPcSmem - width * kSgmvBM * 2;
   if (linear) {
-    // stages of an x and a W tile (or, ahead of the tiles, of the lora_A tiles of up to gmax runs), then output buffers
+    // stages of an x and a W tile (or, ahead of the tiles, of the lora_A tiles of up to gmax lots), then output buffers
     a->stages = prefill_cluster_linear_stages(a->tile_cols, width, a->off_tmp, out_buf, &a->stage_bytes);
-    a->gmax = prefill_cluster_runs(true, width, a->stage_bytes - kSgmvBM * kSgmvBK * 2);
+    a->gmax = prefill_cluster_lots(true, width, a->stage_bytes - kSgmvBM * kSgmvBK * 2);
     a->out_bufs = std::min(2, (a->off_tmp - a->stages * a->stage_bytes) / (2 * out_buf));
     a->part_cols = width;
     while (prefill_cluster_part_bytes(*a, a->part_cols) > 2 * a->out_bufs * out_buf) a->part_cols -= 16;  // (16 always fit)
@@ -684,7 +697,7 @@ inline bool prefill_cluster_plan(const SgmvProblem& b, int n, int n_total, bool 
     a->stage_bytes = a->tile_cols * b.r_max * 2;
     a->out_bufs = 2;
     while (a->stages > 2 && a->off_tmp - a->stages * a->stage_bytes < 2 * a->out_bufs * out_buf) --a->stages;
-    a->gmax = prefill_cluster_runs(false, width, a->off_tmp);
+    a->gmax = prefill_cluster_lots(false, width, a->off_tmp);
     a->part_cols = width;
   }
   a->off_out = a->stages * a->stage_bytes;

@@ -184,3 +184,51 @@ def test_linear_behind_a_shrink_matches_oracle(case):
     assert plan(T, in_dim, outs, r, LINEAR)[0] == kernel
     p = W.make_projection(520 + case, T, in_dim, outs, S, r, token_to_slot=slots, with_weight=True)
     check_linear(p, p.to_device(DEV), p.token_to_slot)
+
+
+# T, in, outs, S, r; form: independent rows, so that a block holds rows of every slot in any order
+SCATTERED = [
+    (64, 1024, [128, 64], 9, 32, ADD), (128, 256, [512], 128, 16, ADD), (333, 512, [256, 64, 64], 8, 64, ADD), (300, 192, [4032], 2, 32, ADD),
+    (4300, 128, [320], 5, 16, ADD),
+    (40, 512, [320], 6, 32, LINEAR), (517, 512, [1024, 128, 128], 9, 64, LINEAR), (1500, 512, [2048, 1088], 40, 16, LINEAR),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", range(len(SCATTERED)))
+def test_rows_of_a_slot_need_not_lie_together(case):
+    T, in_dim, outs, S, r, form = SCATTERED[case]
+    assert plan(T, in_dim, outs, r, form)[0] == CLUSTER
+    slots = torch.randint(-1, S, (T,), generator=torch.Generator().manual_seed(case), dtype=torch.int32)
+    slots[:4] = torch.tensor([0, -1, 1, 0])
+    p = W.make_projection(1010 + case, T, in_dim, outs, S, r, token_to_slot=slots, with_weight=form == LINEAR)
+    d = p.to_device(DEV)
+    if form == LINEAR:
+        return check_linear(p, d, slots)
+    y = d.y.clone()
+    LORA.launch_add(y, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata(slots), 0.5, impl=N.IMPL_SGMV)
+    torch.cuda.synchronize()
+    assert N.device_status(reset=True) == 0
+    assert_lora_close(y, O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, slots, 0.5, p.col_offsets), what="scattered rows")
+    none = slots < 0
+    assert torch.equal(y.cpu()[none].view(torch.int16), p.y[none].view(torch.int16)), "rows without adapter keep their bits"
+    if T <= 64:  # one block: a row's result does not depend on where it lies in it
+        order = slots.argsort(stable=True)
+        z = d.y[order.to(DEV)]
+        LORA.launch_add(z, d.x[order.to(DEV)], d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata(slots[order]), 0.5, impl=N.IMPL_SGMV)
+        assert torch.equal(z.view(torch.int16), y[order.to(DEV)].view(torch.int16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T, S, impl", [(333, 8, N.IMPL_BGMV), (511, 8, N.IMPL_BGMV), (511, 7, N.IMPL_SGMV), (512, 16, N.IMPL_SGMV), (512, 17, N.IMPL_BGMV)])
+def test_few_rows_a_bucket_stay_with_the_bucket_kernel(T, S, impl):
+    """Decode batches over few adapters, whose bytes alone would send them to the prefill kernel: 64 rows a bucket below 512 rows, 32 above."""
+    slots = torch.arange(T, dtype=torch.int32) * 7 % S
+    p = W.make_projection(1040, T, 2048, [6144, 6144], S, 64, token_to_slot=slots)
+    d = p.to_device(DEV)
+    y = [d.y.clone(), d.y.clone()]
+    for out, i in zip(y, (N.IMPL_AUTO, impl)):
+        LORA.launch_add(out, d.x, d.a_slabs, d.b_slabs, d.out_sizes, d.col_offsets, metadata(slots), 0.5, impl=i)
+    torch.cuda.synchronize()
+    assert N.device_status(reset=True) == 0 and torch.equal(*y)
+    assert_lora_close(y[0], O.add_lora(p.y, p.x, p.a_slabs, p.b_slabs, slots, 0.5, p.col_offsets), what="add")
